@@ -3,8 +3,7 @@
 // serves decode (one row per request), MTP verification (a few rows) and chunked
 // prefill rows.  The query heads that share a KV head are processed together so the
 // INT8 K/V rows are read once; long contexts are split along the key axis into
-// partial (max, sum, out) records that a second kernel merges.  INT8 values are
-// dequantised on the fly with their group-64 FP16 scales.  Replaces the decode
+// partial (max, sum, out) records that a second kernel merges.  Replaces the decode
 // configurations of causal_attention_int8 and merge_attention_int8
 // (kernels/cuda/model/attention_rows.py:61-276,280-400).
 #include "api.h"
@@ -14,228 +13,325 @@ namespace orinfer {
 
 constexpr int ATTN_WARPS = 4;
 
-__device__ __forceinline__ void unpack16(const int4& raw, float (&f)[16]) {
-  const int w[4] = {raw.x, raw.y, raw.z, raw.w};
-#pragma unroll
-  for (int i = 0; i < 4; ++i) {
-    f[4 * i + 0] = static_cast<float>(static_cast<signed char>(w[i] & 0xff));
-    f[4 * i + 1] = static_cast<float>(static_cast<signed char>((w[i] >> 8) & 0xff));
-    f[4 * i + 2] = static_cast<float>(static_cast<signed char>((w[i] >> 16) & 0xff));
-    f[4 * i + 3] = static_cast<float>(w[i] >> 24);
-  }
+// Two bytes of `x` (INT8 values plus 128, picked by `sel` from x and 0x64) -> two FP16 values,
+// exactly: 0x64xx is 1024 + xx, and 1152 is subtracted.
+__device__ __forceinline__ uint32_t int8x2_half2(uint32_t x, uint32_t sel) {
+  const uint32_t raw = __byte_perm(x, 0x64646464u, sel);
+  const __half2 v = __hsub2(*reinterpret_cast<const __half2*>(&raw),
+                            __half2half2(__ushort_as_half(0x6480)));
+  return *reinterpret_cast<const uint32_t*>(&v);
 }
 
-// One CTA per (row, group of RPC query heads sharing a KV head, key split).  A key's D INT8
-// channels are covered by D/16 lanes with one 16-byte load each, so a warp takes 32/(D/16)
-// keys per step (4 at D = 128) and the four warps interleave.  Keys are processed in chunks
-// of up to ATTN_CHUNK: pass 1 writes the scores of the chunk to shared memory, the softmax
-// weights are formed there once per (head, key), and pass 2 accumulates weight x V.  No
-// running rescale sits in the inner loops (only one per chunk), so both passes are streams
-// of independent multiply-adds.
-constexpr int ATTN_CHUNK = 512;
+__device__ __forceinline__ uint32_t pack_half2(__half a, __half b) {
+  const __half2 v = __halves2half2(a, b);
+  return *reinterpret_cast<const uint32_t*>(&v);
+}
 
-template <int D, int RPC>
-__global__ void __launch_bounds__(ATTN_WARPS * 32) attn_rows_kernel(
+// The G group scales of one cached row, packed as loaded (G = 1: upper half zero).  WIDE: the
+// scale tensor is aligned to a whole row of scales.
+template <int G, bool WIDE>
+struct RowScales {
+  uint32_t w[(G + 1) / 2];
+  __device__ __forceinline__ void load(const __half* p) {
+    if (G == 1 || !WIDE) {
+      const unsigned short* u = reinterpret_cast<const unsigned short*>(p);
+#pragma unroll
+      for (int i = 0; i < (G + 1) / 2; ++i)
+        w[i] = static_cast<uint32_t>(__ldg(u + 2 * i)) |
+               (G == 1 ? 0u : static_cast<uint32_t>(__ldg(u + 2 * i + 1)) << 16);
+    } else if (G == 2) {
+      w[0] = __ldg(reinterpret_cast<const uint32_t*>(p));
+    } else {
+      const uint2 v = __ldg(reinterpret_cast<const uint2*>(p));
+      w[0] = v.x;
+      w[(G + 1) / 2 - 1] = v.y;
+    }
+  }
+  __device__ __forceinline__ float get(int c) const {
+    const __half2 v = *reinterpret_cast<const __half2*>(&w[c / 2]);
+    return c & 1 ? __high2float(v) : __low2float(v);
+  }
+  __device__ __forceinline__ void clear() {
+#pragma unroll
+    for (int i = 0; i < (G + 1) / 2; ++i) w[i] = 0u;
+  }
+};
+
+// One CTA per (row, KV head, key split); its four warps take blocks of KB keys in turn (a block
+// lies inside one page) and carry their own softmax state, merged in shared memory at the end.
+//
+// Both products run on the tensor cores with the INT8 values as exact FP16 integers.
+//   S = Q K^T: rows 0..7 of A are the query heads; lane (g, t) loads 16 bytes of key g, which
+//   are its B fragments of four steps (the channel order inside a product does not matter, Q
+//   is laid out to match).  Each group of 64 channels is summed by itself and scaled in FP32.
+//   O = P V: the FP32 weight x value scale is split into an FP16 head and an FP16 remainder
+//   in rows g and g + 8 of the same A tile, so the split costs no instruction and keeps 22
+//   bits.  The weights are scaled by a power of two (2^14 over the largest value scale seen,
+//   exact) so that the remainder stays above the smallest FP16 step.
+template <int D>
+struct AttnTile {
+  static constexpr int G = D / 64;                 // scale groups per row
+  static constexpr int KB = D == 256 ? 16 : 32;    // keys per block
+  static constexpr int MIN_CTAS = D == 256 ? 2 : 3;
+};
+
+template <int D, bool WIDE>
+__global__ void __launch_bounds__(ATTN_WARPS * 32, AttnTile<D>::MIN_CTAS) attn_rows_kernel(
     const __half* __restrict__ q, const __half* __restrict__ gate, const int* __restrict__ row_req,
     const int* __restrict__ row_pos, const int* __restrict__ page_table, int max_pages,
     const int8_t* __restrict__ kc, const int8_t* __restrict__ vc, const __half* __restrict__ ks,
     const __half* __restrict__ vs, __half* __restrict__ out, int qh, int kvh, int splits,
     float* __restrict__ scratch, int rep) {
-  constexpr int LPK = D / 16;                  // lanes per key
-  constexpr int KPW = 32 / LPK;                // keys per warp step
-  constexpr int KPI = ATTN_WARPS * KPW;        // keys per CTA step
-  constexpr int GROUPS = D / 64;
-  constexpr int THREADS = ATTN_WARPS * 32;
-  const int row = blockIdx.x, split = blockIdx.z;
-  const int hgroups = rep / RPC;               // CTAs per KV head
-  const int h = blockIdx.y / hgroups;          // KV head
-  const int head0 = h * rep + (blockIdx.y % hgroups) * RPC;   // first query head of this CTA
+  constexpr int G = AttnTile<D>::G, KB = AttnTile<D>::KB;
+  constexpr int NT = KB / 8, UT = KB / 16;         // 8-key score tiles, 16-key value tiles
+  const int row = blockIdx.x, h = blockIdx.y, split = blockIdx.z;
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-  const int sub = lane % LPK, kslot = lane / LPK;
-  const int req = row_req[row];
+  const int g = lane >> 2, t = lane & 3;
   const int kv_len = row_pos[row] + 1;
   const int per = (kv_len + splits - 1) / splits;
   const int k_lo = split * per, k_hi = min(kv_len, k_lo + per);
-  const int group = (sub * 16) / 64;
+  const int* pages = page_table + static_cast<size_t>(row_req[row]) * max_pages;
   const float qscale = rsqrtf(static_cast<float>(D)) * 1.4426950408889634f;
 
-  // query heads (pre-scaled, FP32) in shared memory: every lane group reads the same slice,
-  // so the loads are broadcasts, and the registers go to the accumulators
-  __shared__ __align__(16) float s_q[RPC][D];
-  __shared__ float s_p[RPC][ATTN_CHUNK];       // scores, then softmax weights, of the chunk
-  __shared__ float s_red[ATTN_WARPS][RPC];
-  __shared__ float s_m[RPC], s_l[RPC], s_corr[RPC];
-  __shared__ float s_o[ATTN_WARPS][RPC][D];
-  __shared__ int s_page[ATTN_CHUNK / 128 + 2];  // page ids covering the chunk
-  for (int i = tid; i < RPC * D; i += THREADS)
-    s_q[i / D][i % D] =
-        __half2float(q[(static_cast<size_t>(row) * qh + head0 + i / D) * D + i % D]) * qscale;
-  if (tid < RPC) {
-    s_m[tid] = -INFINITY;
-    s_l[tid] = 0.f;
-  }
-  float acc[RPC][16];
-#pragma unroll
-  for (int r = 0; r < RPC; ++r)
-#pragma unroll
-    for (int e = 0; e < 16; ++e) acc[r][e] = 0.f;
-  __syncthreads();
-  const int* pages = page_table + static_cast<size_t>(req) * max_pages;
+  __shared__ __align__(16) float s_o[ATTN_WARPS][8][D];
+  __shared__ float s_m[ATTN_WARPS][8], s_l[ATTN_WARPS][8];
 
-  for (int c0 = k_lo; c0 < k_hi; c0 += ATTN_CHUNK) {
-    const int n = min(ATTN_CHUNK, k_hi - c0);
-    const int page0 = c0 >> 7;
-    if (tid <= ((c0 + n - 1) >> 7) - page0) s_page[tid] = pages[page0 + tid];
-    __syncthreads();
-    // slot of chunk key kk in the paged cache (page ids come from shared memory, so a key's
-    // address does not wait for a global load)
-    auto slot_of = [&](int kk) {
-      const int key = c0 + kk;
-      return (static_cast<size_t>(s_page[(key >> 7) - page0]) * 128 + (key & 127)) * kvh + h;
-    };
-    // ---- pass 1: scores of the chunk (loop uniform over the warp: the shuffles need every
-    // lane); the loads of the next step are issued before this step's arithmetic
-    float lmax[RPC];
+  // Query fragments in shared memory, one copy for the four warps (16 or 32 registers per lane
+  // buy more loads in flight): halves 4s..4s+3 of a lane's 16 are the A registers of step s.
+  __shared__ __align__(16) uint4 s_q[G][2][32];
+  if (warp == 0) {
 #pragma unroll
-    for (int r = 0; r < RPC; ++r) lmax[r] = -INFINITY;
-    int4 raw = make_int4(0, 0, 0, 0);
-    float sc_next = 0.f;
-    if (warp * KPW + kslot < n) {
-      const size_t slot = slot_of(warp * KPW + kslot);
-      raw = __ldg(reinterpret_cast<const int4*>(kc + slot * D + sub * 16));
-      sc_next = __half2float(ks[slot * GROUPS + group]);
-    }
-    for (int base = warp * KPW; base < n; base += KPI) {
-      const int kk = base + kslot;
-      const bool valid = kk < n;
-      float kf[16];
-      unpack16(raw, kf);
-      const float ksc = valid ? sc_next : 0.f;
-      if (kk + KPI < n) {
-        const size_t slot = slot_of(kk + KPI);
-        raw = __ldg(reinterpret_cast<const int4*>(kc + slot * D + sub * 16));
-        sc_next = __half2float(ks[slot * GROUPS + group]);
-      }
+    for (int c = 0; c < G; ++c) {
+      const __half* p = q + (static_cast<size_t>(row) * qh + h * rep + g) * D + c * 64 + t * 16;
+      uint32_t w[8];
 #pragma unroll
-      for (int r = 0; r < RPC; ++r) {
-        float d = 0.f;
+      for (int i = 0; i < 8; ++i) w[i] = 0u;
+      if (g < rep) {
+        if (WIDE) {
+          *reinterpret_cast<uint4*>(w) = __ldg(reinterpret_cast<const uint4*>(p));
+          *reinterpret_cast<uint4*>(w + 4) = __ldg(reinterpret_cast<const uint4*>(p) + 1);
+        } else {
 #pragma unroll
-        for (int e4 = 0; e4 < 4; ++e4) {
-          const float4 qq = *reinterpret_cast<const float4*>(&s_q[r][sub * 16 + e4 * 4]);
-          d += qq.x * kf[e4 * 4] + qq.y * kf[e4 * 4 + 1] + qq.z * kf[e4 * 4 + 2] +
-               qq.w * kf[e4 * 4 + 3];
-        }
-        d *= ksc;
-#pragma unroll
-        for (int o = 1; o < LPK; o <<= 1) d += __shfl_xor_sync(0xffffffffu, d, o);
-        if (valid) {
-          lmax[r] = fmaxf(lmax[r], d);
-          if (sub == 0) s_p[r][kk] = d;
+          for (int i = 0; i < 8; ++i) w[i] = pack_half2(p[2 * i], p[2 * i + 1]);
         }
       }
+      s_q[c][0][lane] = make_uint4(w[0], w[1], w[2], w[3]);
+      s_q[c][1][lane] = make_uint4(w[4], w[5], w[6], w[7]);
     }
-#pragma unroll
-    for (int r = 0; r < RPC; ++r) {
-      const float m = warp_max(lmax[r]);
-      if (lane == 0) s_red[warp][r] = m;
-    }
-    __syncthreads();
-    // ---- new running maximum, rescale factor of what was accumulated so far
-    if (tid < RPC) {
-      float m = s_m[tid];
-#pragma unroll
-      for (int w = 0; w < ATTN_WARPS; ++w) m = fmaxf(m, s_red[w][tid]);
-      s_corr[tid] = s_m[tid] == -INFINITY ? 0.f : exp2f(s_m[tid] - m);
-      s_m[tid] = m;
-    }
-    __syncthreads();
-    // ---- softmax weights of the chunk, once per (head, key)
-    float lsum[RPC];
-#pragma unroll
-    for (int r = 0; r < RPC; ++r) {
-      const float m = s_m[r];
-      float t = 0.f;
-      for (int kk = tid; kk < n; kk += THREADS) {
-        const float p = exp2f(s_p[r][kk] - m);
-        s_p[r][kk] = p;
-        t += p;
-      }
-      lsum[r] = warp_sum(t);
-    }
-    __syncthreads();                           // every warp is done with s_red's maxima
-    if (lane == 0) {
-#pragma unroll
-      for (int r = 0; r < RPC; ++r) s_red[warp][r] = lsum[r];
-    }
-    __syncthreads();
-    if (tid < RPC) {
-      float l = s_l[tid] * s_corr[tid];
-#pragma unroll
-      for (int w = 0; w < ATTN_WARPS; ++w) l += s_red[w][tid];
-      s_l[tid] = l;
-    }
-    if (c0 > k_lo) {
-#pragma unroll
-      for (int r = 0; r < RPC; ++r) {
-        const float c = s_corr[r];
-#pragma unroll
-        for (int e = 0; e < 16; ++e) acc[r][e] *= c;
-      }
-    }
-    // ---- pass 2: weight x V (same one-step-ahead loads)
-    if (warp * KPW + kslot < n) {
-      const size_t slot = slot_of(warp * KPW + kslot);
-      raw = __ldg(reinterpret_cast<const int4*>(vc + slot * D + sub * 16));
-      sc_next = __half2float(vs[slot * GROUPS + group]);
-    }
-    for (int base = warp * KPW; base < n; base += KPI) {
-      const int kk = base + kslot;
-      if (kk < n) {
-        float vf[16];
-        unpack16(raw, vf);
-        const float vsc = sc_next;
-        if (kk + KPI < n) {
-          const size_t slot = slot_of(kk + KPI);
-          raw = __ldg(reinterpret_cast<const int4*>(vc + slot * D + sub * 16));
-          sc_next = __half2float(vs[slot * GROUPS + group]);
-        }
-#pragma unroll
-        for (int r = 0; r < RPC; ++r) {
-          const float pv = s_p[r][kk] * vsc;
-#pragma unroll
-          for (int e = 0; e < 16; ++e) acc[r][e] += pv * vf[e];
-        }
-      }
-    }
-    __syncthreads();                           // s_p is rewritten by the next chunk
-  }
-  // lanes that only differ in kslot hold sums over disjoint key sets (same reference maximum)
-#pragma unroll
-  for (int o = LPK; o < 32; o <<= 1) {
-#pragma unroll
-    for (int r = 0; r < RPC; ++r)
-#pragma unroll
-      for (int e = 0; e < 16; ++e) acc[r][e] += __shfl_xor_sync(0xffffffffu, acc[r][e], o);
-  }
-  if (kslot == 0) {
-#pragma unroll
-    for (int r = 0; r < RPC; ++r)
-#pragma unroll
-      for (int e = 0; e < 16; ++e) s_o[warp][r][sub * 16 + e] = acc[r][e];
   }
   __syncthreads();
-  for (int i = tid; i < RPC * D; i += THREADS) {
-    const int r = i / D, d = i % D;
-    float o = 0.f;
+  const uint32_t q_addr = smem_u32(&s_q[0][0][lane]);
+  float acc[G * 8][4];
 #pragma unroll
-    for (int w = 0; w < ATTN_WARPS; ++w) o += s_o[w][r][d];
-    const float m = s_m[r], l = s_l[r];
-    const int head = head0 + r;
+  for (int i = 0; i < G * 8; ++i)
+#pragma unroll
+    for (int j = 0; j < 4; ++j) acc[i][j] = 0.f;
+  float m_run = -INFINITY, l_run = 0.f;
+  int e_run = -100;                                // the value scales seen are below 2^e_run
+
+  const int b_hi = k_hi > k_lo ? (k_hi + KB - 1) / KB : 0;
+  int b = k_hi > k_lo ? k_lo / KB + warp : 0;
+  uint4 kraw[NT][G];
+  // (page, first slot) of a block; the page id of the next block is fetched a block ahead
+  auto first_slot = [&](int blk, int page) {
+    return static_cast<size_t>(page) * 128 + ((blk * KB) & 127);
+  };
+  auto load_k = [&](size_t slot0) {
+#pragma unroll
+    for (int i = 0; i < NT; ++i) {
+      const int8_t* p = kc + ((slot0 + i * 8 + g) * kvh + h) * D + t * 16;
+#pragma unroll
+      for (int c = 0; c < G; ++c) kraw[i][c] = __ldg(reinterpret_cast<const uint4*>(p + c * 64));
+    }
+  };
+  int page_next = b + ATTN_WARPS < b_hi ? pages[((b + ATTN_WARPS) * KB) >> 7] : 0;
+  size_t slot0 = 0;
+  if (b < b_hi) {
+    slot0 = first_slot(b, pages[(b * KB) >> 7]);
+    load_k(slot0);
+  }
+  for (; b < b_hi; b += ATTN_WARPS) {
+    const int key0 = b * KB;
+    // values and scales of this block: in flight while the scores are formed
+    uint2 vraw[UT][4][G];
+    RowScales<G, WIDE> vsc[UT][4], ksc[NT][2];
+#pragma unroll
+    for (int i = 0; i < NT; ++i)
+#pragma unroll
+      for (int e = 0; e < 2; ++e)
+        ksc[i][e].load(ks + ((slot0 + i * 8 + 2 * t + e) * kvh + h) * G);
+#pragma unroll
+    for (int u = 0; u < UT; ++u)
+#pragma unroll
+      for (int e = 0; e < 4; ++e) {
+        const size_t cell = (slot0 + u * 16 + 2 * t + (e & 1) + (e >> 1) * 8) * kvh + h;
+#pragma unroll
+        for (int c = 0; c < G; ++c)
+          vraw[u][e][c] = __ldg(reinterpret_cast<const uint2*>(vc + cell * D + c * 64 + g * 8));
+        vsc[u][e].load(vs + cell * G);
+      }
+    // ---- scores: lane (g, t) gets head g against keys 8 i + 2 t and 8 i + 2 t + 1
+    float s[NT][2];
+#pragma unroll
+    for (int i = 0; i < NT; ++i) s[i][0] = s[i][1] = 0.f;
+#pragma unroll
+    for (int c = 0; c < G; ++c) {
+      uint32_t qf[8];
+#pragma unroll
+      for (int j = 0; j < 2; ++j)                     // volatile: not hoisted into registers
+        asm volatile("ld.shared.v4.u32 {%0, %1, %2, %3}, [%4];"
+                     : "=r"(qf[4 * j]), "=r"(qf[4 * j + 1]), "=r"(qf[4 * j + 2]), "=r"(qf[4 * j + 3])
+                     : "r"(q_addr + (c * 2 + j) * 512));
+#pragma unroll
+      for (int i = 0; i < NT; ++i) {
+        float d[4] = {0.f, 0.f, 0.f, 0.f};
+        const uint32_t w[4] = {kraw[i][c].x, kraw[i][c].y, kraw[i][c].z, kraw[i][c].w};
+#pragma unroll
+        for (int st = 0; st < 4; ++st) {
+          const uint32_t x = w[st] ^ 0x80808080u;
+          mma16816(d, qf[2 * st], 0u, qf[2 * st + 1], 0u, int8x2_half2(x, 0x4140),
+                   int8x2_half2(x, 0x4342));
+        }
+        s[i][0] = fmaf(d[0], ksc[i][0].get(c), s[i][0]);
+        s[i][1] = fmaf(d[1], ksc[i][1].get(c), s[i][1]);
+      }
+    }
+#pragma unroll
+    for (int i = 0; i < NT; ++i) {
+      s[i][0] *= qscale;
+      s[i][1] *= qscale;
+    }
+    if (key0 < k_lo || key0 + KB > k_hi) {
+      // keys outside the split: no weight, and their (possibly never written) scales unused
+#pragma unroll
+      for (int i = 0; i < NT; ++i)
+#pragma unroll
+        for (int e = 0; e < 2; ++e) {
+          const int key = key0 + i * 8 + 2 * t + e;
+          if (key < k_lo || key >= k_hi) {
+            s[i][e] = -INFINITY;
+            vsc[i >> 1][(i & 1) * 2 + e].clear();
+          }
+        }
+    }
+    // keys of the next block
+    if (b + ATTN_WARPS < b_hi) {
+      slot0 = first_slot(b + ATTN_WARPS, page_next);
+      load_k(slot0);
+      if (b + 2 * ATTN_WARPS < b_hi) page_next = pages[((b + 2 * ATTN_WARPS) * KB) >> 7];
+    }
+    // ---- softmax state
+    float mb = s[0][0], vmax = 0.f;
+#pragma unroll
+    for (int i = 0; i < NT; ++i) mb = fmaxf(mb, fmaxf(s[i][0], s[i][1]));
+#pragma unroll
+    for (int u = 0; u < UT; ++u)
+#pragma unroll
+      for (int e = 0; e < 4; ++e)
+#pragma unroll
+        for (int c = 0; c < G; ++c) vmax = fmaxf(vmax, fabsf(vsc[u][e].get(c)));
+    mb = fmaxf(mb, __shfl_xor_sync(0xffffffffu, mb, 1));
+    vmax = fmaxf(vmax, __shfl_xor_sync(0xffffffffu, vmax, 1));
+    mb = fmaxf(mb, __shfl_xor_sync(0xffffffffu, mb, 2));
+    vmax = fmaxf(vmax, __shfl_xor_sync(0xffffffffu, vmax, 2));
+    const int e_new = max(e_run, static_cast<int>(__float_as_uint(vmax) >> 23) - 126);
+    const float m_new = fmaxf(m_run, mb);
+    const float corr = m_run == -INFINITY ? 0.f : exp2f(m_run - m_new);
+    const bool same = m_new == m_run && e_new == e_run;
+    if (!__all_sync(0xffffffffu, same)) {
+      const float f = corr * __uint_as_float(static_cast<uint32_t>(127 + max(e_run - e_new, -126)) << 23);
+#pragma unroll
+      for (int i = 0; i < G * 8; ++i)
+#pragma unroll
+        for (int j = 0; j < 4; ++j) acc[i][j] *= f;
+    }
+    m_run = m_new;
+    e_run = e_new;
+    const float unit = __uint_as_float(static_cast<uint32_t>(127 + 14 - e_new) << 23);
+    float lsum = 0.f;
+#pragma unroll
+    for (int i = 0; i < NT; ++i)
+#pragma unroll
+      for (int e = 0; e < 2; ++e) {
+        s[i][e] = exp2f(s[i][e] - m_new);
+        lsum += s[i][e];
+      }
+    l_run = fmaf(l_run, corr, lsum);
+    // ---- values
+#pragma unroll
+    for (int u = 0; u < UT; ++u) {
+#pragma unroll
+      for (int c = 0; c < G; ++c) {
+        __half hi[4], lo[4];
+#pragma unroll
+        for (int e = 0; e < 4; ++e) {
+          const float p = s[2 * u + (e >> 1)][e & 1] * (vsc[u][e].get(c) * unit);
+          hi[e] = __float2half_rn(p);
+          lo[e] = __float2half_rn(p - __half2float(hi[e]));
+        }
+        const uint32_t a0 = pack_half2(hi[0], hi[1]), a1 = pack_half2(lo[0], lo[1]);
+        const uint32_t a2 = pack_half2(hi[2], hi[3]), a3 = pack_half2(lo[2], lo[3]);
+#pragma unroll
+        for (int wd = 0; wd < 2; ++wd) {
+          uint32_t x[4];
+#pragma unroll
+          for (int e = 0; e < 4; ++e)
+            x[e] = (wd == 0 ? vraw[u][e][c].x : vraw[u][e][c].y) ^ 0x80808080u;
+          // bytes of two keys interleaved: (k0 b0, k1 b0, k0 b1, k1 b1), then b2 and b3
+          const uint32_t p01 = __byte_perm(x[0], x[1], 0x5140), p23 = __byte_perm(x[0], x[1], 0x7362);
+          const uint32_t r01 = __byte_perm(x[2], x[3], 0x5140), r23 = __byte_perm(x[2], x[3], 0x7362);
+          float(*o)[4] = &acc[c * 8 + wd * 4];
+          mma16816(o[0], a0, a1, a2, a3, int8x2_half2(p01, 0x4140), int8x2_half2(r01, 0x4140));
+          mma16816(o[1], a0, a1, a2, a3, int8x2_half2(p01, 0x4342), int8x2_half2(r01, 0x4342));
+          mma16816(o[2], a0, a1, a2, a3, int8x2_half2(p23, 0x4140), int8x2_half2(r23, 0x4140));
+          mma16816(o[3], a0, a1, a2, a3, int8x2_half2(p23, 0x4342), int8x2_half2(r23, 0x4342));
+        }
+      }
+    }
+  }
+  // ---- this warp's result: head + remainder rows, back to the unscaled weights
+  l_run += __shfl_xor_sync(0xffffffffu, l_run, 1);
+  l_run += __shfl_xor_sync(0xffffffffu, l_run, 2);
+  const float back = __uint_as_float(static_cast<uint32_t>(127 + max(e_run - 14, -126)) << 23);
+  if (g < rep) {
+#pragma unroll
+    for (int c = 0; c < G; ++c)
+#pragma unroll
+      for (int n = 0; n < 2; ++n) {
+        float* dst = &s_o[warp][g][c * 64 + (2 * t + n) * 8];
+#pragma unroll
+        for (int j = 0; j < 8; j += 4) {
+          float4 v;
+          v.x = (acc[c * 8 + j][n] + acc[c * 8 + j][n + 2]) * back;
+          v.y = (acc[c * 8 + j + 1][n] + acc[c * 8 + j + 1][n + 2]) * back;
+          v.z = (acc[c * 8 + j + 2][n] + acc[c * 8 + j + 2][n + 2]) * back;
+          v.w = (acc[c * 8 + j + 3][n] + acc[c * 8 + j + 3][n + 2]) * back;
+          *reinterpret_cast<float4*>(dst + j) = v;
+        }
+      }
+    if (t == 0) {
+      s_m[warp][g] = m_run;
+      s_l[warp][g] = l_run;
+    }
+  }
+  __syncthreads();
+  for (int i = tid; i < rep * D; i += ATTN_WARPS * 32) {
+    const int r = i / D, d = i % D, head = h * rep + r;
+    float m = s_m[0][r];
+#pragma unroll
+    for (int w = 1; w < ATTN_WARPS; ++w) m = fmaxf(m, s_m[w][r]);
+    float o = 0.f, l = 0.f;
+#pragma unroll
+    for (int w = 0; w < ATTN_WARPS; ++w) {
+      const float f = s_m[w][r] == -INFINITY ? 0.f : exp2f(s_m[w][r] - m);
+      o = fmaf(s_o[w][r][d], f, o);
+      l = fmaf(s_l[w][r], f, l);
+    }
     if (splits == 1) {
       float v = l > 0.f ? o / l : 0.f;
       if (gate) {
-        const float g = __half2float(gate[(static_cast<size_t>(row) * qh + head) * D + d]);
-        v *= __fdiv_rn(1.f, 1.f + expf(-g));
+        const float gv = __half2float(gate[(static_cast<size_t>(row) * qh + head) * D + d]);
+        v *= __fdiv_rn(1.f, 1.f + expf(-gv));
       }
       out[(static_cast<size_t>(row) * qh + head) * D + d] = __float2half_rn(v);
     } else {
@@ -274,15 +370,17 @@ __global__ void attn_merge_kernel(const float* __restrict__ scratch,
   }
 }
 
-template <int D, int RPC>
+template <int D>
 static int launch_attn(const __half* q, const __half* gate, const int* row_req, const int* row_pos,
                        const int* page_table, int max_pages, const int8_t* kc, const int8_t* vc,
                        const __half* ks, const __half* vs, __half* out, int rows, int qh, int kvh,
                        int rep, int splits, float* scratch, cudaStream_t stream) {
-  dim3 grid(rows, kvh * (rep / RPC), splits);
-  attn_rows_kernel<D, RPC><<<grid, ATTN_WARPS * 32, 0, stream>>>(
-      q, gate, row_req, row_pos, page_table, max_pages, kc, vc, ks, vs, out, qh, kvh, splits,
-      scratch, rep);
+  dim3 grid(rows, kvh, splits);
+  const bool wide = ((reinterpret_cast<uintptr_t>(q) & 15) | (reinterpret_cast<uintptr_t>(ks) & 7) |
+                     (reinterpret_cast<uintptr_t>(vs) & 7)) == 0;
+  auto kernel = wide ? attn_rows_kernel<D, true> : attn_rows_kernel<D, false>;
+  kernel<<<grid, ATTN_WARPS * 32, 0, stream>>>(q, gate, row_req, row_pos, page_table, max_pages, kc,
+                                               vc, ks, vs, out, qh, kvh, splits, scratch, rep);
   if (splits > 1)
     attn_merge_kernel<D><<<dim3(rows, qh), D < 128 ? 64 : 128, 0, stream>>>(scratch, gate, out, qh,
                                                                            splits);
@@ -306,15 +404,13 @@ extern "C" int orinfer_attention(const __half* q, const __half* gate, const int*
   if (rows <= 0) return 0;
   if (splits < 1 || (splits > 1 && scratch == nullptr) || kvh <= 0 || qh % kvh) return -1;
   const int rep = qh / kvh;
-  // query heads per CTA: all heads of a KV head up to 5; 8 run as two groups of 4 (their
-  // accumulators would not fit the register file)
-#define CASE(DD, RR, RPC)                                                                     \
-  if (head_dim == DD && rep == RR)                                                            \
-    return launch_attn<DD, RPC>(q, gate, row_req, row_pos, page_table, max_pages, kc, vc, ks, \
-                                vs, out, rows, qh, kvh, rep, splits, scratch, stream);
-  CASE(64, 1, 1) CASE(64, 2, 2) CASE(64, 4, 4) CASE(64, 8, 4)
-  CASE(128, 1, 1) CASE(128, 2, 2) CASE(128, 4, 4) CASE(128, 5, 5) CASE(128, 8, 4)
-  CASE(256, 1, 1) CASE(256, 2, 2) CASE(256, 4, 4) CASE(256, 8, 4)
+#define CASE(DD)                                                                            \
+  if (head_dim == DD)                                                                       \
+    return launch_attn<DD>(q, gate, row_req, row_pos, page_table, max_pages, kc, vc, ks, vs, \
+                           out, rows, qh, kvh, rep, splits, scratch, stream);
+  // query heads per KV head: the eight rows of a score tile (five only at D = 128)
+  if (rep != 1 && rep != 2 && rep != 4 && rep != 8 && !(rep == 5 && head_dim == 128)) return -1;
+  CASE(64) CASE(128) CASE(256)
 #undef CASE
   return -1;
 }

@@ -205,6 +205,19 @@ __device__ __forceinline__ void mma_f16_ss(uint32_t tmem_d, uint64_t adesc, uint
       : "memory");
 }
 
+// ---------------------------------------------------------------- warp-level MMA
+// D += A B on 16 x 8 x 16 FP16 tiles with FP32 accumulators.  Lane (g = lane / 4, t = lane % 4)
+// holds A rows g and g + 8, B column g, and C rows g (c[0..1]) and g + 8 (c[2..3]) at columns
+// 2t and 2t + 1.
+__device__ __forceinline__ void mma16816(float (&c)[4], uint32_t a0, uint32_t a1, uint32_t a2,
+                                         uint32_t a3, uint32_t b0, uint32_t b1) {
+  asm volatile(
+      "mma.sync.aligned.m16n8k16.row.col.f32.f16.f16.f32 {%0, %1, %2, %3}, {%4, %5, %6, %7}, "
+      "{%8, %9}, {%0, %1, %2, %3};"
+      : "+f"(c[0]), "+f"(c[1]), "+f"(c[2]), "+f"(c[3])
+      : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1));
+}
+
 // ---------------------------------------------------------------- CTA pairs (cta_group::2)
 // Two CTAs of a cluster drive one MMA of 256 rows: each holds its 128 rows of A and its half
 // of the B rows in its own shared memory, the even CTA issues the instruction, and each

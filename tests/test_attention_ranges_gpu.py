@@ -1,0 +1,76 @@
+"""Attention kernels at the edges of their tiles and ranges, against 64-bit statements."""
+import math
+
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.fixture(scope="module")
+def dev(cuda):
+    from orinfer_b200.ops import native
+    native.init()
+    return cuda
+
+
+def _unaligned(t):
+    """A contiguous copy whose address is two bytes past a 16-byte boundary."""
+    flat = torch.empty(t.numel() + 8, dtype=t.dtype, device=t.device)
+    out = flat[1:1 + t.numel()].view(t.shape)
+    out.copy_(t)
+    return out
+
+
+def _attention64(q, k, v, ks, vs, gate=None):
+    """q [QH, D] against every row of k, v [T, KVH, D] with group scales [T, KVH, D / 64]."""
+    qh, d = q.shape
+    kk = (k.double().reshape(*k.shape[:2], -1, 64) * ks.double()[..., None]).reshape(k.shape)
+    vv = (v.double().reshape(*v.shape[:2], -1, 64) * vs.double()[..., None]).reshape(v.shape)
+    rep = qh // k.shape[1]
+    s = torch.einsum("hd,thd->ht", q.double(), kk.repeat_interleave(rep, 1)) / math.sqrt(d)
+    o = torch.einsum("ht,thd->hd", torch.softmax(s, 1), vv.repeat_interleave(rep, 1))
+    return o if gate is None else o * torch.sigmoid(gate.double())
+
+
+# contexts around the 16- / 32-key blocks, the pages and the splits
+@pytest.mark.parametrize("qh,kvh,d", [(2, 2, 64), (4, 2, 64), (16, 2, 64), (3, 3, 128), (4, 2, 128),
+                                      (8, 2, 128), (10, 2, 128), (8, 1, 128), (2, 1, 256),
+                                      (8, 1, 256), (4, 1, 256)])
+@pytest.mark.parametrize("splits,wide", [(1, True), (5, True), (3, False)])
+def test_attention_rows_at_block_edges(dev, qh, kvh, d, splits, wide):
+    from orinfer_b200.ops import functional as F
+    g = torch.Generator().manual_seed(qh * 1000 + d + splits)
+    lens = [1, 2, 15, 16, 17, 31, 33, 127, 128, 129, 160, 257, 700]
+    pages = sum((n + 127) // 128 for n in lens) + 1
+    table = torch.zeros(len(lens), 6, dtype=torch.int32)
+    at = 1
+    for i, n in enumerate(lens):
+        for j in range((n + 127) // 128):
+            table[i, j] = at
+            at += 1
+    kc = torch.randint(-127, 128, (pages, 128, kvh, d), generator=g, dtype=torch.int8).to(dev)
+    vc = torch.randint(-127, 128, (pages, 128, kvh, d), generator=g, dtype=torch.int8).to(dev)
+    # value scales over many binades: the weights are rescaled as larger ones turn up
+    ks = (torch.rand(pages, 128, kvh, d // 64, generator=g) * 0.02 + 1e-3).half().to(dev)
+    vs = torch.exp2(torch.rand(pages, 128, kvh, d // 64, generator=g) * 18 - 14).half().to(dev)
+    for i, n in enumerate(lens):                    # slots never written hold anything
+        last = int(table[i, (n - 1) // 128])
+        ks[last, (n - 1) % 128 + 1:] = float("nan")
+        vs[last, (n - 1) % 128 + 1:] = float("inf")
+    q = torch.randn(len(lens), qh, d, generator=g).half().to(dev)
+    gate = torch.randn(len(lens), qh, d, generator=g).half().to(dev) if d == 256 else None
+    if not wide:
+        q, ks, vs = _unaligned(q), _unaligned(ks), _unaligned(vs)
+    t = lambda v: torch.tensor(v, dtype=torch.int32, device=dev)
+    out = F.attention(q, gate, t(list(range(len(lens)))), t([n - 1 for n in lens]), table.to(dev),
+                      kc, vc, ks, vs, splits=splits)
+    for i, n in enumerate(lens):
+        pg = table[i, :(n + 127) // 128].long().to(dev)
+        rows = lambda c: c[pg].reshape(-1, *c.shape[2:])[:n]
+        ref = _attention64(q[i], rows(kc), rows(vc), rows(ks), rows(vs),
+                           None if gate is None else gate[i]).reshape(-1)
+        # one FP16 rounding (2^-11 of the value) on top of FP32 sums over terms that may cancel:
+        # a few 2^-22 of the largest value
+        lim = ref.abs() * 2.0 ** -11 + 2.0 ** -18 * ref.abs().max() + 2.0 ** -25
+        assert bool(((out[i].double() - ref).abs() <= lim).all()), (n, float((out[i] - ref).abs().max()))
