@@ -90,7 +90,86 @@ __global__ void __launch_bounds__(D) gdn_conv_kernel(
   y[static_cast<size_t>(row) * conv_dim + c] = __float2half_rn(val);
 }
 
-// One CTA per segment: new history = last three pre-conv rows of (old history ++ chunk).
+// The same convolution, eight channels per thread (16-byte loads and stores) over R consecutive
+// rows: the three earlier rows stay in registers, so a packet's rows are read once instead of
+// four times two bytes at a time.  A head is D / 8 neighbouring lanes.  Grid (row strips,
+// conv_dim / 2048); R = 1 for decode-sized packets, where the strips would be too few CTAs.
+// 2100 rows x 8192 channels: 89 -> 35 us; 64 rows: 7.9 -> 5.6 us.  What is left is the SiLU.
+template <int D, int R>
+__global__ void __launch_bounds__(256) gdn_conv_vec_kernel(
+    const __half* __restrict__ x, int x_stride, const __half* __restrict__ weight,
+    const __half* __restrict__ hist, const int* __restrict__ row_first,
+    const int* __restrict__ row_slot, const int* __restrict__ row_pos, int rows, int conv_dim,
+    int qk_channels, __half* __restrict__ y) {
+  constexpr int LANES = D / 8;
+  const int c = (blockIdx.y * 256 + threadIdx.x) * 8, row0 = blockIdx.x * R;
+  if (c >= conv_dim) return;                       // whole heads, so whole lane groups
+  const unsigned group = LANES == 32 ? 0xffffffffu
+                                     : ((1u << LANES) - 1u) << (threadIdx.x & 31 & ~(LANES - 1));
+  uint4 wr[4];
+#pragma unroll
+  for (int i = 0; i < 4; ++i)
+    wr[i] = __ldg(reinterpret_cast<const uint4*>(weight + static_cast<size_t>(c) * 4) + i);
+  const __half* wh = reinterpret_cast<const __half*>(wr);
+  uint4 win[4];                                    // rows row-3 .. row (as loaded)
+#pragma unroll
+  for (int j = 0; j < 3; ++j) {
+    const int src = row0 - 3 + j;
+    win[j + 1] = src >= 0 ? __ldg(reinterpret_cast<const uint4*>(
+                                x + static_cast<size_t>(src) * x_stride + c))
+                          : make_uint4(0, 0, 0, 0);
+  }
+#pragma unroll
+  for (int r = 0; r < R; ++r) {
+    const int row = row0 + r;
+    if (row >= rows) break;
+#pragma unroll
+    for (int j = 0; j < 3; ++j) win[j] = win[j + 1];
+    win[3] = __ldg(reinterpret_cast<const uint4*>(x + static_cast<size_t>(row) * x_stride + c));
+    const int first = row_first[row];
+    uint4 tap[3] = {win[0], win[1], win[2]};
+    if (row - first < 3) {                         // rows before the run come from its history
+      const bool fresh = row_pos[first] == 0;
+      const int slot = row_slot[row];
+#pragma unroll
+      for (int j = 0; j < 3; ++j) {
+        const int back = first - (row - 3 + j);    // 1..3 rows before the run
+        if (back > 0)
+          tap[j] = fresh ? make_uint4(0, 0, 0, 0)
+                         : *reinterpret_cast<const uint4*>(
+                               hist + (static_cast<size_t>(slot) * 3 + (3 - back)) * conv_dim + c);
+      }
+    }
+    float val[8], ss = 0.f;
+#pragma unroll
+    for (int e = 0; e < 8; ++e) {
+      float acc = 0.f;
+#pragma unroll
+      for (int j = 0; j < 4; ++j)
+        acc = fmaf(__half2float(reinterpret_cast<const __half*>(j < 3 ? &tap[j] : &win[3])[e]),
+                   __half2float(wh[e * 4 + j]), acc);
+      val[e] = round_f16(acc * __fdiv_rn(1.f, 1.f + expf(-acc)));
+      ss = fmaf(val[e], val[e], ss);
+    }
+    if (c < qk_channels) {
+#pragma unroll
+      for (int o = 1; o < LANES; o <<= 1) ss += __shfl_xor_sync(group, ss, o);
+      const float inv = rsqrtf(ss + 1e-6f);
+#pragma unroll
+      for (int e = 0; e < 8; ++e) val[e] *= inv;
+    }
+    __align__(16) __half h[8];
+#pragma unroll
+    for (int e = 0; e < 8; ++e) h[e] = __float2half_rn(val[e]);
+    *reinterpret_cast<uint4*>(y + static_cast<size_t>(row) * conv_dim + c) =
+        *reinterpret_cast<const uint4*>(h);
+  }
+}
+
+// New history = last three pre-conv rows of (old history ++ chunk).  grid (segments, channel
+// blocks); VEC channels per thread.  (One CTA per segment with 2-byte accesses took 21 us for
+// 64 segments, this form 2.9 us.)
+template <int VEC>
 __global__ void __launch_bounds__(256) gdn_history_kernel(const __half* __restrict__ x,
                                                           int x_stride,
                                                           const Segment* __restrict__ segs,
@@ -102,21 +181,31 @@ __global__ void __launch_bounds__(256) gdn_history_kernel(const __half* __restri
   Segment s = segs[blockIdx.x];
   if (accepted != nullptr) {                 // commit of a verified prefix of the rows
     s.rows = min(accepted[blockIdx.x], s.rows);
-    if (s.rows <= 0) return;
   }
+  if (s.rows <= 0) return;
+  const int c = (blockIdx.y * 256 + threadIdx.x) * VEC;
+  if (c >= conv_dim) return;
+  struct __align__(VEC * 2) Chunk {
+    __half h[VEC];
+  };
   const bool fresh = row_pos[s.row_start] == 0;
   __half* h = hist + static_cast<size_t>(row_slot[s.row_start]) * 3 * conv_dim;
-  for (int c = threadIdx.x; c < conv_dim; c += blockDim.x) {
-    __half v[3];
+  Chunk v[3];
 #pragma unroll
-    for (int j = 0; j < 3; ++j) {
-      const int idx = s.rows - 3 + j;                  // index into the chunk, < 0 = history
-      v[j] = idx >= 0 ? x[static_cast<size_t>(s.row_start + idx) * x_stride + c]
-                      : (fresh ? __float2half(0.f) : h[static_cast<size_t>(3 + idx) * conv_dim + c]);
+  for (int j = 0; j < 3; ++j) {
+    const int idx = s.rows - 3 + j;          // index into the chunk, < 0 = history
+    if (idx >= 0) {
+      v[j] = *reinterpret_cast<const Chunk*>(x + static_cast<size_t>(s.row_start + idx) * x_stride + c);
+    } else if (fresh) {
+#pragma unroll
+      for (int i = 0; i < VEC; ++i) v[j].h[i] = __float2half(0.f);
+    } else {
+      v[j] = *reinterpret_cast<const Chunk*>(h + static_cast<size_t>(3 + idx) * conv_dim + c);
     }
-#pragma unroll
-    for (int j = 0; j < 3; ++j) h[static_cast<size_t>(j) * conv_dim + c] = v[j];
   }
+#pragma unroll
+  for (int j = 0; j < 3; ++j)
+    *reinterpret_cast<Chunk*>(h + static_cast<size_t>(j) * conv_dim + c) = v[j];
 }
 
 // ---------------------------------------------------------------- sequential scan
@@ -133,7 +222,7 @@ __global__ void __launch_bounds__(256) gdn_scan_kernel(
     const float* __restrict__ a_log, const float* __restrict__ dt_bias,
     const Segment* __restrict__ segs, const int* __restrict__ row_slot,
     const int* __restrict__ row_pos, int hk, int hv, float* __restrict__ state,
-    float* __restrict__ out, float* __restrict__ factors) {
+    float* __restrict__ out, float* __restrict__ factors, int long_rows) {
   // factors != nullptr: a verification pass.  The state is NOT written back; instead every
   // step records (decay, k[D], delta[D]) so that gdn_commit can replay exactly the accepted
   // prefix of the rows onto the stored state.
@@ -141,7 +230,7 @@ __global__ void __launch_bounds__(256) gdn_scan_kernel(
   static_assert(ROWS % 4 == 0, "four independent accumulators");
   const int vh = blockIdx.x / SPLIT, c0 = (blockIdx.x % SPLIT) * DC;
   const Segment seg = segs[blockIdx.y];
-  if (seg.rows <= 0) return;
+  if (seg.rows <= 0 || seg.rows >= long_rows) return;  // long runs: gdn_chunk_kernel
   const int kh = vh / (hv / hk);
   const int dv = c0 + threadIdx.x % DC, part_id = threadIdx.x / DC;
   const int slot = row_slot[seg.row_start];
@@ -251,12 +340,12 @@ __global__ void __launch_bounds__(256) gdn_scan_split_kernel(
     const float* __restrict__ a_log, const float* __restrict__ dt_bias,
     const Segment* __restrict__ segs, const int* __restrict__ row_slot,
     const int* __restrict__ row_pos, int hk, int hv, float* __restrict__ state,
-    float* __restrict__ out, float* __restrict__ factors) {
+    float* __restrict__ out, float* __restrict__ factors, int long_rows) {
   constexpr int DC = 32, SPLIT = D / DC, PARTS = 8, ROWS = D / PARTS, T = SCAN_STEPS;
   constexpr int CH = D / 4 + DC / 8;                 // 16-byte units of one staged row
   const int vh = blockIdx.x / SPLIT, c0 = (blockIdx.x % SPLIT) * DC;
   const Segment seg = segs[blockIdx.y];
-  if (seg.rows <= 0) return;
+  if (seg.rows <= 0 || seg.rows >= long_rows) return;  // long runs: gdn_chunk_kernel
   const int kh = vh / (hv / hk);
   const int col = threadIdx.x >> 3, part = threadIdx.x & 7;
   const int slot = row_slot[seg.row_start];
@@ -385,6 +474,408 @@ __global__ void __launch_bounds__(256) gdn_scan_split_kernel(
   }
 }
 
+// ---------------------------------------------------------------- chunked form
+// Long runs (prefill) in chunks of 32 rows: inside a chunk the recurrence is a triangular system
+// and everything else is a matrix product, so a chunk costs a few thousand cycles instead of 32
+// dependent steps.  With G_i the running sum of log decays inside the chunk and S the state
+// before it,
+//   A[i][j] = beta_i e^(G_i - G_j) k_i.k_j (j < i),   T = (I + A)^-1
+//   Delta   = T B,  B_i = beta_i (v_i - e^G_i S^T k_i)
+//   o_i     = e^G_i S^T q_i + sum_{j <= i} P[i][j] Delta_j,  P[i][j] = e^(G_i - G_j) q_i.k_j
+//   S      <- e^G_32 S + sum_j k_j (x) e^(G_32 - G_j) Delta_j
+// grid (2 HV, segments), six warps.  Warps 0..3 own 16 value channels each and keep their
+// 16 x 128 slice of S^T in registers as MMA accumulators, whose layout is also that of an A
+// operand: S^T K^T, B^T T^T, Delta^T P^T and Delta^T K chain through registers and no warp
+// waits for another inside a chunk.  Warps 4 (A, T) and 5 (P) prepare the next chunk, which
+// does not depend on the state, while the chunk after that is copied in.
+//
+// Precision: k, q and v are FP16 and enter products exactly; FP32 operands are split in two
+// (FP16 halves under a power-of-two scale: 22 bits; TF32 pairs: 22 bits) and all sums are FP32.
+// The G are summed in FP64 so that e^(G_i - G_j) keeps FP32 accuracy when |G| is large.
+//
+// 32 heads of 128 channels, two runs of 1050 rows: 610 us as a scan (0.29 us per dependent step),
+// 227 us here.  Runs below GDN_LONG_ROWS keep the scan: two chunks cost about as much as 64 steps,
+// and verification packets (at most 32 rows) must reproduce the scan's bits.
+constexpr int GDN_LONG_ROWS = 64;
+constexpr int CHUNK = 32, CHUNK_THREADS = 192;
+struct ChunkSmem {
+  __half k[3][CHUNK][136], q[3][CHUNK][136];   // rows padded to 17 16-byte units (ldmatrix)
+  __half v[3][CHUNK][72];
+  float t[2][CHUNK][40], p[2][CHUNK][40];      // T and P, row i, column j
+  float at[CHUNK][36];                         // A transposed: [j][i]
+  double g[2][CHUNK];                          // G, one copy per helper warp
+  float eg[2][CHUNK], beta[2][CHUNK], tail[2][CHUNK], total[2];
+};
+
+__device__ __forceinline__ void ldsm_x4(uint32_t (&r)[4], const void* p) {
+  asm volatile("ldmatrix.sync.aligned.m8n8.x4.shared.b16 {%0, %1, %2, %3}, [%4];"
+               : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3])
+               : "r"(smem_u32(p))
+               : "memory");
+}
+__device__ __forceinline__ void ldsm_x4_t(uint32_t (&r)[4], const void* p) {
+  asm volatile("ldmatrix.sync.aligned.m8n8.x4.trans.shared.b16 {%0, %1, %2, %3}, [%4];"
+               : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3])
+               : "r"(smem_u32(p))
+               : "memory");
+}
+// D += A B on 16 x 8 x 8 TF32 tiles: lane (g, t) holds A rows g, g + 8 at k = t (a0, a1) and
+// k = t + 4 (a2, a3), B column g at k = t and t + 4.
+__device__ __forceinline__ void mma_tf32(float (&c)[4], const uint32_t (&a)[4], uint32_t b0,
+                                         uint32_t b1) {
+  asm volatile(
+      "mma.sync.aligned.m16n8k8.row.col.f32.tf32.tf32.f32 {%0, %1, %2, %3}, {%4, %5, %6, %7}, "
+      "{%8, %9}, {%0, %1, %2, %3};"
+      : "+f"(c[0]), "+f"(c[1]), "+f"(c[2]), "+f"(c[3])
+      : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1));
+}
+__device__ __forceinline__ uint32_t to_tf32(float x) {
+  uint32_t r;
+  asm("cvt.rna.tf32.f32 %0, %1;" : "=r"(r) : "f"(x));
+  return r;
+}
+__device__ __forceinline__ void split_tf32(float x, uint32_t& hi, uint32_t& lo) {
+  hi = to_tf32(x);
+  lo = to_tf32(x - __uint_as_float(hi));
+}
+// FP16 head and remainder of two values (already scaled into the FP16 range)
+__device__ __forceinline__ void split_half2(float x, float y, uint32_t& hi, uint32_t& lo) {
+  const __half2 h = __floats2half2_rn(x, y);
+  const float2 f = __half22float2(h);
+  const __half2 l = __floats2half2_rn(x - f.x, y - f.y);
+  hi = *reinterpret_cast<const uint32_t*>(&h);
+  lo = *reinterpret_cast<const uint32_t*>(&l);
+}
+// e with |x| < 2^e (at least -100, at most 129) and powers of two
+__device__ __forceinline__ int bound_exp(float x) {
+  return max(-100, static_cast<int>((__float_as_uint(x) >> 23) & 255u) - 126);
+}
+__device__ __forceinline__ float pow2i(int e) {
+  return __uint_as_float(static_cast<uint32_t>(127 + e) << 23);
+}
+
+// D[i][0..7] (u-th group of eight columns) += X^T(16 x 32) M^T for a lower triangular 32 x 32
+// matrix M in shared memory: X and M split into TF32 pairs.
+__device__ __forceinline__ void mul_lower(float (&d)[4][4], const float (&x)[4][4],
+                                          const float (*m)[40], int g, int t) {
+#pragma unroll
+  for (int s = 0; s < 4; ++s) {
+    uint32_t hi[4], lo[4];
+    // k index t is row 8s + 2t of X, k index t + 4 is row 8s + 2t + 1
+    split_tf32(x[s][0], hi[0], lo[0]);
+    split_tf32(x[s][2], hi[1], lo[1]);
+    split_tf32(x[s][1], hi[2], lo[2]);
+    split_tf32(x[s][3], hi[3], lo[3]);
+#pragma unroll
+    for (int u = s; u < 4; ++u) {
+      const float2 b = *reinterpret_cast<const float2*>(&m[8 * u + g][8 * s + 2 * t]);
+      uint32_t bh0, bl0, bh1, bl1;
+      split_tf32(b.x, bh0, bl0);
+      split_tf32(b.y, bh1, bl1);
+      mma_tf32(d[u], hi, bl0, bl1);
+      mma_tf32(d[u], lo, bh0, bh1);
+      mma_tf32(d[u], hi, bh0, bh1);
+    }
+  }
+}
+
+__global__ void __launch_bounds__(CHUNK_THREADS, 2) gdn_chunk_kernel(
+    const __half* __restrict__ qkv, int conv_dim, const float* __restrict__ ab,
+    const float* __restrict__ a_log, const float* __restrict__ dt_bias,
+    const Segment* __restrict__ segs, const int* __restrict__ row_slot,
+    const int* __restrict__ row_pos, int hk, int hv, float* __restrict__ state,
+    float* __restrict__ out) {
+  constexpr int D = 128;
+  extern __shared__ __align__(16) unsigned char chunk_smem[];
+  ChunkSmem& sm = *reinterpret_cast<ChunkSmem*>(chunk_smem);
+  const Segment seg = segs[blockIdx.y];
+  if (seg.rows < GDN_LONG_ROWS) return;
+  const int vh = blockIdx.x >> 1, kh = vh / (hv / hk), dk_total = hk * D;
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, g = lane >> 2, t = lane & 3;
+  const int mat = lane >> 3, mrow = lane & 7;          // this lane's row in an ldmatrix
+  const int dv0 = (blockIdx.x & 1) * 64;
+  const int chunks = (seg.rows + CHUNK - 1) / CHUNK;
+  const float scale = rsqrtf(static_cast<float>(D));
+
+  // copy of one chunk: 16 + 16 + 8 16-byte units per row; rows past the run become zeros
+  auto stage = [&](int c) {
+    const int st = c % 3, n = min(CHUNK, seg.rows - c * CHUNK);
+    for (int i = tid; i < CHUNK * 40; i += CHUNK_THREADS) {
+      const int r = i / 40, u = i % 40;
+      const __half* row = qkv + static_cast<size_t>(seg.row_start + c * CHUNK + min(r, n - 1)) * conv_dim;
+      const __half* src;
+      __half* dst;
+      if (u < 16) {
+        src = row + kh * D + u * 8;
+        dst = &sm.q[st][r][u * 8];
+      } else if (u < 32) {
+        src = row + dk_total + kh * D + (u - 16) * 8;
+        dst = &sm.k[st][r][(u - 16) * 8];
+      } else {
+        src = row + 2 * dk_total + vh * D + dv0 + (u - 32) * 8;
+        dst = &sm.v[st][r][(u - 32) * 8];
+      }
+      const unsigned a = smem_u32(dst), bytes = r < n ? 16 : 0;
+      asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(a), "l"(src), "r"(bytes)
+                   : "memory");
+    }
+    asm volatile("cp.async.commit_group;" ::: "memory");
+  };
+
+  // ---- helpers: everything of chunk c that does not depend on the state
+  const float alog = expf(a_log[vh]), bias = dt_bias[vh];
+  float n_a = 0.f, n_b = 0.f;
+  auto fetch_gates = [&](int c) {
+    const int r = c * CHUNK + lane;
+    if (r < seg.rows) {
+      const size_t row = static_cast<size_t>(seg.row_start + r);
+      n_a = ab[row * 2 * hv + vh];
+      n_b = ab[row * 2 * hv + hv + vh];
+    }
+  };
+  auto prepare = [&](int c) {
+    const int st = c % 3, buf = c & 1, helper = warp - 4;
+    const bool live = c * CHUNK + lane < seg.rows;
+    const float xg = n_a + bias;
+    const float softplus = xg > 20.f ? xg : log1pf(expf(xg));
+    double big_g = live ? static_cast<double>(-alog * softplus) : 0.0;
+    const float beta = live ? __fdiv_rn(1.f, 1.f + expf(-n_b)) : 0.f;
+    if (c + 1 < chunks) fetch_gates(c + 1);
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+      const double up = __shfl_up_sync(0xffffffffu, big_g, o);
+      if (lane >= o) big_g += up;
+    }
+    const double last = __shfl_sync(0xffffffffu, big_g, 31);
+    sm.g[helper][lane] = big_g;
+    if (helper == 0) {
+      sm.eg[buf][lane] = expf(static_cast<float>(big_g));
+      sm.beta[buf][lane] = beta;
+      sm.tail[buf][lane] = expf(static_cast<float>(last - big_g));
+      if (lane == 0) sm.total[buf] = expf(static_cast<float>(last));
+    }
+    __syncwarp();
+    // rows of X (k or q) times rows of k, the blocks on and below the diagonal:
+    // acc[0..1] rows 0..15 x columns 0..15, acc[2..5] rows 16..31 x columns 0..31
+    const __half(*xs)[136] = helper == 0 ? sm.k[st] : sm.q[st];
+    float acc[6][4];
+#pragma unroll
+    for (int i = 0; i < 6; ++i)
+#pragma unroll
+      for (int j = 0; j < 4; ++j) acc[i][j] = 0.f;
+#pragma unroll
+    for (int s = 0; s < D / 16; ++s) {
+      uint32_t x0[4], x1[4], k0[4], k1[4];
+      const int r = (mat & 1) * 8 + mrow, col = s * 16 + (mat >> 1) * 8;
+      ldsm_x4(k0, &sm.k[st][r][col]);
+      ldsm_x4(k1, &sm.k[st][16 + r][col]);
+      if (helper == 0) {
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+          x0[i] = k0[i];
+          x1[i] = k1[i];
+        }
+      } else {
+        ldsm_x4(x0, &xs[r][col]);
+        ldsm_x4(x1, &xs[16 + r][col]);
+      }
+      mma16816(acc[0], x0[0], x0[1], x0[2], x0[3], k0[0], k0[2]);
+      mma16816(acc[1], x0[0], x0[1], x0[2], x0[3], k0[1], k0[3]);
+      mma16816(acc[2], x1[0], x1[1], x1[2], x1[3], k0[0], k0[2]);
+      mma16816(acc[3], x1[0], x1[1], x1[2], x1[3], k0[1], k0[3]);
+      mma16816(acc[4], x1[0], x1[1], x1[2], x1[3], k1[0], k1[2]);
+      mma16816(acc[5], x1[0], x1[1], x1[2], x1[3], k1[1], k1[3]);
+    }
+#pragma unroll
+    for (int i = 0; i < 6; ++i) {
+      const int i0 = i < 2 ? 0 : 16, j0 = i < 2 ? i * 8 : (i - 2) * 8;
+#pragma unroll
+      for (int e = 0; e < 4; ++e) {
+        const int ri = i0 + g + (e >> 1) * 8, cj = j0 + 2 * t + (e & 1);
+        const float d = expf(static_cast<float>(fmin(sm.g[helper][ri] - sm.g[helper][cj], 0.0)));
+        if (helper == 0) {
+          const float b = __shfl_sync(0xffffffffu, beta, ri);
+          sm.at[cj][ri] = cj < ri ? b * d * acc[i][e] : 0.f;
+        } else {
+          sm.p[buf][ri][cj] = cj <= ri ? scale * d * acc[i][e] : 0.f;
+        }
+      }
+    }
+    if (helper == 0) {
+      __syncwarp();
+      // column `lane` of T by forward substitution: subtract A's column j times T's row j
+      float x[CHUNK];
+#pragma unroll
+      for (int i = 0; i < CHUNK; ++i) x[i] = i == lane ? 1.f : 0.f;
+#pragma unroll
+      for (int j = 0; j < CHUNK - 1; ++j) {
+#pragma unroll
+        for (int i4 = (j + 1) / 4; i4 < CHUNK / 4; ++i4) {
+          const float4 a = *reinterpret_cast<const float4*>(&sm.at[j][i4 * 4]);
+          if (i4 * 4 > j) x[i4 * 4] = fmaf(-a.x, x[j], x[i4 * 4]);
+          if (i4 * 4 + 1 > j) x[i4 * 4 + 1] = fmaf(-a.y, x[j], x[i4 * 4 + 1]);
+          if (i4 * 4 + 2 > j) x[i4 * 4 + 2] = fmaf(-a.z, x[j], x[i4 * 4 + 2]);
+          x[i4 * 4 + 3] = fmaf(-a.w, x[j], x[i4 * 4 + 3]);
+        }
+      }
+#pragma unroll
+      for (int i = 0; i < CHUNK; ++i) sm.t[buf][i][lane] = x[i];
+      __syncwarp();                            // A is rewritten by the next chunk
+    }
+  };
+
+  stage(0);
+  if (chunks > 1) stage(1);
+  if (warp >= 4) fetch_gates(0);
+
+  // ---- this warp's slice of S^T: rows dv, columns dk = 8 u + 2 t (+ 1)
+  const bool fresh = row_pos[seg.row_start] == 0;
+  const int dv = dv0 + (warp & 3) * 16 + g;
+  float* sp = state + (static_cast<size_t>(row_slot[seg.row_start]) * hv + vh) * D * D + dv;
+  float s_acc[16][4];
+  float s_max = 0.f;
+  if (warp < 4) {
+#pragma unroll
+    for (int u = 0; u < 16; ++u)
+#pragma unroll
+      for (int e = 0; e < 4; ++e) {
+        s_acc[u][e] = fresh ? 0.f : sp[(8 * u + 2 * t + (e & 1)) * D + (e >> 1) * 8];
+        s_max = fmaxf(s_max, fabsf(s_acc[u][e]));
+      }
+  }
+  asm volatile("cp.async.wait_group 0;" ::: "memory");
+  __syncthreads();
+  if (warp >= 4) prepare(0);
+  __syncthreads();
+
+  for (int c = 0; c < chunks; ++c) {
+    if (c + 2 < chunks) stage(c + 2);          // its buffer was last read in round c - 1
+    if (warp >= 4) {
+      if (c + 1 < chunks) prepare(c + 1);
+    } else {
+      const int st = c % 3, buf = c & 1;
+      const int e_s = bound_exp(warp_max(s_max));
+      const float up = pow2i(14 - e_s), down = pow2i(e_s - 14);
+      // ---- S^T k and S^T q: columns are the chunk's rows
+      float ak[4][4], aq[4][4];
+#pragma unroll
+      for (int i = 0; i < 4; ++i)
+#pragma unroll
+        for (int j = 0; j < 4; ++j) ak[i][j] = aq[i][j] = 0.f;
+#pragma unroll
+      for (int s = 0; s < D / 16; ++s) {
+        uint32_t hi[4], lo[4];
+        split_half2(s_acc[2 * s][0] * up, s_acc[2 * s][1] * up, hi[0], lo[0]);
+        split_half2(s_acc[2 * s][2] * up, s_acc[2 * s][3] * up, hi[1], lo[1]);
+        split_half2(s_acc[2 * s + 1][0] * up, s_acc[2 * s + 1][1] * up, hi[2], lo[2]);
+        split_half2(s_acc[2 * s + 1][2] * up, s_acc[2 * s + 1][3] * up, hi[3], lo[3]);
+#pragma unroll
+        for (int half = 0; half < 2; ++half) {
+          uint32_t bk[4], bq[4];
+          const int r = half * 16 + (mat >> 1) * 8 + mrow, col = s * 16 + (mat & 1) * 8;
+          ldsm_x4(bk, &sm.k[st][r][col]);
+          ldsm_x4(bq, &sm.q[st][r][col]);
+#pragma unroll
+          for (int v = 0; v < 2; ++v) {
+            mma16816(ak[half * 2 + v], lo[0], lo[1], lo[2], lo[3], bk[2 * v], bk[2 * v + 1]);
+            mma16816(aq[half * 2 + v], lo[0], lo[1], lo[2], lo[3], bq[2 * v], bq[2 * v + 1]);
+          }
+#pragma unroll
+          for (int v = 0; v < 2; ++v) {
+            mma16816(ak[half * 2 + v], hi[0], hi[1], hi[2], hi[3], bk[2 * v], bk[2 * v + 1]);
+            mma16816(aq[half * 2 + v], hi[0], hi[1], hi[2], hi[3], bq[2 * v], bq[2 * v + 1]);
+          }
+        }
+      }
+      // ---- B^T, and e^G S^T q as the start of the output
+#pragma unroll
+      for (int v = 0; v < 4; ++v) {
+        const int r = 8 * v + 2 * t;
+        const float2 eg = *reinterpret_cast<const float2*>(&sm.eg[buf][r]);
+        const float2 be = *reinterpret_cast<const float2*>(&sm.beta[buf][r]);
+#pragma unroll
+        for (int e = 0; e < 4; ++e) {
+          const float ge = (e & 1 ? eg.y : eg.x) * down;
+          const float val = __half2float(sm.v[st][r + (e & 1)][(warp & 3) * 16 + g + (e >> 1) * 8]);
+          ak[v][e] = (e & 1 ? be.y : be.x) * fmaf(-ge, ak[v][e], val);
+          aq[v][e] *= ge * scale;
+        }
+      }
+      float dl[4][4];
+#pragma unroll
+      for (int i = 0; i < 4; ++i)
+#pragma unroll
+        for (int j = 0; j < 4; ++j) dl[i][j] = 0.f;
+      mul_lower(dl, ak, sm.t[buf], g, t);
+      mul_lower(aq, dl, sm.p[buf], g, t);
+      const int n = min(CHUNK, seg.rows - c * CHUNK);
+#pragma unroll
+      for (int v = 0; v < 4; ++v)
+#pragma unroll
+        for (int e = 0; e < 4; ++e) {
+          const int r = 8 * v + 2 * t + (e & 1);
+          if (r < n)
+            out[(static_cast<size_t>(seg.row_start + c * CHUNK + r) * hv + vh) * D + dv +
+                (e >> 1) * 8] = aq[v][e];
+        }
+      // ---- state update
+      float d_max = 0.f;
+#pragma unroll
+      for (int v = 0; v < 4; ++v) {
+        const float2 tl = *reinterpret_cast<const float2*>(&sm.tail[buf][8 * v + 2 * t]);
+#pragma unroll
+        for (int e = 0; e < 4; ++e) {
+          dl[v][e] *= e & 1 ? tl.y : tl.x;
+          d_max = fmaxf(d_max, fabsf(dl[v][e]));
+        }
+      }
+      const int e_d = bound_exp(warp_max(d_max));
+      const float dup = pow2i(14 - e_d), ddown = pow2i(e_d - 14), total = sm.total[buf];
+      uint32_t hi[2][4], lo[2][4];
+#pragma unroll
+      for (int r = 0; r < 2; ++r)
+#pragma unroll
+        for (int i = 0; i < 4; ++i)
+          split_half2(dl[2 * r + (i >> 1)][(i & 1) * 2] * dup,
+                      dl[2 * r + (i >> 1)][(i & 1) * 2 + 1] * dup, hi[r][i], lo[r][i]);
+      s_max = 0.f;
+#pragma unroll
+      for (int u = 0; u < 16; u += 2) {
+        float add[2][4];
+#pragma unroll
+        for (int j = 0; j < 2; ++j)
+#pragma unroll
+          for (int e = 0; e < 4; ++e) add[j][e] = 0.f;
+#pragma unroll
+        for (int r = 0; r < 2; ++r) {
+          uint32_t b[4];
+          ldsm_x4_t(b, &sm.k[st][r * 16 + (mat & 1) * 8 + mrow][(u + (mat >> 1)) * 8]);
+          mma16816(add[0], lo[r][0], lo[r][1], lo[r][2], lo[r][3], b[0], b[1]);
+          mma16816(add[1], lo[r][0], lo[r][1], lo[r][2], lo[r][3], b[2], b[3]);
+          mma16816(add[0], hi[r][0], hi[r][1], hi[r][2], hi[r][3], b[0], b[1]);
+          mma16816(add[1], hi[r][0], hi[r][1], hi[r][2], hi[r][3], b[2], b[3]);
+        }
+#pragma unroll
+        for (int j = 0; j < 2; ++j)
+#pragma unroll
+          for (int e = 0; e < 4; ++e) {
+            s_acc[u + j][e] = fmaf(s_acc[u + j][e], total, add[j][e] * ddown);
+            s_max = fmaxf(s_max, fabsf(s_acc[u + j][e]));
+          }
+      }
+    }
+    asm volatile("cp.async.wait_group 0;" ::: "memory");
+    __syncthreads();
+  }
+  if (warp < 4) {
+#pragma unroll
+    for (int u = 0; u < 16; ++u)
+#pragma unroll
+      for (int e = 0; e < 4; ++e)
+        sp[(8 * u + 2 * t + (e & 1)) * D + (e >> 1) * 8] = s_acc[u][e];
+  }
+}
+
 // Replays the first accepted[seg] recorded steps of every segment onto the stored state:
 // S = decay * S + k (x) delta, in row order.  Same thread layout as the scan.
 template <int D>
@@ -438,6 +929,78 @@ __global__ void __launch_bounds__(D) gdn_gated_norm_kernel(
   y[(static_cast<size_t>(row) * hv + h) * D + d] = __float2half_rn(n * gate);
 }
 
+// The same, one warp per (row, head): D / 32 neighbouring channels per lane, eight heads per
+// CTA, no block barrier.  2100 rows x 32 heads of 128: 37 -> 17 us (69 MB).
+template <int D>
+__global__ void __launch_bounds__(256) gdn_gated_norm_warp_kernel(
+    const float* __restrict__ o, const __half* __restrict__ z, int z_stride,
+    const __half* __restrict__ w, float eps, int sigmoid_gate, int hv, long long items,
+    __half* __restrict__ y) {
+  constexpr int V = D / 32;
+  struct __align__(V * 2) Half {
+    __half h[V];
+  };
+  struct __align__(V * 4) Float {
+    float f[V];
+  };
+  const long long item = static_cast<long long>(blockIdx.x) * 8 + (threadIdx.x >> 5);
+  if (item >= items) return;
+  const int lane = threadIdx.x & 31;
+  const long long row = item / hv;
+  const int h = static_cast<int>(item - row * hv);
+  const Float v = *reinterpret_cast<const Float*>(o + item * D + lane * V);
+  const Half zh = *reinterpret_cast<const Half*>(z + row * z_stride + h * D + lane * V);
+  const Half wh = *reinterpret_cast<const Half*>(w + lane * V);
+  float ss = 0.f;
+#pragma unroll
+  for (int i = 0; i < V; ++i) ss = fmaf(v.f[i], v.f[i], ss);
+  const float r = rsqrtf(warp_sum(ss) / D + eps);
+  Half out;
+#pragma unroll
+  for (int i = 0; i < V; ++i) {
+    const float n = v.f[i] * r * __half2float(wh.h[i]);
+    const float zf = __half2float(zh.h[i]);
+    const float sg = __fdiv_rn(1.f, 1.f + expf(-zf));
+    out.h[i] = __float2half_rn(n * (sigmoid_gate ? sg : zf * sg));
+  }
+  *reinterpret_cast<Half*>(y + item * D + lane * V) = out;
+}
+
+inline bool aligned(const void* p, size_t bytes) {
+  return reinterpret_cast<uintptr_t>(p) % bytes == 0;
+}
+
+template <int D>
+static void launch_conv(const __half* x, int x_stride, const __half* weight, const __half* hist,
+                        const int* row_first, const int* row_slot, const int* row_pos, int rows,
+                        int conv_dim, int hk, __half* y, cudaStream_t stream) {
+  const bool vec = x_stride % 8 == 0 && aligned(x, 16) && aligned(weight, 16) &&
+                   aligned(hist, 16) && aligned(y, 16);
+  if (!vec) {
+    gdn_conv_kernel<D><<<dim3(rows, conv_dim / D), D, 0, stream>>>(
+        x, x_stride, weight, hist, row_first, row_slot, row_pos, conv_dim, 2 * hk, y);
+    return;
+  }
+  const int cols = (conv_dim + 2047) / 2048;
+  if (rows * cols >= 8 * 4 * 148)                // strips of eight rows still fill the machine
+    gdn_conv_vec_kernel<D, 8><<<dim3((rows + 7) / 8, cols), 256, 0, stream>>>(
+        x, x_stride, weight, hist, row_first, row_slot, row_pos, rows, conv_dim, 2 * hk * D, y);
+  else
+    gdn_conv_vec_kernel<D, 1><<<dim3(rows, cols), 256, 0, stream>>>(
+        x, x_stride, weight, hist, row_first, row_slot, row_pos, rows, conv_dim, 2 * hk * D, y);
+}
+
+static void launch_history(const __half* x, int x_stride, const Segment* segs, int n_segs,
+                           const int* row_slot, const int* row_pos, int conv_dim, __half* hist,
+                           const int* accepted, cudaStream_t stream) {
+  if (x_stride % 8 == 0 && aligned(x, 16) && aligned(hist, 16))
+    gdn_history_kernel<8><<<dim3(n_segs, (conv_dim + 2047) / 2048), 256, 0, stream>>>(
+        x, x_stride, segs, row_slot, row_pos, conv_dim, hist, accepted);
+  else
+    gdn_history_kernel<1><<<dim3(n_segs, (conv_dim + 255) / 256), 256, 0, stream>>>(
+        x, x_stride, segs, row_slot, row_pos, conv_dim, hist, accepted);
+}
+
 }  // namespace orinfer
 
 using namespace orinfer;
@@ -462,17 +1025,15 @@ int orinfer_gdn_conv(const __half* x, int x_stride, const __half* weight, __half
   if (rows <= 0) return 0;
   if (head_dim != 128 && head_dim != 64) return -1;
   const int conv_dim = (2 * hk + hv) * head_dim;
-  dim3 grid(rows, 2 * hk + hv);
   if (head_dim == 128)
-    gdn_conv_kernel<128><<<grid, 128, 0, stream>>>(x, x_stride, weight, hist, row_first, row_slot,
-                                                   row_pos, conv_dim, 2 * hk, y);
+    launch_conv<128>(x, x_stride, weight, hist, row_first, row_slot, row_pos, rows, conv_dim, hk, y,
+                     stream);
   else
-    gdn_conv_kernel<64><<<grid, 64, 0, stream>>>(x, x_stride, weight, hist, row_first, row_slot,
-                                                 row_pos, conv_dim, 2 * hk, y);
-  if (update_history)
-    gdn_history_kernel<<<n_segs, 256, 0, stream>>>(x, x_stride,
-                                                   reinterpret_cast<const Segment*>(segs),
-                                                   row_slot, row_pos, conv_dim, hist, nullptr);
+    launch_conv<64>(x, x_stride, weight, hist, row_first, row_slot, row_pos, rows, conv_dim, hk, y,
+                    stream);
+  if (update_history && n_segs > 0)
+    launch_history(x, x_stride, reinterpret_cast<const Segment*>(segs), n_segs, row_slot, row_pos,
+                   conv_dim, hist, nullptr, stream);
   return static_cast<int>(cudaGetLastError());
 }
 
@@ -487,8 +1048,7 @@ int orinfer_gdn_commit(const __half* x, int x_stride, const float* factors, cons
   if (head_dim != 128 && head_dim != 64) return -1;
   const Segment* sg = reinterpret_cast<const Segment*>(segs);
   const int conv_dim = (2 * hk + hv) * head_dim;
-  gdn_history_kernel<<<n_segs, 256, 0, stream>>>(x, x_stride, sg, row_slot, row_pos, conv_dim,
-                                                 hist, accepted);
+  launch_history(x, x_stride, sg, n_segs, row_slot, row_pos, conv_dim, hist, accepted, stream);
   if (head_dim == 128)
     gdn_commit_kernel<128><<<dim3(hv, n_segs), 256, 0, stream>>>(factors, sg, accepted, row_slot,
                                                                 row_pos, hv, state);
@@ -503,7 +1063,7 @@ int orinfer_gdn_commit(const __half* x, int x_stride, const float* factors, cons
 int orinfer_gdn_scan(const __half* qkv, const float* ab, const float* a_log, const float* dt_bias,
                      const int* segs, int n_segs, const int* row_slot, const int* row_pos, int hk,
                      int hv, int head_dim, float* state, float* out, cudaStream_t stream,
-                     float* factors) {
+                     float* factors, int max_seg_rows) {
   if (n_segs <= 0) return 0;
   if ((head_dim != 128 && head_dim != 64) || hv % hk) return -1;
   const Segment* sg = reinterpret_cast<const Segment*>(segs);
@@ -512,10 +1072,25 @@ int orinfer_gdn_scan(const __half* qkv, const float* ab, const float* a_log, con
   // each head over D/32 CTAs.  The rule depends on the segment count only, so a verification
   // pass and the plain pass over the same requests take the same arithmetic.
   const bool split = static_cast<long long>(hv) * n_segs < 2 * 148;
+  // Runs of at least GDN_LONG_ROWS rows take the chunked kernel (which skips the others, as the
+  // scan skips them); verification passes and 64-channel heads never do.
+  int long_rows = 0x7fffffff;
+  if (head_dim == 128 && factors == nullptr && max_seg_rows >= GDN_LONG_ROWS &&
+      aligned(qkv, 16)) {
+    long_rows = GDN_LONG_ROWS;
+    static const int slot = runtime_new_slot();
+    if (runtime_first_use(slot)) {
+      const cudaError_t e = cudaFuncSetAttribute(
+          gdn_chunk_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, sizeof(ChunkSmem));
+      if (e != cudaSuccess) return static_cast<int>(e);
+    }
+    gdn_chunk_kernel<<<dim3(hv * 2, n_segs), CHUNK_THREADS, sizeof(ChunkSmem), stream>>>(
+        qkv, conv_dim, ab, a_log, dt_bias, sg, row_slot, row_pos, hk, hv, state, out);
+  }
 #define ORINFER_SCAN(KERNEL, GRID_X)                                                       \
   KERNEL<<<dim3(GRID_X, n_segs), 256, 0, stream>>>(qkv, conv_dim, ab, a_log, dt_bias, sg,  \
                                                    row_slot, row_pos, hk, hv, state, out,  \
-                                                   factors)
+                                                   factors, long_rows)
   if (head_dim == 128) {
     if (split) ORINFER_SCAN(gdn_scan_split_kernel<128>, hv * 4);
     else ORINFER_SCAN((gdn_scan_kernel<128, 128>), hv);
@@ -531,6 +1106,20 @@ int orinfer_gdn_gated_norm(const float* o, const __half* z, int z_stride, const 
                            float eps, int sigmoid_gate, int rows, int hv, int head_dim,
                            __half* y, cudaStream_t stream) {
   if (rows <= 0) return 0;
+  if (head_dim != 128 && head_dim != 64) return -1;
+  const int v = head_dim / 32;
+  if (z_stride % v == 0 && aligned(z, 2 * v) && aligned(w, 2 * v) && aligned(o, 4 * v) &&
+      aligned(y, 2 * v)) {
+    const long long items = static_cast<long long>(rows) * hv;
+    const unsigned grid = static_cast<unsigned>((items + 7) / 8);
+    if (head_dim == 128)
+      gdn_gated_norm_warp_kernel<128><<<grid, 256, 0, stream>>>(o, z, z_stride, w, eps,
+                                                               sigmoid_gate, hv, items, y);
+    else
+      gdn_gated_norm_warp_kernel<64><<<grid, 256, 0, stream>>>(o, z, z_stride, w, eps,
+                                                              sigmoid_gate, hv, items, y);
+    return static_cast<int>(cudaGetLastError());
+  }
   if (head_dim == 128)
     gdn_gated_norm_kernel<128><<<dim3(rows, hv), 128, 0, stream>>>(o, z, z_stride, w, eps,
                                                                    sigmoid_gate, hv, y);

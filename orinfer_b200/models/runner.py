@@ -355,7 +355,7 @@ class ModelRunner:
         F.gdn_conv(proj, lw.gdn_conv, st["hist"][j], p.row_first, p.row_req, p.row_pos,
                    p.segments, p.n_segments, rows, hk, hv, d, out=st["conv"],
                    update_history=not p.tentative)
-        F.gdn_scan(st["conv"], st["ab"], lw.gdn_a_log, lw.gdn_dt_bias, p.segments, p.n_segments,
+        F.gdn_scan(st["conv"][:rows], st["ab"], lw.gdn_a_log, lw.gdn_dt_bias, p.segments, p.n_segments,
                    p.row_req, p.row_pos, hk, hv, d, st["state"][j], out=st["o"], factors=factors)
         F.gdn_gated_norm(st["o"], proj[:, conv_dim:], lw.gdn_norm, cfg.eps, rows, hv, d,
                          out=st["mix"])

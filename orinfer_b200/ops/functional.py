@@ -375,17 +375,20 @@ def gdn_scan(qkv: torch.Tensor, ab: torch.Tensor, a_log: torch.Tensor, dt_bias: 
              factors: Optional[torch.Tensor] = None) -> torch.Tensor:
     """Sequential gated-delta recurrence; ``state`` fp32 [slots, HV, D, D] updated in place.
     With ``factors`` (fp32 [rows, HV, 2D+1]) the state is left untouched and every step's
-    (decay, k, delta) is recorded for :func:`gdn_commit`."""
+    (decay, k, delta) is recorded for :func:`gdn_commit`.  ``qkv`` should have no more rows than
+    the packet: its row count bounds the longest segment, and only packets that may hold a run
+    of 64 rows or more launch the chunked kernel beside the scan."""
     _cuda(qkv, ab, a_log, dt_bias, segs, state, row_slot, row_pos)
     assert ab.dtype == torch.float32 and state.dtype == torch.float32 and state.is_contiguous()
     assert a_log.dtype == torch.float32 and dt_bias.dtype == torch.float32
     if out is None:
         out = torch.empty(qkv.shape[0], hv, head_dim, dtype=torch.float32, device=qkv.device)
+    longest = qkv.shape[0] - (n_segs - 1)
     check(native.lib().orinfer_gdn_scan(ptr(qkv), ptr(ab), ptr(a_log), ptr(dt_bias), ptr(segs),
                                         n_segs, ptr(row_slot), ptr(row_pos), hk, hv, head_dim,
-                                        ptr(state), ptr(out), stream(), ptr(factors)),
+                                        ptr(state), ptr(out), stream(), ptr(factors), longest),
           "gdn_scan")
-    count_launches(1)
+    count_launches(2 if longest >= 64 and head_dim == 128 and factors is None else 1)
     return out
 
 

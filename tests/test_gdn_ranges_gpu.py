@@ -1,0 +1,135 @@
+"""Recurrent-mixer kernels at the edges of their ranges, against 64-bit statements."""
+import math
+
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.fixture(scope="module")
+def dev(cuda):
+    from orinfer_b200.ops import native
+    native.init()
+    return cuda
+
+
+def _unaligned(t):
+    """A contiguous copy whose address is two bytes past a 16-byte boundary."""
+    flat = torch.empty(t.numel() + 8, dtype=t.dtype, device=t.device)
+    out = flat[1:1 + t.numel()].view(t.shape)
+    out.copy_(t)
+    return out
+
+
+def _recurrence64(q, k, v, g, beta, s):
+    o = torch.empty_like(v)
+    for i in range(v.shape[0]):
+        s = s * torch.exp(g[i])[:, None, None]
+        delta = beta[i][:, None] * (v[i] - torch.einsum("hk,hkv->hv", k[i], s))
+        s = s + k[i][:, :, None] * delta[:, None, :]
+        o[i] = torch.einsum("hk,hkv->hv", q[i], s)
+    return o, s
+
+
+@pytest.mark.parametrize("lens", [[64], [63, 65], [5, 96, 1, 97], [200, 2, 64, 129], [333]])
+@pytest.mark.parametrize("strength", [0.3, 4.0])
+def test_gdn_scan_long_and_short_runs(dev, lens, strength):
+    """Runs on both sides of the chunked kernel's limit, ragged tails, fresh and continued
+    states, mild and very strong decay (running sums of log decays down to several thousand)."""
+    from orinfer_b200.ops import functional as F
+    torch.manual_seed(sum(lens))
+    hk, hv, d = 2, 4, 128
+    rows = sum(lens)
+    a_log = (torch.randn(hv) * 0.5 + strength).to(dev)
+    dt = (torch.randn(hv) * 0.5 - 2).to(dev)
+    ab = torch.randn(rows, 2 * hv, device=dev)
+    qk = torch.nn.functional.normalize(torch.randn(rows, 2 * hk, d, device=dev), dim=-1)
+    v = torch.randn(rows, hv, d, device=dev) * 3
+    qkv = torch.cat([qk.reshape(rows, -1), v.reshape(rows, -1)], 1).half()
+    state = torch.randn(len(lens) + 2, hv, d, d, device=dev) * 0.2
+    start = state.double()
+    segs, slot, pos, at = [], [], [], 0
+    for i, n in enumerate(lens):
+        segs.append([at, n, 0, 0])
+        slot += [i + 1] * n
+        pos += list(range(0 if i % 2 else 50, (0 if i % 2 else 50) + n))
+        at += n
+    t = lambda x: torch.tensor(x, dtype=torch.int32, device=dev)
+    out = F.gdn_scan(qkv, ab, a_log, dt, t(segs), len(lens), t(slot), t(pos), hk, hv, d, state)
+    q64 = qkv[:, :hk * d].double().reshape(rows, hk, d).repeat_interleave(2, 1) / math.sqrt(d)
+    k64 = qkv[:, hk * d:2 * hk * d].double().reshape(rows, hk, d).repeat_interleave(2, 1)
+    v64 = qkv[:, 2 * hk * d:].double().reshape(rows, hv, d)
+    g = -torch.exp(a_log.double()) * torch.nn.functional.softplus(ab[:, :hv].double() + dt.double(),
+                                                                  threshold=60)
+    beta = torch.sigmoid(ab[:, hv:].double())
+    for i, n in enumerate(lens):
+        sl = slice(segs[i][0], segs[i][0] + n)
+        s0 = start[i + 1] * (0.0 if i % 2 else 1.0)
+        ref, s = _recurrence64(q64[sl], k64[sl], v64[sl], g[sl], beta[sl], s0)
+        # FP32 sums and 22-bit splits over at most 333 steps; the decays carry the FP32 rounding
+        # of g itself (2^-24 of up to 400 per step, summed over the steps a value lives)
+        tol = 1e-5 if strength < 1 else 1e-4
+        assert float((out[sl].double() - ref).norm() / ref.norm()) < tol, n
+        assert float((state[i + 1].double() - s).norm() / s.norm().clamp(min=1e-9)) < tol, n
+    assert torch.equal(state[0].double(), start[0]) and torch.equal(state[-1].double(), start[-1])
+
+
+@pytest.mark.parametrize("d,hk,hv", [(64, 1, 2), (128, 1, 2), (128, 2, 5), (64, 3, 5)])
+@pytest.mark.parametrize("rows,segments", [(5, 5), (37, 3), (4801, 3)])
+def test_gdn_conv_forms_agree(dev, d, hk, hv, rows, segments):
+    """Eight-channel strips, single rows and the general form give the same rows and history
+    as the 64-bit convolution; strips cross run boundaries inside the packet."""
+    from orinfer_b200.ops import functional as F
+    torch.manual_seed(rows + d)
+    conv = (2 * hk + hv) * d
+    x = torch.randn(rows, conv + 2 * d, device=dev).half()
+    w = (torch.randn(conv, 4, device=dev) * 0.4).half()
+    hist = torch.randn(segments, 3, conv, device=dev).half()
+    base = rows // segments
+    lens = [rows - base * (segments - 1)] + [base] * (segments - 1)
+    segs, first, slot, pos, at = [], [], [], [], 0
+    for i, n in enumerate(lens):
+        p0 = 0 if i == 1 else 9
+        segs.append([at, n, 0, 0])
+        first += [at] * n
+        slot += [i] * n
+        pos += list(range(p0, p0 + n))
+        at += n
+    t = lambda v: torch.tensor(v, dtype=torch.int32, device=dev)
+    args = (t(first), t(slot), t(pos), t(segs), segments, rows, hk, hv, d)
+    h_vec, h_gen = hist.clone(), _unaligned(hist)
+    y = F.gdn_conv(x, w, h_vec, *args)
+    y_gen = F.gdn_conv(_unaligned(x), w, h_gen, *args)
+    assert torch.equal(h_vec, h_gen)
+    at = 0
+    for i, n in enumerate(lens):
+        prev = hist[i].double() * (0.0 if i == 1 else 1.0)
+        full = torch.cat([prev, x[at:at + n, :conv].double()])
+        ref = sum(full[j:j + n] * w[:, j].double() for j in range(4))
+        ref = (ref * torch.sigmoid(ref)).half().double()
+        qk = ref[:, :2 * hk * d].reshape(n, -1, d)
+        ref[:, :2 * hk * d] = (qk * torch.rsqrt((qk * qk).sum(-1, keepdim=True) + 1e-6)).reshape(n, -1)
+        # two FP16 roundings; the first may fall the other way (one more step)
+        for got in (y[at:at + n], y_gen[at:at + n]):
+            assert bool(((got.double() - ref).abs() <= ref.abs() * 2.0 ** -9 + 1e-6).all())
+        assert torch.equal(h_vec[i].double(), full[-3:])
+        at += n
+
+
+@pytest.mark.parametrize("d", [64, 128])
+@pytest.mark.parametrize("rows,hv", [(1, 1), (3, 5), (130, 4)])
+def test_gdn_gated_norm_forms_agree(dev, d, rows, hv):
+    from orinfer_b200.ops import functional as F
+    torch.manual_seed(rows)
+    o = torch.randn(rows, hv, d, device=dev)
+    proj = torch.randn(rows, 8 + hv * d, device=dev).half()
+    w = (1 + 0.1 * torch.randn(d, device=dev)).half()
+    for z in (proj[:, 8:], proj[:, 3:3 + hv * d]):
+        for sig in (False, True):
+            y = F.gdn_gated_norm(o, z, w, 1e-6, rows, hv, d, sigmoid_gate=sig)
+            oo, zz = o.double(), z.double().reshape(rows, hv, d)
+            gate = torch.sigmoid(zz) * (1.0 if sig else zz)
+            ref = oo * torch.rsqrt((oo * oo).mean(-1, keepdim=True) + 1e-6) * w.double() * gate
+            lim = ref.reshape(rows, -1).abs() * 2.0 ** -10 + 1e-7
+            assert bool(((y.double() - ref.reshape(rows, -1)).abs() <= lim).all())
