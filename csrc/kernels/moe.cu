@@ -4,17 +4,66 @@
 // Replaces router_projection / router_topk (kernels/cuda/model/moe.py:16,413),
 // expert_histogram* / expert_offsets / expert_tiles (moe.py:177-286,558-713),
 // expert_dispatch (moe.py:286) and moe_combine (moe.py:498-557) of the reference.
+#include <cooperative_groups.h>
+
 #include "api.h"
 #include "common.cuh"
 #include "tp_comm.cuh"
 
+namespace cg = cooperative_groups;
+
 namespace orinfer {
 
 // ---------------------------------------------------------------- router + top-k
-// One CTA per token row.  logits[e] = x[row] . W[e] (fp16 inputs, fp32 accumulate);
-// softmax over the first `experts` rows of W; top-k by repeated argmax with ties going to
-// the lower expert id; optional renormalisation; row `experts` of W (when present) is the
-// shared-expert gate, returned as sigmoid(logit).
+// logits[e] = x[row] . W[e] (fp16 inputs, fp32 accumulate); softmax over the first `experts`
+// rows of W; top-k by repeated argmax with ties going to the lower expert id; optional
+// renormalisation; row `experts` of W (when present) is the shared-expert gate, returned as
+// sigmoid(logit).
+
+// Softmax statistics and top-k of one row by one warp; `logits` [experts (+ 1)] in shared
+// memory, overwritten.
+__device__ __forceinline__ void topk_row(float* logits, int row, int experts, int has_shared,
+                                         int top_k, int renorm, int* __restrict__ ids,
+                                         float* __restrict__ probs,
+                                         float* __restrict__ shared_gate) {
+  const int lane = threadIdx.x & 31;
+  float mx = -INFINITY;
+  for (int e = lane; e < experts; e += 32) mx = fmaxf(mx, logits[e]);
+  mx = warp_max(mx);
+  float sum = 0.f;
+  for (int e = lane; e < experts; e += 32) sum += expf(logits[e] - mx);
+  sum = warp_sum(sum);
+  float chosen_sum = 0.f;
+  for (int k = 0; k < top_k; ++k) {
+    float best = -INFINITY;
+    int bidx = 0x7fffffff;
+    for (int e = lane; e < experts; e += 32) {
+      const float v = logits[e];
+      if (v > best) { best = v; bidx = e; }           // ascending e: first maximum wins
+    }
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) {
+      const float ov = __shfl_xor_sync(0xffffffffu, best, o);
+      const int oi = __shfl_xor_sync(0xffffffffu, bidx, o);
+      if (ov > best || (ov == best && oi < bidx)) { best = ov; bidx = oi; }
+    }
+    if (bidx >= experts) bidx = k;                  // no comparable logit left (NaN): any valid id
+    const float p = expf(best - mx) / sum;
+    if (lane == 0) {
+      ids[row * top_k + k] = bidx;
+      probs[row * top_k + k] = p;
+      logits[bidx] = -INFINITY;
+    }
+    chosen_sum += p;
+    __syncwarp();
+  }
+  if (renorm && lane == 0)
+    for (int k = 0; k < top_k; ++k) probs[row * top_k + k] /= chosen_sum;
+  if (has_shared && lane == 0)
+    shared_gate[row] = 1.f / (1.f + expf(-logits[experts]));
+}
+
+// General form: one CTA per token row, one warp per expert at a time.
 __global__ void __launch_bounds__(256) router_topk_kernel(
     const __half* __restrict__ x, const __half* __restrict__ w, int hidden, int experts,
     int has_shared, int top_k, int renorm, int* __restrict__ ids, float* __restrict__ probs,
@@ -43,122 +92,177 @@ __global__ void __launch_bounds__(256) router_topk_kernel(
   }
   __syncthreads();
   if (warp != 0) return;
-  // softmax statistics over the routed experts
-  float mx = -INFINITY;
-  for (int e = lane; e < experts; e += 32) mx = fmaxf(mx, logits[e]);
-  mx = warp_max(mx);
-  float sum = 0.f;
-  for (int e = lane; e < experts; e += 32) sum += expf(logits[e] - mx);
-  sum = warp_sum(sum);
-  float chosen_sum = 0.f;
-  for (int k = 0; k < top_k; ++k) {
-    float best = -INFINITY;
-    int bidx = 0x7fffffff;
-    for (int e = lane; e < experts; e += 32) {
-      const float v = logits[e];
-      if (v > best) { best = v; bidx = e; }           // ascending e: first maximum wins
-    }
+  topk_row(logits, row, experts, has_shared, top_k, renorm, ids, probs, shared_gate);
+}
+
+// Tensor-core form (hidden % 256 == 0, at most 8 * 8 * MAXT expert rows).  The general form
+// streams the whole router matrix (0.5 to 2 MB) through every CTA, once per token row.  Here a
+// cluster of eight CTAs takes 16 rows: CTA c owns an eighth of the 8-expert tiles, its eight
+// warps an eighth of the hidden channels each (FP16 products, FP32 sums on the tensor cores;
+// the eight partial sums are added in a fixed order), and the logits of rows 2c and 2c + 1 are
+// collected in CTA c over distributed shared memory for the top-k.  Lane (g, t) loads 16 bytes
+// of row g: the halves 4s..4s+3 are its fragments of step s, in x and W alike.
+constexpr int ROUTER_CL = 8, ROUTER_ROWS = 16;
+
+template <int MAXT>
+__global__ void __cluster_dims__(ROUTER_CL, 1, 1) __launch_bounds__(256) router_mma_kernel(
+    const __half* __restrict__ x, const __half* __restrict__ w, int rows, int hidden, int experts,
+    int has_shared, int top_k, int renorm, int* __restrict__ ids, float* __restrict__ probs,
+    float* __restrict__ shared_gate) {
+  extern __shared__ float logits[];                 // [2][total]
+  __shared__ float part[8][ROUTER_ROWS][MAXT * 8 + 1];
+  cg::cluster_group cluster = cg::this_cluster();
+  const int crank = static_cast<int>(cluster.block_rank());
+  const int row0 = static_cast<int>(blockIdx.x) / ROUTER_CL * ROUTER_ROWS;
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, g = lane >> 2, t = lane & 3;
+  const int total = experts + (has_shared ? 1 : 0), tiles = (total + 7) / 8;
+  const int t_lo = tiles * crank / ROUTER_CL, nt = tiles * (crank + 1) / ROUTER_CL - t_lo;
+  float acc[MAXT][4];
 #pragma unroll
-    for (int o = 16; o > 0; o >>= 1) {
-      const float ov = __shfl_xor_sync(0xffffffffu, best, o);
-      const int oi = __shfl_xor_sync(0xffffffffu, bidx, o);
-      if (ov > best || (ov == best && oi < bidx)) { best = ov; bidx = oi; }
-    }
-    const float p = expf(best - mx) / sum;
-    if (lane == 0) {
-      ids[row * top_k + k] = bidx;
-      probs[row * top_k + k] = p;
-      logits[bidx] = -INFINITY;
-    }
-    chosen_sum += p;
-    __syncwarp();
-  }
-  if (renorm && lane == 0)
-    for (int k = 0; k < top_k; ++k) probs[row * top_k + k] /= chosen_sum;
-  if (has_shared && lane == 0)
-    shared_gate[row] = 1.f / (1.f + expf(-logits[experts]));
-}
-
-// ---------------------------------------------------------------- counts (one CTA per expert)
-// Under expert parallelism a rank owns experts [base, base + gridDim.x): ids outside that
-// range are left to their owners (their slot stays -1 and the combine skips them).
-__global__ void __launch_bounds__(256) moe_count_kernel(const int* __restrict__ ids, int assigns,
-                                                        int base_expert,
-                                                        int* __restrict__ counts) {
-  const int e = blockIdx.x;
-  int c = 0;
-  for (int i = threadIdx.x; i < assigns; i += blockDim.x) c += ids[i] == e + base_expert;
-  __shared__ int red[8];
-  c = static_cast<int>(warp_sum(static_cast<float>(c)));       // counts < 2^24: exact
-  if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = c;
-  __syncthreads();
-  if (threadIdx.x == 0) {
-    int t = 0;
-    for (int i = 0; i < 8; ++i) t += red[i];
-    counts[e] = t;
-  }
-}
-
-// offsets[e] = exclusive prefix of counts; tile table (expert, first slot, valid rows) for
-// 128-row tiles; meta[0] = number of tiles.  One thread: E <= 512.
-__global__ void moe_offsets_kernel(const int* __restrict__ counts, int experts,
-                                   int* __restrict__ offsets, int* __restrict__ tiles,
-                                   int* __restrict__ meta, int max_tiles) {
-  if (threadIdx.x != 0 || blockIdx.x != 0) return;
-  int off = 0, nt = 0;
-  for (int e = 0; e < experts; ++e) {
-    offsets[e] = off;
-    const int c = counts[e];
-    for (int r = 0; r < c && nt < max_tiles; r += 128) {
-      tiles[nt * 4 + 0] = e;
-      tiles[nt * 4 + 1] = off + r;
-      tiles[nt * 4 + 2] = min(128, c - r);
-      tiles[nt * 4 + 3] = 0;
-      ++nt;
-    }
-    off += c;
-  }
-  offsets[experts] = off;
-  meta[0] = nt;
-}
-
-// slot[i] = offsets[e] + rank of assignment i among the assignments of expert e (stable in
-// (row, k) order); also copies the quantised row and its scale into that slot.
-__global__ void __launch_bounds__(256) moe_dispatch_kernel(
-    const int* __restrict__ ids, int assigns, int top_k, int base_expert,
-    const int* __restrict__ offsets, const int8_t* __restrict__ q8,
-    const float* __restrict__ scale, int K, int* __restrict__ slots,
-    int8_t* __restrict__ q8_sorted, float* __restrict__ scale_sorted) {
-  const int e = blockIdx.x;
-  __shared__ int wsum[8];
-  __shared__ int base;
-  if (threadIdx.x == 0) base = offsets[e];
-  __syncthreads();
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  for (int start = 0; start < assigns; start += 256) {
-    const int i = start + threadIdx.x;
-    const bool mine = i < assigns && ids[i] == e + base_expert;
-    const unsigned ballot = __ballot_sync(0xffffffffu, mine);
-    if (lane == 0) wsum[warp] = __popc(ballot);
-    __syncthreads();
-    int before = 0;
-    for (int w = 0; w < warp; ++w) before += wsum[w];
-    int block_total = 0;
-    for (int w = 0; w < 8; ++w) block_total += wsum[w];
-    if (mine) {
-      const int slot = base + before + __popc(ballot & ((1u << lane) - 1u));
-      slots[i] = slot;
-      if (q8 != nullptr) {                  // nullptr: only the slot numbering is wanted
-        const int row = i / top_k;
-        scale_sorted[slot] = scale[row];
-        const int4* src = reinterpret_cast<const int4*>(q8 + static_cast<size_t>(row) * K);
-        int4* dst = reinterpret_cast<int4*>(q8_sorted + static_cast<size_t>(slot) * K);
-        for (int c = 0; c < K / 16; ++c) dst[c] = src[c];
+  for (int i = 0; i < MAXT; ++i)
+#pragma unroll
+    for (int j = 0; j < 4; ++j) acc[i][j] = 0.f;
+  // rows past the last token or expert read the last one; their sums are not used
+  const __half* xa = x + static_cast<size_t>(min(row0 + g, rows - 1)) * hidden + t * 8;
+  const __half* xb = x + static_cast<size_t>(min(row0 + g + 8, rows - 1)) * hidden + t * 8;
+  const int k_lo = hidden / 8 * warp, k_hi = hidden / 8 * (warp + 1);
+#pragma unroll 2
+  for (int k = k_lo; k < k_hi; k += 32) {
+    const uint4 a = __ldg(reinterpret_cast<const uint4*>(xa + k));
+    const uint4 b = __ldg(reinterpret_cast<const uint4*>(xb + k));
+    uint4 wv[MAXT];
+#pragma unroll
+    for (int i = 0; i < MAXT; ++i)
+      if (i < nt) {
+        const int e = min((t_lo + i) * 8 + g, total - 1);
+        wv[i] = __ldg(reinterpret_cast<const uint4*>(w + static_cast<size_t>(e) * hidden + t * 8 + k));
       }
+#pragma unroll
+    for (int i = 0; i < MAXT; ++i)
+      if (i < nt) {
+        mma16816(acc[i], a.x, b.x, a.y, b.y, wv[i].x, wv[i].y);
+        mma16816(acc[i], a.z, b.z, a.w, b.w, wv[i].z, wv[i].w);
+      }
+  }
+#pragma unroll
+  for (int i = 0; i < MAXT; ++i)
+    if (i < nt) {
+      part[warp][g][i * 8 + 2 * t] = acc[i][0];
+      part[warp][g][i * 8 + 2 * t + 1] = acc[i][1];
+      part[warp][g + 8][i * 8 + 2 * t] = acc[i][2];
+      part[warp][g + 8][i * 8 + 2 * t + 1] = acc[i][3];
     }
-    __syncthreads();
-    if (threadIdx.x == 0) base += block_total;
-    __syncthreads();
+  cluster.sync();                                   // every CTA of the cluster runs
+  for (int i = threadIdx.x; i < ROUTER_ROWS * nt * 8; i += blockDim.x) {
+    const int r = i / (nt * 8), c = i % (nt * 8), e = t_lo * 8 + c;
+    float v = 0.f;
+#pragma unroll
+    for (int q = 0; q < 8; ++q) v += part[q][r][c];
+    if (e < total) cluster.map_shared_rank(logits, r >> 1)[(r & 1) * total + e] = v;
+  }
+  cluster.sync();
+  const int row = row0 + crank * 2 + warp;
+  if (warp < 2 && row < rows)
+    topk_row(logits + warp * total, row, experts, has_shared, top_k, renorm, ids, probs,
+             shared_gate);
+}
+
+// ---------------------------------------------------------------- slots
+// One CTA per local expert, one launch for everything the grouped GEMM needs to know: each CTA
+// counts the assignments of all experts in shared memory (integers: the order does not
+// matter), sums the counts and 128-row tiles before its own expert, writes its offset, count
+// and tile-table entries, and numbers its own assignments in (row, k) order: slot[i] =
+// offset[e] + rank of i among the assignments of e.  Under expert parallelism a rank owns
+// experts [base_expert, base_expert + gridDim.x): ids outside that range get slot -1 (CTA 0
+// writes those) and the combine skips them.
+__global__ void __launch_bounds__(256) moe_plan_kernel(
+    const int* __restrict__ ids, int assigns, int base_expert, int* __restrict__ counts,
+    int* __restrict__ offsets, int* __restrict__ tiles, int* __restrict__ meta, int max_tiles,
+    int* __restrict__ slots) {
+  extern __shared__ int hist[];                     // [experts]
+  __shared__ int red[2][8], warp_count[8];
+  const int e = blockIdx.x, experts = gridDim.x, tid = threadIdx.x;
+  const int warp = tid >> 5, lane = tid & 31;
+  for (int i = tid; i < experts; i += 256) hist[i] = 0;
+  __syncthreads();
+  // a warp walks one contiguous run of assignments, 32 at a time
+  const int steps = (assigns + 255) / 256, lo = warp * steps * 32;
+  int mine = 0;
+#pragma unroll 4
+  for (int s = 0; s < steps; ++s) {
+    const int i = lo + s * 32 + lane;
+    const int id = i < assigns ? ids[i] - base_expert : -1;
+    if (id >= 0 && id < experts) atomicAdd(&hist[id], 1);
+    mine += id == e;
+    if (e == 0 && i < assigns && (id < 0 || id >= experts)) slots[i] = -1;
+  }
+  mine = __reduce_add_sync(0xffffffffu, mine);
+  if (lane == 0) warp_count[warp] = mine;
+  __syncthreads();
+  int rows_before = 0, tiles_before = 0;
+  for (int i = tid; i < e; i += 256) {
+    rows_before += hist[i];
+    tiles_before += (hist[i] + 127) / 128;
+  }
+  rows_before = __reduce_add_sync(0xffffffffu, rows_before);
+  tiles_before = __reduce_add_sync(0xffffffffu, tiles_before);
+  if (lane == 0) {
+    red[0][warp] = rows_before;
+    red[1][warp] = tiles_before;
+  }
+  __syncthreads();
+  int off = 0, tile0 = 0, slot = 0;
+#pragma unroll
+  for (int q = 0; q < 8; ++q) {
+    off += red[0][q];
+    tile0 += red[1][q];
+    if (q < warp) slot += warp_count[q];
+  }
+  const int count = hist[e], own_tiles = (count + 127) / 128;
+  for (int j = tid; j < own_tiles; j += 256)
+    if (tile0 + j < max_tiles) {
+      int* entry = tiles + static_cast<size_t>(tile0 + j) * 4;
+      entry[0] = e;
+      entry[1] = off + j * 128;
+      entry[2] = min(128, count - j * 128);
+      entry[3] = 0;
+    }
+  if (tid == 0) {
+    counts[e] = count;
+    offsets[e] = off;
+    if (e == experts - 1) {
+      offsets[experts] = off + count;
+      meta[0] = min(tile0 + own_tiles, max_tiles);
+    }
+  }
+  if (warp_count[warp] == 0) return;
+  slot += off;
+  for (int s = 0; s < steps; ++s) {
+    const int i = lo + s * 32 + lane;
+    const bool hit = i < assigns && ids[i] - base_expert == e;
+    const unsigned ballot = __ballot_sync(0xffffffffu, hit);
+    if (hit) slots[i] = slot + __popc(ballot & ((1u << lane) - 1u));
+    slot += __popc(ballot);
+  }
+}
+
+// Copies row blockIdx.x (INT8 values and scale) into the slots of its assignments: the row is
+// read once and written top_k times in whole lines.
+__global__ void __launch_bounds__(128) moe_scatter_kernel(
+    const int* __restrict__ slots, int top_k, const int8_t* __restrict__ q8,
+    const float* __restrict__ scale, int K, int8_t* __restrict__ q8_sorted,
+    float* __restrict__ scale_sorted) {
+  const int row = blockIdx.x;
+  const int* sl = slots + static_cast<size_t>(row) * top_k;
+  const float s = scale[row];
+  for (int j = threadIdx.x; j < top_k; j += blockDim.x)
+    if (sl[j] >= 0) scale_sorted[sl[j]] = s;
+  for (int c = threadIdx.x; c < K / 16; c += blockDim.x) {
+    const int4 v = reinterpret_cast<const int4*>(q8 + static_cast<size_t>(row) * K)[c];
+    for (int j = 0; j < top_k; ++j) {
+      const int slot = __ldg(sl + j);
+      if (slot >= 0) reinterpret_cast<int4*>(q8_sorted + static_cast<size_t>(slot) * K)[c] = v;
+    }
   }
 }
 
@@ -206,6 +310,24 @@ __global__ void __launch_bounds__(256) moe_combine_kernel(
   if (peers.tp != 0) peer_signal_done(peers, gridDim.x);
 }
 
+static int launch_dispatch(const int* ids, int rows, int top_k, int base_expert, int experts,
+                           const int8_t* q8, const float* scale, int K, int* counts, int* offsets,
+                           int* tiles, int* meta, int max_tiles, int* slots, int8_t* q8_sorted,
+                           float* scale_sorted, cudaStream_t stream) {
+  const size_t smem = static_cast<size_t>(experts) * sizeof(int);
+  if (smem > 48 * 1024) {                           // more than 12 288 experts on one rank
+    const cudaError_t e = cudaFuncSetAttribute(
+        moe_plan_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem));
+    if (e != cudaSuccess) return static_cast<int>(e);
+  }
+  moe_plan_kernel<<<experts, 256, smem, stream>>>(ids, rows * top_k, base_expert, counts, offsets,
+                                                  tiles, meta, max_tiles, slots);
+  if (q8 != nullptr)                                // nullptr: only the slot numbering is wanted
+    moe_scatter_kernel<<<rows, 128, 0, stream>>>(slots, top_k, q8, scale, K, q8_sorted,
+                                                 scale_sorted);
+  return static_cast<int>(cudaGetLastError());
+}
+
 }  // namespace orinfer
 
 using namespace orinfer;
@@ -217,6 +339,15 @@ int orinfer_router_topk(const __half* x, const __half* w, int rows, int hidden, 
                         float* shared_gate, cudaStream_t stream) {
   if (rows <= 0) return 0;
   if (hidden % 8 || top_k < 1 || top_k > experts || experts > 4096) return -1;
+  const int total = experts + (has_shared ? 1 : 0);
+  if (hidden % 256 == 0 && total <= ROUTER_CL * 8 * 9) {
+    const int grid = (rows + ROUTER_ROWS - 1) / ROUTER_ROWS * ROUTER_CL;
+    const size_t smem = 2 * static_cast<size_t>(total) * sizeof(float);
+    auto kernel = total <= ROUTER_CL * 8 * 3 ? router_mma_kernel<3> : router_mma_kernel<9>;
+    kernel<<<grid, 256, smem, stream>>>(x, w, rows, hidden, experts, has_shared, top_k, renorm, ids,
+                                        probs, shared_gate);
+    return static_cast<int>(cudaGetLastError());
+  }
   router_topk_kernel<<<rows, 256, (experts + 1) * sizeof(float), stream>>>(
       x, w, hidden, experts, has_shared, top_k, renorm, ids, probs, shared_gate);
   return static_cast<int>(cudaGetLastError());
@@ -230,12 +361,8 @@ int orinfer_moe_dispatch(const int* ids, int rows, int top_k, int experts, const
                          float* scale_sorted, cudaStream_t stream) {
   if (rows <= 0) return 0;
   if (K % 16) return -1;
-  const int assigns = rows * top_k;
-  moe_count_kernel<<<experts, 256, 0, stream>>>(ids, assigns, 0, counts);
-  moe_offsets_kernel<<<1, 32, 0, stream>>>(counts, experts, offsets, tiles, meta, max_tiles);
-  moe_dispatch_kernel<<<experts, 256, 0, stream>>>(ids, assigns, top_k, 0, offsets, q8, scale, K,
-                                                   slots, q8_sorted, scale_sorted);
-  return static_cast<int>(cudaGetLastError());
+  return launch_dispatch(ids, rows, top_k, 0, experts, q8, scale, K, counts, offsets, tiles, meta,
+                         max_tiles, slots, q8_sorted, scale_sorted, stream);
 }
 
 // Expert-parallel dispatch: this rank owns experts [base_expert, base_expert + local_experts);
@@ -247,15 +374,8 @@ int orinfer_moe_dispatch_ep(const int* ids, int rows, int top_k, int base_expert
                             cudaStream_t stream) {
   if (rows <= 0) return 0;
   if (K % 16) return -1;
-  const int assigns = rows * top_k;
-  cudaMemsetAsync(slots, 0xFF, sizeof(int) * assigns, stream);
-  moe_count_kernel<<<local_experts, 256, 0, stream>>>(ids, assigns, base_expert, counts);
-  moe_offsets_kernel<<<1, 32, 0, stream>>>(counts, local_experts, offsets, tiles, meta,
-                                           max_tiles);
-  moe_dispatch_kernel<<<local_experts, 256, 0, stream>>>(ids, assigns, top_k, base_expert,
-                                                         offsets, q8, scale, K, slots, q8_sorted,
-                                                         scale_sorted);
-  return static_cast<int>(cudaGetLastError());
+  return launch_dispatch(ids, rows, top_k, base_expert, local_experts, q8, scale, K, counts,
+                         offsets, tiles, meta, max_tiles, slots, q8_sorted, scale_sorted, stream);
 }
 
 // Combine whose result rows are pushed into every rank's inbox (slot [rank]) over NVLink and

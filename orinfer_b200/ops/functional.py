@@ -300,13 +300,13 @@ def moe_dispatch(ids: torch.Tensor, q8: Optional[torch.Tensor], scale: Optional[
             ptr(ids), rows, top_k, base_expert, local_experts, ptr(q8), ptr(scale), width,
             ptr(sc.counts), ptr(sc.offsets), ptr(sc.tiles), ptr(sc.meta), sc.max_tiles,
             ptr(sc.slots), ptr(sc.q8), ptr(sc.scale), stream()), "moe_dispatch_ep")
-        count_launches(3)
+        count_launches(1 if q8 is None else 2)
         return
     check(native.lib().orinfer_moe_dispatch(
         ptr(ids), rows, top_k, experts, ptr(q8), ptr(scale), width, ptr(sc.counts),
         ptr(sc.offsets), ptr(sc.tiles), ptr(sc.meta), sc.max_tiles, ptr(sc.slots), ptr(sc.q8),
         ptr(sc.scale), stream()), "moe_dispatch")
-    count_launches(3)
+    count_launches(1 if q8 is None else 2)
 
 
 def qgemm_grouped(a: torch.Tensor, a_scale: torch.Tensor, codes: torch.Tensor,

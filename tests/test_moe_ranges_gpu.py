@@ -1,0 +1,79 @@
+"""Routing, dispatch and expert projections at the edges of their ranges."""
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.fixture(scope="module")
+def dev(cuda):
+    from orinfer_b200.ops import native
+    native.init()
+    return cuda
+
+
+@pytest.mark.parametrize("rows", [1, 15, 16, 17, 50])
+@pytest.mark.parametrize("hidden,experts,top_k,shared", [
+    (256, 3, 2, False), (256, 64, 4, True), (512, 128, 8, False), (2048, 191, 8, True),
+    (256, 192, 8, True), (2048, 512, 10, True), (256, 576, 6, False), (256, 576, 6, True),
+    (264, 128, 8, False)])
+def test_router_topk_forms(dev, rows, hidden, experts, top_k, shared):
+    """Tensor-core and general router at the edges of their expert and row tiles."""
+    from orinfer_b200.ops import functional as F
+    g = torch.Generator().manual_seed(experts + rows)
+    y = torch.randn(rows, hidden, generator=g).half().to(dev)
+    w = (torch.randn(experts + int(shared), hidden, generator=g) * 0.1).half().to(dev)
+    w[experts - 1] = w[0]                                  # an exact tie: the lower id first
+    ids, probs, gate = F.router_topk(y, w, experts, top_k)
+    logits = y.double() @ w.double().t()
+    p, order = torch.softmax(logits[:, :experts], 1).sort(dim=1, descending=True, stable=True)
+    p, order = p[:, :top_k], order[:, :top_k]
+    p = p / p.sum(1, keepdim=True)
+    # FP32 sums of up to 2048 products: the logits are within 1e-5 of exact, the weights with them
+    assert bool(((probs.double() - p).abs() <= 4e-5 * p + 1e-7).all())
+    picked = torch.gather(logits, 1, ids.long())
+    assert bool(((picked - torch.gather(logits, 1, order)).abs() <= 2e-5).all())
+    for r in range(rows):
+        chosen = ids[r].tolist()
+        assert len(set(chosen)) == top_k
+        if experts - 1 in chosen:
+            assert 0 in chosen and chosen.index(0) < chosen.index(experts - 1)
+    if shared:
+        assert torch.allclose(gate.double(), torch.sigmoid(logits[:, experts]), atol=1e-5)
+
+
+@pytest.mark.parametrize("experts,rows,top_k,k", [(1, 1, 1, 128), (8, 5, 2, 256), (3, 300, 1, 128),
+                                                  (128, 2048, 8, 2048), (512, 16, 10, 2048),
+                                                  (512, 700, 10, 512)])
+@pytest.mark.parametrize("part", [False, True])
+def test_moe_dispatch_numbers_and_copies(dev, experts, rows, top_k, k, part):
+    from orinfer_b200.ops import functional as F
+    g = torch.Generator().manual_seed(rows)
+    ids = torch.stack([torch.randperm(experts, generator=g)[:top_k] for _ in range(rows)])
+    ids = (ids // 2 if experts == 8 else ids).to(torch.int32)      # some experts get no row
+    q8 = torch.randint(-127, 128, (rows, k), generator=g, dtype=torch.int8).to(dev)
+    scale = torch.rand(rows, generator=g).to(dev)
+    base, local = (experts // 3, max(experts // 2, 1)) if part else (0, experts)
+    if base + local > experts:
+        local = experts - base
+    sc = F.MoeScratch(rows, top_k, experts, k, 64, dev)
+    sc.tiles.fill_(-7)
+    F.moe_dispatch(ids.to(dev), q8, scale, experts, sc, rows, base, local)
+    flat = ids.flatten().long() - base
+    flat = torch.where((flat >= 0) & (flat < local), flat, local)
+    order = torch.sort(flat, stable=True).indices
+    want = torch.full((rows * top_k,), -1, dtype=torch.int64)
+    kept = int((flat < local).sum())
+    want[order[:kept]] = torch.arange(kept)
+    counts = torch.bincount(flat, minlength=local + 1)[:local]
+    assert torch.equal(sc.slots.cpu().long(), want)
+    assert torch.equal(sc.counts[:local].cpu().long(), counts)
+    offs = torch.cat([torch.zeros(1, dtype=torch.int64), counts.cumsum(0)])
+    assert torch.equal(sc.offsets[:local + 1].cpu().long(), offs)
+    tiles = [[e, int(offs[e]) + r, min(128, int(counts[e]) - r), 0]
+             for e in range(local) for r in range(0, int(counts[e]), 128)]
+    assert int(sc.meta[0]) == len(tiles)
+    assert sc.tiles[:len(tiles)].cpu().tolist() == tiles
+    src = order[:kept] // top_k
+    assert torch.equal(sc.q8[:kept].cpu(), q8.cpu()[src])
+    assert torch.equal(sc.scale[:kept].cpu(), scale.cpu()[src])
