@@ -51,6 +51,13 @@ struct RowScales {
     const __half2 v = *reinterpret_cast<const __half2*>(&w[c / 2]);
     return c & 1 ? __high2float(v) : __low2float(v);
   }
+  // the scales that `lane` holds
+  __device__ __forceinline__ RowScales from(int lane) const {
+    RowScales r;
+#pragma unroll
+    for (int i = 0; i < (G + 1) / 2; ++i) r.w[i] = __shfl_sync(0xffffffffu, w[i], lane);
+    return r;
+  }
   __device__ __forceinline__ void clear() {
 #pragma unroll
     for (int i = 0; i < (G + 1) / 2; ++i) w[i] = 0u;
@@ -61,19 +68,42 @@ struct RowScales {
 // lies inside one page) and carry their own softmax state, merged in shared memory at the end.
 //
 // Both products run on the tensor cores with the INT8 values as exact FP16 integers.
-//   S = Q K^T: rows 0..7 of A are the query heads; lane (g, t) loads 16 bytes of key g, which
+//   S = Q K^T: rows 0..7 of A are the query heads; lane (g, t) reads 16 bytes of key g, which
 //   are its B fragments of four steps (the channel order inside a product does not matter, Q
 //   is laid out to match).  Each group of 64 channels is summed by itself and scaled in FP32.
 //   O = P V: the FP32 weight x value scale is split into an FP16 head and an FP16 remainder
 //   in rows g and g + 8 of the same A tile, so the split costs no instruction and keeps 22
 //   bits.  The weights are scaled by a power of two (2^14 over the largest value scale seen,
 //   exact) so that the remainder stays above the smallest FP16 step.
+//
+// The first form converted every byte to FP32 and multiplied it once per query head on the CUDA
+// cores, with the weights going through shared memory: it was bound by those instructions.  32
+// query / 8 KV heads of 128: 128 rows of 320..640 keys 209 -> 53 us with the products on the
+// tensor cores and loads through registers, 41 us with the loads in cp.async rings (132 MB: 3.2
+// TB/s); 6 rows of 12000..24000 keys 432 -> 78 -> 62 us (235 MB: 3.8 TB/s).  The loads in flight
+// bound it: three CTAs of 128 threads hold 96 KB of them per SM.
 template <int D>
 struct AttnTile {
   static constexpr int G = D / 64;                 // scale groups per row
   static constexpr int KB = D == 256 ? 16 : 32;    // keys per block
   static constexpr int MIN_CTAS = D == 256 ? 2 : 3;
+  static constexpr int CPK = D / 16;               // 16-byte units of a key row
+  static constexpr int STAGE = 2 * KB * D;         // K and V rows of one block
+  static constexpr int RING = ATTN_WARPS * 2 * STAGE;          // two stages per warp
+  static constexpr int SMEM = RING > ATTN_WARPS * 8 * D * 4 ? RING : ATTN_WARPS * 8 * D * 4;
+  // where 16-byte unit `u` of row `key` of a block lies: the lanes that read together (8 keys
+  // x 4 neighbouring units for K; 4 keys x 32 bytes for V) meet on no bank
+  __device__ static int k_unit(int key, int u) {
+    return key * CPK + (CPK >= 8 ? u ^ ((key & 1) << 2) : u);
+  }
+  __device__ static int v_unit(int key, int u) {
+    return key * CPK + (u ^ (CPK >= 8 ? ((key >> 1) & 3) << 1 : ((key >> 1) & 1) << 1));
+  }
 };
+
+__device__ __forceinline__ void cp_async16(uint32_t smem, const void* gmem) {
+  asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(smem), "l"(gmem) : "memory");
+}
 
 template <int D, bool WIDE>
 __global__ void __launch_bounds__(ATTN_WARPS * 32, AttnTile<D>::MIN_CTAS) attn_rows_kernel(
@@ -93,7 +123,9 @@ __global__ void __launch_bounds__(ATTN_WARPS * 32, AttnTile<D>::MIN_CTAS) attn_r
   const int* pages = page_table + static_cast<size_t>(row_req[row]) * max_pages;
   const float qscale = rsqrtf(static_cast<float>(D)) * 1.4426950408889634f;
 
-  __shared__ __align__(16) float s_o[ATTN_WARPS][8][D];
+  using T = AttnTile<D>;
+  extern __shared__ __align__(16) unsigned char attn_smem[];   // rings, then the warps' results
+  float(*s_o)[8][D] = reinterpret_cast<float(*)[8][D]>(attn_smem);
   __shared__ float s_m[ATTN_WARPS][8], s_l[ATTN_WARPS][8];
 
   // Query fragments in shared memory, one copy for the four warps (16 or 32 registers per lane
@@ -131,44 +163,52 @@ __global__ void __launch_bounds__(ATTN_WARPS * 32, AttnTile<D>::MIN_CTAS) attn_r
 
   const int b_hi = k_hi > k_lo ? (k_hi + KB - 1) / KB : 0;
   int b = k_hi > k_lo ? k_lo / KB + warp : 0;
-  uint4 kraw[NT][G];
-  // (page, first slot) of a block; the page id of the next block is fetched a block ahead
+  // This warp's ring: the block being used and the next one, copied in by cp.async (8 KB in
+  // flight per warp without a register).  Lane l also holds the scales of key l of both.
+  const uint32_t ring = smem_u32(attn_smem) + warp * 2 * T::STAGE;
   auto first_slot = [&](int blk, int page) {
     return static_cast<size_t>(page) * 128 + ((blk * KB) & 127);
   };
-  auto load_k = [&](size_t slot0) {
+  RowScales<G, WIDE> ks_next, vs_next;
+  auto issue = [&](int blk, int page, int st) {
+    const size_t slot0 = first_slot(blk, page);
+    const int8_t* kp = kc + (slot0 * kvh + h) * D;
+    const int8_t* vp = vc + (slot0 * kvh + h) * D;
+    const uint32_t dst = ring + st * T::STAGE;
 #pragma unroll
-    for (int i = 0; i < NT; ++i) {
-      const int8_t* p = kc + ((slot0 + i * 8 + g) * kvh + h) * D + t * 16;
-#pragma unroll
-      for (int c = 0; c < G; ++c) kraw[i][c] = __ldg(reinterpret_cast<const uint4*>(p + c * 64));
+    for (int it = 0; it < KB * T::CPK / 32; ++it) {
+      const int key = (it * 32 + lane) / T::CPK, u = (it * 32 + lane) % T::CPK;
+      const size_t off = static_cast<size_t>(key) * kvh * D + u * 16;
+      cp_async16(dst + T::k_unit(key, u) * 16, kp + off);
+      cp_async16(dst + KB * D + T::v_unit(key, u) * 16, vp + off);
     }
+    const size_t cell = ((slot0 + (lane & (KB - 1))) * kvh + h) * G;
+    ks_next.load(ks + cell);
+    vs_next.load(vs + cell);
   };
+  // the page id of a block is fetched two blocks ahead
   int page_next = b + ATTN_WARPS < b_hi ? pages[((b + ATTN_WARPS) * KB) >> 7] : 0;
-  size_t slot0 = 0;
-  if (b < b_hi) {
-    slot0 = first_slot(b, pages[(b * KB) >> 7]);
-    load_k(slot0);
-  }
-  for (; b < b_hi; b += ATTN_WARPS) {
+  if (b < b_hi) issue(b, pages[(b * KB) >> 7], 0);
+  asm volatile("cp.async.commit_group;" ::: "memory");
+  for (int st = 0; b < b_hi; b += ATTN_WARPS, st ^= 1) {
     const int key0 = b * KB;
-    // values and scales of this block: in flight while the scores are formed
-    uint2 vraw[UT][4][G];
+    RowScales<G, WIDE> ks_cur = ks_next, vs_cur = vs_next;
+    if (b + ATTN_WARPS < b_hi) {
+      issue(b + ATTN_WARPS, page_next, st ^ 1);
+      if (b + 2 * ATTN_WARPS < b_hi) page_next = pages[((b + 2 * ATTN_WARPS) * KB) >> 7];
+    }
+    asm volatile("cp.async.commit_group;" ::: "memory");
+    asm volatile("cp.async.wait_group 1;" ::: "memory");
+    __syncwarp();
+    const uint32_t k_s = ring + st * T::STAGE, v_s = k_s + KB * D;
+    // scales of this lane's keys 8 i + 2 t + e
     RowScales<G, WIDE> vsc[UT][4], ksc[NT][2];
 #pragma unroll
     for (int i = 0; i < NT; ++i)
 #pragma unroll
-      for (int e = 0; e < 2; ++e)
-        ksc[i][e].load(ks + ((slot0 + i * 8 + 2 * t + e) * kvh + h) * G);
-#pragma unroll
-    for (int u = 0; u < UT; ++u)
-#pragma unroll
-      for (int e = 0; e < 4; ++e) {
-        const size_t cell = (slot0 + u * 16 + 2 * t + (e & 1) + (e >> 1) * 8) * kvh + h;
-#pragma unroll
-        for (int c = 0; c < G; ++c)
-          vraw[u][e][c] = __ldg(reinterpret_cast<const uint2*>(vc + cell * D + c * 64 + g * 8));
-        vsc[u][e].load(vs + cell * G);
+      for (int e = 0; e < 2; ++e) {
+        ksc[i][e] = ks_cur.from(8 * i + 2 * t + e);
+        vsc[i >> 1][(i & 1) * 2 + e] = vs_cur.from(8 * i + 2 * t + e);
       }
     // ---- scores: lane (g, t) gets head g against keys 8 i + 2 t and 8 i + 2 t + 1
     float s[NT][2];
@@ -185,7 +225,10 @@ __global__ void __launch_bounds__(ATTN_WARPS * 32, AttnTile<D>::MIN_CTAS) attn_r
 #pragma unroll
       for (int i = 0; i < NT; ++i) {
         float d[4] = {0.f, 0.f, 0.f, 0.f};
-        const uint32_t w[4] = {kraw[i][c].x, kraw[i][c].y, kraw[i][c].z, kraw[i][c].w};
+        uint32_t w[4];
+        asm volatile("ld.shared.v4.u32 {%0, %1, %2, %3}, [%4];"
+                     : "=r"(w[0]), "=r"(w[1]), "=r"(w[2]), "=r"(w[3])
+                     : "r"(k_s + T::k_unit(i * 8 + g, c * 4 + t) * 16));
 #pragma unroll
         for (int st = 0; st < 4; ++st) {
           const uint32_t x = w[st] ^ 0x80808080u;
@@ -213,12 +256,6 @@ __global__ void __launch_bounds__(ATTN_WARPS * 32, AttnTile<D>::MIN_CTAS) attn_r
             vsc[i >> 1][(i & 1) * 2 + e].clear();
           }
         }
-    }
-    // keys of the next block
-    if (b + ATTN_WARPS < b_hi) {
-      slot0 = first_slot(b + ATTN_WARPS, page_next);
-      load_k(slot0);
-      if (b + 2 * ATTN_WARPS < b_hi) page_next = pages[((b + 2 * ATTN_WARPS) * KB) >> 7];
     }
     // ---- softmax state
     float mb = s[0][0], vmax = 0.f;
@@ -271,12 +308,18 @@ __global__ void __launch_bounds__(ATTN_WARPS * 32, AttnTile<D>::MIN_CTAS) attn_r
         }
         const uint32_t a0 = pack_half2(hi[0], hi[1]), a1 = pack_half2(lo[0], lo[1]);
         const uint32_t a2 = pack_half2(hi[2], hi[3]), a3 = pack_half2(lo[2], lo[3]);
+        uint2 vraw[4];                             // 8 channels of keys 2 t, 2 t + 1 (+ 8)
+#pragma unroll
+        for (int e = 0; e < 4; ++e)
+          asm volatile("ld.shared.v2.u32 {%0, %1}, [%2];"
+                       : "=r"(vraw[e].x), "=r"(vraw[e].y)
+                       : "r"(v_s + T::v_unit(u * 16 + 2 * t + (e & 1) + (e >> 1) * 8,
+                                             c * 4 + (g >> 1)) * 16 + (g & 1) * 8));
 #pragma unroll
         for (int wd = 0; wd < 2; ++wd) {
           uint32_t x[4];
 #pragma unroll
-          for (int e = 0; e < 4; ++e)
-            x[e] = (wd == 0 ? vraw[u][e][c].x : vraw[u][e][c].y) ^ 0x80808080u;
+          for (int e = 0; e < 4; ++e) x[e] = (wd == 0 ? vraw[e].x : vraw[e].y) ^ 0x80808080u;
           // bytes of two keys interleaved: (k0 b0, k1 b0, k0 b1, k1 b1), then b2 and b3
           const uint32_t p01 = __byte_perm(x[0], x[1], 0x5140), p23 = __byte_perm(x[0], x[1], 0x7362);
           const uint32_t r01 = __byte_perm(x[2], x[3], 0x5140), r23 = __byte_perm(x[2], x[3], 0x7362);
@@ -288,7 +331,10 @@ __global__ void __launch_bounds__(ATTN_WARPS * 32, AttnTile<D>::MIN_CTAS) attn_r
         }
       }
     }
+    __syncwarp();                                // the stage is refilled next
   }
+  asm volatile("cp.async.wait_group 0;" ::: "memory");
+  __syncthreads();                               // the rings become the result buffers
   // ---- this warp's result: head + remainder rows, back to the unscaled weights
   l_run += __shfl_xor_sync(0xffffffffu, l_run, 1);
   l_run += __shfl_xor_sync(0xffffffffu, l_run, 2);
@@ -379,7 +425,15 @@ static int launch_attn(const __half* q, const __half* gate, const int* row_req, 
   const bool wide = ((reinterpret_cast<uintptr_t>(q) & 15) | (reinterpret_cast<uintptr_t>(ks) & 7) |
                      (reinterpret_cast<uintptr_t>(vs) & 7)) == 0;
   auto kernel = wide ? attn_rows_kernel<D, true> : attn_rows_kernel<D, false>;
-  kernel<<<grid, ATTN_WARPS * 32, 0, stream>>>(q, gate, row_req, row_pos, page_table, max_pages, kc,
+  constexpr int SMEM = AttnTile<D>::SMEM;
+  if (runtime_ensure_init() != cudaSuccess) return -2;
+  static const int slot[2] = {runtime_new_slot(), runtime_new_slot()};
+  if (runtime_first_use(slot[wide])) {
+    const cudaError_t e =
+        cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM);
+    if (e != cudaSuccess) return static_cast<int>(e);
+  }
+  kernel<<<grid, ATTN_WARPS * 32, SMEM, stream>>>(q, gate, row_req, row_pos, page_table, max_pages, kc,
                                                vc, ks, vs, out, qh, kvh, splits, scratch, rep);
   if (splits > 1)
     attn_merge_kernel<D><<<dim3(rows, qh), D < 128 ? 64 : 128, 0, stream>>>(scratch, gate, out, qh,
