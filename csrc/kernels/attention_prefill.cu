@@ -1,21 +1,29 @@
 // Causal GQA flash attention for prefill chunks over the paged INT8 KV cache, on
 // tcgen05 tensor cores with TMEM accumulators.
 //
-// One CTA owns a 128-row query tile: P = 128 / rep consecutive query positions of one
-// request times the `rep` query heads that share one KV head (the heads are packed into
-// the MMA M axis so each INT8 K/V page is dequantised once for all of them).  Per KV
-// page (128 keys = one cache page):
-//   * warps 6-9 read the INT8 page and its group-64 FP16 scales straight from global
-//     memory, dequantise to FP16 and store K and V as 128-byte-swizzled tiles
-//     (K is the K-major B operand of S = Q K^T, V the MN-major B operand of O += P V);
-//   * warp 1 issues tcgen05.mma kind::f16: S (128x128 fp32) and O (128xD fp32) live in TMEM;
-//   * warps 2-5 own one query row per thread: they read S from TMEM, apply scale and the
-//     causal mask, keep the running max / sum, rescale O in TMEM when the max moved,
-//     and write P as FP16 into shared memory for the second MMA;
-//   * warp 0 loads the Q tile once with a 3-D TMA (d, head, position).
-// Head size 256 walks the cache in half pages (KT = 64 keys per step): Q (64 KB), two K and
-// two V buffers (32 KB each) and two P buffers then fill the 227 KB of one CTA exactly, and
-// S0 | S1 | O (64 + 64 + 256 columns) still fit in TMEM.
+// A query tile is 128 rows: P = 128 / rep consecutive query positions of one request times the
+// `rep` query heads that share one KV head (the heads are packed into the MMA M axis so each
+// INT8 K/V page is dequantised once for all of them).  One CTA owns NQ tiles: two neighbouring
+// ones for head sizes 64 and 128, so that a dequantised page serves 256 rows and the tensor core
+// works on one tile while the softmax warps of the other are busy.  Per step of KT keys:
+//   * eight warps, in two groups that take the steps in turn, read the INT8 page and its
+//     group-64 FP16 scales straight from global memory (ahead, in registers), dequantise to FP16 and store K and V as
+//     128-byte-swizzled tiles (K is the K-major B operand of S = Q K^T, V the MN-major B
+//     operand of O += P V);
+//   * warp 1 issues tcgen05.mma kind::f16: S (128 x KT fp32) and O (128 x D fp32) live in TMEM;
+//   * four warps per tile own one query row per thread: they read S from TMEM, apply scale and
+//     the causal mask, and write P as FP16 over S in TMEM, where the second MMA reads it as its
+//     A operand.  The reference maximum of a row only moves when a score exceeds it by 2^8 (P
+//     stays below 256 and the sums in FP32), so rescaling O is rare after the first steps;
+//   * warp 0 loads the Q tiles once with a 3-D TMA (d, head, position).
+// Head size 256 has room for one tile (Q 64 KB, two K and two V buffers of 32 KB; TMEM: two S of
+// 64 columns and O of 256) and walks the cache in half pages, with S double buffered instead.
+// CTAs are ordered from the last query positions (the longest walks) to the first.
+//
+// One 4096-token chunk, 32 / 8 heads of 128: 385 us with one tile per CTA and P in shared memory,
+// 220 us now (625 TFLOP/s causal); of that 158 us remain with the softmax and the conversions
+// switched off, the issue chain of 128 x 128 MMAs.  Chunks of 777 and 646 rows behind 3000
+// positions, 16 / 2 gated heads of 256: 373 -> 279 us (180 CTAs: 1.2 waves).
 // Output is O / sum, optionally times sigmoid(gate), in FP16.  Replaces the prefill
 // configurations of causal_attention_int8 and dequantize_attention_kv
 // (kernels/cuda/model/attention_rows.py:61-276, kernels/cuda/model/kv_int8.py:210-247).
@@ -28,24 +36,41 @@
 namespace orinfer {
 namespace fa {
 
-constexpr int THREADS = 320;                 // 10 warps
-constexpr int TILE = 128;                    // query rows per CTA and keys per KV step
+constexpr int TILE = 128;                    // query rows per tile
+constexpr int DQ_WARPS = 8;                  // dequantisation warps
 
 template <int D>
 struct Smem {
+  static constexpr int NQ = D > 128 ? 1 : 2;             // query tiles per CTA
+  static constexpr int THREADS = (2 + 4 * NQ + DQ_WARPS) * 32;
   static constexpr int KT = D > 128 ? 64 : 128;          // keys per step
-  static constexpr int SUB = TILE * 128;                 // one [128 x 64 fp16] sub-tile (Q, P)
+  static constexpr int SUB = TILE * 128;                 // one [128 x 64 fp16] sub-tile (Q)
   static constexpr int KSUB = KT * 128;                  // one [KT x 64 fp16] sub-tile (K, V)
   static constexpr int NSUB = D / 64;                    // sub-tiles per operand
-  static constexpr int PSUB = KT / 64;                   // sub-tiles of one P buffer
-  static constexpr int Q_OFF = 0;
-  static constexpr int K_OFF = Q_OFF + NSUB * SUB;       // two K buffers
+  static constexpr int Q_OFF = 0;                        // NQ tiles
+  static constexpr int K_OFF = Q_OFF + NQ * NSUB * SUB;  // two K buffers
   static constexpr int V_OFF = K_OFF + 2 * NSUB * KSUB;  // two V buffers
-  static constexpr int P_OFF = V_OFF + 2 * NSUB * KSUB;  // two P buffers of 128 x KT fp16
-  static constexpr int BAR_OFF = P_OFF + 2 * PSUB * SUB;
+  static constexpr int BAR_OFF = V_OFF + 2 * NSUB * KSUB;
   static constexpr int TOTAL = BAR_OFF + 256 + 1024;
   static_assert(TOTAL <= 227 * 1024, "exceeds the shared memory of one CTA");
 };
+
+// D[tmem] (+)= A[tmem] * B[smem]: A holds two FP16 values of a row per 32-bit column.
+__device__ __forceinline__ void mma_f16_ts(uint32_t tmem_d, uint32_t tmem_a, uint64_t bdesc,
+                                           uint32_t idesc, uint32_t accumulate) {
+  asm volatile(
+      "{\n\t.reg .pred p;\n\t"
+      "setp.ne.b32 p, %4, 0;\n\t"
+      "tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], %2, %3, p;\n\t}" ::"r"(tmem_d),
+      "r"(tmem_a), "l"(bdesc), "r"(idesc), "r"(accumulate)
+      : "memory");
+}
+
+__device__ __forceinline__ float ex2(float x) {
+  float y;
+  asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
+  return y;
+}
 
 // Eight INT8 values (two words) -> eight FP16 values times an FP16 scale, exactly
 // half(float(q) * float(scale)): build 1152 + q as a half via byte permute, subtract,
@@ -77,49 +102,56 @@ struct Chunk {            // one prefill chunk of one request
 };
 
 template <int D>
-__global__ void __launch_bounds__(THREADS, 1) attn_prefill_kernel(
+__global__ void __launch_bounds__(Smem<D>::THREADS, 1) attn_prefill_kernel(
     const __grid_constant__ CUtensorMap tmap_q, const Chunk* __restrict__ chunks,
     const int* __restrict__ page_table, int max_pages, const int8_t* __restrict__ kc,
     const int8_t* __restrict__ vc, const __half* __restrict__ ks, const __half* __restrict__ vs,
     const __half* __restrict__ gate, __half* __restrict__ out, int qh, int kvh, int rep,
     int num_pages, int* status) {
   using L = Smem<D>;
-  constexpr int NSUB = L::NSUB;
-  constexpr int KT = L::KT;
+  constexpr int NQ = L::NQ, NSUB = L::NSUB, KT = L::KT;
   constexpr int GROUPS = D / 64;
-  constexpr uint32_t TMEM_COLS = 512;          // S0 | S1 (128 columns each) | O (D columns)
+  constexpr uint32_t TMEM_COLS = 512;
+  constexpr int S_STRIDE = NQ == 2 ? 128 : 64;    // S of tile q (NQ = 2) or of buffer b (NQ = 1)
   extern __shared__ unsigned char smem_raw[];
   unsigned char* smem = smem_raw + ((1024u - (smem_u32(smem_raw) & 1023u)) & 1023u);
   uint64_t* bars = reinterpret_cast<uint64_t*>(smem + L::BAR_OFF);
-  uint64_t* q_full = bars;            // Q tile landed
-  uint64_t* kv_ready = bars + 1;      // [2] dequantised K/V buffer filled (128 arrivals)
-  uint64_t* s_full = bars + 3;        // [2] S[b] = QK^T finished
-  uint64_t* p_ready = bars + 5;       // [2] P[b] written, S[b] consumed, O rescaled (128 arrivals)
-  uint64_t* o_done = bars + 7;        // O += PV finished (O may be rescaled)
-  uint64_t* kv_free = bars + 8;       // [2] the PV that read K/V buffer b finished
-  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 10);
+  uint64_t* q_full = bars;            // Q tiles landed
+  uint64_t* kv_ready = bars + 1;      // [2] dequantised K/V buffer filled
+  uint64_t* s_full = bars + 3;        // [2] S = QK^T finished (per tile, or per buffer)
+  uint64_t* p_ready = bars + 5;       // [2] P written over S, O rescaled (128 arrivals)
+  uint64_t* o_done = bars + 7;        // [2] O += PV finished (per tile)
+  uint64_t* kv_free = bars + 9;       // [2] the last MMA that read K/V buffer b finished
+  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 11);
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const Chunk ch = chunks[blockIdx.z];
   const int h = blockIdx.y;                       // kv head
   const int P = TILE / rep;                       // query positions per tile
-  const int p_first = blockIdx.x * P;             // first chunk-relative position of this tile
+  // first chunk-relative position of this CTA's tiles; long walks start first
+  const int p_first = static_cast<int>(gridDim.x - 1 - blockIdx.x) * NQ * P;
   if (p_first >= ch.q_len) return;
-  const int p_count = min(P, ch.q_len - p_first);
-  const int last_pos = ch.pos0 + p_first + p_count - 1;
-  const int n_tiles = last_pos / KT + 1;          // KV steps that any row of the tile can see
+  // steps that any row of tile q can see (0: the chunk ends before the tile)
+  auto steps_of = [&](int q) {
+    const int first = p_first + q * P;
+    return first >= ch.q_len ? 0 : (ch.pos0 + min(first + P, ch.q_len) - 1) / KT + 1;
+  };
+  int n_steps[NQ], n_max = 0;
+#pragma unroll
+  for (int q = 0; q < NQ; ++q) {
+    n_steps[q] = steps_of(q);
+    n_max = max(n_max, n_steps[q]);
+  }
 
   if (threadIdx.x == 0) {
     mbar_init(q_full, 1);
-    mbar_init(&kv_ready[0], 128);
-    mbar_init(&kv_ready[1], 128);
-    mbar_init(&s_full[0], 1);
-    mbar_init(&s_full[1], 1);
-    mbar_init(&p_ready[0], 128);
-    mbar_init(&p_ready[1], 128);
-    mbar_init(o_done, 1);
-    mbar_init(&kv_free[0], 1);
-    mbar_init(&kv_free[1], 1);
+    for (int b = 0; b < 2; ++b) {
+      mbar_init(&kv_ready[b], 128);
+      mbar_init(&s_full[b], 1);
+      mbar_init(&p_ready[b], 128);
+      mbar_init(&o_done[b], 1);
+      mbar_init(&kv_free[b], 1);
+    }
     mbar_fence_init();
     prefetch_tmap(&tmap_q);
   }
@@ -131,109 +163,127 @@ __global__ void __launch_bounds__(THREADS, 1) attn_prefill_kernel(
   __syncthreads();
   tc_fence_after();
   const uint32_t tmem_base = *tmem_slot;
-  const uint32_t tmem_s = tmem_base, tmem_o = tmem_base + 256;   // S[b] at tmem_s + 128 * b
+  const uint32_t tmem_s = tmem_base, tmem_o = tmem_base + 256;   // O of tile q at + q * 128
   const int* pages = page_table + static_cast<size_t>(ch.slot) * max_pages;
 
   if (warp == 0) {
     if (lane == 0) {
-      mbar_expect_tx(q_full, static_cast<uint32_t>(NSUB) * 64 * 2 * rep * P);
-      for (int s = 0; s < NSUB; ++s)
-        tma_load_3d(smem + L::Q_OFF + s * L::SUB, &tmap_q, q_full, s * 64, h * rep,
-                    ch.row_start + p_first);
-      mbar_wait(q_full, 0, status, STATUS_TMA_WAIT, 1);     // our copy has landed before exit
+      mbar_expect_tx(q_full, static_cast<uint32_t>(NQ) * NSUB * 64 * 2 * rep * P);
+      for (int q = 0; q < NQ; ++q)
+        for (int s = 0; s < NSUB; ++s)
+          tma_load_3d(smem + L::Q_OFF + (q * NSUB + s) * L::SUB, &tmap_q, q_full, s * 64, h * rep,
+                      ch.row_start + p_first + q * P);
+      mbar_wait(q_full, 0, status, STATUS_TMA_WAIT, 1);     // our copies have landed before exit
     }
   } else if (warp == 1) {
     if (lane == 0) {
       constexpr uint32_t idesc_s = umma_idesc(1, 0, 0, 0, 0, TILE, KT);
       constexpr uint32_t idesc_o = umma_idesc(1, 0, 0, 0, 1, TILE, D);
       const uint32_t q_addr = smem_u32(smem + L::Q_OFF);
-      const uint32_t p_addr = smem_u32(smem + L::P_OFF);
       bool ok = mbar_wait(q_full, 0, status, STATUS_MMA_WAIT, 2);
-      // S and P are double buffered: S(j+1) = Q K(j+1)^T is issued before O += P(j) V(j), so
-      // the tensor core works on the next scores while the softmax warps turn S(j) into P(j).
-      auto issue_qk = [&](int j) -> bool {
-        const int b = j & 1;
-        if (!mbar_wait(&kv_ready[b], (j >> 1) & 1, status, STATUS_MMA_WAIT, 0x100 | j))
-          return false;
+      auto wait_kv = [&](int j) {
+        ok = ok && mbar_wait(&kv_ready[j & 1], (j >> 1) & 1, status, STATUS_MMA_WAIT, 0x100 | (j & 0xff));
         tc_fence_after();
-        const uint32_t k_addr = smem_u32(smem + L::K_OFF + b * NSUB * L::KSUB);
-#pragma unroll
-        for (int i = 0; i < D / 16; ++i) {
-          const uint32_t q_off = (i / 4) * L::SUB + (i % 4) * 32;
-          const uint32_t k_off = (i / 4) * L::KSUB + (i % 4) * 32;
-          mma_f16_ss(tmem_s + 128 * b, umma_desc(q_addr + q_off, 16, 1024),
-                     umma_desc(k_addr + k_off, 16, 1024), idesc_s, i != 0 ? 1u : 0u);
-        }
-        tc_commit(&s_full[b]);
-        return true;
       };
-      if (ok) ok = issue_qk(0);
-      for (int j = 0; j < n_tiles && ok; ++j) {
-        const int b = j & 1;
-        // S[(j+1)&1] was last read by the softmax of tile j-1, whose p_ready this thread
-        // waited for before issuing PV(j-1): program order makes the overwrite safe.
-        if (j + 1 < n_tiles) ok = issue_qk(j + 1);
-        if (!ok) break;
-        const uint32_t v_addr = smem_u32(smem + L::V_OFF + b * NSUB * L::KSUB);
-        const uint32_t pj_addr = p_addr + b * L::PSUB * L::SUB;
-        ok = mbar_wait(&p_ready[b], (j >> 1) & 1, status, STATUS_MMA_WAIT, 0x200 | j);
-        if (!ok) break;
-        tc_fence_after();
+      auto issue_qk = [&](int q, int j) {
+        const int sb = NQ == 2 ? q : j & 1;
+        const uint32_t k_addr = smem_u32(smem + L::K_OFF + (j & 1) * NSUB * L::KSUB);
 #pragma unroll
-        for (int i = 0; i < KT / 16; ++i) {
-          const uint32_t a_off = (i / 4) * L::SUB + (i % 4) * 32;
-          mma_f16_ss(tmem_o, umma_desc(pj_addr + a_off, 16, 1024),
+        for (int i = 0; i < D / 16; ++i)
+          mma_f16_ss(tmem_s + S_STRIDE * sb,
+                     umma_desc(q_addr + (q * NSUB + i / 4) * L::SUB + (i % 4) * 32, 16, 1024),
+                     umma_desc(k_addr + (i / 4) * L::KSUB + (i % 4) * 32, 16, 1024), idesc_s,
+                     i != 0 ? 1u : 0u);
+        tc_commit(&s_full[sb]);
+      };
+      auto issue_pv = [&](int q, int j) {
+        const int sb = NQ == 2 ? q : j & 1;
+        const uint32_t parity = (NQ == 2 ? j : j >> 1) & 1;
+        ok = ok && mbar_wait(&p_ready[sb], parity, status, STATUS_MMA_WAIT, 0x200 | (j & 0xff));
+        if (!ok) return;
+        tc_fence_after();
+        const uint32_t v_addr = smem_u32(smem + L::V_OFF + (j & 1) * NSUB * L::KSUB);
+#pragma unroll
+        for (int i = 0; i < KT / 16; ++i)
+          mma_f16_ts(tmem_o + 128 * q, tmem_s + S_STRIDE * sb + i * 8,
                      umma_desc(v_addr + i * 2048, L::KSUB, 1024), idesc_o, (j | i) != 0 ? 1u : 0u);
+        tc_commit(&o_done[q]);
+      };
+      // MMAs of one thread run in order.  NQ = 2: QK of step j + 1 overwrites the P of step j of
+      // the same tile, so it follows that tile's PV; meanwhile the other tile's softmax runs.
+      // NQ = 1: QK of step j + 1 goes into the other S buffer, ahead of PV of step j.
+      wait_kv(0);
+#pragma unroll
+      for (int q = 0; q < NQ; ++q)
+        if (ok && n_steps[q] > 0) issue_qk(q, 0);
+      for (int j = 0; j < n_max && ok; ++j) {
+        const bool more = j + 1 < n_max;
+        if (NQ == 1 && more) {
+          wait_kv(j + 1);
+          if (ok) issue_qk(0, j + 1);
         }
-        tc_commit(o_done);
-        tc_commit(&kv_free[b]);
+#pragma unroll
+        for (int q = 0; q < NQ; ++q) {
+          if (ok && j < n_steps[q]) issue_pv(q, j);
+          if (q == NQ - 1 && ok) tc_commit(&kv_free[j & 1]);
+          if (NQ == 2 && ok && more) {
+            if (q == 0) wait_kv(j + 1);
+            if (ok && j + 1 < n_steps[q]) issue_qk(q, j + 1);
+          }
+        }
       }
     }
-  } else if (warp >= 6) {
+  } else if (warp >= 2 + 4 * NQ) {
     // ---------------- dequant warps: INT8 page -> FP16 swizzled K / V tiles
-    const int t = threadIdx.x - 192;                 // 0..127
-    bool ok = true;
-    for (int j = 0; j < n_tiles && ok; ++j) {
-      const int b = j & 1;
-      int page = pages[j * KT / TILE];
+    // Two groups of four warps take the steps (and their buffer) in turn: a step's loads are in
+    // flight while the other group converts, which a single group could only do with twice the
+    // registers (measured: the wait for the loads bounded a step).
+    const int group = (warp - (2 + 4 * NQ)) >> 2;
+    static_assert(DQ_WARPS == 8, "two groups of 128 threads");
+    constexpr int CPK = D / 16;                      // 16-byte chunks per key
+    constexpr int ITERS = KT * CPK / 128;
+    uint4 kraw[ITERS], vraw[ITERS];
+    __half2 sc[ITERS];                               // key scale, value scale
+    const int u = (threadIdx.x - (2 + 4 * NQ) * 32) & 127;
+    auto load = [&](int j, int page) {
       const int key_base = j * KT % TILE;            // first key of this step inside the page
       if (page < 0 || page >= num_pages) {
         report_status(status, STATUS_BAD_INDEX, 3);
         page = 0;
       }
-      unsigned char* kb = smem + L::K_OFF + b * NSUB * L::KSUB;
-      unsigned char* vb = smem + L::V_OFF + b * NSUB * L::KSUB;
-      constexpr int CPK = D / 16;                    // 16-byte chunks per key
-      constexpr int ITERS = KT * CPK / 128;
-      // every load of the page is issued before the first conversion: one memory round trip
-      // per page instead of one per pair of chunks (the 128 dequant threads have no other
-      // way to hide latency)
-      uint4 kraw[ITERS], vraw[ITERS];
-      __half ksc[ITERS], vsc[ITERS];
+      // one base address per step; the rows of a thread are a fixed distance apart
+      const size_t slot = (static_cast<size_t>(page) * 128 + key_base + u / CPK) * kvh + h;
+      const int8_t* kp = kc + slot * D + (u % CPK) * 16;
+      const int8_t* vp = vc + slot * D + (u % CPK) * 16;
+      const __half* ksp = ks + slot * GROUPS + (u % CPK) / 4;
+      const __half* vsp = vs + slot * GROUPS + (u % CPK) / 4;
+      const int rows = (128 / CPK) * kvh;
 #pragma unroll
       for (int it = 0; it < ITERS; ++it) {
-        const int idx = it * 128 + t;
-        const int key = idx / CPK, c = idx % CPK;
-        const size_t slot = (static_cast<size_t>(page) * 128 + key_base + key) * kvh + h;
-        kraw[it] = __ldg(reinterpret_cast<const uint4*>(kc + slot * D + c * 16));
-        vraw[it] = __ldg(reinterpret_cast<const uint4*>(vc + slot * D + c * 16));
-        ksc[it] = ks[slot * GROUPS + c / 4];
-        vsc[it] = vs[slot * GROUPS + c / 4];
+        kraw[it] = __ldg(reinterpret_cast<const uint4*>(kp + static_cast<size_t>(it) * rows * D));
+        vraw[it] = __ldg(reinterpret_cast<const uint4*>(vp + static_cast<size_t>(it) * rows * D));
+        sc[it] = __halves2half2(ksp[it * rows * GROUPS], vsp[it * rows * GROUPS]);
       }
-      // buffer b was last read by the MMAs of tile j-2: wait for its PV to finish.  A
-      // per-buffer barrier is used because a waiter two phases behind a shared barrier
-      // would alias its parity.
+    };
+    bool ok = true;
+    unsigned char* kb = smem + L::K_OFF + group * NSUB * L::KSUB;
+    unsigned char* vb = smem + L::V_OFF + group * NSUB * L::KSUB;
+    int page = 0;
+    if (group < n_max) load(group, pages[group * KT / TILE]);
+    if (group + 2 < n_max) page = pages[(group + 2) * KT / TILE];
+    for (int j = group; j < n_max && ok; j += 2) {
+      // buffer `group` was last read by the MMAs of step j - 2.  A per-buffer barrier is used
+      // because a waiter two phases behind a shared barrier would alias its parity.
       if (j >= 2)
-        ok = mbar_wait(&kv_free[b], ((j >> 1) - 1) & 1, status, STATUS_DECODE_WAIT, j);
+        ok = mbar_wait(&kv_free[group], ((j >> 1) - 1) & 1, status, STATUS_DECODE_WAIT, j);
       if (!ok) break;
 #pragma unroll
       for (int it = 0; it < ITERS; ++it) {
-        const int idx = it * 128 + t;
-        const int key = idx / CPK, c = idx % CPK;
-        const __half2 k2 = __half2half2(ksc[it]), v2 = __half2half2(vsc[it]);
-        const int sub = c / 4, chunk = (c % 4) * 2;
-        unsigned char* kd = kb + sub * L::KSUB;
-        unsigned char* vd = vb + sub * L::KSUB;
+        const int key = it * (128 / CPK) + u / CPK, c = u % CPK;
+        const __half2 k2 = __low2half2(sc[it]), v2 = __high2half2(sc[it]);
+        const int chunk = (c % 4) * 2;
+        unsigned char* kd = kb + (c / 4) * L::KSUB;
+        unsigned char* vd = vb + (c / 4) * L::KSUB;
         *reinterpret_cast<uint4*>(kd + swz128(key, chunk)) = dequant8(kraw[it].x, kraw[it].y, k2);
         *reinterpret_cast<uint4*>(kd + swz128(key, chunk + 1)) =
             dequant8(kraw[it].z, kraw[it].w, k2);
@@ -242,128 +292,144 @@ __global__ void __launch_bounds__(THREADS, 1) attn_prefill_kernel(
             dequant8(vraw[it].z, vraw[it].w, v2);
       }
       fence_proxy_async();
-      mbar_arrive(&kv_ready[b]);
+      mbar_arrive(&kv_ready[group]);
+      if (j + 2 < n_max) {
+        load(j + 2, page);
+        if (j + 4 < n_max) page = pages[(j + 4) * KT / TILE];
+      }
     }
   } else {
     // ---------------- softmax warps: one query row per thread
+    const int q = (warp - 2) >> 2;                          // tile
     const int quad = warp & 3;
     const int row = quad * 32 + lane;                       // row of the tile = TMEM lane
+    const int first = p_first + q * P;
     const int p_rel = row / rep, head = h * rep + row % rep;
-    const bool valid = p_rel < p_count;
-    const int q_pos = valid ? ch.pos0 + p_first + p_rel : -1;
+    const bool valid = row < P * rep && first + p_rel < ch.q_len;
+    const int q_pos = valid ? ch.pos0 + first + p_rel : -1;
     const float scale = rsqrtf(static_cast<float>(D)) * 1.4426950408889634f;
     const uint32_t lane_addr = static_cast<uint32_t>(quad * 32) << 16;
-    float m_run = -INFINITY, l_run = 0.f;
+    const uint32_t tmem_oq = tmem_o + 128 * q + lane_addr;
+    const int steps = NQ == 2 && q == 1 ? n_steps[NQ - 1] : n_steps[0];
+    float m_ref = -INFINITY, l_run = 0.f;
     bool ok = true;
-    for (int j = 0; j < n_tiles; ++j) {
-      const int sb = j & 1;
-      const uint32_t tmem_sj = tmem_s + 128 * sb;
-      unsigned char* pb = smem + L::P_OFF + sb * L::PSUB * L::SUB;
-      ok = mbar_wait(&s_full[sb], (j >> 1) & 1, status, STATUS_EPILOGUE_WAIT, j);
+    for (int j = 0; j < steps; ++j) {
+      const int sb = NQ == 2 ? q : j & 1;
+      const uint32_t parity = (NQ == 2 ? j : j >> 1) & 1;
+      const uint32_t tmem_sj = tmem_s + S_STRIDE * sb + lane_addr;
+      ok = mbar_wait(&s_full[sb], parity, status, STATUS_EPILOGUE_WAIT, j);
       ok = __all_sync(0xffffffffu, ok);
       if (!ok) break;
       tc_fence_after();
       const int key0 = j * KT;
       // Only the last page of a row can hold keys beyond its position; every earlier page
-      // takes the mask-free path (one FMNMX per score here, FFMA + EX2 per score below).
-      const bool full = key0 + KT - 1 <= q_pos;
+      // takes the mask-free path.
+      const bool full_warp = __all_sync(0xffffffffu, key0 + KT - 1 <= q_pos);
       // pass 1: row maximum (of the raw scores: the scale is positive)
-      float m_raw = -INFINITY;
+      float m0 = -INFINITY, m1 = -INFINITY;
 #pragma unroll 1
       for (int c0 = 0; c0 < KT; c0 += 64) {
         uint32_t r[32], r2[32];                           // two TMEM loads in flight
-        tmem_ld_32x32(tmem_sj + lane_addr + c0, r);
-        tmem_ld_32x32(tmem_sj + lane_addr + c0 + 32, r2);
+        tmem_ld_32x32(tmem_sj + c0, r);
+        tmem_ld_32x32(tmem_sj + c0 + 32, r2);
         tc_wait_ld();
-        if (full) {
+        if (full_warp) {
 #pragma unroll
-          for (int i = 0; i < 32; ++i)
-            m_raw = fmaxf(m_raw, fmaxf(__uint_as_float(r[i]), __uint_as_float(r2[i])));
+          for (int i = 0; i < 32; ++i) {
+            m0 = fmaxf(m0, __uint_as_float(r[i]));
+            m1 = fmaxf(m1, __uint_as_float(r2[i]));
+          }
         } else {
 #pragma unroll
           for (int i = 0; i < 32; ++i) {
-            if (key0 + c0 + i <= q_pos) m_raw = fmaxf(m_raw, __uint_as_float(r[i]));
-            if (key0 + c0 + 32 + i <= q_pos) m_raw = fmaxf(m_raw, __uint_as_float(r2[i]));
+            if (key0 + c0 + i <= q_pos) m0 = fmaxf(m0, __uint_as_float(r[i]));
+            if (key0 + c0 + 32 + i <= q_pos) m1 = fmaxf(m1, __uint_as_float(r2[i]));
           }
         }
       }
-      const float m_tile = m_raw * scale;               // -inf stays -inf
-      const float m_new = fmaxf(m_run, m_tile);
-      const float corr = (m_new == -INFINITY) ? 1.f : exp2f(m_run - m_new);
-      // P buffer and O are free once PV of tile j-1 has finished
+      const float m_tile = fmaxf(m0, m1) * scale;       // -inf stays -inf
+      // O holds steps 0..j-1 once PV of step j-1 is done.  Waited for at every step, so that no
+      // wait is ever two phases away from its barrier; NQ = 2: it is done, QK ran after it.
       if (j >= 1) {
-        ok = mbar_wait(o_done, (j - 1) & 1, status, STATUS_EPILOGUE_WAIT, 0x100 | j);
+        ok = mbar_wait(&o_done[q], (j - 1) & 1, status, STATUS_EPILOGUE_WAIT, 0x100 | j);
         ok = __all_sync(0xffffffffu, ok);
         if (!ok) break;
         tc_fence_after();
-        if (!__all_sync(0xffffffffu, corr == 1.f)) {
+      }
+      // the reference moves when a score is above it by more than 2^8 (or it has none yet)
+      const bool moves = m_tile > m_ref + 8.f || (m_ref == -INFINITY && m_tile > -INFINITY);
+      if (__any_sync(0xffffffffu, moves)) {
+        const float m_new = moves ? m_tile : m_ref;
+        const float corr = moves ? (m_ref == -INFINITY ? 0.f : ex2(m_ref - m_new)) : 1.f;
+        m_ref = m_new;
+        l_run *= corr;
+        if (j >= 1) {
 #pragma unroll 1
           for (int c0 = 0; c0 < D; c0 += 32) {
             uint32_t r[32];
-            tmem_ld_32x32(tmem_o + lane_addr + c0, r);
+            tmem_ld_32x32(tmem_oq + c0, r);
             tc_wait_ld();
 #pragma unroll
             for (int i = 0; i < 32; ++i) r[i] = __float_as_uint(__uint_as_float(r[i]) * corr);
-            tmem_st_32x32(tmem_o + lane_addr + c0, r);
+            tmem_st_32x32(tmem_oq + c0, r);
           }
           tc_wait_st();
         }
       }
-      // pass 2: probabilities -> FP16 P tile, row sum
-      float l_tile = 0.f;
+      // pass 2: probabilities -> FP16 over the scores already read, row sum
+      const float m_use = m_ref == -INFINITY ? 0.f : m_ref;
+      float l0 = 0.f, l1 = 0.f;
 #pragma unroll 1
-      for (int c0 = 0; c0 < KT; c0 += 32) {
-        uint32_t r[32];
-        tmem_ld_32x32(tmem_sj + lane_addr + c0, r);
-        tc_wait_ld();
-        uint32_t packed[16];
-        if (full) {
+      for (int c0 = 0; c0 < KT; c0 += 64) {
+        uint32_t packed[32];
 #pragma unroll
-          for (int i = 0; i < 32; i += 2) {
-            const float p0 = exp2f(fmaf(__uint_as_float(r[i]), scale, -m_new));
-            const float p1 = exp2f(fmaf(__uint_as_float(r[i + 1]), scale, -m_new));
-            l_tile += p0 + p1;
-            const __half2 hp = __floats2half2_rn(p0, p1);
-            packed[i / 2] = *reinterpret_cast<const uint32_t*>(&hp);
-          }
-        } else {
+        for (int hf = 0; hf < 2; ++hf) {
+          uint32_t r[32];
+          tmem_ld_32x32(tmem_sj + c0 + hf * 32, r);
+          tc_wait_ld();
+          if (full_warp) {
 #pragma unroll
-          for (int i = 0; i < 32; i += 2) {
-            float p0 = 0.f, p1 = 0.f;
-            if (key0 + c0 + i <= q_pos) p0 = exp2f(fmaf(__uint_as_float(r[i]), scale, -m_new));
-            if (key0 + c0 + i + 1 <= q_pos)
-              p1 = exp2f(fmaf(__uint_as_float(r[i + 1]), scale, -m_new));
-            l_tile += p0 + p1;
-            const __half2 hp = __floats2half2_rn(p0, p1);
-            packed[i / 2] = *reinterpret_cast<const uint32_t*>(&hp);
+            for (int i = 0; i < 32; i += 2) {
+              const float p0 = ex2(fmaf(__uint_as_float(r[i]), scale, -m_use));
+              const float p1 = ex2(fmaf(__uint_as_float(r[i + 1]), scale, -m_use));
+              l0 += p0;
+              l1 += p1;
+              const __half2 hp = __floats2half2_rn(p0, p1);
+              packed[hf * 16 + i / 2] = *reinterpret_cast<const uint32_t*>(&hp);
+            }
+          } else {
+#pragma unroll
+            for (int i = 0; i < 32; i += 2) {
+              float p0 = ex2(fmaf(__uint_as_float(r[i]), scale, -m_use));
+              float p1 = ex2(fmaf(__uint_as_float(r[i + 1]), scale, -m_use));
+              if (key0 + c0 + hf * 32 + i > q_pos) p0 = 0.f;
+              if (key0 + c0 + hf * 32 + i + 1 > q_pos) p1 = 0.f;
+              l0 += p0;
+              l1 += p1;
+              const __half2 hp = __floats2half2_rn(p0, p1);
+              packed[hf * 16 + i / 2] = *reinterpret_cast<const uint32_t*>(&hp);
+            }
           }
         }
-        // keys c0..c0+31 -> sub-tile c0/64, 16-byte chunks ((c0 % 64) / 8) .. +3
-        unsigned char* dst = pb + (c0 / 64) * L::SUB;
-        const int chunk0 = (c0 % 64) / 8;
-#pragma unroll
-        for (int q = 0; q < 4; ++q)
-          *reinterpret_cast<uint4*>(dst + swz128(row, chunk0 + q)) =
-              make_uint4(packed[q * 4], packed[q * 4 + 1], packed[q * 4 + 2], packed[q * 4 + 3]);
+        tmem_st_32x32(tmem_sj + c0 / 2, packed);
       }
-      l_run = l_run * corr + l_tile;
-      m_run = m_new;
+      tc_wait_st();
+      l_run += l0 + l1;
       tc_fence_before();
-      fence_proxy_async();
       mbar_arrive(&p_ready[sb]);
     }
-    if (ok) {
-      ok = mbar_wait(o_done, (n_tiles - 1) & 1, status, STATUS_EPILOGUE_WAIT, 0x300);
+    if (ok && steps > 0) {
+      ok = mbar_wait(&o_done[q], (steps - 1) & 1, status, STATUS_EPILOGUE_WAIT, 0x300);
       ok = __all_sync(0xffffffffu, ok);
     }
-    if (ok) {
+    if (ok && steps > 0) {
       tc_fence_after();
       const float inv = l_run > 0.f ? 1.f / l_run : 0.f;
-      const size_t orow = static_cast<size_t>(ch.row_start + p_first + p_rel) * qh + head;
+      const size_t orow = static_cast<size_t>(ch.row_start + first + p_rel) * qh + head;
 #pragma unroll 1
       for (int c0 = 0; c0 < D; c0 += 32) {
         uint32_t r[32];
-        tmem_ld_32x32(tmem_o + lane_addr + c0, r);
+        tmem_ld_32x32(tmem_oq + c0, r);
         tc_wait_ld();
         if (valid) {
           __align__(16) __half hv[32];
@@ -371,14 +437,14 @@ __global__ void __launch_bounds__(THREADS, 1) attn_prefill_kernel(
           for (int i = 0; i < 32; ++i) {
             float v = __uint_as_float(r[i]) * inv;
             if (gate) {
-              const float g = __half2float(gate[orow * D + c0 + i]);
-              v *= __fdiv_rn(1.f, 1.f + expf(-g));
+              const float gv = __half2float(gate[orow * D + c0 + i]);
+              v *= __fdiv_rn(1.f, 1.f + expf(-gv));
             }
             hv[i] = __float2half_rn(v);
           }
           uint4* o = reinterpret_cast<uint4*>(out + orow * D + c0);
 #pragma unroll
-          for (int q = 0; q < 4; ++q) o[q] = reinterpret_cast<const uint4*>(hv)[q];
+          for (int i = 0; i < 4; ++i) o[i] = reinterpret_cast<const uint4*>(hv)[i];
         }
       }
     }
@@ -414,8 +480,8 @@ int launch(const __half* q, const __half* gate, const Chunk* chunks, int n_chunk
                                          cudaFuncAttributeMaxDynamicSharedMemorySize, L::TOTAL);
     if (e != cudaSuccess) return static_cast<int>(e);
   }
-  dim3 grid((max_q_len + P - 1) / P, kvh, n_chunks);
-  attn_prefill_kernel<D><<<grid, THREADS, L::TOTAL, stream>>>(
+  dim3 grid((max_q_len + L::NQ * P - 1) / (L::NQ * P), kvh, n_chunks);
+  attn_prefill_kernel<D><<<grid, L::THREADS, L::TOTAL, stream>>>(
       tq, chunks, page_table, max_pages, kc, vc, ks, vs, gate, out, qh, kvh, rep, num_pages,
       runtime_status_ptr());
   return static_cast<int>(cudaGetLastError());

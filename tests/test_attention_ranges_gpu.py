@@ -74,3 +74,50 @@ def test_attention_rows_at_block_edges(dev, qh, kvh, d, splits, wide):
         # a few 2^-22 of the largest value
         lim = ref.abs() * 2.0 ** -11 + 2.0 ** -18 * ref.abs().max() + 2.0 ** -25
         assert bool(((out[i].double() - ref).abs() <= lim).all()), (n, float((out[i] - ref).abs().max()))
+
+
+@pytest.mark.parametrize("qh,kvh,d,gated", [(2, 2, 64, False), (8, 1, 64, False), (3, 3, 128, False),
+                                            (8, 2, 128, True), (10, 2, 128, False),
+                                            (16, 1, 128, False), (8, 1, 256, True),
+                                            (4, 4, 256, False)])
+@pytest.mark.parametrize("spec", [[(1, 0)], [(63, 0), (65, 64), (1, 200)], [(129, 127), (257, 5)],
+                                  [(400, 1000)]])
+def test_attention_prefill_at_tile_edges(dev, qh, kvh, d, gated, spec):
+    """Chunks that end inside the first or second query tile of a CTA, pages cut by the first
+    position, against the 64-bit statement."""
+    from orinfer_b200.ops import functional as F
+    g = torch.Generator().manual_seed(qh * d + spec[0][0])
+    width = max((n + p + 127) // 128 for n, p in spec)
+    need = sum((n + p + 127) // 128 for n, p in spec)
+    table = torch.zeros(len(spec), width, dtype=torch.int32)
+    at = 1
+    for i, (n, p) in enumerate(spec):
+        for j in range((n + p + 127) // 128):
+            table[i, j] = at
+            at += 1
+    kc = torch.randint(-127, 128, (need + 1, 128, kvh, d), generator=g, dtype=torch.int8).to(dev)
+    vc = torch.randint(-127, 128, (need + 1, 128, kvh, d), generator=g, dtype=torch.int8).to(dev)
+    ks = (torch.rand(need + 1, 128, kvh, d // 64, generator=g) * 0.02 + 1e-3).half().to(dev)
+    vs = (torch.rand(need + 1, 128, kvh, d // 64, generator=g) * 0.02 + 1e-3).half().to(dev)
+    rows = sum(n for n, _ in spec)
+    q = torch.randn(rows, qh, d, generator=g).half().to(dev)
+    gate = torch.randn(rows, qh, d, generator=g).half().to(dev) if gated else None
+    chunks, first = [], 0
+    for i, (n, p) in enumerate(spec):
+        chunks.append([first, n, p, i])
+        first += n
+    out = torch.full((rows, qh * d), float("nan"), dtype=torch.float16, device=dev)
+    assert F.attention_prefill(q, gate, torch.tensor(chunks, dtype=torch.int32, device=dev),
+                               max(n for n, _ in spec), table.to(dev), kc, vc, ks, vs, out=out)
+    for i, (n, p) in enumerate(spec):
+        pg = table[i, :(n + p + 127) // 128].long().to(dev)
+        flat = lambda c: c[pg].reshape(-1, *c.shape[2:])
+        for r in sorted({0, 1, n // 2, n - 2, n - 1} & set(range(n))):
+            seen = p + r + 1
+            ref = _attention64(q[chunks[i][0] + r], flat(kc)[:seen], flat(vc)[:seen],
+                               flat(ks)[:seen], flat(vs)[:seen],
+                               None if gate is None else gate[chunks[i][0] + r]).reshape(-1)
+            got = out[chunks[i][0] + r].double()
+            # FP16 keys, values and weights (2^-11 each, scores up to about 20): 2^-8 of the
+            # largest value
+            assert float((got - ref).abs().max()) <= 2.0 ** -8 * float(ref.abs().max()), (n, p, r)
