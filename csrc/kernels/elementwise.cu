@@ -96,7 +96,7 @@ __global__ void __launch_bounds__(512) act_prep_kernel(
 #pragma unroll
       for (int j = 0; j < 8; ++j) {
         const float gv = __half2float(gh[j]);
-        const float sg = __fdiv_rn(1.f, 1.f + expf(-gv));
+        const float sg = sigmoid_f32(gv);
         rowbuf[i + j] = round_f16(__fmul_rn(__fmul_rn(gv, sg), __half2float(uh[j])));
       }
     }
@@ -253,94 +253,141 @@ __global__ void __launch_bounds__(512) act_prep_kernel(
   if (CL > 1) cg::this_cluster().sync();
 }
 
-// One warp per row, the whole row in registers (K = 128 * NBLK <= 5120): no block barrier and
-// no shared memory, only shuffles.  Serves the plain forms (x and / or residual, optional
-// RMSNorm, optional rotation) of packets with many rows; same helpers and the same order of
-// operations as the CTA-per-row kernel, so a row gives the same bits through either.
-template <int NBLK>
-__global__ void __launch_bounds__(128) act_prep_warp_kernel(
+// Plain forms (x and / or residual, optional RMSNorm, optional rotation, or SwiGLU; no peers):
+// one CTA per row, the row in registers, warp w holding 128-channel blocks w, w + W, ... with
+// four channels per lane.  Every load of a row is in flight at once, a block's sums and its
+// rotation are shuffles inside one warp, and the CTA meets twice (block sums, row maximum)
+// instead of at every phase; the first form kept the row in shared memory and spent its time
+// between barriers.  Same helpers and the same order of operations as act_prep_kernel, so a row
+// gives the same bits through either.  Few rows take many warps each (latency), thousands of
+// rows four blocks per warp (instructions per row).  512 rows x 2560 9.0 -> 6.1 us, SwiGLU 512 x
+// 9728 18.6 -> 13.1, eight rows 6.5 -> 3.1 (a cluster of eight CTAs per row before), 16384 rows x
+// 768 SwiGLU 51 -> 27.5, 2048 rows x 2048 20.5 -> 15.8 (a warp per row before).
+template <bool SWIGLU, int NB>
+__global__ void __launch_bounds__(NB <= 4 ? 1024 : 512) act_prep_regs_kernel(
     const __half* __restrict__ x, float* __restrict__ resid, const __half* __restrict__ norm_w,
     const int8_t* __restrict__ signs, int8_t* __restrict__ q_out, float* __restrict__ scale_out,
-    __half* __restrict__ y_out, int rows, float eps, int zero_centered) {
-  constexpr int K = NBLK * 128;
-  const int lane = threadIdx.x & 31;
-  const int row = blockIdx.x * 4 + (threadIdx.x >> 5);
-  if (row >= rows) return;
-  float v[NBLK][4];
-  const __half* xr = x ? x + static_cast<size_t>(row) * K : nullptr;
-  float* rr = resid ? resid + static_cast<size_t>(row) * K : nullptr;
+    __half* __restrict__ y_out, int nblk, float eps, int zero_centered,
+    const int* __restrict__ row_limit) {
+  const int row = blockIdx.x, warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int W = blockDim.x >> 5, K = nblk * 128;
+  if (row_limit != nullptr && row >= *row_limit) return;
+  __shared__ float blk_sum[MAX_NORM_BLOCKS];
+  __shared__ float red[32];
+  float v[NB][4];
+  if (SWIGLU) {
+    const __half* g = x + static_cast<size_t>(row) * 2 * K + lane * 4;
+    uint2 gr[NB], ur[NB];
 #pragma unroll
-  for (int b = 0; b < NBLK; ++b) {
-    const int i = b * 128 + lane * 4;
-    if (xr) {
-      const uint2 raw = *reinterpret_cast<const uint2*>(xr + i);
-      const __half* h = reinterpret_cast<const __half*>(&raw);
-#pragma unroll
-      for (int j = 0; j < 4; ++j) v[b][j] = __half2float(h[j]);
-    } else {
-#pragma unroll
-      for (int j = 0; j < 4; ++j) v[b][j] = 0.f;
+    for (int i = 0; i < NB; ++i) {
+      const int b = i * W + warp;
+      if (b < nblk) {
+        gr[i] = *reinterpret_cast<const uint2*>(g + b * 128);
+        ur[i] = *reinterpret_cast<const uint2*>(g + K + b * 128);
+      }
     }
-    if (rr) {
-      const float4 r = *reinterpret_cast<const float4*>(rr + i);
-      v[b][0] += r.x; v[b][1] += r.y; v[b][2] += r.z; v[b][3] += r.w;
-      *reinterpret_cast<float4*>(rr + i) = make_float4(v[b][0], v[b][1], v[b][2], v[b][3]);
-    }
-  }
-  if (norm_w) {
-    float total = 0.f;
 #pragma unroll
-    for (int b = 0; b < NBLK; ++b)
-      total = __fadd_rn(total, block128_sumsq_regs(v[b][0], v[b][1], v[b][2], v[b][3]));
-    const float r = rsqrtf(total / static_cast<float>(K) + eps);
-    const float add = zero_centered ? 1.f : 0.f;
+    for (int i = 0; i < NB; ++i) {
+      if (i * W + warp >= nblk) break;
+      const __half* gh = reinterpret_cast<const __half*>(&gr[i]);
+      const __half* uh = reinterpret_cast<const __half*>(&ur[i]);
 #pragma unroll
-    for (int b = 0; b < NBLK; ++b) {
-      const uint2 raw = *reinterpret_cast<const uint2*>(norm_w + b * 128 + lane * 4);
-      const __half* wh = reinterpret_cast<const __half*>(&raw);
-#pragma unroll
-      for (int j = 0; j < 4; ++j)
-        v[b][j] = round_f16(__fmul_rn(__fmul_rn(v[b][j], r), __half2float(wh[j]) + add));
+      for (int j = 0; j < 4; ++j) {
+        const float gv = __half2float(gh[j]);
+        const float sg = sigmoid_f32(gv);
+        v[i][j] = round_f16(__fmul_rn(__fmul_rn(gv, sg), __half2float(uh[j])));
+      }
     }
   } else {
+    const __half* xr = x ? x + static_cast<size_t>(row) * K + lane * 4 : nullptr;
+    float* rr = resid ? resid + static_cast<size_t>(row) * K + lane * 4 : nullptr;
+    uint2 wr[NB];
 #pragma unroll
-    for (int b = 0; b < NBLK; ++b)
+    for (int i = 0; i < NB; ++i) {
+      const int b = i * W + warp;
+      if (b >= nblk) break;
 #pragma unroll
-      for (int j = 0; j < 4; ++j) v[b][j] = round_f16(v[b][j]);
-  }
-  if (y_out) {
-    __half* yr = y_out + static_cast<size_t>(row) * K;
+      for (int j = 0; j < 4; ++j) v[i][j] = 0.f;
+      if (xr) {
+        const uint2 raw = *reinterpret_cast<const uint2*>(xr + b * 128);
+        const __half* h = reinterpret_cast<const __half*>(&raw);
 #pragma unroll
-    for (int b = 0; b < NBLK; ++b) {
-      __align__(8) __half h[4];
+        for (int j = 0; j < 4; ++j) v[i][j] = __half2float(h[j]);
+      }
+      if (rr) {
+        const float4 r = *reinterpret_cast<const float4*>(rr + b * 128);
+        v[i][0] += r.x; v[i][1] += r.y; v[i][2] += r.z; v[i][3] += r.w;
+        *reinterpret_cast<float4*>(rr + b * 128) =
+            make_float4(v[i][0], v[i][1], v[i][2], v[i][3]);
+      }
+      if (norm_w) wr[i] = *reinterpret_cast<const uint2*>(norm_w + b * 128 + lane * 4);
+    }
+    if (norm_w) {
 #pragma unroll
-      for (int j = 0; j < 4; ++j) h[j] = __float2half_rn(v[b][j]);
-      *reinterpret_cast<uint2*>(yr + b * 128 + lane * 4) = *reinterpret_cast<const uint2*>(h);
+      for (int i = 0; i < NB; ++i) {
+        if (i * W + warp >= nblk) break;
+        const float sq = block128_sumsq_regs(v[i][0], v[i][1], v[i][2], v[i][3]);
+        if (lane == 0) blk_sum[i * W + warp] = sq;
+      }
+      __syncthreads();
+      float total = 0.f;
+      for (int b = 0; b < nblk; ++b) total = __fadd_rn(total, blk_sum[b]);
+      const float r = rsqrtf(total / static_cast<float>(K) + eps);
+      const float add = zero_centered ? 1.f : 0.f;
+#pragma unroll
+      for (int i = 0; i < NB; ++i) {
+        if (i * W + warp >= nblk) break;
+        const __half* wh = reinterpret_cast<const __half*>(&wr[i]);
+#pragma unroll
+        for (int j = 0; j < 4; ++j)
+          v[i][j] = round_f16(__fmul_rn(__fmul_rn(v[i][j], r), __half2float(wh[j]) + add));
+      }
+    } else {
+#pragma unroll
+      for (int i = 0; i < NB; ++i) {
+        if (i * W + warp >= nblk) break;
+#pragma unroll
+        for (int j = 0; j < 4; ++j) v[i][j] = round_f16(v[i][j]);
+      }
     }
   }
   float amax = 0.f;
 #pragma unroll
-  for (int b = 0; b < NBLK; ++b) {
+  for (int i = 0; i < NB; ++i) {
+    const int b = i * W + warp;
+    if (b >= nblk) break;
+    if (y_out) {
+      __align__(8) __half h[4];
+#pragma unroll
+      for (int j = 0; j < 4; ++j) h[j] = __float2half_rn(v[i][j]);
+      *reinterpret_cast<uint2*>(y_out + static_cast<size_t>(row) * K + b * 128 + lane * 4) =
+          *reinterpret_cast<const uint2*>(h);
+    }
     if (signs) {
       const char4 sg = *reinterpret_cast<const char4*>(signs + b * 128 + lane * 4);
-      amax = fmaxf(amax, hadamard128_regs(v[b][0], v[b][1], v[b][2], v[b][3], sg, lane));
+      amax = fmaxf(amax, hadamard128_regs(v[i][0], v[i][1], v[i][2], v[i][3], sg, lane));
     } else {
-      amax = fmaxf(amax, fmaxf(fmaxf(fabsf(v[b][0]), fabsf(v[b][1])),
-                               fmaxf(fabsf(v[b][2]), fabsf(v[b][3]))));
+      amax = fmaxf(amax, fmaxf(fmaxf(fabsf(v[i][0]), fabsf(v[i][1])),
+                               fmaxf(fabsf(v[i][2]), fabsf(v[i][3]))));
     }
   }
   amax = warp_max(amax);
+  if (lane == 0) red[warp] = amax;
+  __syncthreads();
+  amax = warp_max(lane < W ? red[lane] : 0.f);
   const float scale = a8_scale(amax);
-  if (lane == 0) scale_out[row] = scale;
-  int8_t* qr = q_out + static_cast<size_t>(row) * K;
+  if (threadIdx.x == 0) scale_out[row] = scale;
+  int8_t* qr = q_out + static_cast<size_t>(row) * K + lane * 4;
 #pragma unroll
-  for (int b = 0; b < NBLK; ++b) {
+  for (int i = 0; i < NB; ++i) {
+    const int b = i * W + warp;
+    if (b >= nblk) break;
     char4 c;
-    c.x = static_cast<signed char>(a8_code(v[b][0], scale));
-    c.y = static_cast<signed char>(a8_code(v[b][1], scale));
-    c.z = static_cast<signed char>(a8_code(v[b][2], scale));
-    c.w = static_cast<signed char>(a8_code(v[b][3], scale));
-    *reinterpret_cast<char4*>(qr + b * 128 + lane * 4) = c;
+    c.x = static_cast<signed char>(a8_code(v[i][0], scale));
+    c.y = static_cast<signed char>(a8_code(v[i][1], scale));
+    c.z = static_cast<signed char>(a8_code(v[i][2], scale));
+    c.w = static_cast<signed char>(a8_code(v[i][3], scale));
+    *reinterpret_cast<char4*>(qr + b * 128) = c;
   }
 }
 
@@ -629,11 +676,32 @@ static int act_prep_launch(const __half* x, float* resid, const __half* norm_w, 
                          200 * 1024);
   }
   if (smem > 200 * 1024) return -1;
-  // A few rows (decode steps): one row would keep a single SM busy, so a cluster of CTAs
-  // shares each row.  Not for the sequence-parallel and count-limited forms, whose CTAs may
-  // leave early.
+  if (ag.tp == 0 && in.inbox == nullptr && in.ll == nullptr && row_base == 0 &&
+      q_out != nullptr && scale_out != nullptr && K / 128 <= 16 * 16) {
+    const int nblk = K / 128;
+    const int aim = rows >= 2048 ? 4 : (rows >= 256 ? 2 : 1);        // blocks per warp
+    const int most = rows <= 148 ? 32 : 16;                          // warps per row
+    int warps = (nblk + aim - 1) / aim;
+    warps = warps > most ? most : warps;
+    int nb = (nblk + warps - 1) / warps;
+    if (nb > 4 && warps > 16) nb = (nblk + 15) / 16;                 // register limit
+    warps = (nblk + nb - 1) / nb;
+#define REG_ROWS(NBV)                                                                           \
+  if (nb <= NBV) {                                                                              \
+    auto kernel = swiglu ? act_prep_regs_kernel<true, NBV> : act_prep_regs_kernel<false, NBV>;  \
+    kernel<<<rows, warps * 32, 0, stream>>>(x, resid, norm_w, signs, q_out, scale_out, y_out,   \
+                                            nblk, eps, zero_centered, row_limit);               \
+    return static_cast<int>(cudaGetLastError());                                                \
+  }
+    REG_ROWS(1) REG_ROWS(2) REG_ROWS(3) REG_ROWS(4) REG_ROWS(5) REG_ROWS(6) REG_ROWS(8)
+    REG_ROWS(12) REG_ROWS(16)
+#undef REG_ROWS
+  }
+  // Inbox forms of a few rows (decode steps under tensor parallelism): one row would keep a
+  // single SM busy, so a cluster of CTAs shares each row.  Not for the sequence-parallel and
+  // count-limited forms, whose CTAs may leave early.
   constexpr int CL = 8;
-  if (rows <= 16 && ag.tp == 0 && row_limit == nullptr && K / 128 >= CL) {
+  if (rows <= 16 && ag.tp == 0 && row_limit == nullptr && K / 128 >= CL && !swiglu) {
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3(rows * CL);
     cfg.blockDim = dim3(256);
@@ -648,34 +716,11 @@ static int act_prep_launch(const __half* x, float* resid, const __half* norm_w, 
     cfg.numAttrs = 1;
     const AgOut no_ag{};
     const int* no_limit = nullptr;
-    cudaError_t e;
-    if (swiglu) {
-      float* no_resid = nullptr;
-      const __half* no_norm = nullptr;
-      e = cudaLaunchKernelEx(&cfg, act_prep_kernel<true, CL>, x, no_resid, no_norm, signs, q_out,
-                             scale_out, y_out, K, eps, zero_centered, in, status, no_ag, rows,
-                             no_limit, 0);
-    } else {
-      e = cudaLaunchKernelEx(&cfg, act_prep_kernel<false, CL>, x, resid, norm_w, signs, q_out,
-                             scale_out, y_out, K, eps, zero_centered, in, status, no_ag, rows,
-                             no_limit, row_base);
-    }
+    const cudaError_t e =
+        cudaLaunchKernelEx(&cfg, act_prep_kernel<false, CL>, x, resid, norm_w, signs, q_out,
+                           scale_out, y_out, K, eps, zero_centered, in, status, no_ag, rows,
+                           no_limit, row_base);
     return static_cast<int>(e != cudaSuccess ? e : cudaGetLastError());
-  }
-  // Thousands of plain rows of moderate width: one warp per row, the row in registers.  With
-  // fewer rows there are too few warps in flight to hide the latency of a row's loads, and
-  // the CTA-per-row kernel below is more than twice as fast (512 rows of 2560: 11 us
-  // against 27 us).
-  if (!swiglu && rows >= 2048 && ag.tp == 0 && row_limit == nullptr && in.inbox == nullptr &&
-      in.ll == nullptr && row_base == 0 && q_out != nullptr && scale_out != nullptr) {
-#define WARP_ROWS(NB)                                                                         \
-  if (K == NB * 128) {                                                                        \
-    act_prep_warp_kernel<NB><<<(rows + 3) / 4, 128, 0, stream>>>(                             \
-        x, resid, norm_w, signs, q_out, scale_out, y_out, rows, eps, zero_centered);          \
-    return static_cast<int>(cudaGetLastError());                                              \
-  }
-    WARP_ROWS(2) WARP_ROWS(8) WARP_ROWS(16) WARP_ROWS(20) WARP_ROWS(32) WARP_ROWS(40)
-#undef WARP_ROWS
   }
   // SwiGLU rows are wide and spend their time in exp / divide: more threads per row
   const int threads = swiglu && K >= 4096 ? 512 : 256;

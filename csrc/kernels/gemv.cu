@@ -172,7 +172,7 @@ __global__ void __launch_bounds__(GemvThreads<MT>::value, 1) e8p_gemv_kernel(
 #pragma unroll
           for (int j = 0; j < 8; ++j) {
             const float gv = __half2float(gh[j]);
-            const float sg = __fdiv_rn(1.f, 1.f + expf(-gv));
+            const float sg = sigmoid_f32(gv);
             fb[i + j] = round_f16(__fmul_rn(__fmul_rn(gv, sg), __half2float(uh[j])));
           }
         }
