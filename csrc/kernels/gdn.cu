@@ -76,7 +76,7 @@ __global__ void __launch_bounds__(D) gdn_conv_kernel(
     }
     acc = fmaf(v, __half2float(wc[j]), acc);
   }
-  float val = round_f16(acc * __fdiv_rn(1.f, 1.f + expf(-acc)));
+  float val = round_f16(acc * sigmoid_f32(acc));
   if (head < qk_heads) {
     __shared__ float red[D / 32];
     float ss = warp_sum(val * val);
@@ -94,7 +94,7 @@ __global__ void __launch_bounds__(D) gdn_conv_kernel(
 // rows: the three earlier rows stay in registers, so a packet's rows are read once instead of
 // four times two bytes at a time.  A head is D / 8 neighbouring lanes.  Grid (row strips,
 // conv_dim / 2048); R = 1 for decode-sized packets, where the strips would be too few CTAs.
-// 2100 rows x 8192 channels: 89 -> 35 us; 64 rows: 7.9 -> 5.6 us.  What is left is the SiLU.
+// 2100 rows x 8192 channels: 89 -> 25 us; 64 rows: 7.9 -> 5.0 us.
 template <int D, int R>
 __global__ void __launch_bounds__(256) gdn_conv_vec_kernel(
     const __half* __restrict__ x, int x_stride, const __half* __restrict__ weight,
@@ -148,7 +148,7 @@ __global__ void __launch_bounds__(256) gdn_conv_vec_kernel(
       for (int j = 0; j < 4; ++j)
         acc = fmaf(__half2float(reinterpret_cast<const __half*>(j < 3 ? &tap[j] : &win[3])[e]),
                    __half2float(wh[e * 4 + j]), acc);
-      val[e] = round_f16(acc * __fdiv_rn(1.f, 1.f + expf(-acc)));
+      val[e] = round_f16(acc * sigmoid_f32(acc));
       ss = fmaf(val[e], val[e], ss);
     }
     if (c < qk_channels) {
@@ -277,7 +277,7 @@ __global__ void __launch_bounds__(256) gdn_scan_kernel(
     const float xg = a + bias;
     const float softplus = xg > 20.f ? xg : log1pf(expf(xg));
     const float decay = expf(-alog * softplus);
-    const float beta = __fdiv_rn(1.f, 1.f + expf(-b));
+    const float beta = __frcp_rn(1.f + expf(-b));
     part[part_id][threadIdx.x % DC] = ((p0 + p1) + (p2 + p3)) * decay;
     __syncthreads();
     float full = 0.f;
@@ -394,7 +394,7 @@ __global__ void __launch_bounds__(256) gdn_scan_split_kernel(
       const float xg = n_a + bias;
       const float softplus = xg > 20.f ? xg : log1pf(expf(xg));
       dec_s[buf][threadIdx.x] = expf(-alog * softplus);
-      beta_s[buf][threadIdx.x] = __fdiv_rn(1.f, 1.f + expf(-n_b));
+      beta_s[buf][threadIdx.x] = __frcp_rn(1.f + expf(-n_b));
     }
     asm volatile("cp.async.wait_group 0;" ::: "memory");
     __syncthreads();                  // block b staged; everyone has left block b-1
@@ -491,10 +491,12 @@ __global__ void __launch_bounds__(256) gdn_scan_split_kernel(
 //
 // Precision: k, q and v are FP16 and enter products exactly; FP32 operands are split in two
 // (FP16 halves under a power-of-two scale: 22 bits; TF32 pairs: 22 bits) and all sums are FP32.
-// The G are summed in FP64 so that e^(G_i - G_j) keeps FP32 accuracy when |G| is large.
+// The G are summed in FP64 and subtracted as FP32 pairs, so that e^(G_i - G_j) keeps FP32 accuracy
+// when |G| is large.
 //
 // 32 heads of 128 channels, two runs of 1050 rows: 610 us as a scan (0.29 us per dependent step),
-// 227 us here.  Runs below GDN_LONG_ROWS keep the scan: two chunks cost about as much as 64 steps,
+// 185 us here: 75 us of staging and barriers, 63 of the state warps and 65 of the helpers, which
+// add up more than they overlap.  Runs below GDN_LONG_ROWS keep the scan: two chunks cost about as much as 64 steps,
 // and verification packets (at most 32 rows) must reproduce the scan's bits.
 constexpr int GDN_LONG_ROWS = 64;
 constexpr int CHUNK = 32, CHUNK_THREADS = 192;
@@ -503,7 +505,6 @@ struct ChunkSmem {
   __half v[3][CHUNK][72];
   float t[2][CHUNK][40], p[2][CHUNK][40];      // T and P, row i, column j
   float at[CHUNK][36];                         // A transposed: [j][i]
-  double g[2][CHUNK];                          // G, one copy per helper warp
   float eg[2][CHUNK], beta[2][CHUNK], tail[2][CHUNK], total[2];
 };
 
@@ -639,7 +640,7 @@ __global__ void __launch_bounds__(CHUNK_THREADS, 2) gdn_chunk_kernel(
     const float xg = n_a + bias;
     const float softplus = xg > 20.f ? xg : log1pf(expf(xg));
     double big_g = live ? static_cast<double>(-alog * softplus) : 0.0;
-    const float beta = live ? __fdiv_rn(1.f, 1.f + expf(-n_b)) : 0.f;
+    const float beta = live ? __frcp_rn(1.f + expf(-n_b)) : 0.f;
     if (c + 1 < chunks) fetch_gates(c + 1);
 #pragma unroll
     for (int o = 1; o < 32; o <<= 1) {
@@ -647,14 +648,29 @@ __global__ void __launch_bounds__(CHUNK_THREADS, 2) gdn_chunk_kernel(
       if (lane >= o) big_g += up;
     }
     const double last = __shfl_sync(0xffffffffu, big_g, 31);
-    sm.g[helper][lane] = big_g;
     if (helper == 0) {
       sm.eg[buf][lane] = expf(static_cast<float>(big_g));
       sm.beta[buf][lane] = beta;
       sm.tail[buf][lane] = expf(static_cast<float>(last - big_g));
       if (lane == 0) sm.total[buf] = expf(static_cast<float>(last));
     }
-    __syncwarp();
+    // G as an FP32 pair: differences of the heads round in proportion to themselves, and the
+    // remainders restore what the heads lost
+    const float g_hi = static_cast<float>(big_g);
+    const float g_lo = static_cast<float>(big_g - static_cast<double>(g_hi));
+    // this lane's rows g + 8 i and columns 8 i + 2 t (+ 1)
+    float rh[4], rl[4], rb[4], ch[8], cl[8];
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+      rh[i] = __shfl_sync(0xffffffffu, g_hi, g + 8 * i);
+      rl[i] = __shfl_sync(0xffffffffu, g_lo, g + 8 * i);
+      rb[i] = __shfl_sync(0xffffffffu, beta, g + 8 * i);
+#pragma unroll
+      for (int e = 0; e < 2; ++e) {
+        ch[2 * i + e] = __shfl_sync(0xffffffffu, g_hi, 8 * i + 2 * t + e);
+        cl[2 * i + e] = __shfl_sync(0xffffffffu, g_lo, 8 * i + 2 * t + e);
+      }
+    }
     // rows of X (k or q) times rows of k, the blocks on and below the diagonal:
     // acc[0..1] rows 0..15 x columns 0..15, acc[2..5] rows 16..31 x columns 0..31
     const __half(*xs)[136] = helper == 0 ? sm.k[st] : sm.q[st];
@@ -686,19 +702,26 @@ __global__ void __launch_bounds__(CHUNK_THREADS, 2) gdn_chunk_kernel(
       mma16816(acc[4], x1[0], x1[1], x1[2], x1[3], k1[0], k1[2]);
       mma16816(acc[5], x1[0], x1[1], x1[2], x1[3], k1[1], k1[3]);
     }
+    // every factor first, then the stores: nothing in between waits for shared memory
+#pragma unroll
+    for (int i = 0; i < 6; ++i) {
+#pragma unroll
+      for (int e = 0; e < 4; ++e) {
+        const int rn = (i < 2 ? 0 : 2) + (e >> 1), cn = (i < 2 ? i : i - 2) * 2 + (e & 1);
+        const float d = (rh[rn] - ch[cn]) + (rl[rn] - cl[cn]);
+        acc[i][e] *= expf(fminf(d, 0.f)) * (helper == 0 ? rb[rn] : scale);
+      }
+    }
 #pragma unroll
     for (int i = 0; i < 6; ++i) {
       const int i0 = i < 2 ? 0 : 16, j0 = i < 2 ? i * 8 : (i - 2) * 8;
 #pragma unroll
       for (int e = 0; e < 4; ++e) {
         const int ri = i0 + g + (e >> 1) * 8, cj = j0 + 2 * t + (e & 1);
-        const float d = expf(static_cast<float>(fmin(sm.g[helper][ri] - sm.g[helper][cj], 0.0)));
-        if (helper == 0) {
-          const float b = __shfl_sync(0xffffffffu, beta, ri);
-          sm.at[cj][ri] = cj < ri ? b * d * acc[i][e] : 0.f;
-        } else {
-          sm.p[buf][ri][cj] = cj <= ri ? scale * d * acc[i][e] : 0.f;
-        }
+        if (helper == 0)
+          sm.at[cj][ri] = cj < ri ? acc[i][e] : 0.f;
+        else
+          sm.p[buf][ri][cj] = cj <= ri ? acc[i][e] : 0.f;
       }
     }
     if (helper == 0) {
@@ -924,13 +947,13 @@ __global__ void __launch_bounds__(D) gdn_gated_norm_kernel(
   for (int i = 0; i < D / 32; ++i) tot += red[i];
   const float n = v * rsqrtf(tot / D + eps) * __half2float(w[d]);
   const float zf = __half2float(z[static_cast<size_t>(row) * z_stride + h * D + d]);
-  const float sg = __fdiv_rn(1.f, 1.f + expf(-zf));
+  const float sg = sigmoid_f32(zf);
   const float gate = sigmoid_gate ? sg : zf * sg;
   y[(static_cast<size_t>(row) * hv + h) * D + d] = __float2half_rn(n * gate);
 }
 
 // The same, one warp per (row, head): D / 32 neighbouring channels per lane, eight heads per
-// CTA, no block barrier.  2100 rows x 32 heads of 128: 37 -> 17 us (69 MB).
+// CTA, no block barrier.  2100 rows x 32 heads of 128: 37 -> 13 us (69 MB).
 template <int D>
 __global__ void __launch_bounds__(256) gdn_gated_norm_warp_kernel(
     const float* __restrict__ o, const __half* __restrict__ z, int z_stride,
@@ -960,7 +983,7 @@ __global__ void __launch_bounds__(256) gdn_gated_norm_warp_kernel(
   for (int i = 0; i < V; ++i) {
     const float n = v.f[i] * r * __half2float(wh.h[i]);
     const float zf = __half2float(zh.h[i]);
-    const float sg = __fdiv_rn(1.f, 1.f + expf(-zf));
+    const float sg = sigmoid_f32(zf);
     out.h[i] = __float2half_rn(n * (sigmoid_gate ? sg : zf * sg));
   }
   *reinterpret_cast<Half*>(y + item * D + lane * V) = out;
