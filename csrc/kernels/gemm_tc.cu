@@ -27,6 +27,9 @@ namespace orinfer {
 int qgemv_dispatch(int fmt, const int8_t* a, const float* as, const void* w, const __half* ws,
                    void* out, int M, int N, int K, int out_f32, cudaStream_t stream,
                    const PeerOut* peer);
+int qgemv_grouped_dispatch(int fmt, const int8_t* a, const float* as, const void* w,
+                           const __half* ws, void* out, int N, int K, long long bank,
+                           const int* tiles, const int* meta, cudaStream_t stream);
 
 namespace tc {
 
@@ -61,7 +64,12 @@ struct Layout {
   static constexpr int SA_FIT = (BUDGET - SB * BC_BYTES) / A_BYTES;
   static constexpr int SA = SA_FIT >= 4 ? 4 : SA_FIT;
   static_assert(SA >= 2 && SB >= 2, "at least double buffering");
-  static constexpr int LUT_COPIES = 4;
+  // as many copies of the decode tables as the rings leave room for: the lookups of a warp are
+  // random and collide about 3-fold with 4 copies, 1.5-fold with 16
+  static constexpr int RINGS = SA * A_BYTES + SB * BC_BYTES;
+  static constexpr int LUT_COPIES = RINGS + 32 * 1024 + 1280 <= 227 * 1024
+                                        ? 16
+                                        : (RINGS + 16 * 1024 + 1280 <= 227 * 1024 ? 8 : 4);
   static constexpr int LUT_BYTES = FMT == 0 ? 0 : static_cast<int>(sizeof(E8pLut<LUT_COPIES>));
   static constexpr int A_OFF = 0;
   static constexpr int B_OFF = A_OFF + SA * A_BYTES;
@@ -116,12 +124,21 @@ __global__ void __launch_bounds__(THREADS, 1) qgemm_tc_kernel(
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int n0 = n_begin + blockIdx.x * BN;    // this launch covers columns [n_begin, n_end)
-  int m0 = blockIdx.y * BM * MT, m_limit = M, b_row0 = n0;
+  int m0 = blockIdx.y * BM * MT, m_limit = M, b_row0 = n0, mt_act = MT;
   if (grp.tiles != nullptr) {
-    if (static_cast<int>(blockIdx.y) >= grp.meta[0]) return;
-    const int expert = grp.tiles[blockIdx.y * 4];
-    m0 = grp.tiles[blockIdx.y * 4 + 1];
-    m_limit = m0 + grp.tiles[blockIdx.y * 4 + 2];
+    // MT neighbouring 128-row tiles of one expert go to one CTA (the fourth word counts an
+    // expert's tiles), so its weights are decoded once for all of them
+    const int tiles = grp.meta[0], tile = static_cast<int>(blockIdx.y);
+    if (tile >= tiles) return;
+    const int* entry = grp.tiles + tile * 4;
+    const int expert = entry[0];
+    if (MT > 1 && entry[3] % MT != 0) return;
+    m0 = entry[1];
+    m_limit = m0 + entry[2];
+#pragma unroll
+    for (int i = 1; i < MT; ++i)
+      if (tile + i < tiles && entry[i * 4] == expert) m_limit += entry[i * 4 + 2];
+    mt_act = (m_limit - m0 + BM - 1) / BM;          // row tiles that hold rows (and are loaded)
     w += static_cast<long long>(expert) * grp.w_stride;
     w_scale += static_cast<long long>(expert) * grp.n_per_expert;
     b_row0 = expert * grp.n_per_expert + n0;
@@ -184,10 +201,10 @@ __global__ void __launch_bounds__(THREADS, 1) qgemm_tc_kernel(
         if (probe & 2) {
           mbar_arrive(&a_full[s]);
         } else {
-          mbar_expect_tx(&a_full[s], MT * TILE_BYTES);
+          mbar_expect_tx(&a_full[s], mt_act * TILE_BYTES);
 #pragma unroll
           for (int t = 0; t < MT; ++t)
-            tma_load_2d(a_s + (s * MT + t) * TILE_BYTES, &tmap_a, &a_full[s], (kb0 + kb) * BK,
+            if (t < mt_act) tma_load_2d(a_s + (s * MT + t) * TILE_BYTES, &tmap_a, &a_full[s], (kb0 + kb) * BK,
                         m0 + t * BM);
         }
         issued = kb + 1;
@@ -1567,7 +1584,8 @@ inline int plan_splits(int M, int N, int K, int out_f32) {
 // (crates/orinfer-model-sdk/src/operators/rows.rs:10-60) and of its offline projection tuner
 // (python/orinfer_build/tuning/).
 struct Plan {
-  int mt, nb, splits, tail_splits;   // tail_splits > 0: peel ntiles % 148 weight tiles
+  int mt, nb, splits, tail_splits;   // tail_splits > 0: peel the last tail_tiles weight tiles
+  int tail_tiles;
 };
 
 struct Variant {
@@ -1588,6 +1606,15 @@ inline bool variant_valid(const Variant& v) {
       static_cast<size_t>(v.splits) * padded_cells(v.m_hi, v.n) * 4 > SPLITK_WORKSPACE_BYTES)
     return false;
   return true;
+}
+
+// K splits of the tail launch (128-row tiles): fill the machine once, keep at least four
+// k-blocks per split.
+inline int tail_splits_for(int M, int K, int tail_tiles) {
+  const long ctas = static_cast<long>(tail_tiles) * ((M + BM - 1) / BM);
+  long ts = 148 / (ctas > 0 ? ctas : 1);
+  ts = ts > K / BK / 4 ? K / BK / 4 : ts;
+  return static_cast<int>(ts > 8 ? 8 : (ts < 1 ? 1 : ts));
 }
 
 inline Plan make_plan(int fmt, int M, int N, int K, int out_f32, bool fused) {
@@ -1638,25 +1665,18 @@ inline Plan make_plan(int fmt, int M, int N, int K, int out_f32, bool fused) {
   // and the weight decode work for no gain: 128-wide tiles won every such case measured.
   p.nb = (out_f32 || p.splits > 1 || c128 >= 120 || (p.mt == 4 && mtiles >= 4)) ? 128
                                                                  : (ctas(64) >= 120 ? 64 : 32);
-  // Wave quantisation: a grid of one M tile that is a few CTAs larger than the machine would
-  // run a second, almost empty wave.  The full wave runs as one launch; the last few weight
-  // tiles follow as a split-K launch of their own, which occupies the SMs the tail left idle.
-  if (!out_f32 && p.splits == 1 && p.nb == 128 && mtiles == 1 && !fused && ntiles > 148 &&
-      ntiles % 148 > 0 && ntiles % 148 <= 40 && K / BK >= 8 && N % 128 == 0) {
-    int ts = static_cast<int>(148 / (ntiles % 148));
-    ts = ts > K / BK / 4 ? K / BK / 4 : ts;
-    p.tail_splits = ts > 8 ? 8 : (ts < 1 ? 1 : ts);
+  // Wave quantisation: a grid a few CTAs larger than a whole number of waves would run one more,
+  // almost empty wave.  The full waves run as one launch; the last few weight tiles follow as a
+  // launch of 128-row tiles split along K, which occupies the SMs the tail left idle.  Measured
+  // at K = 2560, N = 19456: M = 512 (152 CTAs) 61 -> 44 us, M = 2048 (608 CTAs) 138 -> 128 us.
+  const long total = mtiles * ntiles;
+  if (!out_f32 && p.splits == 1 && p.nb == 128 && !fused && total > 148 && total % 148 > 0 &&
+      total % 148 <= 40 && K / BK >= 8 && N % 128 == 0) {
+    const long keep = total / 148 * 148 / mtiles;       // weight tiles of the full waves
+    p.tail_tiles = static_cast<int>(ntiles - keep);
+    p.tail_splits = tail_splits_for(M, K, p.tail_tiles);
   }
   return p;
-}
-
-// K splits of the tail launch (128-row tiles): fill the machine once, keep at least four
-// k-blocks per split.
-inline int tail_splits_for(int M, int K, int tail_tiles) {
-  const long ctas = static_cast<long>(tail_tiles) * ((M + BM - 1) / BM);
-  long ts = 148 / (ctas > 0 ? ctas : 1);
-  ts = ts > K / BK / 4 ? K / BK / 4 : ts;
-  return static_cast<int>(ts > 8 ? 8 : (ts < 1 ? 1 : ts));
 }
 
 template <int FMT>
@@ -1672,11 +1692,10 @@ int launch_fmt(const int8_t* a, const float* a_scale, const void* w, const __hal
   const int mt = plan.mt, nb = plan.nb, splits = plan.splits;
   if (plan.tail_splits > 0) {
     const long ntiles = (N + 127) / 128;
-    const int tail_tiles = static_cast<int>(ntiles % 148);
-    const int cut = static_cast<int>(ntiles - tail_tiles) * 128;
+    const int cut = static_cast<int>(ntiles - plan.tail_tiles) * 128;
     // the tail runs as 128-row tiles: more CTAs of less work each, and small accumulator
     // tiles whose splits are added inside the kernel
-    const int ts = tail_splits_for(M, K, tail_tiles);
+    const int ts = plan.tail_splits;
 #define ORINFER_TWO(MTV)                                                                        \
   {                                                                                             \
     const int r = launch<FMT, false, MTV, 128>(a, a_scale, w, w_scale, out, M, N, K, stream, po, \
@@ -1757,9 +1776,7 @@ extern "C" int orinfer_qgemm_launches_fmt(int fmt, int M, int N, int K, int out_
   // K splits are added up inside the one-tile kernel when the tiles are small; otherwise,
   // and in the persistent forms, a second pass adds them
   if (p.tail_splits > 0) {
-    const int ts = tc::g_impl == 1
-                       ? tc::tail_splits_for(M, K, static_cast<int>(((N + 127) / 128) % 148))
-                       : p.tail_splits;
+    const int ts = p.tail_splits;
     const bool second = ts > 1 && !(tc::g_impl == 1 && tc::splitk_in_kernel(1, 128, ts));
     return second ? 3 : 2;
   }
@@ -1855,6 +1872,12 @@ extern "C" int orinfer_qgemm_ag(int fmt, const int8_t* a, const float* a_scale, 
   return tc::launch_fmt<2>(a, a_scale, w, w_scale, out, M, N, K, out_f32, stream, po, ag);
 }
 
+// Rows per expert, on average over the experts, up to which a grouped projection runs on the
+// small-M kernel (both projections of a layer, H = 2048).  128 Q4 experts of 768: 155 against 253 us
+// at 4 rows, 198 against 256 at 8, 258 against 256 at 12; 512 Q2 experts of 512: 155 against 535 us
+// at 1.25, 213 against 602 at 2.5, 383 against 650 at 10, 681 against 650 at 20.
+inline int grouped_gemv_rows(int fmt) { return fmt == 2 ? 18 : (fmt == 1 ? 10 : 8); }
+
 // Grouped expert GEMM: rows of `a` are sorted by expert; tile t of the table covers rows
 // [first, first + valid) of expert e, multiplied with that expert's bank.  out is fp16 [S, N].
 extern "C" int orinfer_qgemm_grouped(int fmt, const int8_t* a, const float* a_scale, const void* w,
@@ -1866,14 +1889,23 @@ extern "C" int orinfer_qgemm_grouped(int fmt, const int8_t* a, const float* a_sc
   if (runtime_ensure_init() != cudaSuccess) return -2;
   const long long bank = fmt == 0 ? static_cast<long long>(N) * K
                                   : static_cast<long long>(K / 128) * N * (fmt == 1 ? 64 : 32);
+  // Few rows per expert: the tile table mostly holds tiles of one or two rows.
+  if (S <= static_cast<long long>(grouped_gemv_rows(fmt)) * experts)
+    return qgemv_grouped_dispatch(fmt, a, a_scale, w, w_scale, out, N, K, bank, tiles, meta, stream);
   tc::GroupDesc g{tiles, meta, bank, N};
-  PeerOut po{};
-  if (fmt == 0)
-    return tc::launch<0, false, 1, 128>(a, a_scale, w, w_scale, out, S, N, K, stream, po, g, experts,
-                                   max_tiles);
-  if (fmt == 1)
-    return tc::launch<1, false, 1, 128>(a, a_scale, w, w_scale, out, S, N, K, stream, po, g, experts,
-                                   max_tiles);
-  return tc::launch<2, false, 1, 128>(a, a_scale, w, w_scale, out, S, N, K, stream, po, g, experts,
-                                 max_tiles);
+  const PeerOut po{};
+  // Row tiles of one expert per CTA: two where experts have about a tile of rows (half of them
+  // then have a second, nearly empty one), four where they have several.
+  const int mt = tc::g_impl != 1 ? 1 : (S >= 256LL * experts ? 4 : (S >= 64LL * experts ? 2 : 1));
+#define ORINFER_GROUPED(FMT)                                                                       \
+  return mt == 4   ? tc::launch<FMT, false, 4, 128>(a, a_scale, w, w_scale, out, S, N, K, stream,  \
+                                                    po, g, experts, max_tiles)                     \
+         : mt == 2 ? tc::launch<FMT, false, 2, 128>(a, a_scale, w, w_scale, out, S, N, K, stream,  \
+                                                    po, g, experts, max_tiles)                     \
+                   : tc::launch<FMT, false, 1, 128>(a, a_scale, w, w_scale, out, S, N, K, stream,  \
+                                                    po, g, experts, max_tiles)
+  if (fmt == 0) ORINFER_GROUPED(0);
+  if (fmt == 1) ORINFER_GROUPED(1);
+  ORINFER_GROUPED(2);
+#undef ORINFER_GROUPED
 }

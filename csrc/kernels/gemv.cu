@@ -1,7 +1,7 @@
 // Small-M quantised GEMM (decode path, M <= 8): weight-bandwidth bound.  Each CTA
-// owns a few output rows and streams their codes once; warps split K, lanes decode
-// E8P codes through a shared-memory value table and accumulate with dp4a against
-// the INT8 activations staged in shared memory.  Replaces the reference's dp4a /
+// owns a few output rows and streams their weights once; lanes decode E8P codes through a
+// shared-memory value table and the products with the INT8 activations staged in shared
+// memory run on the tensor cores (mma.sync, 16 weight rows x 8 activation rows).  Replaces the reference's dp4a /
 // gemv projections (kernels/cuda/model/integer_core.py:275,
 // kernels/cuda/model/integer_vq.py:381 integer_e8p_gemv,
 // kernels/cuda/model/int8_projection.py:66).
@@ -11,7 +11,7 @@
 
 namespace orinfer {
 
-constexpr int GEMV_WARPS = 8;
+constexpr int W8_WARPS = 8;
 
 template <int MT>
 __device__ __forceinline__ void stage_activations(int8_t* dst, const int8_t* __restrict__ a, int M,
@@ -40,27 +40,70 @@ __device__ __forceinline__ void store_row(void* out, int out_f32, int m, int n, 
   else reinterpret_cast<__half*>(out)[static_cast<size_t>(m) * N + n] = __float2half_rn(v);
 }
 
-// FMT 1: Q4 (U32 codes, 8 output rows per group, 4 lanes per row); FMT 2: Q2 (U16 codes, 16
-// rows, 2 lanes).  One persistent CTA per SM: the decode tables (32 interleaved copies, so a
-// lane's lookups never meet another lane's on a bank) and the activations are staged once.
-// The grid is n_parts x k_parts CTAs; a CTA owns a contiguous range of row groups and one
-// range of k-blocks, its warps take contiguous runs of (group, k-block) units, every lane
-// keeps DEPTH 16-byte code loads in flight, and the partial dot products meet in shared
-// memory (integer atomics: exact, so the result does not depend on the order).
+// FMT 0: INT8 weights, 1: Q4 (U32 codes), 2: Q2 (U16 codes).  One persistent CTA per SM: the
+// decode tables (32 interleaved copies, so a lane's lookups never meet another lane's on a
+// bank) and the activations are staged once.  The grid is n_parts x k_parts CTAs; a CTA owns a
+// contiguous range of 16-row groups and one range of 128-wide k-blocks, its warps take
+// contiguous runs of (group, k-block) units, every lane keeps DEPTH units of weight loads in
+// flight (the first ones are issued before the tables are filled), and the partial dot products
+// meet in shared memory (integer atomics: exact, so the result does not depend on the order).
+//
+// Products: m16n8k32 INT8 MMAs with the weights as A (lane (g, t) holds rows g and g + 8) and
+// the activation rows as the eight columns of B.  A lane's four code words of a k-block are
+// weight octets 4t .. 4t + 3; step j multiplies octets {4t + j}, so the activations are staged
+// octet-wise as [k-block][j][t][row] and a step reads 8 bytes per lane without a bank conflict.
+// One MMA replaces 4 M dp4a and 2 M shared-memory loads: the time no longer grows with M.
 //
 // The decode never forms the weights.  With v the 4-bit fields of a code (common.cuh), a Q4
 // weight is 8*v0 + 2*v1 - 75, so
 //     sum_k a_k w_k = 2 * sum_k a_k (4*v0 + v1)_k  -  75 * sum_k a_k
-// and the first sum is one dp4a per four weights on bytes built with two masks and one
-// multiply-add; sum_k a_k is computed once per activation row while it is staged.  Q2
-// likewise with 2*v - 15.
+// and the first sum multiplies bytes built with two masks and one multiply-add; sum_k a_k is
+// computed once per activation row while it is staged.  Q2 likewise with 2*v - 15.
 //
-// k_parts > 1 (projections too narrow for one CTA per SM): the CTAs of one n-part add their
+// k_parts > 1 (E8P projections too narrow for one CTA per SM): the CTAs of one n-part add their
 // integers into a zeroed workspace; the last one to finish (ticket) applies the scales,
 // writes the outputs and zeroes what it read.  Launches that use the workspace must not
 // overlap on the device (they are issued on one stream).
 constexpr int GEMV_COPIES = 32;
-constexpr int GEMV_DEPTH = 4;
+constexpr int GEMV_THREADS = 1024;
+
+__device__ __forceinline__ void mma_i8_16832(int (&c)[4], uint32_t a0, uint32_t a1, uint32_t a2,
+                                             uint32_t a3, uint32_t b0, uint32_t b1) {
+  asm volatile(
+      "mma.sync.aligned.m16n8k32.row.col.s32.s8.s8.s32 {%0, %1, %2, %3}, {%4, %5, %6, %7}, "
+      "{%8, %9}, {%0, %1, %2, %3};"
+      : "+r"(c[0]), "+r"(c[1]), "+r"(c[2]), "+r"(c[3])
+      : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1));
+}
+
+// One or two rows of Q4 weights keep the dp4a form: an MMA spends eight columns on them, and
+// eight-row units divide more evenly over the warps (19456 x 2560, one row: 13.5 us against 14.9
+// with MMAs; from four rows on the MMAs win, 23.1 against 16.5 us at eight).  Lane l then holds
+// row l / 4 of a group of eight and a quarter of the k-block.
+template <int FMT, int MT>
+struct GemvMode {
+  static constexpr bool DP4A = FMT == 1 && MT <= 2;
+  static constexpr int ROWS = DP4A ? 8 : 16;                         // output rows of a group
+  static constexpr int DEPTH = DP4A || FMT == 2 ? 4 : 2;             // units in flight per lane
+};
+
+// Weights of one (group, k-block) unit as loaded by a lane: HALVES rows (g, and g + 8).
+template <int FMT, int HALVES = 2>
+struct GemvUnit {
+  static constexpr int WORDS = FMT == 0 ? 8 : (FMT == 1 ? 4 : 2);    // 32-bit words per row
+  uint32_t w[HALVES][WORDS];
+};
+
+// Position of channel k of activation row m in the staged activations (bytes).  dp4a: octets
+// in order, rows next to each other; E8P: octets ordered [k-block][octet % 4][octet / 4][row]; INT8 weights: 16-byte pieces ordered
+// [64 channels][row][piece], a lane's pieces being two steps each.
+template <int FMT, int MT>
+__device__ __forceinline__ int act_pos(int m, int k) {
+  if (FMT == 0) return ((k >> 6) * MT + m) * 64 + (k & 63);
+  if (GemvMode<FMT, MT>::DP4A) return ((k >> 3) * MT + m) * 8 + (k & 7);
+  const int o = (k >> 3) & 15;
+  return (((k >> 7) * 16 + (o & 3) * 4 + (o >> 2)) * MT + m) * 8 + (k & 7);
+}
 
 // Optional fusion of the decode step's row kernels into the projection (at most 8 rows, no
 // peers).  `pre` builds the INT8 activations inside every CTA instead of reading them:
@@ -86,31 +129,27 @@ struct GemvFuse {
   float* resid_accum;
 };
 
-template <int MT>
-struct GemvThreads {
-  static constexpr int value = MT <= 2 ? 1024 : 512;
-};
-
 template <int FMT, int MT>
-__global__ void __launch_bounds__(GemvThreads<MT>::value, 1) e8p_gemv_kernel(
-    const int8_t* __restrict__ a, const float* __restrict__ a_scale, const uint4* __restrict__ w,
+__global__ void __launch_bounds__(GEMV_THREADS, 1) qgemv_kernel(
+    const int8_t* __restrict__ a, const float* __restrict__ a_scale, const void* __restrict__ w,
     const __half* __restrict__ w_scale, void* __restrict__ out, int M, int N, int K, int out_f32,
     const E8pTables* __restrict__ tables, PeerOut po, int n_parts, int k_parts, int max_groups,
     int* __restrict__ ws, GemvFuse fz) {
-  constexpr int THREADS = GemvThreads<MT>::value;
-  constexpr int ROWS = FMT == 1 ? 8 : 16;
-  constexpr int LPR = 32 / ROWS;                 // lanes per row
-  constexpr int WPL = 128 / LPR;                 // weights per lane per k-block
-  constexpr int DEPTH = GEMV_DEPTH;
+  constexpr int THREADS = GEMV_THREADS;
+  using Mode = GemvMode<FMT, MT>;
+  constexpr bool DP4A = Mode::DP4A;
+  constexpr int ROWS = Mode::ROWS, HALVES = ROWS / 8, DEPTH = Mode::DEPTH;
+  using Unit = GemvUnit<FMT, HALVES>;
   using Lut = E8pLut<GEMV_COPIES>;
+  constexpr int LUT_BYTES = FMT == 0 ? 0 : static_cast<int>(sizeof(Lut));
   const PeerOut* peer = po.tp > 0 ? &po : nullptr;
   const bool ll = peer != nullptr && po.rows_per == LL_MODE;
   const int ll_seq = ll ? *reinterpret_cast<volatile int*>(po.sent) + 1 : 0;
   extern __shared__ __align__(16) unsigned char smem_raw[];
   Lut* lut = reinterpret_cast<Lut*>(smem_raw);
-  int8_t* act = reinterpret_cast<int8_t*>(smem_raw) + sizeof(Lut);
-  int* acc_s = reinterpret_cast<int*>(act + static_cast<size_t>(MT) * K);   // [groups][ROWS][MT]
-  int* asum = acc_s + max_groups * ROWS * MT;                                // [MT]
+  int8_t* act = reinterpret_cast<int8_t*>(smem_raw) + LUT_BYTES;
+  int* acc_s = reinterpret_cast<int*>(act + static_cast<size_t>(MT) * K);   // [16 max_groups][MT]
+  int* asum = acc_s + max_groups * 16 * MT;                                  // [MT]
   float* scale_s = reinterpret_cast<float*>(asum + MT);                      // [MT]
   float* fbuf = reinterpret_cast<float*>(                                    // [K], pre only
       (reinterpret_cast<uintptr_t>(scale_s + MT) + 15) & ~static_cast<uintptr_t>(15));
@@ -119,10 +158,64 @@ __global__ void __launch_bounds__(GemvThreads<MT>::value, 1) e8p_gemv_kernel(
   __shared__ float blk_sum[128];
 
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-  e8p_lut_init(lut, tables, tid, THREADS);
-  for (int i = tid; i < max_groups * ROWS * MT + MT; i += THREADS) acc_s[i] = 0;
+  const int g = lane >> 2, t = lane & 3;
+  const int kb_all = K / 128;
+  // a CTA's rows are a multiple of eight (the SMs then differ by 8 rows, not 16); its last group
+  // may be half a group
+  const int oct = N / 8;
+  const int np = blockIdx.x % n_parts, kp = blockIdx.x / n_parts;
+  const int n_base = static_cast<int>(static_cast<long long>(oct) * np / n_parts) * 8;
+  const int n_count = static_cast<int>(static_cast<long long>(oct) * (np + 1) / n_parts) * 8 - n_base;
+  const int groups = (n_count + ROWS - 1) / ROWS;
+  const int kb_lo = kb_all * kp / k_parts, kb_hi = kb_all * (kp + 1) / k_parts;
+  const int kbs = kb_hi - kb_lo;
+  const int units = groups * kbs;
+  constexpr int NW = THREADS / 32;
+  const int u_lo = static_cast<int>(static_cast<long long>(units) * warp / NW);
+  const int u_hi = static_cast<int>(static_cast<long long>(units) * (warp + 1) / NW);
+  // (group, k-block) of the unit being loaded, and of the unit being consumed
+  int lg = 0, lkb = 0;
+  if (u_lo < u_hi) {
+    lg = u_lo / kbs;
+    lkb = kb_lo + u_lo % kbs;
+  }
+  int cg = lg, ckb = lkb;
+  Unit buf[DEPTH];
+  auto fetch = [&](Unit& v, int uu) {
+    if (uu >= u_hi) return;
+#pragma unroll
+    for (int h = 0; h < HALVES; ++h) {
+      if (h == 1 && lg * ROWS + 8 >= n_count) break;       // half a group
+      const int n = n_base + lg * ROWS + g + h * 8;
+      if (FMT == 0) {
+        const uint4* p = reinterpret_cast<const uint4*>(w) + static_cast<size_t>(n) * (K / 16) +
+                         lkb * 8 + t;
+        const uint4 x = __ldg(p), y = __ldg(p + 4);
+        v.w[h][0] = x.x; v.w[h][1] = x.y; v.w[h][2] = x.z; v.w[h][3] = x.w;
+        v.w[h][4 % Unit::WORDS] = y.x; v.w[h][5 % Unit::WORDS] = y.y;
+        v.w[h][6 % Unit::WORDS] = y.z; v.w[h][7 % Unit::WORDS] = y.w;
+      } else if (FMT == 1) {
+        const uint4 x =
+            __ldg(reinterpret_cast<const uint4*>(w) + (static_cast<size_t>(lkb) * N + n) * 4 + t);
+        v.w[h][0] = x.x; v.w[h][1] = x.y;
+        v.w[h][2 % Unit::WORDS] = x.z; v.w[h][3 % Unit::WORDS] = x.w;
+      } else {
+        const uint2 x =
+            __ldg(reinterpret_cast<const uint2*>(w) + (static_cast<size_t>(lkb) * N + n) * 4 + t);
+        v.w[h][0] = x.x; v.w[h][1] = x.y;
+      }
+    }
+    if (++lkb == kb_hi) {
+      lkb = kb_lo;
+      ++lg;
+    }
+  };
+#pragma unroll
+  for (int i = 0; i < DEPTH; ++i) fetch(buf[i], u_lo + i);
+  if (FMT != 0) e8p_lut_init(lut, tables, tid, THREADS);
+  for (int i = tid; i < max_groups * 16 * MT + MT; i += THREADS) acc_s[i] = 0;
   __syncthreads();
-  if (fz.pre == 0) {
+  if (FMT == 0 || fz.pre == 0) {
     // stage the activations; their row sums ride along
     const int chunks = MT * K / 16;
     int part_sum[MT];
@@ -132,7 +225,9 @@ __global__ void __launch_bounds__(GemvThreads<MT>::value, 1) e8p_gemv_kernel(
       const int m = (c * 16) / K;
       int4 v = make_int4(0, 0, 0, 0);
       if (m < M) v = *reinterpret_cast<const int4*>(a + static_cast<size_t>(c) * 16);
-      *reinterpret_cast<int4*>(act + static_cast<size_t>(c) * 16) = v;
+      const int k = c * 16 - m * K;
+      *reinterpret_cast<int2*>(act + act_pos<FMT, MT>(m, k)) = make_int2(v.x, v.y);
+      *reinterpret_cast<int2*>(act + act_pos<FMT, MT>(m, k + 8)) = make_int2(v.z, v.w);
       int s = __dp4a(v.x, 0x01010101, 0);
       s = __dp4a(v.y, 0x01010101, s);
       s = __dp4a(v.z, 0x01010101, s);
@@ -154,12 +249,7 @@ __global__ void __launch_bounds__(GemvThreads<MT>::value, 1) e8p_gemv_kernel(
     constexpr int NWP = THREADS / 32;
     const bool first_cta = blockIdx.x == 0;
     for (int m = 0; m < MT; ++m) {
-      int8_t* arow = act + static_cast<size_t>(m) * K;
-      if (m >= M) {
-        for (int i = tid * 16; i < K; i += THREADS * 16)
-          *reinterpret_cast<int4*>(arow + i) = make_int4(0, 0, 0, 0);
-        continue;
-      }
+      if (m >= M) break;                         // columns past the last row are not used
       float* fb = fbuf;                          // one row at a time
       if (fz.pre == 3) {
         const __half* g = fz.x + static_cast<size_t>(m) * 2 * K;
@@ -250,7 +340,7 @@ __global__ void __launch_bounds__(GemvThreads<MT>::value, 1) e8p_gemv_kernel(
         c.y = static_cast<signed char>(a8_code(fb[i + 1], scale));
         c.z = static_cast<signed char>(a8_code(fb[i + 2], scale));
         c.w = static_cast<signed char>(a8_code(fb[i + 3], scale));
-        *reinterpret_cast<char4*>(arow + i) = c;
+        *reinterpret_cast<char4*>(act + act_pos<FMT, MT>(m, i)) = c;
         if (fz.q_out != nullptr && first_cta)
           *reinterpret_cast<char4*>(fz.q_out + static_cast<size_t>(m) * K + i) = c;
         psum = __dp4a(*reinterpret_cast<const int*>(&c), 0x01010101, psum);
@@ -267,97 +357,93 @@ __global__ void __launch_bounds__(GemvThreads<MT>::value, 1) e8p_gemv_kernel(
   }
   __syncthreads();
 
-  const int row = lane / LPR, part = lane % LPR;
-  const int kb_all = K / 128;
-  const int groups = (N + ROWS - 1) / ROWS;
-  const int np = blockIdx.x % n_parts, kp = blockIdx.x / n_parts;
-  const int g_lo = static_cast<int>(static_cast<long long>(groups) * np / n_parts);
-  const int g_hi = static_cast<int>(static_cast<long long>(groups) * (np + 1) / n_parts);
-  const int kb_lo = kb_all * kp / k_parts, kb_hi = kb_all * (kp + 1) / k_parts;
-  const int kbs = kb_hi - kb_lo;
-  const int units = (g_hi - g_lo) * kbs;
-  constexpr int NW = THREADS / 32;
-  const int u_lo = static_cast<int>(static_cast<long long>(units) * warp / NW);
-  const int u_hi = static_cast<int>(static_cast<long long>(units) * (warp + 1) / NW);
-
-  int acc[MT];
-#pragma unroll
-  for (int m = 0; m < MT; ++m) acc[m] = 0;
+  int acc[4] = {0, 0, 0, 0};
   const int copy = lane;                                   // GEMV_COPIES == 32
-
-  if (u_lo < u_hi) {
-    // (group, k-block) of the unit being loaded, and of the unit being consumed
-    int lg = g_lo + u_lo / kbs, lkb = kb_lo + u_lo % kbs;
-    int g = lg, kb = lkb;
-    uint4 buf[DEPTH];
-    auto fetch = [&](int uu) -> uint4 {
-      uint4 v = make_uint4(0, 0, 0, 0);
-      if (uu < u_hi) {
-        const int n = min(lg * ROWS + row, N - 1);
-        v = __ldg(w + (static_cast<size_t>(lkb) * N + n) * LPR + part);
-        if (++lkb == kb_hi) {
-          lkb = kb_lo;
-          ++lg;
+  for (int base = u_lo; base < u_hi; base += DEPTH) {
+#pragma unroll
+    for (int i = 0; i < DEPTH; ++i) {
+      if (base + i < u_hi) {
+        const bool half = HALVES == 2 && cg * ROWS + 8 >= n_count;
+        if (DP4A) {
+          const Unit cur = buf[i];
+          fetch(buf[i], base + i + DEPTH);
+#pragma unroll
+          for (int j = 0; j < 4; ++j) {
+            const uint32_t word = cur.w[0][j % Unit::WORDS];
+            const uint32_t v0 = e8p_fields<GEMV_COPIES, 0>(word, lut, copy);
+            const uint32_t v1 = e8p_fields<GEMV_COPIES, 1>(word, lut, copy);
+            const int xlo = static_cast<int>((v0 & E8P_NIB) * 4u + (v1 & E8P_NIB));
+            const int xhi = static_cast<int>(((v0 >> 4) & E8P_NIB) * 4u + ((v1 >> 4) & E8P_NIB));
+#pragma unroll
+            for (int m = 0; m < MT && m < 2; ++m) {
+              const int2 av =
+                  *reinterpret_cast<const int2*>(act + ((ckb * 16 + t * 4 + j) * MT + m) * 8);
+              acc[m] = __dp4a(xhi, av.y, __dp4a(xlo, av.x, acc[m]));
+            }
+          }
+        } else if (FMT == 0) {
+#pragma unroll
+          for (int j = 0; j < 2; ++j) {
+            int4 b = make_int4(0, 0, 0, 0);
+            if (g < MT)
+              b = *reinterpret_cast<const int4*>(act + act_pos<FMT, MT>(g, ckb * 128 + j * 64 + t * 16));
+            const uint32_t* r0 = buf[i].w[0] + (j * 4) % Unit::WORDS;
+            const uint32_t* r1 = buf[i].w[HALVES - 1] + (j * 4) % Unit::WORDS;
+            mma_i8_16832(acc, r0[0], r1[0], r0[1], r1[1], b.x, b.y);
+            mma_i8_16832(acc, r0[2 % Unit::WORDS], r1[2 % Unit::WORDS], r0[3 % Unit::WORDS],
+                         r1[3 % Unit::WORDS], b.z, b.w);
+          }
+        } else {
+#pragma unroll
+          for (int j = 0; j < 4; ++j) {
+            int2 b = make_int2(0, 0);
+            if (g < MT)
+              b = *reinterpret_cast<const int2*>(act + ((ckb * 16 + j * 4 + t) * MT + g) * 8);
+            uint32_t lo[2] = {0u, 0u}, hi[2] = {0u, 0u};
+#pragma unroll
+            for (int h = 0; h < 2; ++h) {
+              if (h == 1 && half) break;
+              if (FMT == 1) {
+                const uint32_t word = buf[i].w[h % HALVES][j % Unit::WORDS];
+                const uint32_t v0 = e8p_fields<GEMV_COPIES, 0>(word, lut, copy);
+                const uint32_t v1 = e8p_fields<GEMV_COPIES, 1>(word, lut, copy);
+                lo[h] = (v0 & E8P_NIB) * 4u + (v1 & E8P_NIB);
+                hi[h] = ((v0 >> 4) & E8P_NIB) * 4u + ((v1 >> 4) & E8P_NIB);
+              } else {
+                const uint32_t word = buf[i].w[h % HALVES][(j >> 1) % Unit::WORDS];
+                const uint32_t v = (j & 1) ? e8p_fields<GEMV_COPIES, 1>(word, lut, copy)
+                                           : e8p_fields<GEMV_COPIES, 0>(word, lut, copy);
+                lo[h] = v & E8P_NIB;
+                hi[h] = (v >> 4) & E8P_NIB;
+              }
+            }
+            mma_i8_16832(acc, lo[0], lo[1], hi[0], hi[1], b.x, b.y);
+          }
         }
-      }
-      return v;
-    };
+        if (!DP4A) fetch(buf[i], base + i + DEPTH);
+        const bool last_of_group = ckb + 1 == kb_hi, last_unit = base + i + 1 == u_hi;
+        if (last_of_group || last_unit) {
 #pragma unroll
-    for (int i = 0; i < DEPTH; ++i) buf[i] = fetch(u_lo + i);
-    for (int base = u_lo; base < u_hi; base += DEPTH) {
-#pragma unroll
-      for (int i = 0; i < DEPTH; ++i) {
-        const uint4 cur = buf[i];
-        buf[i] = fetch(base + i + DEPTH);
-        if (base + i < u_hi) {
-          const int8_t* abase = act + kb * 128 + part * WPL;
-          const uint32_t words[4] = {cur.x, cur.y, cur.z, cur.w};
-          if (FMT == 1) {
-#pragma unroll
-            for (int j = 0; j < 4; ++j) {
-              const uint32_t v0 = e8p_fields<GEMV_COPIES, 0>(words[j], lut, copy);
-              const uint32_t v1 = e8p_fields<GEMV_COPIES, 1>(words[j], lut, copy);
-              const int xlo = static_cast<int>((v0 & E8P_NIB) * 4u + (v1 & E8P_NIB));
-              const int xhi = static_cast<int>(((v0 >> 4) & E8P_NIB) * 4u + ((v1 >> 4) & E8P_NIB));
-#pragma unroll
-              for (int m = 0; m < MT; ++m) {
-                const int2 av = *reinterpret_cast<const int2*>(abase + m * K + j * 8);
-                acc[m] = __dp4a(xlo, av.x, acc[m]);
-                acc[m] = __dp4a(xhi, av.y, acc[m]);
-              }
+          for (int e = 0; e < 4; ++e) {
+            if (DP4A) {
+              if (e >= MT) break;
+              int v = acc[e];
+              v += __shfl_xor_sync(0xffffffffu, v, 1);
+              v += __shfl_xor_sync(0xffffffffu, v, 2);
+              if (t == 0) atomicAdd(&acc_s[(cg * ROWS + g) * MT + e], v);
+            } else {
+              const int m = 2 * t + (e & 1);
+              if (m < MT && !(half && e >= 2))
+                atomicAdd(&acc_s[(cg * ROWS + g + (e >> 1) * 8) * MT + m], acc[e]);
             }
-          } else {
-#pragma unroll
-            for (int j = 0; j < 8; ++j) {
-              const uint32_t v = (j & 1) ? e8p_fields<GEMV_COPIES, 1>(words[j >> 1], lut, copy)
-                                         : e8p_fields<GEMV_COPIES, 0>(words[j >> 1], lut, copy);
-              const int xlo = static_cast<int>(v & E8P_NIB);
-              const int xhi = static_cast<int>((v >> 4) & E8P_NIB);
-#pragma unroll
-              for (int m = 0; m < MT; ++m) {
-                const int2 av = *reinterpret_cast<const int2*>(abase + m * K + j * 8);
-                acc[m] = __dp4a(xlo, av.x, acc[m]);
-                acc[m] = __dp4a(xhi, av.y, acc[m]);
-              }
-            }
+            acc[e] = 0;
           }
-          const bool last_of_group = kb + 1 == kb_hi, last_unit = base + i + 1 == u_hi;
-          if (last_of_group || last_unit) {
-#pragma unroll
-            for (int m = 0; m < MT; ++m) {
-              int v = acc[m];
-#pragma unroll
-              for (int o = 1; o < LPR; o <<= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
-              if (part == 0) atomicAdd(&acc_s[((g - g_lo) * ROWS + row) * MT + m], v);
-              acc[m] = 0;
-            }
-          }
-          if (last_of_group) {
-            kb = kb_lo;
-            ++g;
-          } else {
-            ++kb;
-          }
+        }
+        if (last_of_group) {
+          ckb = kb_lo;
+          ++cg;
+        } else {
+          ++ckb;
         }
       }
     }
@@ -365,9 +451,7 @@ __global__ void __launch_bounds__(GemvThreads<MT>::value, 1) e8p_gemv_kernel(
   __syncthreads();
 
   // sum_k a_k w_k from the staged integers: Q4 2*acc - 75*S, Q2 2*acc - 15*S
-  constexpr int BIAS = FMT == 1 ? 75 : 15;
-  const int n_base = g_lo * ROWS;
-  const int n_count = min(g_hi * ROWS, N) - n_base;        // output columns of this n-part
+  constexpr int UNIT = FMT == 0 ? 1 : 2, BIAS = FMT == 0 ? 0 : (FMT == 1 ? 75 : 15);
   bool finalize = true;
   if (k_parts > 1) {
     // add this CTA's integers to the workspace; the last CTA of the n-part finishes
@@ -414,7 +498,7 @@ __global__ void __launch_bounds__(GemvThreads<MT>::value, 1) e8p_gemv_kernel(
           const int bias = BIAS * asum[m];
 #pragma unroll
           for (int r = 0; r < 8; ++r) {
-            const int total = 2 * acc_s[(seg * 8 + r) * MT + m] - bias;
+            const int total = UNIT * acc_s[(seg * 8 + r) * MT + m] - bias;
             h[r] = __float2half_rn(
                 (static_cast<float>(total) * __half2float(w_scale[n_base + seg * 8 + r])) * sa);
           }
@@ -432,9 +516,9 @@ __global__ void __launch_bounds__(GemvThreads<MT>::value, 1) e8p_gemv_kernel(
       for (int i = tid; i < n_count * MT; i += THREADS) {
         const int m = i / n_count, r = i % n_count;
         if (m < M) {
-          const int total = 2 * acc_s[r * MT + m] - BIAS * asum[m];
+          const int total = UNIT * acc_s[r * MT + m] - BIAS * asum[m];
           const float sw = __half2float(w_scale[n_base + r]);
-          if (fz.resid_accum != nullptr) {
+          if (FMT != 0 && fz.resid_accum != nullptr) {
             const __half hv = __float2half_rn((static_cast<float>(total) * sw) * scale_s[m]);
             float* dst = fz.resid_accum + static_cast<size_t>(m) * N + n_base + r;
             *dst = *dst + __half2float(hv);
@@ -451,9 +535,12 @@ __global__ void __launch_bounds__(GemvThreads<MT>::value, 1) e8p_gemv_kernel(
   else if (peer != nullptr) peer_signal_done(po, gridDim.x);
 }
 
-// W8: one warp per output row, 16 weights per lane per step.
+// INT8 weights, one or two rows: one warp per output row, 16 weights per lane per step, as many
+// CTAs as rows need.  Small projections that sit in L2 are twice as fast this way (6144 x 2560,
+// one row: 3.7 us against 6.9 with persistent CTAs; the 151936-row head 74 against 75); from four
+// rows on the shared-memory reads per row lose to the MMAs (head, eight rows: 205 against 77 us).
 template <int MT>
-__global__ void __launch_bounds__(GEMV_WARPS * 32) w8_gemv_kernel(
+__global__ void __launch_bounds__(W8_WARPS * 32) w8_gemv_kernel(
     const int8_t* __restrict__ a, const float* __restrict__ a_scale, const int8_t* __restrict__ w,
     const __half* __restrict__ w_scale, void* __restrict__ out, int M, int N, int K, int out_f32,
     PeerOut po) {
@@ -463,7 +550,7 @@ __global__ void __launch_bounds__(GEMV_WARPS * 32) w8_gemv_kernel(
   stage_activations<MT>(act, a, M, K);
   __syncthreads();
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int n = blockIdx.x * GEMV_WARPS + warp;
+  const int n = blockIdx.x * W8_WARPS + warp;
   if (n < N) {
   const int8_t* wr = w + static_cast<size_t>(n) * K;
   int acc[MT];
@@ -493,59 +580,282 @@ __global__ void __launch_bounds__(GEMV_WARPS * 32) w8_gemv_kernel(
   if (peer != nullptr) peer_signal_done(po, gridDim.x);
 }
 
-// Grid shape of the E8P GEMV: n_parts x k_parts CTAs on the 148 SMs.  K is split (2, 4 or
-// 8 ways, at least 4 k-blocks each) when whole row groups divide badly over the SMs.
+// ---------------------------------------------------------------- experts with few rows each
+// Grouped form for decode batches: the tile table of the MoE plan lists (expert, first row, rows),
+// most experts have one or two rows, and the tensor-core GEMM would spend a 128-row tile on
+// each.  Here a warp takes one (tile, 16-row group of its expert's bank) item at a time over the
+// whole K, weights as A and up to eight activation rows as B as above; the activations are read
+// from global memory with the weights (a tile's rows are shared by the warps of a CTA through
+// L1).  Tiles of more rows repeat the decode once per sixteen rows.
+template <int FMT>
+struct ExpertUnit {
+  GemvUnit<FMT> u;
+  uint4 act[2];                                    // this lane's 32 bytes of activation row g
+};
+
+template <int FMT>
+__global__ void __launch_bounds__(GEMV_THREADS, 1) qgemv_grouped_kernel(
+    const int8_t* __restrict__ a, const float* __restrict__ a_scale,
+    const unsigned char* __restrict__ w, const __half* __restrict__ w_scale,
+    __half* __restrict__ out, int N, int K, long long bank_bytes,
+    const E8pTables* __restrict__ tables, const int* __restrict__ tiles,
+    const int* __restrict__ meta) {
+  using Lut = E8pLut<GEMV_COPIES>;
+  using W = GemvUnit<FMT>;
+  constexpr int NB = 2;                            // eight-row blocks per pass over the weights
+  extern __shared__ __align__(16) unsigned char smem_raw[];
+  constexpr int WARPS = GEMV_THREADS / 32;
+  Lut* lut = reinterpret_cast<Lut*>(smem_raw);
+  int(*red)[NB * 5][32] = reinterpret_cast<int(*)[NB * 5][32]>(
+      smem_raw + (FMT == 0 ? 0 : sizeof(Lut)));        // [WARPS]
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, g = lane >> 2, t = lane & 3;
+  if (FMT != 0) e8p_lut_init(lut, tables, tid, GEMV_THREADS);
+  __syncthreads();
+  const int groups = N / 16, kbs = K / 128, items = meta[0] * groups;
+  // With fewer items than warps (a decode step of one or two rows) KS neighbouring warps share
+  // an item's K and the first of them adds the parts: the walk over K is a chain of loads.
+  int ks = 1;
+  while (ks < 8 && kbs >= 4 * ks && items * ks * 2 <= static_cast<int>(gridDim.x) * WARPS) ks *= 2;
+  const int sub = warp % ks, kb_lo = kbs * sub / ks, kb_hi = kbs * (sub + 1) / ks;
+  const int stride = gridDim.x * (WARPS / ks);
+  constexpr int UNIT = FMT == 0 ? 1 : 2, BIAS = FMT == 0 ? 0 : (FMT == 1 ? 75 : 15);
+  // byte offset of this lane's two 16-byte pieces inside a 128-channel block of a row
+  const int piece0 = FMT == 0 ? t * 16 : t * 32, piece1 = FMT == 0 ? 64 + t * 16 : t * 32 + 16;
+
+  for (int item = blockIdx.x * (WARPS / ks) + warp / ks; item < items; item += stride) {
+    const int tile = item / groups, n0 = (item - tile * groups) * 16;
+    const int expert = __ldg(tiles + tile * 4), first = __ldg(tiles + tile * 4 + 1);
+    const int rows = __ldg(tiles + tile * 4 + 2);
+    const unsigned char* bank = w + static_cast<size_t>(expert) * bank_bytes;
+    for (int r0 = 0; r0 < rows; r0 += 8 * NB) {
+      const int nb = min(NB, (rows - r0 + 7) / 8);
+      // rows past the tile's last one repeat it; their results are not stored
+      const int8_t* arow[NB];
+#pragma unroll
+      for (int b = 0; b < NB; ++b)
+        arow[b] = a + static_cast<size_t>(first + min(r0 + b * 8 + g, rows - 1)) * K;
+      auto fetch = [&](ExpertUnit<FMT>& v, int kb) {
+        if (kb >= kb_hi) return;
+#pragma unroll
+        for (int h = 0; h < 2; ++h) {
+          const int n = n0 + g + h * 8;
+          if (FMT == 0) {
+            const uint4* p = reinterpret_cast<const uint4*>(bank) +
+                             static_cast<size_t>(n) * (K / 16) + kb * 8 + t;
+            const uint4 x = __ldg(p), y = __ldg(p + 4);
+            v.u.w[h][0] = x.x; v.u.w[h][1] = x.y; v.u.w[h][2 % W::WORDS] = x.z;
+            v.u.w[h][3 % W::WORDS] = x.w; v.u.w[h][4 % W::WORDS] = y.x;
+            v.u.w[h][5 % W::WORDS] = y.y; v.u.w[h][6 % W::WORDS] = y.z;
+            v.u.w[h][7 % W::WORDS] = y.w;
+          } else if (FMT == 1) {
+            const uint4 x = __ldg(reinterpret_cast<const uint4*>(bank) +
+                                  (static_cast<size_t>(kb) * N + n) * 4 + t);
+            v.u.w[h][0] = x.x; v.u.w[h][1] = x.y;
+            v.u.w[h][2 % W::WORDS] = x.z; v.u.w[h][3 % W::WORDS] = x.w;
+          } else {
+            const uint2 x = __ldg(reinterpret_cast<const uint2*>(bank) +
+                                  (static_cast<size_t>(kb) * N + n) * 4 + t);
+            v.u.w[h][0] = x.x; v.u.w[h][1] = x.y;
+          }
+        }
+        v.act[0] = __ldg(reinterpret_cast<const uint4*>(arow[0] + kb * 128 + piece0));
+        v.act[1] = __ldg(reinterpret_cast<const uint4*>(arow[0] + kb * 128 + piece1));
+      };
+      int acc[NB][4], asum[NB];
+#pragma unroll
+      for (int b = 0; b < NB; ++b) {
+        asum[b] = 0;
+#pragma unroll
+        for (int e = 0; e < 4; ++e) acc[b][e] = 0;
+      }
+      constexpr int DEPTH = FMT == 0 ? 1 : 2;
+      ExpertUnit<FMT> buf[DEPTH];
+#pragma unroll
+      for (int i = 0; i < DEPTH; ++i) fetch(buf[i], kb_lo + i);
+      for (int base = kb_lo; base < kb_hi; base += DEPTH) {
+#pragma unroll
+        for (int i = 0; i < DEPTH; ++i) {
+          const int kb = base + i;
+          if (kb >= kb_hi) break;
+#pragma unroll
+          for (int j = 0; j < 4; ++j) {
+            uint32_t f[4];                         // {row g, row g + 8} x {low, high} words
+#pragma unroll
+            for (int h = 0; h < 2; ++h) {
+              if (FMT == 0) {
+                f[h] = buf[i].u.w[h][(2 * j) % W::WORDS];
+                f[2 + h] = buf[i].u.w[h][(2 * j + 1) % W::WORDS];
+              } else if (FMT == 1) {
+                const uint32_t word = buf[i].u.w[h][j % W::WORDS];
+                const uint32_t v0 = e8p_fields<GEMV_COPIES, 0>(word, lut, lane);
+                const uint32_t v1 = e8p_fields<GEMV_COPIES, 1>(word, lut, lane);
+                f[h] = (v0 & E8P_NIB) * 4u + (v1 & E8P_NIB);
+                f[2 + h] = ((v0 >> 4) & E8P_NIB) * 4u + ((v1 >> 4) & E8P_NIB);
+              } else {
+                const uint32_t word = buf[i].u.w[h][(j >> 1) % W::WORDS];
+                const uint32_t v = (j & 1) ? e8p_fields<GEMV_COPIES, 1>(word, lut, lane)
+                                           : e8p_fields<GEMV_COPIES, 0>(word, lut, lane);
+                f[h] = v & E8P_NIB;
+                f[2 + h] = (v >> 4) & E8P_NIB;
+              }
+            }
+#pragma unroll
+            for (int b = 0; b < NB; ++b) {
+              uint32_t x0, x1;
+              if (b == 0) {
+                const uint4& p = buf[i].act[j >> 1];
+                x0 = j & 1 ? p.z : p.x;
+                x1 = j & 1 ? p.w : p.y;
+              } else {
+                if (b >= nb) break;
+                const uint2 p = __ldg(reinterpret_cast<const uint2*>(
+                    arow[b] + kb * 128 + (j >> 1 ? piece1 : piece0) + (j & 1) * 8));
+                x0 = p.x;
+                x1 = p.y;
+              }
+              if (FMT != 0)
+                asum[b] = __dp4a(static_cast<int>(x1), 0x01010101,
+                                 __dp4a(static_cast<int>(x0), 0x01010101, asum[b]));
+              mma_i8_16832(acc[b], f[0], f[1], f[2], f[3], x0, x1);
+            }
+          }
+          fetch(buf[i], kb + DEPTH);
+        }
+      }
+      if (ks > 1) {
+        // the warps of an item meet at their own named barrier, before and after the exchange
+        if (sub != 0) {
+#pragma unroll
+          for (int b = 0; b < NB; ++b) {
+#pragma unroll
+            for (int e = 0; e < 4; ++e) red[warp][b * 5 + e][lane] = acc[b][e];
+            red[warp][b * 5 + 4][lane] = asum[b];
+          }
+        }
+        asm volatile("bar.sync %0, %1;" ::"r"(warp / ks), "r"(ks * 32) : "memory");
+        if (sub == 0) {
+          for (int q = 1; q < ks; ++q) {
+#pragma unroll
+            for (int b = 0; b < NB; ++b) {
+#pragma unroll
+              for (int e = 0; e < 4; ++e) acc[b][e] += red[warp + q][b * 5 + e][lane];
+              asum[b] += red[warp + q][b * 5 + 4][lane];
+            }
+          }
+        }
+        asm volatile("bar.sync %0, %1;" ::"r"(warp / ks), "r"(ks * 32) : "memory");
+        if (sub != 0) continue;
+      }
+#pragma unroll
+      for (int b = 0; b < NB; ++b) {
+        if (b >= nb) break;
+        asum[b] += __shfl_xor_sync(0xffffffffu, asum[b], 1);
+        asum[b] += __shfl_xor_sync(0xffffffffu, asum[b], 2);
+#pragma unroll
+        for (int e = 0; e < 4; ++e) {
+          const int m = r0 + b * 8 + 2 * t + (e & 1), n = n0 + g + (e >> 1) * 8;
+          const int sum = __shfl_sync(0xffffffffu, asum[b], (2 * t + (e & 1)) * 4);
+          if (m < rows) {
+            const int total = UNIT * acc[b][e] - BIAS * sum;
+            const float sw = __half2float(w_scale[static_cast<size_t>(expert) * N + n]);
+            out[static_cast<size_t>(first + m) * N + n] =
+                __float2half_rn((static_cast<float>(total) * sw) * a_scale[first + m]);
+          }
+        }
+      }
+    }
+  }
+}
+
+template <int FMT>
+static int launch_grouped(const int8_t* a, const float* as, const void* w, const __half* ws,
+                          void* out, int N, int K, long long bank, const int* tiles,
+                          const int* meta, cudaStream_t stream) {
+  const size_t smem = (FMT == 0 ? 0 : sizeof(E8pLut<GEMV_COPIES>)) + GEMV_THREADS * 10 * sizeof(int);
+  static const int slot = runtime_new_slot();
+  if (runtime_first_use(slot)) {
+    cudaError_t e = cudaFuncSetAttribute(qgemv_grouped_kernel<FMT>,
+                                         cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                         static_cast<int>(smem));
+    if (e != cudaSuccess) return static_cast<int>(e);
+  }
+  qgemv_grouped_kernel<FMT><<<148, GEMV_THREADS, smem, stream>>>(
+      a, as, reinterpret_cast<const unsigned char*>(w), ws, reinterpret_cast<__half*>(out), N, K,
+      bank, runtime_e8p_tables(), tiles, meta);
+  return static_cast<int>(cudaGetLastError());
+}
+
+int qgemv_grouped_dispatch(int fmt, const int8_t* a, const float* as, const void* w,
+                           const __half* ws, void* out, int N, int K, long long bank,
+                           const int* tiles, const int* meta, cudaStream_t stream) {
+  if (fmt == 0) return launch_grouped<0>(a, as, w, ws, out, N, K, bank, tiles, meta, stream);
+  if (fmt == 1) return launch_grouped<1>(a, as, w, ws, out, N, K, bank, tiles, meta, stream);
+  return launch_grouped<2>(a, as, w, ws, out, N, K, bank, tiles, meta, stream);
+}
+
+// Grid shape: n_parts x k_parts CTAs on the 148 SMs.  E8P projections may split K (2, 4 or 8
+// ways, at least 4 k-blocks each) when their rows divide badly over the SMs.  The costs are
+// measured: 0.03 us per eight rows x 128 channels on a full SM (Q4; 19456 x 2560: 16.4 x 20 of
+// them in 10 us), and about 2.5 us for the round trip through the workspace, which is why
+// splitting pays for long K only (2560 x 4096 took 10.3 us in eight parts, 6.7 us for a 2048 x
+// 4096 projection unsplit).
 struct GemvGrid {
   int n_parts, k_parts, max_groups;
 };
-static GemvGrid gemv_grid(int rows_per_group, int N, int K) {
-  const int groups = (N + rows_per_group - 1) / rows_per_group, kb = K / 128;
-  GemvGrid best{groups < 148 ? groups : 148, 1, 0};
-  double best_eff = 0.0;
-  for (int kp = 1; kp <= 8; kp *= 2) {
-    if (kp > 1 && (kb / kp < 4 || N > GEMV_WS_COLS || 148 / kp > GEMV_WS_TICKETS)) break;
-    const int np = groups < 148 / kp ? groups : 148 / kp;
-    const int per = (groups + np - 1) / np;
-    double eff = (static_cast<double>(groups) / np / per) * (static_cast<double>(np) * kp / 148.0);
-    if (kp > 1) eff *= 0.97;                       // the workspace round trip is not free
-    if (eff > best_eff + 1e-9) {
-      best_eff = eff;
-      best = GemvGrid{np, kp, 0};
+static GemvGrid gemv_grid(int fmt, int N, int K) {
+  const int oct = N / 8, kb = K / 128;
+  GemvGrid best{1, 1, 0};
+  if (fmt == 0) {
+    best.n_parts = oct < 148 ? oct : 148;
+  } else {
+    double best_cost = 0.0;
+    for (int kp = 1; kp <= 8; kp *= 2) {
+      if (kp > 1 && (kb / kp < 4 || N > GEMV_WS_COLS || 148 / kp > GEMV_WS_TICKETS)) break;
+      const int np = oct < 148 / kp ? oct : 148 / kp;
+      const double cost = ((oct + np - 1) / np) * ((kb + kp - 1) / kp) * (fmt == 1 ? 0.03 : 0.02) +
+                          (kp > 1 ? 2.5 : 0.0);
+      if (kp == 1 || cost < best_cost) {
+        best_cost = cost;
+        best = GemvGrid{np, kp, 0};
+      }
     }
   }
-  best.max_groups = (groups + best.n_parts - 1) / best.n_parts;
+  best.max_groups = ((oct + best.n_parts - 1) / best.n_parts + 1) / 2;
   return best;
 }
 
 constexpr size_t GEMV_SMEM_LIMIT = 220 * 1024;
 
-// Dynamic shared memory of the E8P GEMV for `mt` staged activation rows.
-static size_t e8p_gemv_smem(int fmt, int mt, int N, int K, bool fused) {
-  const int rows = fmt == 1 ? 8 : 16;
-  const GemvGrid g = gemv_grid(rows, N, K);
-  size_t smem = sizeof(E8pLut<GEMV_COPIES>) + static_cast<size_t>(mt) * K +
-                (static_cast<size_t>(g.max_groups) * rows * mt + 2 * mt) * sizeof(int) + 16;
+// Dynamic shared memory for `mt` staged activation rows.
+static size_t gemv_smem(int fmt, int mt, const GemvGrid& g, int K, bool fused) {
+  size_t smem = (fmt == 0 ? 0 : sizeof(E8pLut<GEMV_COPIES>)) + static_cast<size_t>(mt) * K +
+                (static_cast<size_t>(g.max_groups) * 16 * mt + 2 * mt) * sizeof(int) + 16;
   if (fused) smem += static_cast<size_t>(K) * sizeof(float);
   return smem;
 }
 
 template <int FMT, int MT>
-static int launch_e8p(const int8_t* a, const float* as, const void* w, const __half* ws, void* out,
-                      int M, int N, int K, int out_f32, cudaStream_t stream, const PeerOut& po,
-                      const GemvFuse& fz = GemvFuse{}) {
-  constexpr int ROWS = FMT == 1 ? 8 : 16;
-  const GemvGrid g = gemv_grid(ROWS, N, K);
-  const size_t smem = e8p_gemv_smem(FMT, MT, N, K, fz.pre != 0);
+static int launch_gemv(const int8_t* a, const float* as, const void* w, const __half* ws, void* out,
+                       int M, int N, int K, int out_f32, cudaStream_t stream, const PeerOut& po,
+                       const GemvFuse& fz = GemvFuse{}) {
+  GemvGrid g = gemv_grid(FMT, N, K);
+  size_t smem = gemv_smem(FMT, MT, g, K, fz.pre != 0);
+  // very wide INT8 projections under long rows: several waves of CTAs with fewer groups each
+  while (FMT == 0 && smem > GEMV_SMEM_LIMIT && g.max_groups > 1) {
+    g.n_parts *= 2;
+    g.max_groups = ((N / 8 + g.n_parts - 1) / g.n_parts + 1) / 2;
+    smem = gemv_smem(FMT, MT, g, K, fz.pre != 0);
+  }
   if (smem > GEMV_SMEM_LIMIT) return -1;
   static const int slot = runtime_new_slot();
   if (runtime_first_use(slot)) {
-    cudaError_t e = cudaFuncSetAttribute(e8p_gemv_kernel<FMT, MT>,
-                                         cudaFuncAttributeMaxDynamicSharedMemorySize, 220 * 1024);
+    cudaError_t e = cudaFuncSetAttribute(
+        qgemv_kernel<FMT, MT>, cudaFuncAttributeMaxDynamicSharedMemorySize, GEMV_SMEM_LIMIT);
     if (e != cudaSuccess) return static_cast<int>(e);
   }
-  e8p_gemv_kernel<FMT, MT><<<g.n_parts * g.k_parts, GemvThreads<MT>::value, smem, stream>>>(
-      a, as, reinterpret_cast<const uint4*>(w), ws, out, M, N, K, out_f32, runtime_e8p_tables(),
-      po, g.n_parts, g.k_parts, g.max_groups, runtime_gemv_workspace(), fz);
+  qgemv_kernel<FMT, MT><<<g.n_parts * g.k_parts, GEMV_THREADS, smem, stream>>>(
+      a, as, w, ws, out, M, N, K, out_f32, runtime_e8p_tables(), po, g.n_parts, g.k_parts,
+      g.max_groups, runtime_gemv_workspace(), fz);
   return static_cast<int>(cudaGetLastError());
 }
 
@@ -558,7 +868,7 @@ static int launch_w8(const int8_t* a, const float* as, const void* w, const __ha
   if (runtime_first_use(slot))
     cudaFuncSetAttribute(w8_gemv_kernel<MT>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                          200 * 1024);
-  w8_gemv_kernel<MT><<<(N + GEMV_WARPS - 1) / GEMV_WARPS, GEMV_WARPS * 32, smem, stream>>>(
+  w8_gemv_kernel<MT><<<(N + W8_WARPS - 1) / W8_WARPS, W8_WARPS * 32, smem, stream>>>(
       a, as, reinterpret_cast<const int8_t*>(w), ws, out, M, N, K, out_f32, po);
   return static_cast<int>(cudaGetLastError());
 }
@@ -568,12 +878,13 @@ int qgemv_dispatch(int fmt, const int8_t* a, const float* as, const void* w, con
                    const PeerOut* peer) {
   PeerOut po{};
   if (peer != nullptr) po = *peer;
-  if (M < 1 || M > 8 || K % 128) return -1;
+  if (M < 1 || M > 8 || K % 128 || N % 8) return -1;
   if (fmt != 0) {
     // Very long rows (K above about 19 000 at eight rows): the staged activations of all
     // rows do not fit beside the tables, so the rows go in several launches.
     int fit = 8;
-    while (fit > 1 && e8p_gemv_smem(fmt, fit, N, K, false) > GEMV_SMEM_LIMIT) fit /= 2;
+    const GemvGrid grid = gemv_grid(fmt, N, K);
+    while (fit > 1 && gemv_smem(fmt, fit, grid, K, false) > GEMV_SMEM_LIMIT) fit /= 2;
     if (M > fit) {
       if (peer != nullptr && peer->tp > 0) return -1;      // row indices of the push would shift
       const size_t out_row = static_cast<size_t>(N) * (out_f32 ? 4 : 2);
@@ -592,12 +903,14 @@ int qgemv_dispatch(int fmt, const int8_t* a, const float* as, const void* w, con
    : M == 2 ? FN<__VA_ARGS__ 2>(a, as, w, ws, out, M, N, K, out_f32, stream, po) \
    : M <= 4 ? FN<__VA_ARGS__ 4>(a, as, w, ws, out, M, N, K, out_f32, stream, po) \
             : FN<__VA_ARGS__ 8>(a, as, w, ws, out, M, N, K, out_f32, stream, po))
-  if (fmt == 0) {
-    if (K % 16) return -1;
-    return BY_M(launch_w8, );
-  }
-  if (fmt == 1) return BY_M(launch_e8p, 1, );
-  if (fmt == 2) return BY_M(launch_e8p, 2, );
+  if (fmt == 0 && M <= 2)
+    return M == 1 ? launch_w8<1>(a, as, w, ws, out, M, N, K, out_f32, stream, po)
+                  : launch_w8<2>(a, as, w, ws, out, M, N, K, out_f32, stream, po);
+  if (fmt == 0)
+    return M <= 4 ? launch_gemv<0, 4>(a, as, w, ws, out, M, N, K, out_f32, stream, po)
+                  : launch_gemv<0, 8>(a, as, w, ws, out, M, N, K, out_f32, stream, po);
+  if (fmt == 1) return BY_M(launch_gemv, 1, );
+  if (fmt == 2) return BY_M(launch_gemv, 2, );
 #undef BY_M
   return -1;
 }
@@ -605,14 +918,14 @@ int qgemv_dispatch(int fmt, const int8_t* a, const float* as, const void* w, con
 // Projection of at most 8 rows with the row preparation fused in (see GemvFuse); E8P weights.
 int qgemv_fused_dispatch(int fmt, const void* w, const __half* ws, void* out, int M, int N, int K,
                          cudaStream_t stream, const GemvFuse& fz) {
-  if (M < 1 || M > 8 || K % 128 || fz.pre < 1 || fz.pre > 3 || (fmt != 1 && fmt != 2)) return -1;
+  if (M < 1 || M > 8 || K % 128 || N % 8 || fz.pre < 1 || fz.pre > 3 || (fmt != 1 && fmt != 2)) return -1;
   if (fz.norm_w != nullptr && K / 128 > 128) return -1;
   const PeerOut po{};
 #define BY_M(F)                                                                                   \
-  (M == 1 ? launch_e8p<F, 1>(nullptr, nullptr, w, ws, out, M, N, K, 0, stream, po, fz)            \
-   : M == 2 ? launch_e8p<F, 2>(nullptr, nullptr, w, ws, out, M, N, K, 0, stream, po, fz)          \
-   : M <= 4 ? launch_e8p<F, 4>(nullptr, nullptr, w, ws, out, M, N, K, 0, stream, po, fz)          \
-            : launch_e8p<F, 8>(nullptr, nullptr, w, ws, out, M, N, K, 0, stream, po, fz))
+  (M == 1 ? launch_gemv<F, 1>(nullptr, nullptr, w, ws, out, M, N, K, 0, stream, po, fz)            \
+   : M == 2 ? launch_gemv<F, 2>(nullptr, nullptr, w, ws, out, M, N, K, 0, stream, po, fz)          \
+   : M <= 4 ? launch_gemv<F, 4>(nullptr, nullptr, w, ws, out, M, N, K, 0, stream, po, fz)          \
+            : launch_gemv<F, 8>(nullptr, nullptr, w, ws, out, M, N, K, 0, stream, po, fz))
   if (fmt == 1) return BY_M(1);
   return BY_M(2);
 #undef BY_M

@@ -95,28 +95,32 @@ __global__ void __launch_bounds__(256) router_topk_kernel(
   topk_row(logits, row, experts, has_shared, top_k, renorm, ids, probs, shared_gate);
 }
 
-// Tensor-core form (hidden % 256 == 0, at most 8 * 8 * MAXT expert rows).  The general form
+// Tensor-core form (hidden % 256 == 0, at most 64 MAXT expert rows).  The general form
 // streams the whole router matrix (0.5 to 2 MB) through every CTA, once per token row.  Here a
-// cluster of eight CTAs takes 16 rows: CTA c owns an eighth of the 8-expert tiles, its eight
-// warps an eighth of the hidden channels each (FP16 products, FP32 sums on the tensor cores;
-// the eight partial sums are added in a fixed order), and the logits of rows 2c and 2c + 1 are
-// collected in CTA c over distributed shared memory for the top-k.  Lane (g, t) loads 16 bytes
-// of row g: the halves 4s..4s+3 are its fragments of step s, in x and W alike.
-constexpr int ROUTER_CL = 8, ROUTER_ROWS = 16;
+// cluster of eight CTAs takes 16 rows: CTA c owns an eighth of the 8-expert tiles, its WARPS
+// warps a WARPS-th of the hidden channels each (FP16 products, FP32 sums on the tensor cores;
+// the partial sums are added in a fixed order that depends on the router alone, so a row's logits
+// do not depend on the packet), and each CTA collects the logits of its share of the rows
+// over distributed shared memory for the top-k.  Lane (g, t) loads 16 bytes of row g:
+// the halves 4s..4s+3 are its fragments of step s, in x and W alike.
 
-template <int MAXT>
-__global__ void __cluster_dims__(ROUTER_CL, 1, 1) __launch_bounds__(256) router_mma_kernel(
+constexpr int ROUTER_CL = 8;
+
+template <int MAXT, int WARPS>
+__global__ void __cluster_dims__(ROUTER_CL, 1, 1) __launch_bounds__(WARPS * 32) router_mma_kernel(
     const __half* __restrict__ x, const __half* __restrict__ w, int rows, int hidden, int experts,
     int has_shared, int top_k, int renorm, int* __restrict__ ids, float* __restrict__ probs,
     float* __restrict__ shared_gate) {
-  extern __shared__ float logits[];                 // [2][total]
-  __shared__ float part[8][ROUTER_ROWS][MAXT * 8 + 1];
+  constexpr int CL = ROUTER_CL, ROWS = 16, COLS = MAXT * 8 + 1, OWN = ROWS / CL;
+  extern __shared__ float router_smem[];
+  float(*part)[ROWS][COLS] = reinterpret_cast<float(*)[ROWS][COLS]>(router_smem);
+  float* logits = router_smem + WARPS * ROWS * COLS;              // [OWN][total]
   cg::cluster_group cluster = cg::this_cluster();
   const int crank = static_cast<int>(cluster.block_rank());
-  const int row0 = static_cast<int>(blockIdx.x) / ROUTER_CL * ROUTER_ROWS;
+  const int row0 = static_cast<int>(blockIdx.x) / CL * ROWS;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, g = lane >> 2, t = lane & 3;
   const int total = experts + (has_shared ? 1 : 0), tiles = (total + 7) / 8;
-  const int t_lo = tiles * crank / ROUTER_CL, nt = tiles * (crank + 1) / ROUTER_CL - t_lo;
+  const int t_lo = tiles * crank / CL, nt = tiles * (crank + 1) / CL - t_lo;
   float acc[MAXT][4];
 #pragma unroll
   for (int i = 0; i < MAXT; ++i)
@@ -125,8 +129,8 @@ __global__ void __cluster_dims__(ROUTER_CL, 1, 1) __launch_bounds__(256) router_
   // rows past the last token or expert read the last one; their sums are not used
   const __half* xa = x + static_cast<size_t>(min(row0 + g, rows - 1)) * hidden + t * 8;
   const __half* xb = x + static_cast<size_t>(min(row0 + g + 8, rows - 1)) * hidden + t * 8;
-  const int k_lo = hidden / 8 * warp, k_hi = hidden / 8 * (warp + 1);
-#pragma unroll 2
+  const int k_lo = hidden / WARPS * warp, k_hi = k_lo + hidden / WARPS;
+#pragma unroll(MAXT * WARPS > 72 ? 1 : 2)
   for (int k = k_lo; k < k_hi; k += 32) {
     const uint4 a = __ldg(reinterpret_cast<const uint4*>(xa + k));
     const uint4 b = __ldg(reinterpret_cast<const uint4*>(xb + k));
@@ -146,25 +150,43 @@ __global__ void __cluster_dims__(ROUTER_CL, 1, 1) __launch_bounds__(256) router_
   }
 #pragma unroll
   for (int i = 0; i < MAXT; ++i)
-    if (i < nt) {
-      part[warp][g][i * 8 + 2 * t] = acc[i][0];
-      part[warp][g][i * 8 + 2 * t + 1] = acc[i][1];
-      part[warp][g + 8][i * 8 + 2 * t] = acc[i][2];
-      part[warp][g + 8][i * 8 + 2 * t + 1] = acc[i][3];
-    }
+    if (i < nt)
+#pragma unroll
+      for (int e = 0; e < 4; ++e)
+        part[warp][g + (e >> 1) * 8][i * 8 + 2 * t + (e & 1)] = acc[i][e];
   cluster.sync();                                   // every CTA of the cluster runs
-  for (int i = threadIdx.x; i < ROUTER_ROWS * nt * 8; i += blockDim.x) {
+  for (int i = threadIdx.x; i < ROWS * nt * 8; i += WARPS * 32) {
     const int r = i / (nt * 8), c = i % (nt * 8), e = t_lo * 8 + c;
     float v = 0.f;
 #pragma unroll
-    for (int q = 0; q < 8; ++q) v += part[q][r][c];
-    if (e < total) cluster.map_shared_rank(logits, r >> 1)[(r & 1) * total + e] = v;
+    for (int q = 0; q < WARPS; ++q) v += part[q][r][c];
+    if (e < total) cluster.map_shared_rank(logits, r / OWN)[(r % OWN) * total + e] = v;
   }
   cluster.sync();
-  const int row = row0 + crank * 2 + warp;
-  if (warp < 2 && row < rows)
+  const int row = row0 + crank * OWN + warp;
+  if (warp < OWN && row < rows)
     topk_row(logits + warp * total, row, experts, has_shared, top_k, renorm, ids, probs,
              shared_gate);
+}
+
+template <int MAXT, int WARPS>
+static int launch_router(const __half* x, const __half* w, int rows, int hidden, int experts,
+                         int has_shared, int top_k, int renorm, int* ids, float* probs,
+                         float* shared_gate, cudaStream_t stream) {
+  const int total = experts + (has_shared ? 1 : 0);
+  constexpr int PART = WARPS * 16 * (MAXT * 8 + 1);
+  const size_t smem = (PART + 2 * static_cast<size_t>(total)) * sizeof(float);
+  static const int slot = runtime_new_slot();
+  if (runtime_first_use(slot)) {
+    const cudaError_t e = cudaFuncSetAttribute(router_mma_kernel<MAXT, WARPS>,
+                                               cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                               (PART + 2 * 8 * ROUTER_CL * MAXT) * sizeof(float));
+    if (e != cudaSuccess) return static_cast<int>(e);
+  }
+  const int grid = (rows + 15) / 16 * ROUTER_CL;
+  router_mma_kernel<MAXT, WARPS><<<grid, WARPS * 32, smem, stream>>>(
+      x, w, rows, hidden, experts, has_shared, top_k, renorm, ids, probs, shared_gate);
+  return static_cast<int>(cudaGetLastError());
 }
 
 // ---------------------------------------------------------------- slots
@@ -175,18 +197,21 @@ __global__ void __cluster_dims__(ROUTER_CL, 1, 1) __launch_bounds__(256) router_
 // offset[e] + rank of i among the assignments of e.  Under expert parallelism a rank owns
 // experts [base_expert, base_expert + gridDim.x): ids outside that range get slot -1 (CTA 0
 // writes those) and the combine skips them.
-__global__ void __launch_bounds__(256) moe_plan_kernel(
+// More threads where there are many assignments to walk (16384 of them: 26 us with 256).
+template <int THREADS>
+__global__ void __launch_bounds__(THREADS) moe_plan_kernel(
     const int* __restrict__ ids, int assigns, int base_expert, int* __restrict__ counts,
     int* __restrict__ offsets, int* __restrict__ tiles, int* __restrict__ meta, int max_tiles,
     int* __restrict__ slots) {
   extern __shared__ int hist[];                     // [experts]
-  __shared__ int red[2][8], warp_count[8];
+  constexpr int WARPS = THREADS / 32;
+  __shared__ int red[2][WARPS], warp_count[WARPS];
   const int e = blockIdx.x, experts = gridDim.x, tid = threadIdx.x;
   const int warp = tid >> 5, lane = tid & 31;
-  for (int i = tid; i < experts; i += 256) hist[i] = 0;
+  for (int i = tid; i < experts; i += THREADS) hist[i] = 0;
   __syncthreads();
   // a warp walks one contiguous run of assignments, 32 at a time
-  const int steps = (assigns + 255) / 256, lo = warp * steps * 32;
+  const int steps = (assigns + THREADS - 1) / THREADS, lo = warp * steps * 32;
   int mine = 0;
 #pragma unroll 4
   for (int s = 0; s < steps; ++s) {
@@ -200,7 +225,7 @@ __global__ void __launch_bounds__(256) moe_plan_kernel(
   if (lane == 0) warp_count[warp] = mine;
   __syncthreads();
   int rows_before = 0, tiles_before = 0;
-  for (int i = tid; i < e; i += 256) {
+  for (int i = tid; i < e; i += THREADS) {
     rows_before += hist[i];
     tiles_before += (hist[i] + 127) / 128;
   }
@@ -213,19 +238,19 @@ __global__ void __launch_bounds__(256) moe_plan_kernel(
   __syncthreads();
   int off = 0, tile0 = 0, slot = 0;
 #pragma unroll
-  for (int q = 0; q < 8; ++q) {
+  for (int q = 0; q < WARPS; ++q) {
     off += red[0][q];
     tile0 += red[1][q];
     if (q < warp) slot += warp_count[q];
   }
   const int count = hist[e], own_tiles = (count + 127) / 128;
-  for (int j = tid; j < own_tiles; j += 256)
+  for (int j = tid; j < own_tiles; j += THREADS)
     if (tile0 + j < max_tiles) {
       int* entry = tiles + static_cast<size_t>(tile0 + j) * 4;
       entry[0] = e;
       entry[1] = off + j * 128;
       entry[2] = min(128, count - j * 128);
-      entry[3] = 0;
+      entry[3] = j;
     }
   if (tid == 0) {
     counts[e] = count;
@@ -275,15 +300,24 @@ __global__ void __launch_bounds__(256) moe_combine_kernel(
   const int row = blockIdx.x;
   for (int i = threadIdx.x * 8; i < hidden; i += blockDim.x * 8) {
     float acc[8] = {0, 0, 0, 0, 0, 0, 0, 0};
-    for (int k = 0; k < top_k; ++k) {
-      const float p = probs[row * top_k + k];
-      const int slot = slots[row * top_k + k];
-      if (slot < 0) continue;                        // routed to an expert of another rank
-      const int4 raw =
-          *reinterpret_cast<const int4*>(expert_out + static_cast<size_t>(slot) * hidden + i);
-      const __half* h = reinterpret_cast<const __half*>(&raw);
+    // four expert rows in flight at a time; a slot of another rank counts as weight zero
+    for (int k0 = 0; k0 < top_k; k0 += 4) {
+      float p[4];
+      int4 raw[4];
 #pragma unroll
-      for (int j = 0; j < 8; ++j) acc[j] = fmaf(p, __half2float(h[j]), acc[j]);
+      for (int q = 0; q < 4; ++q) {
+        const int k = k0 + q, slot = k < top_k ? slots[row * top_k + k] : -1;
+        p[q] = slot >= 0 ? probs[row * top_k + k] : 0.f;
+        raw[q] = slot >= 0 ? *reinterpret_cast<const int4*>(
+                                 expert_out + static_cast<size_t>(slot) * hidden + i)
+                           : make_int4(0, 0, 0, 0);
+      }
+#pragma unroll
+      for (int q = 0; q < 4; ++q) {
+        const __half* h = reinterpret_cast<const __half*>(&raw[q]);
+#pragma unroll
+        for (int j = 0; j < 8; ++j) acc[j] = fmaf(p[q], __half2float(h[j]), acc[j]);
+      }
     }
     if (shared_out != nullptr) {
       const float g = shared_gate[row];
@@ -315,13 +349,14 @@ static int launch_dispatch(const int* ids, int rows, int top_k, int base_expert,
                            int* tiles, int* meta, int max_tiles, int* slots, int8_t* q8_sorted,
                            float* scale_sorted, cudaStream_t stream) {
   const size_t smem = static_cast<size_t>(experts) * sizeof(int);
+  auto kernel = rows * top_k >= 4096 ? moe_plan_kernel<1024> : moe_plan_kernel<256>;
   if (smem > 48 * 1024) {                           // more than 12 288 experts on one rank
     const cudaError_t e = cudaFuncSetAttribute(
-        moe_plan_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem));
+        kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem));
     if (e != cudaSuccess) return static_cast<int>(e);
   }
-  moe_plan_kernel<<<experts, 256, smem, stream>>>(ids, rows * top_k, base_expert, counts, offsets,
-                                                  tiles, meta, max_tiles, slots);
+  kernel<<<experts, rows * top_k >= 4096 ? 1024 : 256, smem, stream>>>(
+      ids, rows * top_k, base_expert, counts, offsets, tiles, meta, max_tiles, slots);
   if (q8 != nullptr)                                // nullptr: only the slot numbering is wanted
     moe_scatter_kernel<<<rows, 128, 0, stream>>>(slots, top_k, q8, scale, K, q8_sorted,
                                                  scale_sorted);
@@ -340,20 +375,26 @@ int orinfer_router_topk(const __half* x, const __half* w, int rows, int hidden, 
   if (rows <= 0) return 0;
   if (hidden % 8 || top_k < 1 || top_k > experts || experts > 4096) return -1;
   const int total = experts + (has_shared ? 1 : 0);
-  if (hidden % 256 == 0 && total <= ROUTER_CL * 8 * 9) {
-    const int grid = (rows + ROUTER_ROWS - 1) / ROUTER_ROWS * ROUTER_CL;
-    const size_t smem = 2 * static_cast<size_t>(total) * sizeof(float);
-    auto kernel = total <= ROUTER_CL * 8 * 3 ? router_mma_kernel<3> : router_mma_kernel<9>;
-    kernel<<<grid, 256, smem, stream>>>(x, w, rows, hidden, experts, has_shared, top_k, renorm, ids,
-                                        probs, shared_gate);
-    return static_cast<int>(cudaGetLastError());
+  if (hidden % 256 == 0 && total <= 8 * 8 * 9 && runtime_ensure_init() == cudaSuccess) {
+    // Wide routers read their matrix from few SMs in a decode step: more warps, more loads in
+    // flight (16 rows, 512 experts: 26 -> 16 us).
+#define ORINFER_ROUTER(MAXT, WARPS)                                                  \
+  return launch_router<MAXT, WARPS>(x, w, rows, hidden, experts, has_shared, top_k,  \
+                                            renorm, ids, probs, shared_gate, stream)
+    if (total > 8 * 8 * 3) {
+      if (hidden % 512 == 0) ORINFER_ROUTER(9, 16);
+      ORINFER_ROUTER(9, 8);
+    }
+    ORINFER_ROUTER(3, 8);
+#undef ORINFER_ROUTER
   }
   router_topk_kernel<<<rows, 256, (experts + 1) * sizeof(float), stream>>>(
       x, w, hidden, experts, has_shared, top_k, renorm, ids, probs, shared_gate);
   return static_cast<int>(cudaGetLastError());
 }
 
-// counts [E], offsets [E+1], tiles int32 [max_tiles,4] = (expert, first slot, rows, 0),
+// counts [E], offsets [E+1], tiles int32 [max_tiles,4] = (expert, first slot, rows,
+// number of the tile within its expert),
 // meta[0] = tile count, slots [rows*top_k]; q8_sorted / scale_sorted get the dispatched rows.
 int orinfer_moe_dispatch(const int* ids, int rows, int top_k, int experts, const int8_t* q8,
                          const float* scale, int K, int* counts, int* offsets, int* tiles,

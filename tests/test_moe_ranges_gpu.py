@@ -12,6 +12,25 @@ def dev(cuda):
     return cuda
 
 
+def _int_weight(fmt, n, k, g):
+    """(codes, FP16 scales, integer weights) of a random projection."""
+    from orinfer_b200.models.weights import QLinear
+    if fmt == "w8":
+        codes = torch.randint(-127, 128, (n, k), generator=g, dtype=torch.int8)
+    elif fmt == "q4":
+        codes = torch.randint(-2 ** 31, 2 ** 31, (k // 128, n, 16), generator=g, dtype=torch.int32)
+    else:
+        codes = torch.randint(-2 ** 15, 2 ** 15, (k // 128, n, 16), generator=g, dtype=torch.int16)
+    scale = (torch.rand(n, generator=g) * 0.01 + 1e-3).half()
+    return codes, scale, QLinear(fmt, n, k, codes, scale, None).integers()
+
+
+def _scaled(a, sa, w, ws):
+    """The integer product with its two FP32 scales, in the kernels' order."""
+    acc = (a.double() @ w.double().t()).float()
+    return (acc * ws.float()[None]) * sa.float()[:, None]
+
+
 @pytest.mark.parametrize("rows", [1, 15, 16, 17, 50])
 @pytest.mark.parametrize("hidden,experts,top_k,shared", [
     (256, 3, 2, False), (256, 64, 4, True), (512, 128, 8, False), (2048, 191, 8, True),
@@ -70,10 +89,40 @@ def test_moe_dispatch_numbers_and_copies(dev, experts, rows, top_k, k, part):
     assert torch.equal(sc.counts[:local].cpu().long(), counts)
     offs = torch.cat([torch.zeros(1, dtype=torch.int64), counts.cumsum(0)])
     assert torch.equal(sc.offsets[:local + 1].cpu().long(), offs)
-    tiles = [[e, int(offs[e]) + r, min(128, int(counts[e]) - r), 0]
+    tiles = [[e, int(offs[e]) + r, min(128, int(counts[e]) - r), r // 128]
              for e in range(local) for r in range(0, int(counts[e]), 128)]
     assert int(sc.meta[0]) == len(tiles)
     assert sc.tiles[:len(tiles)].cpu().tolist() == tiles
     src = order[:kept] // top_k
     assert torch.equal(sc.q8[:kept].cpu(), q8.cpu()[src])
     assert torch.equal(sc.scale[:kept].cpu(), scale.cpu()[src])
+
+
+# few rows per expert (small-M kernel, K shared by several warps or not), a tile of rows and
+# several tiles of rows per expert (one, two or four row tiles per CTA)
+@pytest.mark.parametrize("fmt", ["w8", "q4", "q2"])
+@pytest.mark.parametrize("counts", [[1, 0, 2, 7, 8, 9, 0, 1, 3, 0, 0, 0, 1, 1, 1, 1],
+                                    [0] * 30 + [16, 17, 33], [0] * 40 + [129] + [0] * 9,
+                                    [1, 1, 0, 1], [40, 0, 13, 1], [300, 0, 129, 128, 5, 256],
+                                    [513, 257, 300]])
+@pytest.mark.parametrize("n,k", [(128, 128), (384, 640), (256, 4096)])
+def test_grouped_projection_is_exact(dev, fmt, counts, n, k):
+    from orinfer_b200.ops import functional as F
+    experts, s = len(counts), sum(counts)
+    g = torch.Generator().manual_seed(s)
+    banks = [_int_weight(fmt, n, k, g) for _ in range(experts)]
+    a = torch.randint(-127, 128, (s, k), generator=g, dtype=torch.int8)
+    sa = torch.rand(s, generator=g) * 0.05 + 1e-3
+    ids = torch.tensor([e for e, c in enumerate(counts) for _ in range(c)], dtype=torch.int32)
+    sc = F.MoeScratch(s, 1, experts, k, 64, dev)
+    F.moe_dispatch(ids[:, None].to(dev), a.to(dev), sa.to(dev), experts, sc, s)
+    out = torch.full((s, n), float("nan"), dtype=torch.float16, device=dev)
+    F.qgemm_grouped(sc.q8, sc.scale, torch.stack([b[0] for b in banks]).to(dev),
+                    torch.stack([b[1] for b in banks]).to(dev), fmt, n, out, sc, s)
+    at = 0
+    for e, c in enumerate(counts):                       # the rows are in expert order already
+        if c:
+            want = _scaled(a[at:at + c].to(dev), sa[at:at + c].to(dev), banks[e][2].to(dev),
+                           banks[e][1].to(dev))
+            assert torch.equal(out[at:at + c], want.half()), e
+        at += c

@@ -1,0 +1,89 @@
+"""Projections and row preparation at the edges of their tiles."""
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.fixture(scope="module")
+def dev(cuda):
+    from orinfer_b200.ops import native
+    native.init()
+    return cuda
+
+
+def _int_weight(fmt, n, k, g):
+    """(codes, FP16 scales, integer weights) of a random projection."""
+    from orinfer_b200.models.weights import QLinear
+    if fmt == "w8":
+        codes = torch.randint(-127, 128, (n, k), generator=g, dtype=torch.int8)
+    elif fmt == "q4":
+        codes = torch.randint(-2 ** 31, 2 ** 31, (k // 128, n, 16), generator=g, dtype=torch.int32)
+    else:
+        codes = torch.randint(-2 ** 15, 2 ** 15, (k // 128, n, 16), generator=g, dtype=torch.int16)
+    scale = (torch.rand(n, generator=g) * 0.01 + 1e-3).half()
+    return codes, scale, QLinear(fmt, n, k, codes, scale, None).integers()
+
+
+def _scaled(a, sa, w, ws):
+    """The integer product with its two FP32 scales, in the kernels' order."""
+    acc = (a.double() @ w.double().t()).float()
+    return (acc * ws.float()[None]) * sa.float()[:, None]
+
+
+@pytest.mark.parametrize("fmt", ["w8", "q4", "q2"])
+@pytest.mark.parametrize("m", [1, 2, 3, 4, 5, 8])
+@pytest.mark.parametrize("n,k", [(8, 128), (24, 384), (16, 1152), (2560, 1024), (2376, 512),
+                                 (40000, 256)])
+def test_small_row_projections_are_exact(dev, fmt, m, n, k):
+    """Row groups of sixteen cut by N, single k-blocks, K splits and several groups per CTA."""
+    from orinfer_b200.ops import functional as F
+    g = torch.Generator().manual_seed(m * n + k)
+    codes, ws, w = _int_weight(fmt, n, k, g)
+    a = torch.randint(-127, 128, (m, k), generator=g, dtype=torch.int8)
+    sa = torch.rand(m, generator=g) * 0.05 + 1e-3
+    want = _scaled(a, sa, w, ws)
+    for f32 in (False, True):
+        out = F.qgemm(a.to(dev), sa.to(dev), codes.to(dev), ws.to(dev), fmt, n, out_f32=f32, path=1)
+        assert torch.equal(out.cpu(), want if f32 else want.half())
+
+
+@pytest.mark.parametrize("m,n", [(600, 19456), (1024, 19456), (2048, 2432), (1500, 6400)])
+def test_peeled_tail_tiles_are_exact(dev, m, n):
+    """Grids a few CTAs past a whole number of waves, M tiles cut by the last row."""
+    from orinfer_b200.ops import functional as F
+    g = torch.Generator().manual_seed(m)
+    codes, ws, w = _int_weight("q4", n, 1024, g)
+    a = torch.randint(-127, 128, (m, 1024), generator=g, dtype=torch.int8)
+    sa = torch.rand(m, generator=g) * 0.05 + 1e-3
+    out = F.qgemm(a.to(dev), sa.to(dev), codes.to(dev), ws.to(dev), "q4", n)
+    want = _scaled(a.to(dev), sa.to(dev), w.to(dev), ws.to(dev)).half()
+    assert torch.equal(out, want)
+
+
+@pytest.mark.parametrize("rows", [1, 7, 149, 300, 2049])
+@pytest.mark.parametrize("k", [128, 384, 768, 2176, 9728, 16384])
+@pytest.mark.parametrize("mode", ["norm", "plain", "swiglu", "bare"])
+def test_act_prep_row_splits(dev, rows, k, mode):
+    """Blocks of a row over one to 32 warps, uneven splits, against the torch statement: INT8
+    codes may differ by one where a value sits on a rounding boundary."""
+    from orinfer_b200.ops import functional as F
+    from orinfer_b200.ref import ops_ref as R
+    if rows * k > 1 << 23:
+        rows = (1 << 23) // k
+    g = torch.Generator(device=dev).manual_seed(rows + k)
+    x = torch.randn(rows, 2 * k if mode == "swiglu" else k, generator=g, device=dev).half()
+    signs = (1 - 2 * torch.randint(0, 2, (k,), generator=g, device=dev)).to(torch.int8)
+    resid = torch.randn(rows, k, generator=g, device=dev) if mode == "norm" else None
+    w = (1 + 0.1 * torch.randn(k, generator=g, device=dev)).half() if mode == "norm" else None
+    if mode == "bare":
+        signs = None
+    ref_q, ref_s, ref_r, ref_y = R.act_prep(x, resid, w, signs, swiglu=mode == "swiglu")
+    y = torch.empty(rows, k, dtype=torch.float16, device=dev)
+    q, s = F.act_prep(x, resid, w, signs, swiglu=mode == "swiglu", y_out=y)
+    diff = (q.int() - ref_q.int()).abs()
+    assert int(diff.max()) <= 1 and float((diff > 0).float().mean()) < 0.01
+    assert bool(((s - ref_s).abs() <= ref_s * 2.0 ** -10).all())      # one FP16 step
+    assert bool(((y.float() - ref_y).abs() <= ref_y.abs() * 2.0 ** -10 + 1e-7).all())
+    if resid is not None:
+        assert torch.equal(resid, ref_r)
