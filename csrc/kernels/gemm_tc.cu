@@ -64,12 +64,17 @@ struct Layout {
   static constexpr int SA_FIT = (BUDGET - SB * BC_BYTES) / A_BYTES;
   static constexpr int SA = SA_FIT >= 4 ? 4 : SA_FIT;
   static_assert(SA >= 2 && SB >= 2, "at least double buffering");
-  // as many copies of the decode tables as the rings leave room for: the lookups of a warp are
-  // random and collide about 3-fold with 4 copies, 1.5-fold with 16
+  // Copies of the decode tables: the lookups of a warp are random and collide about 3-fold with 4
+  // copies, 1.5-fold with 16.  Q4 looks up twice per code and gains where a CTA decodes wide tiles
+  // (19456 x 2560: 128 rows 33.6 -> 30.6 us, 2048 rows 128 -> 125 for the projection); Q2 and
+  // narrow tiles lose the time it takes to fill more copies (5120 x 2048, 512 rows, Q2: 25.0
+  // against 25.9 us), as do they all once the rings leave no room.
   static constexpr int RINGS = SA * A_BYTES + SB * BC_BYTES;
-  static constexpr int LUT_COPIES = RINGS + 32 * 1024 + 1280 <= 227 * 1024
-                                        ? 16
-                                        : (RINGS + 16 * 1024 + 1280 <= 227 * 1024 ? 8 : 4);
+  static constexpr int LUT_COPIES =
+      FMT != 1 || NB != 128 ? 4
+                            : (RINGS + 32 * 1024 + 1280 <= 227 * 1024
+                                   ? 16
+                                   : (RINGS + 16 * 1024 + 1280 <= 227 * 1024 ? 8 : 4));
   static constexpr int LUT_BYTES = FMT == 0 ? 0 : static_cast<int>(sizeof(E8pLut<LUT_COPIES>));
   static constexpr int A_OFF = 0;
   static constexpr int B_OFF = A_OFF + SA * A_BYTES;

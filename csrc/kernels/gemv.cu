@@ -210,8 +210,13 @@ __global__ void __launch_bounds__(GEMV_THREADS, 1) qgemv_kernel(
       ++lg;
     }
   };
+  // The first weights are requested before the tables are filled, except where the row
+  // preparation needs the registers, and by the dp4a form, which has none to spare (a spilled
+  // register costs every launch its local memory).
+  if (!DP4A && (FMT == 0 || fz.pre == 0)) {
 #pragma unroll
-  for (int i = 0; i < DEPTH; ++i) fetch(buf[i], u_lo + i);
+    for (int i = 0; i < DEPTH; ++i) fetch(buf[i], u_lo + i);
+  }
   if (FMT != 0) e8p_lut_init(lut, tables, tid, THREADS);
   for (int i = tid; i < max_groups * 16 * MT + MT; i += THREADS) acc_s[i] = 0;
   __syncthreads();
@@ -357,6 +362,10 @@ __global__ void __launch_bounds__(GEMV_THREADS, 1) qgemv_kernel(
   }
   __syncthreads();
 
+  if (DP4A || (FMT != 0 && fz.pre != 0)) {
+#pragma unroll
+    for (int i = 0; i < DEPTH; ++i) fetch(buf[i], u_lo + i);
+  }
   int acc[4] = {0, 0, 0, 0};
   const int copy = lane;                                   // GEMV_COPIES == 32
   for (int base = u_lo; base < u_hi; base += DEPTH) {
