@@ -77,8 +77,8 @@ __device__ __forceinline__ void mma_i8_16832(int (&c)[4], uint32_t a0, uint32_t 
 }
 
 // One or two rows of Q4 weights keep the dp4a form: an MMA spends eight columns on them, and
-// eight-row units divide more evenly over the warps (19456 x 2560, one row: 13.5 us against 14.9
-// with MMAs; from four rows on the MMAs win, 23.1 against 16.5 us at eight).  Lane l then holds
+// eight-row units divide more evenly over the warps (19456 x 2560, one row: 13.8 us against 14.9
+// with MMAs; at eight rows the MMAs win, 16.2 against 23.1 us).  Lane l then holds
 // row l / 4 of a group of eight and a quarter of the k-block.
 template <int FMT, int MT>
 struct GemvMode {
@@ -94,13 +94,13 @@ struct GemvUnit {
   uint32_t w[HALVES][WORDS];
 };
 
-// Position of channel k of activation row m in the staged activations (bytes).  dp4a: octets
-// in order, rows next to each other; E8P: octets ordered [k-block][octet % 4][octet / 4][row]; INT8 weights: 16-byte pieces ordered
+// Position of channel k of activation row m in the staged activations (bytes).  dp4a: rows
+// as they are (a warp reads four octets 32 bytes apart); E8P: octets ordered [k-block][octet % 4][octet / 4][row]; INT8 weights: 16-byte pieces ordered
 // [64 channels][row][piece], a lane's pieces being two steps each.
 template <int FMT, int MT>
-__device__ __forceinline__ int act_pos(int m, int k) {
+__device__ __forceinline__ int act_pos(int m, int k, int K) {
   if (FMT == 0) return ((k >> 6) * MT + m) * 64 + (k & 63);
-  if (GemvMode<FMT, MT>::DP4A) return ((k >> 3) * MT + m) * 8 + (k & 7);
+  if (GemvMode<FMT, MT>::DP4A) return m * K + k;
   const int o = (k >> 3) & 15;
   return (((k >> 7) * 16 + (o & 3) * 4 + (o >> 2)) * MT + m) * 8 + (k & 7);
 }
@@ -231,8 +231,8 @@ __global__ void __launch_bounds__(GEMV_THREADS, 1) qgemv_kernel(
       int4 v = make_int4(0, 0, 0, 0);
       if (m < M) v = *reinterpret_cast<const int4*>(a + static_cast<size_t>(c) * 16);
       const int k = c * 16 - m * K;
-      *reinterpret_cast<int2*>(act + act_pos<FMT, MT>(m, k)) = make_int2(v.x, v.y);
-      *reinterpret_cast<int2*>(act + act_pos<FMT, MT>(m, k + 8)) = make_int2(v.z, v.w);
+      *reinterpret_cast<int2*>(act + act_pos<FMT, MT>(m, k, K)) = make_int2(v.x, v.y);
+      *reinterpret_cast<int2*>(act + act_pos<FMT, MT>(m, k + 8, K)) = make_int2(v.z, v.w);
       int s = __dp4a(v.x, 0x01010101, 0);
       s = __dp4a(v.y, 0x01010101, s);
       s = __dp4a(v.z, 0x01010101, s);
@@ -345,7 +345,7 @@ __global__ void __launch_bounds__(GEMV_THREADS, 1) qgemv_kernel(
         c.y = static_cast<signed char>(a8_code(fb[i + 1], scale));
         c.z = static_cast<signed char>(a8_code(fb[i + 2], scale));
         c.w = static_cast<signed char>(a8_code(fb[i + 3], scale));
-        *reinterpret_cast<char4*>(act + act_pos<FMT, MT>(m, i)) = c;
+        *reinterpret_cast<char4*>(act + act_pos<FMT, MT>(m, i, K)) = c;
         if (fz.q_out != nullptr && first_cta)
           *reinterpret_cast<char4*>(fz.q_out + static_cast<size_t>(m) * K + i) = c;
         psum = __dp4a(*reinterpret_cast<const int*>(&c), 0x01010101, psum);
@@ -386,7 +386,7 @@ __global__ void __launch_bounds__(GEMV_THREADS, 1) qgemv_kernel(
 #pragma unroll
             for (int m = 0; m < MT && m < 2; ++m) {
               const int2 av =
-                  *reinterpret_cast<const int2*>(act + ((ckb * 16 + t * 4 + j) * MT + m) * 8);
+                  *reinterpret_cast<const int2*>(act + m * K + (ckb * 16 + t * 4 + j) * 8);
               acc[m] = __dp4a(xhi, av.y, __dp4a(xlo, av.x, acc[m]));
             }
           }
@@ -395,7 +395,7 @@ __global__ void __launch_bounds__(GEMV_THREADS, 1) qgemv_kernel(
           for (int j = 0; j < 2; ++j) {
             int4 b = make_int4(0, 0, 0, 0);
             if (g < MT)
-              b = *reinterpret_cast<const int4*>(act + act_pos<FMT, MT>(g, ckb * 128 + j * 64 + t * 16));
+              b = *reinterpret_cast<const int4*>(act + act_pos<FMT, MT>(g, ckb * 128 + j * 64 + t * 16, K));
             const uint32_t* r0 = buf[i].w[0] + (j * 4) % Unit::WORDS;
             const uint32_t* r1 = buf[i].w[HALVES - 1] + (j * 4) % Unit::WORDS;
             mma_i8_16832(acc, r0[0], r1[0], r0[1], r1[1], b.x, b.y);
