@@ -7,23 +7,24 @@
 // ones for head sizes 64 and 128, so that a dequantised page serves 256 rows and the tensor core
 // works on one tile while the softmax warps of the other are busy.  Per step of KT keys:
 //   * eight warps, in two groups that take the steps in turn, read the INT8 page and its
-//     group-64 FP16 scales straight from global memory (ahead, in registers), dequantise to FP16 and store K and V as
-//     128-byte-swizzled tiles (K is the K-major B operand of S = Q K^T, V the MN-major B
-//     operand of O += P V);
+//     group-64 FP16 scales straight from global memory (ahead, in registers), dequantise to
+//     FP16 and store K and V as 128-byte-swizzled tiles (K is the K-major B operand of
+//     S = Q K^T, V the MN-major B operand of O += P V);
 //   * warp 1 issues tcgen05.mma kind::f16: S (128 x KT fp32) and O (128 x D fp32) live in TMEM;
 //   * four warps per tile own one query row per thread: they read S from TMEM, apply scale and
 //     the causal mask, and write P as FP16 over S in TMEM, where the second MMA reads it as its
-//     A operand.  The reference maximum of a row only moves when a score exceeds it by 2^8 (P
-//     stays below 256 and the sums in FP32), so rescaling O is rare after the first steps;
+//     A operand.  P is relative to the row's running maximum, so its largest weight is exactly 1
+//     and O is rescaled whenever a row of the warp finds a larger score;
 //   * warp 0 loads the Q tiles once with a 3-D TMA (d, head, position).
 // Head size 256 has room for one tile (Q 64 KB, two K and two V buffers of 32 KB; TMEM: two S of
 // 64 columns and O of 256) and walks the cache in half pages, with S double buffered instead.
 // CTAs are ordered from the last query positions (the longest walks) to the first.
 //
-// One 4096-token chunk, 32 / 8 heads of 128: 385 us with one tile per CTA and P in shared memory,
-// 220 us now (625 TFLOP/s causal); of that 158 us remain with the softmax and the conversions
-// switched off, the issue chain of 128 x 128 MMAs.  Chunks of 777 and 646 rows behind 3000
-// positions, 16 / 2 gated heads of 256: 373 -> 279 us (180 CTAs: 1.2 waves).
+// One 4096-token chunk, 32 / 8 heads of 128: 377 us with one tile per CTA and P in shared memory,
+// 242 us now (568 TFLOP/s causal).  A reference that follows the maximum only when it lags by
+// 2^8 takes 215 us (fewer rescales of O) but rounds the largest weights in FP16: the error
+// against 64 bits grows by 1.8 % there and by 3.7 % for 500 rows behind 1000.  Chunks of 777 and
+// 646 rows behind 3000 positions, 16 / 2 gated heads of 256: 354 -> 274 us (180 CTAs: 1.2 waves).
 // Output is O / sum, optionally times sigmoid(gate), in FP16.  Replaces the prefill
 // configurations of causal_attention_int8 and dequantize_attention_kv
 // (kernels/cuda/model/attention_rows.py:61-276, kernels/cuda/model/kv_int8.py:210-247).
@@ -311,7 +312,7 @@ __global__ void __launch_bounds__(Smem<D>::THREADS, 1) attn_prefill_kernel(
     const uint32_t lane_addr = static_cast<uint32_t>(quad * 32) << 16;
     const uint32_t tmem_oq = tmem_o + 128 * q + lane_addr;
     const int steps = NQ == 2 && q == 1 ? n_steps[NQ - 1] : n_steps[0];
-    float m_ref = -INFINITY, l_run = 0.f;
+    float m_run = -INFINITY, l_run = 0.f;
     bool ok = true;
     for (int j = 0; j < steps; ++j) {
       const int sb = NQ == 2 ? q : j & 1;
@@ -356,29 +357,22 @@ __global__ void __launch_bounds__(Smem<D>::THREADS, 1) attn_prefill_kernel(
         if (!ok) break;
         tc_fence_after();
       }
-      // the reference moves when a score is above it by more than 2^8 (or it has none yet)
-      const bool moves = m_tile > m_ref + 8.f || (m_ref == -INFINITY && m_tile > -INFINITY);
-      if (__any_sync(0xffffffffu, moves)) {
-        const float m_new = moves ? m_tile : m_ref;
-        const float corr = moves ? (m_ref == -INFINITY ? 0.f : ex2(m_ref - m_new)) : 1.f;
-        m_ref = m_new;
-        l_run *= corr;
-        if (j >= 1) {
+      const float m_new = fmaxf(m_run, m_tile);
+      const float corr = m_new == -INFINITY ? 1.f : ex2(m_run - m_new);
+      if (j >= 1 && !__all_sync(0xffffffffu, corr == 1.f)) {
 #pragma unroll 1
-          for (int c0 = 0; c0 < D; c0 += 32) {
-            uint32_t r[32];
-            tmem_ld_32x32(tmem_oq + c0, r);
-            tc_wait_ld();
+        for (int c0 = 0; c0 < D; c0 += 32) {
+          uint32_t r[32];
+          tmem_ld_32x32(tmem_oq + c0, r);
+          tc_wait_ld();
 #pragma unroll
-            for (int i = 0; i < 32; ++i) r[i] = __float_as_uint(__uint_as_float(r[i]) * corr);
-            tmem_st_32x32(tmem_oq + c0, r);
-          }
-          tc_wait_st();
+          for (int i = 0; i < 32; ++i) r[i] = __float_as_uint(__uint_as_float(r[i]) * corr);
+          tmem_st_32x32(tmem_oq + c0, r);
         }
+        tc_wait_st();
       }
       // pass 2: probabilities -> FP16 over the scores already read, row sum
-      const float m_use = m_ref == -INFINITY ? 0.f : m_ref;
-      float l0 = 0.f, l1 = 0.f;
+      float l_tile = 0.f;
 #pragma unroll 1
       for (int c0 = 0; c0 < KT; c0 += 64) {
         uint32_t packed[32];
@@ -390,22 +384,20 @@ __global__ void __launch_bounds__(Smem<D>::THREADS, 1) attn_prefill_kernel(
           if (full_warp) {
 #pragma unroll
             for (int i = 0; i < 32; i += 2) {
-              const float p0 = ex2(fmaf(__uint_as_float(r[i]), scale, -m_use));
-              const float p1 = ex2(fmaf(__uint_as_float(r[i + 1]), scale, -m_use));
-              l0 += p0;
-              l1 += p1;
+              const float p0 = ex2(fmaf(__uint_as_float(r[i]), scale, -m_new));
+              const float p1 = ex2(fmaf(__uint_as_float(r[i + 1]), scale, -m_new));
+              l_tile += p0 + p1;
               const __half2 hp = __floats2half2_rn(p0, p1);
               packed[hf * 16 + i / 2] = *reinterpret_cast<const uint32_t*>(&hp);
             }
           } else {
 #pragma unroll
             for (int i = 0; i < 32; i += 2) {
-              float p0 = ex2(fmaf(__uint_as_float(r[i]), scale, -m_use));
-              float p1 = ex2(fmaf(__uint_as_float(r[i + 1]), scale, -m_use));
+              float p0 = ex2(fmaf(__uint_as_float(r[i]), scale, -m_new));
+              float p1 = ex2(fmaf(__uint_as_float(r[i + 1]), scale, -m_new));
               if (key0 + c0 + hf * 32 + i > q_pos) p0 = 0.f;
               if (key0 + c0 + hf * 32 + i + 1 > q_pos) p1 = 0.f;
-              l0 += p0;
-              l1 += p1;
+              l_tile += p0 + p1;
               const __half2 hp = __floats2half2_rn(p0, p1);
               packed[hf * 16 + i / 2] = *reinterpret_cast<const uint32_t*>(&hp);
             }
@@ -414,7 +406,8 @@ __global__ void __launch_bounds__(Smem<D>::THREADS, 1) attn_prefill_kernel(
         tmem_st_32x32(tmem_sj + c0 / 2, packed);
       }
       tc_wait_st();
-      l_run += l0 + l1;
+      l_run = l_run * corr + l_tile;
+      m_run = m_new;
       tc_fence_before();
       mbar_arrive(&p_ready[sb]);
     }

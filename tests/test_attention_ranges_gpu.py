@@ -121,3 +121,36 @@ def test_attention_prefill_at_tile_edges(dev, qh, kvh, d, gated, spec):
             # FP16 keys, values and weights (2^-11 each, scores up to about 20): 2^-8 of the
             # largest value
             assert float((got - ref).abs().max()) <= 2.0 ** -8 * float(ref.abs().max()), (n, p, r)
+
+
+@pytest.mark.parametrize("d,kvh,qh", [(64, 2, 4), (128, 1, 5), (256, 1, 8)])
+@pytest.mark.parametrize("rows", [40, 300])
+def test_attention_prefill_largest_weight_is_exact(dev, d, kvh, qh, rows):
+    """A late key that dominates by up to 2^8, the only one with a value: its weight is the row's
+    largest, 1 in FP16 whatever the earlier pages held, so only the output is rounded."""
+    from orinfer_b200.ops import functional as F
+    g = torch.Generator().manual_seed(d + rows)
+    past, peak = 300, 270
+    pages = (rows + past + 127) // 128
+    kc = torch.zeros(pages + 1, 128, kvh, d, dtype=torch.int8)
+    vc = torch.zeros_like(kc)
+    table = torch.arange(1, pages + 1, dtype=torch.int32)[None]
+    kc[1:, :, :, 0] = torch.randint(0, 60, (pages, 128, kvh), generator=g, dtype=torch.int8)
+    kc[1 + peak // 128, peak % 128, :, 0] = 127
+    vc[1 + peak // 128, peak % 128] = torch.randint(20, 127, (kvh, d), generator=g, dtype=torch.int8)
+    scale = lambda v: torch.full((pages + 1, 128, kvh, d // 64), v, dtype=torch.float16, device=dev)
+    q = torch.zeros(rows, qh, d)
+    # the peak is above the others by 2^0.5 .. 2^8 of the softmax weight
+    q[:, :, 0] = torch.linspace(0.5, 8, rows * qh).reshape(rows, qh) * math.sqrt(d) * math.log(2) * 127 / 67
+    q = q.half().to(dev)
+    kc, vc, ks, vs = kc.to(dev), vc.to(dev), scale(1 / 128), scale(1 / 64)
+    out = torch.empty(rows, qh * d, dtype=torch.float16, device=dev)
+    chunk = torch.tensor([[0, rows, past, 0]], dtype=torch.int32, device=dev)
+    assert F.attention_prefill(q, None, chunk, rows, table.to(dev), kc, vc, ks, vs, out=out)
+    flat = lambda c: c[1:].reshape(-1, *c.shape[2:])
+    for r in range(rows):
+        n = past + r + 1
+        ref = _attention64(q[r], flat(kc)[:n], flat(vc)[:n], flat(ks)[:n], flat(vs)[:n]).reshape(-1)
+        # one FP16 rounding of the output (2^-11); scores of up to 2^4 in FP32, a sum of up to 600
+        # FP32 weights and their exponentials: below 2^-17
+        assert bool(((out[r].double() - ref).abs() <= ref.abs() * (2.0 ** -11 + 2.0 ** -17)).all()), r
