@@ -470,15 +470,11 @@ __device__ __forceinline__ float block_reduce(float v, float* red, bool is_max) 
   return r;
 }
 
-// 1 / (1 + e^-x) by the hardware exponential and reciprocal: within a few 2^-22, ahead of a
-// rounding to FP16 everywhere it is used.  The correctly rounded forms were a third of the
-// instructions of the SwiGLU rows.
-__device__ __forceinline__ float sigmoid_f32(float x) {
-  float e, r;
-  asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(e) : "f"(x * -1.4426950408889634f));
-  asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(1.f + e));
-  return r;
-}
+// 1 / (1 + e^-x) with the accurate exponential and a correctly rounded reciprocal (the bits of
+// the division 1 / y, without its scaling of the numerator).  The hardware forms (ex2.approx of
+// the rounded product x log2 e, rcp.approx) are faster, but their relative error grows with |x|:
+// 2^-18 at x = -40, against 2^-22 here.
+__device__ __forceinline__ float sigmoid_f32(float x) { return __frcp_rn(1.f + expf(-x)); }
 
 // Signed block-128 Hadamard rotation of one block held as floats, in place: lane l holds
 // channels 4l..4l+3.  Returns the largest magnitude of the lane's four results.  Shared by

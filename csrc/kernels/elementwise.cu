@@ -261,10 +261,17 @@ __global__ void __launch_bounds__(512) act_prep_kernel(
 // between barriers.  Same helpers and the same order of operations as act_prep_kernel, so a row
 // gives the same bits through either.  Few rows take many warps each (latency), thousands of
 // rows four blocks per warp (instructions per row).  512 rows x 2560 9.0 -> 6.1 us, SwiGLU 512 x
-// 9728 18.6 -> 13.1, eight rows 6.5 -> 3.1 (a cluster of eight CTAs per row before), 16384 rows x
-// 768 SwiGLU 51 -> 27.5, 2048 rows x 2048 20.5 -> 15.8 (a warp per row before).
+// 9728 18.0 -> 14.6, eight rows 7.1 -> 3.1 (a cluster of eight CTAs per row before), 8192 rows x
+// 768 SwiGLU 24.0 -> 16.6, 2048 rows x 2048 18.3 -> 12.9 (a warp per row before).
+// Five to eight blocks: two CTAs of 512 threads fit an SM (SwiGLU 512 x 16384: 23 us, 31 with 73
+// registers and one CTA).
+template <int NB>
+struct RegRows {
+  static constexpr int THREADS = NB <= 4 ? 1024 : 512;
+  static constexpr int CTAS = NB > 4 && NB <= 8 ? 2 : 1;
+};
 template <bool SWIGLU, int NB>
-__global__ void __launch_bounds__(NB <= 4 ? 1024 : 512) act_prep_regs_kernel(
+__global__ void __launch_bounds__(RegRows<NB>::THREADS, RegRows<NB>::CTAS) act_prep_regs_kernel(
     const __half* __restrict__ x, float* __restrict__ resid, const __half* __restrict__ norm_w,
     const int8_t* __restrict__ signs, int8_t* __restrict__ q_out, float* __restrict__ scale_out,
     __half* __restrict__ y_out, int nblk, float eps, int zero_centered,

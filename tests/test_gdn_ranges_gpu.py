@@ -133,3 +133,22 @@ def test_gdn_gated_norm_forms_agree(dev, d, rows, hv):
             ref = oo * torch.rsqrt((oo * oo).mean(-1, keepdim=True) + 1e-6) * w.double() * gate
             lim = ref.reshape(rows, -1).abs() * 2.0 ** -10 + 1e-7
             assert bool(((y.double() - ref.reshape(rows, -1)).abs() <= lim).all())
+
+
+@pytest.mark.parametrize("d", [64, 128])
+def test_gdn_gated_norm_sigmoid_keeps_fp32_accuracy(dev, d):
+    """Rows whose norm is exactly one, strongly negative gates and large weights: only the sigmoid
+    and its product stand under the FP16 rounding."""
+    from orinfer_b200.ops import functional as F
+    torch.manual_seed(d)
+    rows, hv = 4000, 8
+    o = torch.full((rows, hv, d), 4.0, device=dev)
+    z = (-19 + 4 * torch.rand(rows, hv * d, device=dev)).half()
+    w = (2e4 + 4e4 * torch.rand(d, device=dev)).half()      # products above the subnormals
+    for form in (z, _unaligned(z)):
+        y = F.gdn_gated_norm(o, form, w, 0.0, rows, hv, d, sigmoid_gate=True).double()
+        ref = (torch.sigmoid(z.double().reshape(rows, hv, d)) * w.double()).reshape(rows, -1)
+        half_ulp = torch.exp2(torch.floor(torch.log2(ref)) - 11)
+        # e^-x within one step (2^-23), then a sum, a reciprocal and a product (2^-24 each); the
+        # square root's reciprocal of a power of two within one step
+        assert bool(((y - ref).abs() <= half_ulp + ref * 3.5 * 2.0 ** -23).all())

@@ -87,3 +87,26 @@ def test_act_prep_row_splits(dev, rows, k, mode):
     assert bool(((y.float() - ref_y).abs() <= ref_y.abs() * 2.0 ** -10 + 1e-7).all())
     if resid is not None:
         assert torch.equal(resid, ref_r)
+
+
+@pytest.mark.parametrize("rows,k,fused", [(300, 4096, False), (8, 16384, False), (8, 4096, True)])
+def test_swiglu_sigmoid_keeps_fp32_accuracy(dev, rows, k, fused):
+    """Strongly negative gates times large values: the FP32 product under the FP16 rounding."""
+    from orinfer_b200.ops import functional as F
+    g = torch.Generator(device=dev).manual_seed(k)
+    y = torch.empty(rows, k, dtype=torch.float16, device=dev)
+    for _ in range(8 if rows > 8 else 60):
+        gate = -21 + 6 * torch.rand(rows, k, generator=g, device=dev)
+        x = torch.cat([gate, 2e4 + 4e4 * torch.rand(rows, k, generator=g, device=dev)], 1).half()
+        if fused:
+            codes, ws, _ = _int_weight("q4", 8, k, torch.Generator().manual_seed(1))
+            assert F.qgemv_fused(F.PRE_SWIGLU, x, None, None, None, codes.to(dev), ws.to(dev), "q4",
+                                 8, k, rows, y_out=y,
+                                 out=torch.empty(rows, 8, dtype=torch.float16, device=dev))
+        else:
+            F.act_prep(x, None, None, None, swiglu=True, y_out=y)
+        a, u = x.double().chunk(2, 1)
+        ref = a * torch.sigmoid(a) * u
+        half_ulp = torch.exp2(torch.floor(torch.log2(ref.abs())) - 11)
+        # e^-x within one step (2^-23), then a sum, a reciprocal and two products (2^-24 each)
+        assert bool(((y.double() - ref).abs() <= half_ulp + ref.abs() * 3 * 2.0 ** -23).all())
