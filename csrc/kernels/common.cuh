@@ -536,9 +536,14 @@ __device__ __forceinline__ float a8_scale(float amax) {
   if (!(amax > 0.f)) return 1.f;
   return round_f16(fmaxf(__fdiv_rn(amax, 127.f), 5.9604644775390625e-08f));
 }
-// round(v / scale) to the nearest even integer, clamped to +-127.  The quotient by the reciprocal
-// is within 2^-22 of v / scale, so both round alike unless it lies that close to half an integer
-// (|q| <= 128: 1e-4 is ample); only then is the division carried out.
+// round(v / scale) to the nearest even integer, clamped to +-127
+__device__ __forceinline__ int a8_code_div(float v, float scale) {
+  const float r = rintf(__fdiv_rn(v, scale));
+  return static_cast<int>(fminf(127.f, fmaxf(-127.f, r)));
+}
+// The same code by the reciprocal of the scale.  That quotient is within 2^-22 of v / scale, so
+// both round alike unless it lies that close to half an integer (|q| <= 128: 1e-4 is ample);
+// only then is the division carried out.
 __device__ __forceinline__ int a8_code_inv(float v, float scale, float inv) {
   const float q = v * inv;
   float r = rintf(q);

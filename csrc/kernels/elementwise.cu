@@ -59,6 +59,14 @@ __device__ __forceinline__ float cluster_reduce(float v, float* slot, bool is_ma
   return r;
 }
 
+// A row over a cluster leaves a thread one or two values, where the division is quicker than
+// the reciprocal and the test for a tie (SwiGLU 1 x 9728: 4.2 against 4.3 us); whole rows per CTA
+// divide many by one scale (512 x 9728: 16.5 against 14.6 us).  Same codes.
+template <int CL>
+__device__ __forceinline__ int a8_code_of(float v, float scale) {
+  return CL > 1 ? a8_code_div(v, scale) : a8_code(v, scale);
+}
+
 template <bool SWIGLU, int CL>
 __global__ void __launch_bounds__(512) act_prep_kernel(
     const __half* __restrict__ x, float* __restrict__ resid, const __half* __restrict__ norm_w,
@@ -229,7 +237,7 @@ __global__ void __launch_bounds__(512) act_prep_kernel(
     for (int i = k_lo + tid * 16; i < k_hi; i += blockDim.x * 16) {
       __align__(16) signed char c[16];
 #pragma unroll
-      for (int j = 0; j < 16; ++j) c[j] = static_cast<signed char>(a8_code(rowbuf[i + j], scale));
+      for (int j = 0; j < 16; ++j) c[j] = static_cast<signed char>(a8_code_of<CL>(rowbuf[i + j], scale));
       for (int d = 0; d < ag.tp; ++d)
         *reinterpret_cast<int4*>(ag.q[d] + static_cast<size_t>(row) * K + i) =
             *reinterpret_cast<const int4*>(c);
@@ -242,10 +250,10 @@ __global__ void __launch_bounds__(512) act_prep_kernel(
   int8_t* qr = q_out + static_cast<size_t>(row) * K;
   for (int i = k_lo + tid * 4; i < k_hi; i += blockDim.x * 4) {
     char4 c;
-    c.x = static_cast<signed char>(a8_code(rowbuf[i + 0], scale));
-    c.y = static_cast<signed char>(a8_code(rowbuf[i + 1], scale));
-    c.z = static_cast<signed char>(a8_code(rowbuf[i + 2], scale));
-    c.w = static_cast<signed char>(a8_code(rowbuf[i + 3], scale));
+    c.x = static_cast<signed char>(a8_code_of<CL>(rowbuf[i + 0], scale));
+    c.y = static_cast<signed char>(a8_code_of<CL>(rowbuf[i + 1], scale));
+    c.z = static_cast<signed char>(a8_code_of<CL>(rowbuf[i + 2], scale));
+    c.w = static_cast<signed char>(a8_code_of<CL>(rowbuf[i + 3], scale));
     *reinterpret_cast<char4*>(qr + i) = c;
   }
   if (!SWIGLU && (in.inbox != nullptr || in.ll != nullptr)) inbox_consumed(in, gridDim.x);
@@ -260,9 +268,10 @@ __global__ void __launch_bounds__(512) act_prep_kernel(
 // instead of at every phase; the first form kept the row in shared memory and spent its time
 // between barriers.  Same helpers and the same order of operations as act_prep_kernel, so a row
 // gives the same bits through either.  Few rows take many warps each (latency), thousands of
-// rows four blocks per warp (instructions per row).  512 rows x 2560 9.0 -> 6.1 us, SwiGLU 512 x
-// 9728 18.0 -> 14.6, eight rows 7.1 -> 3.1 (a cluster of eight CTAs per row before), 8192 rows x
-// 768 SwiGLU 24.0 -> 16.6, 2048 rows x 2048 18.3 -> 12.9 (a warp per row before).
+// rows four blocks per warp (instructions per row); short rows one up to 1024 rows (SwiGLU 512 x
+// 768: 3.0 us, two blocks per warp 3.6).  512 rows x 2560 9.0 -> 6.1 us, SwiGLU 512 x 9728
+// 18.0 -> 14.6, eight rows 7.1 -> 3.1 (a cluster of eight CTAs per row before), 8192 rows x 768
+// SwiGLU 24.0 -> 16.6, 2048 rows x 2048 18.3 -> 12.9 (a warp per row before).
 // Five to eight blocks: two CTAs of 512 threads fit an SM (SwiGLU 512 x 16384: 23 us, 31 with 73
 // registers and one CTA).
 template <int NB>
@@ -683,10 +692,19 @@ static int act_prep_launch(const __half* x, float* resid, const __half* norm_w, 
                          200 * 1024);
   }
   if (smem > 200 * 1024) return -1;
-  if (ag.tp == 0 && in.inbox == nullptr && in.ll == nullptr && row_base == 0 &&
+  // One row keeps a single SM busy, so a cluster of CTAs shares each of a few rows (decode
+  // steps): the inbox forms, and rows too wide for one block per warp.  SwiGLU 1 x 8192 3.4 us
+  // against 4.2 in one CTA, 1 x 16384 4.2 against 7.2, plain 1 x 16384 4.1 against 5.6; at 4096
+  // channels one CTA is quicker (3.1 against 3.6), as it is for normalised rows, which need one
+  // more exchange (1 x 9728: 6.3 against 9.0).  Not for the sequence-parallel and count-limited
+  // forms, whose CTAs may leave early.
+  constexpr int CL = 8;
+  const bool clustered = rows <= 16 && ag.tp == 0 && row_limit == nullptr && K / 128 >= CL;
+  const bool spread = clustered && norm_w == nullptr && K / 128 > 48;
+  if (!spread && ag.tp == 0 && in.inbox == nullptr && in.ll == nullptr && row_base == 0 &&
       q_out != nullptr && scale_out != nullptr && K / 128 <= 16 * 16) {
     const int nblk = K / 128;
-    const int aim = rows >= 2048 ? 4 : (rows >= 256 ? 2 : 1);        // blocks per warp
+    const int aim = rows >= 2048 ? 4 : (rows >= (nblk > 8 ? 256 : 1024) ? 2 : 1);  // per warp
     const int most = rows <= 148 ? 32 : 16;                          // warps per row
     int warps = (nblk + aim - 1) / aim;
     warps = warps > most ? most : warps;
@@ -704,11 +722,7 @@ static int act_prep_launch(const __half* x, float* resid, const __half* norm_w, 
     REG_ROWS(12) REG_ROWS(16)
 #undef REG_ROWS
   }
-  // Inbox forms of a few rows (decode steps under tensor parallelism): one row would keep a
-  // single SM busy, so a cluster of CTAs shares each row.  Not for the sequence-parallel and
-  // count-limited forms, whose CTAs may leave early.
-  constexpr int CL = 8;
-  if (rows <= 16 && ag.tp == 0 && row_limit == nullptr && K / 128 >= CL && !swiglu) {
+  if (clustered) {
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3(rows * CL);
     cfg.blockDim = dim3(256);
@@ -723,10 +737,18 @@ static int act_prep_launch(const __half* x, float* resid, const __half* norm_w, 
     cfg.numAttrs = 1;
     const AgOut no_ag{};
     const int* no_limit = nullptr;
-    const cudaError_t e =
-        cudaLaunchKernelEx(&cfg, act_prep_kernel<false, CL>, x, resid, norm_w, signs, q_out,
-                           scale_out, y_out, K, eps, zero_centered, in, status, no_ag, rows,
-                           no_limit, row_base);
+    cudaError_t e;
+    if (swiglu) {
+      float* no_resid = nullptr;
+      const __half* no_norm = nullptr;
+      e = cudaLaunchKernelEx(&cfg, act_prep_kernel<true, CL>, x, no_resid, no_norm, signs, q_out,
+                             scale_out, y_out, K, eps, zero_centered, in, status, no_ag, rows,
+                             no_limit, 0);
+    } else {
+      e = cudaLaunchKernelEx(&cfg, act_prep_kernel<false, CL>, x, resid, norm_w, signs, q_out,
+                             scale_out, y_out, K, eps, zero_centered, in, status, no_ag, rows,
+                             no_limit, row_base);
+    }
     return static_cast<int>(e != cudaSuccess ? e : cudaGetLastError());
   }
   // SwiGLU rows are wide and spend their time in exp / divide: more threads per row

@@ -62,7 +62,7 @@ def test_peeled_tail_tiles_are_exact(dev, m, n):
 
 
 @pytest.mark.parametrize("rows", [1, 7, 149, 300, 2049])
-@pytest.mark.parametrize("k", [128, 384, 768, 2176, 9728, 16384])
+@pytest.mark.parametrize("k", [128, 384, 768, 2176, 6144, 6272, 9728, 16384])
 @pytest.mark.parametrize("mode", ["norm", "plain", "swiglu", "bare"])
 def test_act_prep_row_splits(dev, rows, k, mode):
     """Blocks of a row over one to 32 warps, uneven splits, against the torch statement: INT8
