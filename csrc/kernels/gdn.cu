@@ -489,21 +489,28 @@ __global__ void __launch_bounds__(256) gdn_scan_split_kernel(
 // waits for another inside a chunk.  Warps 4 (A, T) and 5 (P) prepare the next chunk, which
 // does not depend on the state, while the chunk after that is copied in.
 //
-// Precision: k, q and v are FP16 and enter products exactly; FP32 operands are split in two
-// (FP16 halves under a power-of-two scale: 22 bits; TF32 pairs: 22 bits) and all sums are FP32.
-// The G are summed in FP64 and subtracted as FP32 pairs, so that e^(G_i - G_j) keeps FP32 accuracy
-// when |G| is large.
+// Precision: k, q and v are FP16 and enter products exactly.  FP32 operands are split: S into
+// FP16 halves under a power-of-two scale per value channel, Delta for the state update into three
+// FP16 parts, T and P off the diagonal into TF32 pairs; their diagonals, which carry most of the
+// sums, are multiplied in FP32.  A tensor-core sum is cut off, not rounded, so each holds 32
+// products at most and is added to the others by FP32 additions.  The G are summed in FP64 and
+// subtracted as FP32 pairs, so that e^(G_i - G_j) keeps FP32 accuracy when |G| is large.
+// Relative error against 64 bits, one run of 1050 rows: output 1.7e-7, state 1.1e-7 (the scan:
+// 1.8e-7 and 1.3e-7; chained tensor-core sums of whole rows: 4.4e-7); with a memory of thousands
+// of rows 2.0e-7 and 1.5e-7 (the scan, which rounds at every step: 1.9e-6 and 2.1e-6); with decays
+// below 1/2 a row 1.6e-7 and 1.1e-7 (1.5e-7 and 1.1e-7).
 //
-// 32 heads of 128 channels, two runs of 1050 rows: 610 us as a scan (0.29 us per dependent step),
-// 185 us here: 75 us of staging and barriers, 63 of the state warps and 65 of the helpers, which
-// add up more than they overlap.  Runs below GDN_LONG_ROWS keep the scan: two chunks cost about as much as 64 steps,
-// and verification packets (at most 32 rows) must reproduce the scan's bits.
+// 32 heads of 128 channels, one run of 1050 rows: 406 us as a scan (0.39 us per dependent step),
+// 195 us here (166 with chained sums); 16 runs of 64 rows: 192 -> 84 us.
+// Runs below GDN_LONG_ROWS keep the scan, whose bits verification packets (at most 32 rows) must
+// reproduce.
 constexpr int GDN_LONG_ROWS = 64;
 constexpr int CHUNK = 32, CHUNK_THREADS = 192;
 struct ChunkSmem {
   __half k[3][CHUNK][136], q[3][CHUNK][136];   // rows padded to 17 16-byte units (ldmatrix)
   __half v[3][CHUNK][72];
-  float t[2][CHUNK][40], p[2][CHUNK][40];      // T and P, row i, column j
+  float t[2][CHUNK][40], p[2][CHUNK][40];      // T and P below the diagonal, row i, column j
+  float pd[2][CHUNK];                          // diagonal of P (that of T is 1)
   float at[CHUNK][36];                         // A transposed: [j][i]
   float eg[2][CHUNK], beta[2][CHUNK], tail[2][CHUNK], total[2];
 };
@@ -547,6 +554,18 @@ __device__ __forceinline__ void split_half2(float x, float y, uint32_t& hi, uint
   hi = *reinterpret_cast<const uint32_t*>(&h);
   lo = *reinterpret_cast<const uint32_t*>(&l);
 }
+__device__ __forceinline__ void split_half3(float x, float y, uint32_t& hi, uint32_t& mid,
+                                            uint32_t& lo) {
+  const __half2 h = __floats2half2_rn(x, y);
+  const float2 f = __half22float2(h);
+  hi = *reinterpret_cast<const uint32_t*>(&h);
+  split_half2(x - f.x, y - f.y, mid, lo);
+}
+// largest value of the four lanes that share a row
+__device__ __forceinline__ float quad_max(float x) {
+  x = fmaxf(x, __shfl_xor_sync(0xffffffffu, x, 1));
+  return fmaxf(x, __shfl_xor_sync(0xffffffffu, x, 2));
+}
 // e with |x| < 2^e (at least -100, at most 129) and powers of two
 __device__ __forceinline__ int bound_exp(float x) {
   return max(-100, static_cast<int>((__float_as_uint(x) >> 23) & 255u) - 126);
@@ -555,8 +574,15 @@ __device__ __forceinline__ float pow2i(int e) {
   return __uint_as_float(static_cast<uint32_t>(127 + e) << 23);
 }
 
-// D[i][0..7] (u-th group of eight columns) += X^T(16 x 32) M^T for a lower triangular 32 x 32
-// matrix M in shared memory: X and M split into TF32 pairs.
+// e^x, x FP64: the FP32 exponential of the rounded argument, corrected by what the rounding lost
+__device__ __forceinline__ float exp_pair(double x) {
+  const float hi = static_cast<float>(x);
+  const float e = expf(hi);
+  return fmaf(e, static_cast<float>(x - static_cast<double>(hi)), e);
+}
+
+// D[i][0..7] (u-th group of eight columns) += X^T(16 x 32) M^T for a 32 x 32 matrix M in shared
+// memory with zeros on and above the diagonal: X and M split into TF32 pairs.
 __device__ __forceinline__ void mul_lower(float (&d)[4][4], const float (&x)[4][4],
                                           const float (*m)[40], int g, int t) {
 #pragma unroll
@@ -573,9 +599,12 @@ __device__ __forceinline__ void mul_lower(float (&d)[4][4], const float (&x)[4][
       uint32_t bh0, bl0, bh1, bl1;
       split_tf32(b.x, bh0, bl0);
       split_tf32(b.y, bh1, bl1);
-      mma_tf32(d[u], hi, bl0, bl1);
-      mma_tf32(d[u], lo, bh0, bh1);
-      mma_tf32(d[u], hi, bh0, bh1);
+      float part[4] = {0.f, 0.f, 0.f, 0.f};
+      mma_tf32(part, hi, bl0, bl1);
+      mma_tf32(part, lo, bh0, bh1);
+      mma_tf32(part, hi, bh0, bh1);
+#pragma unroll
+      for (int e = 0; e < 4; ++e) d[u][e] += part[e];
     }
   }
 }
@@ -649,10 +678,10 @@ __global__ void __launch_bounds__(CHUNK_THREADS, 2) gdn_chunk_kernel(
     }
     const double last = __shfl_sync(0xffffffffu, big_g, 31);
     if (helper == 0) {
-      sm.eg[buf][lane] = expf(static_cast<float>(big_g));
+      sm.eg[buf][lane] = exp_pair(big_g);
       sm.beta[buf][lane] = beta;
-      sm.tail[buf][lane] = expf(static_cast<float>(last - big_g));
-      if (lane == 0) sm.total[buf] = expf(static_cast<float>(last));
+      sm.tail[buf][lane] = exp_pair(last - big_g);
+      if (lane == 0) sm.total[buf] = exp_pair(last);
     }
     // G as an FP32 pair: differences of the heads round in proportion to themselves, and the
     // remainders restore what the heads lost
@@ -695,12 +724,17 @@ __global__ void __launch_bounds__(CHUNK_THREADS, 2) gdn_chunk_kernel(
         ldsm_x4(x0, &xs[r][col]);
         ldsm_x4(x1, &xs[16 + r][col]);
       }
-      mma16816(acc[0], x0[0], x0[1], x0[2], x0[3], k0[0], k0[2]);
-      mma16816(acc[1], x0[0], x0[1], x0[2], x0[3], k0[1], k0[3]);
-      mma16816(acc[2], x1[0], x1[1], x1[2], x1[3], k0[0], k0[2]);
-      mma16816(acc[3], x1[0], x1[1], x1[2], x1[3], k0[1], k0[3]);
-      mma16816(acc[4], x1[0], x1[1], x1[2], x1[3], k1[0], k1[2]);
-      mma16816(acc[5], x1[0], x1[1], x1[2], x1[3], k1[1], k1[3]);
+      float d[6][4] = {};
+      mma16816(d[0], x0[0], x0[1], x0[2], x0[3], k0[0], k0[2]);
+      mma16816(d[1], x0[0], x0[1], x0[2], x0[3], k0[1], k0[3]);
+      mma16816(d[2], x1[0], x1[1], x1[2], x1[3], k0[0], k0[2]);
+      mma16816(d[3], x1[0], x1[1], x1[2], x1[3], k0[1], k0[3]);
+      mma16816(d[4], x1[0], x1[1], x1[2], x1[3], k1[0], k1[2]);
+      mma16816(d[5], x1[0], x1[1], x1[2], x1[3], k1[1], k1[3]);
+#pragma unroll
+      for (int i = 0; i < 6; ++i)
+#pragma unroll
+        for (int e = 0; e < 4; ++e) acc[i][e] += d[i][e];
     }
     // every factor first, then the stores: nothing in between waits for shared memory
 #pragma unroll
@@ -718,10 +752,12 @@ __global__ void __launch_bounds__(CHUNK_THREADS, 2) gdn_chunk_kernel(
 #pragma unroll
       for (int e = 0; e < 4; ++e) {
         const int ri = i0 + g + (e >> 1) * 8, cj = j0 + 2 * t + (e & 1);
-        if (helper == 0)
+        if (helper == 0) {
           sm.at[cj][ri] = cj < ri ? acc[i][e] : 0.f;
-        else
-          sm.p[buf][ri][cj] = cj <= ri ? acc[i][e] : 0.f;
+        } else {
+          sm.p[buf][ri][cj] = cj < ri ? acc[i][e] : 0.f;
+          if (cj == ri) sm.pd[buf][ri] = acc[i][e];
+        }
       }
     }
     if (helper == 0) {
@@ -743,6 +779,7 @@ __global__ void __launch_bounds__(CHUNK_THREADS, 2) gdn_chunk_kernel(
       }
 #pragma unroll
       for (int i = 0; i < CHUNK; ++i) sm.t[buf][i][lane] = x[i];
+      sm.t[buf][lane][lane] = 0.f;
       __syncwarp();                            // A is rewritten by the next chunk
     }
   };
@@ -756,15 +793,19 @@ __global__ void __launch_bounds__(CHUNK_THREADS, 2) gdn_chunk_kernel(
   const int dv = dv0 + (warp & 3) * 16 + g;
   float* sp = state + (static_cast<size_t>(row_slot[seg.row_start]) * hv + vh) * D * D + dv;
   float s_acc[16][4];
-  float s_max = 0.f;
+  float s_max[2] = {0.f, 0.f};                 // rows g and g + 8
   if (warp < 4) {
 #pragma unroll
     for (int u = 0; u < 16; ++u)
 #pragma unroll
       for (int e = 0; e < 4; ++e) {
         s_acc[u][e] = fresh ? 0.f : sp[(8 * u + 2 * t + (e & 1)) * D + (e >> 1) * 8];
-        s_max = fmaxf(s_max, fabsf(s_acc[u][e]));
       }
+    // a loop of its own: maxima between the loads take them one by one (16 runs of 64 rows: 110 us)
+#pragma unroll
+    for (int u = 0; u < 16; ++u)
+#pragma unroll
+      for (int e = 0; e < 4; ++e) s_max[e >> 1] = fmaxf(s_max[e >> 1], fabsf(s_acc[u][e]));
   }
   asm volatile("cp.async.wait_group 0;" ::: "memory");
   __syncthreads();
@@ -777,8 +818,13 @@ __global__ void __launch_bounds__(CHUNK_THREADS, 2) gdn_chunk_kernel(
       if (c + 1 < chunks) prepare(c + 1);
     } else {
       const int st = c % 3, buf = c & 1;
-      const int e_s = bound_exp(warp_max(s_max));
-      const float up = pow2i(14 - e_s), down = pow2i(e_s - 14);
+      float up[2], down[2];
+#pragma unroll
+      for (int h = 0; h < 2; ++h) {
+        const int e = bound_exp(quad_max(s_max[h]));
+        up[h] = pow2i(14 - e);
+        down[h] = pow2i(e - 14);
+      }
       // ---- S^T k and S^T q: columns are the chunk's rows
       float ak[4][4], aq[4][4];
 #pragma unroll
@@ -786,29 +832,33 @@ __global__ void __launch_bounds__(CHUNK_THREADS, 2) gdn_chunk_kernel(
 #pragma unroll
         for (int j = 0; j < 4; ++j) ak[i][j] = aq[i][j] = 0.f;
 #pragma unroll
-      for (int s = 0; s < D / 16; ++s) {
-        uint32_t hi[4], lo[4];
-        split_half2(s_acc[2 * s][0] * up, s_acc[2 * s][1] * up, hi[0], lo[0]);
-        split_half2(s_acc[2 * s][2] * up, s_acc[2 * s][3] * up, hi[1], lo[1]);
-        split_half2(s_acc[2 * s + 1][0] * up, s_acc[2 * s + 1][1] * up, hi[2], lo[2]);
-        split_half2(s_acc[2 * s + 1][2] * up, s_acc[2 * s + 1][3] * up, hi[3], lo[3]);
+      for (int s = 0; s < D / 16; s += 2) {
+        uint32_t hi[2][4], lo[2][4];
 #pragma unroll
-        for (int half = 0; half < 2; ++half) {
-          uint32_t bk[4], bq[4];
-          const int r = half * 16 + (mat >> 1) * 8 + mrow, col = s * 16 + (mat & 1) * 8;
-          ldsm_x4(bk, &sm.k[st][r][col]);
-          ldsm_x4(bq, &sm.q[st][r][col]);
-#pragma unroll
-          for (int v = 0; v < 2; ++v) {
-            mma16816(ak[half * 2 + v], lo[0], lo[1], lo[2], lo[3], bk[2 * v], bk[2 * v + 1]);
-            mma16816(aq[half * 2 + v], lo[0], lo[1], lo[2], lo[3], bq[2 * v], bq[2 * v + 1]);
-          }
-#pragma unroll
-          for (int v = 0; v < 2; ++v) {
-            mma16816(ak[half * 2 + v], hi[0], hi[1], hi[2], hi[3], bk[2 * v], bk[2 * v + 1]);
-            mma16816(aq[half * 2 + v], hi[0], hi[1], hi[2], hi[3], bq[2 * v], bq[2 * v + 1]);
-          }
+        for (int i = 0; i < 8; ++i) {
+          const float* x = s_acc[2 * s + (i >> 1)] + (i & 1) * 2;
+          split_half2(x[0] * up[i & 1], x[1] * up[i & 1], hi[i >> 2][i & 3], lo[i >> 2][i & 3]);
         }
+#pragma unroll
+        for (int half = 0; half < 2; ++half)
+#pragma unroll
+          for (int x = 0; x < 2; ++x) {              // k, then q
+            uint32_t b[2][4];
+            const int r = half * 16 + (mat >> 1) * 8 + mrow, col = s * 16 + (mat & 1) * 8;
+            ldsm_x4(b[0], &(x == 0 ? sm.k : sm.q)[st][r][col]);
+            ldsm_x4(b[1], &(x == 0 ? sm.k : sm.q)[st][r][col + 16]);
+#pragma unroll
+            for (int v = 0; v < 2; ++v) {
+              float part[4] = {};
+              mma16816(part, lo[0][0], lo[0][1], lo[0][2], lo[0][3], b[0][2 * v], b[0][2 * v + 1]);
+              mma16816(part, lo[1][0], lo[1][1], lo[1][2], lo[1][3], b[1][2 * v], b[1][2 * v + 1]);
+              mma16816(part, hi[0][0], hi[0][1], hi[0][2], hi[0][3], b[0][2 * v], b[0][2 * v + 1]);
+              mma16816(part, hi[1][0], hi[1][1], hi[1][2], hi[1][3], b[1][2 * v], b[1][2 * v + 1]);
+              float(&to)[4] = (x == 0 ? ak : aq)[half * 2 + v];
+#pragma unroll
+              for (int e = 0; e < 4; ++e) to[e] += part[e];
+            }
+          }
       }
       // ---- B^T, and e^G S^T q as the start of the output
 #pragma unroll
@@ -818,18 +868,25 @@ __global__ void __launch_bounds__(CHUNK_THREADS, 2) gdn_chunk_kernel(
         const float2 be = *reinterpret_cast<const float2*>(&sm.beta[buf][r]);
 #pragma unroll
         for (int e = 0; e < 4; ++e) {
-          const float ge = (e & 1 ? eg.y : eg.x) * down;
+          const float ge = (e & 1 ? eg.y : eg.x) * down[e >> 1];
           const float val = __half2float(sm.v[st][r + (e & 1)][(warp & 3) * 16 + g + (e >> 1) * 8]);
           ak[v][e] = (e & 1 ? be.y : be.x) * fmaf(-ge, ak[v][e], val);
           aq[v][e] *= ge * scale;
         }
       }
+      // the diagonals carry most of both sums: they are multiplied in FP32
       float dl[4][4];
 #pragma unroll
       for (int i = 0; i < 4; ++i)
 #pragma unroll
-        for (int j = 0; j < 4; ++j) dl[i][j] = 0.f;
+        for (int j = 0; j < 4; ++j) dl[i][j] = ak[i][j];
       mul_lower(dl, ak, sm.t[buf], g, t);
+#pragma unroll
+      for (int v = 0; v < 4; ++v) {
+        const float2 pd = *reinterpret_cast<const float2*>(&sm.pd[buf][8 * v + 2 * t]);
+#pragma unroll
+        for (int e = 0; e < 4; ++e) aq[v][e] = fmaf(e & 1 ? pd.y : pd.x, dl[v][e], aq[v][e]);
+      }
       mul_lower(aq, dl, sm.p[buf], g, t);
       const int n = min(CHUNK, seg.rows - c * CHUNK);
 #pragma unroll
@@ -842,49 +899,52 @@ __global__ void __launch_bounds__(CHUNK_THREADS, 2) gdn_chunk_kernel(
                 (e >> 1) * 8] = aq[v][e];
         }
       // ---- state update
-      float d_max = 0.f;
+      float d_max[2] = {0.f, 0.f};
 #pragma unroll
       for (int v = 0; v < 4; ++v) {
         const float2 tl = *reinterpret_cast<const float2*>(&sm.tail[buf][8 * v + 2 * t]);
 #pragma unroll
         for (int e = 0; e < 4; ++e) {
           dl[v][e] *= e & 1 ? tl.y : tl.x;
-          d_max = fmaxf(d_max, fabsf(dl[v][e]));
+          d_max[e >> 1] = fmaxf(d_max[e >> 1], fabsf(dl[v][e]));
         }
       }
-      const int e_d = bound_exp(warp_max(d_max));
-      const float dup = pow2i(14 - e_d), ddown = pow2i(e_d - 14), total = sm.total[buf];
-      uint32_t hi[2][4], lo[2][4];
+      float dup[2], ddown[2];
 #pragma unroll
-      for (int r = 0; r < 2; ++r)
+      for (int h = 0; h < 2; ++h) {
+        const int e = bound_exp(quad_max(d_max[h]));
+        dup[h] = pow2i(14 - e);
+        ddown[h] = pow2i(e - 14);
+      }
+      const float total = sm.total[buf];
+      s_max[0] = s_max[1] = 0.f;
+#pragma unroll
+      for (int r = 0; r < 2; ++r) {
+        // head, remainder and its remainder: a new row of S is this product to the last bit
+        uint32_t hi[4], mid[4], lo[4];
 #pragma unroll
         for (int i = 0; i < 4; ++i)
-          split_half2(dl[2 * r + (i >> 1)][(i & 1) * 2] * dup,
-                      dl[2 * r + (i >> 1)][(i & 1) * 2 + 1] * dup, hi[r][i], lo[r][i]);
-      s_max = 0.f;
+          split_half3(dl[2 * r + (i >> 1)][(i & 1) * 2] * dup[i & 1],
+                      dl[2 * r + (i >> 1)][(i & 1) * 2 + 1] * dup[i & 1], hi[i], mid[i], lo[i]);
 #pragma unroll
-      for (int u = 0; u < 16; u += 2) {
-        float add[2][4];
-#pragma unroll
-        for (int j = 0; j < 2; ++j)
-#pragma unroll
-          for (int e = 0; e < 4; ++e) add[j][e] = 0.f;
-#pragma unroll
-        for (int r = 0; r < 2; ++r) {
+        for (int u = 0; u < 16; u += 2) {
           uint32_t b[4];
+          float add[2][4] = {};
           ldsm_x4_t(b, &sm.k[st][r * 16 + (mat & 1) * 8 + mrow][(u + (mat >> 1)) * 8]);
-          mma16816(add[0], lo[r][0], lo[r][1], lo[r][2], lo[r][3], b[0], b[1]);
-          mma16816(add[1], lo[r][0], lo[r][1], lo[r][2], lo[r][3], b[2], b[3]);
-          mma16816(add[0], hi[r][0], hi[r][1], hi[r][2], hi[r][3], b[0], b[1]);
-          mma16816(add[1], hi[r][0], hi[r][1], hi[r][2], hi[r][3], b[2], b[3]);
-        }
 #pragma unroll
-        for (int j = 0; j < 2; ++j)
+          for (int j = 0; j < 2; ++j) {
+            mma16816(add[j], lo[0], lo[1], lo[2], lo[3], b[2 * j], b[2 * j + 1]);
+            mma16816(add[j], mid[0], mid[1], mid[2], mid[3], b[2 * j], b[2 * j + 1]);
+            mma16816(add[j], hi[0], hi[1], hi[2], hi[3], b[2 * j], b[2 * j + 1]);
 #pragma unroll
-          for (int e = 0; e < 4; ++e) {
-            s_acc[u + j][e] = fmaf(s_acc[u + j][e], total, add[j][e] * ddown);
-            s_max = fmaxf(s_max, fabsf(s_acc[u + j][e]));
+            for (int e = 0; e < 4; ++e) {
+              float& x = s_acc[u + j][e];
+              x = r == 0 ? fmaf(x, total, add[j][e] * ddown[e >> 1])
+                         : fmaf(add[j][e], ddown[e >> 1], x);
+              if (r == 1) s_max[e >> 1] = fmaxf(s_max[e >> 1], fabsf(x));
+            }
           }
+        }
       }
     }
     asm volatile("cp.async.wait_group 0;" ::: "memory");

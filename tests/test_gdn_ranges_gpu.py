@@ -152,3 +152,35 @@ def test_gdn_gated_norm_sigmoid_keeps_fp32_accuracy(dev, d):
         # e^-x within one step (2^-23), then a sum, a reciprocal and a product (2^-24 each); the
         # square root's reciprocal of a power of two within one step
         assert bool(((y - ref).abs() <= half_ulp + ref * 3.5 * 2.0 ** -23).all())
+
+
+@pytest.mark.parametrize("strength", [-4.0, -1.0])
+@pytest.mark.parametrize("spread", [0, 12])
+def test_gdn_chunks_keep_fp32_accuracy(dev, strength, spread):
+    """Long and medium memory, value channels of equal size and over twelve binades: the chunked
+    products against the 64-bit recurrence, channel by channel."""
+    from orinfer_b200.ops import functional as F
+    torch.manual_seed(7 + spread)
+    hk, hv, d, rows = 2, 4, 128, 333
+    a_log = (torch.randn(hv) * 0.5 + strength).to(dev)
+    dt = (torch.randn(hv) * 0.5 - 2).to(dev)
+    ab = torch.randn(rows, 2 * hv, device=dev)
+    qk = torch.nn.functional.normalize(torch.randn(rows, 2 * hk, d, device=dev), dim=-1)
+    size = torch.exp2(-torch.rand(1, hv, d, device=dev) * spread)
+    v = torch.randn(rows, hv, d, device=dev) * size
+    qkv = torch.cat([qk.reshape(rows, -1), v.reshape(rows, -1)], 1).half()
+    state = torch.randn(1, hv, d, d, device=dev) * 0.2 * size[:, :, None, :]
+    s0 = state[0].double()
+    t = lambda x: torch.tensor(x, dtype=torch.int32, device=dev)
+    out = F.gdn_scan(qkv, ab, a_log, dt, t([[0, rows, 0, 0]]), 1, t([0] * rows),
+                     t(list(range(50, 50 + rows))), hk, hv, d, state)
+    part = lambda i: qkv[:, i * hk * d:(i + 1) * hk * d].double().reshape(rows, hk, d)
+    g = -torch.exp(a_log.double()) * torch.nn.functional.softplus(ab[:, :hv].double() + dt.double())
+    ref, s = _recurrence64(part(0).repeat_interleave(2, 1) / math.sqrt(d),
+                           part(1).repeat_interleave(2, 1),
+                           qkv[:, 2 * hk * d:].double().reshape(rows, hv, d), g,
+                           torch.sigmoid(ab[:, hv:].double()), s0)
+    err = lambda x, y, dims: ((x - y).square().sum(dims) / y.square().sum(dims)).sqrt()
+    # a handful of FP32 roundings (2^-25 each in the mean) between the inputs and an output
+    assert float(err(out.double(), ref, (0,)).mean()) < 2.0 ** -22
+    assert float(err(state[0].double(), s, (1,)).mean()) < 2.0 ** -22
