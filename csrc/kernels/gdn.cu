@@ -195,7 +195,8 @@ __global__ void __launch_bounds__(256) gdn_history_kernel(const __half* __restri
   for (int j = 0; j < 3; ++j) {
     const int idx = s.rows - 3 + j;          // index into the chunk, < 0 = history
     if (idx >= 0) {
-      v[j] = *reinterpret_cast<const Chunk*>(x + static_cast<size_t>(s.row_start + idx) * x_stride + c);
+      const __half* row = x + static_cast<size_t>(s.row_start + idx) * x_stride;
+      v[j] = *reinterpret_cast<const Chunk*>(row + c);
     } else if (fresh) {
 #pragma unroll
       for (int i = 0; i < VEC; ++i) v[j].h[i] = __float2half(0.f);
@@ -582,7 +583,9 @@ __device__ __forceinline__ float exp_pair(double x) {
 }
 
 // D[i][0..7] (u-th group of eight columns) += X^T(16 x 32) M^T for a 32 x 32 matrix M in shared
-// memory with zeros on and above the diagonal: X and M split into TF32 pairs.
+// memory with zeros on and above the diagonal: X and M split into TF32 pairs.  A zero does not
+// hide an infinity or a NaN of a later row in a tensor-core product, so a block on the diagonal
+// whose rows hold one is summed term by term: earlier rows stay as they are.
 __device__ __forceinline__ void mul_lower(float (&d)[4][4], const float (&x)[4][4],
                                           const float (*m)[40], int g, int t) {
 #pragma unroll
@@ -593,8 +596,28 @@ __device__ __forceinline__ void mul_lower(float (&d)[4][4], const float (&x)[4][
     split_tf32(x[s][2], hi[1], lo[1]);
     split_tf32(x[s][1], hi[2], lo[2]);
     split_tf32(x[s][3], hi[3], lo[3]);
+    const float size = (fabsf(x[s][0]) + fabsf(x[s][1])) + (fabsf(x[s][2]) + fabsf(x[s][3]));
+    const bool wild = __any_sync(0xffffffffu, !(size < INFINITY));
+    if (wild) {
+#pragma unroll 1
+      for (int src = 0; src < 4; ++src)
+#pragma unroll
+        for (int e = 0; e < 2; ++e) {
+          const int j = 8 * s + 2 * src + e, from = (threadIdx.x & 28) | src;
+          const float xa = __shfl_sync(0xffffffffu, x[s][e], from);
+          const float xb = __shfl_sync(0xffffffffu, x[s][2 + e], from);
+#pragma unroll
+          for (int c = 0; c < 2; ++c) {
+            const int i = 8 * s + 2 * t + c;
+            if (j >= i) continue;
+            d[s][c] = fmaf(xa, m[i][j], d[s][c]);
+            d[s][2 + c] = fmaf(xb, m[i][j], d[s][2 + c]);
+          }
+        }
+    }
 #pragma unroll
     for (int u = s; u < 4; ++u) {
+      if (u == s && wild) continue;
       const float2 b = *reinterpret_cast<const float2*>(&m[8 * u + g][8 * s + 2 * t]);
       uint32_t bh0, bl0, bh1, bl1;
       split_tf32(b.x, bh0, bl0);
@@ -632,7 +655,8 @@ __global__ void __launch_bounds__(CHUNK_THREADS, 2) gdn_chunk_kernel(
     const int st = c % 3, n = min(CHUNK, seg.rows - c * CHUNK);
     for (int i = tid; i < CHUNK * 40; i += CHUNK_THREADS) {
       const int r = i / 40, u = i % 40;
-      const __half* row = qkv + static_cast<size_t>(seg.row_start + c * CHUNK + min(r, n - 1)) * conv_dim;
+      const size_t at = static_cast<size_t>(seg.row_start + c * CHUNK + min(r, n - 1));
+      const __half* row = qkv + at * conv_dim;
       const __half* src;
       __half* dst;
       if (u < 16) {
@@ -668,7 +692,11 @@ __global__ void __launch_bounds__(CHUNK_THREADS, 2) gdn_chunk_kernel(
     const bool live = c * CHUNK + lane < seg.rows;
     const float xg = n_a + bias;
     const float softplus = xg > 20.f ? xg : log1pf(expf(xg));
-    double big_g = live ? static_cast<double>(-alog * softplus) : 0.0;
+    // a decay that is zero in FP32 ends what a value was, also as the exponential of an infinity:
+    // kept finite, so that differences of the sums stay defined (a NaN stays one)
+    float log_decay = -alog * softplus;
+    if (log_decay < -200.f) log_decay = -200.f;
+    double big_g = live ? static_cast<double>(log_decay) : 0.0;
     const float beta = live ? __frcp_rn(1.f + expf(-n_b)) : 0.f;
     if (c + 1 < chunks) fetch_gates(c + 1);
 #pragma unroll

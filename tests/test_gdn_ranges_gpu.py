@@ -184,3 +184,45 @@ def test_gdn_chunks_keep_fp32_accuracy(dev, strength, spread):
     # a handful of FP32 roundings (2^-25 each in the mean) between the inputs and an output
     assert float(err(out.double(), ref, (0,)).mean()) < 2.0 ** -22
     assert float(err(state[0].double(), s, (1,)).mean()) < 2.0 ** -22
+
+
+@pytest.mark.parametrize("what", ["v_nan", "v_inf", "q_nan", "k_nan", "beta_nan", "decay_zero"])
+@pytest.mark.parametrize("row", [1, 13, 40, 94])
+def test_gdn_chunks_contain_non_finite_rows(dev, what, row):
+    """A run of 100 rows with one non-finite value, or with a log decay of minus infinity: as in
+    the recurrence, rows before it and channels beside it do not see it."""
+    from orinfer_b200.ops import functional as F
+    torch.manual_seed(row)
+    hk, hv, d, rows = 2, 4, 128, 100
+    a_log = (torch.randn(hv) * 0.5 - 1).to(dev)
+    dt = (torch.randn(hv) * 0.5 - 2).to(dev)
+    ab = torch.randn(rows, 2 * hv, device=dev)
+    qk = torch.nn.functional.normalize(torch.randn(rows, 2 * hk, d, device=dev), dim=-1)
+    qkv = torch.cat([qk.reshape(rows, -1), torch.randn(rows, hv * d, device=dev)], 1).half()
+    head, channel = 1, 37
+    if what[0] == "v":
+        qkv[row, 2 * hk * d + head * d + channel] = math.inf if what == "v_inf" else math.nan
+    elif what == "q_nan":
+        qkv[row, 5] = math.nan
+    elif what == "k_nan":
+        qkv[row, hk * d + 5] = math.nan
+    elif what == "beta_nan":
+        ab[row, hv + head] = math.nan
+    else:
+        ab[row, head] = math.inf                       # softplus and with it the log decay
+    state = torch.randn(1, hv, d, d, device=dev) * 0.2
+    s0 = state[0].double()
+    t = lambda x: torch.tensor(x, dtype=torch.int32, device=dev)
+    out = F.gdn_scan(qkv, ab, a_log, dt, t([[0, rows, 0, 0]]), 1, t([0] * rows),
+                     t(list(range(50, 50 + rows))), hk, hv, d, state)
+    part = lambda i: qkv[:, i * hk * d:(i + 1) * hk * d].double().reshape(rows, hk, d)
+    g = -torch.exp(a_log.double()) * torch.nn.functional.softplus(ab[:, :hv].double() + dt.double())
+    ref, s = _recurrence64(part(0).repeat_interleave(2, 1) / math.sqrt(d),
+                           part(1).repeat_interleave(2, 1),
+                           qkv[:, 2 * hk * d:].double().reshape(rows, hv, d), g,
+                           torch.sigmoid(ab[:, hv:].double()), s0)
+    for got, want in ((out, ref), (state[0], s)):
+        fine = torch.isfinite(want)
+        assert torch.equal(torch.isfinite(got), fine)
+        diff = (got.double() - want)[fine]
+        assert float(diff.norm() / want[fine].norm()) < 1e-6
