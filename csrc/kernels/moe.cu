@@ -98,11 +98,16 @@ __global__ void __launch_bounds__(256) router_topk_kernel(
 // Tensor-core form (hidden % 256 == 0, at most 64 MAXT expert rows).  The general form
 // streams the whole router matrix (0.5 to 2 MB) through every CTA, once per token row.  Here a
 // cluster of eight CTAs takes 16 rows: CTA c owns an eighth of the 8-expert tiles, its WARPS
-// warps a WARPS-th of the hidden channels each (FP16 products, FP32 sums on the tensor cores;
-// the partial sums are added in a fixed order that depends on the router alone, so a row's logits
-// do not depend on the packet), and each CTA collects the logits of its share of the rows
-// over distributed shared memory for the top-k.  Lane (g, t) loads 16 bytes of row g:
+// warps a WARPS-th of the hidden channels each, and each CTA collects the logits of its share of
+// the rows over distributed shared memory for the top-k.  Lane (g, t) loads 16 bytes of row g:
 // the halves 4s..4s+3 are its fragments of step s, in x and W alike.
+// The tensor core sums 16 FP16 products at a time and cuts the sum off instead of rounding it, so
+// every such sum starts at zero and is added in FP32, the warps' parts pairwise: probabilities of
+// 256 experts under 4096 channels are within 1.9e-7 of exact (the general form 2.9e-7, sums chained
+// through the tensor core 6.6e-7).  The order depends on the router alone, so a row's logits do not
+// depend on the packet's other rows.
+// 128 experts x 2048 channels: 16 rows 25.9 -> 9.5 us, 2048 rows 95 -> 48; one step per turn of the
+// loop: two take 57 us at 2048 rows.
 
 constexpr int ROUTER_CL = 8;
 
@@ -130,7 +135,7 @@ __global__ void __cluster_dims__(ROUTER_CL, 1, 1) __launch_bounds__(WARPS * 32) 
   const __half* xa = x + static_cast<size_t>(min(row0 + g, rows - 1)) * hidden + t * 8;
   const __half* xb = x + static_cast<size_t>(min(row0 + g + 8, rows - 1)) * hidden + t * 8;
   const int k_lo = hidden / WARPS * warp, k_hi = k_lo + hidden / WARPS;
-#pragma unroll(MAXT * WARPS > 72 ? 1 : 2)
+#pragma unroll 1
   for (int k = k_lo; k < k_hi; k += 32) {
     const uint4 a = __ldg(reinterpret_cast<const uint4*>(xa + k));
     const uint4 b = __ldg(reinterpret_cast<const uint4*>(xb + k));
@@ -139,13 +144,17 @@ __global__ void __cluster_dims__(ROUTER_CL, 1, 1) __launch_bounds__(WARPS * 32) 
     for (int i = 0; i < MAXT; ++i)
       if (i < nt) {
         const int e = min((t_lo + i) * 8 + g, total - 1);
-        wv[i] = __ldg(reinterpret_cast<const uint4*>(w + static_cast<size_t>(e) * hidden + t * 8 + k));
+        const __half* we = w + static_cast<size_t>(e) * hidden + t * 8 + k;
+        wv[i] = __ldg(reinterpret_cast<const uint4*>(we));
       }
 #pragma unroll
     for (int i = 0; i < MAXT; ++i)
       if (i < nt) {
-        mma16816(acc[i], a.x, b.x, a.y, b.y, wv[i].x, wv[i].y);
-        mma16816(acc[i], a.z, b.z, a.w, b.w, wv[i].z, wv[i].w);
+        float d[4] = {0.f, 0.f, 0.f, 0.f}, f[4] = {0.f, 0.f, 0.f, 0.f};
+        mma16816(d, a.x, b.x, a.y, b.y, wv[i].x, wv[i].y);
+        mma16816(f, a.z, b.z, a.w, b.w, wv[i].z, wv[i].w);
+#pragma unroll
+        for (int j = 0; j < 4; ++j) acc[i][j] += d[j] + f[j];
       }
   }
 #pragma unroll
@@ -157,10 +166,14 @@ __global__ void __cluster_dims__(ROUTER_CL, 1, 1) __launch_bounds__(WARPS * 32) 
   cluster.sync();                                   // every CTA of the cluster runs
   for (int i = threadIdx.x; i < ROWS * nt * 8; i += WARPS * 32) {
     const int r = i / (nt * 8), c = i % (nt * 8), e = t_lo * 8 + c;
-    float v = 0.f;
+    float v[WARPS];
 #pragma unroll
-    for (int q = 0; q < WARPS; ++q) v += part[q][r][c];
-    if (e < total) cluster.map_shared_rank(logits, r / OWN)[(r % OWN) * total + e] = v;
+    for (int q = 0; q < WARPS; ++q) v[q] = part[q][r][c];
+#pragma unroll
+    for (int n = WARPS / 2; n > 0; n /= 2)
+#pragma unroll
+      for (int q = 0; q < n; ++q) v[q] += v[q + n];
+    if (e < total) cluster.map_shared_rank(logits, r / OWN)[(r % OWN) * total + e] = v[0];
   }
   cluster.sync();
   const int row = row0 + crank * OWN + warp;

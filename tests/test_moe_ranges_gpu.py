@@ -35,7 +35,7 @@ def _scaled(a, sa, w, ws):
 @pytest.mark.parametrize("hidden,experts,top_k,shared", [
     (256, 3, 2, False), (256, 64, 4, True), (512, 128, 8, False), (2048, 191, 8, True),
     (256, 192, 8, True), (2048, 512, 10, True), (256, 576, 6, False), (256, 576, 6, True),
-    (264, 128, 8, False)])
+    (264, 128, 8, False), (4096, 9, 2, False), (2304, 16, 3, True)])
 def test_router_topk_forms(dev, rows, hidden, experts, top_k, shared):
     """Tensor-core and general router at the edges of their expert and row tiles."""
     from orinfer_b200.ops import functional as F
@@ -59,6 +59,23 @@ def test_router_topk_forms(dev, rows, hidden, experts, top_k, shared):
             assert 0 in chosen and chosen.index(0) < chosen.index(experts - 1)
     if shared:
         assert torch.allclose(gate.double(), torch.sigmoid(logits[:, experts]), atol=1e-5)
+
+
+@pytest.mark.parametrize("hidden,experts,shared", [(512, 64, False), (2048, 128, False),
+                                                   (2048, 512, True), (4096, 256, True)])
+def test_router_sums_keep_fp32_accuracy(dev, hidden, experts, shared):
+    """Probabilities against 64 bits: no further than rounded FP32 sums in blocks would be."""
+    from orinfer_b200.ops import functional as F
+    g = torch.Generator().manual_seed(hidden)
+    y = torch.randn(1024, hidden, generator=g).half().to(dev)
+    w = (torch.randn(experts + int(shared), hidden, generator=g) * 0.02).half().to(dev)
+    ids, probs, _ = F.router_topk(y, w, experts, 6, renorm=False)
+    p = torch.softmax((y.double() @ w.double().t())[:, :experts], 1)
+    p = torch.gather(p, 1, ids.long())
+    # logits of about 0.02 sqrt(hidden) with a few roundings of 2^-25 each in the mean, and as many
+    # again in the exponential, the sum over the experts and the division
+    limit = 2.0 ** -25 * (4 + 0.02 * hidden ** 0.5 * 3)
+    assert float((probs.double() - p).norm() / p.norm()) < limit
 
 
 @pytest.mark.parametrize("experts,rows,top_k,k", [(1, 1, 1, 128), (8, 5, 2, 256), (3, 300, 1, 128),
