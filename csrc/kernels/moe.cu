@@ -388,7 +388,17 @@ int orinfer_router_topk(const __half* x, const __half* w, int rows, int hidden, 
   if (rows <= 0) return 0;
   if (hidden % 8 || top_k < 1 || top_k > experts || experts > 4096) return -1;
   const int total = experts + (has_shared ? 1 : 0);
-  if (hidden % 256 == 0 && total <= 8 * 8 * 9 && runtime_ensure_init() == cudaSuccess) {
+  // Few experts leave most of a cluster's CTAs without a tile, and its two exchanges cost more than
+  // reading a small matrix per row: 8 experts x 2048 channels, 16 rows, 4.6 us in the general
+  // form against 6.3, 2048 rows 13.6 against 17.7; 16 experts 5.9 against 6.6; but 16 x 4096 11.0
+  // against 9.2 and 24 x 2048 8.1 against 7.4.  Up to 32 x 2048 the general form is also ahead
+  // where the clusters need one more wave than its CTAs (24 x 2048: 512 rows 8.7 against 9.8 us,
+  // 768 rows 11.1 against 12.1, 1024 rows 18.0 against 12.6, 1536 rows 19.7 against 21.5).
+  const int cells = total * hidden;
+  const bool few = (total <= 17 && cells <= 17 * 2048) ||
+                   (cells <= 32 * 2048 &&
+                    ((rows >= 256 && rows <= 640) || (rows > 1100 && rows < 1900)));
+  if (!few && hidden % 256 == 0 && total <= 8 * 8 * 9 && runtime_ensure_init() == cudaSuccess) {
     // Wide routers read their matrix from few SMs in a decode step: more warps, more loads in
     // flight (16 rows, 512 experts: 26 -> 16 us).
 #define ORINFER_ROUTER(MAXT, WARPS)                                                  \
