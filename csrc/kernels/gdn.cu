@@ -1018,7 +1018,8 @@ __global__ void __launch_bounds__(256) gdn_commit_kernel(
 }
 
 // ---------------------------------------------------------------- gated norm
-// grid (rows, HV), D threads: y = rmsnorm(o) * w * silu(z)  (sigmoid(z) when sigmoid_gate)
+// grid (rows, HV), D threads: y = rmsnorm(o) * w * silu(z)  (sigmoid(z) when sigmoid_gate).  The
+// sum of squares is built as in the warp form below, so a row gives the same bits through both.
 template <int D>
 __global__ void __launch_bounds__(D) gdn_gated_norm_kernel(
     const float* __restrict__ o, const __half* __restrict__ z, int z_stride,
@@ -1026,13 +1027,17 @@ __global__ void __launch_bounds__(D) gdn_gated_norm_kernel(
     __half* __restrict__ y) {
   const int row = blockIdx.x, h = blockIdx.y, d = threadIdx.x;
   const float v = o[(static_cast<size_t>(row) * hv + h) * D + d];
-  __shared__ float red[D / 32];
-  const float ss = warp_sum(v * v);
-  if ((d & 31) == 0) red[d >> 5] = ss;
-  __syncthreads();
-  float tot = 0.f;
+  constexpr int V = D / 32;
+  __shared__ float red[32];
+  float ss = 0.f;
 #pragma unroll
-  for (int i = 0; i < D / 32; ++i) tot += red[i];
+  for (int i = 0; i < V; ++i) {
+    const float x = __shfl_sync(0xffffffffu, v, (d & 31 & ~(V - 1)) + i);
+    ss = fmaf(x, x, ss);
+  }
+  if (d % V == 0) red[d / V] = ss;
+  __syncthreads();
+  const float tot = warp_sum(red[d & 31]);
   const float n = v * rsqrtf(tot / D + eps) * __half2float(w[d]);
   const float zf = __half2float(z[static_cast<size_t>(row) * z_stride + h * D + d]);
   const float sg = sigmoid_f32(zf);
@@ -1040,8 +1045,10 @@ __global__ void __launch_bounds__(D) gdn_gated_norm_kernel(
   y[(static_cast<size_t>(row) * hv + h) * D + d] = __float2half_rn(n * gate);
 }
 
-// The same, one warp per (row, head): D / 32 neighbouring channels per lane, eight heads per
-// CTA, no block barrier.  2100 rows x 32 heads of 128: 37 -> 13 us (69 MB).
+// The same, one warp per (row, head): D / 32 neighbouring channels per lane, no block barrier.
+// 2600 rows x 32 heads of 128: 45 -> 19 us (85 MB).  A few heads are quicker with a thread per
+// channel, which computes one sigmoid instead of four: 4 rows x 32 heads 1.2 us against 1.6, 48
+// rows 1.9 against 2.0, 64 rows 2.1 against 2.0.
 template <int D>
 __global__ void __launch_bounds__(256) gdn_gated_norm_warp_kernel(
     const float* __restrict__ o, const __half* __restrict__ z, int z_stride,
@@ -1219,9 +1226,9 @@ int orinfer_gdn_gated_norm(const float* o, const __half* z, int z_stride, const 
   if (rows <= 0) return 0;
   if (head_dim != 128 && head_dim != 64) return -1;
   const int v = head_dim / 32;
-  if (z_stride % v == 0 && aligned(z, 2 * v) && aligned(w, 2 * v) && aligned(o, 4 * v) &&
-      aligned(y, 2 * v)) {
-    const long long items = static_cast<long long>(rows) * hv;
+  const long long items = static_cast<long long>(rows) * hv;
+  if (items >= 1536 && z_stride % v == 0 && aligned(z, 2 * v) && aligned(w, 2 * v) &&
+      aligned(o, 4 * v) && aligned(y, 2 * v)) {
     const unsigned grid = static_cast<unsigned>((items + 7) / 8);
     if (head_dim == 128)
       gdn_gated_norm_warp_kernel<128><<<grid, 256, 0, stream>>>(o, z, z_stride, w, eps,

@@ -118,7 +118,7 @@ def test_gdn_conv_forms_agree(dev, d, hk, hv, rows, segments):
 
 
 @pytest.mark.parametrize("d", [64, 128])
-@pytest.mark.parametrize("rows,hv", [(1, 1), (3, 5), (130, 4)])
+@pytest.mark.parametrize("rows,hv", [(1, 1), (3, 5), (130, 4), (384, 4), (700, 3)])
 def test_gdn_gated_norm_forms_agree(dev, d, rows, hv):
     from orinfer_b200.ops import functional as F
     torch.manual_seed(rows)
@@ -133,6 +133,8 @@ def test_gdn_gated_norm_forms_agree(dev, d, rows, hv):
             ref = oo * torch.rsqrt((oo * oo).mean(-1, keepdim=True) + 1e-6) * w.double() * gate
             lim = ref.reshape(rows, -1).abs() * 2.0 ** -10 + 1e-7
             assert bool(((y.double() - ref.reshape(rows, -1)).abs() <= lim).all())
+            one = F.gdn_gated_norm(o[:1], z[:1], w, 1e-6, 1, hv, d, sigmoid_gate=sig)
+            assert torch.equal(one, y[:1])               # a row alone gives the same bits
 
 
 @pytest.mark.parametrize("d", [64, 128])
