@@ -222,7 +222,7 @@ int orinfer_gdn_scan(const __half* qkv, const float* ab, const float* a_log, con
                      const int* segs, int n_segs, const int* row_slot, const int* row_pos, int hk,
                      int hv, int head_dim, float* state, float* out, cudaStream_t stream,
                      float* factors, int max_seg_rows);
-// max_seg_rows: no segment has more rows (0: unknown but short, see gdn.cu).
+// max_seg_rows: no segment has more rows, where none is empty; it only chooses the kernels.
 // factors: fp32 [rows, HV, 2*D + 1] recorded by a scan with factors != NULL (which leaves the
 // state untouched); accepted: int32 [n_segs] rows of each segment to keep.
 int orinfer_gdn_commit(const __half* x, int x_stride, const float* factors, const int* segs,

@@ -3,8 +3,9 @@
 //   small_proj   : fp32 out[M,N] = x[M,H] . W[N,H]^T for narrow N (the a/b gate projection)
 //   gdn_conv     : width-4 causal depthwise conv over q|k|v channels with a 3-row per-request
 //                  history, SiLU, per-head L2 norm of q and k; then the history update
-//   gdn_scan     : exact sequential recurrence on the FP32 state (one CTA per segment and
-//                  value head; the 128x128 state lives in registers across the segment)
+//   gdn_scan     : recurrence on the FP32 state, which lives in registers across a segment: row by
+//                  row for short segments, in chunks of 32 rows (a triangular system and matrix
+//                  products on the tensor cores) for long ones
 //   gdn_gated_norm : per-head RMSNorm(o) * w * SiLU(z) (or sigmoid(z))
 // Replace gdn_ab_tensorcore (kernels/cuda/operators/op07_gdn_ab.py:16), gdn_conv_prep
 // (op08_gdn_conv_prep.py:23-278), gdn_gates (op09_gdn_gates.py:26-76), gdn_sequence
@@ -503,9 +504,10 @@ __global__ void __launch_bounds__(256) gdn_scan_split_kernel(
 //
 // 32 heads of 128 channels, one run of 1050 rows: 406 us as a scan (0.39 us per dependent step),
 // 195 us here (166 with chained sums); 16 runs of 64 rows: 192 -> 84 us.
-// Runs below GDN_LONG_ROWS keep the scan, whose bits verification packets (at most 32 rows) must
-// reproduce.
-constexpr int GDN_LONG_ROWS = 64;
+// Runs below GDN_LONG_ROWS keep the scan: one run of 36 rows takes 17.2 us there and 19.4 here, of
+// 40 rows 19.4 both ways, of 63 rows 28.0 and 19.4 (two runs of 50: 33 and 20).  The scan's bits
+// are those of a verification pass, whose segments are shorter.
+constexpr int GDN_LONG_ROWS = 40;
 constexpr int CHUNK = 32, CHUNK_THREADS = 192;
 struct ChunkSmem {
   __half k[3][CHUNK][136], q[3][CHUNK][136];   // rows padded to 17 16-byte units (ldmatrix)
@@ -1191,10 +1193,13 @@ int orinfer_gdn_scan(const __half* qkv, const float* ab, const float* a_log, con
   // pass and the plain pass over the same requests take the same arithmetic.
   const bool split = static_cast<long long>(hv) * n_segs < 2 * 148;
   // Runs of at least GDN_LONG_ROWS rows take the chunked kernel (which skips the others, as the
-  // scan skips them); verification passes and 64-channel heads never do.
+  // scan skips them); verification passes and 64-channel heads never do.  Which runs are long only
+  // the device knows, and a launch that finds none costs 1.5 to 3 us (8 runs of 20 rows: 48 -> 51
+  // us), so a packet of several runs that leaves one at most 63 rows does without: one run among
+  // them of 40 to 63 rows loses up to 9 us by that.
   int long_rows = 0x7fffffff;
-  if (head_dim == 128 && factors == nullptr && max_seg_rows >= GDN_LONG_ROWS &&
-      aligned(qkv, 16)) {
+  if (head_dim == 128 && factors == nullptr && aligned(qkv, 16) &&
+      max_seg_rows >= (n_segs == 1 ? GDN_LONG_ROWS : 64)) {
     long_rows = GDN_LONG_ROWS;
     static const int slot = runtime_new_slot();
     if (runtime_first_use(slot)) {

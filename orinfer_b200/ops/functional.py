@@ -373,11 +373,12 @@ def gdn_scan(qkv: torch.Tensor, ab: torch.Tensor, a_log: torch.Tensor, dt_bias: 
              hk: int, hv: int, head_dim: int, state: torch.Tensor,
              out: Optional[torch.Tensor] = None,
              factors: Optional[torch.Tensor] = None) -> torch.Tensor:
-    """Sequential gated-delta recurrence; ``state`` fp32 [slots, HV, D, D] updated in place.
-    With ``factors`` (fp32 [rows, HV, 2D+1]) the state is left untouched and every step's
-    (decay, k, delta) is recorded for :func:`gdn_commit`.  ``qkv`` should have no more rows than
-    the packet: its row count bounds the longest segment, and only packets that may hold a run
-    of 64 rows or more launch the chunked kernel beside the scan."""
+    """Gated-delta recurrence, row by row for short segments and in chunks of 32 rows for long
+    ones; ``state`` fp32 [slots, HV, D, D] updated in place.  With ``factors`` (fp32 [rows, HV,
+    2D+1]) the state is left untouched and every step's (decay, k, delta) is recorded for
+    :func:`gdn_commit`.  The chunked kernel is launched where a segment may be long: no longer
+    than the rows of ``qkv`` less one for every other segment, so ``qkv`` should hold the packet
+    alone and every segment a row (results do not depend on it, the choice of kernel does)."""
     _cuda(qkv, ab, a_log, dt_bias, segs, state, row_slot, row_pos)
     assert ab.dtype == torch.float32 and state.dtype == torch.float32 and state.is_contiguous()
     assert a_log.dtype == torch.float32 and dt_bias.dtype == torch.float32
@@ -388,7 +389,8 @@ def gdn_scan(qkv: torch.Tensor, ab: torch.Tensor, a_log: torch.Tensor, dt_bias: 
                                         n_segs, ptr(row_slot), ptr(row_pos), hk, hv, head_dim,
                                         ptr(state), ptr(out), stream(), ptr(factors), longest),
           "gdn_scan")
-    count_launches(2 if longest >= 64 and head_dim == 128 and factors is None else 1)
+    chunked = longest >= (40 if n_segs == 1 else 64) and head_dim == 128 and factors is None
+    count_launches(2 if chunked and qkv.data_ptr() % 16 == 0 else 1)
     return out
 
 

@@ -32,7 +32,8 @@ def _recurrence64(q, k, v, g, beta, s):
     return o, s
 
 
-@pytest.mark.parametrize("lens", [[64], [63, 65], [5, 96, 1, 97], [200, 2, 64, 129], [333]])
+@pytest.mark.parametrize("lens", [[39], [40], [41, 39], [64], [63, 65], [5, 96, 1, 97],
+                                  [200, 2, 64, 129], [333]])
 @pytest.mark.parametrize("strength", [0.3, 4.0])
 def test_gdn_scan_long_and_short_runs(dev, lens, strength):
     """Runs on both sides of the chunked kernel's limit, ragged tails, fresh and continued
