@@ -137,6 +137,7 @@ __global__ void __launch_bounds__(Smem<D>::THREADS, 1) attn_prefill_kernel(
     const int first = p_first + q * P;
     return first >= ch.q_len ? 0 : (ch.pos0 + min(first + P, ch.q_len) - 1) / KT + 1;
   };
+  const int kv_end = ch.pos0 + min(p_first + NQ * P, ch.q_len);
   int n_steps[NQ], n_max = 0;
 #pragma unroll
   for (int q = 0; q < NQ; ++q) {
@@ -183,7 +184,8 @@ __global__ void __launch_bounds__(Smem<D>::THREADS, 1) attn_prefill_kernel(
       const uint32_t q_addr = smem_u32(smem + L::Q_OFF);
       bool ok = mbar_wait(q_full, 0, status, STATUS_MMA_WAIT, 2);
       auto wait_kv = [&](int j) {
-        ok = ok && mbar_wait(&kv_ready[j & 1], (j >> 1) & 1, status, STATUS_MMA_WAIT, 0x100 | (j & 0xff));
+        ok = ok && mbar_wait(&kv_ready[j & 1], (j >> 1) & 1, status, STATUS_MMA_WAIT,
+                             0x100 | (j & 0xff));
         tc_fence_after();
       };
       auto issue_qk = [&](int q, int j) {
@@ -259,11 +261,15 @@ __global__ void __launch_bounds__(Smem<D>::THREADS, 1) attn_prefill_kernel(
       const __half* ksp = ks + slot * GROUPS + (u % CPK) / 4;
       const __half* vsp = vs + slot * GROUPS + (u % CPK) / 4;
       const int rows = (128 / CPK) * kvh;
+      // Keys past the last position that a row of this CTA sees may be slots never written.  Their
+      // weight is zero, but zero times an infinite or NaN value is not: they get no value scale.
+      const int live = kv_end - j * KT - u / CPK;
 #pragma unroll
       for (int it = 0; it < ITERS; ++it) {
         kraw[it] = __ldg(reinterpret_cast<const uint4*>(kp + static_cast<size_t>(it) * rows * D));
         vraw[it] = __ldg(reinterpret_cast<const uint4*>(vp + static_cast<size_t>(it) * rows * D));
-        sc[it] = __halves2half2(ksp[it * rows * GROUPS], vsp[it * rows * GROUPS]);
+        const __half vsc = it * (128 / CPK) < live ? vsp[it * rows * GROUPS] : __half(0.f);
+        sc[it] = __halves2half2(ksp[it * rows * GROUPS], vsc);
       }
     };
     bool ok = true;

@@ -99,6 +99,10 @@ def test_attention_prefill_at_tile_edges(dev, qh, kvh, d, gated, spec):
     vc = torch.randint(-127, 128, (need + 1, 128, kvh, d), generator=g, dtype=torch.int8).to(dev)
     ks = (torch.rand(need + 1, 128, kvh, d // 64, generator=g) * 0.02 + 1e-3).half().to(dev)
     vs = (torch.rand(need + 1, 128, kvh, d // 64, generator=g) * 0.02 + 1e-3).half().to(dev)
+    for i, (n, p) in enumerate(spec):               # slots never written hold anything
+        last, used = int(table[i, (n + p - 1) // 128]), (n + p - 1) % 128 + 1
+        ks[last, used:] = float("nan")
+        vs[last, used:] = float("inf")
     rows = sum(n for n, _ in spec)
     q = torch.randn(rows, qh, d, generator=g).half().to(dev)
     gate = torch.randn(rows, qh, d, generator=g).half().to(dev) if gated else None
