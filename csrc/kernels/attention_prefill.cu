@@ -3,9 +3,10 @@
 //
 // A query tile is 128 rows: P = 128 / rep consecutive query positions of one request times the
 // `rep` query heads that share one KV head (the heads are packed into the MMA M axis so each
-// INT8 K/V page is dequantised once for all of them).  One CTA owns NQ tiles: two neighbouring
-// ones for head sizes 64 and 128, so that a dequantised page serves 256 rows and the tensor core
-// works on one tile while the softmax warps of the other are busy.  Per step of KT keys:
+// INT8 K/V page is dequantised once for all of them).  One CTA owns NQ tiles: in large packets of
+// head sizes 64 and 128 two neighbouring ones, so that a dequantised page serves 256 rows and the
+// tensor core works on one tile while the softmax warps of the other are busy.  Per step of KT
+// keys:
 //   * eight warps, in two groups that take the steps in turn, read the INT8 page and its
 //     group-64 FP16 scales straight from global memory (ahead, in registers), dequantise to
 //     FP16 and store K and V as 128-byte-swizzled tiles (K is the K-major B operand of
@@ -16,8 +17,9 @@
 //     A operand.  P is relative to the row's running maximum, so its largest weight is exactly 1
 //     and O is rescaled whenever a row of the warp finds a larger score;
 //   * warp 0 loads the Q tiles once with a 3-D TMA (d, head, position).
-// Head size 256 has room for one tile (Q 64 KB, two K and two V buffers of 32 KB; TMEM: two S of
-// 64 columns and O of 256) and walks the cache in half pages, with S double buffered instead.
+// With one tile S is double buffered instead.  Head size 256 has room for no more (Q 64 KB, two K
+// and two V buffers of 32 KB; TMEM: two S of 64 columns and O of 256) and walks the cache in half
+// pages.
 // CTAs are ordered from the last query positions (the longest walks) to the first.
 //
 // One 4096-token chunk, 32 / 8 heads of 128: 377 us with one tile per CTA and P in shared memory,
@@ -40,9 +42,8 @@ namespace fa {
 constexpr int TILE = 128;                    // query rows per tile
 constexpr int DQ_WARPS = 8;                  // dequantisation warps
 
-template <int D>
+template <int D, int NQ>                                 // NQ: query tiles per CTA
 struct Smem {
-  static constexpr int NQ = D > 128 ? 1 : 2;             // query tiles per CTA
   static constexpr int THREADS = (2 + 4 * NQ + DQ_WARPS) * 32;
   static constexpr int KT = D > 128 ? 64 : 128;          // keys per step
   static constexpr int SUB = TILE * 128;                 // one [128 x 64 fp16] sub-tile (Q)
@@ -102,18 +103,18 @@ struct Chunk {            // one prefill chunk of one request
   int slot;               // row of the page table
 };
 
-template <int D>
-__global__ void __launch_bounds__(Smem<D>::THREADS, 1) attn_prefill_kernel(
+template <int D, int NQ>
+__global__ void __launch_bounds__(Smem<D, NQ>::THREADS, 1) attn_prefill_kernel(
     const __grid_constant__ CUtensorMap tmap_q, const Chunk* __restrict__ chunks,
     const int* __restrict__ page_table, int max_pages, const int8_t* __restrict__ kc,
     const int8_t* __restrict__ vc, const __half* __restrict__ ks, const __half* __restrict__ vs,
     const __half* __restrict__ gate, __half* __restrict__ out, int qh, int kvh, int rep,
     int num_pages, int* status) {
-  using L = Smem<D>;
-  constexpr int NQ = L::NQ, NSUB = L::NSUB, KT = L::KT;
+  using L = Smem<D, NQ>;
+  constexpr int NSUB = L::NSUB, KT = L::KT;
   constexpr int GROUPS = D / 64;
   constexpr uint32_t TMEM_COLS = 512;
-  constexpr int S_STRIDE = NQ == 2 ? 128 : 64;    // S of tile q (NQ = 2) or of buffer b (NQ = 1)
+  constexpr int S_STRIDE = KT;                    // S of tile q (NQ = 2) or of buffer b (NQ = 1)
   extern __shared__ unsigned char smem_raw[];
   unsigned char* smem = smem_raw + ((1024u - (smem_u32(smem_raw) & 1023u)) & 1023u);
   uint64_t* bars = reinterpret_cast<uint64_t*>(smem + L::BAR_OFF);
@@ -453,12 +454,12 @@ __global__ void __launch_bounds__(Smem<D>::THREADS, 1) attn_prefill_kernel(
   if (warp == 1) tmem_dealloc(tmem_base, TMEM_COLS);
 }
 
-template <int D>
+template <int D, int NQ>
 int launch(const __half* q, const __half* gate, const Chunk* chunks, int n_chunks, int max_q_len,
            int total_rows, const int* page_table, int max_pages, const int8_t* kc,
            const int8_t* vc, const __half* ks, const __half* vs, __half* out, int qh, int kvh,
            int num_pages, cudaStream_t stream) {
-  using L = Smem<D>;
+  using L = Smem<D, NQ>;
   const int rep = qh / kvh;
   const int P = TILE / rep;
   PFN_encodeTiled enc = runtime_tma_encoder();
@@ -475,12 +476,12 @@ int launch(const __half* q, const __half* gate, const Chunk* chunks, int n_chunk
     return -3;
   static const int slot = runtime_new_slot();
   if (runtime_first_use(slot)) {
-    cudaError_t e = cudaFuncSetAttribute(attn_prefill_kernel<D>,
+    cudaError_t e = cudaFuncSetAttribute(attn_prefill_kernel<D, NQ>,
                                          cudaFuncAttributeMaxDynamicSharedMemorySize, L::TOTAL);
     if (e != cudaSuccess) return static_cast<int>(e);
   }
-  dim3 grid((max_q_len + L::NQ * P - 1) / (L::NQ * P), kvh, n_chunks);
-  attn_prefill_kernel<D><<<grid, L::THREADS, L::TOTAL, stream>>>(
+  dim3 grid((max_q_len + NQ * P - 1) / (NQ * P), kvh, n_chunks);
+  attn_prefill_kernel<D, NQ><<<grid, L::THREADS, L::TOTAL, stream>>>(
       tq, chunks, page_table, max_pages, kc, vc, ks, vs, gate, out, qh, kvh, rep, num_pages,
       runtime_status_ptr());
   return static_cast<int>(cudaGetLastError());
@@ -502,14 +503,24 @@ extern "C" int orinfer_attention_prefill(const __half* q, const __half* gate, co
   if (kvh <= 0 || qh % kvh || qh / kvh > 16) return -1;
   if (runtime_ensure_init() != cudaSuccess) return -2;
   const fa::Chunk* ch = reinterpret_cast<const fa::Chunk*>(chunks);
-  if (head_dim == 128)
-    return fa::launch<128>(q, gate, ch, n_chunks, max_q_len, total_rows, page_table, max_pages, kc,
-                           vc, ks, vs, out, qh, kvh, num_pages, stream);
-  if (head_dim == 64)
-    return fa::launch<64>(q, gate, ch, n_chunks, max_q_len, total_rows, page_table, max_pages, kc,
-                          vc, ks, vs, out, qh, kvh, num_pages, stream);
-  if (head_dim == 256)
-    return fa::launch<256>(q, gate, ch, n_chunks, max_q_len, total_rows, page_table, max_pages,
-                           kc, vc, ks, vs, out, qh, kvh, num_pages, stream);
+  // One tile per CTA while those CTAs fit about one wave: 512 rows of 32 / 8 heads of 128 17.7 us
+  // against 21.8 with two (128 and 64 CTAs), 152 tiles 20.9 against 24.2; from 168 tiles on two
+  // share their pages' conversion at no loss of width (28.4 against 25.4 us; 4096 rows 279 against
+  // 241).  The longest chunk times their number overstates ragged packets, the rows in all and one
+  // cut tile per chunk those that do not fill the buffer: the smaller of the two counts.
+  const int tile_rows = fa::TILE / (qh / kvh);
+  const long long longest =
+      static_cast<long long>((max_q_len + tile_rows - 1) / tile_rows) * n_chunks;
+  const long long packed = static_cast<long long>(total_rows / tile_rows) + n_chunks;
+  const bool one = (longest < packed ? longest : packed) * kvh <= 160;
+#define ORINFER_PREFILL(D, NQ)                                                                 \
+  return fa::launch<D, NQ>(q, gate, ch, n_chunks, max_q_len, total_rows, page_table, max_pages, \
+                           kc, vc, ks, vs, out, qh, kvh, num_pages, stream)
+  if (head_dim == 128 && one) ORINFER_PREFILL(128, 1);
+  if (head_dim == 128) ORINFER_PREFILL(128, 2);
+  if (head_dim == 64 && one) ORINFER_PREFILL(64, 1);
+  if (head_dim == 64) ORINFER_PREFILL(64, 2);
+  if (head_dim == 256) ORINFER_PREFILL(256, 1);
+#undef ORINFER_PREFILL
   return -4;          // unsupported head size: caller falls back to the row kernel
 }

@@ -81,10 +81,10 @@ def test_attention_rows_at_block_edges(dev, qh, kvh, d, splits, wide):
                                             (16, 1, 128, False), (8, 1, 256, True),
                                             (4, 4, 256, False)])
 @pytest.mark.parametrize("spec", [[(1, 0)], [(63, 0), (65, 64), (1, 200)], [(129, 127), (257, 5)],
-                                  [(400, 1000)]])
+                                  [(400, 1000)], [(5200, 0), (1, 70)]])
 def test_attention_prefill_at_tile_edges(dev, qh, kvh, d, gated, spec):
-    """Chunks that end inside the first or second query tile of a CTA, pages cut by the first
-    position, against the 64-bit statement."""
+    """Chunks that end inside the first or second query tile of a CTA, one or two tiles per CTA,
+    pages cut by the first position, against the 64-bit statement."""
     from orinfer_b200.ops import functional as F
     g = torch.Generator().manual_seed(qh * d + spec[0][0])
     width = max((n + p + 127) // 128 for n, p in spec)
