@@ -1,8 +1,8 @@
 // Small-M quantised GEMM (decode path, M <= 8): weight-bandwidth bound.  Each CTA
 // owns a few output rows and streams their weights once; lanes decode E8P codes through a
 // shared-memory value table and the products with the INT8 activations staged in shared
-// memory run on the tensor cores (mma.sync, 16 weight rows x 8 activation rows).  Replaces the reference's dp4a /
-// gemv projections (kernels/cuda/model/integer_core.py:275,
+// memory run on the tensor cores (mma.sync, 16 weight rows x 8 activation rows), or by dp4a for
+// one or two rows.  Replaces the reference's dp4a / gemv projections (kernels/cuda/model/integer_core.py:275,
 // kernels/cuda/model/integer_vq.py:381 integer_e8p_gemv,
 // kernels/cuda/model/int8_projection.py:66).
 #include "api.h"
@@ -45,8 +45,9 @@ __device__ __forceinline__ void store_row(void* out, int out_f32, int m, int n, 
 // bank) and the activations are staged once.  The grid is n_parts x k_parts CTAs; a CTA owns a
 // contiguous range of 16-row groups and one range of 128-wide k-blocks, its warps take
 // contiguous runs of (group, k-block) units, every lane keeps DEPTH units of weight loads in
-// flight (the first ones are issued before the tables are filled), and the partial dot products
-// meet in shared memory (integer atomics: exact, so the result does not depend on the order).
+// flight (the first ones are issued before the tables are filled, except in the fused forms), and
+// the partial dot products meet in shared memory (integer atomics: exact, so the result does not
+// depend on the order).
 //
 // Products: m16n8k32 INT8 MMAs with the weights as A (lane (g, t) holds rows g and g + 8) and
 // the activation rows as the eight columns of B.  A lane's four code words of a k-block are
@@ -76,31 +77,24 @@ __device__ __forceinline__ void mma_i8_16832(int (&c)[4], uint32_t a0, uint32_t 
       : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1));
 }
 
-// One or two rows of Q4 weights keep the dp4a form: an MMA spends eight columns on them, and
-// eight-row units divide more evenly over the warps (19456 x 2560, one row: 13.8 us against 14.9
-// with MMAs; at eight rows the MMAs win, 16.2 against 23.1 us).  Lane l then holds
-// row l / 4 of a group of eight and a quarter of the k-block.
-template <int FMT, int MT>
-struct GemvMode {
-  static constexpr bool DP4A = FMT == 1 && MT <= 2;
-  static constexpr int ROWS = DP4A ? 8 : 16;                         // output rows of a group
-  static constexpr int DEPTH = DP4A || FMT == 2 ? 4 : 2;             // units in flight per lane
-};
-
-// Weights of one (group, k-block) unit as loaded by a lane: HALVES rows (g, and g + 8).
-template <int FMT, int HALVES = 2>
+// Weights of one (group, k-block) unit as loaded by a lane: rows g and g + 8.
+template <int FMT>
 struct GemvUnit {
   static constexpr int WORDS = FMT == 0 ? 8 : (FMT == 1 ? 4 : 2);    // 32-bit words per row
-  uint32_t w[HALVES][WORDS];
+  uint32_t w[2][WORDS];
 };
 
-// Position of channel k of activation row m in the staged activations (bytes).  dp4a: rows
-// as they are (a warp reads four octets 32 bytes apart); E8P: octets ordered [k-block][octet % 4][octet / 4][row]; INT8 weights: 16-byte pieces ordered
+// Whether a projection runs on q4_dp4a_kernel.
+constexpr bool gemv_dp4a(int fmt, int mt) { return fmt == 1 && mt <= 2; }
+
+// Position of channel k of activation row m in the staged activations (bytes).  dp4a: rows as they
+// are (a warp reads four octets 32 bytes apart); E8P MMAs: octets ordered
+// [k-block][octet % 4][octet / 4][row]; INT8 weights: 16-byte pieces ordered
 // [64 channels][row][piece], a lane's pieces being two steps each.
 template <int FMT, int MT>
 __device__ __forceinline__ int act_pos(int m, int k, int K) {
   if (FMT == 0) return ((k >> 6) * MT + m) * 64 + (k & 63);
-  if (GemvMode<FMT, MT>::DP4A) return m * K + k;
+  if (gemv_dp4a(FMT, MT)) return m * K + k;
   const int o = (k >> 3) & 15;
   return (((k >> 7) * 16 + (o & 3) * 4 + (o >> 2)) * MT + m) * 8 + (k & 7);
 }
@@ -129,97 +123,15 @@ struct GemvFuse {
   float* resid_accum;
 };
 
+// Fills the staged activations, their row sums (asum, zeroed before) and their scales: from INT8
+// rows, or by the row preparation of fz.pre, one row at a time in fbuf [K].
 template <int FMT, int MT>
-__global__ void __launch_bounds__(GEMV_THREADS, 1) qgemv_kernel(
-    const int8_t* __restrict__ a, const float* __restrict__ a_scale, const void* __restrict__ w,
-    const __half* __restrict__ w_scale, void* __restrict__ out, int M, int N, int K, int out_f32,
-    const E8pTables* __restrict__ tables, PeerOut po, int n_parts, int k_parts, int max_groups,
-    int* __restrict__ ws, GemvFuse fz) {
+__device__ __forceinline__ void gemv_rows(int8_t* act, int* asum, float* scale_s, float* fbuf,
+                                          float* red, float* blk_sum, const int8_t* __restrict__ a,
+                                          const float* __restrict__ a_scale, int M, int K,
+                                          const GemvFuse& fz) {
   constexpr int THREADS = GEMV_THREADS;
-  using Mode = GemvMode<FMT, MT>;
-  constexpr bool DP4A = Mode::DP4A;
-  constexpr int ROWS = Mode::ROWS, HALVES = ROWS / 8, DEPTH = Mode::DEPTH;
-  using Unit = GemvUnit<FMT, HALVES>;
-  using Lut = E8pLut<GEMV_COPIES>;
-  constexpr int LUT_BYTES = FMT == 0 ? 0 : static_cast<int>(sizeof(Lut));
-  const PeerOut* peer = po.tp > 0 ? &po : nullptr;
-  const bool ll = peer != nullptr && po.rows_per == LL_MODE;
-  const int ll_seq = ll ? *reinterpret_cast<volatile int*>(po.sent) + 1 : 0;
-  extern __shared__ __align__(16) unsigned char smem_raw[];
-  Lut* lut = reinterpret_cast<Lut*>(smem_raw);
-  int8_t* act = reinterpret_cast<int8_t*>(smem_raw) + LUT_BYTES;
-  int* acc_s = reinterpret_cast<int*>(act + static_cast<size_t>(MT) * K);   // [16 max_groups][MT]
-  int* asum = acc_s + max_groups * 16 * MT;                                  // [MT]
-  float* scale_s = reinterpret_cast<float*>(asum + MT);                      // [MT]
-  float* fbuf = reinterpret_cast<float*>(                                    // [K], pre only
-      (reinterpret_cast<uintptr_t>(scale_s + MT) + 15) & ~static_cast<uintptr_t>(15));
-  __shared__ int last_flag;
-  __shared__ float red[32];
-  __shared__ float blk_sum[128];
-
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-  const int g = lane >> 2, t = lane & 3;
-  const int kb_all = K / 128;
-  // a CTA's rows are a multiple of eight (the SMs then differ by 8 rows, not 16); its last group
-  // may be half a group
-  const int oct = N / 8;
-  const int np = blockIdx.x % n_parts, kp = blockIdx.x / n_parts;
-  const int n_base = static_cast<int>(static_cast<long long>(oct) * np / n_parts) * 8;
-  const int n_count = static_cast<int>(static_cast<long long>(oct) * (np + 1) / n_parts) * 8 - n_base;
-  const int groups = (n_count + ROWS - 1) / ROWS;
-  const int kb_lo = kb_all * kp / k_parts, kb_hi = kb_all * (kp + 1) / k_parts;
-  const int kbs = kb_hi - kb_lo;
-  const int units = groups * kbs;
-  constexpr int NW = THREADS / 32;
-  const int u_lo = static_cast<int>(static_cast<long long>(units) * warp / NW);
-  const int u_hi = static_cast<int>(static_cast<long long>(units) * (warp + 1) / NW);
-  // (group, k-block) of the unit being loaded, and of the unit being consumed
-  int lg = 0, lkb = 0;
-  if (u_lo < u_hi) {
-    lg = u_lo / kbs;
-    lkb = kb_lo + u_lo % kbs;
-  }
-  int cg = lg, ckb = lkb;
-  Unit buf[DEPTH];
-  auto fetch = [&](Unit& v, int uu) {
-    if (uu >= u_hi) return;
-#pragma unroll
-    for (int h = 0; h < HALVES; ++h) {
-      if (h == 1 && lg * ROWS + 8 >= n_count) break;       // half a group
-      const int n = n_base + lg * ROWS + g + h * 8;
-      if (FMT == 0) {
-        const uint4* p = reinterpret_cast<const uint4*>(w) + static_cast<size_t>(n) * (K / 16) +
-                         lkb * 8 + t;
-        const uint4 x = __ldg(p), y = __ldg(p + 4);
-        v.w[h][0] = x.x; v.w[h][1] = x.y; v.w[h][2] = x.z; v.w[h][3] = x.w;
-        v.w[h][4 % Unit::WORDS] = y.x; v.w[h][5 % Unit::WORDS] = y.y;
-        v.w[h][6 % Unit::WORDS] = y.z; v.w[h][7 % Unit::WORDS] = y.w;
-      } else if (FMT == 1) {
-        const uint4 x =
-            __ldg(reinterpret_cast<const uint4*>(w) + (static_cast<size_t>(lkb) * N + n) * 4 + t);
-        v.w[h][0] = x.x; v.w[h][1] = x.y;
-        v.w[h][2 % Unit::WORDS] = x.z; v.w[h][3 % Unit::WORDS] = x.w;
-      } else {
-        const uint2 x =
-            __ldg(reinterpret_cast<const uint2*>(w) + (static_cast<size_t>(lkb) * N + n) * 4 + t);
-        v.w[h][0] = x.x; v.w[h][1] = x.y;
-      }
-    }
-    if (++lkb == kb_hi) {
-      lkb = kb_lo;
-      ++lg;
-    }
-  };
-  // The first weights are requested before the tables are filled, except where the row
-  // preparation needs the registers, and by the dp4a form, which has none to spare (a spilled
-  // register costs every launch its local memory).
-  if (!DP4A && (FMT == 0 || fz.pre == 0)) {
-#pragma unroll
-    for (int i = 0; i < DEPTH; ++i) fetch(buf[i], u_lo + i);
-  }
-  if (FMT != 0) e8p_lut_init(lut, tables, tid, THREADS);
-  for (int i = tid; i < max_groups * 16 * MT + MT; i += THREADS) acc_s[i] = 0;
-  __syncthreads();
   if (FMT == 0 || fz.pre == 0) {
     // stage the activations; their row sums ride along
     const int chunks = MT * K / 16;
@@ -360,105 +272,20 @@ __global__ void __launch_bounds__(GEMV_THREADS, 1) qgemv_kernel(
       __syncthreads();
     }
   }
-  __syncthreads();
+}
 
-  if (DP4A || (FMT != 0 && fz.pre != 0)) {
-#pragma unroll
-    for (int i = 0; i < DEPTH; ++i) fetch(buf[i], u_lo + i);
-  }
-  int acc[4] = {0, 0, 0, 0};
-  const int copy = lane;                                   // GEMV_COPIES == 32
-  for (int base = u_lo; base < u_hi; base += DEPTH) {
-#pragma unroll
-    for (int i = 0; i < DEPTH; ++i) {
-      if (base + i < u_hi) {
-        const bool half = HALVES == 2 && cg * ROWS + 8 >= n_count;
-        if (DP4A) {
-          const Unit cur = buf[i];
-          fetch(buf[i], base + i + DEPTH);
-#pragma unroll
-          for (int j = 0; j < 4; ++j) {
-            const uint32_t word = cur.w[0][j % Unit::WORDS];
-            const uint32_t v0 = e8p_fields<GEMV_COPIES, 0>(word, lut, copy);
-            const uint32_t v1 = e8p_fields<GEMV_COPIES, 1>(word, lut, copy);
-            const int xlo = static_cast<int>((v0 & E8P_NIB) * 4u + (v1 & E8P_NIB));
-            const int xhi = static_cast<int>(((v0 >> 4) & E8P_NIB) * 4u + ((v1 >> 4) & E8P_NIB));
-#pragma unroll
-            for (int m = 0; m < MT && m < 2; ++m) {
-              const int2 av =
-                  *reinterpret_cast<const int2*>(act + m * K + (ckb * 16 + t * 4 + j) * 8);
-              acc[m] = __dp4a(xhi, av.y, __dp4a(xlo, av.x, acc[m]));
-            }
-          }
-        } else if (FMT == 0) {
-#pragma unroll
-          for (int j = 0; j < 2; ++j) {
-            int4 b = make_int4(0, 0, 0, 0);
-            if (g < MT)
-              b = *reinterpret_cast<const int4*>(act + act_pos<FMT, MT>(g, ckb * 128 + j * 64 + t * 16, K));
-            const uint32_t* r0 = buf[i].w[0] + (j * 4) % Unit::WORDS;
-            const uint32_t* r1 = buf[i].w[HALVES - 1] + (j * 4) % Unit::WORDS;
-            mma_i8_16832(acc, r0[0], r1[0], r0[1], r1[1], b.x, b.y);
-            mma_i8_16832(acc, r0[2 % Unit::WORDS], r1[2 % Unit::WORDS], r0[3 % Unit::WORDS],
-                         r1[3 % Unit::WORDS], b.z, b.w);
-          }
-        } else {
-#pragma unroll
-          for (int j = 0; j < 4; ++j) {
-            int2 b = make_int2(0, 0);
-            if (g < MT)
-              b = *reinterpret_cast<const int2*>(act + ((ckb * 16 + j * 4 + t) * MT + g) * 8);
-            uint32_t lo[2] = {0u, 0u}, hi[2] = {0u, 0u};
-#pragma unroll
-            for (int h = 0; h < 2; ++h) {
-              if (h == 1 && half) break;
-              if (FMT == 1) {
-                const uint32_t word = buf[i].w[h % HALVES][j % Unit::WORDS];
-                const uint32_t v0 = e8p_fields<GEMV_COPIES, 0>(word, lut, copy);
-                const uint32_t v1 = e8p_fields<GEMV_COPIES, 1>(word, lut, copy);
-                lo[h] = (v0 & E8P_NIB) * 4u + (v1 & E8P_NIB);
-                hi[h] = ((v0 >> 4) & E8P_NIB) * 4u + ((v1 >> 4) & E8P_NIB);
-              } else {
-                const uint32_t word = buf[i].w[h % HALVES][(j >> 1) % Unit::WORDS];
-                const uint32_t v = (j & 1) ? e8p_fields<GEMV_COPIES, 1>(word, lut, copy)
-                                           : e8p_fields<GEMV_COPIES, 0>(word, lut, copy);
-                lo[h] = v & E8P_NIB;
-                hi[h] = (v >> 4) & E8P_NIB;
-              }
-            }
-            mma_i8_16832(acc, lo[0], lo[1], hi[0], hi[1], b.x, b.y);
-          }
-        }
-        if (!DP4A) fetch(buf[i], base + i + DEPTH);
-        const bool last_of_group = ckb + 1 == kb_hi, last_unit = base + i + 1 == u_hi;
-        if (last_of_group || last_unit) {
-#pragma unroll
-          for (int e = 0; e < 4; ++e) {
-            if (DP4A) {
-              if (e >= MT) break;
-              int v = acc[e];
-              v += __shfl_xor_sync(0xffffffffu, v, 1);
-              v += __shfl_xor_sync(0xffffffffu, v, 2);
-              if (t == 0) atomicAdd(&acc_s[(cg * ROWS + g) * MT + e], v);
-            } else {
-              const int m = 2 * t + (e & 1);
-              if (m < MT && !(half && e >= 2))
-                atomicAdd(&acc_s[(cg * ROWS + g + (e >> 1) * 8) * MT + m], acc[e]);
-            }
-            acc[e] = 0;
-          }
-        }
-        if (last_of_group) {
-          ckb = kb_lo;
-          ++cg;
-        } else {
-          ++ckb;
-        }
-      }
-    }
-  }
-  __syncthreads();
-
+// Scales and writes the outputs n_base .. n_base + n_count from the integers in acc_s.
+template <int FMT, int MT>
+__device__ __forceinline__ void gemv_finish(int* acc_s, const int* asum, const float* scale_s,
+                                            int* last_flag, const __half* __restrict__ w_scale,
+                                            void* __restrict__ out, int M, int N, int out_f32,
+                                            const PeerOut& po, int ll_seq, int np, int k_parts,
+                                            int n_base, int n_count, int* __restrict__ ws,
+                                            const GemvFuse& fz) {
+  constexpr int THREADS = GEMV_THREADS;
+  const int tid = threadIdx.x;
+  const PeerOut* peer = po.tp > 0 ? &po : nullptr;
+  const bool ll = peer != nullptr && po.rows_per == LL_MODE;
   // sum_k a_k w_k from the staged integers: Q4 2*acc - 75*S, Q2 2*acc - 15*S
   constexpr int UNIT = FMT == 0 ? 1 : 2, BIAS = FMT == 0 ? 0 : (FMT == 1 ? 75 : 15);
   bool finalize = true;
@@ -474,11 +301,11 @@ __global__ void __launch_bounds__(GEMV_THREADS, 1) qgemv_kernel(
     if (tid == 0) {
       unsigned int* ticket = reinterpret_cast<unsigned int*>(ws + 8 * GEMV_WS_COLS) + np;
       const unsigned int t = atomicAdd(ticket, 1u);
-      last_flag = t == static_cast<unsigned int>(k_parts - 1);
-      if (last_flag) *ticket = 0;
+      *last_flag = t == static_cast<unsigned int>(k_parts - 1);
+      if (*last_flag) *ticket = 0;
     }
     __syncthreads();
-    finalize = last_flag != 0;
+    finalize = *last_flag != 0;
     if (finalize) {
       __threadfence();
       for (int i = tid; i < n_count * MT; i += THREADS) {
@@ -542,6 +369,287 @@ __global__ void __launch_bounds__(GEMV_THREADS, 1) qgemv_kernel(
   }
   if (ll) ll_done(po, ll_seq, gridDim.x);
   else if (peer != nullptr) peer_signal_done(po, gridDim.x);
+}
+
+template <int FMT, int MT>
+__global__ void __launch_bounds__(GEMV_THREADS, 1) qgemv_kernel(
+    const int8_t* __restrict__ a, const float* __restrict__ a_scale, const void* __restrict__ w,
+    const __half* __restrict__ w_scale, void* __restrict__ out, int M, int N, int K, int out_f32,
+    const E8pTables* __restrict__ tables, PeerOut po, int n_parts, int k_parts, int max_groups,
+    int* __restrict__ ws, GemvFuse fz) {
+  constexpr int THREADS = GEMV_THREADS;
+  constexpr int ROWS = 16, DEPTH = FMT == 2 ? 4 : 2;     // rows of a group, units in flight
+  using Unit = GemvUnit<FMT>;
+  using Lut = E8pLut<GEMV_COPIES>;
+  constexpr int LUT_BYTES = FMT == 0 ? 0 : static_cast<int>(sizeof(Lut));
+  const bool ll = po.tp > 0 && po.rows_per == LL_MODE;
+  const int ll_seq = ll ? *reinterpret_cast<volatile int*>(po.sent) + 1 : 0;
+  extern __shared__ __align__(16) unsigned char smem_raw[];
+  Lut* lut = reinterpret_cast<Lut*>(smem_raw);
+  int8_t* act = reinterpret_cast<int8_t*>(smem_raw) + LUT_BYTES;
+  int* acc_s = reinterpret_cast<int*>(act + static_cast<size_t>(MT) * K);   // [16 max_groups][MT]
+  int* asum = acc_s + max_groups * 16 * MT;                                  // [MT]
+  float* scale_s = reinterpret_cast<float*>(asum + MT);                      // [MT]
+  float* fbuf = reinterpret_cast<float*>(                                    // [K], pre only
+      (reinterpret_cast<uintptr_t>(scale_s + MT) + 15) & ~static_cast<uintptr_t>(15));
+  __shared__ int last_flag;
+  __shared__ float red[32];
+  __shared__ float blk_sum[128];
+
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  const int g = lane >> 2, t = lane & 3;
+  const int kb_all = K / 128;
+  // a CTA's rows are a multiple of eight (the SMs then differ by 8 rows, not 16); its last group
+  // may be half a group
+  const int oct = N / 8;
+  const int np = blockIdx.x % n_parts, kp = blockIdx.x / n_parts;
+  const int n_base = static_cast<int>(static_cast<long long>(oct) * np / n_parts) * 8;
+  const int n_count = static_cast<int>(static_cast<long long>(oct) * (np + 1) / n_parts) * 8 - n_base;
+  const int groups = (n_count + ROWS - 1) / ROWS;
+  const int kb_lo = kb_all * kp / k_parts, kb_hi = kb_all * (kp + 1) / k_parts;
+  const int kbs = kb_hi - kb_lo;
+  const int units = groups * kbs;
+  constexpr int NW = THREADS / 32;
+  const int u_lo = static_cast<int>(static_cast<long long>(units) * warp / NW);
+  const int u_hi = static_cast<int>(static_cast<long long>(units) * (warp + 1) / NW);
+  // (group, k-block) of the unit being loaded, and of the unit being consumed
+  int lg = 0, lkb = 0;
+  if (u_lo < u_hi) {
+    lg = u_lo / kbs;
+    lkb = kb_lo + u_lo % kbs;
+  }
+  int cg = lg, ckb = lkb;
+  Unit buf[DEPTH];
+  auto fetch = [&](Unit& v, int uu) {
+    if (uu >= u_hi) return;
+#pragma unroll
+    for (int h = 0; h < 2; ++h) {
+      if (h == 1 && lg * ROWS + 8 >= n_count) break;       // half a group
+      const int n = n_base + lg * ROWS + g + h * 8;
+      if (FMT == 0) {
+        const uint4* p = reinterpret_cast<const uint4*>(w) + static_cast<size_t>(n) * (K / 16) +
+                         lkb * 8 + t;
+        const uint4 x = __ldg(p), y = __ldg(p + 4);
+        v.w[h][0] = x.x; v.w[h][1] = x.y; v.w[h][2] = x.z; v.w[h][3] = x.w;
+        v.w[h][4 % Unit::WORDS] = y.x; v.w[h][5 % Unit::WORDS] = y.y;
+        v.w[h][6 % Unit::WORDS] = y.z; v.w[h][7 % Unit::WORDS] = y.w;
+      } else if (FMT == 1) {
+        const uint4 x =
+            __ldg(reinterpret_cast<const uint4*>(w) + (static_cast<size_t>(lkb) * N + n) * 4 + t);
+        v.w[h][0] = x.x; v.w[h][1] = x.y;
+        v.w[h][2 % Unit::WORDS] = x.z; v.w[h][3 % Unit::WORDS] = x.w;
+      } else {
+        const uint2 x =
+            __ldg(reinterpret_cast<const uint2*>(w) + (static_cast<size_t>(lkb) * N + n) * 4 + t);
+        v.w[h][0] = x.x; v.w[h][1] = x.y;
+      }
+    }
+    if (++lkb == kb_hi) {
+      lkb = kb_lo;
+      ++lg;
+    }
+  };
+  // The first weights are requested before the tables are filled, except where the row
+  // preparation needs the registers.
+  if (FMT == 0 || fz.pre == 0) {
+#pragma unroll
+    for (int i = 0; i < DEPTH; ++i) fetch(buf[i], u_lo + i);
+  }
+  if (FMT != 0) e8p_lut_init(lut, tables, tid, THREADS);
+  for (int i = tid; i < max_groups * 16 * MT + MT; i += THREADS) acc_s[i] = 0;
+  __syncthreads();
+  gemv_rows<FMT, MT>(act, asum, scale_s, fbuf, red, blk_sum, a, a_scale, M, K, fz);
+  __syncthreads();
+
+  if (FMT != 0 && fz.pre != 0) {
+#pragma unroll
+    for (int i = 0; i < DEPTH; ++i) fetch(buf[i], u_lo + i);
+  }
+  int acc[4] = {0, 0, 0, 0};
+  const int copy = lane;                                   // GEMV_COPIES == 32
+  for (int base = u_lo; base < u_hi; base += DEPTH) {
+#pragma unroll
+    for (int i = 0; i < DEPTH; ++i) {
+      if (base + i < u_hi) {
+        const bool half = cg * ROWS + 8 >= n_count;
+        if (FMT == 0) {
+#pragma unroll
+          for (int j = 0; j < 2; ++j) {
+            int4 b = make_int4(0, 0, 0, 0);
+            if (g < MT)
+              b = *reinterpret_cast<const int4*>(act + act_pos<FMT, MT>(g, ckb * 128 + j * 64 + t * 16, K));
+            const uint32_t* r0 = buf[i].w[0] + (j * 4) % Unit::WORDS;
+            const uint32_t* r1 = buf[i].w[1] + (j * 4) % Unit::WORDS;
+            mma_i8_16832(acc, r0[0], r1[0], r0[1], r1[1], b.x, b.y);
+            mma_i8_16832(acc, r0[2 % Unit::WORDS], r1[2 % Unit::WORDS], r0[3 % Unit::WORDS],
+                         r1[3 % Unit::WORDS], b.z, b.w);
+          }
+        } else {
+#pragma unroll
+          for (int j = 0; j < 4; ++j) {
+            int2 b = make_int2(0, 0);
+            if (g < MT)
+              b = *reinterpret_cast<const int2*>(act + ((ckb * 16 + j * 4 + t) * MT + g) * 8);
+            uint32_t lo[2] = {0u, 0u}, hi[2] = {0u, 0u};
+#pragma unroll
+            for (int h = 0; h < 2; ++h) {
+              if (h == 1 && half) break;
+              if (FMT == 1) {
+                const uint32_t word = buf[i].w[h][j % Unit::WORDS];
+                const uint32_t v0 = e8p_fields<GEMV_COPIES, 0>(word, lut, copy);
+                const uint32_t v1 = e8p_fields<GEMV_COPIES, 1>(word, lut, copy);
+                lo[h] = (v0 & E8P_NIB) * 4u + (v1 & E8P_NIB);
+                hi[h] = ((v0 >> 4) & E8P_NIB) * 4u + ((v1 >> 4) & E8P_NIB);
+              } else {
+                const uint32_t word = buf[i].w[h][(j >> 1) % Unit::WORDS];
+                const uint32_t v = (j & 1) ? e8p_fields<GEMV_COPIES, 1>(word, lut, copy)
+                                           : e8p_fields<GEMV_COPIES, 0>(word, lut, copy);
+                lo[h] = v & E8P_NIB;
+                hi[h] = (v >> 4) & E8P_NIB;
+              }
+            }
+            mma_i8_16832(acc, lo[0], lo[1], hi[0], hi[1], b.x, b.y);
+          }
+        }
+        fetch(buf[i], base + i + DEPTH);
+        const bool last_of_group = ckb + 1 == kb_hi, last_unit = base + i + 1 == u_hi;
+        if (last_of_group || last_unit) {
+#pragma unroll
+          for (int e = 0; e < 4; ++e) {
+            const int m = 2 * t + (e & 1);
+            if (m < MT && !(half && e >= 2))
+              atomicAdd(&acc_s[(cg * ROWS + g + (e >> 1) * 8) * MT + m], acc[e]);
+            acc[e] = 0;
+          }
+        }
+        if (last_of_group) {
+          ckb = kb_lo;
+          ++cg;
+        } else {
+          ++ckb;
+        }
+      }
+    }
+  }
+  __syncthreads();
+
+  gemv_finish<FMT, MT>(acc_s, asum, scale_s, &last_flag, w_scale, out, M, N, out_f32, po, ll_seq, np,
+                       k_parts, n_base, n_count, ws, fz);
+}
+
+// One or two rows of Q4 weights: dp4a instead of MMAs, in a kernel of its own (the registers of
+// the shared one cost the commonest call of a decode step half a microsecond).  An MMA spends eight
+// columns on these rows, and eight-row units divide more evenly over the warps.  Lane l holds row
+// l / 4 of a group of eight and a quarter of the k-block, DEPTH units in flight.
+// 19456 x 2560: one row 13.4 us against 14.9 with MMAs (13.8 inside the shared kernel), two rows
+// 14.3 (14.9); at eight rows the MMAs win, 16.2 against 23.1 us.
+template <int MT>
+__global__ void __launch_bounds__(GEMV_THREADS, 1) q4_dp4a_kernel(
+    const int8_t* __restrict__ a, const float* __restrict__ a_scale, const uint4* __restrict__ w,
+    const __half* __restrict__ w_scale, void* __restrict__ out, int M, int N, int K, int out_f32,
+    const E8pTables* __restrict__ tables, PeerOut po, int n_parts, int k_parts, int max_groups,
+    int* __restrict__ ws, GemvFuse fz) {
+  constexpr int THREADS = GEMV_THREADS, ROWS = 8, LPR = 4, DEPTH = 4;
+  using Lut = E8pLut<GEMV_COPIES>;
+  const bool ll = po.tp > 0 && po.rows_per == LL_MODE;
+  const int ll_seq = ll ? *reinterpret_cast<volatile int*>(po.sent) + 1 : 0;
+  extern __shared__ __align__(16) unsigned char smem_raw[];
+  Lut* lut = reinterpret_cast<Lut*>(smem_raw);
+  int8_t* act = reinterpret_cast<int8_t*>(smem_raw) + sizeof(Lut);
+  int* acc_s = reinterpret_cast<int*>(act + static_cast<size_t>(MT) * K);   // [16 max_groups][MT]
+  int* asum = acc_s + max_groups * 16 * MT;                                  // [MT]
+  float* scale_s = reinterpret_cast<float*>(asum + MT);                      // [MT]
+  float* fbuf = reinterpret_cast<float*>(                                    // [K], pre only
+      (reinterpret_cast<uintptr_t>(scale_s + MT) + 15) & ~static_cast<uintptr_t>(15));
+  __shared__ int last_flag;
+  __shared__ float red[32];
+  __shared__ float blk_sum[128];
+
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  e8p_lut_init(lut, tables, tid, THREADS);
+  for (int i = tid; i < max_groups * 16 * MT + MT; i += THREADS) acc_s[i] = 0;
+  __syncthreads();
+  gemv_rows<1, MT>(act, asum, scale_s, fbuf, red, blk_sum, a, a_scale, M, K, fz);
+  __syncthreads();
+
+  const int row = lane / LPR, part = lane % LPR;
+  const int kb_all = K / 128, groups = N / ROWS;
+  const int np = blockIdx.x % n_parts, kp = blockIdx.x / n_parts;
+  const int g_lo = static_cast<int>(static_cast<long long>(groups) * np / n_parts);
+  const int g_hi = static_cast<int>(static_cast<long long>(groups) * (np + 1) / n_parts);
+  const int kb_lo = kb_all * kp / k_parts, kb_hi = kb_all * (kp + 1) / k_parts;
+  const int kbs = kb_hi - kb_lo;
+  const int units = (g_hi - g_lo) * kbs;
+  constexpr int NW = THREADS / 32;
+  const int u_lo = static_cast<int>(static_cast<long long>(units) * warp / NW);
+  const int u_hi = static_cast<int>(static_cast<long long>(units) * (warp + 1) / NW);
+  int acc[MT];
+#pragma unroll
+  for (int m = 0; m < MT; ++m) acc[m] = 0;
+  const int copy = lane;                                   // GEMV_COPIES == 32
+  if (u_lo < u_hi) {
+    // (group, k-block) of the unit being loaded, and of the unit being consumed
+    int lg = g_lo + u_lo / kbs, lkb = kb_lo + u_lo % kbs;
+    int g = lg, kb = lkb;
+    uint4 buf[DEPTH];
+    auto fetch = [&](int uu) -> uint4 {
+      uint4 v = make_uint4(0, 0, 0, 0);
+      if (uu < u_hi) {
+        v = __ldg(w + (static_cast<size_t>(lkb) * N + lg * ROWS + row) * LPR + part);
+        if (++lkb == kb_hi) {
+          lkb = kb_lo;
+          ++lg;
+        }
+      }
+      return v;
+    };
+#pragma unroll
+    for (int i = 0; i < DEPTH; ++i) buf[i] = fetch(u_lo + i);
+    for (int base = u_lo; base < u_hi; base += DEPTH) {
+#pragma unroll
+      for (int i = 0; i < DEPTH; ++i) {
+        const uint4 cur = buf[i];
+        buf[i] = fetch(base + i + DEPTH);
+        if (base + i < u_hi) {
+          const int8_t* abase = act + kb * 128 + part * 32;
+          const uint32_t words[4] = {cur.x, cur.y, cur.z, cur.w};
+#pragma unroll
+          for (int j = 0; j < 4; ++j) {
+            const uint32_t v0 = e8p_fields<GEMV_COPIES, 0>(words[j], lut, copy);
+            const uint32_t v1 = e8p_fields<GEMV_COPIES, 1>(words[j], lut, copy);
+            const int xlo = static_cast<int>((v0 & E8P_NIB) * 4u + (v1 & E8P_NIB));
+            const int xhi = static_cast<int>(((v0 >> 4) & E8P_NIB) * 4u + ((v1 >> 4) & E8P_NIB));
+#pragma unroll
+            for (int m = 0; m < MT; ++m) {
+              const int2 av = *reinterpret_cast<const int2*>(abase + m * K + j * 8);
+              acc[m] = __dp4a(xlo, av.x, acc[m]);
+              acc[m] = __dp4a(xhi, av.y, acc[m]);
+            }
+          }
+          const bool last_of_group = kb + 1 == kb_hi, last_unit = base + i + 1 == u_hi;
+          if (last_of_group || last_unit) {
+#pragma unroll
+            for (int m = 0; m < MT; ++m) {
+              int v = acc[m];
+              v += __shfl_xor_sync(0xffffffffu, v, 1);
+              v += __shfl_xor_sync(0xffffffffu, v, 2);
+              if (part == 0) atomicAdd(&acc_s[((g - g_lo) * ROWS + row) * MT + m], v);
+              acc[m] = 0;
+            }
+          }
+          if (last_of_group) {
+            kb = kb_lo;
+            ++g;
+          } else {
+            ++kb;
+          }
+        }
+      }
+    }
+  }
+  __syncthreads();
+  gemv_finish<1, MT>(acc_s, asum, scale_s, &last_flag, w_scale, out, M, N, out_f32, po, ll_seq, np,
+                     k_parts, g_lo * ROWS, (g_hi - g_lo) * ROWS, ws, fz);
 }
 
 // INT8 weights, one or two rows: one warp per output row, 16 weights per lane per step, as many
@@ -857,15 +965,19 @@ static int launch_gemv(const int8_t* a, const float* as, const void* w, const __
   }
   if (smem > GEMV_SMEM_LIMIT) return -1;
   static const int slot = runtime_new_slot();
-  if (runtime_first_use(slot)) {
-    cudaError_t e = cudaFuncSetAttribute(
-        qgemv_kernel<FMT, MT>, cudaFuncAttributeMaxDynamicSharedMemorySize, GEMV_SMEM_LIMIT);
-    if (e != cudaSuccess) return static_cast<int>(e);
-  }
-  qgemv_kernel<FMT, MT><<<g.n_parts * g.k_parts, GEMV_THREADS, smem, stream>>>(
-      a, as, w, ws, out, M, N, K, out_f32, runtime_e8p_tables(), po, g.n_parts, g.k_parts,
-      g.max_groups, runtime_gemv_workspace(), fz);
-  return static_cast<int>(cudaGetLastError());
+  auto start = [&](auto kernel, auto* weights) -> int {
+    if (runtime_first_use(slot)) {
+      const cudaError_t e = cudaFuncSetAttribute(
+          kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, GEMV_SMEM_LIMIT);
+      if (e != cudaSuccess) return static_cast<int>(e);
+    }
+    kernel<<<g.n_parts * g.k_parts, GEMV_THREADS, smem, stream>>>(
+        a, as, weights, ws, out, M, N, K, out_f32, runtime_e8p_tables(), po, g.n_parts, g.k_parts,
+        g.max_groups, runtime_gemv_workspace(), fz);
+    return static_cast<int>(cudaGetLastError());
+  };
+  if constexpr (gemv_dp4a(FMT, MT)) return start(q4_dp4a_kernel<MT>, static_cast<const uint4*>(w));
+  else return start(qgemv_kernel<FMT, MT>, w);
 }
 
 template <int MT>
