@@ -2,7 +2,8 @@
 // owns a few output rows and streams their weights once; lanes decode E8P codes through a
 // shared-memory value table and the products with the INT8 activations staged in shared
 // memory run on the tensor cores (mma.sync, 16 weight rows x 8 activation rows), or by dp4a for
-// one or two rows.  Replaces the reference's dp4a / gemv projections (kernels/cuda/model/integer_core.py:275,
+// small products.  Replaces the reference's dp4a / gemv projections
+// (kernels/cuda/model/integer_core.py:275,
 // kernels/cuda/model/integer_vq.py:381 integer_e8p_gemv,
 // kernels/cuda/model/int8_projection.py:66).
 #include "api.h"
@@ -84,17 +85,14 @@ struct GemvUnit {
   uint32_t w[2][WORDS];
 };
 
-// Whether a projection runs on q4_dp4a_kernel.
-constexpr bool gemv_dp4a(int fmt, int mt) { return fmt == 1 && mt <= 2; }
-
 // Position of channel k of activation row m in the staged activations (bytes).  dp4a: rows as they
 // are (a warp reads four octets 32 bytes apart); E8P MMAs: octets ordered
 // [k-block][octet % 4][octet / 4][row]; INT8 weights: 16-byte pieces ordered
 // [64 channels][row][piece], a lane's pieces being two steps each.
-template <int FMT, int MT>
+template <int FMT, int MT, bool DP4A>
 __device__ __forceinline__ int act_pos(int m, int k, int K) {
+  if (DP4A) return m * K + k;
   if (FMT == 0) return ((k >> 6) * MT + m) * 64 + (k & 63);
-  if (gemv_dp4a(FMT, MT)) return m * K + k;
   const int o = (k >> 3) & 15;
   return (((k >> 7) * 16 + (o & 3) * 4 + (o >> 2)) * MT + m) * 8 + (k & 7);
 }
@@ -125,12 +123,11 @@ struct GemvFuse {
 
 // Fills the staged activations, their row sums (asum, zeroed before) and their scales: from INT8
 // rows, or by the row preparation of fz.pre, one row at a time in fbuf [K].
-template <int FMT, int MT>
+template <int FMT, int MT, int THREADS, bool DP4A>
 __device__ __forceinline__ void gemv_rows(int8_t* act, int* asum, float* scale_s, float* fbuf,
                                           float* red, float* blk_sum, const int8_t* __restrict__ a,
                                           const float* __restrict__ a_scale, int M, int K,
                                           const GemvFuse& fz) {
-  constexpr int THREADS = GEMV_THREADS;
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   if (FMT == 0 || fz.pre == 0) {
     // stage the activations; their row sums ride along
@@ -143,8 +140,8 @@ __device__ __forceinline__ void gemv_rows(int8_t* act, int* asum, float* scale_s
       int4 v = make_int4(0, 0, 0, 0);
       if (m < M) v = *reinterpret_cast<const int4*>(a + static_cast<size_t>(c) * 16);
       const int k = c * 16 - m * K;
-      *reinterpret_cast<int2*>(act + act_pos<FMT, MT>(m, k, K)) = make_int2(v.x, v.y);
-      *reinterpret_cast<int2*>(act + act_pos<FMT, MT>(m, k + 8, K)) = make_int2(v.z, v.w);
+      *reinterpret_cast<int2*>(act + act_pos<FMT, MT, DP4A>(m, k, K)) = make_int2(v.x, v.y);
+      *reinterpret_cast<int2*>(act + act_pos<FMT, MT, DP4A>(m, k + 8, K)) = make_int2(v.z, v.w);
       int s = __dp4a(v.x, 0x01010101, 0);
       s = __dp4a(v.y, 0x01010101, s);
       s = __dp4a(v.z, 0x01010101, s);
@@ -257,7 +254,7 @@ __device__ __forceinline__ void gemv_rows(int8_t* act, int* asum, float* scale_s
         c.y = static_cast<signed char>(a8_code(fb[i + 1], scale));
         c.z = static_cast<signed char>(a8_code(fb[i + 2], scale));
         c.w = static_cast<signed char>(a8_code(fb[i + 3], scale));
-        *reinterpret_cast<char4*>(act + act_pos<FMT, MT>(m, i, K)) = c;
+        *reinterpret_cast<char4*>(act + act_pos<FMT, MT, DP4A>(m, i, K)) = c;
         if (fz.q_out != nullptr && first_cta)
           *reinterpret_cast<char4*>(fz.q_out + static_cast<size_t>(m) * K + i) = c;
         psum = __dp4a(*reinterpret_cast<const int*>(&c), 0x01010101, psum);
@@ -275,14 +272,13 @@ __device__ __forceinline__ void gemv_rows(int8_t* act, int* asum, float* scale_s
 }
 
 // Scales and writes the outputs n_base .. n_base + n_count from the integers in acc_s.
-template <int FMT, int MT>
+template <int FMT, int MT, int THREADS>
 __device__ __forceinline__ void gemv_finish(int* acc_s, const int* asum, const float* scale_s,
                                             int* last_flag, const __half* __restrict__ w_scale,
                                             void* __restrict__ out, int M, int N, int out_f32,
                                             const PeerOut& po, int ll_seq, int np, int k_parts,
                                             int n_base, int n_count, int* __restrict__ ws,
                                             const GemvFuse& fz) {
-  constexpr int THREADS = GEMV_THREADS;
   const int tid = threadIdx.x;
   const PeerOut* peer = po.tp > 0 ? &po : nullptr;
   const bool ll = peer != nullptr && po.rows_per == LL_MODE;
@@ -458,7 +454,7 @@ __global__ void __launch_bounds__(GEMV_THREADS, 1) qgemv_kernel(
   if (FMT != 0) e8p_lut_init(lut, tables, tid, THREADS);
   for (int i = tid; i < max_groups * 16 * MT + MT; i += THREADS) acc_s[i] = 0;
   __syncthreads();
-  gemv_rows<FMT, MT>(act, asum, scale_s, fbuf, red, blk_sum, a, a_scale, M, K, fz);
+  gemv_rows<FMT, MT, THREADS, false>(act, asum, scale_s, fbuf, red, blk_sum, a, a_scale, M, K, fz);
   __syncthreads();
 
   if (FMT != 0 && fz.pre != 0) {
@@ -477,7 +473,8 @@ __global__ void __launch_bounds__(GEMV_THREADS, 1) qgemv_kernel(
           for (int j = 0; j < 2; ++j) {
             int4 b = make_int4(0, 0, 0, 0);
             if (g < MT)
-              b = *reinterpret_cast<const int4*>(act + act_pos<FMT, MT>(g, ckb * 128 + j * 64 + t * 16, K));
+              b = *reinterpret_cast<const int4*>(
+                  act + act_pos<FMT, MT, false>(g, ckb * 128 + j * 64 + t * 16, K));
             const uint32_t* r0 = buf[i].w[0] + (j * 4) % Unit::WORDS;
             const uint32_t* r1 = buf[i].w[1] + (j * 4) % Unit::WORDS;
             mma_i8_16832(acc, r0[0], r1[0], r0[1], r1[1], b.x, b.y);
@@ -533,23 +530,29 @@ __global__ void __launch_bounds__(GEMV_THREADS, 1) qgemv_kernel(
   }
   __syncthreads();
 
-  gemv_finish<FMT, MT>(acc_s, asum, scale_s, &last_flag, w_scale, out, M, N, out_f32, po, ll_seq, np,
-                       k_parts, n_base, n_count, ws, fz);
+  gemv_finish<FMT, MT, THREADS>(acc_s, asum, scale_s, &last_flag, w_scale, out, M, N, out_f32, po,
+                                ll_seq, np, k_parts, n_base, n_count, ws, fz);
 }
 
-// One or two rows of Q4 weights: dp4a instead of MMAs, in a kernel of its own (the registers of
-// the shared one cost the commonest call of a decode step half a microsecond).  An MMA spends eight
-// columns on these rows, and eight-row units divide more evenly over the warps.  Lane l holds row
-// l / 4 of a group of eight and a quarter of the k-block, DEPTH units in flight.
-// 19456 x 2560: one row 13.4 us against 14.9 with MMAs (13.8 inside the shared kernel), two rows
-// 14.3 (14.9); at eight rows the MMAs win, 16.2 against 23.1 us.
-template <int MT>
-__global__ void __launch_bounds__(GEMV_THREADS, 1) q4_dp4a_kernel(
+// E8P products by dp4a instead of MMAs (see gemv_dp4a for where).  An MMA spends eight columns on
+// however few rows, its form keeps two weight rows and less of them in flight per lane, and its
+// registers leave the row preparation little; this one spends four dp4a and two reads of
+// activations per row and code word.  Lane l holds row l / LPR of a group and an LPR-th of the
+// k-block, DEPTH units in flight.
+template <int FMT, int MT>
+struct Dp4a {
+  static constexpr int THREADS = MT <= 2 ? 1024 : 512;             // registers
+};
+
+template <int FMT, int MT>
+__global__ void __launch_bounds__(Dp4a<FMT, MT>::THREADS, 1) e8p_dp4a_kernel(
     const int8_t* __restrict__ a, const float* __restrict__ a_scale, const uint4* __restrict__ w,
     const __half* __restrict__ w_scale, void* __restrict__ out, int M, int N, int K, int out_f32,
     const E8pTables* __restrict__ tables, PeerOut po, int n_parts, int k_parts, int max_groups,
     int* __restrict__ ws, GemvFuse fz) {
-  constexpr int THREADS = GEMV_THREADS, ROWS = 8, LPR = 4, DEPTH = 4;
+  constexpr int THREADS = Dp4a<FMT, MT>::THREADS, DEPTH = 4;
+  constexpr int ROWS = FMT == 1 ? 8 : 16;        // output rows of a group
+  constexpr int LPR = 32 / ROWS;                 // lanes per row, 16 bytes of codes each
   using Lut = E8pLut<GEMV_COPIES>;
   const bool ll = po.tp > 0 && po.rows_per == LL_MODE;
   const int ll_seq = ll ? *reinterpret_cast<volatile int*>(po.sent) + 1 : 0;
@@ -569,11 +572,11 @@ __global__ void __launch_bounds__(GEMV_THREADS, 1) q4_dp4a_kernel(
   e8p_lut_init(lut, tables, tid, THREADS);
   for (int i = tid; i < max_groups * 16 * MT + MT; i += THREADS) acc_s[i] = 0;
   __syncthreads();
-  gemv_rows<1, MT>(act, asum, scale_s, fbuf, red, blk_sum, a, a_scale, M, K, fz);
+  gemv_rows<FMT, MT, THREADS, true>(act, asum, scale_s, fbuf, red, blk_sum, a, a_scale, M, K, fz);
   __syncthreads();
 
   const int row = lane / LPR, part = lane % LPR;
-  const int kb_all = K / 128, groups = N / ROWS;
+  const int kb_all = K / 128, groups = (N + ROWS - 1) / ROWS;
   const int np = blockIdx.x % n_parts, kp = blockIdx.x / n_parts;
   const int g_lo = static_cast<int>(static_cast<long long>(groups) * np / n_parts);
   const int g_hi = static_cast<int>(static_cast<long long>(groups) * (np + 1) / n_parts);
@@ -595,7 +598,8 @@ __global__ void __launch_bounds__(GEMV_THREADS, 1) q4_dp4a_kernel(
     auto fetch = [&](int uu) -> uint4 {
       uint4 v = make_uint4(0, 0, 0, 0);
       if (uu < u_hi) {
-        v = __ldg(w + (static_cast<size_t>(lkb) * N + lg * ROWS + row) * LPR + part);
+        const int n = min(lg * ROWS + row, N - 1);
+        v = __ldg(w + (static_cast<size_t>(lkb) * N + n) * LPR + part);
         if (++lkb == kb_hi) {
           lkb = kb_lo;
           ++lg;
@@ -611,14 +615,22 @@ __global__ void __launch_bounds__(GEMV_THREADS, 1) q4_dp4a_kernel(
         const uint4 cur = buf[i];
         buf[i] = fetch(base + i + DEPTH);
         if (base + i < u_hi) {
-          const int8_t* abase = act + kb * 128 + part * 32;
+          const int8_t* abase = act + kb * 128 + part * (128 / LPR);
           const uint32_t words[4] = {cur.x, cur.y, cur.z, cur.w};
 #pragma unroll
-          for (int j = 0; j < 4; ++j) {
-            const uint32_t v0 = e8p_fields<GEMV_COPIES, 0>(words[j], lut, copy);
-            const uint32_t v1 = e8p_fields<GEMV_COPIES, 1>(words[j], lut, copy);
-            const int xlo = static_cast<int>((v0 & E8P_NIB) * 4u + (v1 & E8P_NIB));
-            const int xhi = static_cast<int>(((v0 >> 4) & E8P_NIB) * 4u + ((v1 >> 4) & E8P_NIB));
+          for (int j = 0; j < (FMT == 1 ? 4 : 8); ++j) {
+            int xlo, xhi;
+            if (FMT == 1) {
+              const uint32_t v0 = e8p_fields<GEMV_COPIES, 0>(words[j & 3], lut, copy);
+              const uint32_t v1 = e8p_fields<GEMV_COPIES, 1>(words[j & 3], lut, copy);
+              xlo = static_cast<int>((v0 & E8P_NIB) * 4u + (v1 & E8P_NIB));
+              xhi = static_cast<int>(((v0 >> 4) & E8P_NIB) * 4u + ((v1 >> 4) & E8P_NIB));
+            } else {
+              const uint32_t v = (j & 1) ? e8p_fields<GEMV_COPIES, 1>(words[j >> 1], lut, copy)
+                                         : e8p_fields<GEMV_COPIES, 0>(words[j >> 1], lut, copy);
+              xlo = static_cast<int>(v & E8P_NIB);
+              xhi = static_cast<int>((v >> 4) & E8P_NIB);
+            }
 #pragma unroll
             for (int m = 0; m < MT; ++m) {
               const int2 av = *reinterpret_cast<const int2*>(abase + m * K + j * 8);
@@ -631,8 +643,8 @@ __global__ void __launch_bounds__(GEMV_THREADS, 1) q4_dp4a_kernel(
 #pragma unroll
             for (int m = 0; m < MT; ++m) {
               int v = acc[m];
-              v += __shfl_xor_sync(0xffffffffu, v, 1);
-              v += __shfl_xor_sync(0xffffffffu, v, 2);
+#pragma unroll
+              for (int o = 1; o < LPR; o <<= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
               if (part == 0) atomicAdd(&acc_s[((g - g_lo) * ROWS + row) * MT + m], v);
               acc[m] = 0;
             }
@@ -648,8 +660,9 @@ __global__ void __launch_bounds__(GEMV_THREADS, 1) q4_dp4a_kernel(
     }
   }
   __syncthreads();
-  gemv_finish<1, MT>(acc_s, asum, scale_s, &last_flag, w_scale, out, M, N, out_f32, po, ll_seq, np,
-                     k_parts, g_lo * ROWS, (g_hi - g_lo) * ROWS, ws, fz);
+  gemv_finish<FMT, MT, THREADS>(acc_s, asum, scale_s, &last_flag, w_scale, out, M, N, out_f32, po,
+                                ll_seq, np, k_parts, g_lo * ROWS, min(g_hi * ROWS, N) - g_lo * ROWS,
+                                ws, fz);
 }
 
 // INT8 weights, one or two rows: one warp per output row, 16 weights per lane per step, as many
@@ -943,6 +956,26 @@ static GemvGrid gemv_grid(int fmt, int N, int K) {
 
 constexpr size_t GEMV_SMEM_LIMIT = 220 * 1024;
 
+// Whether an E8P projection runs on e8p_dp4a_kernel: where it was the quicker of the two, over 250
+// to 19456 columns x 1024 to 9728 channels, alone and with each row preparation.
+//   alone: Q4 one or two rows always (1 x 19456 x 2560 13.4 us against 14.9); four rows under short
+//     or narrow products (2048 x 1024 6.1 against 7.2, 9728 x 2048 10.2 against 10.6, 5120 x 4096
+//     11.1 against 10.7), eight under small ones (2048 x 1024 6.9 against 7.7, 2560 x 1024 both
+//     7.7).  Q2 one or two rows from 8 M weights on (2048 x 9728 7.3 against 8.0, 2048 x 2048 both
+//     6.2), four and eight rows as for Q4 (4 x 2048 x 4096 7.2 against 7.3, 4 x 2560 x 4096 8.1
+//     against 7.9; 8 x 2048 x 2048 7.6 against 7.7, 8 x 5120 x 1024 7.8 against 7.3).
+//   with the row preparation, which dominates and leaves the MMA form few registers: always (4 x
+//     2048 x 1024 13.4 against 17.7), but for five to eight rows under large products of long rows
+//     (5 x 19456 x 2560 36.2 against 32.4; 5 x 12288 x 2048 24.8 against 25.9).
+inline bool gemv_dp4a(int fmt, int mt, int N, int K, bool fused) {
+  const long long cells = static_cast<long long>(N) * K, M = 1024 * 1024;
+  if (fused) return mt <= 4 || K <= 2048 || cells < 23 * M;
+  if (mt <= 2) return fmt == 1 || cells >= 8 * M;
+  if (mt <= 4)
+    return (K <= 2048 && cells <= 20 * M) || (fmt == 1 ? N <= 1024 : N <= 2048 && K <= 4096);
+  return fmt == 1 ? K <= 1024 && N <= 2048 : K <= 2048 && cells <= 4 * M;
+}
+
 // Dynamic shared memory for `mt` staged activation rows.
 static size_t gemv_smem(int fmt, int mt, const GemvGrid& g, int K, bool fused) {
   size_t smem = (fmt == 0 ? 0 : sizeof(E8pLut<GEMV_COPIES>)) + static_cast<size_t>(mt) * K +
@@ -964,20 +997,24 @@ static int launch_gemv(const int8_t* a, const float* as, const void* w, const __
     smem = gemv_smem(FMT, MT, g, K, fz.pre != 0);
   }
   if (smem > GEMV_SMEM_LIMIT) return -1;
-  static const int slot = runtime_new_slot();
-  auto start = [&](auto kernel, auto* weights) -> int {
-    if (runtime_first_use(slot)) {
+  static const int slot[2] = {runtime_new_slot(), runtime_new_slot()};
+  auto start = [&](auto kernel, int threads, auto* weights, int sl) -> int {
+    if (runtime_first_use(sl)) {
       const cudaError_t e = cudaFuncSetAttribute(
           kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, GEMV_SMEM_LIMIT);
       if (e != cudaSuccess) return static_cast<int>(e);
     }
-    kernel<<<g.n_parts * g.k_parts, GEMV_THREADS, smem, stream>>>(
+    kernel<<<g.n_parts * g.k_parts, threads, smem, stream>>>(
         a, as, weights, ws, out, M, N, K, out_f32, runtime_e8p_tables(), po, g.n_parts, g.k_parts,
         g.max_groups, runtime_gemv_workspace(), fz);
     return static_cast<int>(cudaGetLastError());
   };
-  if constexpr (gemv_dp4a(FMT, MT)) return start(q4_dp4a_kernel<MT>, static_cast<const uint4*>(w));
-  else return start(qgemv_kernel<FMT, MT>, w);
+  if constexpr (FMT != 0)
+    if (gemv_dp4a(FMT, MT, N, K, fz.pre != 0))
+      return start(e8p_dp4a_kernel<FMT, MT>, Dp4a<FMT, MT>::THREADS, static_cast<const uint4*>(w),
+                   slot[0]);
+  if constexpr (FMT != 1 || MT > 2) return start(qgemv_kernel<FMT, MT>, GEMV_THREADS, w, slot[1]);
+  return -1;
 }
 
 template <int MT>

@@ -34,9 +34,10 @@ def _scaled(a, sa, w, ws):
 @pytest.mark.parametrize("fmt", ["w8", "q4", "q2"])
 @pytest.mark.parametrize("m", [1, 2, 3, 4, 5, 8])
 @pytest.mark.parametrize("n,k", [(8, 128), (24, 384), (16, 1152), (2560, 1024), (2376, 512),
-                                 (40000, 256)])
+                                 (40000, 256), (3976, 2176), (6152, 2176), (264, 8448)])
 def test_small_row_projections_are_exact(dev, fmt, m, n, k):
-    """Row groups of sixteen cut by N, single k-blocks, K splits and several groups per CTA."""
+    """Row groups of sixteen cut by N, single k-blocks, K splits and several groups per CTA, on both
+    sides of the lines between the dp4a, row-per-warp and MMA forms."""
     from orinfer_b200.ops import functional as F
     g = torch.Generator().manual_seed(m * n + k)
     codes, ws, w = _int_weight(fmt, n, k, g)
@@ -110,3 +111,22 @@ def test_swiglu_sigmoid_keeps_fp32_accuracy(dev, rows, k, fused):
         half_ulp = torch.exp2(torch.floor(torch.log2(ref.abs())) - 11)
         # e^-x within one step (2^-23), then a sum, a reciprocal and two products (2^-24 each)
         assert bool(((y.double() - ref).abs() <= half_ulp + ref.abs() * 3 * 2.0 ** -23).all())
+
+
+@pytest.mark.parametrize("fmt", ["q4", "q2"])
+@pytest.mark.parametrize("m,n,k", [(2, 24, 384), (4, 2376, 512), (8, 1040, 1152), (5, 9736, 2560),
+                                   (8, 9736, 2560)])
+def test_fused_projection_forms_equal_separate_kernels(dev, fmt, m, n, k):
+    """dp4a and MMA forms with a row preparation give the bits of act_prep and qgemm."""
+    from orinfer_b200.ops import functional as F
+    g = torch.Generator().manual_seed(m * n + k)
+    codes, ws, _ = _int_weight(fmt, n, k, g)
+    codes, ws = codes.to(dev), ws.to(dev)
+    signs = (1 - 2 * torch.randint(0, 2, (k,), generator=g)).to(torch.int8).to(dev)
+    for pre, width in ((F.PRE_PLAIN, k), (F.PRE_SWIGLU, 2 * k)):
+        x = torch.randn(m, width, generator=g).half().to(dev)
+        q8, sc = F.act_prep(x, None, None, signs, swiglu=pre == F.PRE_SWIGLU)
+        want = F.qgemm(q8, sc, codes, ws, fmt, n)
+        out = torch.empty_like(want)
+        assert F.qgemv_fused(pre, x, None, None, signs, codes, ws, fmt, n, k, m, out=out)
+        assert torch.equal(out, want)
