@@ -665,10 +665,22 @@ __global__ void __launch_bounds__(Dp4a<FMT, MT>::THREADS, 1) e8p_dp4a_kernel(
                                 ws, fz);
 }
 
-// INT8 weights, one or two rows: one warp per output row, 16 weights per lane per step, as many
-// CTAs as rows need.  Small projections that sit in L2 are twice as fast this way (6144 x 2560,
-// one row: 3.7 us against 6.9 with persistent CTAs; the 151936-row head 74 against 75); from four
-// rows on the shared-memory reads per row lose to the MMAs (head, eight rows: 205 against 77 us).
+// INT8 weights by one warp per output row: 16 weights per lane per step, as many CTAs as rows
+// need, the activations read from shared memory once per weight row.  Small projections are up to
+// twice as fast this way as with the persistent CTAs of the MMA form; from three rows on its reads
+// lose to the MMAs once there is work for every SM.
+//   one row: 6144 x 2560 3.7 us against 6.9, the 151936-row head 74 against 75
+//   four: 1024 x 1024 2.7 against 5.2, 4096 x 4096 6.0 against 6.9, 5120 x 9728 15.7 against 16.2,
+//     6144 x 2560 7.4 against 6.7, 9728 x 1024 5.8 against 6.0, 12288 x 1024 7.0 against 6.1
+//   eight: 1024 x 1024 4.0 against 5.9, 2048 x 4096 6.5 against 6.9, 4096 x 2560 7.7 against 7.2,
+//     512 x 9728 9.4 against 8.8, head 205 against 77
+inline bool w8_by_rows(int M, int N, int K) {
+  const long long cells = static_cast<long long>(N) * K;
+  if (M <= 2) return true;
+  if (M <= 4) return K <= 16384 && (N < 6144 || (N < 12288 && cells < 12500000));
+  return K <= 8192 && cells <= 8 * 1024 * 1024;
+}
+
 template <int MT>
 __global__ void __launch_bounds__(W8_WARPS * 32) w8_gemv_kernel(
     const int8_t* __restrict__ a, const float* __restrict__ a_scale, const int8_t* __restrict__ w,
@@ -1061,9 +1073,7 @@ int qgemv_dispatch(int fmt, const int8_t* a, const float* as, const void* w, con
    : M == 2 ? FN<__VA_ARGS__ 2>(a, as, w, ws, out, M, N, K, out_f32, stream, po) \
    : M <= 4 ? FN<__VA_ARGS__ 4>(a, as, w, ws, out, M, N, K, out_f32, stream, po) \
             : FN<__VA_ARGS__ 8>(a, as, w, ws, out, M, N, K, out_f32, stream, po))
-  if (fmt == 0 && M <= 2)
-    return M == 1 ? launch_w8<1>(a, as, w, ws, out, M, N, K, out_f32, stream, po)
-                  : launch_w8<2>(a, as, w, ws, out, M, N, K, out_f32, stream, po);
+  if (fmt == 0 && w8_by_rows(M, N, K)) return BY_M(launch_w8, );
   if (fmt == 0)
     return M <= 4 ? launch_gemv<0, 4>(a, as, w, ws, out, M, N, K, out_f32, stream, po)
                   : launch_gemv<0, 8>(a, as, w, ws, out, M, N, K, out_f32, stream, po);
