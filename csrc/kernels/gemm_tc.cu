@@ -209,8 +209,9 @@ __global__ void __launch_bounds__(THREADS, 1) qgemm_tc_kernel(
           mbar_expect_tx(&a_full[s], mt_act * TILE_BYTES);
 #pragma unroll
           for (int t = 0; t < MT; ++t)
-            if (t < mt_act) tma_load_2d(a_s + (s * MT + t) * TILE_BYTES, &tmap_a, &a_full[s], (kb0 + kb) * BK,
-                        m0 + t * BM);
+            if (t < mt_act)
+              tma_load_2d(a_s + (s * MT + t) * TILE_BYTES, &tmap_a, &a_full[s], (kb0 + kb) * BK,
+                          m0 + t * BM);
         }
         issued = kb + 1;
       }
@@ -255,15 +256,30 @@ __global__ void __launch_bounds__(THREADS, 1) qgemm_tc_kernel(
         if (!ok) break;
         tc_fence_after();
         const uint32_t b_addr = smem_u32(b_s + sb * L::B_BYTES);
+        if (mt_act == MT) {
 #pragma unroll
-        for (int j = 0; j < BK / 32; ++j) {
-          if (probe & 1) break;
-          const uint64_t bdesc = umma_desc(b_addr + j * 32, 16, 1024);
+          for (int j = 0; j < BK / 32; ++j) {
+            if (probe & 1) break;
+            const uint64_t bdesc = umma_desc(b_addr + j * 32, 16, 1024);
 #pragma unroll
-          for (int t = 0; t < MT; ++t) {
-            const uint32_t a_addr = smem_u32(a_s + (sa * MT + t) * TILE_BYTES);
-            mma_i8_ss(tmem_base + t * BN, umma_desc(a_addr + j * 32, 16, 1024), bdesc, idesc,
-                      (kb | j) != 0 ? 1u : 0u);
+            for (int t = 0; t < MT; ++t) {
+              const uint32_t a_addr = smem_u32(a_s + (sa * MT + t) * TILE_BYTES);
+              mma_i8_ss(tmem_base + t * BN, umma_desc(a_addr + j * 32, 16, 1024), bdesc, idesc,
+                        (kb | j) != 0 ? 1u : 0u);
+            }
+          }
+        } else {
+          // an expert's last row tiles: the others are not loaded, and nobody reads them
+#pragma unroll
+          for (int j = 0; j < BK / 32; ++j) {
+            const uint64_t bdesc = umma_desc(b_addr + j * 32, 16, 1024);
+#pragma unroll
+            for (int t = 0; t < MT - 1; ++t) {
+              const uint32_t a_addr = smem_u32(a_s + (sa * MT + t) * TILE_BYTES);
+              if (t < mt_act)
+                mma_i8_ss(tmem_base + t * BN, umma_desc(a_addr + j * 32, 16, 1024), bdesc, idesc,
+                          (kb | j) != 0 ? 1u : 0u);
+            }
           }
         }
         tc_commit(&a_empty[sa]);
