@@ -161,7 +161,11 @@ void orinfer_qgemm_clear_variants();
 void orinfer_qgemm_plan(int fmt, int M, int N, int K, int out_f32, int* out);
 int orinfer_qgemm_grouped(int fmt, const int8_t* a, const float* a_scale, const void* w,
                           const __half* w_scale, void* out, int S, int N, int K, int experts,
-                          const int* tiles, const int* meta, int max_tiles, cudaStream_t stream);
+                          const int* tiles, const int* meta, int max_tiles, cudaStream_t stream,
+                          int expected, int tallest);
+// Number of kernel launches it makes.
+int orinfer_qgemm_grouped_launches(int fmt, int S, int experts, int max_tiles, int expected,
+                                   int tallest);
 
 // ---- attention over the paged INT8 KV cache
 size_t orinfer_attention_scratch_bytes(int rows, int qh, int head_dim, int splits);

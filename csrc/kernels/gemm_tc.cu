@@ -29,7 +29,8 @@ int qgemv_dispatch(int fmt, const int8_t* a, const float* as, const void* w, con
                    const PeerOut* peer);
 int qgemv_grouped_dispatch(int fmt, const int8_t* a, const float* as, const void* w,
                            const __half* ws, void* out, int N, int K, long long bank,
-                           const int* tiles, const int* meta, cudaStream_t stream);
+                           const int* tiles, const int* meta, int most_rows, int max_tiles,
+                           cudaStream_t stream);
 
 namespace tc {
 
@@ -92,6 +93,9 @@ struct GroupDesc {
   const int* meta;             // meta[0] = number of tiles
   long long w_stride;          // bytes between consecutive experts' weight banks
   int n_per_expert;            // rows of one expert's bank (= N)
+  // persistent kernel: over > 0 leaves the tiles of at most that many rows to another kernel;
+  // its list has room for `listed` of the others
+  int over = 0, listed = 0;
 };
 
 template <int FMT, bool OUT_F32, int MT, int NB>
@@ -575,7 +579,9 @@ struct PsLayout {
   static constexpr int CODE_OFF = B_OFF + SBD * B_BYTES;
   static constexpr int LUT_OFF = CODE_OFF + SC * CODE_BYTES;
   static constexpr int BAR_OFF = LUT_OFF + LUT_BYTES;
-  static constexpr int TOTAL = BAR_OFF + 512 + 1024;    // barriers + alignment slack
+  static constexpr int LIST_OFF = BAR_OFF + 512;        // list of tiles, where one is kept
+  static constexpr int TOTAL = LIST_OFF + 1024;         // alignment slack
+  static constexpr int LIST_ROOM = (226 * 1024 - TOTAL) / 4;   // entries a list may have
   static_assert(TOTAL <= 227 * 1024, "exceeds the shared memory of one CTA");
 };
 
@@ -622,7 +628,31 @@ __global__ void __launch_bounds__(THREADS, 1) qgemm_ps_kernel(
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const bool peer_stage = po.tp > 0 && partial == nullptr;
   const int n_tiles = (n_end - n_begin + BN - 1) / BN;
-  const int m_tiles = grp.tiles != nullptr ? grp.meta[0] : (M + BM * MT - 1) / (BM * MT);
+  int m_tiles = grp.tiles != nullptr ? grp.meta[0] : (M + BM * MT - 1) / (BM * MT);
+  const int* list = nullptr;                    // the table's entries that this kernel takes
+  if (grp.tiles != nullptr && grp.over > 0) {
+    int* found = reinterpret_cast<int*>(smem + L::LIST_OFF);
+    __shared__ int hits[THREADS / 32];
+    int count = 0;
+    for (int base = 0; base < m_tiles; base += THREADS) {
+      const int t = base + threadIdx.x;
+      const bool hit = t < m_tiles && grp.tiles[t * 4 + 2] > grp.over;
+      const unsigned ballot = __ballot_sync(0xffffffffu, hit);
+      if (lane == 0) hits[warp] = __popc(ballot);
+      __syncthreads();
+      int at = count + __popc(ballot & ((1u << lane) - 1u));
+#pragma unroll 1
+      for (int q = 0; q < THREADS / 32; ++q) {
+        at += q < warp ? hits[q] : 0;
+        count += hits[q];
+      }
+      if (hit && at < grp.listed) found[at] = t;
+      __syncthreads();
+    }
+    if (count == 0) return;
+    m_tiles = min(count, grp.listed);
+    list = found;
+  }
   const int total = n_tiles * m_tiles * splits;
   const int kb_all = K / BK, kb_per = (kb_all + splits - 1) / splits;
 
@@ -630,7 +660,9 @@ __global__ void __launch_bounds__(THREADS, 1) qgemm_ps_kernel(
     PsTile T;
     T.z = t / (n_tiles * m_tiles);
     const int r = t - T.z * (n_tiles * m_tiles);
-    const int nt = r / m_tiles, mi = r - nt * m_tiles;
+    const int nt = r / m_tiles;
+    int mi = r - nt * m_tiles;
+    if (list != nullptr) mi = list[mi];
     T.n0 = n_begin + nt * BN;
     T.m0 = mi * BM * MT;
     T.m_limit = M;
@@ -1499,7 +1531,7 @@ int launch_ps(const int8_t* a, const float* a_scale, const void* w, const __half
   static const int slot = runtime_new_slot();
   if (runtime_first_use(slot)) {
     cudaError_t e = cudaFuncSetAttribute(qgemm_ps_kernel<FMT, OUT_F32, MT, NB>,
-                                         cudaFuncAttributeMaxDynamicSharedMemorySize, L::TOTAL);
+                                         cudaFuncAttributeMaxDynamicSharedMemorySize, 226 * 1024);
     if (e != cudaSuccess) return static_cast<int>(e);
   }
   const int width = n_end - n_begin;
@@ -1510,7 +1542,8 @@ int launch_ps(const int8_t* a, const float* a_scale, const void* w, const __half
   const int grid = static_cast<int>(total < NUM_SMS ? total : NUM_SMS);
   int* partial = splits > 1 ? runtime_splitk_workspace() : nullptr;
   if (splits > 1 && static_cast<size_t>(splits) * M * width * 4 > SPLITK_WORKSPACE_BYTES) return -1;
-  qgemm_ps_kernel<FMT, OUT_F32, MT, NB><<<grid, THREADS, L::TOTAL, stream>>>(
+  const int smem = L::TOTAL + (grp.over > 0 ? grp.listed * 4 : 0);
+  qgemm_ps_kernel<FMT, OUT_F32, MT, NB><<<grid, THREADS, smem, stream>>>(
       ta, tb, reinterpret_cast<const unsigned char*>(w), a_scale, w_scale, out, M, N, K,
       runtime_e8p_tables(), runtime_status_ptr(), po, grp, ag, partial, n_begin, n_end, splits);
   if (splits > 1) {
@@ -1893,40 +1926,101 @@ extern "C" int orinfer_qgemm_ag(int fmt, const int8_t* a, const float* a_scale, 
   return tc::launch_fmt<2>(a, a_scale, w, w_scale, out, M, N, K, out_f32, stream, po, ag);
 }
 
-// Rows per expert, on average over the experts, up to which a grouped projection runs on the
-// small-M kernel (both projections of a layer, H = 2048).  128 Q4 experts of 768: 155 against 253 us
-// at 4 rows, 198 against 256 at 8, 258 against 256 at 12; 512 Q2 experts of 512: 155 against 535 us
-// at 1.25, 213 against 602 at 2.5, 383 against 650 at 10, 681 against 650 at 20.
-inline int grouped_gemv_rows(int fmt) { return fmt == 2 ? 18 : (fmt == 1 ? 10 : 8); }
+// Expected rows per expert, on average over the experts, up to which the small-M kernel takes
+// part.  Evenly spread rows: 128 Q4 experts of 768, both projections, 131 against 228 us at 1.5
+// rows, 200 against 286 at 8.75, tensor cores alone from 9 on (168 against 177 us for the wider
+// one at 10); 512 Q2 experts of 512 154 against 469 us at 1.25 and 420 against 655 at 10; 128 INT8
+// experts 75 against 89 us at 1.5 and 104 against 112 at 6 (wider projection).
+inline int grouped_gemv_rows(int fmt) { return fmt == 2 ? 18 : (fmt == 1 ? 9 : 7); }
+// It decodes an expert's weights once per sixteen rows, so a mean says little where routing is
+// skewed: 110 rows of which most go to a few of 128 Q4 experts took 294 us on it alone and 92 on
+// tensor cores alone.  Tiles of more rows than this therefore go to the persistent tensor-core
+// kernel, in a second launch (102 us; all rows to the same eight experts 74 -> 22; 3 us more where
+// no tile is that tall).  Each kernel finds its tiles on the device.
+constexpr int GROUPED_SMALL = 16;
+// Below so many rows an expert, of all that a launch could give to one, the split does not pay.
+// E8P, 20 rows with half of the experts' tiles on either side: 128 Q4 experts of 768 30 against 34
+// us, 24 rows on eight experts 24 against 30; 512 Q2 experts 21 against 25.  INT8 has no tables to
+// fill and pays for a second pass over the weights: 54 against 41 us at 20 skewed rows.
+inline int grouped_alone(int fmt) { return fmt == 0 ? GROUPED_SMALL : 24; }
 
 // Grouped expert GEMM: rows of `a` are sorted by expert; tile t of the table covers rows
 // [first, first + valid) of expert e, multiplied with that expert's bank.  out is fp16 [S, N].
+// S bounds the rows of all tiles.  expected: how many there will be (0: S); tallest: most rows that
+// one expert can have (0: S).  Both only choose the kernels.
+struct GroupedPlan {
+  bool rows_kernel;            // the small-M kernel, all tiles or those of few rows
+  int listed;                  // > 0: the persistent kernel takes the others, at most so many
+};
+static GroupedPlan grouped_plan(int fmt, int S, int experts, int max_tiles, int expected,
+                                int tallest) {
+  if (expected <= 0 || expected > S) expected = S;
+  if (tallest <= 0 || tallest > S) tallest = S;
+  if (expected > static_cast<long long>(grouped_gemv_rows(fmt)) * experts) return {false, 0};
+  if (tallest <= grouped_alone(fmt)) return {true, 0};
+  const int tall = S / (GROUPED_SMALL + 1);
+  const int room = fmt == 0 ? tc::PsLayout<0, 1, 128>::LIST_ROOM
+                   : fmt == 1 ? tc::PsLayout<1, 1, 128>::LIST_ROOM
+                              : tc::PsLayout<2, 1, 128>::LIST_ROOM;
+  // both kernels list their tiles in shared memory
+  return tall > room || max_tiles > 16384 ? GroupedPlan{false, 0} : GroupedPlan{true, tall};
+}
+
+template <int FMT>
+static int qgemm_grouped_fmt(const int8_t* a, const float* a_scale, const void* w,
+                             const __half* w_scale, void* out, int S, int N, int K, int experts,
+                             const int* tiles, const int* meta, int max_tiles, int expected,
+                             int tallest, cudaStream_t stream) {
+  const long long bank = FMT == 0 ? static_cast<long long>(N) * K
+                                  : static_cast<long long>(K / 128) * N * (FMT == 1 ? 64 : 32);
+  tc::GroupDesc g{tiles, meta, bank, N};
+  const PeerOut po{};
+  const GroupedPlan plan = grouped_plan(FMT, S, experts, max_tiles, expected, tallest);
+  if (plan.rows_kernel) {
+    const int r = qgemv_grouped_dispatch(FMT, a, a_scale, w, w_scale, out, N, K, bank, tiles, meta,
+                                         plan.listed > 0 ? GROUPED_SMALL : 0, max_tiles, stream);
+    if (r || plan.listed == 0) return r;
+    g.over = GROUPED_SMALL;
+    g.listed = plan.listed;
+    const AgIn ag{nullptr, nullptr, 0, 0};
+    return tc::launch_ps<FMT, false, 1, 128>(a, a_scale, w, w_scale, out, S, N, K, stream, po, g,
+                                             experts, plan.listed < max_tiles ? plan.listed
+                                                                              : max_tiles,
+                                             ag, 1, 0, N);
+  }
+  // Row tiles of one expert per CTA: two where experts have about half a tile of rows or more (INT8
+  // nearly a whole one: nothing to decode, so a second tile only saves the copy of the weights),
+  // four where they have several.
+  const long long two = (FMT == 0 ? 112LL : 64LL) * experts;
+  const int mt = tc::g_impl != 1 ? 1 : (expected >= 256LL * experts ? 4 : (expected >= two ? 2 : 1));
+  if (mt == 4)
+    return tc::launch<FMT, false, 4, 128>(a, a_scale, w, w_scale, out, S, N, K, stream, po, g,
+                                          experts, max_tiles);
+  if (mt == 2)
+    return tc::launch<FMT, false, 2, 128>(a, a_scale, w, w_scale, out, S, N, K, stream, po, g,
+                                          experts, max_tiles);
+  return tc::launch<FMT, false, 1, 128>(a, a_scale, w, w_scale, out, S, N, K, stream, po, g, experts,
+                                        max_tiles);
+}
+
 extern "C" int orinfer_qgemm_grouped(int fmt, const int8_t* a, const float* a_scale, const void* w,
                                      const __half* w_scale, void* out, int S, int N, int K,
-                                     int experts, const int* tiles, const int* meta,
-                                     int max_tiles, cudaStream_t stream) {
+                                     int experts, const int* tiles, const int* meta, int max_tiles,
+                                     cudaStream_t stream, int expected, int tallest) {
   if (S <= 0 || max_tiles <= 0) return 0;
   if (K <= 0 || K % 128 || N % 128 || fmt < 0 || fmt > 2 || experts < 1) return -1;
   if (runtime_ensure_init() != cudaSuccess) return -2;
-  const long long bank = fmt == 0 ? static_cast<long long>(N) * K
-                                  : static_cast<long long>(K / 128) * N * (fmt == 1 ? 64 : 32);
-  // Few rows per expert: the tile table mostly holds tiles of one or two rows.
-  if (S <= static_cast<long long>(grouped_gemv_rows(fmt)) * experts)
-    return qgemv_grouped_dispatch(fmt, a, a_scale, w, w_scale, out, N, K, bank, tiles, meta, stream);
-  tc::GroupDesc g{tiles, meta, bank, N};
-  const PeerOut po{};
-  // Row tiles of one expert per CTA: two where experts have about a tile of rows (half of them
-  // then have a second, nearly empty one), four where they have several.
-  const int mt = tc::g_impl != 1 ? 1 : (S >= 256LL * experts ? 4 : (S >= 64LL * experts ? 2 : 1));
-#define ORINFER_GROUPED(FMT)                                                                       \
-  return mt == 4   ? tc::launch<FMT, false, 4, 128>(a, a_scale, w, w_scale, out, S, N, K, stream,  \
-                                                    po, g, experts, max_tiles)                     \
-         : mt == 2 ? tc::launch<FMT, false, 2, 128>(a, a_scale, w, w_scale, out, S, N, K, stream,  \
-                                                    po, g, experts, max_tiles)                     \
-                   : tc::launch<FMT, false, 1, 128>(a, a_scale, w, w_scale, out, S, N, K, stream,  \
-                                                    po, g, experts, max_tiles)
+  if (expected <= 0 || expected > S) expected = S;
+#define ORINFER_GROUPED(FMT)                                                                  \
+  return qgemm_grouped_fmt<FMT>(a, a_scale, w, w_scale, out, S, N, K, experts, tiles, meta,   \
+                                max_tiles, expected, tallest, stream)
   if (fmt == 0) ORINFER_GROUPED(0);
   if (fmt == 1) ORINFER_GROUPED(1);
   ORINFER_GROUPED(2);
 #undef ORINFER_GROUPED
+}
+
+extern "C" int orinfer_qgemm_grouped_launches(int fmt, int S, int experts, int max_tiles,
+                                              int expected, int tallest) {
+  return grouped_plan(fmt, S, experts, max_tiles, expected, tallest).listed > 0 ? 2 : 1;
 }

@@ -68,6 +68,7 @@ __device__ __forceinline__ void store_row(void* out, int out_f32, int m, int n, 
 // overlap on the device (they are issued on one stream).
 constexpr int GEMV_COPIES = 32;
 constexpr int GEMV_THREADS = 1024;
+constexpr size_t GEMV_SMEM_LIMIT = 220 * 1024;
 
 __device__ __forceinline__ void mma_i8_16832(int (&c)[4], uint32_t a0, uint32_t a1, uint32_t a2,
                                              uint32_t a3, uint32_t b0, uint32_t b1) {
@@ -729,19 +730,31 @@ __global__ void __launch_bounds__(W8_WARPS * 32) w8_gemv_kernel(
 // whole K, weights as A and up to eight activation rows as B as above; the activations are read
 // from global memory with the weights (a tile's rows are shared by the warps of a CTA through
 // L1).  Tiles of more rows repeat the decode once per sixteen rows.
+constexpr int GROUPED_CTAS = 148;
+
+__device__ __forceinline__ int warp_scan(int v) {              // sums of lanes 0..l
+#pragma unroll
+  for (int o = 1; o < 32; o <<= 1) {
+    const int up = __shfl_up_sync(0xffffffffu, v, o);
+    if ((threadIdx.x & 31) >= static_cast<unsigned>(o)) v += up;
+  }
+  return v;
+}
+
 template <int FMT>
 struct ExpertUnit {
   GemvUnit<FMT> u;
   uint4 act[2];                                    // this lane's 32 bytes of activation row g
 };
 
-template <int FMT>
+// MIXED takes the tiles of at most most_rows rows and leaves the others to another kernel.
+template <int FMT, bool MIXED>
 __global__ void __launch_bounds__(GEMV_THREADS, 1) qgemv_grouped_kernel(
     const int8_t* __restrict__ a, const float* __restrict__ a_scale,
     const unsigned char* __restrict__ w, const __half* __restrict__ w_scale,
     __half* __restrict__ out, int N, int K, long long bank_bytes,
     const E8pTables* __restrict__ tables, const int* __restrict__ tiles,
-    const int* __restrict__ meta) {
+    const int* __restrict__ meta, int most_rows, int listed) {
   using Lut = E8pLut<GEMV_COPIES>;
   using W = GemvUnit<FMT>;
   constexpr int NB = 2;                            // eight-row blocks per pass over the weights
@@ -751,13 +764,43 @@ __global__ void __launch_bounds__(GEMV_THREADS, 1) qgemv_grouped_kernel(
   int(*red)[NB * 5][32] = reinterpret_cast<int(*)[NB * 5][32]>(
       smem_raw + (FMT == 0 ? 0 : sizeof(Lut)));        // [WARPS]
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, g = lane >> 2, t = lane & 3;
-  if (FMT != 0) e8p_lut_init(lut, tables, tid, GEMV_THREADS);
+  // MIXED lists its tiles in shared memory before the tables are filled: there may be none.
+  if (FMT != 0 && !MIXED) e8p_lut_init(lut, tables, tid, GEMV_THREADS);
+  int n_tiles = meta[0];
+  const int* list = nullptr;
+  if (MIXED && most_rows > 0) {
+    int* found = reinterpret_cast<int*>(&red[WARPS]);
+    __shared__ int hits[WARPS];
+    int count = 0;
+    for (int base = 0; base < n_tiles; base += GEMV_THREADS) {
+      const int at = base + tid;
+      const bool hit = at < n_tiles && __ldg(tiles + at * 4 + 2) <= most_rows;
+      const unsigned ballot = __ballot_sync(0xffffffffu, hit);
+      if (lane == 0) hits[warp] = __popc(ballot);
+      __syncthreads();
+      const int inc = warp_scan(hits[lane]);                // of the warps up to this lane's
+      const int before = __shfl_sync(0xffffffffu, inc, warp) - hits[warp];
+      const int slot = count + before + __popc(ballot & ((1u << lane) - 1u));
+      if (hit && slot < listed) found[slot] = at;
+      count += __shfl_sync(0xffffffffu, inc, 31);
+      __syncthreads();
+    }
+    if (count == 0) return;
+    n_tiles = min(count, listed);
+    list = found;
+    if (FMT != 0) e8p_lut_init(lut, tables, tid, GEMV_THREADS);
+  }
   __syncthreads();
-  const int groups = N / 16, kbs = K / 128, items = meta[0] * groups;
+  const int groups = N / 16, kbs = K / 128, items = n_tiles * groups;
   // With fewer items than warps (a decode step of one or two rows) KS neighbouring warps share
   // an item's K and the first of them adds the parts: the walk over K is a chain of loads.
+  // Two share it where whole items would leave a second round to a third of the warps or fewer.
   int ks = 1;
   while (ks < 8 && kbs >= 4 * ks && items * ks * 2 <= static_cast<int>(gridDim.x) * WARPS) ks *= 2;
+  if (MIXED) {
+    constexpr int ALL = GROUPED_CTAS * WARPS;
+    if (kbs >= 4 && items > ALL && items <= ALL + ALL / 3) ks = 2;
+  }
   const int sub = warp % ks, kb_lo = kbs * sub / ks, kb_hi = kbs * (sub + 1) / ks;
   const int stride = gridDim.x * (WARPS / ks);
   constexpr int UNIT = FMT == 0 ? 1 : 2, BIAS = FMT == 0 ? 0 : (FMT == 1 ? 75 : 15);
@@ -765,7 +808,8 @@ __global__ void __launch_bounds__(GEMV_THREADS, 1) qgemv_grouped_kernel(
   const int piece0 = FMT == 0 ? t * 16 : t * 32, piece1 = FMT == 0 ? 64 + t * 16 : t * 32 + 16;
 
   for (int item = blockIdx.x * (WARPS / ks) + warp / ks; item < items; item += stride) {
-    const int tile = item / groups, n0 = (item - tile * groups) * 16;
+    const int at = item / groups, n0 = (item - at * groups) * 16;
+    const int tile = MIXED && list != nullptr ? list[at] : at;
     const int expert = __ldg(tiles + tile * 4), first = __ldg(tiles + tile * 4 + 1);
     const int rows = __ldg(tiles + tile * 4 + 2);
     const unsigned char* bank = w + static_cast<size_t>(expert) * bank_bytes;
@@ -909,30 +953,37 @@ __global__ void __launch_bounds__(GEMV_THREADS, 1) qgemv_grouped_kernel(
   }
 }
 
-template <int FMT>
+template <int FMT, bool MIXED>
 static int launch_grouped(const int8_t* a, const float* as, const void* w, const __half* ws,
                           void* out, int N, int K, long long bank, const int* tiles,
-                          const int* meta, cudaStream_t stream) {
-  const size_t smem = (FMT == 0 ? 0 : sizeof(E8pLut<GEMV_COPIES>)) + GEMV_THREADS * 10 * sizeof(int);
+                          const int* meta, int most_rows, int max_tiles, cudaStream_t stream) {
+  const int listed = most_rows > 0 ? max_tiles : 0;
+  const size_t smem = (FMT == 0 ? 0 : sizeof(E8pLut<GEMV_COPIES>)) +
+                      (static_cast<size_t>(GEMV_THREADS) * 10 + listed) * sizeof(int);
+  if (smem > GEMV_SMEM_LIMIT) return -1;
   static const int slot = runtime_new_slot();
   if (runtime_first_use(slot)) {
-    cudaError_t e = cudaFuncSetAttribute(qgemv_grouped_kernel<FMT>,
+    cudaError_t e = cudaFuncSetAttribute(qgemv_grouped_kernel<FMT, MIXED>,
                                          cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                         static_cast<int>(smem));
+                                         static_cast<int>(MIXED ? GEMV_SMEM_LIMIT : smem));
     if (e != cudaSuccess) return static_cast<int>(e);
   }
-  qgemv_grouped_kernel<FMT><<<148, GEMV_THREADS, smem, stream>>>(
+  qgemv_grouped_kernel<FMT, MIXED><<<GROUPED_CTAS, GEMV_THREADS, smem, stream>>>(
       a, as, reinterpret_cast<const unsigned char*>(w), ws, reinterpret_cast<__half*>(out), N, K,
-      bank, runtime_e8p_tables(), tiles, meta);
+      bank, runtime_e8p_tables(), tiles, meta, most_rows, listed);
   return static_cast<int>(cudaGetLastError());
 }
 
 int qgemv_grouped_dispatch(int fmt, const int8_t* a, const float* as, const void* w,
                            const __half* ws, void* out, int N, int K, long long bank,
-                           const int* tiles, const int* meta, cudaStream_t stream) {
-  if (fmt == 0) return launch_grouped<0>(a, as, w, ws, out, N, K, bank, tiles, meta, stream);
-  if (fmt == 1) return launch_grouped<1>(a, as, w, ws, out, N, K, bank, tiles, meta, stream);
-  return launch_grouped<2>(a, as, w, ws, out, N, K, bank, tiles, meta, stream);
+                           const int* tiles, const int* meta, int most_rows, int max_tiles,
+                           cudaStream_t stream) {
+  // INT8 has the one form for both: its loop comes out better with the list (128 experts of 1536 x
+  // 2048, 14 skewed rows: 31 us against 36); the E8P forms pay 0.4 us of 6 for it.
+  const auto run = fmt == 0   ? launch_grouped<0, true>
+                   : fmt == 1 ? (most_rows > 0 ? launch_grouped<1, true> : launch_grouped<1, false>)
+                              : (most_rows > 0 ? launch_grouped<2, true> : launch_grouped<2, false>);
+  return run(a, as, w, ws, out, N, K, bank, tiles, meta, most_rows, max_tiles, stream);
 }
 
 // Grid shape: n_parts x k_parts CTAs on the 148 SMs.  E8P projections may split K (2, 4 or 8
@@ -965,8 +1016,6 @@ static GemvGrid gemv_grid(int fmt, int N, int K) {
   best.max_groups = ((oct + best.n_parts - 1) / best.n_parts + 1) / 2;
   return best;
 }
-
-constexpr size_t GEMV_SMEM_LIMIT = 220 * 1024;
 
 // Whether an E8P projection runs on e8p_dp4a_kernel: where it was the quicker of the two, over 250
 // to 19456 columns x 1024 to 9728 channels, alone and with each row preparation.

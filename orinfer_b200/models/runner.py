@@ -509,13 +509,14 @@ class ModelRunner:
         else:
             F.moe_dispatch(sc.ids, q8, s8, cfg.experts, sc, rows, bank_up.base, bank_up.experts)
         total = rows * cfg.top_k
+        expected = total if pager is not None else total * bank_up.experts // cfg.experts
         F.qgemm_grouped(sc.q8, sc.scale, bank_up.codes, bank_up.scale, bank_up.fmt, 2 * f,
-                        sc.gate_up, sc, total)
+                        sc.gate_up, sc, total, expected)
         # offsets[n_local_experts] = rows actually routed to this rank's experts
         F.act_prep_limited(sc.gate_up, bank_dn.signs, sc.offsets[bank_up.experts:], swiglu=True,
                            rows=total, q_out=sc.q8_mid, scale_out=sc.scale_mid)
         F.qgemm_grouped(sc.q8_mid, sc.scale_mid, bank_dn.codes, bank_dn.scale, bank_dn.fmt, h,
-                        sc.down, sc, total)
+                        sc.down, sc, total, expected)
         shared = None
         tp = getattr(self.w, "tp", None)
         if lw.shared_gate_up is not None and (tp is None or lw.shared_owner in (-1, tp.rank)):

@@ -311,13 +311,20 @@ def moe_dispatch(ids: torch.Tensor, q8: Optional[torch.Tensor], scale: Optional[
 
 def qgemm_grouped(a: torch.Tensor, a_scale: torch.Tensor, codes: torch.Tensor,
                   w_scale: torch.Tensor, fmt: str, n: int, out: torch.Tensor, sc: MoeScratch,
-                  total_rows: int) -> torch.Tensor:
+                  total_rows: int, expected_rows: Optional[int] = None) -> torch.Tensor:
+    """Grouped projection over the dispatched rows of ``sc``.  ``total_rows`` bounds them; where
+    it is far above the rows that this bank will get (its share of the experts, receive buffers
+    sized for the worst case) ``expected_rows`` says how many to expect.  The choice of kernels
+    follows it, and that a row goes to an expert once."""
     experts = codes.shape[0]
+    expected = total_rows if expected_rows is None else max(1, expected_rows)
+    tallest = total_rows // sc.ids.shape[1]
     check(native.lib().orinfer_qgemm_grouped(
         FMT[fmt], ptr(a), ptr(a_scale), ptr(codes), ptr(w_scale), ptr(out), total_rows, n,
-        a.shape[1], experts, ptr(sc.tiles), ptr(sc.meta), sc.max_tiles, stream()),
-        "qgemm_grouped")
-    count_launches(1)
+        a.shape[1], experts, ptr(sc.tiles), ptr(sc.meta), sc.max_tiles, stream(), expected,
+        tallest), "qgemm_grouped")
+    count_launches(native.lib().orinfer_qgemm_grouped_launches(FMT[fmt], total_rows, experts,
+                                                               sc.max_tiles, expected, tallest))
     return out
 
 

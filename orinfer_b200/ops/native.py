@@ -59,7 +59,8 @@ def _load() -> ctypes.CDLL:
         "orinfer_router_topk": ([P, P, I, I, I, I, I, I, P, P, P, P], I),
         "orinfer_moe_dispatch": ([P, I, I, I, P, P, I, P, P, P, P, I, P, P, P, P], I),
         "orinfer_moe_combine": ([P, P, P, I, I, P, P, P, I, P], I),
-        "orinfer_qgemm_grouped": ([I, P, P, P, P, P, I, I, I, I, P, P, I, P], I),
+        "orinfer_qgemm_grouped": ([I, P, P, P, P, P, I, I, I, I, P, P, I, P, I, I], I),
+        "orinfer_qgemm_grouped_launches": ([I, I, I, I, I, I], I),
         "orinfer_moe_dispatch_ep": ([P, I, I, I, I, P, P, I, P, P, P, P, I, P, P, P, P], I),
         "orinfer_sample_topk": ([P, I, I, c_longlong, P, P, P, P, P, P, P], I),
         "orinfer_qgemm_launches": ([I, I, I, I, I], I),

@@ -154,12 +154,13 @@ class ExpertA2A:
         be, total = self.by_expert, tp * cap
         F.moe_dispatch(self.recv_expert, self.recv_rows, self.recv_scale, self.experts_total, be,
                        total, up.base, self.local_experts)
+        # the receive buffers are sized for the worst case: expect what this rank sends away
         F.qgemm_grouped(be.q8, be.scale, up.codes, up.scale, up.fmt, 2 * self.ffn, be.gate_up, be,
-                        total)
+                        total, rows * self.top_k)
         F.act_prep_limited(be.gate_up, dn.signs, be.offsets[self.local_experts:], swiglu=True,
                            rows=total, q_out=be.q8_mid, scale_out=be.scale_mid)
         F.qgemm_grouped(be.q8_mid, be.scale_mid, dn.codes, dn.scale, dn.fmt, self.h, be.down, be,
-                        total)
+                        total, rows * self.top_k)
         # 4. combine all-to-all
         check(lib.orinfer_a2a_return_push(ptr(be.down), ptr(be.slots), self._p["header"], self.h,
                                           ctypes.byref(self.r), s), "a2a_return_push")

@@ -25,6 +25,11 @@ def _int_weight(fmt, n, k, g):
     return codes, scale, QLinear(fmt, n, k, codes, scale, None).integers()
 
 
+def _int_weight_of(fmt, codes, scale, n, k):
+    from orinfer_b200.models.weights import QLinear
+    return QLinear(fmt, n, k, codes, scale, None).integers()
+
+
 def _scaled(a, sa, w, ws):
     """The integer product with its two FP32 scales, in the kernels' order."""
     acc = (a.double() @ w.double().t()).float()
@@ -143,3 +148,86 @@ def test_grouped_projection_is_exact(dev, fmt, counts, n, k):
                            banks[e][1].to(dev))
             assert torch.equal(out[at:at + c], want.half()), e
         at += c
+
+
+@pytest.mark.parametrize("fmt", ["w8", "q4", "q2"])
+@pytest.mark.parametrize("experts,rows,top_k,tall", [
+    (1100, 40, 3, [5]), (1100, 300, 2, [0, 1, 600, 1024, 1099]), (64, 25, 4, [3, 63]),
+    (64, 17, 4, [3, 63]), (16, 100, 1, [9]), (40, 130, 2, [0, 39])])
+@pytest.mark.parametrize("expected", [None, 1])
+def test_grouped_projection_splits_by_tile_height(dev, fmt, experts, rows, top_k, tall, expected):
+    """Few rows per expert but many for some: every row is written, by one kernel or the other,
+    over tile lists of more entries than a CTA has threads and experts of several tiles."""
+    from orinfer_b200.ops import functional as F
+    n = k = 128
+    g = torch.Generator().manual_seed(experts + rows)
+    ids = torch.stack([torch.randperm(experts, generator=g)[:top_k] for _ in range(rows)])
+    for r in range(rows - 3):                              # most rows go to the tall experts too
+        e = tall[r % len(tall)]
+        if e not in ids[r]:
+            ids[r, 0] = e
+    codes, ws, _ = _int_weight(fmt, experts * n, k, g)
+    split = [codes[i * n:(i + 1) * n] if fmt == "w8" else codes[:, i * n:(i + 1) * n]
+             for i in range(experts)]
+    ints = _int_weight_of(fmt, codes, ws, experts * n, k).to(dev)
+    a = torch.randint(-127, 128, (rows, k), generator=g, dtype=torch.int8).to(dev)
+    sa = (torch.rand(rows, generator=g) * 0.05 + 1e-3).to(dev)
+    sc = F.MoeScratch(rows, top_k, experts, k, 64, dev)
+    F.moe_dispatch(ids.to(torch.int32).to(dev), a, sa, experts, sc, rows)
+    out = torch.full((rows * top_k, n), float("nan"), dtype=torch.float16, device=dev)
+    F.qgemm_grouped(sc.q8, sc.scale, torch.stack(split).contiguous().to(dev),
+                    ws.view(experts, n).to(dev), fmt, n, out, sc, rows * top_k, expected)
+    flat = ids.flatten()
+    order = torch.sort(flat, stable=True).indices.to(dev)
+    flat = flat.to(dev)
+    src = a[order // top_k].double()
+    acc = torch.einsum("rk,rnk->rn", src, ints.view(experts, n, k)[flat[order]].double()).float()
+    want = acc * ws.view(experts, n).to(dev)[flat[order]].float() * sa[order // top_k, None]
+    assert torch.equal(out, want.half())
+
+
+def _grouped_us(dev, ids, experts, n, k, fmt, banks):
+    from orinfer_b200.ops import functional as F
+    rows, top_k = ids.shape
+    sc = F.MoeScratch(rows, top_k, experts, k, 64, dev)
+    a = torch.randint(-127, 128, (rows, k), dtype=torch.int8, device=dev)
+    F.moe_dispatch(ids.to(torch.int32).to(dev), a, torch.rand(rows, device=dev), experts, sc, rows)
+    out = torch.empty(rows * top_k, n, dtype=torch.float16, device=dev)
+    times = []
+    for _ in range(15):
+        b, e = torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True)
+        b.record()
+        for _ in range(10):
+            F.qgemm_grouped(sc.q8, sc.scale, banks[0], banks[1], fmt, n, out, sc, rows * top_k)
+        e.record()
+        e.synchronize()
+        times.append(b.elapsed_time(e) * 100)
+    return sorted(times)[len(times) // 2]
+
+
+@pytest.mark.parametrize("fmt", ["w8", "q4", "q2"])
+def test_grouped_projection_takes_skew(dev, fmt):
+    """Rows that crowd on a few experts read fewer weights than evenly spread ones: they take no
+    longer.  (A kernel that walks each expert's weights once per sixteen rows took 2.5 times as
+    long; the margin is for the clock.)"""
+    experts, n, k, rows, top_k = 128, 1536, 2048, 110, 8
+    g = torch.Generator().manual_seed(1)
+    codes, ws, _ = _int_weight(fmt, n, k, g)
+    banks = (codes[None].expand(experts, *codes.shape).contiguous().to(dev),
+             ws[None].expand(experts, n).contiguous().to(dev))
+    even = torch.stack([torch.randperm(experts, generator=g)[:top_k] for _ in range(rows)])
+    weight = 1.0 / torch.arange(1, experts + 1).float() ** 1.2
+    skew = torch.stack([torch.multinomial(weight, top_k, generator=g) for _ in range(rows)])
+    t = [_grouped_us(dev, i, experts, n, k, fmt, banks) for i in (even, skew)]
+    assert t[1] < 1.25 * t[0], t
+
+
+def test_grouped_projection_follows_expected_rows():
+    """The choice of kernels follows the rows to be expected, not the room for them."""
+    from orinfer_b200.ops import native
+    lib = native.lib()
+    # 16 experts, room for 4096 rows of top 8: tensor cores alone (one launch) ...
+    assert lib.orinfer_qgemm_grouped_launches(1, 4096, 16, 48, 4096, 512) == 1
+    # ... with 64 expected both kernels, and one where no expert can have many
+    assert lib.orinfer_qgemm_grouped_launches(1, 4096, 16, 48, 64, 512) == 2
+    assert lib.orinfer_qgemm_grouped_launches(1, 128, 16, 48, 64, 16) == 1
