@@ -120,6 +120,34 @@ def test_moe_dispatch_numbers_and_copies(dev, experts, rows, top_k, k, part):
     assert torch.equal(sc.scale[:kept].cpu(), scale.cpu()[src])
 
 
+@pytest.mark.parametrize("local", [4, 12])
+@pytest.mark.parametrize("k", [16, 2048, 4112])
+def test_moe_dispatch_of_a_mostly_free_buffer(dev, local, k):
+    """One slot a row, most of them free (-1) or of another rank: the free rows' values and
+    scales, here never written, go nowhere."""
+    from orinfer_b200.ops import functional as F
+    rows, base = 700, 0 if local == 12 else 3
+    g = torch.Generator().manual_seed(k)
+    ids = torch.full((rows, 1), -1, dtype=torch.int32)
+    live = torch.randperm(rows, generator=g)[:30]
+    ids[live, 0] = torch.randint(0, 12, (30,), generator=g, dtype=torch.int32)
+    q8 = torch.full((rows, k), -128, dtype=torch.int8)
+    scale = torch.full((rows,), float("nan"))
+    q8[live] = torch.randint(-127, 128, (30, k), generator=g, dtype=torch.int8)
+    scale[live] = torch.rand(30, generator=g)
+    sc = F.MoeScratch(rows, 1, 12, k, 64, dev)
+    sc.q8.fill_(7)
+    sc.scale.fill_(7.0)
+    F.moe_dispatch(ids.to(dev), q8.to(dev), scale.to(dev), 12, sc, rows, base, local)
+    flat = ids.flatten() - base
+    flat = torch.where((flat >= 0) & (flat < local) & (ids.flatten() >= 0), flat, local)
+    kept = int((flat < local).sum())
+    order = torch.sort(flat, stable=True).indices[:kept]
+    assert torch.equal(sc.q8[:kept].cpu(), q8[order])
+    assert torch.equal(sc.scale[:kept].cpu(), scale[order])
+    assert bool((sc.q8[kept:] == 7).all()) and bool((sc.scale[kept:] == 7.0).all())
+
+
 # few rows per expert (small-M kernel, K shared by several warps or not), a tile of rows and
 # several tiles of rows per expert (one, two or four row tiles per CTA)
 @pytest.mark.parametrize("fmt", ["w8", "q4", "q2"])
