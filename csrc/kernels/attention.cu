@@ -73,7 +73,8 @@ struct RowScales {
 //   is laid out to match).  Each group of 64 channels is summed by itself and scaled in FP32.
 //   O = P V: the FP32 weight x value scale is split into an FP16 head and an FP16 remainder
 //   in rows g and g + 8 of the same A tile, so the split costs no instruction and keeps 22
-//   bits.  The weights are scaled by a power of two (2^14 over the largest value scale seen,
+//   bits (error against 64 bits as with FP32 products: 2.07e-4 both, the FP16 result's
+//   rounding).  The weights are scaled by a power of two (2^14 over the largest value scale seen,
 //   exact) so that the remainder stays above the smallest FP16 step.
 //
 // The first form converted every byte to FP32 and multiplied it once per query head on the CUDA
@@ -86,7 +87,7 @@ template <int D>
 struct AttnTile {
   static constexpr int G = D / 64;                 // scale groups per row
   static constexpr int KB = D == 256 ? 16 : 32;    // keys per block
-  static constexpr int MIN_CTAS = D == 256 ? 2 : 3;
+  static constexpr int MIN_CTAS = D == 256 ? 2 : D == 128 ? 3 : 4;   // resident per SM
   static constexpr int CPK = D / 16;               // 16-byte units of a key row
   static constexpr int STAGE = 2 * KB * D;         // K and V rows of one block
   static constexpr int RING = ATTN_WARPS * 2 * STAGE;          // two stages per warp
@@ -101,23 +102,41 @@ struct AttnTile {
   }
 };
 
+__device__ __forceinline__ void attn_store(float v, const __half* gate, __half* out, size_t at) {
+  if (gate) v *= __fdiv_rn(1.f, 1.f + expf(-__half2float(gate[at])));
+  out[at] = __float2half_rn(v);
+}
+
 __device__ __forceinline__ void cp_async16(uint32_t smem, const void* gmem) {
   asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(smem), "l"(gmem) : "memory");
 }
 
-template <int D, bool WIDE>
-__global__ void __launch_bounds__(ATTN_WARPS * 32, AttnTile<D>::MIN_CTAS) attn_rows_kernel(
+// APART: rows of at most apart_keys keys have only a few blocks, of which a warp of a CTA gets one
+// or none, and a large launch of them is bound by its waves of CTAs.  Four KV heads then share the
+// CTA of the first of them, a warp each, and the other three CTAs return at once.  Used for up to
+// as many blocks (four at most) as the launch has waves: a warp then walks them in less time than
+// three waves of CTAs take.  16 query / 16 KV heads of 128, 512 rows: about 30 keys 71 -> 33 us,
+// 120 keys 87 -> 62; 32 / 8, 128 rows of 64 keys 13.2 -> 12.3, but 64 rows (no second wave) 9.0 ->
+// 9.9; fewer than four KV heads leave warps idle (16 / 2 of 256, 512 rows of 60 keys 28 -> 30).
+// Longer rows of such a launch pay up to 3 % for the form (8 / 8 of 64, 128 rows of 640 keys).
+template <int D, bool WIDE, bool APART>
+__global__ void __launch_bounds__(
+    ATTN_WARPS * 32, D == 64 && !APART ? 3 : AttnTile<D>::MIN_CTAS) attn_rows_kernel(
     const __half* __restrict__ q, const __half* __restrict__ gate, const int* __restrict__ row_req,
     const int* __restrict__ row_pos, const int* __restrict__ page_table, int max_pages,
     const int8_t* __restrict__ kc, const int8_t* __restrict__ vc, const __half* __restrict__ ks,
     const __half* __restrict__ vs, __half* __restrict__ out, int qh, int kvh, int splits,
-    float* __restrict__ scratch, int rep) {
+    float* __restrict__ scratch, int rep, int apart_keys) {
   constexpr int G = AttnTile<D>::G, KB = AttnTile<D>::KB;
   constexpr int NT = KB / 8, UT = KB / 16;         // 8-key score tiles, 16-key value tiles
-  const int row = blockIdx.x, h = blockIdx.y, split = blockIdx.z;
+  const int row = blockIdx.x, split = blockIdx.z;
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   const int g = lane >> 2, t = lane & 3;
   const int kv_len = row_pos[row] + 1;
+  const bool apart = APART && kv_len <= apart_keys;
+  if (apart && (blockIdx.y & (ATTN_WARPS - 1)) != 0) return;
+  const int h = apart ? min(static_cast<int>(blockIdx.y) + warp, kvh - 1) : blockIdx.y;
+  const bool idle = apart && static_cast<int>(blockIdx.y) + warp >= kvh;
   const int per = (kv_len + splits - 1) / splits;
   const int k_lo = split * per, k_hi = min(kv_len, k_lo + per);
   const int* pages = page_table + static_cast<size_t>(row_req[row]) * max_pages;
@@ -128,10 +147,11 @@ __global__ void __launch_bounds__(ATTN_WARPS * 32, AttnTile<D>::MIN_CTAS) attn_r
   float(*s_o)[8][D] = reinterpret_cast<float(*)[8][D]>(attn_smem);
   __shared__ float s_m[ATTN_WARPS][8], s_l[ATTN_WARPS][8];
 
-  // Query fragments in shared memory, one copy for the four warps (16 or 32 registers per lane
-  // buy more loads in flight): halves 4s..4s+3 of a lane's 16 are the A registers of step s.
-  __shared__ __align__(16) uint4 s_q[G][2][32];
-  if (warp == 0) {
+  // Query fragments in shared memory, one copy for the four warps of a head (16 or 32 registers per
+  // lane buy more loads in flight): halves 4s..4s+3 of a lane's 16 are the A registers of step s.
+  __shared__ __align__(16) uint4 s_qs[APART ? ATTN_WARPS : 1][G][2][32];
+  uint4(*s_q)[2][32] = s_qs[apart ? warp : 0];
+  if (warp == 0 || apart) {
 #pragma unroll
     for (int c = 0; c < G; ++c) {
       const __half* p = q + (static_cast<size_t>(row) * qh + h * rep + g) * D + c * 64 + t * 16;
@@ -161,8 +181,9 @@ __global__ void __launch_bounds__(ATTN_WARPS * 32, AttnTile<D>::MIN_CTAS) attn_r
   float m_run = -INFINITY, l_run = 0.f;
   int e_run = -100;                                // the value scales seen are below 2^e_run
 
-  const int b_hi = k_hi > k_lo ? (k_hi + KB - 1) / KB : 0;
-  int b = k_hi > k_lo ? k_lo / KB + warp : 0;
+  const int step = apart ? 1 : ATTN_WARPS;
+  const int b_hi = k_hi > k_lo && !idle ? (k_hi + KB - 1) / KB : 0;
+  int b = k_hi > k_lo ? k_lo / KB + (apart ? 0 : warp) : 0;
   // This warp's ring: the block being used and the next one, copied in by cp.async (8 KB in
   // flight per warp without a register).  Lane l also holds the scales of key l of both.
   const uint32_t ring = smem_u32(attn_smem) + warp * 2 * T::STAGE;
@@ -187,15 +208,15 @@ __global__ void __launch_bounds__(ATTN_WARPS * 32, AttnTile<D>::MIN_CTAS) attn_r
     vs_next.load(vs + cell);
   };
   // the page id of a block is fetched two blocks ahead
-  int page_next = b + ATTN_WARPS < b_hi ? pages[((b + ATTN_WARPS) * KB) >> 7] : 0;
+  int page_next = b + step < b_hi ? pages[((b + step) * KB) >> 7] : 0;
   if (b < b_hi) issue(b, pages[(b * KB) >> 7], 0);
   asm volatile("cp.async.commit_group;" ::: "memory");
-  for (int st = 0; b < b_hi; b += ATTN_WARPS, st ^= 1) {
+  for (int st = 0; b < b_hi; b += step, st ^= 1) {
     const int key0 = b * KB;
     RowScales<G, WIDE> ks_cur = ks_next, vs_cur = vs_next;
-    if (b + ATTN_WARPS < b_hi) {
-      issue(b + ATTN_WARPS, page_next, st ^ 1);
-      if (b + 2 * ATTN_WARPS < b_hi) page_next = pages[((b + 2 * ATTN_WARPS) * KB) >> 7];
+    if (b + step < b_hi) {
+      issue(b + step, page_next, st ^ 1);
+      if (b + 2 * step < b_hi) page_next = pages[((b + 2 * step) * KB) >> 7];
     }
     asm volatile("cp.async.commit_group;" ::: "memory");
     asm volatile("cp.async.wait_group 1;" ::: "memory");
@@ -361,6 +382,16 @@ __global__ void __launch_bounds__(ATTN_WARPS * 32, AttnTile<D>::MIN_CTAS) attn_r
     }
   }
   __syncthreads();
+  if (apart) {
+    if (idle) return;
+    for (int i = lane; i < rep * D; i += 32) {
+      const int r = i / D, d = i % D;
+      const float l = s_l[warp][r];
+      attn_store(l > 0.f ? s_o[warp][r][d] / l : 0.f, gate, out,
+                    (static_cast<size_t>(row) * qh + h * rep + r) * D + d);
+    }
+    return;
+  }
   for (int i = tid; i < rep * D; i += ATTN_WARPS * 32) {
     const int r = i / D, d = i % D, head = h * rep + r;
     float m = s_m[0][r];
@@ -374,12 +405,8 @@ __global__ void __launch_bounds__(ATTN_WARPS * 32, AttnTile<D>::MIN_CTAS) attn_r
       l = fmaf(s_l[w][r], f, l);
     }
     if (splits == 1) {
-      float v = l > 0.f ? o / l : 0.f;
-      if (gate) {
-        const float gv = __half2float(gate[(static_cast<size_t>(row) * qh + head) * D + d]);
-        v *= __fdiv_rn(1.f, 1.f + expf(-gv));
-      }
-      out[(static_cast<size_t>(row) * qh + head) * D + d] = __float2half_rn(v);
+      attn_store(l > 0.f ? o / l : 0.f, gate, out,
+                 (static_cast<size_t>(row) * qh + head) * D + d);
     } else {
       float* rec = scratch + ((static_cast<size_t>(row) * qh + head) * splits + split) * (D + 2);
       if (d == 0) {
@@ -407,12 +434,7 @@ __global__ void attn_merge_kernel(const float* __restrict__ scratch,
       l += rec[s * (D + 2) + 1] * f;
       o += rec[s * (D + 2) + 2 + d] * f;
     }
-    float v = l > 0.f ? o / l : 0.f;
-    if (gate) {
-      const float g = __half2float(gate[(static_cast<size_t>(row) * qh + head) * D + d]);
-      v *= __fdiv_rn(1.f, 1.f + expf(-g));
-    }
-    out[(static_cast<size_t>(row) * qh + head) * D + d] = __float2half_rn(v);
+    attn_store(l > 0.f ? o / l : 0.f, gate, out, (static_cast<size_t>(row) * qh + head) * D + d);
   }
 }
 
@@ -424,17 +446,24 @@ static int launch_attn(const __half* q, const __half* gate, const int* row_req, 
   dim3 grid(rows, kvh, splits);
   const bool wide = ((reinterpret_cast<uintptr_t>(q) & 15) | (reinterpret_cast<uintptr_t>(ks) & 7) |
                      (reinterpret_cast<uintptr_t>(vs) & 7)) == 0;
-  auto kernel = wide ? attn_rows_kernel<D, true> : attn_rows_kernel<D, false>;
   constexpr int SMEM = AttnTile<D>::SMEM;
+  const long long waves = splits > 1 || kvh < ATTN_WARPS
+                              ? 0 : static_cast<long long>(rows) * kvh / (148 * AttnTile<D>::MIN_CTAS);
+  const int apart_keys = AttnTile<D>::KB * static_cast<int>(waves < 4 ? waves : 4);
+  const bool apart = apart_keys > 0;
+  auto kernel = wide ? (apart ? attn_rows_kernel<D, true, true> : attn_rows_kernel<D, true, false>)
+                     : (apart ? attn_rows_kernel<D, false, true> : attn_rows_kernel<D, false, false>);
   if (runtime_ensure_init() != cudaSuccess) return -2;
-  static const int slot[2] = {runtime_new_slot(), runtime_new_slot()};
-  if (runtime_first_use(slot[wide])) {
+  static const int slot[4] = {runtime_new_slot(), runtime_new_slot(), runtime_new_slot(),
+                              runtime_new_slot()};
+  if (runtime_first_use(slot[2 * apart + wide])) {
     const cudaError_t e =
         cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM);
     if (e != cudaSuccess) return static_cast<int>(e);
   }
   kernel<<<grid, ATTN_WARPS * 32, SMEM, stream>>>(q, gate, row_req, row_pos, page_table, max_pages, kc,
-                                               vc, ks, vs, out, qh, kvh, splits, scratch, rep);
+                                               vc, ks, vs, out, qh, kvh, splits, scratch, rep,
+                                               apart_keys);
   if (splits > 1)
     attn_merge_kernel<D><<<dim3(rows, qh), D < 128 ? 64 : 128, 0, stream>>>(scratch, gate, out, qh,
                                                                            splits);

@@ -76,6 +76,72 @@ def test_attention_rows_at_block_edges(dev, qh, kvh, d, splits, wide):
         assert bool(((out[i].double() - ref).abs() <= lim).all()), (n, float((out[i] - ref).abs().max()))
 
 
+def _short_rows(dev, rows, qh, kvh, d, lens):
+    """One request per length, each attended by rows / len(lens) equal query rows."""
+    g = torch.Generator().manual_seed(rows + d)
+    n = len(lens)
+    table = torch.arange(1, 2 * n + 1, dtype=torch.int32).view(n, 2).to(dev)
+    shape = (2 * n + 1, 128, kvh)
+    kc = torch.randint(-127, 128, (*shape, d), generator=g, dtype=torch.int8).to(dev)
+    vc = torch.randint(-127, 128, (*shape, d), generator=g, dtype=torch.int8).to(dev)
+    ks = (torch.rand(*shape, d // 64, generator=g) * 0.02 + 1e-3).half().to(dev)
+    vs = (torch.rand(*shape, d // 64, generator=g) * 0.02 + 1e-3).half().to(dev)
+    q = torch.randn(n, qh, d, generator=g).half().to(dev)
+    req = torch.arange(rows, device=dev, dtype=torch.int32) % n
+    pos = torch.tensor(lens, dtype=torch.int32, device=dev)[req.long()] - 1
+    return q, req, pos, table, kc, vc, ks, vs
+
+
+# launches of less than one to more than four waves of CTAs, lengths around the limits of each;
+# the last warps of a CTA have no head where the KV heads are no multiple of four
+@pytest.mark.parametrize("qh,kvh,d", [(8, 8, 64), (7, 7, 64), (5, 5, 128), (40, 8, 128), (8, 4, 256)])
+@pytest.mark.parametrize("waves", [0.9, 1.1, 2.1, 3.5, 4.2])
+@pytest.mark.parametrize("wide", [True, False])
+def test_attention_rows_of_short_contexts(dev, qh, kvh, d, waves, wide):
+    from orinfer_b200.ops import functional as F
+    lens = [1, 2, 15, 16, 17, 31, 32, 33, 48, 49, 63, 64, 65, 96, 97, 127, 128, 129, 160, 256]
+    rows = int(waves * 148 * {64: 4, 128: 3, 256: 2}[d] / kvh)
+    q, req, pos, table, kc, vc, ks, vs = _short_rows(dev, rows, qh, kvh, d, lens)
+    gate = torch.randn_like(q.float()).half() if d == 256 else None
+    for i, n in enumerate(lens):                    # slots never written hold anything
+        if n % 128:
+            page = table[i, (n - 1) // 128].long()
+            ks[page, (n - 1) % 128 + 1:] = float("nan")
+            vs[page, (n - 1) % 128 + 1:] = float("inf")
+    if not wide:
+        ks, vs = _unaligned(ks), _unaligned(vs)
+    out = F.attention(q[req.long()].contiguous(), None if gate is None else gate[req.long()], req,
+                      pos, table, kc, vc, ks, vs, splits=1).view(rows, qh * d)
+    for i, n in enumerate(lens[:rows]):
+        pick = lambda c: c[table[i].long()].reshape(-1, *c.shape[2:])[:n]
+        ref = _attention64(q[i], pick(kc), pick(vc), pick(ks), pick(vs),
+                           None if gate is None else gate[i]).reshape(-1)
+        # as above: one FP16 rounding and FP32 sums over terms that may cancel
+        lim = ref.abs() * 2.0 ** -11 + 2.0 ** -18 * ref.abs().max() + 2.0 ** -25
+        got = out[i::len(lens)].double()
+        assert bool(((got - ref).abs() <= lim).all()), n
+
+
+def test_attention_rows_fill_the_chip_with_short_contexts(dev):
+    """A warp without a block costs as much as one with: contexts of one block are clearly quicker
+    than contexts of four."""
+    from orinfer_b200.ops import functional as F
+    us = []
+    for n in (30, 110):
+        q, req, pos, table, kc, vc, ks, vs = _short_rows(dev, 512, 16, 16, 128, [n] * 512)
+        times = []
+        for _ in range(15):
+            b, e = torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True)
+            b.record()
+            for _ in range(10):
+                F.attention(q, None, req, pos, table, kc, vc, ks, vs, splits=1)
+            e.record()
+            e.synchronize()
+            times.append(b.elapsed_time(e) * 100)
+        us.append(sorted(times)[7])
+    assert us[0] < 0.75 * us[1], us                 # about 0.6; 0.83 with a CTA to each head
+
+
 @pytest.mark.parametrize("qh,kvh,d,gated", [(2, 2, 64, False), (8, 1, 64, False), (3, 3, 128, False),
                                             (8, 2, 128, True), (10, 2, 128, False),
                                             (16, 1, 128, False), (8, 1, 256, True),
