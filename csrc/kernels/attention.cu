@@ -456,11 +456,7 @@ static int launch_attn(const __half* q, const __half* gate, const int* row_req, 
   if (runtime_ensure_init() != cudaSuccess) return -2;
   static const int slot[4] = {runtime_new_slot(), runtime_new_slot(), runtime_new_slot(),
                               runtime_new_slot()};
-  if (runtime_first_use(slot[2 * apart + wide])) {
-    const cudaError_t e =
-        cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM);
-    if (e != cudaSuccess) return static_cast<int>(e);
-  }
+  if (const int e = runtime_allow_smem(slot[2 * apart + wide], kernel, SMEM)) return e;
   kernel<<<grid, ATTN_WARPS * 32, SMEM, stream>>>(q, gate, row_req, row_pos, page_table, max_pages, kc,
                                                vc, ks, vs, out, qh, kvh, splits, scratch, rep,
                                                apart_keys);

@@ -475,11 +475,7 @@ int launch(const __half* q, const __half* gate, const Chunk* chunks, int n_chunk
           CU_TENSOR_MAP_L2_PROMOTION_L2_128B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) != CUDA_SUCCESS)
     return -3;
   static const int slot = runtime_new_slot();
-  if (runtime_first_use(slot)) {
-    cudaError_t e = cudaFuncSetAttribute(attn_prefill_kernel<D, NQ>,
-                                         cudaFuncAttributeMaxDynamicSharedMemorySize, L::TOTAL);
-    if (e != cudaSuccess) return static_cast<int>(e);
-  }
+  if (const int e = runtime_allow_smem(slot, attn_prefill_kernel<D, NQ>, L::TOTAL)) return e;
   dim3 grid((max_q_len + NQ * P - 1) / (NQ * P), kvh, n_chunks);
   attn_prefill_kernel<D, NQ><<<grid, L::THREADS, L::TOTAL, stream>>>(
       tq, chunks, page_table, max_pages, kc, vc, ks, vs, gate, out, qh, kvh, rep, num_pages,

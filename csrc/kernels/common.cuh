@@ -441,9 +441,14 @@ constexpr int GEMV_WS_TICKETS = 1024;
 int* runtime_gemv_workspace();
 const E8pTables* runtime_e8p_tables();
 cudaError_t runtime_ensure_init();
-// True the first time it is called for (current device, slot); kernels use it to set their
-// dynamic shared-memory attribute once per device.
-bool runtime_first_use(int slot);
+// Lets `kernel` have `bytes` of dynamic shared memory on the current device: set once per (device,
+// slot), a slot belonging to one kernel.  No thread is past it before it is set, and a failure is
+// returned (non-zero) and tried again by the next call.
+int runtime_allow_smem(int slot, const void* kernel, size_t bytes);
+template <class Kernel>
+int runtime_allow_smem(int slot, Kernel* kernel, size_t bytes) {
+  return runtime_allow_smem(slot, reinterpret_cast<const void*>(kernel), bytes);
+}
 int runtime_new_slot();
 
 // ---------------------------------------------------------------- math

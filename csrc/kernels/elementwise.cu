@@ -684,14 +684,10 @@ static int act_prep_launch(const __half* x, float* resid, const __half* norm_w, 
   if (K % 128) return -1;
   if (norm_w != nullptr && K / 128 > MAX_NORM_BLOCKS) return -1;
   const size_t smem = static_cast<size_t>(K) * sizeof(float);
-  static const int slot = runtime_new_slot();
-  if (runtime_first_use(slot)) {
-    cudaFuncSetAttribute(act_prep_kernel<true, 1>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                         200 * 1024);
-    cudaFuncSetAttribute(act_prep_kernel<false, 1>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                         200 * 1024);
-  }
   if (smem > 200 * 1024) return -1;
+  static const int slot[2] = {runtime_new_slot(), runtime_new_slot()};
+  if (const int e = runtime_allow_smem(slot[0], act_prep_kernel<false, 1>, 200 * 1024)) return e;
+  if (const int e = runtime_allow_smem(slot[1], act_prep_kernel<true, 1>, 200 * 1024)) return e;
   // One row keeps a single SM busy, so a cluster of CTAs shares each of a few rows (decode
   // steps): the inbox forms, and rows too wide for one block per warp.  SwiGLU 1 x 8192 3.4 us
   // against 4.2 in one CTA, 1 x 16384 4.2 against 7.2, plain 1 x 16384 4.1 against 5.6; at 4096

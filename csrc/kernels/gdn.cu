@@ -1202,11 +1202,7 @@ int orinfer_gdn_scan(const __half* qkv, const float* ab, const float* a_log, con
       max_seg_rows >= (n_segs == 1 ? GDN_LONG_ROWS : 64)) {
     long_rows = GDN_LONG_ROWS;
     static const int slot = runtime_new_slot();
-    if (runtime_first_use(slot)) {
-      const cudaError_t e = cudaFuncSetAttribute(
-          gdn_chunk_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, sizeof(ChunkSmem));
-      if (e != cudaSuccess) return static_cast<int>(e);
-    }
+    if (const int e = runtime_allow_smem(slot, gdn_chunk_kernel, sizeof(ChunkSmem))) return e;
     gdn_chunk_kernel<<<dim3(hv * 2, n_segs), CHUNK_THREADS, sizeof(ChunkSmem), stream>>>(
         qkv, conv_dim, ab, a_log, dt_bias, sg, row_slot, row_pos, hk, hv, state, out);
   }

@@ -1437,11 +1437,7 @@ int launch_pair(const int8_t* a, const float* a_scale, const void* w, const __ha
     if (reinterpret_cast<uintptr_t>(w) % 16) return -1;
   }
   static const int slot = runtime_new_slot();
-  if (runtime_first_use(slot)) {
-    cudaError_t e = cudaFuncSetAttribute(qgemm_pair_kernel<FMT, OUT_F32>,
-                                         cudaFuncAttributeMaxDynamicSharedMemorySize, L::TOTAL);
-    if (e != cudaSuccess) return static_cast<int>(e);
-  }
+  if (const int e = runtime_allow_smem(slot, qgemm_pair_kernel<FMT, OUT_F32>, L::TOTAL)) return e;
   const long tiles = static_cast<long>((N + L::BN - 1) / L::BN) * ((M + 511) / 512);
   const int pairs = static_cast<int>(tiles < NUM_SMS / 2 ? tiles : NUM_SMS / 2);
   cudaLaunchConfig_t cfg = {};
@@ -1529,11 +1525,7 @@ int launch_ps(const int8_t* a, const float* a_scale, const void* w, const __half
     if (reinterpret_cast<uintptr_t>(w) % 16) return -1;
   }
   static const int slot = runtime_new_slot();
-  if (runtime_first_use(slot)) {
-    cudaError_t e = cudaFuncSetAttribute(qgemm_ps_kernel<FMT, OUT_F32, MT, NB>,
-                                         cudaFuncAttributeMaxDynamicSharedMemorySize, 226 * 1024);
-    if (e != cudaSuccess) return static_cast<int>(e);
-  }
+  if (const int e = runtime_allow_smem(slot, qgemm_ps_kernel<FMT, OUT_F32, MT, NB>, 226 * 1024)) return e;
   const int width = n_end - n_begin;
   if (width <= 0) return 0;
   const long n_tiles = (width + NB - 1) / NB;
@@ -1577,11 +1569,7 @@ int launch(const int8_t* a, const float* a_scale, const void* w, const __half* w
     if (reinterpret_cast<uintptr_t>(w) % 16) return -1;
   }
   static const int slot = runtime_new_slot();
-  if (runtime_first_use(slot)) {
-    cudaError_t e = cudaFuncSetAttribute(qgemm_tc_kernel<FMT, OUT_F32, MT, NB>,
-                                         cudaFuncAttributeMaxDynamicSharedMemorySize, L::TOTAL);
-    if (e != cudaSuccess) return static_cast<int>(e);
-  }
+  if (const int e = runtime_allow_smem(slot, qgemm_tc_kernel<FMT, OUT_F32, MT, NB>, L::TOTAL)) return e;
   const int width = n_end - n_begin;
   if (width <= 0) return 0;
   dim3 grid((width + NB - 1) / NB, grp.tiles ? max_tiles : (M + BM * MT - 1) / (BM * MT), splits);

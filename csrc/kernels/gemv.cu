@@ -962,12 +962,9 @@ static int launch_grouped(const int8_t* a, const float* as, const void* w, const
                       (static_cast<size_t>(GEMV_THREADS) * 10 + listed) * sizeof(int);
   if (smem > GEMV_SMEM_LIMIT) return -1;
   static const int slot = runtime_new_slot();
-  if (runtime_first_use(slot)) {
-    cudaError_t e = cudaFuncSetAttribute(qgemv_grouped_kernel<FMT, MIXED>,
-                                         cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                         static_cast<int>(MIXED ? GEMV_SMEM_LIMIT : smem));
-    if (e != cudaSuccess) return static_cast<int>(e);
-  }
+  if (const int e = runtime_allow_smem(slot, qgemv_grouped_kernel<FMT, MIXED>,
+                                       MIXED ? GEMV_SMEM_LIMIT : smem))
+    return e;
   qgemv_grouped_kernel<FMT, MIXED><<<GROUPED_CTAS, GEMV_THREADS, smem, stream>>>(
       a, as, reinterpret_cast<const unsigned char*>(w), ws, reinterpret_cast<__half*>(out), N, K,
       bank, runtime_e8p_tables(), tiles, meta, most_rows, listed);
@@ -1060,11 +1057,7 @@ static int launch_gemv(const int8_t* a, const float* as, const void* w, const __
   if (smem > GEMV_SMEM_LIMIT) return -1;
   static const int slot[2] = {runtime_new_slot(), runtime_new_slot()};
   auto start = [&](auto kernel, int threads, auto* weights, int sl) -> int {
-    if (runtime_first_use(sl)) {
-      const cudaError_t e = cudaFuncSetAttribute(
-          kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, GEMV_SMEM_LIMIT);
-      if (e != cudaSuccess) return static_cast<int>(e);
-    }
+    if (const int e = runtime_allow_smem(sl, kernel, GEMV_SMEM_LIMIT)) return e;
     kernel<<<g.n_parts * g.k_parts, threads, smem, stream>>>(
         a, as, weights, ws, out, M, N, K, out_f32, runtime_e8p_tables(), po, g.n_parts, g.k_parts,
         g.max_groups, runtime_gemv_workspace(), fz);
@@ -1084,9 +1077,7 @@ static int launch_w8(const int8_t* a, const float* as, const void* w, const __ha
   const size_t smem = static_cast<size_t>(MT) * K;
   if (smem > 200 * 1024) return -1;
   static const int slot = runtime_new_slot();
-  if (runtime_first_use(slot))
-    cudaFuncSetAttribute(w8_gemv_kernel<MT>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                         200 * 1024);
+  if (const int e = runtime_allow_smem(slot, w8_gemv_kernel<MT>, 200 * 1024)) return e;
   w8_gemv_kernel<MT><<<(N + W8_WARPS - 1) / W8_WARPS, W8_WARPS * 32, smem, stream>>>(
       a, as, reinterpret_cast<const int8_t*>(w), ws, out, M, N, K, out_f32, po);
   return static_cast<int>(cudaGetLastError());

@@ -190,12 +190,9 @@ static int launch_router(const __half* x, const __half* w, int rows, int hidden,
   constexpr int PART = WARPS * 16 * (MAXT * 8 + 1);
   const size_t smem = (PART + 2 * static_cast<size_t>(total)) * sizeof(float);
   static const int slot = runtime_new_slot();
-  if (runtime_first_use(slot)) {
-    const cudaError_t e = cudaFuncSetAttribute(router_mma_kernel<MAXT, WARPS>,
-                                               cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                               (PART + 2 * 8 * ROUTER_CL * MAXT) * sizeof(float));
-    if (e != cudaSuccess) return static_cast<int>(e);
-  }
+  if (const int e = runtime_allow_smem(slot, router_mma_kernel<MAXT, WARPS>,
+                                       (PART + 2 * 8 * ROUTER_CL * MAXT) * sizeof(float)))
+    return e;
   const int grid = (rows + 15) / 16 * ROUTER_CL;
   router_mma_kernel<MAXT, WARPS><<<grid, WARPS * 32, smem, stream>>>(
       x, w, rows, hidden, experts, has_shared, top_k, renorm, ids, probs, shared_gate);

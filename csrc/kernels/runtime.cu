@@ -10,6 +10,7 @@
 #include "api.h"
 #include "common.cuh"
 #include "e8p_basis.h"
+#include "once.h"
 #include "tma.h"
 
 namespace orinfer {
@@ -25,11 +26,11 @@ struct DeviceState {
   int* splitk = nullptr;
   int* splitk_tickets = nullptr;  // int32 [SPLITK_TICKETS], zero between launches
   int* gemv_ws = nullptr;
-  bool used[MAX_SLOTS] = {};
 };
 
 std::mutex g_mutex;
 DeviceState g_dev[MAX_DEVICES];
+OncePerSlot<MAX_DEVICES, MAX_SLOTS> g_smem;
 PFN_encodeTiled g_encode = nullptr;
 std::atomic<int> g_slots{0};
 
@@ -137,13 +138,11 @@ int runtime_new_slot() {
   return s < MAX_SLOTS ? s : -1;
 }
 
-bool runtime_first_use(int slot) {
-  const int dev = current_device();
-  if (dev < 0 || slot < 0 || slot >= MAX_SLOTS) return true;
-  std::lock_guard<std::mutex> lock(g_mutex);
-  if (g_dev[dev].used[slot]) return false;
-  g_dev[dev].used[slot] = true;
-  return true;
+int runtime_allow_smem(int slot, const void* kernel, size_t bytes) {
+  return g_smem.run(current_device(), slot, [&] {
+    return static_cast<int>(cudaFuncSetAttribute(
+        kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(bytes)));
+  });
 }
 
 }  // namespace orinfer
