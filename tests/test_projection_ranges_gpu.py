@@ -49,17 +49,25 @@ def test_small_row_projections_are_exact(dev, fmt, m, n, k):
         assert torch.equal(out.cpu(), want if f32 else want.half())
 
 
-@pytest.mark.parametrize("m,n", [(600, 19456), (1024, 19456), (2048, 2432), (1500, 6400)])
-def test_peeled_tail_tiles_are_exact(dev, m, n):
+@pytest.mark.parametrize("fmt", ["w8", "q4", "q2"])
+@pytest.mark.parametrize("m,n", [(260, 19456), (600, 19456), (1024, 19456), (1500, 6400),
+                                 (2047, 9728), (2048, 19456)])
+def test_peeled_tail_tiles_are_exact(dev, fmt, m, n):
     """Grids a few CTAs past a whole number of waves, M tiles cut by the last row."""
+    import ctypes
     from orinfer_b200.ops import functional as F
+    from orinfer_b200.ops import native
+    plan = (ctypes.c_int * 4)()
+    native.lib().orinfer_qgemm_plan(F.FMT[fmt], m, n, 1024, 0, plan)
+    assert plan[3] > 0                                # these shapes do peel tiles
     g = torch.Generator().manual_seed(m)
-    codes, ws, w = _int_weight("q4", n, 1024, g)
+    codes, ws, w = _int_weight(fmt, n, 1024, g)
     a = torch.randint(-127, 128, (m, 1024), generator=g, dtype=torch.int8)
     sa = torch.rand(m, generator=g) * 0.05 + 1e-3
-    out = F.qgemm(a.to(dev), sa.to(dev), codes.to(dev), ws.to(dev), "q4", n)
-    want = _scaled(a.to(dev), sa.to(dev), w.to(dev), ws.to(dev)).half()
-    assert torch.equal(out, want)
+    want = _scaled(a.to(dev), sa.to(dev), w.to(dev), ws.to(dev))
+    for f32 in (False, True):
+        out = F.qgemm(a.to(dev), sa.to(dev), codes.to(dev), ws.to(dev), fmt, n, out_f32=f32)
+        assert torch.equal(out, want if f32 else want.half())
 
 
 @pytest.mark.parametrize("rows", [1, 7, 149, 300, 2049])
