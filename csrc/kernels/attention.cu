@@ -241,7 +241,8 @@ __global__ void __launch_bounds__(
 #pragma unroll
       for (int j = 0; j < 2; ++j)                     // volatile: not hoisted into registers
         asm volatile("ld.shared.v4.u32 {%0, %1, %2, %3}, [%4];"
-                     : "=r"(qf[4 * j]), "=r"(qf[4 * j + 1]), "=r"(qf[4 * j + 2]), "=r"(qf[4 * j + 3])
+                     : "=r"(qf[4 * j]), "=r"(qf[4 * j + 1]), "=r"(qf[4 * j + 2]),
+                       "=r"(qf[4 * j + 3])
                      : "r"(q_addr + (c * 2 + j) * 512));
 #pragma unroll
       for (int i = 0; i < NT; ++i) {
@@ -297,7 +298,8 @@ __global__ void __launch_bounds__(
     const float corr = m_run == -INFINITY ? 0.f : exp2f(m_run - m_new);
     const bool same = m_new == m_run && e_new == e_run;
     if (!__all_sync(0xffffffffu, same)) {
-      const float f = corr * __uint_as_float(static_cast<uint32_t>(127 + max(e_run - e_new, -126)) << 23);
+      const float f =
+          corr * __uint_as_float(static_cast<uint32_t>(127 + max(e_run - e_new, -126)) << 23);
 #pragma unroll
       for (int i = 0; i < G * 8; ++i)
 #pragma unroll
@@ -342,8 +344,10 @@ __global__ void __launch_bounds__(
 #pragma unroll
           for (int e = 0; e < 4; ++e) x[e] = (wd == 0 ? vraw[e].x : vraw[e].y) ^ 0x80808080u;
           // bytes of two keys interleaved: (k0 b0, k1 b0, k0 b1, k1 b1), then b2 and b3
-          const uint32_t p01 = __byte_perm(x[0], x[1], 0x5140), p23 = __byte_perm(x[0], x[1], 0x7362);
-          const uint32_t r01 = __byte_perm(x[2], x[3], 0x5140), r23 = __byte_perm(x[2], x[3], 0x7362);
+          const uint32_t p01 = __byte_perm(x[0], x[1], 0x5140);
+          const uint32_t p23 = __byte_perm(x[0], x[1], 0x7362);
+          const uint32_t r01 = __byte_perm(x[2], x[3], 0x5140);
+          const uint32_t r23 = __byte_perm(x[2], x[3], 0x7362);
           float(*o)[4] = &acc[c * 8 + wd * 4];
           mma16816(o[0], a0, a1, a2, a3, int8x2_half2(p01, 0x4140), int8x2_half2(r01, 0x4140));
           mma16816(o[1], a0, a1, a2, a3, int8x2_half2(p01, 0x4342), int8x2_half2(r01, 0x4342));
@@ -447,19 +451,20 @@ static int launch_attn(const __half* q, const __half* gate, const int* row_req, 
   const bool wide = ((reinterpret_cast<uintptr_t>(q) & 15) | (reinterpret_cast<uintptr_t>(ks) & 7) |
                      (reinterpret_cast<uintptr_t>(vs) & 7)) == 0;
   constexpr int SMEM = AttnTile<D>::SMEM;
-  const long long waves = splits > 1 || kvh < ATTN_WARPS
-                              ? 0 : static_cast<long long>(rows) * kvh / (148 * AttnTile<D>::MIN_CTAS);
+  const long long ctas = splits > 1 || kvh < ATTN_WARPS ? 0 : static_cast<long long>(rows) * kvh;
+  const long long waves = ctas / (148 * AttnTile<D>::MIN_CTAS);
   const int apart_keys = AttnTile<D>::KB * static_cast<int>(waves < 4 ? waves : 4);
   const bool apart = apart_keys > 0;
-  auto kernel = wide ? (apart ? attn_rows_kernel<D, true, true> : attn_rows_kernel<D, true, false>)
-                     : (apart ? attn_rows_kernel<D, false, true> : attn_rows_kernel<D, false, false>);
+  auto kernel =
+      wide ? (apart ? attn_rows_kernel<D, true, true> : attn_rows_kernel<D, true, false>)
+           : (apart ? attn_rows_kernel<D, false, true> : attn_rows_kernel<D, false, false>);
   if (runtime_ensure_init() != cudaSuccess) return -2;
   static const int slot[4] = {runtime_new_slot(), runtime_new_slot(), runtime_new_slot(),
                               runtime_new_slot()};
   if (const int e = runtime_allow_smem(slot[2 * apart + wide], kernel, SMEM)) return e;
-  kernel<<<grid, ATTN_WARPS * 32, SMEM, stream>>>(q, gate, row_req, row_pos, page_table, max_pages, kc,
-                                               vc, ks, vs, out, qh, kvh, splits, scratch, rep,
-                                               apart_keys);
+  kernel<<<grid, ATTN_WARPS * 32, SMEM, stream>>>(q, gate, row_req, row_pos, page_table, max_pages,
+                                                  kc, vc, ks, vs, out, qh, kvh, splits, scratch,
+                                                  rep, apart_keys);
   if (splits > 1)
     attn_merge_kernel<D><<<dim3(rows, qh), D < 128 ? 64 : 128, 0, stream>>>(scratch, gate, out, qh,
                                                                            splits);

@@ -237,7 +237,8 @@ __global__ void __launch_bounds__(512) act_prep_kernel(
     for (int i = k_lo + tid * 16; i < k_hi; i += blockDim.x * 16) {
       __align__(16) signed char c[16];
 #pragma unroll
-      for (int j = 0; j < 16; ++j) c[j] = static_cast<signed char>(a8_code_of<CL>(rowbuf[i + j], scale));
+      for (int j = 0; j < 16; ++j)
+        c[j] = static_cast<signed char>(a8_code_of<CL>(rowbuf[i + j], scale));
       for (int d = 0; d < ag.tp; ++d)
         *reinterpret_cast<int4*>(ag.q[d] + static_cast<size_t>(row) * K + i) =
             *reinterpret_cast<const int4*>(c);

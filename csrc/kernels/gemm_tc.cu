@@ -108,7 +108,8 @@ __global__ void __launch_bounds__(THREADS, 1) qgemm_tc_kernel(
   // probe (timing experiments only; results are then meaningless): bit 0 = issue no MMAs,
   // bit 1 = copy no operands (the loaders only signal), bit 2 = decode nothing, bit 3 = the
   // epilogue stores nothing to global memory, bit 4 = no epilogue at all, bit 5 = no k-blocks,
-  // bit 6 = leave at once, bit 7 = no TMEM allocation (with bits 0 and 4), bit 8 = no table copy, bit 9 = accumulators are reinterpreted, not converted
+  // bit 6 = leave at once, bit 7 = no TMEM allocation (with bits 0 and 4), bit 8 = no table copy,
+  // bit 9 = accumulators are reinterpreted, not converted
   using L = Layout<FMT, MT, NB>;
   constexpr int SA = L::SA, SB = L::SB;
   constexpr int BN = NB;
@@ -1525,7 +1526,8 @@ int launch_ps(const int8_t* a, const float* a_scale, const void* w, const __half
     if (reinterpret_cast<uintptr_t>(w) % 16) return -1;
   }
   static const int slot = runtime_new_slot();
-  if (const int e = runtime_allow_smem(slot, qgemm_ps_kernel<FMT, OUT_F32, MT, NB>, 226 * 1024)) return e;
+  if (const int e = runtime_allow_smem(slot, qgemm_ps_kernel<FMT, OUT_F32, MT, NB>, 226 * 1024))
+    return e;
   const int width = n_end - n_begin;
   if (width <= 0) return 0;
   const long n_tiles = (width + NB - 1) / NB;
@@ -1569,7 +1571,8 @@ int launch(const int8_t* a, const float* a_scale, const void* w, const __half* w
     if (reinterpret_cast<uintptr_t>(w) % 16) return -1;
   }
   static const int slot = runtime_new_slot();
-  if (const int e = runtime_allow_smem(slot, qgemm_tc_kernel<FMT, OUT_F32, MT, NB>, L::TOTAL)) return e;
+  if (const int e = runtime_allow_smem(slot, qgemm_tc_kernel<FMT, OUT_F32, MT, NB>, L::TOTAL))
+    return e;
   const int width = n_end - n_begin;
   if (width <= 0) return 0;
   dim3 grid((width + NB - 1) / NB, grp.tiles ? max_tiles : (M + BM * MT - 1) / (BM * MT), splits);
@@ -1612,7 +1615,8 @@ inline int plan_splits(int M, int N, int K, int out_f32) {
     splits = static_cast<int>(148 / c128);
     splits = splits > K / BK / 8 ? K / BK / 8 : splits;          // at least 8 k-blocks each
     splits = splits > 8 ? 8 : splits;
-    while (splits > 1 && static_cast<size_t>(splits) * padded_cells(M, N) * 4 > SPLITK_WORKSPACE_BYTES)
+    while (splits > 1 &&
+           static_cast<size_t>(splits) * padded_cells(M, N) * 4 > SPLITK_WORKSPACE_BYTES)
       --splits;
   }
   return splits < 1 ? 1 : splits;
@@ -1699,7 +1703,8 @@ inline Plan make_plan(int fmt, int M, int N, int K, int out_f32, bool fused) {
     const int per = M <= BM ? 2 : 8;                    // k-blocks a split must keep
     splits = splits > K / BK / per ? K / BK / per : splits;
     splits = splits > 8 ? 8 : splits;
-    while (splits > 1 && static_cast<size_t>(splits) * padded_cells(M, N) * 4 > SPLITK_WORKSPACE_BYTES)
+    while (splits > 1 &&
+           static_cast<size_t>(splits) * padded_cells(M, N) * 4 > SPLITK_WORKSPACE_BYTES)
       --splits;
     p.splits = splits < 1 ? 1 : splits;
   }
@@ -1727,7 +1732,8 @@ int launch_fmt(const int8_t* a, const float* a_scale, const void* w, const __hal
                const PeerOut& po, const AgIn& ag = AgIn{nullptr, nullptr, 0, 0}) {
   const GroupDesc none{nullptr, nullptr, 0, 0};
   if (g_impl == 2 && M > BM && N >= 256) {
-    if (out_f32) return launch_pair<FMT, true>(a, a_scale, w, w_scale, out, M, N, K, stream, po, ag);
+    if (out_f32)
+      return launch_pair<FMT, true>(a, a_scale, w, w_scale, out, M, N, K, stream, po, ag);
     return launch_pair<FMT, false>(a, a_scale, w, w_scale, out, M, N, K, stream, po, ag);
   }
   const Plan plan = make_plan(FMT, M, N, K, out_f32, po.tp != 0);
@@ -1788,7 +1794,7 @@ static int qgemm_any(int fmt, const int8_t* a, const float* a_scale, const void*
   if (runtime_ensure_init() != cudaSuccess) return -2;
   const bool simt = force_path == 1 || (force_path == 0 && M <= 8);
   if (simt) {
-    // The SIMT kernel takes at most 8 rows per launch (one launch when fused with peers,
+    // The small-M kernels take at most 8 rows per launch (one launch when fused with peers,
     // because every launch bumps the peers' sequence flags).
     if (peer != nullptr && M > 8) return -1;
     for (int m = 0; m < M; m += 8) {
@@ -1822,7 +1828,8 @@ extern "C" int orinfer_qgemm_launches_fmt(int fmt, int M, int N, int K, int out_
     const bool second = ts > 1 && !(tc::g_impl == 1 && tc::splitk_in_kernel(1, 128, ts));
     return second ? 3 : 2;
   }
-  const bool second = p.splits > 1 && !(tc::g_impl == 1 && tc::splitk_in_kernel(p.mt, 128, p.splits));
+  const bool second =
+      p.splits > 1 && !(tc::g_impl == 1 && tc::splitk_in_kernel(p.mt, 128, p.splits));
   return second ? 2 : 1;
 }
 
@@ -1980,15 +1987,16 @@ static int qgemm_grouped_fmt(const int8_t* a, const float* a_scale, const void* 
   // nearly a whole one: nothing to decode, so a second tile only saves the copy of the weights),
   // four where they have several.
   const long long two = (FMT == 0 ? 112LL : 64LL) * experts;
-  const int mt = tc::g_impl != 1 ? 1 : (expected >= 256LL * experts ? 4 : (expected >= two ? 2 : 1));
+  const long long four = 256LL * experts;
+  const int mt = tc::g_impl != 1 ? 1 : (expected >= four ? 4 : (expected >= two ? 2 : 1));
   if (mt == 4)
     return tc::launch<FMT, false, 4, 128>(a, a_scale, w, w_scale, out, S, N, K, stream, po, g,
                                           experts, max_tiles);
   if (mt == 2)
     return tc::launch<FMT, false, 2, 128>(a, a_scale, w, w_scale, out, S, N, K, stream, po, g,
                                           experts, max_tiles);
-  return tc::launch<FMT, false, 1, 128>(a, a_scale, w, w_scale, out, S, N, K, stream, po, g, experts,
-                                        max_tiles);
+  return tc::launch<FMT, false, 1, 128>(a, a_scale, w, w_scale, out, S, N, K, stream, po, g,
+                                        experts, max_tiles);
 }
 
 extern "C" int orinfer_qgemm_grouped(int fmt, const int8_t* a, const float* a_scale, const void* w,

@@ -401,7 +401,8 @@ __global__ void __launch_bounds__(GEMV_THREADS, 1) qgemv_kernel(
   const int oct = N / 8;
   const int np = blockIdx.x % n_parts, kp = blockIdx.x / n_parts;
   const int n_base = static_cast<int>(static_cast<long long>(oct) * np / n_parts) * 8;
-  const int n_count = static_cast<int>(static_cast<long long>(oct) * (np + 1) / n_parts) * 8 - n_base;
+  const int n_count =
+      static_cast<int>(static_cast<long long>(oct) * (np + 1) / n_parts) * 8 - n_base;
   const int groups = (n_count + ROWS - 1) / ROWS;
   const int kb_lo = kb_all * kp / k_parts, kb_hi = kb_all * (kp + 1) / k_parts;
   const int kbs = kb_hi - kb_lo;
@@ -977,9 +978,10 @@ int qgemv_grouped_dispatch(int fmt, const int8_t* a, const float* as, const void
                            cudaStream_t stream) {
   // INT8 has the one form for both: its loop comes out better with the list (128 experts of 1536 x
   // 2048, 14 skewed rows: 31 us against 36); the E8P forms pay 0.4 us of 6 for it.
+  const bool mixed = most_rows > 0;
   const auto run = fmt == 0   ? launch_grouped<0, true>
-                   : fmt == 1 ? (most_rows > 0 ? launch_grouped<1, true> : launch_grouped<1, false>)
-                              : (most_rows > 0 ? launch_grouped<2, true> : launch_grouped<2, false>);
+                   : fmt == 1 ? (mixed ? launch_grouped<1, true> : launch_grouped<1, false>)
+                              : (mixed ? launch_grouped<2, true> : launch_grouped<2, false>);
   return run(a, as, w, ws, out, N, K, bank, tiles, meta, most_rows, max_tiles, stream);
 }
 
@@ -1126,7 +1128,8 @@ int qgemv_dispatch(int fmt, const int8_t* a, const float* as, const void* w, con
 // Projection of at most 8 rows with the row preparation fused in (see GemvFuse); E8P weights.
 int qgemv_fused_dispatch(int fmt, const void* w, const __half* ws, void* out, int M, int N, int K,
                          cudaStream_t stream, const GemvFuse& fz) {
-  if (M < 1 || M > 8 || K % 128 || N % 8 || fz.pre < 1 || fz.pre > 3 || (fmt != 1 && fmt != 2)) return -1;
+  if (M < 1 || M > 8 || K % 128 || N % 8 || fz.pre < 1 || fz.pre > 3) return -1;
+  if (fmt != 1 && fmt != 2) return -1;
   if (fz.norm_w != nullptr && K / 128 > 128) return -1;
   const PeerOut po{};
 #define BY_M(F)                                                                                   \

@@ -1,5 +1,6 @@
 // Mixture-of-experts routing and data movement: fused router projection + softmax + top-k,
-// deterministic (atomics-free) expert counts / offsets / tile table / slot assignment,
+// deterministic expert counts / offsets / tile table / slot assignment (counts by shared-memory
+// atomics, whose order shows nowhere; slots in row order),
 // dispatch of quantised rows into expert-contiguous slots, and the weighted combine.
 // Replaces router_projection / router_topk (kernels/cuda/model/moe.py:16,413),
 // expert_histogram* / expert_offsets / expert_tiles (moe.py:177-286,558-713),
@@ -284,8 +285,8 @@ __global__ void __launch_bounds__(THREADS) moe_plan_kernel(
 // Copies row blockIdx.x (INT8 values and scale) into the slots of its assignments: the row is
 // read once and written top_k times in whole lines.  SPARSE (one slot a row): most rows may be free
 // entries of a receive buffer, which are not read (131072 entries, 100 in use, 128 -> 105 us of
-// which most is the numbering; all in use 159 -> 174).  With several slots a row, few rows of a rank
-// go nowhere, and looking first costs 0.2 to 0.5 us of 4 to 7.
+// which most is the numbering; all in use 159 -> 174).  With several slots a row, few rows of a
+// rank go nowhere, and looking first costs 0.2 to 0.5 us of 4 to 7.
 template <bool SPARSE>
 __global__ void __launch_bounds__(128) moe_scatter_kernel(
     const int* __restrict__ slots, int top_k, const int8_t* __restrict__ q8,
