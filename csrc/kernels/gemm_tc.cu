@@ -98,7 +98,7 @@ struct GroupDesc {
   int over = 0, listed = 0;
 };
 
-template <int FMT, bool OUT_F32, int MT, int NB>
+template <int FMT, bool OUT_F32, int MT, int NB, bool GROUPED>
 __global__ void __launch_bounds__(THREADS, 1) qgemm_tc_kernel(
     const __grid_constant__ CUtensorMap tmap_a, const __grid_constant__ CUtensorMap tmap_b,
     const unsigned char* __restrict__ w, const float* __restrict__ a_scale,
@@ -261,30 +261,18 @@ __global__ void __launch_bounds__(THREADS, 1) qgemm_tc_kernel(
         if (!ok) break;
         tc_fence_after();
         const uint32_t b_addr = smem_u32(b_s + sb * L::B_BYTES);
-        if (mt_act == MT) {
 #pragma unroll
-          for (int j = 0; j < BK / 32; ++j) {
-            if (probe & 1) break;
-            const uint64_t bdesc = umma_desc(b_addr + j * 32, 16, 1024);
+        for (int j = 0; j < BK / 32; ++j) {
+          if (probe & 1) break;
+          const uint64_t bdesc = umma_desc(b_addr + j * 32, 16, 1024);
 #pragma unroll
-            for (int t = 0; t < MT; ++t) {
-              const uint32_t a_addr = smem_u32(a_s + (sa * MT + t) * TILE_BYTES);
+          for (int t = 0; t < MT; ++t) {
+            const uint32_t a_addr = smem_u32(a_s + (sa * MT + t) * TILE_BYTES);
+            // An expert's last row tiles are often not loaded, and nobody reads them.  The one
+            // cut packet of the other calls is not worth the test (2 % at 1024 x 2560 x 4096).
+            if (!GROUPED || t == 0 || t < mt_act)
               mma_i8_ss(tmem_base + t * BN, umma_desc(a_addr + j * 32, 16, 1024), bdesc, idesc,
                         (kb | j) != 0 ? 1u : 0u);
-            }
-          }
-        } else {
-          // an expert's last row tiles: the others are not loaded, and nobody reads them
-#pragma unroll
-          for (int j = 0; j < BK / 32; ++j) {
-            const uint64_t bdesc = umma_desc(b_addr + j * 32, 16, 1024);
-#pragma unroll
-            for (int t = 0; t < MT - 1; ++t) {
-              const uint32_t a_addr = smem_u32(a_s + (sa * MT + t) * TILE_BYTES);
-              if (t < mt_act)
-                mma_i8_ss(tmem_base + t * BN, umma_desc(a_addr + j * 32, 16, 1024), bdesc, idesc,
-                          (kb | j) != 0 ? 1u : 0u);
-            }
           }
         }
         tc_commit(&a_empty[sa]);
@@ -1570,9 +1558,12 @@ int launch(const int8_t* a, const float* a_scale, const void* w, const __half* w
     tb = ta;
     if (reinterpret_cast<uintptr_t>(w) % 16) return -1;
   }
-  static const int slot = runtime_new_slot();
-  if (const int e = runtime_allow_smem(slot, qgemm_tc_kernel<FMT, OUT_F32, MT, NB>, L::TOTAL))
-    return e;
+  constexpr bool MAY_GROUP = MT > 1 && NB == 128 && !OUT_F32;
+  const bool grouped = MAY_GROUP && grp.tiles != nullptr;
+  const auto kernel = grouped ? qgemm_tc_kernel<FMT, OUT_F32, MT, NB, MAY_GROUP>
+                              : qgemm_tc_kernel<FMT, OUT_F32, MT, NB, false>;
+  static const int slot[2] = {runtime_new_slot(), runtime_new_slot()};
+  if (const int e = runtime_allow_smem(slot[grouped], kernel, L::TOTAL)) return e;
   const int width = n_end - n_begin;
   if (width <= 0) return 0;
   dim3 grid((width + NB - 1) / NB, grp.tiles ? max_tiles : (M + BM * MT - 1) / (BM * MT), splits);
@@ -1584,7 +1575,7 @@ int launch(const int8_t* a, const float* a_scale, const void* w, const __half* w
   if (splits > 1 && (tiles > static_cast<size_t>(SPLITK_TICKETS) ||
                      tiles * splits * MT * BM * NB * 4 > SPLITK_WORKSPACE_BYTES))
     return -1;
-  qgemm_tc_kernel<FMT, OUT_F32, MT, NB><<<grid, THREADS, L::TOTAL, stream>>>(
+  kernel<<<grid, THREADS, L::TOTAL, stream>>>(
       ta, tb, reinterpret_cast<const unsigned char*>(w), a_scale, w_scale, out, M, N, K,
       runtime_e8p_tables(), runtime_status_ptr(), po, grp, ag, partial,
       in_kernel ? runtime_splitk_tickets() : nullptr, n_begin, n_end, g_probe);
