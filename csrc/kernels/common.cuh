@@ -400,6 +400,68 @@ __device__ __forceinline__ uint32_t e8p_fields(uint32_t word, const E8pLut<COPIE
 
 constexpr uint32_t E8P_NIB = 0x0f0f0f0fu;
 
+// The form of the small-M kernels: 32 replicas, and an entry's two words in one 256-byte row, so
+// that an address is a byte permute of the code word and the lane's offset (4 * lane) and nothing
+// else.  It must stand at the start of the dynamic shared memory.
+struct E8pRows {
+  uint32_t w[256][2][32];                               // [entry][e2, sg][lane]
+};
+
+// Filled in two steps, so that other loads can be under way between them: a thread's words, then its
+// 16-byte stores.
+template <int THREADS>
+struct E8pFill {
+  static constexpr int PER = 256 * 16 / THREADS;
+  uint32_t v[PER];
+  __device__ __forceinline__ void load(const E8pTables* __restrict__ g, int tid) {
+#pragma unroll
+    for (int q = 0; q < PER; ++q) {
+      const int j = tid + q * THREADS;
+      v[q] = __ldg((j & 8 ? g->sg : g->e2) + (j >> 4));
+    }
+  }
+  __device__ __forceinline__ void store(unsigned char* rows, int tid) const {
+#pragma unroll
+    for (int q = 0; q < PER; ++q)
+      reinterpret_cast<uint4*>(rows)[tid + q * THREADS] = make_uint4(v[q], v[q], v[q], v[q]);
+  }
+};
+
+// (e2 ^ sg) of the code in the low (HALF = 0) or high (HALF = 1) half of `word`, as its even
+// fields in the low halves of the bytes (lo) and its odd fields still in the high halves (hi).
+template <int HALF>
+__device__ __forceinline__ void e8p_lookup(uint32_t word, const unsigned char* rows, uint32_t lane4,
+                                           uint32_t& lo, uint32_t& hi) {
+  const uint32_t at = __byte_perm(word, lane4, HALF ? 0x5534 : 0x5514);
+  const uint32_t sat = __byte_perm(word, lane4, HALF ? 0x5524 : 0x5504);
+  const uint32_t e = *reinterpret_cast<const uint32_t*>(rows + at);
+  const uint32_t s = *reinterpret_cast<const uint32_t*>(rows + 128 + sat);
+  // one instruction each: (e ^ s) & NIB, (e ^ s) & ~NIB
+  asm("lop3.b32 %0, %1, %2, %3, 0x28;" : "=r"(lo) : "r"(e), "r"(s), "r"(E8P_NIB));
+  asm("lop3.b32 %0, %1, %2, %3, 0x14;" : "=r"(hi) : "r"(e), "r"(s), "r"(E8P_NIB));
+}
+// Eight bytes 4 * v0 + v1 of a Q4 word (weights + 75, halved), or v of a Q2 code, in k order.
+__device__ __forceinline__ uint2 e8p_bytes_q4(uint32_t word, const unsigned char* rows,
+                                              uint32_t lane4) {
+  uint32_t l0, h0, l1, h1;
+  e8p_lookup<0>(word, rows, lane4, l0, h0);
+  e8p_lookup<1>(word, rows, lane4, l1, h1);
+  return make_uint2(l0 * 4u + l1, (h0 >> 2) + (h1 >> 4));
+}
+template <int HALF>
+__device__ __forceinline__ uint2 e8p_bytes_q2(uint32_t word, const unsigned char* rows,
+                                              uint32_t lane4) {
+  uint32_t lo, hi;
+  e8p_lookup<HALF>(word, rows, lane4, lo, hi);
+  return make_uint2(lo, hi >> 4);
+}
+// Sum of the products of four unsigned bytes of w and four signed bytes of a, plus c.
+__device__ __forceinline__ int dp4a_us(uint32_t w, int a, int c) {
+  int d;
+  asm("dp4a.u32.s32 %0, %1, %2, %3;" : "=r"(d) : "r"(w), "r"(a), "r"(c));
+  return d;
+}
+
 // One Q4 word (coarse U16 low, residual U16 high) -> eight INT8 weights 4*c0 + c1.
 template <int COPIES>
 __device__ __forceinline__ uint2 e8p_decode_q4(uint32_t word, const E8pLut<COPIES>* __restrict__ sm,

@@ -43,7 +43,7 @@ __device__ __forceinline__ void store_row(void* out, int out_f32, int m, int n, 
 
 // FMT 0: INT8 weights, 1: Q4 (U32 codes), 2: Q2 (U16 codes).  One persistent CTA per SM: the
 // decode tables (32 interleaved copies, so a lane's lookups never meet another lane's on a
-// bank) and the activations are staged once.  The grid is n_parts x k_parts CTAs; a CTA owns a
+// bank, and an address is one byte permute: see E8pRows) and the activations are staged once.  The grid is n_parts x k_parts CTAs; a CTA owns a
 // contiguous range of 16-row groups and one range of 128-wide k-blocks, its warps take
 // contiguous runs of (group, k-block) units, every lane keeps DEPTH units of weight loads in
 // flight (the first ones are issued before the tables are filled, except in the fused forms), and
@@ -56,6 +56,9 @@ __device__ __forceinline__ void store_row(void* out, int out_f32, int m, int n, 
 // octet-wise as [k-block][j][t][row] and a step reads 8 bytes per lane without a bank conflict.
 // One MMA replaces 4 M dp4a and 2 M shared-memory loads: the time no longer grows with M.
 //
+// 8 x 19456 x 2560 18.0 -> 16.3 us, 8 x 2560 x 4096 9.9 -> 8.9, 4 x 6144 x 2560 9.6 -> 8.6 with the
+// permuted addresses and the small loads ahead of the weights (see GemvEarly).
+//
 // The decode never forms the weights.  With v the 4-bit fields of a code (common.cuh), a Q4
 // weight is 8*v0 + 2*v1 - 75, so
 //     sum_k a_k w_k = 2 * sum_k a_k (4*v0 + v1)_k  -  75 * sum_k a_k
@@ -66,7 +69,6 @@ __device__ __forceinline__ void store_row(void* out, int out_f32, int m, int n, 
 // integers into a zeroed workspace; the last one to finish (ticket) applies the scales,
 // writes the outputs and zeroes what it read.  Launches that use the workspace must not
 // overlap on the device (they are issued on one stream).
-constexpr int GEMV_COPIES = 32;
 constexpr int GEMV_THREADS = 1024;
 constexpr size_t GEMV_SMEM_LIMIT = 220 * 1024;
 
@@ -122,13 +124,53 @@ struct GemvFuse {
   float* resid_accum;
 };
 
+// What a CTA needs before its first product besides weights: the decode tables, the activation rows
+// and the scales.  They are requested ahead of the weights.  Behind them they waited for a CTA's
+// first 64 KB, three times in a row: the first product came 5 us into the 13 us of 1 x 19456 x 2560,
+// 6 us into the 8 us of 8 x 2560 x 4096.
+template <int FMT, int THREADS>
+struct GemvEarly {
+  static constexpr int ROWS = 2;                 // 16-byte pieces of the rows per thread
+  E8pFill<THREADS> fill;
+  int4 rows[ROWS];
+  float scale;
+  __half w_scale;
+  __device__ __forceinline__ void load(const E8pTables* __restrict__ tables,
+                                       const int8_t* __restrict__ a,
+                                       const float* __restrict__ a_scale,
+                                       const __half* __restrict__ ws, int n_count, int M, int K,
+                                       bool plain, int tid) {
+    if (FMT != 0) fill.load(tables, tid);
+    w_scale = tid < n_count ? __ldg(ws + tid) : __half(0.f);
+    scale = 0.f;
+    if (plain) {
+#pragma unroll
+      for (int i = 0; i < ROWS; ++i) {
+        const int c = tid + i * THREADS;
+        rows[i] = c * 16 < M * K ? __ldg(reinterpret_cast<const int4*>(a) + c)
+                                 : make_int4(0, 0, 0, 0);
+      }
+      if (tid < M) scale = __ldg(a_scale + tid);
+    }
+  }
+  // the tables, the outputs' scales (sw) and zeroed sums
+  __device__ __forceinline__ void store(unsigned char* smem, float* sw,
+                                        const __half* __restrict__ ws, int n_count, int* sums,
+                                        int n_sums, int tid) const {
+    if (FMT != 0) fill.store(smem, tid);
+    if (tid < n_count) sw[tid] = __half2float(w_scale);
+    for (int i = tid + THREADS; i < n_count; i += THREADS) sw[i] = __half2float(ws[i]);
+    for (int i = tid; i < n_sums; i += THREADS) sums[i] = 0;
+  }
+};
+
 // Fills the staged activations, their row sums (asum, zeroed before) and their scales: from INT8
 // rows, or by the row preparation of fz.pre, one row at a time in fbuf [K].
 template <int FMT, int MT, int THREADS, bool DP4A>
 __device__ __forceinline__ void gemv_rows(int8_t* act, int* asum, float* scale_s, float* fbuf,
                                           float* red, float* blk_sum, const int8_t* __restrict__ a,
                                           const float* __restrict__ a_scale, int M, int K,
-                                          const GemvFuse& fz) {
+                                          const GemvFuse& fz, const GemvEarly<FMT, THREADS>& early) {
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   if (FMT == 0 || fz.pre == 0) {
     // stage the activations; their row sums ride along
@@ -136,11 +178,8 @@ __device__ __forceinline__ void gemv_rows(int8_t* act, int* asum, float* scale_s
     int part_sum[MT];
 #pragma unroll
     for (int m = 0; m < MT; ++m) part_sum[m] = 0;
-    for (int c = tid; c < chunks; c += THREADS) {
-      const int m = (c * 16) / K;
-      int4 v = make_int4(0, 0, 0, 0);
-      if (m < M) v = *reinterpret_cast<const int4*>(a + static_cast<size_t>(c) * 16);
-      const int k = c * 16 - m * K;
+    auto place = [&](int c, const int4& v) {
+      const int m = (c * 16) / K, k = c * 16 - m * K;
       *reinterpret_cast<int2*>(act + act_pos<FMT, MT, DP4A>(m, k, K)) = make_int2(v.x, v.y);
       *reinterpret_cast<int2*>(act + act_pos<FMT, MT, DP4A>(m, k + 8, K)) = make_int2(v.z, v.w);
       int s = __dp4a(v.x, 0x01010101, 0);
@@ -150,6 +189,14 @@ __device__ __forceinline__ void gemv_rows(int8_t* act, int* asum, float* scale_s
 #pragma unroll
       for (int mm = 0; mm < MT; ++mm)
         if (mm == m) part_sum[mm] += s;
+    };
+#pragma unroll
+    for (int i = 0; i < early.ROWS; ++i)
+      if (tid + i * THREADS < chunks) place(tid + i * THREADS, early.rows[i]);
+    for (int c = tid + early.ROWS * THREADS; c < chunks; c += THREADS) {
+      int4 v = make_int4(0, 0, 0, 0);
+      if (c * 16 < M * K) v = *reinterpret_cast<const int4*>(a + static_cast<size_t>(c) * 16);
+      place(c, v);
     }
 #pragma unroll
     for (int m = 0; m < MT; ++m) {
@@ -158,7 +205,7 @@ __device__ __forceinline__ void gemv_rows(int8_t* act, int* asum, float* scale_s
       for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
       if (lane == 0 && s != 0) atomicAdd(&asum[m], s);
     }
-    if (tid < MT) scale_s[tid] = tid < M ? a_scale[tid] : 0.f;
+    if (tid < MT) scale_s[tid] = early.scale;
   } else {
     // build the activations: the row kernels' work, repeated by every CTA
     constexpr int NWP = THREADS / 32;
@@ -275,7 +322,7 @@ __device__ __forceinline__ void gemv_rows(int8_t* act, int* asum, float* scale_s
 // Scales and writes the outputs n_base .. n_base + n_count from the integers in acc_s.
 template <int FMT, int MT, int THREADS>
 __device__ __forceinline__ void gemv_finish(int* acc_s, const int* asum, const float* scale_s,
-                                            int* last_flag, const __half* __restrict__ w_scale,
+                                            int* last_flag, const float* sw_s,
                                             void* __restrict__ out, int M, int N, int out_f32,
                                             const PeerOut& po, int ll_seq, int np, int k_parts,
                                             int n_base, int n_count, int* __restrict__ ws,
@@ -333,7 +380,7 @@ __device__ __forceinline__ void gemv_finish(int* acc_s, const int* asum, const f
           for (int r = 0; r < 8; ++r) {
             const int total = UNIT * acc_s[(seg * 8 + r) * MT + m] - bias;
             h[r] = __float2half_rn(
-                (static_cast<float>(total) * __half2float(w_scale[n_base + seg * 8 + r])) * sa);
+                (static_cast<float>(total) * sw_s[seg * 8 + r]) * sa);
           }
           if (ll) {
             ll_store8(po, ll_seq, m, n_base + seg * 8, N, h);
@@ -350,7 +397,7 @@ __device__ __forceinline__ void gemv_finish(int* acc_s, const int* asum, const f
         const int m = i / n_count, r = i % n_count;
         if (m < M) {
           const int total = UNIT * acc_s[r * MT + m] - BIAS * asum[m];
-          const float sw = __half2float(w_scale[n_base + r]);
+          const float sw = sw_s[r];
           if (FMT != 0 && fz.resid_accum != nullptr) {
             const __half hv = __float2half_rn((static_cast<float>(total) * sw) * scale_s[m]);
             float* dst = fz.resid_accum + static_cast<size_t>(m) * N + n_base + r;
@@ -377,18 +424,17 @@ __global__ void __launch_bounds__(GEMV_THREADS, 1) qgemv_kernel(
   constexpr int THREADS = GEMV_THREADS;
   constexpr int ROWS = 16, DEPTH = FMT == 2 ? 4 : 2;     // rows of a group, units in flight
   using Unit = GemvUnit<FMT>;
-  using Lut = E8pLut<GEMV_COPIES>;
-  constexpr int LUT_BYTES = FMT == 0 ? 0 : static_cast<int>(sizeof(Lut));
+  constexpr int LUT_BYTES = FMT == 0 ? 0 : static_cast<int>(sizeof(E8pRows));
   const bool ll = po.tp > 0 && po.rows_per == LL_MODE;
   const int ll_seq = ll ? *reinterpret_cast<volatile int*>(po.sent) + 1 : 0;
   extern __shared__ __align__(16) unsigned char smem_raw[];
-  Lut* lut = reinterpret_cast<Lut*>(smem_raw);
   int8_t* act = reinterpret_cast<int8_t*>(smem_raw) + LUT_BYTES;
   int* acc_s = reinterpret_cast<int*>(act + static_cast<size_t>(MT) * K);   // [16 max_groups][MT]
   int* asum = acc_s + max_groups * 16 * MT;                                  // [MT]
   float* scale_s = reinterpret_cast<float*>(asum + MT);                      // [MT]
+  float* sw_s = scale_s + MT;                                                // [16 max_groups]
   float* fbuf = reinterpret_cast<float*>(                                    // [K], pre only
-      (reinterpret_cast<uintptr_t>(scale_s + MT) + 15) & ~static_cast<uintptr_t>(15));
+      (reinterpret_cast<uintptr_t>(sw_s + max_groups * 16) + 15) & ~static_cast<uintptr_t>(15));
   __shared__ int last_flag;
   __shared__ float red[32];
   __shared__ float blk_sum[128];
@@ -449,14 +495,16 @@ __global__ void __launch_bounds__(GEMV_THREADS, 1) qgemv_kernel(
   };
   // The first weights are requested before the tables are filled, except where the row
   // preparation needs the registers.
+  GemvEarly<FMT, THREADS> early;
+  early.load(tables, a, a_scale, w_scale + n_base, n_count, M, K, FMT == 0 || fz.pre == 0, tid);
   if (FMT == 0 || fz.pre == 0) {
 #pragma unroll
     for (int i = 0; i < DEPTH; ++i) fetch(buf[i], u_lo + i);
   }
-  if (FMT != 0) e8p_lut_init(lut, tables, tid, THREADS);
-  for (int i = tid; i < max_groups * 16 * MT + MT; i += THREADS) acc_s[i] = 0;
+  early.store(smem_raw, sw_s, w_scale + n_base, n_count, acc_s, max_groups * 16 * MT + MT, tid);
   __syncthreads();
-  gemv_rows<FMT, MT, THREADS, false>(act, asum, scale_s, fbuf, red, blk_sum, a, a_scale, M, K, fz);
+  gemv_rows<FMT, MT, THREADS, false>(act, asum, scale_s, fbuf, red, blk_sum, a, a_scale, M, K, fz,
+                                     early);
   __syncthreads();
 
   if (FMT != 0 && fz.pre != 0) {
@@ -464,7 +512,7 @@ __global__ void __launch_bounds__(GEMV_THREADS, 1) qgemv_kernel(
     for (int i = 0; i < DEPTH; ++i) fetch(buf[i], u_lo + i);
   }
   int acc[4] = {0, 0, 0, 0};
-  const int copy = lane;                                   // GEMV_COPIES == 32
+  const uint32_t lane4 = lane * 4;
   for (int base = u_lo; base < u_hi; base += DEPTH) {
 #pragma unroll
     for (int i = 0; i < DEPTH; ++i) {
@@ -493,19 +541,12 @@ __global__ void __launch_bounds__(GEMV_THREADS, 1) qgemv_kernel(
 #pragma unroll
             for (int h = 0; h < 2; ++h) {
               if (h == 1 && half) break;
-              if (FMT == 1) {
-                const uint32_t word = buf[i].w[h][j % Unit::WORDS];
-                const uint32_t v0 = e8p_fields<GEMV_COPIES, 0>(word, lut, copy);
-                const uint32_t v1 = e8p_fields<GEMV_COPIES, 1>(word, lut, copy);
-                lo[h] = (v0 & E8P_NIB) * 4u + (v1 & E8P_NIB);
-                hi[h] = ((v0 >> 4) & E8P_NIB) * 4u + ((v1 >> 4) & E8P_NIB);
-              } else {
-                const uint32_t word = buf[i].w[h][(j >> 1) % Unit::WORDS];
-                const uint32_t v = (j & 1) ? e8p_fields<GEMV_COPIES, 1>(word, lut, copy)
-                                           : e8p_fields<GEMV_COPIES, 0>(word, lut, copy);
-                lo[h] = v & E8P_NIB;
-                hi[h] = (v >> 4) & E8P_NIB;
-              }
+              const uint32_t word = buf[i].w[h][(FMT == 1 ? j : j >> 1) % Unit::WORDS];
+              const uint2 v = FMT == 1 ? e8p_bytes_q4(word, smem_raw, lane4)
+                              : j & 1  ? e8p_bytes_q2<1>(word, smem_raw, lane4)
+                                       : e8p_bytes_q2<0>(word, smem_raw, lane4);
+              lo[h] = v.x;
+              hi[h] = v.y;
             }
             mma_i8_16832(acc, lo[0], lo[1], hi[0], hi[1], b.x, b.y);
           }
@@ -532,15 +573,18 @@ __global__ void __launch_bounds__(GEMV_THREADS, 1) qgemv_kernel(
   }
   __syncthreads();
 
-  gemv_finish<FMT, MT, THREADS>(acc_s, asum, scale_s, &last_flag, w_scale, out, M, N, out_f32, po,
+  gemv_finish<FMT, MT, THREADS>(acc_s, asum, scale_s, &last_flag, sw_s, out, M, N, out_f32, po,
                                 ll_seq, np, k_parts, n_base, n_count, ws, fz);
 }
 
 // E8P products by dp4a instead of MMAs (see gemv_dp4a for where).  An MMA spends eight columns on
 // however few rows, its form keeps two weight rows and less of them in flight per lane, and its
-// registers leave the row preparation little; this one spends four dp4a and two reads of
+// registers leave the row preparation little; this one spends two to four dp4a and a read of
 // activations per row and code word.  Lane l holds row l / LPR of a group and an LPR-th of the
-// k-block, DEPTH units in flight.
+// k-block, DEPTH units in flight.  1 x 19456 x 2560 14.8 -> 12.9 us, 1 x 2560 x 9728 12.1 -> 10.9,
+// 1 x 6144 x 2560 Q2 6.8 -> 6.6 with the fields multiplied as they are looked up and the small loads
+// ahead of the weights.  About 2 us are launch, 2.5 the first loads, 6 the products (two thirds of
+// the shared-memory reads and of the instructions that an SM can issue), 1 the outputs.
 template <int FMT, int MT>
 struct Dp4a {
   static constexpr int THREADS = MT <= 2 ? 1024 : 512;             // registers
@@ -555,28 +599,21 @@ __global__ void __launch_bounds__(Dp4a<FMT, MT>::THREADS, 1) e8p_dp4a_kernel(
   constexpr int THREADS = Dp4a<FMT, MT>::THREADS, DEPTH = 4;
   constexpr int ROWS = FMT == 1 ? 8 : 16;        // output rows of a group
   constexpr int LPR = 32 / ROWS;                 // lanes per row, 16 bytes of codes each
-  using Lut = E8pLut<GEMV_COPIES>;
   const bool ll = po.tp > 0 && po.rows_per == LL_MODE;
   const int ll_seq = ll ? *reinterpret_cast<volatile int*>(po.sent) + 1 : 0;
   extern __shared__ __align__(16) unsigned char smem_raw[];
-  Lut* lut = reinterpret_cast<Lut*>(smem_raw);
-  int8_t* act = reinterpret_cast<int8_t*>(smem_raw) + sizeof(Lut);
+  int8_t* act = reinterpret_cast<int8_t*>(smem_raw) + sizeof(E8pRows);
   int* acc_s = reinterpret_cast<int*>(act + static_cast<size_t>(MT) * K);   // [16 max_groups][MT]
   int* asum = acc_s + max_groups * 16 * MT;                                  // [MT]
   float* scale_s = reinterpret_cast<float*>(asum + MT);                      // [MT]
+  float* sw_s = scale_s + MT;                                                // [16 max_groups]
   float* fbuf = reinterpret_cast<float*>(                                    // [K], pre only
-      (reinterpret_cast<uintptr_t>(scale_s + MT) + 15) & ~static_cast<uintptr_t>(15));
+      (reinterpret_cast<uintptr_t>(sw_s + max_groups * 16) + 15) & ~static_cast<uintptr_t>(15));
   __shared__ int last_flag;
   __shared__ float red[32];
   __shared__ float blk_sum[128];
 
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-  e8p_lut_init(lut, tables, tid, THREADS);
-  for (int i = tid; i < max_groups * 16 * MT + MT; i += THREADS) acc_s[i] = 0;
-  __syncthreads();
-  gemv_rows<FMT, MT, THREADS, true>(act, asum, scale_s, fbuf, red, blk_sum, a, a_scale, M, K, fz);
-  __syncthreads();
-
   const int row = lane / LPR, part = lane % LPR;
   const int kb_all = K / 128, groups = (N + ROWS - 1) / ROWS;
   const int np = blockIdx.x % n_parts, kp = blockIdx.x / n_parts;
@@ -588,83 +625,115 @@ __global__ void __launch_bounds__(Dp4a<FMT, MT>::THREADS, 1) e8p_dp4a_kernel(
   constexpr int NW = THREADS / 32;
   const int u_lo = static_cast<int>(static_cast<long long>(units) * warp / NW);
   const int u_hi = static_cast<int>(static_cast<long long>(units) * (warp + 1) / NW);
-  int acc[MT];
-#pragma unroll
-  for (int m = 0; m < MT; ++m) acc[m] = 0;
-  const int copy = lane;                                   // GEMV_COPIES == 32
+  // (group, k-block) of the unit being loaded, and of the unit being consumed
+  int lg = g_lo, lkb = kb_lo;
   if (u_lo < u_hi) {
-    // (group, k-block) of the unit being loaded, and of the unit being consumed
-    int lg = g_lo + u_lo / kbs, lkb = kb_lo + u_lo % kbs;
-    int g = lg, kb = lkb;
-    uint4 buf[DEPTH];
-    auto fetch = [&](int uu) -> uint4 {
-      uint4 v = make_uint4(0, 0, 0, 0);
-      if (uu < u_hi) {
-        const int n = min(lg * ROWS + row, N - 1);
-        v = __ldg(w + (static_cast<size_t>(lkb) * N + n) * LPR + part);
-        if (++lkb == kb_hi) {
-          lkb = kb_lo;
-          ++lg;
-        }
+    lg += u_lo / kbs;
+    lkb += u_lo % kbs;
+  }
+  int g = lg, kb = lkb;
+  uint4 buf[DEPTH];
+  auto fetch = [&](int uu) -> uint4 {
+    uint4 v = make_uint4(0, 0, 0, 0);
+    if (uu < u_hi) {
+      const int n = min(lg * ROWS + row, N - 1);
+      v = __ldg(w + (static_cast<size_t>(lkb) * N + n) * LPR + part);
+      if (++lkb == kb_hi) {
+        lkb = kb_lo;
+        ++lg;
       }
-      return v;
-    };
+    }
+    return v;
+  };
+  // requested before the tables are filled, except where the row preparation needs the registers
+  const int n_base = g_lo * ROWS, n_count = min(g_hi * ROWS, N) - n_base;
+  GemvEarly<FMT, THREADS> early;
+  early.load(tables, a, a_scale, w_scale + n_base, n_count, M, K, fz.pre == 0, tid);
+  if (fz.pre == 0) {
 #pragma unroll
     for (int i = 0; i < DEPTH; ++i) buf[i] = fetch(u_lo + i);
-    for (int base = u_lo; base < u_hi; base += DEPTH) {
+  }
+  early.store(smem_raw, sw_s, w_scale + n_base, n_count, acc_s, max_groups * 16 * MT + MT, tid);
+  __syncthreads();
+  gemv_rows<FMT, MT, THREADS, true>(act, asum, scale_s, fbuf, red, blk_sum, a, a_scale, M, K, fz,
+                                    early);
+  __syncthreads();
+  if (fz.pre != 0) {
 #pragma unroll
-      for (int i = 0; i < DEPTH; ++i) {
-        const uint4 cur = buf[i];
-        buf[i] = fetch(base + i + DEPTH);
-        if (base + i < u_hi) {
-          const int8_t* abase = act + kb * 128 + part * (128 / LPR);
-          const uint32_t words[4] = {cur.x, cur.y, cur.z, cur.w};
+    for (int i = 0; i < DEPTH; ++i) buf[i] = fetch(u_lo + i);
+  }
+
+  // One or two rows: the fields are multiplied as they come out of the lookup (four dp4a per row
+  // and word), the odd ones sixteenfold in sums of their own; more rows: four dp4a would cost more
+  // than forming 4 * v0 + v1.
+  constexpr bool RAW = FMT == 1 && MT <= 2;
+  constexpr int SUMS = RAW ? 4 : 1;
+  int acc[MT][SUMS];
 #pragma unroll
-          for (int j = 0; j < (FMT == 1 ? 4 : 8); ++j) {
-            int xlo, xhi;
-            if (FMT == 1) {
-              const uint32_t v0 = e8p_fields<GEMV_COPIES, 0>(words[j & 3], lut, copy);
-              const uint32_t v1 = e8p_fields<GEMV_COPIES, 1>(words[j & 3], lut, copy);
-              xlo = static_cast<int>((v0 & E8P_NIB) * 4u + (v1 & E8P_NIB));
-              xhi = static_cast<int>(((v0 >> 4) & E8P_NIB) * 4u + ((v1 >> 4) & E8P_NIB));
-            } else {
-              const uint32_t v = (j & 1) ? e8p_fields<GEMV_COPIES, 1>(words[j >> 1], lut, copy)
-                                         : e8p_fields<GEMV_COPIES, 0>(words[j >> 1], lut, copy);
-              xlo = static_cast<int>(v & E8P_NIB);
-              xhi = static_cast<int>((v >> 4) & E8P_NIB);
-            }
+  for (int m = 0; m < MT; ++m)
+#pragma unroll
+    for (int q = 0; q < SUMS; ++q) acc[m][q] = 0;
+  const uint32_t lane4 = lane * 4;
+  for (int base = u_lo; base < u_hi; base += DEPTH) {
+#pragma unroll
+    for (int i = 0; i < DEPTH; ++i) {
+      const uint4 cur = buf[i];
+      buf[i] = fetch(base + i + DEPTH);
+      if (base + i < u_hi) {
+        const int8_t* abase = act + kb * 128 + part * (128 / LPR);
+        const uint32_t words[4] = {cur.x, cur.y, cur.z, cur.w};
+#pragma unroll
+        for (int j = 0; j < (FMT == 1 ? 4 : 8); ++j) {
+          if constexpr (RAW) {
+            uint32_t l0, h0, l1, h1;
+            e8p_lookup<0>(words[j & 3], smem_raw, lane4, l0, h0);
+            e8p_lookup<1>(words[j & 3], smem_raw, lane4, l1, h1);
 #pragma unroll
             for (int m = 0; m < MT; ++m) {
               const int2 av = *reinterpret_cast<const int2*>(abase + m * K + j * 8);
-              acc[m] = __dp4a(xlo, av.x, acc[m]);
-              acc[m] = __dp4a(xhi, av.y, acc[m]);
+              acc[m][0] = dp4a_us(l0, av.x, acc[m][0]);
+              acc[m][1] = dp4a_us(h0, av.y, acc[m][1]);
+              acc[m][2 % SUMS] = dp4a_us(l1, av.x, acc[m][2 % SUMS]);
+              acc[m][3 % SUMS] = dp4a_us(h1, av.y, acc[m][3 % SUMS]);
             }
-          }
-          const bool last_of_group = kb + 1 == kb_hi, last_unit = base + i + 1 == u_hi;
-          if (last_of_group || last_unit) {
+          } else {
+            const uint2 v = FMT == 1 ? e8p_bytes_q4(words[j & 3], smem_raw, lane4)
+                            : j & 1  ? e8p_bytes_q2<1>(words[j >> 1], smem_raw, lane4)
+                                     : e8p_bytes_q2<0>(words[j >> 1], smem_raw, lane4);
 #pragma unroll
             for (int m = 0; m < MT; ++m) {
-              int v = acc[m];
-#pragma unroll
-              for (int o = 1; o < LPR; o <<= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
-              if (part == 0) atomicAdd(&acc_s[((g - g_lo) * ROWS + row) * MT + m], v);
-              acc[m] = 0;
+              const int2 av = *reinterpret_cast<const int2*>(abase + m * K + j * 8);
+              acc[m][0] = dp4a_us(v.x, av.x, acc[m][0]);
+              acc[m][0] = dp4a_us(v.y, av.y, acc[m][0]);
             }
           }
-          if (last_of_group) {
-            kb = kb_lo;
-            ++g;
-          } else {
-            ++kb;
+        }
+        const bool last_of_group = kb + 1 == kb_hi, last_unit = base + i + 1 == u_hi;
+        if (last_of_group || last_unit) {
+#pragma unroll
+          for (int m = 0; m < MT; ++m) {
+            int v = acc[m][0];
+            if (RAW)
+              v = 4 * (v + acc[m][1 % SUMS] / 16) + acc[m][2 % SUMS] + acc[m][3 % SUMS] / 16;
+#pragma unroll
+            for (int o = 1; o < LPR; o <<= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+            if (part == 0) atomicAdd(&acc_s[((g - g_lo) * ROWS + row) * MT + m], v);
+#pragma unroll
+            for (int q = 0; q < SUMS; ++q) acc[m][q] = 0;
           }
+        }
+        if (last_of_group) {
+          kb = kb_lo;
+          ++g;
+        } else {
+          ++kb;
         }
       }
     }
   }
   __syncthreads();
-  gemv_finish<FMT, MT, THREADS>(acc_s, asum, scale_s, &last_flag, w_scale, out, M, N, out_f32, po,
-                                ll_seq, np, k_parts, g_lo * ROWS, min(g_hi * ROWS, N) - g_lo * ROWS,
-                                ws, fz);
+  gemv_finish<FMT, MT, THREADS>(acc_s, asum, scale_s, &last_flag, sw_s, out, M, N, out_f32, po,
+                                ll_seq, np, k_parts, n_base, n_count, ws, fz);
 }
 
 // INT8 weights by one warp per output row: 16 weights per lane per step, as many CTAs as rows
@@ -756,17 +825,20 @@ __global__ void __launch_bounds__(GEMV_THREADS, 1) qgemv_grouped_kernel(
     __half* __restrict__ out, int N, int K, long long bank_bytes,
     const E8pTables* __restrict__ tables, const int* __restrict__ tiles,
     const int* __restrict__ meta, int most_rows, int listed) {
-  using Lut = E8pLut<GEMV_COPIES>;
   using W = GemvUnit<FMT>;
   constexpr int NB = 2;                            // eight-row blocks per pass over the weights
   extern __shared__ __align__(16) unsigned char smem_raw[];
   constexpr int WARPS = GEMV_THREADS / 32;
-  Lut* lut = reinterpret_cast<Lut*>(smem_raw);
   int(*red)[NB * 5][32] = reinterpret_cast<int(*)[NB * 5][32]>(
-      smem_raw + (FMT == 0 ? 0 : sizeof(Lut)));        // [WARPS]
+      smem_raw + (FMT == 0 ? 0 : sizeof(E8pRows)));    // [WARPS]
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, g = lane >> 2, t = lane & 3;
+  const uint32_t lane4 = lane * 4;
   // MIXED lists its tiles in shared memory before the tables are filled: there may be none.
-  if (FMT != 0 && !MIXED) e8p_lut_init(lut, tables, tid, GEMV_THREADS);
+  E8pFill<GEMV_THREADS> fill;
+  if (FMT != 0 && !MIXED) {
+    fill.load(tables, tid);
+    fill.store(smem_raw, tid);
+  }
   int n_tiles = meta[0];
   const int* list = nullptr;
   if (MIXED && most_rows > 0) {
@@ -789,7 +861,10 @@ __global__ void __launch_bounds__(GEMV_THREADS, 1) qgemv_grouped_kernel(
     if (count == 0) return;
     n_tiles = min(count, listed);
     list = found;
-    if (FMT != 0) e8p_lut_init(lut, tables, tid, GEMV_THREADS);
+    if (FMT != 0) {
+      fill.load(tables, tid);
+      fill.store(smem_raw, tid);
+    }
   }
   __syncthreads();
   const int groups = N / 16, kbs = K / 128, items = n_tiles * groups;
@@ -872,18 +947,13 @@ __global__ void __launch_bounds__(GEMV_THREADS, 1) qgemv_grouped_kernel(
               if (FMT == 0) {
                 f[h] = buf[i].u.w[h][(2 * j) % W::WORDS];
                 f[2 + h] = buf[i].u.w[h][(2 * j + 1) % W::WORDS];
-              } else if (FMT == 1) {
-                const uint32_t word = buf[i].u.w[h][j % W::WORDS];
-                const uint32_t v0 = e8p_fields<GEMV_COPIES, 0>(word, lut, lane);
-                const uint32_t v1 = e8p_fields<GEMV_COPIES, 1>(word, lut, lane);
-                f[h] = (v0 & E8P_NIB) * 4u + (v1 & E8P_NIB);
-                f[2 + h] = ((v0 >> 4) & E8P_NIB) * 4u + ((v1 >> 4) & E8P_NIB);
               } else {
-                const uint32_t word = buf[i].u.w[h][(j >> 1) % W::WORDS];
-                const uint32_t v = (j & 1) ? e8p_fields<GEMV_COPIES, 1>(word, lut, lane)
-                                           : e8p_fields<GEMV_COPIES, 0>(word, lut, lane);
-                f[h] = v & E8P_NIB;
-                f[2 + h] = (v >> 4) & E8P_NIB;
+                const uint32_t word = buf[i].u.w[h][(FMT == 1 ? j : j >> 1) % W::WORDS];
+                const uint2 v = FMT == 1 ? e8p_bytes_q4(word, smem_raw, lane4)
+                                : j & 1  ? e8p_bytes_q2<1>(word, smem_raw, lane4)
+                                         : e8p_bytes_q2<0>(word, smem_raw, lane4);
+                f[h] = v.x;
+                f[2 + h] = v.y;
               }
             }
 #pragma unroll
@@ -959,7 +1029,7 @@ static int launch_grouped(const int8_t* a, const float* as, const void* w, const
                           void* out, int N, int K, long long bank, const int* tiles,
                           const int* meta, int most_rows, int max_tiles, cudaStream_t stream) {
   const int listed = most_rows > 0 ? max_tiles : 0;
-  const size_t smem = (FMT == 0 ? 0 : sizeof(E8pLut<GEMV_COPIES>)) +
+  const size_t smem = (FMT == 0 ? 0 : sizeof(E8pRows)) +
                       (static_cast<size_t>(GEMV_THREADS) * 10 + listed) * sizeof(int);
   if (smem > GEMV_SMEM_LIMIT) return -1;
   static const int slot = runtime_new_slot();
@@ -1038,8 +1108,8 @@ inline bool gemv_dp4a(int fmt, int mt, int N, int K, bool fused) {
 
 // Dynamic shared memory for `mt` staged activation rows.
 static size_t gemv_smem(int fmt, int mt, const GemvGrid& g, int K, bool fused) {
-  size_t smem = (fmt == 0 ? 0 : sizeof(E8pLut<GEMV_COPIES>)) + static_cast<size_t>(mt) * K +
-                (static_cast<size_t>(g.max_groups) * 16 * mt + 2 * mt) * sizeof(int) + 16;
+  size_t smem = (fmt == 0 ? 0 : sizeof(E8pRows)) + static_cast<size_t>(mt) * K +
+                (static_cast<size_t>(g.max_groups) * 16 * (mt + 1) + 2 * mt) * sizeof(int) + 16;
   if (fused) smem += static_cast<size_t>(K) * sizeof(float);
   return smem;
 }
