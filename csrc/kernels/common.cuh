@@ -407,8 +407,8 @@ struct E8pRows {
   uint32_t w[256][2][32];                               // [entry][e2, sg][lane]
 };
 
-// Filled in two steps, so that other loads can be under way between them: a thread's words, then its
-// 16-byte stores.
+// Filled in two steps, so that other loads can be under way between them: a thread's words, then
+// its 16-byte stores.
 template <int THREADS>
 struct E8pFill {
   static constexpr int PER = 256 * 16 / THREADS;

@@ -43,12 +43,12 @@ __device__ __forceinline__ void store_row(void* out, int out_f32, int m, int n, 
 
 // FMT 0: INT8 weights, 1: Q4 (U32 codes), 2: Q2 (U16 codes).  One persistent CTA per SM: the
 // decode tables (32 interleaved copies, so a lane's lookups never meet another lane's on a
-// bank, and an address is one byte permute: see E8pRows) and the activations are staged once.  The grid is n_parts x k_parts CTAs; a CTA owns a
-// contiguous range of 16-row groups and one range of 128-wide k-blocks, its warps take
-// contiguous runs of (group, k-block) units, every lane keeps DEPTH units of weight loads in
-// flight (the first ones are issued before the tables are filled, except in the fused forms), and
-// the partial dot products meet in shared memory (integer atomics: exact, so the result does not
-// depend on the order).
+// bank, and an address is one byte permute: see E8pRows) and the activations are staged once.  The
+// grid is n_parts x k_parts CTAs; a CTA owns a contiguous range of 16-row groups and one range of
+// 128-wide k-blocks, its warps take contiguous runs of (group, k-block) units, every lane keeps
+// DEPTH units of weight loads in flight (the first ones are issued before the tables are filled,
+// except in the fused forms), and the partial dot products meet in shared memory (integer atomics:
+// exact, so the result does not depend on the order).
 //
 // Products: m16n8k32 INT8 MMAs with the weights as A (lane (g, t) holds rows g and g + 8) and
 // the activation rows as the eight columns of B.  A lane's four code words of a k-block are
@@ -126,8 +126,8 @@ struct GemvFuse {
 
 // What a CTA needs before its first product besides weights: the decode tables, the activation rows
 // and the scales.  They are requested ahead of the weights.  Behind them they waited for a CTA's
-// first 64 KB, three times in a row: the first product came 5 us into the 13 us of 1 x 19456 x 2560,
-// 6 us into the 8 us of 8 x 2560 x 4096.
+// first 64 KB, three times in a row: the first product came 5 us into the 13 us of 1 x 19456 x
+// 2560, 6 us into the 8 us of 8 x 2560 x 4096.
 template <int FMT, int THREADS>
 struct GemvEarly {
   static constexpr int ROWS = 2;                 // 16-byte pieces of the rows per thread
@@ -170,7 +170,8 @@ template <int FMT, int MT, int THREADS, bool DP4A>
 __device__ __forceinline__ void gemv_rows(int8_t* act, int* asum, float* scale_s, float* fbuf,
                                           float* red, float* blk_sum, const int8_t* __restrict__ a,
                                           const float* __restrict__ a_scale, int M, int K,
-                                          const GemvFuse& fz, const GemvEarly<FMT, THREADS>& early) {
+                                          const GemvFuse& fz,
+                                          const GemvEarly<FMT, THREADS>& early) {
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   if (FMT == 0 || fz.pre == 0) {
     // stage the activations; their row sums ride along
@@ -582,9 +583,9 @@ __global__ void __launch_bounds__(GEMV_THREADS, 1) qgemv_kernel(
 // registers leave the row preparation little; this one spends two to four dp4a and a read of
 // activations per row and code word.  Lane l holds row l / LPR of a group and an LPR-th of the
 // k-block, DEPTH units in flight.  1 x 19456 x 2560 14.8 -> 12.9 us, 1 x 2560 x 9728 12.1 -> 10.9,
-// 1 x 6144 x 2560 Q2 6.8 -> 6.6 with the fields multiplied as they are looked up and the small loads
-// ahead of the weights.  About 2 us are launch, 2.5 the first loads, 6 the products (two thirds of
-// the shared-memory reads and of the instructions that an SM can issue), 1 the outputs.
+// 1 x 6144 x 2560 Q2 6.8 -> 6.6 with the fields multiplied as they are looked up and the small
+// loads ahead of the weights.  About 2 us are launch, 2.5 the first loads, 6 the products (two
+// thirds of the shared-memory reads and of the instructions that an SM can issue), 1 the outputs.
 template <int FMT, int MT>
 struct Dp4a {
   static constexpr int THREADS = MT <= 2 ? 1024 : 512;             // registers
@@ -791,6 +792,109 @@ __global__ void __launch_bounds__(W8_WARPS * 32) w8_gemv_kernel(
   }
   }
   if (peer != nullptr) peer_signal_done(po, gridDim.x);
+}
+
+// Large INT8 projections (the vocabulary head): a stream.  The forms above walk many short pieces
+// of rows at once (16 rows x 128 bytes per warp, or one row per warp), which left DRAM at 5 TB/s
+// however many loads were in flight.  Here a CTA per SM takes tiles of 16 whole rows, neighbouring
+// CTAs neighbouring tiles, so that all of them read one region of the matrix; a warp copies rows
+// into a ring with bulk copies, and each stage of the ring has a warp of its own that multiplies
+// the tile it holds (MMAs as above: 16 weight rows x 8 activation rows) and stores its outputs.
+// Rows lie 64 bytes past a multiple of 128 apart in shared memory, so 16-byte reads of two rows
+// meet on no bank. 151936 x 2560 (389 MB): one row 73.7 -> 57.8 us (6.7 TB/s), four 74.5 -> 60.2,
+// eight 76.7 -> 63.4. Below about 24 M weights the set-up of the rings costs more than it gives:
+// one row of 12288 x 2560 9.3 -> 9.1 us, eight rows 12.5 both ways, but 6144 x 2560 5.7 -> 6.7 and
+// 9.1 -> 9.9.  It takes three stages: with the two that eight rows of 4096 channels leave, 32000
+// rows gain nothing.
+constexpr int STREAM_ROWS = 16, STREAM_MAX = 8;
+
+inline int w8_stream_stages(int M, int K) {
+  const size_t row = K + 64;
+  const size_t rows = M * row;
+  const size_t fit = rows > GEMV_SMEM_LIMIT ? 0 : (GEMV_SMEM_LIMIT - rows) / (STREAM_ROWS * row);
+  return static_cast<int>(fit < STREAM_MAX ? fit : STREAM_MAX);
+}
+
+inline bool w8_streams(int M, int N, int K) {
+  return w8_stream_stages(M, K) >= 3 && static_cast<long long>(N) * K >= 24000000;
+}
+
+__global__ void __launch_bounds__((1 + STREAM_MAX) * 32) w8_stream_kernel(
+    const int8_t* __restrict__ a, const float* __restrict__ a_scale, const int8_t* __restrict__ w,
+    const __half* __restrict__ w_scale, void* __restrict__ out, int M, int N, int K, int out_f32,
+    int stages, int* status) {
+  extern __shared__ __align__(16) unsigned char smem_raw[];
+  __shared__ __align__(8) uint64_t full[STREAM_MAX], empty[STREAM_MAX];
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, g = lane >> 2, t = lane & 3;
+  const int stride = K + 64, tiles = (N + STREAM_ROWS - 1) / STREAM_ROWS;
+  unsigned char* act = smem_raw;                           // [M][stride]
+  unsigned char* ring = smem_raw + M * stride;             // [stages][16][stride]
+  const int count = (tiles - static_cast<int>(blockIdx.x) + gridDim.x - 1) / gridDim.x;
+  if (threadIdx.x == 0) {
+    for (int s = 0; s < stages; ++s) {
+      mbar_init(&full[s], 1);
+      mbar_init(&empty[s], 1);
+    }
+    mbar_fence_init();
+  }
+  for (int c = threadIdx.x; c < M * (K / 16); c += blockDim.x) {
+    const int m = c / (K / 16), k = (c - m * (K / 16)) * 16;
+    *reinterpret_cast<int4*>(act + m * stride + k) =
+        *reinterpret_cast<const int4*>(a + static_cast<size_t>(m) * K + k);
+  }
+  __syncthreads();
+  if (warp == 0) {
+    int issued = 0;
+    for (int i = 0; i < count; ++i) {
+      const int s = i % stages;
+      const bool ok = mbar_wait(&empty[s], ((i / stages) & 1) ^ 1, status, STATUS_TMA_WAIT, i);
+      if (!__all_sync(0xffffffffu, ok)) break;
+      const int n0 = (blockIdx.x + i * gridDim.x) * STREAM_ROWS, rows = min(STREAM_ROWS, N - n0);
+      if (lane == 0) mbar_expect_tx(&full[s], rows * K);
+      __syncwarp();
+      if (lane < rows)
+        bulk_load(ring + static_cast<size_t>(s * STREAM_ROWS + lane) * stride,
+                  w + static_cast<size_t>(n0 + lane) * K, K, &full[s]);
+      issued = i + 1;
+    }
+    // no copy of ours is in flight when the CTA ends
+    for (int i = max(0, issued - stages); i < issued; ++i)
+      mbar_wait(&full[i % stages], (i / stages) & 1, status, STATUS_TMA_WAIT, 0x4000);
+    return;
+  }
+  const int s = warp - 1;
+  const float sa0 = 2 * t < M ? a_scale[2 * t] : 0.f;
+  const float sa1 = 2 * t + 1 < M ? a_scale[2 * t + 1] : 0.f;
+  const unsigned char* brow = act + min(g, M - 1) * stride + t * 16;
+  const unsigned char* r0 = ring + static_cast<size_t>(s * STREAM_ROWS + g) * stride + t * 16;
+  const unsigned char* r1 = r0 + 8 * stride;
+  const bool live = g < M;                                 // columns past the last row are zero
+  for (int i = s; i < count; i += stages) {
+    const int n = (blockIdx.x + i * gridDim.x) * STREAM_ROWS + g;
+    const float w0 = n < N ? __half2float(w_scale[n]) : 0.f;
+    const float w1 = n + 8 < N ? __half2float(w_scale[n + 8]) : 0.f;
+    const bool ok = mbar_wait(&full[s], (i / stages) & 1, status, STATUS_DECODE_WAIT, i);
+    if (!__all_sync(0xffffffffu, ok)) break;
+    int acc[2][4] = {};
+#pragma unroll 4
+    for (int k = 0; k < K; k += 64) {
+      const uint4 x = *reinterpret_cast<const uint4*>(r0 + k);
+      const uint4 y = *reinterpret_cast<const uint4*>(r1 + k);
+      uint4 b = make_uint4(0, 0, 0, 0);
+      if (live) b = *reinterpret_cast<const uint4*>(brow + k);
+      mma_i8_16832(acc[0], x.x, y.x, x.y, y.y, b.x, b.y);
+      mma_i8_16832(acc[1], x.z, y.z, x.w, y.w, b.z, b.w);
+    }
+    __syncwarp();
+    if (lane == 0) mbar_arrive(&empty[s]);
+#pragma unroll
+    for (int e = 0; e < 4; ++e) {
+      const int m = 2 * t + (e & 1), at = n + (e >> 1) * 8;
+      if (m < M && at < N)
+        store_row<1>(out, out_f32, m, at, N, acc[0][e] + acc[1][e], e >> 1 ? w1 : w0,
+                     e & 1 ? sa1 : sa0);
+    }
+  }
 }
 
 // ---------------------------------------------------------------- experts with few rows each
@@ -1155,6 +1259,19 @@ static int launch_w8(const int8_t* a, const float* as, const void* w, const __ha
   return static_cast<int>(cudaGetLastError());
 }
 
+static int launch_w8_stream(const int8_t* a, const float* as, const void* w, const __half* ws,
+                            void* out, int M, int N, int K, int out_f32, cudaStream_t stream) {
+  const int stages = w8_stream_stages(M, K);
+  const size_t smem = static_cast<size_t>(K + 64) * (M + stages * STREAM_ROWS);
+  static const int slot = runtime_new_slot();
+  if (const int e = runtime_allow_smem(slot, w8_stream_kernel, GEMV_SMEM_LIMIT)) return e;
+  const int tiles = (N + STREAM_ROWS - 1) / STREAM_ROWS;
+  w8_stream_kernel<<<tiles < 148 ? tiles : 148, (1 + stages) * 32, smem, stream>>>(
+      a, as, reinterpret_cast<const int8_t*>(w), ws, out, M, N, K, out_f32, stages,
+      runtime_status_ptr());
+  return static_cast<int>(cudaGetLastError());
+}
+
 int qgemv_dispatch(int fmt, const int8_t* a, const float* as, const void* w, const __half* ws,
                    void* out, int M, int N, int K, int out_f32, cudaStream_t stream,
                    const PeerOut* peer) {
@@ -1185,6 +1302,8 @@ int qgemv_dispatch(int fmt, const int8_t* a, const float* as, const void* w, con
    : M == 2 ? FN<__VA_ARGS__ 2>(a, as, w, ws, out, M, N, K, out_f32, stream, po) \
    : M <= 4 ? FN<__VA_ARGS__ 4>(a, as, w, ws, out, M, N, K, out_f32, stream, po) \
             : FN<__VA_ARGS__ 8>(a, as, w, ws, out, M, N, K, out_f32, stream, po))
+  if (fmt == 0 && po.tp == 0 && w8_streams(M, N, K))
+    return launch_w8_stream(a, as, w, ws, out, M, N, K, out_f32, stream);
   if (fmt == 0 && w8_by_rows(M, N, K)) return BY_M(launch_w8, );
   if (fmt == 0)
     return M <= 4 ? launch_gemv<0, 4>(a, as, w, ws, out, M, N, K, out_f32, stream, po)

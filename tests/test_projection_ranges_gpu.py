@@ -49,6 +49,24 @@ def test_small_row_projections_are_exact(dev, fmt, m, n, k):
         assert torch.equal(out.cpu(), want if f32 else want.half())
 
 
+@pytest.mark.parametrize("m", [1, 2, 3, 8])
+@pytest.mark.parametrize("n,k", [(93752, 256), (187504, 128), (23440, 1024), (7512, 3200),
+                                 (24008, 1024)])
+def test_streamed_int8_projections_are_exact(dev, m, n, k):
+    """From 24 million weights on: short rows and the longest that keep three ring stages, a last
+    tile of eight rows, CTAs with one tile more than others."""
+    from orinfer_b200.ops import functional as F
+    g = torch.Generator(device=dev).manual_seed(m * n + k)
+    w = torch.randint(-127, 128, (n, k), generator=g, device=dev, dtype=torch.int8)
+    ws = (torch.rand(n, generator=g, device=dev) * 0.01 + 1e-3).half()
+    a = torch.randint(-127, 128, (m, k), generator=g, device=dev, dtype=torch.int8)
+    sa = torch.rand(m, generator=g, device=dev) * 0.05 + 1e-3
+    want = _scaled(a, sa, w, ws)
+    for f32 in (False, True):
+        out = F.qgemm(a, sa, w, ws, "w8", n, out_f32=f32, path=1)
+        assert torch.equal(out, want if f32 else want.half())
+
+
 @pytest.mark.parametrize("fmt", ["w8", "q4", "q2"])
 @pytest.mark.parametrize("m,n", [(260, 19456), (600, 19456), (1024, 19456), (1500, 6400),
                                  (2047, 9728), (2048, 19456)])
