@@ -503,7 +503,8 @@ __global__ void __launch_bounds__(256) gdn_scan_split_kernel(
 // below 1/2 a row 1.6e-7 and 1.1e-7 (1.5e-7 and 1.1e-7).
 //
 // 32 heads of 128 channels, one run of 1050 rows: 406 us as a scan (0.39 us per dependent step),
-// 195 us here (166 with chained sums); 16 runs of 64 rows: 192 -> 84 us.
+// 195 us here (166 with chained sums), 164 since the helpers alone copy the chunks; 16 runs of 64
+// rows: 192 -> 84 -> 78 us.
 // Runs below GDN_LONG_ROWS keep the scan: one run of 36 rows takes 17.2 us there and 19.4 here, of
 // 40 rows 19.4 both ways, of 63 rows 28.0 and 19.4 (two runs of 50: 33 and 20).  The scan's bits
 // are those of a verification pass, whose segments are shorter.
@@ -652,28 +653,27 @@ __global__ void __launch_bounds__(CHUNK_THREADS, 2) gdn_chunk_kernel(
   const int chunks = (seg.rows + CHUNK - 1) / CHUNK;
   const float scale = rsqrtf(static_cast<float>(D));
 
-  // copy of one chunk: 16 + 16 + 8 16-byte units per row; rows past the run become zeros
+  // Copy of one chunk by the two helper warps, eight threads a row, five 16-byte units each; rows
+  // past the run become zeros.  (Spread over all threads, the copies held up the warps that carry
+  // the state.)
   auto stage = [&](int c) {
     const int st = c % 3, n = min(CHUNK, seg.rows - c * CHUNK);
-    for (int i = tid; i < CHUNK * 40; i += CHUNK_THREADS) {
-      const int r = i / 40, u = i % 40;
-      const size_t at = static_cast<size_t>(seg.row_start + c * CHUNK + min(r, n - 1));
-      const __half* row = qkv + at * conv_dim;
-      const __half* src;
-      __half* dst;
-      if (u < 16) {
-        src = row + kh * D + u * 8;
-        dst = &sm.q[st][r][u * 8];
-      } else if (u < 32) {
-        src = row + dk_total + kh * D + (u - 16) * 8;
-        dst = &sm.k[st][r][(u - 16) * 8];
-      } else {
-        src = row + 2 * dk_total + vh * D + dv0 + (u - 32) * 8;
-        dst = &sm.v[st][r][(u - 32) * 8];
-      }
-      const unsigned a = smem_u32(dst), bytes = r < n ? 16 : 0;
-      asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(a), "l"(src), "r"(bytes)
-                   : "memory");
+    const int at = (tid - 128) >> 3, s = (tid & 7) * 8;
+#pragma unroll
+    for (int pass = 0; pass < CHUNK / 8; ++pass) {
+      const int r = pass * 8 + at, bytes = r < n ? 16 : 0;
+      const __half* row =
+          qkv + static_cast<size_t>(seg.row_start + c * CHUNK + min(r, n - 1)) * conv_dim + s;
+      auto copy = [&](__half* dst, const __half* src) {
+        asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(smem_u32(dst)), "l"(src),
+                     "r"(bytes)
+                     : "memory");
+      };
+      copy(&sm.q[st][r][s], row + kh * D);
+      copy(&sm.q[st][r][s + 64], row + kh * D + 64);
+      copy(&sm.k[st][r][s], row + dk_total + kh * D);
+      copy(&sm.k[st][r][s + 64], row + dk_total + kh * D + 64);
+      copy(&sm.v[st][r][s], row + 2 * dk_total + vh * D + dv0);
     }
     asm volatile("cp.async.commit_group;" ::: "memory");
   };
@@ -814,9 +814,11 @@ __global__ void __launch_bounds__(CHUNK_THREADS, 2) gdn_chunk_kernel(
     }
   };
 
-  stage(0);
-  if (chunks > 1) stage(1);
-  if (warp >= 4) fetch_gates(0);
+  if (warp >= 4) {
+    stage(0);
+    if (chunks > 1) stage(1);
+    fetch_gates(0);
+  }
 
   // ---- this warp's slice of S^T: rows dv, columns dk = 8 u + 2 t (+ 1)
   const bool fresh = row_pos[seg.row_start] == 0;
@@ -843,8 +845,8 @@ __global__ void __launch_bounds__(CHUNK_THREADS, 2) gdn_chunk_kernel(
   __syncthreads();
 
   for (int c = 0; c < chunks; ++c) {
-    if (c + 2 < chunks) stage(c + 2);          // its buffer was last read in round c - 1
     if (warp >= 4) {
+      if (c + 2 < chunks) stage(c + 2);        // its buffer was last read in round c - 1
       if (c + 1 < chunks) prepare(c + 1);
     } else {
       const int st = c % 3, buf = c & 1;
