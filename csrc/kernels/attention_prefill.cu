@@ -7,26 +7,31 @@
 // head sizes 64 and 128 two neighbouring ones, so that a dequantised page serves 256 rows and the
 // tensor core works on one tile while the softmax warps of the other are busy.  Per step of KT
 // keys:
-//   * eight warps, in two groups that take the steps in turn, read the INT8 page and its
-//     group-64 FP16 scales straight from global memory (ahead, in registers), dequantise to
-//     FP16 and store K and V as 128-byte-swizzled tiles (K is the K-major B operand of
-//     S = Q K^T, V the MN-major B operand of O += P V);
+//   * eight warps read the INT8 page and its group-64 FP16 scales straight from global memory (a
+//     step ahead, in registers), dequantise to FP16 and store K and V as 128-byte-swizzled tiles
+//     (K is the K-major B operand of S = Q K^T, V the MN-major B operand of O += P V);
 //   * warp 1 issues tcgen05.mma kind::f16: S (128 x KT fp32) and O (128 x D fp32) live in TMEM;
-//   * four warps per tile own one query row per thread: they read S from TMEM, apply scale and
-//     the causal mask, and write P as FP16 over S in TMEM, where the second MMA reads it as its
-//     A operand.  P is relative to the row's running maximum, so its largest weight is exactly 1
-//     and O is rescaled whenever a row of the warp finds a larger score;
+//   * eight warps per tile own two threads per query row, each with half of the step's keys: they
+//     read S from TMEM, apply scale and the causal mask, and write P as FP16 over their half of S,
+//     where the second MMA reads it as its A operand.  The two meet once per step, for the row's
+//     maximum.  P is relative to the row's running maximum, so its largest weight is exactly 1 and
+//     O is rescaled whenever a row of the warp finds a larger score;
 //   * warp 0 loads the Q tiles once with a 3-D TMA (d, head, position).
 // With one tile S is double buffered instead.  Head size 256 has room for no more (Q 64 KB, two K
 // and two V buffers of 32 KB; TMEM: two S of 64 columns and O of 256) and walks the cache in half
 // pages.
 // CTAs are ordered from the last query positions (the longest walks) to the first.
 //
+// A step of two tiles is a chain per tile (softmax, P V, Q K^T of the next step) and two of them
+// hide each other only in part: with one thread per row 5500 cycles for 128 keys, of which softmax
+// 3700, with two threads 5000 and 2700.  The tensor core needs 3000 of them, the exponentials 2050.
 // One 4096-token chunk, 32 / 8 heads of 128: 377 us with one tile per CTA and P in shared memory,
-// 242 us now (568 TFLOP/s causal).  A reference that follows the maximum only when it lags by
-// 2^8 takes 215 us (fewer rescales of O) but rounds the largest weights in FP16: the error
-// against 64 bits grows by 1.8 % there and by 3.7 % for 500 rows behind 1000.  Chunks of 777 and
-// 646 rows behind 3000 positions, 16 / 2 gated heads of 256: 354 -> 274 us (180 CTAs: 1.2 waves).
+// 244 with two tiles and P in TMEM, 213 with two threads per row (645 TFLOP/s causal); 512 tokens
+// 18.3 -> 15.3 us with the last change, 17 tokens 10.8 -> 8.5.  A reference that follows the
+// maximum only when it lags by 2^8 saves another tenth (fewer rescales of O) but rounds the largest
+// weights in FP16: the error against 64 bits grows by 1.8 % there and by 3.7 % for 500 rows behind
+// 1000.  Chunks of 777 and 646 rows behind 3000 positions, 16 / 2 gated heads of 256: 354 -> 284 ->
+// 276 us (180 CTAs: 1.2 waves).
 // Output is O / sum, optionally times sigmoid(gate), in FP16.  Replaces the prefill
 // configurations of causal_attention_int8 and dequantize_attention_kv
 // (kernels/cuda/model/attention_rows.py:61-276, kernels/cuda/model/kv_int8.py:210-247).
@@ -44,7 +49,7 @@ constexpr int DQ_WARPS = 8;                  // dequantisation warps
 
 template <int D, int NQ>                                 // NQ: query tiles per CTA
 struct Smem {
-  static constexpr int THREADS = (2 + 4 * NQ + DQ_WARPS) * 32;
+  static constexpr int THREADS = (2 + 8 * NQ + DQ_WARPS) * 32;
   static constexpr int KT = D > 128 ? 64 : 128;          // keys per step
   static constexpr int SUB = TILE * 128;                 // one [128 x 64 fp16] sub-tile (Q)
   static constexpr int KSUB = KT * 128;                  // one [KT x 64 fp16] sub-tile (K, V)
@@ -53,7 +58,8 @@ struct Smem {
   static constexpr int K_OFF = Q_OFF + NQ * NSUB * SUB;  // two K buffers
   static constexpr int V_OFF = K_OFF + 2 * NSUB * KSUB;  // two V buffers
   static constexpr int BAR_OFF = V_OFF + 2 * NSUB * KSUB;
-  static constexpr int TOTAL = BAR_OFF + 256 + 1024;
+  static constexpr int MAX_OFF = BAR_OFF + 256;          // [NQ][2 steps][2 halves][128] row maxima
+  static constexpr int TOTAL = MAX_OFF + NQ * 4 * TILE * 4 + 1024;
   static_assert(TOTAL <= 227 * 1024, "exceeds the shared memory of one CTA");
 };
 
@@ -65,6 +71,16 @@ __device__ __forceinline__ void mma_f16_ts(uint32_t tmem_d, uint32_t tmem_a, uin
       "setp.ne.b32 p, %4, 0;\n\t"
       "tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], %2, %3, p;\n\t}" ::"r"(tmem_d),
       "r"(tmem_a), "l"(bdesc), "r"(idesc), "r"(accumulate)
+      : "memory");
+}
+
+// 32 lanes x 16 consecutive 32-bit columns
+__device__ __forceinline__ void tmem_st_32x16(uint32_t taddr, const uint32_t (&r)[16]) {
+  asm volatile(
+      "tcgen05.st.sync.aligned.32x32b.x16.b32 [%0], "
+      "{%1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15, %16};" ::"r"(taddr),
+      "r"(r[0]), "r"(r[1]), "r"(r[2]), "r"(r[3]), "r"(r[4]), "r"(r[5]), "r"(r[6]), "r"(r[7]),
+      "r"(r[8]), "r"(r[9]), "r"(r[10]), "r"(r[11]), "r"(r[12]), "r"(r[13]), "r"(r[14]), "r"(r[15])
       : "memory");
 }
 
@@ -149,9 +165,9 @@ __global__ void __launch_bounds__(Smem<D, NQ>::THREADS, 1) attn_prefill_kernel(
   if (threadIdx.x == 0) {
     mbar_init(q_full, 1);
     for (int b = 0; b < 2; ++b) {
-      mbar_init(&kv_ready[b], 128);
+      mbar_init(&kv_ready[b], DQ_WARPS);
       mbar_init(&s_full[b], 1);
-      mbar_init(&p_ready[b], 128);
+      mbar_init(&p_ready[b], 8);
       mbar_init(&o_done[b], 1);
       mbar_init(&kv_free[b], 1);
     }
@@ -209,7 +225,8 @@ __global__ void __launch_bounds__(Smem<D, NQ>::THREADS, 1) attn_prefill_kernel(
         const uint32_t v_addr = smem_u32(smem + L::V_OFF + (j & 1) * NSUB * L::KSUB);
 #pragma unroll
         for (int i = 0; i < KT / 16; ++i)
-          mma_f16_ts(tmem_o + 128 * q, tmem_s + S_STRIDE * sb + i * 8,
+          mma_f16_ts(tmem_o + 128 * q,
+                     tmem_s + S_STRIDE * sb + i / (KT / 32) * (KT / 2) + i % (KT / 32) * 8,
                      umma_desc(v_addr + i * 2048, L::KSUB, 1024), idesc_o, (j | i) != 0 ? 1u : 0u);
         tc_commit(&o_done[q]);
       };
@@ -237,18 +254,14 @@ __global__ void __launch_bounds__(Smem<D, NQ>::THREADS, 1) attn_prefill_kernel(
         }
       }
     }
-  } else if (warp >= 2 + 4 * NQ) {
+  } else if (warp >= 2 + 8 * NQ) {
     // ---------------- dequant warps: INT8 page -> FP16 swizzled K / V tiles
-    // Two groups of four warps take the steps (and their buffer) in turn: a step's loads are in
-    // flight while the other group converts, which a single group could only do with twice the
-    // registers (measured: the wait for the loads bounded a step).
-    const int group = (warp - (2 + 4 * NQ)) >> 2;
-    static_assert(DQ_WARPS == 8, "two groups of 128 threads");
+    // The raw rows of step j + 1 are in flight while step j is multiplied; a step has two buffers.
     constexpr int CPK = D / 16;                      // 16-byte chunks per key
-    constexpr int ITERS = KT * CPK / 128;
+    constexpr int DQ = DQ_WARPS * 32, ITERS = KT * CPK / DQ;
     uint4 kraw[ITERS], vraw[ITERS];
     __half2 sc[ITERS];                               // key scale, value scale
-    const int u = (threadIdx.x - (2 + 4 * NQ) * 32) & 127;
+    const int u = threadIdx.x - (2 + 8 * NQ) * 32;
     auto load = [&](int j, int page) {
       const int key_base = j * KT % TILE;            // first key of this step inside the page
       if (page < 0 || page >= num_pages) {
@@ -261,7 +274,7 @@ __global__ void __launch_bounds__(Smem<D, NQ>::THREADS, 1) attn_prefill_kernel(
       const int8_t* vp = vc + slot * D + (u % CPK) * 16;
       const __half* ksp = ks + slot * GROUPS + (u % CPK) / 4;
       const __half* vsp = vs + slot * GROUPS + (u % CPK) / 4;
-      const int rows = (128 / CPK) * kvh;
+      const int rows = (DQ / CPK) * kvh;
       // Keys past the last position that a row of this CTA sees may be slots never written.  Their
       // weight is zero, but zero times an infinite or NaN value is not: they get no value scale.
       const int live = kv_end - j * KT - u / CPK;
@@ -269,25 +282,25 @@ __global__ void __launch_bounds__(Smem<D, NQ>::THREADS, 1) attn_prefill_kernel(
       for (int it = 0; it < ITERS; ++it) {
         kraw[it] = __ldg(reinterpret_cast<const uint4*>(kp + static_cast<size_t>(it) * rows * D));
         vraw[it] = __ldg(reinterpret_cast<const uint4*>(vp + static_cast<size_t>(it) * rows * D));
-        const __half vsc = it * (128 / CPK) < live ? vsp[it * rows * GROUPS] : __half(0.f);
+        const __half vsc = it * (DQ / CPK) < live ? vsp[it * rows * GROUPS] : __half(0.f);
         sc[it] = __halves2half2(ksp[it * rows * GROUPS], vsc);
       }
     };
     bool ok = true;
-    unsigned char* kb = smem + L::K_OFF + group * NSUB * L::KSUB;
-    unsigned char* vb = smem + L::V_OFF + group * NSUB * L::KSUB;
     int page = 0;
-    if (group < n_max) load(group, pages[group * KT / TILE]);
-    if (group + 2 < n_max) page = pages[(group + 2) * KT / TILE];
-    for (int j = group; j < n_max && ok; j += 2) {
-      // buffer `group` was last read by the MMAs of step j - 2.  A per-buffer barrier is used
-      // because a waiter two phases behind a shared barrier would alias its parity.
-      if (j >= 2)
-        ok = mbar_wait(&kv_free[group], ((j >> 1) - 1) & 1, status, STATUS_DECODE_WAIT, j);
+    load(0, pages[0]);
+    if (n_max > 1) page = pages[KT / TILE];
+    for (int j = 0; j < n_max && ok; ++j) {
+      const int buf = j & 1;
+      unsigned char* kb = smem + L::K_OFF + buf * NSUB * L::KSUB;
+      unsigned char* vb = smem + L::V_OFF + buf * NSUB * L::KSUB;
+      // the buffer was last read by the MMAs of step j - 2
+      if (j >= 2) ok = mbar_wait(&kv_free[buf], ((j >> 1) - 1) & 1, status, STATUS_DECODE_WAIT, j);
+      ok = __all_sync(0xffffffffu, ok);
       if (!ok) break;
 #pragma unroll
       for (int it = 0; it < ITERS; ++it) {
-        const int key = it * (128 / CPK) + u / CPK, c = u % CPK;
+        const int key = it * (DQ / CPK) + u / CPK, c = u % CPK;
         const __half2 k2 = __low2half2(sc[it]), v2 = __high2half2(sc[it]);
         const int chunk = (c % 4) * 2;
         unsigned char* kd = kb + (c / 4) * L::KSUB;
@@ -300,15 +313,17 @@ __global__ void __launch_bounds__(Smem<D, NQ>::THREADS, 1) attn_prefill_kernel(
             dequant8(vraw[it].z, vraw[it].w, v2);
       }
       fence_proxy_async();
-      mbar_arrive(&kv_ready[group]);
-      if (j + 2 < n_max) {
-        load(j + 2, page);
-        if (j + 4 < n_max) page = pages[(j + 4) * KT / TILE];
+      __syncwarp();
+      if (lane == 0) mbar_arrive(&kv_ready[buf]);
+      if (j + 1 < n_max) {
+        load(j + 1, page);
+        if (j + 2 < n_max) page = pages[(j + 2) * KT / TILE];
       }
     }
   } else {
-    // ---------------- softmax warps: one query row per thread
-    const int q = (warp - 2) >> 2;                          // tile
+    // ---------------- softmax warps: two threads per query row, each with half of a step's keys
+    const int q = (warp - 2) >> 3;                          // tile
+    const int half = ((warp - 2) >> 2) & 1;
     const int quad = warp & 3;
     const int row = quad * 32 + lane;                       // row of the tile = TMEM lane
     const int first = p_first + q * P;
@@ -317,132 +332,147 @@ __global__ void __launch_bounds__(Smem<D, NQ>::THREADS, 1) attn_prefill_kernel(
     const int q_pos = valid ? ch.pos0 + first + p_rel : -1;
     const float scale = rsqrtf(static_cast<float>(D)) * 1.4426950408889634f;
     const uint32_t lane_addr = static_cast<uint32_t>(quad * 32) << 16;
-    const uint32_t tmem_oq = tmem_o + 128 * q + lane_addr;
+    constexpr int KH = KT / 2, DH = D / 2;                  // keys and channels of a thread
+    const uint32_t tmem_oq = tmem_o + 128 * q + half * DH + lane_addr;
     const int steps = NQ == 2 && q == 1 ? n_steps[NQ - 1] : n_steps[0];
+    // maxima of both halves, double buffered: a slot is rewritten two exchanges later
+    float* row_max = reinterpret_cast<float*>(smem + L::MAX_OFF) + q * 4 * TILE + row;
+    auto meet = [&]() {                                     // the two warps of these rows
+      asm volatile("bar.sync %0, 64;" ::"r"(1 + q * 4 + quad) : "memory");
+    };
     float m_run = -INFINITY, l_run = 0.f;
     bool ok = true;
     for (int j = 0; j < steps; ++j) {
       const int sb = NQ == 2 ? q : j & 1;
       const uint32_t parity = (NQ == 2 ? j : j >> 1) & 1;
-      const uint32_t tmem_sj = tmem_s + S_STRIDE * sb + lane_addr;
-      ok = mbar_wait(&s_full[sb], parity, status, STATUS_EPILOGUE_WAIT, j);
+      const uint32_t tmem_sj = tmem_s + S_STRIDE * sb + half * KH + lane_addr;
+      ok = ok && mbar_wait(&s_full[sb], parity, status, STATUS_EPILOGUE_WAIT, j);
       ok = __all_sync(0xffffffffu, ok);
-      if (!ok) break;
+      if (!ok) {                                  // a warp that gave up still meets its partner
+        meet();
+        continue;
+      }
       tc_fence_after();
-      const int key0 = j * KT;
+      const int key0 = j * KT + half * KH;
       // Only the last page of a row can hold keys beyond its position; every earlier page
       // takes the mask-free path.
-      const bool full_warp = __all_sync(0xffffffffu, key0 + KT - 1 <= q_pos);
-      // pass 1: row maximum (of the raw scores: the scale is positive)
+      const bool full_warp = __all_sync(0xffffffffu, key0 + KH - 1 <= q_pos);
+      // pass 1: row maximum (of the raw scores: the scale is positive); the first 32 scores stay in
+      // registers
+      uint32_t r[32];
       float m0 = -INFINITY, m1 = -INFINITY;
-#pragma unroll 1
-      for (int c0 = 0; c0 < KT; c0 += 64) {
-        uint32_t r[32], r2[32];                           // two TMEM loads in flight
+      auto peak = [&](int c0) {
         tmem_ld_32x32(tmem_sj + c0, r);
-        tmem_ld_32x32(tmem_sj + c0 + 32, r2);
         tc_wait_ld();
         if (full_warp) {
 #pragma unroll
-          for (int i = 0; i < 32; ++i) {
+          for (int i = 0; i < 32; i += 2) {
             m0 = fmaxf(m0, __uint_as_float(r[i]));
-            m1 = fmaxf(m1, __uint_as_float(r2[i]));
+            m1 = fmaxf(m1, __uint_as_float(r[i + 1]));
           }
         } else {
 #pragma unroll
-          for (int i = 0; i < 32; ++i) {
+          for (int i = 0; i < 32; ++i)
             if (key0 + c0 + i <= q_pos) m0 = fmaxf(m0, __uint_as_float(r[i]));
-            if (key0 + c0 + 32 + i <= q_pos) m1 = fmaxf(m1, __uint_as_float(r2[i]));
+        }
+      };
+      if (KH == 64) peak(32);
+      peak(0);
+      float* slot = row_max + (j & 1) * 2 * TILE;
+      slot[half * TILE] = fmaxf(m0, m1);
+      meet();
+      const float m_tile = fmaxf(slot[0], slot[TILE]) * scale;      // -inf stays -inf
+      const float m_new = fmaxf(m_run, m_tile);
+      const float corr = m_new == -INFINITY ? 1.f : ex2(m_run - m_new);
+      // pass 2: probabilities -> FP16 over the scores already read, row sum
+      float l_tile = 0.f;
+      auto weigh = [&](int c0) {
+        uint32_t packed[16];
+        if (full_warp) {
+#pragma unroll
+          for (int i = 0; i < 32; i += 2) {
+            const float p0 = ex2(fmaf(__uint_as_float(r[i]), scale, -m_new));
+            const float p1 = ex2(fmaf(__uint_as_float(r[i + 1]), scale, -m_new));
+            l_tile += p0 + p1;
+            const __half2 hp = __floats2half2_rn(p0, p1);
+            packed[i / 2] = *reinterpret_cast<const uint32_t*>(&hp);
+          }
+        } else {
+#pragma unroll
+          for (int i = 0; i < 32; i += 2) {
+            float p0 = ex2(fmaf(__uint_as_float(r[i]), scale, -m_new));
+            float p1 = ex2(fmaf(__uint_as_float(r[i + 1]), scale, -m_new));
+            if (key0 + c0 + i > q_pos) p0 = 0.f;
+            if (key0 + c0 + i + 1 > q_pos) p1 = 0.f;
+            l_tile += p0 + p1;
+            const __half2 hp = __floats2half2_rn(p0, p1);
+            packed[i / 2] = *reinterpret_cast<const uint32_t*>(&hp);
           }
         }
+        tmem_st_32x16(tmem_sj + c0 / 2, packed);
+      };
+      weigh(0);
+      if (KH == 64) {
+        tmem_ld_32x32(tmem_sj + 32, r);
+        tc_wait_ld();
+        weigh(32);
       }
-      const float m_tile = fmaxf(m0, m1) * scale;       // -inf stays -inf
       // O holds steps 0..j-1 once PV of step j-1 is done.  Waited for at every step, so that no
       // wait is ever two phases away from its barrier; NQ = 2: it is done, QK ran after it.
       if (j >= 1) {
         ok = mbar_wait(&o_done[q], (j - 1) & 1, status, STATUS_EPILOGUE_WAIT, 0x100 | j);
         ok = __all_sync(0xffffffffu, ok);
-        if (!ok) break;
+        if (!ok) continue;
         tc_fence_after();
       }
-      const float m_new = fmaxf(m_run, m_tile);
-      const float corr = m_new == -INFINITY ? 1.f : ex2(m_run - m_new);
       if (j >= 1 && !__all_sync(0xffffffffu, corr == 1.f)) {
 #pragma unroll 1
-        for (int c0 = 0; c0 < D; c0 += 32) {
-          uint32_t r[32];
+        for (int c0 = 0; c0 < DH; c0 += 32) {
           tmem_ld_32x32(tmem_oq + c0, r);
           tc_wait_ld();
 #pragma unroll
           for (int i = 0; i < 32; ++i) r[i] = __float_as_uint(__uint_as_float(r[i]) * corr);
           tmem_st_32x32(tmem_oq + c0, r);
         }
-        tc_wait_st();
-      }
-      // pass 2: probabilities -> FP16 over the scores already read, row sum
-      float l_tile = 0.f;
-#pragma unroll 1
-      for (int c0 = 0; c0 < KT; c0 += 64) {
-        uint32_t packed[32];
-#pragma unroll
-        for (int hf = 0; hf < 2; ++hf) {
-          uint32_t r[32];
-          tmem_ld_32x32(tmem_sj + c0 + hf * 32, r);
-          tc_wait_ld();
-          if (full_warp) {
-#pragma unroll
-            for (int i = 0; i < 32; i += 2) {
-              const float p0 = ex2(fmaf(__uint_as_float(r[i]), scale, -m_new));
-              const float p1 = ex2(fmaf(__uint_as_float(r[i + 1]), scale, -m_new));
-              l_tile += p0 + p1;
-              const __half2 hp = __floats2half2_rn(p0, p1);
-              packed[hf * 16 + i / 2] = *reinterpret_cast<const uint32_t*>(&hp);
-            }
-          } else {
-#pragma unroll
-            for (int i = 0; i < 32; i += 2) {
-              float p0 = ex2(fmaf(__uint_as_float(r[i]), scale, -m_new));
-              float p1 = ex2(fmaf(__uint_as_float(r[i + 1]), scale, -m_new));
-              if (key0 + c0 + hf * 32 + i > q_pos) p0 = 0.f;
-              if (key0 + c0 + hf * 32 + i + 1 > q_pos) p1 = 0.f;
-              l_tile += p0 + p1;
-              const __half2 hp = __floats2half2_rn(p0, p1);
-              packed[hf * 16 + i / 2] = *reinterpret_cast<const uint32_t*>(&hp);
-            }
-          }
-        }
-        tmem_st_32x32(tmem_sj + c0 / 2, packed);
       }
       tc_wait_st();
       l_run = l_run * corr + l_tile;
       m_run = m_new;
       tc_fence_before();
-      mbar_arrive(&p_ready[sb]);
+      __syncwarp();
+      if (lane == 0) mbar_arrive(&p_ready[sb]);
     }
     if (ok && steps > 0) {
       ok = mbar_wait(&o_done[q], (steps - 1) & 1, status, STATUS_EPILOGUE_WAIT, 0x300);
       ok = __all_sync(0xffffffffu, ok);
     }
+    // both halves of the row sum
+    float* sums = row_max + (steps & 1) * 2 * TILE;
+    sums[half * TILE] = l_run;
+    meet();
     if (ok && steps > 0) {
       tc_fence_after();
-      const float inv = l_run > 0.f ? 1.f / l_run : 0.f;
+      const float l_all = sums[0] + sums[TILE];
+      const float inv = l_all > 0.f ? 1.f / l_all : 0.f;
       const size_t orow = static_cast<size_t>(ch.row_start + first + p_rel) * qh + head;
 #pragma unroll 1
-      for (int c0 = 0; c0 < D; c0 += 32) {
+      for (int c0 = 0; c0 < DH; c0 += 32) {
         uint32_t r[32];
         tmem_ld_32x32(tmem_oq + c0, r);
         tc_wait_ld();
         if (valid) {
+          const size_t at = orow * D + half * DH + c0;
           __align__(16) __half hv[32];
 #pragma unroll
           for (int i = 0; i < 32; ++i) {
             float v = __uint_as_float(r[i]) * inv;
             if (gate) {
-              const float gv = __half2float(gate[orow * D + c0 + i]);
+              const float gv = __half2float(gate[at + i]);
               v *= __fdiv_rn(1.f, 1.f + expf(-gv));
             }
             hv[i] = __float2half_rn(v);
           }
-          uint4* o = reinterpret_cast<uint4*>(out + orow * D + c0);
+          uint4* o = reinterpret_cast<uint4*>(out + at);
 #pragma unroll
           for (int i = 0; i < 4; ++i) o[i] = reinterpret_cast<const uint4*>(hv)[i];
         }
