@@ -23,15 +23,16 @@
 // CTAs are ordered from the last query positions (the longest walks) to the first.
 //
 // A step of two tiles is a chain per tile (softmax, P V, Q K^T of the next step) and two of them
-// hide each other only in part: with one thread per row 5500 cycles for 128 keys, of which softmax
-// 3700, with two threads 5000 and 2700.  The tensor core needs 3000 of them, the exponentials 2050.
+// hide each other only in part: 5500 cycles for 128 keys with one softmax thread per row and the
+// MMAs issued inside a branch on the lane, 5000 with two threads, about 4400 since the whole warp
+// runs the issuing loop.  The tensor core needs 2050 of them, the exponentials as many.
 // One 4096-token chunk, 32 / 8 heads of 128: 377 us with one tile per CTA and P in shared memory,
-// 244 with two tiles and P in TMEM, 213 with two threads per row (645 TFLOP/s causal); 512 tokens
-// 18.3 -> 15.3 us with the last change, 17 tokens 10.8 -> 8.5.  A reference that follows the
+// 244 with two tiles and P in TMEM, 213 with two threads per row, 194 now (709 TFLOP/s causal);
+// 512 tokens 18.3 -> 15.3 -> 13.8 us, 17 tokens 10.8 -> 8.5 -> 7.7.  A reference that follows the
 // maximum only when it lags by 2^8 saves another tenth (fewer rescales of O) but rounds the largest
 // weights in FP16: the error against 64 bits grows by 1.8 % there and by 3.7 % for 500 rows behind
 // 1000.  Chunks of 777 and 646 rows behind 3000 positions, 16 / 2 gated heads of 256: 354 -> 284 ->
-// 276 us (180 CTAs: 1.2 waves).
+// 244 with K and V freed apart, 227 now (180 CTAs: 1.2 waves).
 // Output is O / sum, optionally times sigmoid(gate), in FP16.  Replaces the prefill
 // configurations of causal_attention_int8 and dequantize_attention_kv
 // (kernels/cuda/model/attention_rows.py:61-276, kernels/cuda/model/kv_int8.py:210-247).
@@ -63,14 +64,27 @@ struct Smem {
   static_assert(TOTAL <= 227 * 1024, "exceeds the shared memory of one CTA");
 };
 
-// D[tmem] (+)= A[tmem] * B[smem]: A holds two FP16 values of a row per 32-bit column.
-__device__ __forceinline__ void mma_f16_ts(uint32_t tmem_d, uint32_t tmem_a, uint64_t bdesc,
-                                           uint32_t idesc, uint32_t accumulate) {
+__device__ __forceinline__ void mma_f16_ss_by(uint32_t leader, uint32_t tmem_d, uint64_t adesc,
+                                              uint64_t bdesc, uint32_t idesc,
+                                              uint32_t accumulate) {
   asm volatile(
-      "{\n\t.reg .pred p;\n\t"
+      "{\n\t.reg .pred p, q;\n\t"
       "setp.ne.b32 p, %4, 0;\n\t"
-      "tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], %2, %3, p;\n\t}" ::"r"(tmem_d),
-      "r"(tmem_a), "l"(bdesc), "r"(idesc), "r"(accumulate)
+      "setp.ne.b32 q, %5, 0;\n\t"
+      "@q tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n\t}" ::"r"(tmem_d),
+      "l"(adesc), "l"(bdesc), "r"(idesc), "r"(accumulate), "r"(leader)
+      : "memory");
+}
+// D[tmem] (+)= A[tmem] * B[smem]: A holds two FP16 values of a row per 32-bit column.
+__device__ __forceinline__ void mma_f16_ts_by(uint32_t leader, uint32_t tmem_d, uint32_t tmem_a,
+                                              uint64_t bdesc, uint32_t idesc,
+                                              uint32_t accumulate) {
+  asm volatile(
+      "{\n\t.reg .pred p, q;\n\t"
+      "setp.ne.b32 p, %4, 0;\n\t"
+      "setp.ne.b32 q, %5, 0;\n\t"
+      "@q tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], %2, %3, p;\n\t}" ::"r"(tmem_d),
+      "r"(tmem_a), "l"(bdesc), "r"(idesc), "r"(accumulate), "r"(leader)
       : "memory");
 }
 
@@ -144,7 +158,7 @@ __global__ void __launch_bounds__(Smem<D, NQ>::THREADS, 1) attn_prefill_kernel(
   uint64_t* v_free = bars + 13;       // [2] the same for V
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 15);
 
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int warp = warp_same(threadIdx.x >> 5), lane = threadIdx.x & 31;
   const Chunk ch = chunks[blockIdx.z];
   const int h = blockIdx.y;                       // kv head
   const int P = TILE / rep;                       // query positions per tile
@@ -185,7 +199,7 @@ __global__ void __launch_bounds__(Smem<D, NQ>::THREADS, 1) attn_prefill_kernel(
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
-  const uint32_t tmem_base = *tmem_slot;
+  const uint32_t tmem_base = warp_same(*tmem_slot);
   const uint32_t tmem_s = tmem_base, tmem_o = tmem_base + 256;   // O of tile q at + q * 128
   const int* pages = page_table + static_cast<size_t>(ch.slot) * max_pages;
 
@@ -199,70 +213,73 @@ __global__ void __launch_bounds__(Smem<D, NQ>::THREADS, 1) attn_prefill_kernel(
       mbar_wait(q_full, 0, status, STATUS_TMA_WAIT, 1);     // our copies have landed before exit
     }
   } else if (warp == 1) {
-    if (lane == 0) {
-      constexpr uint32_t idesc_s = umma_idesc(1, 0, 0, 0, 0, TILE, KT);
-      constexpr uint32_t idesc_o = umma_idesc(1, 0, 0, 0, 1, TILE, D);
-      const uint32_t q_addr = smem_u32(smem + L::Q_OFF);
-      bool ok = mbar_wait(q_full, 0, status, STATUS_MMA_WAIT, 2);
-      auto wait_for = [&](uint64_t* ready, int j) {
-        ok = ok && mbar_wait(&ready[j & 1], (j >> 1) & 1, status, STATUS_MMA_WAIT,
-                             0x100 | (j & 0xff));
-        tc_fence_after();
-      };
-      auto issue_qk = [&](int q, int j) {
-        const int sb = NQ == 2 ? q : j & 1;
-        const uint32_t k_addr = smem_u32(smem + L::K_OFF + (j & 1) * NSUB * L::KSUB);
+    // the whole warp runs the loop (see elect_one)
+    constexpr uint32_t idesc_s = umma_idesc(1, 0, 0, 0, 0, TILE, KT);
+    constexpr uint32_t idesc_o = umma_idesc(1, 0, 0, 0, 1, TILE, D);
+    const uint32_t leader = elect_one();
+    const uint64_t qd = umma_desc(smem_u32(smem + L::Q_OFF), 16, 1024);
+    const uint64_t kd = umma_desc(smem_u32(smem + L::K_OFF), 16, 1024);
+    const uint64_t vd = umma_desc(smem_u32(smem + L::V_OFF), L::KSUB, 1024);
+    int steps[NQ];
 #pragma unroll
-        for (int i = 0; i < D / 16; ++i)
-          mma_f16_ss(tmem_s + S_STRIDE * sb,
-                     umma_desc(q_addr + (q * NSUB + i / 4) * L::SUB + (i % 4) * 32, 16, 1024),
-                     umma_desc(k_addr + (i / 4) * L::KSUB + (i % 4) * 32, 16, 1024), idesc_s,
-                     i != 0 ? 1u : 0u);
-        tc_commit(&s_full[sb]);
-      };
-      auto issue_pv = [&](int q, int j) {
-        const int sb = NQ == 2 ? q : j & 1;
-        const uint32_t parity = (NQ == 2 ? j : j >> 1) & 1;
-        ok = ok && mbar_wait(&p_ready[sb], parity, status, STATUS_MMA_WAIT, 0x200 | (j & 0xff));
-        if (!ok) return;
-        tc_fence_after();
-        const uint32_t v_addr = smem_u32(smem + L::V_OFF + (j & 1) * NSUB * L::KSUB);
+    for (int q = 0; q < NQ; ++q) steps[q] = warp_same(n_steps[q]);
+    const int last = warp_same(n_max);
+    bool ok = __all_sync(0xffffffffu, mbar_wait(q_full, 0, status, STATUS_MMA_WAIT, 2));
+    auto wait_for = [&](uint64_t* bar, uint32_t parity, int detail) {
+      if (ok) ok = __all_sync(0xffffffffu, mbar_wait(bar, parity, status, STATUS_MMA_WAIT, detail));
+      tc_fence_after();
+    };
+    auto issue_qk = [&](int q, int j) {
+      const int sb = NQ == 2 ? q : j & 1;
+      const uint64_t kb = kd + static_cast<uint64_t>((j & 1) * NSUB * L::KSUB / 16);
 #pragma unroll
-        for (int i = 0; i < KT / 16; ++i)
-          mma_f16_ts(tmem_o + 128 * q,
-                     tmem_s + S_STRIDE * sb + i / (KT / 32) * (KT / 2) + i % (KT / 32) * 8,
-                     umma_desc(v_addr + i * 2048, L::KSUB, 1024), idesc_o, (j | i) != 0 ? 1u : 0u);
-        tc_commit(&o_done[q]);
-      };
-      // MMAs of one thread run in order.  NQ = 2: QK of step j + 1 overwrites the P of step j of
-      // the same tile, so it follows that tile's PV; meanwhile the other tile's softmax runs.
-      // NQ = 1: QK of step j + 1 goes into the other S buffer, ahead of PV of step j.
-      auto next_qk = [&](int q, int j) {              // tile q's part of QK of step j
-        if (q == 0) wait_for(k_ready, j);
-        if (ok && j < n_steps[q]) issue_qk(q, j);
-        if (ok && q == NQ - 1) tc_commit(&k_free[j & 1]);
-      };
+      for (int i = 0; i < D / 16; ++i)
+        mma_f16_ss_by(leader, tmem_s + S_STRIDE * sb,
+                      qd + ((q * NSUB + i / 4) * L::SUB + i % 4 * 32) / 16,
+                      kb + (i / 4 * L::KSUB + i % 4 * 32) / 16, idesc_s, i != 0 ? 1u : 0u);
+      tc_commit_by(leader, &s_full[sb]);
+    };
+    auto issue_pv = [&](int q, int j) {
+      const int sb = NQ == 2 ? q : j & 1;
+      wait_for(&p_ready[sb], (NQ == 2 ? j : j >> 1) & 1, 0x200 | (j & 0xff));
+      if (!ok) return;
+      const uint64_t vb = vd + static_cast<uint64_t>((j & 1) * NSUB * L::KSUB / 16);
 #pragma unroll
-      for (int q = 0; q < NQ; ++q) next_qk(q, 0);
-      for (int j = 0; j < n_max && ok; ++j) {
-        const bool more = j + 1 < n_max;
-        if (NQ == 1 && more) next_qk(0, j + 1);
-        wait_for(v_ready, j);
+      for (int i = 0; i < KT / 16; ++i)
+        mma_f16_ts_by(leader, tmem_o + 128 * q,
+                      tmem_s + S_STRIDE * sb + i / (KT / 32) * (KT / 2) + i % (KT / 32) * 8,
+                      vb + i * 2048 / 16, idesc_o, (j | i) != 0 ? 1u : 0u);
+      tc_commit_by(leader, &o_done[q]);
+    };
+    // MMAs of one thread run in order.  NQ = 2: QK of step j + 1 overwrites the P of step j of
+    // the same tile, so it follows that tile's PV; meanwhile the other tile's softmax runs.
+    // NQ = 1: QK of step j + 1 goes into the other S buffer, ahead of PV of step j.
+    auto next_qk = [&](int q, int j) {                // tile q's part of QK of step j
+      if (q == 0) wait_for(&k_ready[j & 1], (j >> 1) & 1, 0x100 | (j & 0xff));
+      if (ok && j < steps[q]) issue_qk(q, j);
+      if (ok && q == NQ - 1) tc_commit_by(leader, &k_free[j & 1]);
+    };
 #pragma unroll
-        for (int q = 0; q < NQ; ++q) {
-          if (ok && j < n_steps[q]) issue_pv(q, j);
-          if (q == NQ - 1 && ok) tc_commit(&v_free[j & 1]);
-          if (NQ == 2 && ok && more) next_qk(q, j + 1);
-        }
+    for (int q = 0; q < NQ; ++q) next_qk(q, 0);
+    for (int j = 0; j < last && ok; ++j) {
+      const bool more = j + 1 < last;
+      if (NQ == 1 && more) next_qk(0, j + 1);
+      wait_for(&v_ready[j & 1], (j >> 1) & 1, 0x180 | (j & 0x7f));
+#pragma unroll
+      for (int q = 0; q < NQ; ++q) {
+        if (ok && j < steps[q]) issue_pv(q, j);
+        if (q == NQ - 1 && ok) tc_commit_by(leader, &v_free[j & 1]);
+        if (NQ == 2 && ok && more) next_qk(q, j + 1);
       }
     }
+    __syncwarp();
   } else if (warp >= 2 + 8 * NQ) {
     // ---------------- dequant warps: INT8 page -> FP16 swizzled K / V tiles
     // The raw rows of step j + 1 are in flight while step j is multiplied.  K and V have two buffers
     // each, freed apart.  With one tile K of step j + 1 is converted while PV of step j - 1 still
     // reads V, so that the next Q K^T does not wait for it (777 and 646 rows behind 3000, 16 / 2
-    // heads of 256: 276 -> 247 us; 512 rows, 32 / 8 heads of 128: 15.3 -> 14.8).  With two tiles
-    // that wait is hidden, and the conversions do better in one piece (4096 rows 213 us, 218 apart).
+    // heads of 256: 276 -> 244 us; 512 rows, 32 / 8 heads of 128: 15.3 -> 14.6).  With two tiles
+    // that wait is hidden, and the conversions do better in one piece (4096 rows 216 us, 219 apart).
     constexpr int CPK = D / 16;                      // 16-byte chunks per key
     constexpr int DQ = DQ_WARPS * 32, ITERS = KT * CPK / DQ;
     uint4 kraw[ITERS], vraw[ITERS];

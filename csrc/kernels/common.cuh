@@ -195,13 +195,39 @@ __device__ __forceinline__ void mma_i8_ss(uint32_t tmem_d, uint64_t adesc, uint6
       "l"(adesc), "l"(bdesc), "r"(idesc), "r"(accumulate)
       : "memory");
 }
-__device__ __forceinline__ void mma_f16_ss(uint32_t tmem_d, uint64_t adesc, uint64_t bdesc,
-                                           uint32_t idesc, uint32_t accumulate) {
+
+// The same for a warp that runs its loop as a whole, `leader` being elect_one's answer: the operands
+// of an MMA live in uniform registers, and under a branch on the lane the compiler has to move each
+// of them there (a warp that waited, multiplied and signalled inside `if (lane == 0)` took 1450
+// cycles for eight 128 x 128 x 32 MMAs whose operands were there).
+__device__ __forceinline__ uint32_t elect_one() {
+  uint32_t r;
   asm volatile(
       "{\n\t.reg .pred p;\n\t"
+      "elect.sync _|p, 0xffffffff;\n\t"
+      "selp.u32 %0, 1, 0, p;\n\t}"
+      : "=r"(r));
+  return r;
+}
+// `x` of lane 0, which the compiler then knows to be the same in every lane
+__device__ __forceinline__ int warp_same(int x) { return __shfl_sync(0xffffffffu, x, 0); }
+__device__ __forceinline__ void mma_i8_ss_by(uint32_t leader, uint32_t tmem_d, uint64_t adesc,
+                                             uint64_t bdesc, uint32_t idesc, uint32_t accumulate) {
+  asm volatile(
+      "{\n\t.reg .pred p, q;\n\t"
       "setp.ne.b32 p, %4, 0;\n\t"
-      "tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n\t}" ::"r"(tmem_d),
-      "l"(adesc), "l"(bdesc), "r"(idesc), "r"(accumulate)
+      "setp.ne.b32 q, %5, 0;\n\t"
+      "@q tcgen05.mma.cta_group::1.kind::i8 [%0], %1, %2, %3, p;\n\t}" ::"r"(tmem_d),
+      "l"(adesc), "l"(bdesc), "r"(idesc), "r"(accumulate), "r"(leader)
+      : "memory");
+}
+__device__ __forceinline__ void tc_commit_by(uint32_t leader, uint64_t* bar) {
+  asm volatile(
+      "{\n\t.reg .pred q;\n\t"
+      "setp.ne.b32 q, %1, 0;\n\t"
+      "@q tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];\n\t}" ::"r"(
+          smem_u32(bar)),
+      "r"(leader)
       : "memory");
 }
 
