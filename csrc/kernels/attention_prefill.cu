@@ -275,11 +275,12 @@ __global__ void __launch_bounds__(Smem<D, NQ>::THREADS, 1) attn_prefill_kernel(
     __syncwarp();
   } else if (warp >= 2 + 8 * NQ) {
     // ---------------- dequant warps: INT8 page -> FP16 swizzled K / V tiles
-    // The raw rows of step j + 1 are in flight while step j is multiplied.  K and V have two buffers
-    // each, freed apart.  With one tile K of step j + 1 is converted while PV of step j - 1 still
-    // reads V, so that the next Q K^T does not wait for it (777 and 646 rows behind 3000, 16 / 2
-    // heads of 256: 276 -> 244 us; 512 rows, 32 / 8 heads of 128: 15.3 -> 14.6).  With two tiles
-    // that wait is hidden, and the conversions do better in one piece (4096 rows 216 us, 219 apart).
+    // The raw rows of step j + 1 are in flight while step j is multiplied.  K and V have two
+    // buffers each, freed apart.  With one tile K of step j + 1 is converted while PV of step j - 1
+    // still reads V, so that the next Q K^T does not wait for it (777 and 646 rows behind 3000, 16
+    // / 2 heads of 256: 276 -> 244 us; 512 rows, 32 / 8 heads of 128: 15.3 -> 14.6).  With two
+    // tiles that wait is hidden, and the conversions do better in one piece (4096 rows 216 us, 219
+    // apart).
     constexpr int CPK = D / 16;                      // 16-byte chunks per key
     constexpr int DQ = DQ_WARPS * 32, ITERS = KT * CPK / DQ;
     uint4 kraw[ITERS], vraw[ITERS];

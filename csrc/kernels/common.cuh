@@ -196,10 +196,10 @@ __device__ __forceinline__ void mma_i8_ss(uint32_t tmem_d, uint64_t adesc, uint6
       : "memory");
 }
 
-// The same for a warp that runs its loop as a whole, `leader` being elect_one's answer: the operands
-// of an MMA live in uniform registers, and under a branch on the lane the compiler has to move each
-// of them there (a warp that waited, multiplied and signalled inside `if (lane == 0)` took 1450
-// cycles for eight 128 x 128 x 32 MMAs whose operands were there).
+// The same for a warp that runs its loop as a whole, `leader` being elect_one's answer: the
+// operands of an MMA live in uniform registers, and under a branch on the lane the compiler has to
+// move each of them there (a warp that waited, multiplied and signalled inside `if (lane == 0)`
+// took 1450 cycles for eight 128 x 128 x 32 MMAs whose operands were there).
 __device__ __forceinline__ uint32_t elect_one() {
   uint32_t r;
   asm volatile(

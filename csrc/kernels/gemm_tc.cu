@@ -19,6 +19,7 @@
 
 #include "api.h"
 #include "common.cuh"
+#include "gemm_walk.h"
 #include "tma.h"
 #include "tp_comm.cuh"
 
@@ -39,8 +40,9 @@ constexpr int TILE_BYTES = 128 * 128;        // one INT8 activation tile (128 ro
 constexpr int PRODUCERS = 512;               // warps 3..18
 constexpr int PWARPS = PRODUCERS / 32;
 constexpr int NUM_SMS = 148;
-// 0: persistent kernel; 1: one tile per CTA (default: the fastest measured so far); 2: CTA
-// pairs (cta_group::2) where the shape allows, else persistent.  All give the same bits.
+// 0: persistent kernel; 1 (default): one tile per CTA, or the walking kernel (gemm_walk.cu) where
+// there are many; 2: CTA pairs (cta_group::2) where the shape allows, else persistent.  All give
+// the same bits.
 static int g_impl = 1;
 static int g_probe = 0;      // timing experiments of the one-tile kernel (see its `probe`)
 // warp 0: activation loader, warp 1: MMA issuer, warp 2: weight loader, warps 3..18: lattice
@@ -132,7 +134,7 @@ __global__ void __launch_bounds__(THREADS, 1) qgemm_tc_kernel(
   int* ticket_slot = reinterpret_cast<int*>(tmem_slot + 1);
   bool writes_output = true;                   // false: another split finishes this tile
 
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int warp = warp_same(threadIdx.x >> 5), lane = threadIdx.x & 31;
   const int n0 = n_begin + blockIdx.x * BN;    // this launch covers columns [n_begin, n_end)
   int m0 = blockIdx.y * BM * MT, m_limit = M, b_row0 = n0, mt_act = MT;
   if (grp.tiles != nullptr) {
@@ -170,7 +172,7 @@ __global__ void __launch_bounds__(THREADS, 1) qgemm_tc_kernel(
     }
     for (int s = 0; s < SB; ++s) {
       mbar_init(&c_full[s], 1);
-      mbar_init(&b_full[s], FMT == 0 ? 1 : PRODUCERS);
+      mbar_init(&b_full[s], FMT == 0 ? 1 : PWARPS);
       mbar_init(&b_empty[s], 1);
     }
     mbar_init(tmem_full, 1);
@@ -188,7 +190,7 @@ __global__ void __launch_bounds__(THREADS, 1) qgemm_tc_kernel(
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
-  const uint32_t tmem_base = *tmem_slot;
+  const uint32_t tmem_base = warp_same(*tmem_slot);
   // peer epilogue staging: one padded FP16 row per output row (pad keeps 16-byte stores of
   // 32 consecutive rows on distinct banks)
   constexpr int STAGE_ROW = BN * 2 + 16;
@@ -251,35 +253,48 @@ __global__ void __launch_bounds__(THREADS, 1) qgemm_tc_kernel(
         mbar_wait(&landed[kb % SB], (kb / SB) & 1, status, STATUS_TMA_WAIT, 0x5000 | kb);
     }
   } else if (warp == 1) {
-    if (lane == 0) {
-      constexpr uint32_t idesc = umma_idesc(2, 1, 1, 0, 0, BM, BN);
-      bool ok = true;
-      for (int kb = 0; kb < kblocks && ok; ++kb) {
-        const int sa = kb % SA, sb = kb % SB;
-        ok = mbar_wait(&a_full[sa], (kb / SA) & 1, status, STATUS_MMA_WAIT, kb);
-        if (ok) ok = mbar_wait(&b_full[sb], (kb / SB) & 1, status, STATUS_MMA_WAIT, 0x2000 | kb);
-        if (!ok) break;
-        tc_fence_after();
-        const uint32_t b_addr = smem_u32(b_s + sb * L::B_BYTES);
+    // the whole warp runs the loop (see elect_one)
+    constexpr uint32_t idesc = umma_idesc(2, 1, 1, 0, 0, BM, BN);
+    const uint32_t leader = elect_one();
+    const uint64_t a_ring = umma_desc(smem_u32(a_s), 16, 1024);
+    const uint64_t b_ring = umma_desc(smem_u32(b_s), 16, 1024);
+    const int blocks = warp_same(kblocks), tiles = warp_same(mt_act);
+    int sa = 0, sb = 0;
+    uint32_t pa = 0, pb = 0;                              // phases of the two rings
+    bool ok = true;
+    for (int kb = 0; kb < blocks && ok; ++kb) {
+      ok = mbar_wait(&b_full[sb], pb, status, STATUS_MMA_WAIT, 0x2000 | kb) &&
+           mbar_wait(&a_full[sa], pa, status, STATUS_MMA_WAIT, kb);
+      ok = __all_sync(0xffffffffu, ok);
+      if (!ok) break;
+      tc_fence_after();
+      const uint64_t ad = a_ring + static_cast<uint64_t>(sa * MT * TILE_BYTES / 16);
+      const uint64_t bd = b_ring + static_cast<uint64_t>(sb * L::B_BYTES / 16);
 #pragma unroll
-        for (int j = 0; j < BK / 32; ++j) {
-          if (probe & 1) break;
-          const uint64_t bdesc = umma_desc(b_addr + j * 32, 16, 1024);
+      for (int j = 0; j < BK / 32; ++j) {
+        if (probe & 1) break;
 #pragma unroll
-          for (int t = 0; t < MT; ++t) {
-            const uint32_t a_addr = smem_u32(a_s + (sa * MT + t) * TILE_BYTES);
-            // An expert's last row tiles are often not loaded, and nobody reads them.  The one
-            // cut packet of the other calls is not worth the test (2 % at 1024 x 2560 x 4096).
-            if (!GROUPED || t == 0 || t < mt_act)
-              mma_i8_ss(tmem_base + t * BN, umma_desc(a_addr + j * 32, 16, 1024), bdesc, idesc,
-                        (kb | j) != 0 ? 1u : 0u);
-          }
+        for (int t = 0; t < MT; ++t) {
+          // An expert's last row tiles are often not loaded, and nobody reads them.  The one
+          // cut packet of the other calls is not worth the test (2 % at 1024 x 2560 x 4096).
+          if (!GROUPED || t == 0 || t < tiles)
+            mma_i8_ss_by(leader, tmem_base + t * BN, ad + (t * TILE_BYTES + j * 32) / 16,
+                         bd + j * 32 / 16, idesc, (kb | j) != 0 ? 1u : 0u);
         }
-        tc_commit(&a_empty[sa]);
-        tc_commit(&b_empty[sb]);
       }
-      if (ok && kblocks > 0) tc_commit(tmem_full);
+      tc_commit_by(leader, &a_empty[sa]);
+      tc_commit_by(leader, &b_empty[sb]);
+      if (++sa == SA) {
+        sa = 0;
+        pa ^= 1;
+      }
+      if (++sb == SB) {
+        sb = 0;
+        pb ^= 1;
+      }
     }
+    if (ok && blocks > 0) tc_commit_by(leader, tmem_full);
+    __syncwarp();
   } else {
     const int t = threadIdx.x - ROLE_THREADS;                     // 0..511
     bool ok = true;
@@ -315,7 +330,8 @@ __global__ void __launch_bounds__(THREADS, 1) qgemm_tc_kernel(
           *reinterpret_cast<uint4*>(bs + swz128(row, chunk)) = v;
         }
         fence_proxy_async();
-        mbar_arrive(&b_full[s]);
+        __syncwarp();
+        if (lane == 0) mbar_arrive(&b_full[s]);
       }
     }
     const int quad = warp & 3;                          // TMEM lane quadrant of this warp
@@ -1717,6 +1733,16 @@ inline Plan make_plan(int fmt, int M, int N, int K, int out_f32, bool fused) {
   return p;
 }
 
+// Whether an (MT * 128) x 128 tiling of M rows and n columns goes to the kernel that walks many
+// tiles per CTA: from a second wave of tiles on.  Its tiles have two row tiles at most, so lattice
+// codes that serve four stay here: 2048 x 19456 x 2560 Q4 118 us against 139, 1024 rows 67 against
+// 79, 600 rows 64 against 62; 200 x 40000 x 1024 31 against 27; INT8 2048 x 19456 x 2560 117
+// against 86.
+inline bool walks(int fmt, int mt, int M, int n) {
+  const long tiles = static_cast<long>((M + BM * mt - 1) / (BM * mt)) * ((n + 127) / 128);
+  return g_impl == 1 && g_probe == 0 && tiles > NUM_SMS && (fmt == 0 || mt <= 2);
+}
+
 template <int FMT>
 int launch_fmt(const int8_t* a, const float* a_scale, const void* w, const __half* w_scale,
                void* out, int M, int N, int K, int out_f32, cudaStream_t stream,
@@ -1729,6 +1755,10 @@ int launch_fmt(const int8_t* a, const float* a_scale, const void* w, const __hal
   }
   const Plan plan = make_plan(FMT, M, N, K, out_f32, po.tp != 0);
   const int mt = plan.mt, nb = plan.nb, splits = plan.splits;
+  auto walk_call = [&](int n_end) {
+    return WalkCall{a, a_scale, w, w_scale, static_cast<__half*>(out), M, N, K, n_end, nullptr,
+                    nullptr, 0, 1, 0};
+  };
   if (plan.tail_splits > 0) {
     const long ntiles = (N + 127) / 128;
     const int cut = static_cast<int>(ntiles - plan.tail_tiles) * 128;
@@ -1737,8 +1767,11 @@ int launch_fmt(const int8_t* a, const float* a_scale, const void* w, const __hal
     const int ts = plan.tail_splits;
 #define ORINFER_TWO(MTV)                                                                        \
   {                                                                                             \
-    const int r = launch<FMT, false, MTV, 128>(a, a_scale, w, w_scale, out, M, N, K, stream, po, \
-                                               none, 1, 0, ag, 1, 0, cut);                     \
+    const int r =                                                                               \
+        walks(FMT, MTV, M, cut) && ag.tp == 0                                                   \
+            ? qgemm_walk_dispatch(FMT, MTV > 1 ? 2 : 1, walk_call(cut), stream)                 \
+            : launch<FMT, false, MTV, 128>(a, a_scale, w, w_scale, out, M, N, K, stream, po,    \
+                                           none, 1, 0, ag, 1, 0, cut);                          \
     if (r) return r;                                                                            \
     return launch<FMT, false, 1, 128>(a, a_scale, w, w_scale, out, M, N, K, stream, po, none,  \
                                       1, 0, ag, ts, cut, N);                                   \
@@ -1748,6 +1781,8 @@ int launch_fmt(const int8_t* a, const float* a_scale, const void* w, const __hal
     ORINFER_TWO(1)
 #undef ORINFER_TWO
   }
+  if (!out_f32 && nb == 128 && splits == 1 && po.tp == 0 && ag.tp == 0 && walks(FMT, mt, M, N))
+    return qgemm_walk_dispatch(FMT, mt > 1 ? 2 : 1, walk_call(N), stream);
 #define ORINFER_GO(F32, MTV, NBV)                                                              \
   return launch<FMT, F32, MTV, NBV>(a, a_scale, w, w_scale, out, M, N, K, stream, po, none, 1, \
                                     0, ag, splits)
@@ -1846,7 +1881,8 @@ extern "C" void orinfer_qgemm_clear_variants() {
   tc::g_variant_count = 0;
 }
 
-// 0 = persistent kernel, 1 = one tile per CTA (default), 2 = CTA pairs; for comparisons and tests.
+// 0 = persistent kernel, 1 = one tile per CTA or many tiles walked (default), 2 = CTA pairs; for
+// comparisons and tests.
 // Timing experiments of the one-tile kernel: bit 0 no MMAs, bit 1 no operand copies, bit 2
 // no lattice decode.  Outputs are meaningless while a bit is set.
 extern "C" int orinfer_qgemm_set_probe(int bits) {
@@ -1980,6 +2016,15 @@ static int qgemm_grouped_fmt(const int8_t* a, const float* a_scale, const void* 
   const long long two = (FMT == 0 ? 112LL : 64LL) * experts;
   const long long four = 256LL * experts;
   const int mt = tc::g_impl != 1 ? 1 : (expected >= four ? 4 : (expected >= two ? 2 : 1));
+  // More tiles than SMs: the walking kernel (128 Q4 experts of 768, both projections and all: 2048
+  // rows 447 -> 340 us, 300 rows 300 -> 213; INT8 390 -> 281).  Codes that serve four row tiles
+  // stay with the one-tile kernel, as in `walks`.
+  if (tc::g_impl == 1 && tc::g_probe == 0 && max_tiles <= walk_list_room(FMT) &&
+      (FMT == 0 || mt <= 2))
+    return qgemm_walk_dispatch(FMT, mt > 1 ? 2 : 1,
+                               WalkCall{a, a_scale, w, w_scale, static_cast<__half*>(out), S, N, K,
+                                        N, tiles, meta, bank, experts, max_tiles},
+                               stream);
   if (mt == 4)
     return tc::launch<FMT, false, 4, 128>(a, a_scale, w, w_scale, out, S, N, K, stream, po, g,
                                           experts, max_tiles);

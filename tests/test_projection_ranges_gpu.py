@@ -88,6 +88,25 @@ def test_peeled_tail_tiles_are_exact(dev, fmt, m, n):
         assert torch.equal(out, want if f32 else want.half())
 
 
+@pytest.mark.parametrize("fmt", ["w8", "q4", "q2"])
+@pytest.mark.parametrize("m,n,k", [(9, 25600, 128), (128, 25560, 384), (129, 25560, 1152),
+                                   (255, 40000, 640), (256, 25608, 2560), (385, 25560, 384),
+                                   (1030, 12200, 768)])
+def test_walked_tiles_are_exact(dev, fmt, m, n, k):
+    """More tiles than SMs: one row tile and two, the last of them cut, columns cut inside an
+    eight-row piece of a tile, single k-blocks, fewer k-blocks than ring stages; repeated, since its
+    warps run ahead of each other."""
+    from orinfer_b200.ops import functional as F
+    g = torch.Generator().manual_seed(m + n + k)
+    codes, ws, w = _int_weight(fmt, n, k, g)
+    a = torch.randint(-127, 128, (m, k), generator=g, dtype=torch.int8)
+    sa = torch.rand(m, generator=g) * 0.05 + 1e-3
+    want = _scaled(a.to(dev), sa.to(dev), w.to(dev), ws.to(dev)).half()
+    a, sa, codes, ws = a.to(dev), sa.to(dev), codes.to(dev), ws.to(dev)
+    for _ in range(5):
+        assert torch.equal(F.qgemm(a, sa, codes, ws, fmt, n), want)
+
+
 @pytest.mark.parametrize("rows", [1, 7, 149, 300, 2049])
 @pytest.mark.parametrize("k", [128, 384, 768, 2176, 6144, 6272, 9728, 16384])
 @pytest.mark.parametrize("mode", ["norm", "plain", "swiglu", "bare"])
