@@ -34,32 +34,53 @@ __device__ __forceinline__ void topk_row(float* logits, int row, int experts, in
   float sum = 0.f;
   for (int e = lane; e < experts; e += 32) sum += expf(logits[e] - mx);
   sum = warp_sum(sum);
-  float chosen_sum = 0.f;
-  for (int k = 0; k < top_k; ++k) {
-    float best = -INFINITY;
-    int bidx = 0x7fffffff;
+  // Every lane keeps the best of its own logits and looks for another only when that one is taken;
+  // lane k holds the k-th choice (the first 32; later ones go through memory).
+  float best = -INFINITY;
+  int bidx = 0x7fffffff;
+  auto scan = [&]() {
+    best = -INFINITY;
+    bidx = 0x7fffffff;
     for (int e = lane; e < experts; e += 32) {
       const float v = logits[e];
       if (v > best) { best = v; bidx = e; }           // ascending e: first maximum wins
     }
+  };
+  scan();
+  float chosen_sum = 0.f, my_prob = 0.f;
+  int my_id = 0;
+  for (int k = 0; k < top_k; ++k) {
+    float top = best;
+    int at = bidx;
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) {
-      const float ov = __shfl_xor_sync(0xffffffffu, best, o);
-      const int oi = __shfl_xor_sync(0xffffffffu, bidx, o);
-      if (ov > best || (ov == best && oi < bidx)) { best = ov; bidx = oi; }
+      const float ov = __shfl_xor_sync(0xffffffffu, top, o);
+      const int oi = __shfl_xor_sync(0xffffffffu, at, o);
+      if (ov > top || (ov == top && oi < at)) { top = ov; at = oi; }
     }
-    if (bidx >= experts) bidx = k;                  // no comparable logit left (NaN): any valid id
-    const float p = expf(best - mx) / sum;
-    if (lane == 0) {
-      ids[row * top_k + k] = bidx;
-      probs[row * top_k + k] = p;
-      logits[bidx] = -INFINITY;
-    }
+    if (at >= experts) at = k;                      // no comparable logit left (NaN): any valid id
+    const float p = expf(top - mx) / sum;
     chosen_sum += p;
-    __syncwarp();
+    if (k < 32) {
+      if (lane == k) {
+        my_id = at;
+        my_prob = p;
+      }
+    } else if (lane == 0) {
+      ids[row * top_k + k] = at;
+      probs[row * top_k + k] = p;
+    }
+    if ((at & 31) == lane) {
+      logits[at] = -INFINITY;
+      scan();
+    }
+  }
+  if (lane < top_k) {
+    ids[row * top_k + lane] = my_id;
+    probs[row * top_k + lane] = renorm ? my_prob / chosen_sum : my_prob;
   }
   if (renorm && lane == 0)
-    for (int k = 0; k < top_k; ++k) probs[row * top_k + k] /= chosen_sum;
+    for (int k = 32; k < top_k; ++k) probs[row * top_k + k] /= chosen_sum;
   if (has_shared && lane == 0)
     shared_gate[row] = 1.f / (1.f + expf(-logits[experts]));
 }
@@ -197,6 +218,144 @@ static int launch_router(const __half* x, const __half* w, int rows, int hidden,
   const int grid = (rows + 15) / 16 * ROUTER_CL;
   router_mma_kernel<MAXT, WARPS><<<grid, WARPS * 32, smem, stream>>>(
       x, w, rows, hidden, experts, has_shared, top_k, renorm, ids, probs, shared_gate);
+  return static_cast<int>(cudaGetLastError());
+}
+
+// The same product for many rows (at most 136 expert rows, hidden / CL 384 or 512 channels).
+// The form above reads a row eight times and the matrix once per 16 rows, in 64-byte pieces: 128 MB
+// from L2 for 2048 rows.  Here a cluster of CL CTAs takes 64 rows and each of them a CL-th of the
+// channels, copied to shared memory once (192 KB); eight warps hold 32 rows x a quarter of the
+// expert tiles each, and the CTAs add up each other's parts for 64 / CL rows of the top-k.  Sums as
+// above: 16 products in the tensor core, pairs of those added in FP32 in two alternating sums per
+// CTA (probabilities of 128 experts: 1.18e-7 from exact at 2048 channels, 1.50e-7 at 4096; above
+// 1.18e-7 and 1.62e-7). 128 experts x 2048 channels, 2048 rows: 46.4 -> 19.8 us, 1024 rows 27.2 ->
+// 19.5, 512 rows 22.8 -> 19.5; fewer rows are one wave of the form above (384: 10.1 us).  Half of
+// it is the top-k, two rows per warp: with choices kept in memory and renormalised there it took 15
+// us more.
+constexpr int ROUTER_ROWS = 64, ROUTER_TILES = 17, ROUTER_MANY = 512;
+
+__device__ __forceinline__ void ldmatrix4(uint32_t (&r)[4], const void* p) {
+  asm volatile("ldmatrix.sync.aligned.m8n8.x4.shared.b16 {%0, %1, %2, %3}, [%4];"
+               : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3])
+               : "r"(smem_u32(p))
+               : "memory");
+}
+
+template <int CL>
+__global__ void __cluster_dims__(CL, 1, 1) __launch_bounds__(256, 1) router_rows_kernel(
+    const __half* __restrict__ x, const __half* __restrict__ w, int rows, int hidden, int experts,
+    int has_shared, int top_k, int renorm, int* __restrict__ ids, float* __restrict__ probs,
+    float* __restrict__ shared_gate) {
+  constexpr int ROWS = ROUTER_ROWS, OWN = ROWS / CL, PER = (ROUTER_TILES + 3) / 4;
+  extern __shared__ __align__(16) unsigned char router_raw[];
+  const int total = experts + (has_shared ? 1 : 0), tiles = (total + 7) / 8;
+  const int span = hidden / CL, pitch = span + 8;           // halves; rows 16 bytes apart in banks
+  __half* xs = reinterpret_cast<__half*>(router_raw);       // [ROWS][pitch]
+  __half* ws = xs + ROWS * pitch;                           // [8 tiles][pitch]
+  cg::cluster_group cluster = cg::this_cluster();
+  const int crank = static_cast<int>(cluster.block_rank());
+  const int row0 = static_cast<int>(blockIdx.x) / CL * ROWS;
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, g = lane >> 2, t = lane & 3;
+  const int slabs = span / 128;
+  for (int s = 0; s < slabs; ++s) {
+    // rows past the last token or expert are copies of the last one; their sums are not used
+    for (int i = tid; i < (ROWS + tiles * 8) * 16; i += 256) {
+      const int r = i >> 4, c = s * 128 + (i & 15) * 8;
+      const __half* src =
+          r < ROWS ? x + static_cast<size_t>(min(row0 + r, rows - 1)) * hidden
+                   : w + static_cast<size_t>(min(r - ROWS, total - 1)) * hidden;
+      asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(smem_u32(xs + r * pitch + c)),
+                   "l"(src + crank * span + c)
+                   : "memory");
+    }
+    asm volatile("cp.async.commit_group;" ::: "memory");
+  }
+  const int m0 = (warp & 1) * 32, first = warp >> 1;        // expert tiles first, first + 4, ...
+  float acc[2][2][PER][4] = {};                             // [alternating sum][16 rows][tile]
+  for (int s = 0; s < slabs; ++s) {
+    // the copies of slab s have landed when at most slabs - 1 - s groups are under way
+    if (s + 1 >= slabs) asm volatile("cp.async.wait_group 0;" ::: "memory");
+    else if (s + 2 >= slabs) asm volatile("cp.async.wait_group 1;" ::: "memory");
+    else if (s + 3 >= slabs) asm volatile("cp.async.wait_group 2;" ::: "memory");
+    else asm volatile("cp.async.wait_group 3;" ::: "memory");
+    __syncthreads();
+#pragma unroll
+    for (int kk = 0; kk < 4; ++kk) {
+      const int k = s * 128 + kk * 32;
+      uint32_t a[2][2][4];                                  // [16 rows][16 channels]
+#pragma unroll
+      for (int m = 0; m < 2; ++m)
+#pragma unroll
+        for (int h = 0; h < 2; ++h)
+          ldmatrix4(a[m][h], xs + (m0 + m * 16 + (lane & 15)) * pitch + k + h * 16 + (lane >> 4) * 8);
+#pragma unroll
+      for (int i = 0; i < PER; ++i) {
+        const int tile = first + i * 4;
+        if (tile >= tiles) break;
+        uint32_t b[4];
+        ldmatrix4(b, ws + (tile * 8 + (lane & 7)) * pitch + k + (lane >> 3) * 8);
+#pragma unroll
+        for (int m = 0; m < 2; ++m) {
+          float d[4] = {0.f, 0.f, 0.f, 0.f}, f[4] = {0.f, 0.f, 0.f, 0.f};
+          mma16816(d, a[m][0][0], a[m][0][1], a[m][0][2], a[m][0][3], b[0], b[1]);
+          mma16816(f, a[m][1][0], a[m][1][1], a[m][1][2], a[m][1][3], b[2], b[3]);
+#pragma unroll
+          for (int e = 0; e < 4; ++e) acc[kk & 1][m][i][e] += d[e] + f[e];
+        }
+      }
+    }
+  }
+  __syncthreads();                                          // xs becomes the parts' buffer
+  float* part = reinterpret_cast<float*>(xs);               // [ROWS][cols]
+  const int cols = tiles * 8 + 1;
+#pragma unroll
+  for (int i = 0; i < PER; ++i) {
+    const int tile = first + i * 4;
+    if (tile >= tiles) break;
+#pragma unroll
+    for (int m = 0; m < 2; ++m)
+#pragma unroll
+      for (int e = 0; e < 4; ++e)
+        part[(m0 + m * 16 + g + (e >> 1) * 8) * cols + tile * 8 + 2 * t + (e & 1)] =
+            acc[0][m][i][e] + acc[1][m][i][e];
+  }
+  cluster.sync();
+  float* logits = reinterpret_cast<float*>(ws);             // [OWN][total]
+  for (int i = tid; i < OWN * total; i += 256) {
+    const int r = i / total, e = i - r * total;
+    float v[CL];
+#pragma unroll
+    for (int q = 0; q < CL; ++q)
+      v[q] = cluster.map_shared_rank(part, q)[(crank * OWN + r) * cols + e];
+#pragma unroll
+    for (int n = CL / 2; n > 0; n /= 2)
+#pragma unroll
+      for (int q = 0; q < n; ++q) v[q] += v[q + n];
+    logits[i] = v[0];
+  }
+  cluster.sync();                                           // nobody leaves while it is read
+  for (int r = warp; r < OWN; r += 8) {
+    const int row = row0 + crank * OWN + r;
+    if (row < rows)
+      topk_row(logits + r * total, row, experts, has_shared, top_k, renorm, ids, probs,
+               shared_gate);
+  }
+}
+
+inline size_t router_rows_smem(int hidden, int total, int cl) {
+  return static_cast<size_t>(ROUTER_ROWS + (total + 7) / 8 * 8) * (hidden / cl + 8) * 2;
+}
+
+template <int CL>
+static int launch_router_rows(const __half* x, const __half* w, int rows, int hidden, int experts,
+                              int has_shared, int top_k, int renorm, int* ids, float* probs,
+                              float* shared_gate, cudaStream_t stream) {
+  static const int slot = runtime_new_slot();
+  if (const int e = runtime_allow_smem(slot, router_rows_kernel<CL>, 220 * 1024)) return e;
+  const int grid = (rows + ROUTER_ROWS - 1) / ROUTER_ROWS * CL;
+  router_rows_kernel<CL>
+      <<<grid, 256, router_rows_smem(hidden, experts + (has_shared ? 1 : 0), CL), stream>>>(
+          x, w, rows, hidden, experts, has_shared, top_k, renorm, ids, probs, shared_gate);
   return static_cast<int>(cudaGetLastError());
 }
 
@@ -401,6 +560,12 @@ int orinfer_router_topk(const __half* x, const __half* w, int rows, int hidden, 
   const bool few = (total <= 17 && cells <= 17 * 2048) ||
                    (cells <= 32 * 2048 &&
                     ((rows >= 256 && rows <= 640) || (rows > 1100 && rows < 1900)));
+  const int cl = hidden <= 2048 ? 4 : 8;
+  if (!few && rows >= ROUTER_MANY && hidden % (cl * 128) == 0 && hidden / cl >= 384 &&
+      hidden / cl <= 512 && total <= ROUTER_TILES * 8 && router_rows_smem(hidden, total, cl) <= 220 * 1024 &&
+      runtime_ensure_init() == cudaSuccess)
+    return (cl == 4 ? launch_router_rows<4> : launch_router_rows<8>)(
+        x, w, rows, hidden, experts, has_shared, top_k, renorm, ids, probs, shared_gate, stream);
   if (!few && hidden % 256 == 0 && total <= 8 * 8 * 9 && runtime_ensure_init() == cudaSuccess) {
     // Wide routers read their matrix from few SMs in a decode step: more warps, more loads in
     // flight (16 rows, 512 experts: 26 -> 16 us).

@@ -83,6 +83,36 @@ def test_router_sums_keep_fp32_accuracy(dev, hidden, experts, shared):
     assert float((probs.double() - p).norm() / p.norm()) < limit
 
 
+@pytest.mark.parametrize("rows,hidden,experts,top_k,shared", [
+    (512, 2048, 128, 8, False), (513, 2048, 135, 8, True), (575, 1536, 40, 40, False),
+    (1100, 3072, 97, 6, True), (640, 4096, 129, 1, False), (700, 2048, 33, 33, False),
+    (40, 2048, 64, 35, True)])
+def test_router_rows_form_and_long_choices(dev, rows, hidden, experts, top_k, shared):
+    """The form for many rows at the edges of its row and expert tiles and both spans, and choices
+    past the 32nd."""
+    from orinfer_b200.ops import functional as F
+    g = torch.Generator(device=dev).manual_seed(experts + rows)
+    y = torch.randn(rows, hidden, generator=g, device=dev).half()
+    w = (torch.randn(experts + int(shared), hidden, generator=g, device=dev) * 0.02).half()
+    w[experts - 1] = w[0]                                  # an exact tie: the lower id first
+    logits = y.double() @ w.double().t()
+    p, order = torch.softmax(logits[:, :experts], 1).sort(dim=1, descending=True, stable=True)
+    p, order = p[:, :top_k], order[:, :top_k]
+    for renorm in (True, False):
+        ids, probs, gate = F.router_topk(y, w, experts, top_k, renorm=renorm)
+        want = p / p.sum(1, keepdim=True) if renorm else p
+        # FP32 sums of up to 4096 products, as above
+        assert bool(((probs.double() - want).abs() <= 4e-5 * want + 1e-7).all())
+        picked = torch.gather(logits, 1, ids.long())
+        assert bool(((picked - torch.gather(logits, 1, order)).abs() <= 2e-5).all())
+        assert bool((ids.sort(1).values.diff(dim=1) > 0).all())            # no expert twice
+        first, last = ((ids == e).int().argmax(1) for e in (0, experts - 1))
+        both = (ids == 0).any(1) & (ids == experts - 1).any(1)
+        assert bool((first[both] < last[both]).all())
+        if shared:
+            assert torch.allclose(gate.double(), torch.sigmoid(logits[:, experts]), atol=1e-5)
+
+
 @pytest.mark.parametrize("experts,rows,top_k,k", [(1, 1, 1, 128), (8, 5, 2, 256), (3, 300, 1, 128),
                                                   (128, 2048, 8, 2048), (512, 16, 10, 2048),
                                                   (512, 700, 10, 512)])
