@@ -129,6 +129,8 @@ __global__ void __launch_bounds__(
     float* __restrict__ scratch, int rep, int apart_keys) {
   constexpr int G = AttnTile<D>::G, KB = AttnTile<D>::KB;
   constexpr int NT = KB / 8, UT = KB / 16;         // 8-key score tiles, 16-key value tiles
+  grid_wait();
+  grid_release();
   const int row = blockIdx.x, split = blockIdx.z;
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   const int g = lane >> 2, t = lane & 3;
@@ -426,6 +428,8 @@ template <int D>
 __global__ void attn_merge_kernel(const float* __restrict__ scratch,
                                   const __half* __restrict__ gate, __half* __restrict__ out,
                                   int qh, int splits) {
+  grid_wait();
+  grid_release();
   const int row = blockIdx.x, head = blockIdx.y;
   const float* rec = scratch + (static_cast<size_t>(row) * qh + head) * splits * (D + 2);
   float m = -INFINITY;
@@ -462,12 +466,11 @@ static int launch_attn(const __half* q, const __half* gate, const int* row_req, 
   static const int slot[4] = {runtime_new_slot(), runtime_new_slot(), runtime_new_slot(),
                               runtime_new_slot()};
   if (const int e = runtime_allow_smem(slot[2 * apart + wide], kernel, SMEM)) return e;
-  kernel<<<grid, ATTN_WARPS * 32, SMEM, stream>>>(q, gate, row_req, row_pos, page_table, max_pages,
-                                                  kc, vc, ks, vs, out, qh, kvh, splits, scratch,
-                                                  rep, apart_keys);
+  launch_early(kernel, grid, ATTN_WARPS * 32, SMEM, stream, q, gate, row_req, row_pos, page_table,
+               max_pages, kc, vc, ks, vs, out, qh, kvh, splits, scratch, rep, apart_keys);
   if (splits > 1)
-    attn_merge_kernel<D><<<dim3(rows, qh), D < 128 ? 64 : 128, 0, stream>>>(scratch, gate, out, qh,
-                                                                           splits);
+    launch_early(attn_merge_kernel<D>, dim3(rows, qh), D < 128 ? 64 : 128, 0, stream, scratch, gate,
+                 out, qh, splits);
   return static_cast<int>(cudaGetLastError());
 }
 

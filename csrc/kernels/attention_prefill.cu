@@ -159,6 +159,7 @@ __global__ void __launch_bounds__(Smem<D, NQ>::THREADS, 1) attn_prefill_kernel(
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 15);
 
   const int warp = warp_same(threadIdx.x >> 5), lane = threadIdx.x & 31;
+  grid_wait();
   const Chunk ch = chunks[blockIdx.z];
   const int h = blockIdx.y;                       // kv head
   const int P = TILE / rep;                       // query positions per tile
@@ -200,6 +201,7 @@ __global__ void __launch_bounds__(Smem<D, NQ>::THREADS, 1) attn_prefill_kernel(
   __syncthreads();
   tc_fence_after();
   const uint32_t tmem_base = warp_same(*tmem_slot);
+  grid_release();
   const uint32_t tmem_s = tmem_base, tmem_o = tmem_base + 256;   // O of tile q at + q * 128
   const int* pages = page_table + static_cast<size_t>(ch.slot) * max_pages;
 
@@ -545,9 +547,9 @@ int launch(const __half* q, const __half* gate, const Chunk* chunks, int n_chunk
   static const int slot = runtime_new_slot();
   if (const int e = runtime_allow_smem(slot, attn_prefill_kernel<D, NQ>, L::TOTAL)) return e;
   dim3 grid((max_q_len + NQ * P - 1) / (NQ * P), kvh, n_chunks);
-  attn_prefill_kernel<D, NQ><<<grid, L::THREADS, L::TOTAL, stream>>>(
-      tq, chunks, page_table, max_pages, kc, vc, ks, vs, gate, out, qh, kvh, rep, num_pages,
-      runtime_status_ptr());
+  launch_early(attn_prefill_kernel<D, NQ>, grid, L::THREADS, L::TOTAL, stream, tq, chunks,
+               page_table, max_pages, kc, vc, ks, vs, gate, out, qh, kvh, rep, num_pages,
+               runtime_status_ptr());
   return static_cast<int>(cudaGetLastError());
 }
 

@@ -113,6 +113,18 @@ __device__ __forceinline__ bool mbar_wait_abortable(uint64_t* bar, uint32_t pari
   }
 }
 
+// ---------------------------------------------------------------- overlapping launches
+// A kernel started by launch_early may be resident before the kernels ahead of it on its stream
+// have ended.  Every CTA of it calls grid_wait before it touches memory that they write or read and
+// before it may exit (a grid that ended early would release its successors too soon); only what is
+// constant from start-up on, such as the decode tables, is read ahead of it.  grid_release lets the
+// next kernel become resident in turn; kernels that allocate tensor memory call it after that, so
+// that a successor cannot take what they need.
+__device__ __forceinline__ void grid_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+__device__ __forceinline__ void grid_release() {
+  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+}
+
 // ---------------------------------------------------------------- TMA
 __device__ __forceinline__ void tma_load_2d(void* smem_dst, const void* tmap, uint64_t* bar, int x,
                                             int y) {
@@ -538,6 +550,29 @@ int runtime_allow_smem(int slot, Kernel* kernel, size_t bytes) {
   return runtime_allow_smem(slot, reinterpret_cast<const void*>(kernel), bytes);
 }
 int runtime_new_slot();
+// Launch of a kernel that calls grid_wait (see there): what lies between two kernels of a stream,
+// also inside a graph, falls together with the end of the first (one decode step of eight requests,
+// 27 kernels, 241 -> 232 us; of one request 197; 1 x 19456 x 2560 12.9 -> 11.8; 16 rows on 512 Q2
+// experts 113 -> 105).  Not for grids of many CTAs, each of which pays for the wait: with all of
+// them started this way 2048 rows on 128 experts took 348 us, 310 now and 311 without, and a
+// recurrent mixer of two prompts 274, 256 now.
+constexpr long long EARLY_CTAS = 4 * 148;
+template <class... P, class... A>
+void launch_early(void (*kernel)(P...), dim3 grid, dim3 block, size_t smem, cudaStream_t stream,
+                  A&&... args) {
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = grid;
+  cfg.blockDim = block;
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = stream;
+  cudaLaunchAttribute attr[1];
+  attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr[0].val.programmaticStreamSerializationAllowed = 1;
+  cfg.attrs = attr;
+  const long long ctas = static_cast<long long>(grid.x) * grid.y * grid.z;
+  cfg.numAttrs = ctas <= EARLY_CTAS ? 1 : 0;
+  cudaLaunchKernelEx(&cfg, kernel, static_cast<P>(args)...);   // failures: cudaGetLastError
+}
 
 // ---------------------------------------------------------------- math
 __device__ __forceinline__ float warp_sum(float v) {

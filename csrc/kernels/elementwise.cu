@@ -21,6 +21,8 @@ namespace orinfer {
 __global__ void embed_w8_kernel(const int* __restrict__ ids, const int8_t* __restrict__ table,
                                 const __half* __restrict__ scales, __half* __restrict__ out,
                                 int hidden, int vocab, int* status) {
+  grid_wait();
+  grid_release();
   const int row = blockIdx.x;
   int id = ids[row];
   if (id < 0 || id >= vocab) {
@@ -77,6 +79,8 @@ __global__ void __launch_bounds__(512) act_prep_kernel(
   __shared__ float red[32];
   __shared__ float cl_slot[2];
   __shared__ float blk_sum[MAX_NORM_BLOCKS];
+  grid_wait();
+  grid_release();
   const int tid = threadIdx.x;
   const int crank = CL > 1 ? static_cast<int>(blockIdx.x) % CL : 0;
   const int nblk = K / 128;
@@ -287,6 +291,8 @@ __global__ void __launch_bounds__(RegRows<NB>::THREADS, RegRows<NB>::CTAS) act_p
     __half* __restrict__ y_out, int nblk, float eps, int zero_centered,
     const int* __restrict__ row_limit) {
   const int row = blockIdx.x, warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  grid_wait();
+  grid_release();
   const int W = blockDim.x >> 5, K = nblk * 128;
   if (row_limit != nullptr && row >= *row_limit) return;
   __shared__ float blk_sum[MAX_NORM_BLOCKS];
@@ -415,6 +421,8 @@ __global__ void ag_wait_kernel(AgIn in, int rows, int* status) {
 // ------------------------------------------------------------------ RoPE tables
 __global__ void rope_table_kernel(const int* __restrict__ positions, float* __restrict__ cosb,
                                   float* __restrict__ sinb, int rows, int half_dim, double theta) {
+  grid_wait();
+  grid_release();
   const int idx = blockIdx.x * blockDim.x + threadIdx.x;
   if (idx >= rows * half_dim) return;
   const int r = idx / half_dim, j = idx % half_dim;
@@ -441,6 +449,8 @@ __global__ void __launch_bounds__(256) qk_rope_kv_kernel(
   constexpr int HALF = D / 2;
   constexpr int PER = HALF / 32;          // pairs per lane
   constexpr int GROUPS = D / 64;
+  grid_wait();
+  grid_release();
   const int row = blockIdx.x;
   const int head = blockIdx.y * (blockDim.x >> 5) + (threadIdx.x >> 5);
   const int lane = threadIdx.x & 31;
@@ -565,7 +575,7 @@ int orinfer_embed_w8(const int* ids, const int8_t* table, const __half* scales, 
   if (rows <= 0) return 0;
   if (hidden % 16) return -1;
   if (runtime_ensure_init() != cudaSuccess) return -2;
-  embed_w8_kernel<<<rows, 128, 0, stream>>>(ids, table, scales, out, hidden, vocab,
+  launch_early(embed_w8_kernel, rows, 128, 0, stream, ids, table, scales, out, hidden, vocab,
                                             runtime_status_ptr());
   return static_cast<int>(cudaGetLastError());
 }
@@ -711,8 +721,8 @@ static int act_prep_launch(const __half* x, float* resid, const __half* norm_w, 
 #define REG_ROWS(NBV)                                                                           \
   if (nb <= NBV) {                                                                              \
     auto kernel = swiglu ? act_prep_regs_kernel<true, NBV> : act_prep_regs_kernel<false, NBV>;  \
-    kernel<<<rows, warps * 32, 0, stream>>>(x, resid, norm_w, signs, q_out, scale_out, y_out,   \
-                                            nblk, eps, zero_centered, row_limit);               \
+    launch_early(kernel, rows, warps * 32, 0, stream, x, resid, norm_w, signs, q_out, scale_out, \
+                 y_out, nblk, eps, zero_centered, row_limit);                                   \
     return static_cast<int>(cudaGetLastError());                                                \
   }
     REG_ROWS(1) REG_ROWS(2) REG_ROWS(3) REG_ROWS(4) REG_ROWS(5) REG_ROWS(6) REG_ROWS(8)
@@ -725,13 +735,15 @@ static int act_prep_launch(const __half* x, float* resid, const __half* norm_w, 
     cfg.blockDim = dim3(256);
     cfg.dynamicSmemBytes = (static_cast<size_t>(K / 128 + CL - 1) / CL) * 128 * sizeof(float);
     cfg.stream = stream;
-    cudaLaunchAttribute attr[1];
+    cudaLaunchAttribute attr[2];
     attr[0].id = cudaLaunchAttributeClusterDimension;
     attr[0].val.clusterDim.x = CL;
     attr[0].val.clusterDim.y = 1;
     attr[0].val.clusterDim.z = 1;
+    attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[1].val.programmaticStreamSerializationAllowed = 1;
     cfg.attrs = attr;
-    cfg.numAttrs = 1;
+    cfg.numAttrs = in.inbox == nullptr && in.ll == nullptr ? 2 : 1;   // early: nothing from peers
     const AgOut no_ag{};
     const int* no_limit = nullptr;
     cudaError_t e;
@@ -767,8 +779,8 @@ int orinfer_rope_table(const int* positions, float* cosb, float* sinb, int rows,
                        double theta, cudaStream_t stream) {
   if (rows <= 0) return 0;
   const int total = rows * (head_dim / 2);
-  rope_table_kernel<<<(total + 255) / 256, 256, 0, stream>>>(positions, cosb, sinb, rows,
-                                                             head_dim / 2, theta);
+  launch_early(rope_table_kernel, (total + 255) / 256, 256, 0, stream, positions, cosb, sinb, rows,
+               head_dim / 2, theta);
   return static_cast<int>(cudaGetLastError());
 }
 
@@ -784,9 +796,9 @@ int orinfer_qk_rope_kv(const __half* qkv, const __half* wq, const __half* wk, co
   dim3 grid(rows, (heads + 7) / 8);
   int* st = runtime_status_ptr();
 #define LAUNCH(DD, GG)                                                                          \
-  qk_rope_kv_kernel<DD, GG><<<grid, 256, 0, stream>>>(                                          \
-      qkv, wq, wk, cosb, sinb, row_req, row_pos, page_table, max_pages, qh, kvh, eps,           \
-      zero_centered, q_out, gate_out, kcache, vcache, kscale, vscale, num_pages, st)
+  launch_early(qk_rope_kv_kernel<DD, GG>, grid, 256, 0, stream, qkv, wq, wk, cosb, sinb,           \
+               row_req, row_pos, page_table, max_pages, qh, kvh, eps, zero_centered, q_out,        \
+               gate_out, kcache, vcache, kscale, vscale, num_pages, st)
   if (head_dim == 64 && !gated) LAUNCH(64, false);
   else if (head_dim == 64 && gated) LAUNCH(64, true);
   else if (head_dim == 128 && !gated) LAUNCH(128, false);

@@ -27,6 +27,8 @@ __global__ void __launch_bounds__(256) small_proj_kernel(const __half* __restric
                                                          const __half* __restrict__ w,
                                                          float* __restrict__ out, int hidden,
                                                          int n) {
+  grid_wait();
+  grid_release();
   const int row = blockIdx.x, warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const __half* xr = x + static_cast<size_t>(row) * hidden;
   for (int e = warp; e < n; e += blockDim.x >> 5) {
@@ -103,6 +105,8 @@ __global__ void __launch_bounds__(256) gdn_conv_vec_kernel(
     const int* __restrict__ row_slot, const int* __restrict__ row_pos, int rows, int conv_dim,
     int qk_channels, __half* __restrict__ y) {
   constexpr int LANES = D / 8;
+  grid_wait();
+  grid_release();
   const int c = (blockIdx.y * 256 + threadIdx.x) * 8, row0 = blockIdx.x * R;
   if (c >= conv_dim) return;                       // whole heads, so whole lane groups
   const unsigned group = LANES == 32 ? 0xffffffffu
@@ -179,6 +183,8 @@ __global__ void __launch_bounds__(256) gdn_history_kernel(const __half* __restri
                                                           int conv_dim,
                                                           __half* __restrict__ hist,
                                                           const int* __restrict__ accepted) {
+  grid_wait();
+  grid_release();
   Segment s = segs[blockIdx.x];
   if (accepted != nullptr) {                 // commit of a verified prefix of the rows
     s.rows = min(accepted[blockIdx.x], s.rows);
@@ -230,6 +236,8 @@ __global__ void __launch_bounds__(256) gdn_scan_kernel(
   // prefix of the rows onto the stored state.
   constexpr int SPLIT = D / DC, PARTS = 256 / DC, ROWS = D / PARTS;
   static_assert(ROWS % 4 == 0, "four independent accumulators");
+  grid_wait();
+  grid_release();
   const int vh = blockIdx.x / SPLIT, c0 = (blockIdx.x % SPLIT) * DC;
   const Segment seg = segs[blockIdx.y];
   if (seg.rows <= 0 || seg.rows >= long_rows) return;  // long runs: gdn_chunk_kernel
@@ -345,6 +353,8 @@ __global__ void __launch_bounds__(256) gdn_scan_split_kernel(
     float* __restrict__ out, float* __restrict__ factors, int long_rows) {
   constexpr int DC = 32, SPLIT = D / DC, PARTS = 8, ROWS = D / PARTS, T = SCAN_STEPS;
   constexpr int CH = D / 4 + DC / 8;                 // 16-byte units of one staged row
+  grid_wait();
+  grid_release();
   const int vh = blockIdx.x / SPLIT, c0 = (blockIdx.x % SPLIT) * DC;
   const Segment seg = segs[blockIdx.y];
   if (seg.rows <= 0 || seg.rows >= long_rows) return;  // long runs: gdn_chunk_kernel
@@ -644,6 +654,8 @@ __global__ void __launch_bounds__(CHUNK_THREADS, 2) gdn_chunk_kernel(
   constexpr int D = 128;
   extern __shared__ __align__(16) unsigned char chunk_smem[];
   ChunkSmem& sm = *reinterpret_cast<ChunkSmem*>(chunk_smem);
+  grid_wait();
+  grid_release();
   const Segment seg = segs[blockIdx.y];
   if (seg.rows < GDN_LONG_ROWS) return;
   const int vh = blockIdx.x >> 1, kh = vh / (hv / hk), dk_total = hk * D;
@@ -1029,6 +1041,8 @@ __global__ void __launch_bounds__(D) gdn_gated_norm_kernel(
     const float* __restrict__ o, const __half* __restrict__ z, int z_stride,
     const __half* __restrict__ w, float eps, int sigmoid_gate, int hv,
     __half* __restrict__ y) {
+  grid_wait();
+  grid_release();
   const int row = blockIdx.x, h = blockIdx.y, d = threadIdx.x;
   const float v = o[(static_cast<size_t>(row) * hv + h) * D + d];
   constexpr int V = D / 32;
@@ -1065,6 +1079,8 @@ __global__ void __launch_bounds__(256) gdn_gated_norm_warp_kernel(
   struct __align__(V * 4) Float {
     float f[V];
   };
+  grid_wait();
+  grid_release();
   const long long item = static_cast<long long>(blockIdx.x) * 8 + (threadIdx.x >> 5);
   if (item >= items) return;
   const int lane = threadIdx.x & 31;
@@ -1105,22 +1121,23 @@ static void launch_conv(const __half* x, int x_stride, const __half* weight, con
   }
   const int cols = (conv_dim + 2047) / 2048;
   if (rows * cols >= 8 * 4 * 148)                // strips of eight rows still fill the machine
-    gdn_conv_vec_kernel<D, 8><<<dim3((rows + 7) / 8, cols), 256, 0, stream>>>(
-        x, x_stride, weight, hist, row_first, row_slot, row_pos, rows, conv_dim, 2 * hk * D, y);
+    launch_early(gdn_conv_vec_kernel<D, 8>, dim3((rows + 7) / 8, cols), 256, 0, stream, x,
+                 x_stride, weight, hist, row_first, row_slot, row_pos, rows, conv_dim, 2 * hk * D,
+                 y);
   else
-    gdn_conv_vec_kernel<D, 1><<<dim3(rows, cols), 256, 0, stream>>>(
-        x, x_stride, weight, hist, row_first, row_slot, row_pos, rows, conv_dim, 2 * hk * D, y);
+    launch_early(gdn_conv_vec_kernel<D, 1>, dim3(rows, cols), 256, 0, stream, x, x_stride, weight,
+                 hist, row_first, row_slot, row_pos, rows, conv_dim, 2 * hk * D, y);
 }
 
 static void launch_history(const __half* x, int x_stride, const Segment* segs, int n_segs,
                            const int* row_slot, const int* row_pos, int conv_dim, __half* hist,
                            const int* accepted, cudaStream_t stream) {
   if (x_stride % 8 == 0 && aligned(x, 16) && aligned(hist, 16))
-    gdn_history_kernel<8><<<dim3(n_segs, (conv_dim + 2047) / 2048), 256, 0, stream>>>(
-        x, x_stride, segs, row_slot, row_pos, conv_dim, hist, accepted);
+    launch_early(gdn_history_kernel<8>, dim3(n_segs, (conv_dim + 2047) / 2048), 256, 0, stream, x,
+                 x_stride, segs, row_slot, row_pos, conv_dim, hist, accepted);
   else
-    gdn_history_kernel<1><<<dim3(n_segs, (conv_dim + 255) / 256), 256, 0, stream>>>(
-        x, x_stride, segs, row_slot, row_pos, conv_dim, hist, accepted);
+    launch_early(gdn_history_kernel<1>, dim3(n_segs, (conv_dim + 255) / 256), 256, 0, stream, x,
+                 x_stride, segs, row_slot, row_pos, conv_dim, hist, accepted);
 }
 
 }  // namespace orinfer
@@ -1133,7 +1150,7 @@ int orinfer_small_proj(const __half* x, const __half* w, float* out, int rows, i
                        cudaStream_t stream) {
   if (rows <= 0) return 0;
   if (hidden % 8) return -1;
-  small_proj_kernel<<<rows, 256, 0, stream>>>(x, w, out, hidden, n);
+  launch_early(small_proj_kernel, rows, 256, 0, stream, x, w, out, hidden, n);
   return static_cast<int>(cudaGetLastError());
 }
 
@@ -1205,13 +1222,12 @@ int orinfer_gdn_scan(const __half* qkv, const float* ab, const float* a_log, con
     long_rows = GDN_LONG_ROWS;
     static const int slot = runtime_new_slot();
     if (const int e = runtime_allow_smem(slot, gdn_chunk_kernel, sizeof(ChunkSmem))) return e;
-    gdn_chunk_kernel<<<dim3(hv * 2, n_segs), CHUNK_THREADS, sizeof(ChunkSmem), stream>>>(
-        qkv, conv_dim, ab, a_log, dt_bias, sg, row_slot, row_pos, hk, hv, state, out);
+    launch_early(gdn_chunk_kernel, dim3(hv * 2, n_segs), CHUNK_THREADS, sizeof(ChunkSmem), stream,
+                 qkv, conv_dim, ab, a_log, dt_bias, sg, row_slot, row_pos, hk, hv, state, out);
   }
 #define ORINFER_SCAN(KERNEL, GRID_X)                                                       \
-  KERNEL<<<dim3(GRID_X, n_segs), 256, 0, stream>>>(qkv, conv_dim, ab, a_log, dt_bias, sg,  \
-                                                   row_slot, row_pos, hk, hv, state, out,  \
-                                                   factors, long_rows)
+  launch_early(KERNEL, dim3(GRID_X, n_segs), 256, 0, stream, qkv, conv_dim, ab, a_log,     \
+               dt_bias, sg, row_slot, row_pos, hk, hv, state, out, factors, long_rows)
   if (head_dim == 128) {
     if (split) ORINFER_SCAN(gdn_scan_split_kernel<128>, hv * 4);
     else ORINFER_SCAN((gdn_scan_kernel<128, 128>), hv);
@@ -1234,18 +1250,18 @@ int orinfer_gdn_gated_norm(const float* o, const __half* z, int z_stride, const 
       aligned(o, 4 * v) && aligned(y, 2 * v)) {
     const unsigned grid = static_cast<unsigned>((items + 7) / 8);
     if (head_dim == 128)
-      gdn_gated_norm_warp_kernel<128><<<grid, 256, 0, stream>>>(o, z, z_stride, w, eps,
+      launch_early(gdn_gated_norm_warp_kernel<128>, grid, 256, 0, stream, o, z, z_stride, w, eps,
                                                                sigmoid_gate, hv, items, y);
     else
-      gdn_gated_norm_warp_kernel<64><<<grid, 256, 0, stream>>>(o, z, z_stride, w, eps,
+      launch_early(gdn_gated_norm_warp_kernel<64>, grid, 256, 0, stream, o, z, z_stride, w, eps,
                                                               sigmoid_gate, hv, items, y);
     return static_cast<int>(cudaGetLastError());
   }
   if (head_dim == 128)
-    gdn_gated_norm_kernel<128><<<dim3(rows, hv), 128, 0, stream>>>(o, z, z_stride, w, eps,
+    launch_early(gdn_gated_norm_kernel<128>, dim3(rows, hv), 128, 0, stream, o, z, z_stride, w, eps,
                                                                    sigmoid_gate, hv, y);
   else if (head_dim == 64)
-    gdn_gated_norm_kernel<64><<<dim3(rows, hv), 64, 0, stream>>>(o, z, z_stride, w, eps,
+    launch_early(gdn_gated_norm_kernel<64>, dim3(rows, hv), 64, 0, stream, o, z, z_stride, w, eps,
                                                                  sigmoid_gate, hv, y);
   else
     return -1;

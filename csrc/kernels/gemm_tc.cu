@@ -136,6 +136,7 @@ __global__ void __launch_bounds__(THREADS, 1) qgemm_tc_kernel(
 
   const int warp = warp_same(threadIdx.x >> 5), lane = threadIdx.x & 31;
   const int n0 = n_begin + blockIdx.x * BN;    // this launch covers columns [n_begin, n_end)
+  if (grp.tiles != nullptr) grid_wait();       // the table
   int m0 = blockIdx.y * BM * MT, m_limit = M, b_row0 = n0, mt_act = MT;
   if (grp.tiles != nullptr) {
     // MT neighbouring 128-row tiles of one expert go to one CTA (the fourth word counts an
@@ -191,6 +192,8 @@ __global__ void __launch_bounds__(THREADS, 1) qgemm_tc_kernel(
   __syncthreads();
   tc_fence_after();
   const uint32_t tmem_base = warp_same(*tmem_slot);
+  grid_wait();
+  grid_release();
   // peer epilogue staging: one padded FP16 row per output row (pad keeps 16-byte stores of
   // 32 consecutive rows on distinct banks)
   constexpr int STAGE_ROW = BN * 2 + 16;
@@ -1471,6 +1474,8 @@ __global__ void __launch_bounds__(256) splitk_finalize_kernel(
     const int* __restrict__ partial, int splits, const float* __restrict__ a_scale,
     const __half* __restrict__ w_scale, __half* __restrict__ out, int M, int N, PeerOut po,
     int ag_scales, int n_begin, int width) {
+  grid_wait();
+  grid_release();
   const int groups = width / 8;
   const long long idx = static_cast<long long>(blockIdx.x) * blockDim.x + threadIdx.x;
   if (idx < static_cast<long long>(M) * groups) {
@@ -1591,15 +1596,27 @@ int launch(const int8_t* a, const float* a_scale, const void* w, const __half* w
   if (splits > 1 && (tiles > static_cast<size_t>(SPLITK_TICKETS) ||
                      tiles * splits * MT * BM * NB * 4 > SPLITK_WORKSPACE_BYTES))
     return -1;
-  kernel<<<grid, THREADS, L::TOTAL, stream>>>(
-      ta, tb, reinterpret_cast<const unsigned char*>(w), a_scale, w_scale, out, M, N, K,
-      runtime_e8p_tables(), runtime_status_ptr(), po, grp, ag, partial,
-      in_kernel ? runtime_splitk_tickets() : nullptr, n_begin, n_end, g_probe);
+  int* tickets = in_kernel ? runtime_splitk_tickets() : nullptr;
+  const unsigned char* codes = reinterpret_cast<const unsigned char*>(w);
+  // with peers the launch keeps its place behind the kernels before it
+  if (po.tp == 0 && ag.tp == 0)
+    launch_early(kernel, grid, THREADS, L::TOTAL, stream, ta, tb, codes, a_scale, w_scale, out, M,
+                 N, K, runtime_e8p_tables(), runtime_status_ptr(), po, grp, ag, partial, tickets,
+                 n_begin, n_end, g_probe);
+  else
+    kernel<<<grid, THREADS, L::TOTAL, stream>>>(
+        ta, tb, codes, a_scale, w_scale, out, M, N, K, runtime_e8p_tables(), runtime_status_ptr(),
+        po, grp, ag, partial, tickets, n_begin, n_end, g_probe);
   if (splits > 1 && !in_kernel) {
     const long long items = static_cast<long long>(M) * (width / 8);
-    splitk_finalize_kernel<<<static_cast<unsigned>((items + 255) / 256), 256, 0, stream>>>(
-        partial, splits, a_scale, w_scale, reinterpret_cast<__half*>(out), M, N, po,
-        ag.tp > 0 ? 1 : 0, n_begin, width);
+    const unsigned blocks = static_cast<unsigned>((items + 255) / 256);
+    if (po.tp == 0 && ag.tp == 0)
+      launch_early(splitk_finalize_kernel, blocks, 256, 0, stream, partial, splits, a_scale,
+                   w_scale, reinterpret_cast<__half*>(out), M, N, po, 0, n_begin, width);
+    else
+      splitk_finalize_kernel<<<blocks, 256, 0, stream>>>(
+          partial, splits, a_scale, w_scale, reinterpret_cast<__half*>(out), M, N, po,
+          ag.tp > 0 ? 1 : 0, n_begin, width);
   }
   return static_cast<int>(cudaGetLastError());
 }

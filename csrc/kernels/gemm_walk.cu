@@ -132,6 +132,7 @@ __global__ void __launch_bounds__(Layout<FMT, MT>::THREADS, 1) qgemm_walk_kernel
   static_assert((2 * S + 2 * SC + 2 * BUFS) * 8 + 8 + 128 <= 512, "barriers");
 
   const int tid = threadIdx.x, warp = warp_same(tid >> 5), lane = tid & 31;
+  if (p.tiles != nullptr) grid_wait();          // the table
   const int n_tiles = (p.n_end + BN - 1) / BN, kblocks = p.K / BK;
   int m_tiles = (p.M + BM * MT - 1) / (BM * MT);
   if (p.tiles != nullptr) {
@@ -212,6 +213,8 @@ __global__ void __launch_bounds__(Layout<FMT, MT>::THREADS, 1) qgemm_walk_kernel
   __syncthreads();
   tc_fence_after();
   const uint32_t tmem_base = warp_same(*tmem_slot);
+  grid_wait();
+  grid_release();
 
 #define WALK_WAIT(bar, par, code, detail) \
   mbar_wait_abortable((bar), (par), status, (code), (detail), abort_w)
@@ -484,8 +487,8 @@ int launch(const WalkCall& c, cudaStream_t stream) {
                      (c.tiles ? c.max_tiles : (c.M + BM * MT - 1) / (BM * MT));
   const Args p{static_cast<const unsigned char*>(c.w), c.a_scale, c.w_scale, c.out, c.M, c.N, c.K,
                c.n_end, c.tiles, c.meta, c.w_stride};
-  qgemm_walk_kernel<FMT, MT><<<static_cast<int>(tiles < 148 ? tiles : 148), L::THREADS, L::TOTAL,
-                               stream>>>(ta, tb, p, runtime_e8p_tables(), runtime_status_ptr());
+  launch_early(qgemm_walk_kernel<FMT, MT>, static_cast<unsigned>(tiles < 148 ? tiles : 148),
+               L::THREADS, L::TOTAL, stream, ta, tb, p, runtime_e8p_tables(), runtime_status_ptr());
   return static_cast<int>(cudaGetLastError());
 }
 

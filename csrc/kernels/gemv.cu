@@ -141,6 +141,8 @@ struct GemvEarly {
                                        const __half* __restrict__ ws, int n_count, int M, int K,
                                        bool plain, int tid) {
     if (FMT != 0) fill.load(tables, tid);
+    grid_wait();
+    grid_release();
     w_scale = tid < n_count ? __ldg(ws + tid) : __half(0.f);
     scale = 0.f;
     if (plain) {
@@ -759,6 +761,8 @@ __global__ void __launch_bounds__(W8_WARPS * 32) w8_gemv_kernel(
     const __half* __restrict__ w_scale, void* __restrict__ out, int M, int N, int K, int out_f32,
     PeerOut po) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
+  grid_wait();
+  grid_release();
   int8_t* act = reinterpret_cast<int8_t*>(smem_raw);
   const PeerOut* peer = po.tp > 0 ? &po : nullptr;
   stage_activations<MT>(act, a, M, K);
@@ -837,6 +841,8 @@ __global__ void __launch_bounds__((1 + STREAM_MAX) * 32) w8_stream_kernel(
     }
     mbar_fence_init();
   }
+  grid_wait();
+  grid_release();
   for (int c = threadIdx.x; c < M * (K / 16); c += blockDim.x) {
     const int m = c / (K / 16), k = (c - m * (K / 16)) * 16;
     *reinterpret_cast<int4*>(act + m * stride + k) =
@@ -943,6 +949,8 @@ __global__ void __launch_bounds__(GEMV_THREADS, 1) qgemv_grouped_kernel(
     fill.load(tables, tid);
     fill.store(smem_raw, tid);
   }
+  grid_wait();
+  grid_release();
   int n_tiles = meta[0];
   const int* list = nullptr;
   if (MIXED && most_rows > 0) {
@@ -1140,9 +1148,9 @@ static int launch_grouped(const int8_t* a, const float* as, const void* w, const
   if (const int e = runtime_allow_smem(slot, qgemv_grouped_kernel<FMT, MIXED>,
                                        MIXED ? GEMV_SMEM_LIMIT : smem))
     return e;
-  qgemv_grouped_kernel<FMT, MIXED><<<GROUPED_CTAS, GEMV_THREADS, smem, stream>>>(
-      a, as, reinterpret_cast<const unsigned char*>(w), ws, reinterpret_cast<__half*>(out), N, K,
-      bank, runtime_e8p_tables(), tiles, meta, most_rows, listed);
+  launch_early(qgemv_grouped_kernel<FMT, MIXED>, GROUPED_CTAS, GEMV_THREADS, smem, stream, a, as,
+               reinterpret_cast<const unsigned char*>(w), ws, reinterpret_cast<__half*>(out), N,
+               K, bank, runtime_e8p_tables(), tiles, meta, most_rows, listed);
   return static_cast<int>(cudaGetLastError());
 }
 
@@ -1234,9 +1242,16 @@ static int launch_gemv(const int8_t* a, const float* as, const void* w, const __
   static const int slot[2] = {runtime_new_slot(), runtime_new_slot()};
   auto start = [&](auto kernel, int threads, auto* weights, int sl) -> int {
     if (const int e = runtime_allow_smem(sl, kernel, GEMV_SMEM_LIMIT)) return e;
-    kernel<<<g.n_parts * g.k_parts, threads, smem, stream>>>(
-        a, as, weights, ws, out, M, N, K, out_f32, runtime_e8p_tables(), po, g.n_parts, g.k_parts,
-        g.max_groups, runtime_gemv_workspace(), fz);
+    const int grid = g.n_parts * g.k_parts;
+    // with peers the launch keeps its place behind the kernels before it
+    if (po.tp == 0)
+      launch_early(kernel, grid, threads, smem, stream, a, as, weights, ws, out, M, N, K, out_f32,
+                   runtime_e8p_tables(), po, g.n_parts, g.k_parts, g.max_groups,
+                   runtime_gemv_workspace(), fz);
+    else
+      kernel<<<grid, threads, smem, stream>>>(a, as, weights, ws, out, M, N, K, out_f32,
+                                              runtime_e8p_tables(), po, g.n_parts, g.k_parts,
+                                              g.max_groups, runtime_gemv_workspace(), fz);
     return static_cast<int>(cudaGetLastError());
   };
   if constexpr (FMT != 0)
@@ -1254,8 +1269,14 @@ static int launch_w8(const int8_t* a, const float* as, const void* w, const __ha
   if (smem > 200 * 1024) return -1;
   static const int slot = runtime_new_slot();
   if (const int e = runtime_allow_smem(slot, w8_gemv_kernel<MT>, 200 * 1024)) return e;
-  w8_gemv_kernel<MT><<<(N + W8_WARPS - 1) / W8_WARPS, W8_WARPS * 32, smem, stream>>>(
-      a, as, reinterpret_cast<const int8_t*>(w), ws, out, M, N, K, out_f32, po);
+  const int grid = (N + W8_WARPS - 1) / W8_WARPS;
+  const int8_t* weights = reinterpret_cast<const int8_t*>(w);
+  if (po.tp == 0)
+    launch_early(w8_gemv_kernel<MT>, grid, W8_WARPS * 32, smem, stream, a, as, weights, ws, out,
+                 M, N, K, out_f32, po);
+  else
+    w8_gemv_kernel<MT><<<grid, W8_WARPS * 32, smem, stream>>>(a, as, weights, ws, out, M, N, K,
+                                                              out_f32, po);
   return static_cast<int>(cudaGetLastError());
 }
 
@@ -1266,9 +1287,9 @@ static int launch_w8_stream(const int8_t* a, const float* as, const void* w, con
   static const int slot = runtime_new_slot();
   if (const int e = runtime_allow_smem(slot, w8_stream_kernel, GEMV_SMEM_LIMIT)) return e;
   const int tiles = (N + STREAM_ROWS - 1) / STREAM_ROWS;
-  w8_stream_kernel<<<tiles < 148 ? tiles : 148, (1 + stages) * 32, smem, stream>>>(
-      a, as, reinterpret_cast<const int8_t*>(w), ws, out, M, N, K, out_f32, stages,
-      runtime_status_ptr());
+  launch_early(w8_stream_kernel, tiles < 148 ? tiles : 148, (1 + stages) * 32, smem, stream, a,
+               as, reinterpret_cast<const int8_t*>(w), ws, out, M, N, K, out_f32, stages,
+               runtime_status_ptr());
   return static_cast<int>(cudaGetLastError());
 }
 

@@ -91,6 +91,8 @@ __global__ void __launch_bounds__(256) router_topk_kernel(
     int has_shared, int top_k, int renorm, int* __restrict__ ids, float* __restrict__ probs,
     float* __restrict__ shared_gate) {
   extern __shared__ float logits[];                 // [experts + 1]
+  grid_wait();
+  grid_release();
   const int row = blockIdx.x, warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int nw = blockDim.x >> 5, total = experts + (has_shared ? 1 : 0);
   const __half* xr = x + static_cast<size_t>(row) * hidden;
@@ -142,6 +144,8 @@ __global__ void __cluster_dims__(ROUTER_CL, 1, 1) __launch_bounds__(WARPS * 32) 
   extern __shared__ float router_smem[];
   float(*part)[ROWS][COLS] = reinterpret_cast<float(*)[ROWS][COLS]>(router_smem);
   float* logits = router_smem + WARPS * ROWS * COLS;              // [OWN][total]
+  grid_wait();
+  grid_release();
   cg::cluster_group cluster = cg::this_cluster();
   const int crank = static_cast<int>(cluster.block_rank());
   const int row0 = static_cast<int>(blockIdx.x) / CL * ROWS;
@@ -216,8 +220,8 @@ static int launch_router(const __half* x, const __half* w, int rows, int hidden,
                                        (PART + 2 * 8 * ROUTER_CL * MAXT) * sizeof(float)))
     return e;
   const int grid = (rows + 15) / 16 * ROUTER_CL;
-  router_mma_kernel<MAXT, WARPS><<<grid, WARPS * 32, smem, stream>>>(
-      x, w, rows, hidden, experts, has_shared, top_k, renorm, ids, probs, shared_gate);
+  launch_early(router_mma_kernel<MAXT, WARPS>, grid, WARPS * 32, smem, stream, x, w, rows, hidden,
+               experts, has_shared, top_k, renorm, ids, probs, shared_gate);
   return static_cast<int>(cudaGetLastError());
 }
 
@@ -252,6 +256,8 @@ __global__ void __cluster_dims__(CL, 1, 1) __launch_bounds__(256, 1) router_rows
   const int span = hidden / CL, pitch = span + 8;           // halves; rows 16 bytes apart in banks
   __half* xs = reinterpret_cast<__half*>(router_raw);       // [ROWS][pitch]
   __half* ws = xs + ROWS * pitch;                           // [8 tiles][pitch]
+  grid_wait();
+  grid_release();
   cg::cluster_group cluster = cg::this_cluster();
   const int crank = static_cast<int>(cluster.block_rank());
   const int row0 = static_cast<int>(blockIdx.x) / CL * ROWS;
@@ -287,7 +293,8 @@ __global__ void __cluster_dims__(CL, 1, 1) __launch_bounds__(256, 1) router_rows
       for (int m = 0; m < 2; ++m)
 #pragma unroll
         for (int h = 0; h < 2; ++h)
-          ldmatrix4(a[m][h], xs + (m0 + m * 16 + (lane & 15)) * pitch + k + h * 16 + (lane >> 4) * 8);
+          ldmatrix4(a[m][h],
+                    xs + (m0 + m * 16 + (lane & 15)) * pitch + k + h * 16 + (lane >> 4) * 8);
 #pragma unroll
       for (int i = 0; i < PER; ++i) {
         const int tile = first + i * 4;
@@ -353,9 +360,9 @@ static int launch_router_rows(const __half* x, const __half* w, int rows, int hi
   static const int slot = runtime_new_slot();
   if (const int e = runtime_allow_smem(slot, router_rows_kernel<CL>, 220 * 1024)) return e;
   const int grid = (rows + ROUTER_ROWS - 1) / ROUTER_ROWS * CL;
-  router_rows_kernel<CL>
-      <<<grid, 256, router_rows_smem(hidden, experts + (has_shared ? 1 : 0), CL), stream>>>(
-          x, w, rows, hidden, experts, has_shared, top_k, renorm, ids, probs, shared_gate);
+  launch_early(router_rows_kernel<CL>, grid, 256,
+               router_rows_smem(hidden, experts + (has_shared ? 1 : 0), CL), stream, x, w, rows,
+               hidden, experts, has_shared, top_k, renorm, ids, probs, shared_gate);
   return static_cast<int>(cudaGetLastError());
 }
 
@@ -378,6 +385,8 @@ __global__ void __launch_bounds__(THREADS) moe_plan_kernel(
   __shared__ int red[2][WARPS], warp_count[WARPS];
   const int e = blockIdx.x, experts = gridDim.x, tid = threadIdx.x;
   const int warp = tid >> 5, lane = tid & 31;
+  grid_wait();
+  grid_release();
   for (int i = tid; i < experts; i += THREADS) hist[i] = 0;
   __syncthreads();
   // a warp walks one contiguous run of assignments, 32 at a time
@@ -451,6 +460,8 @@ __global__ void __launch_bounds__(128) moe_scatter_kernel(
     const int* __restrict__ slots, int top_k, const int8_t* __restrict__ q8,
     const float* __restrict__ scale, int K, int8_t* __restrict__ q8_sorted,
     float* __restrict__ scale_sorted) {
+  grid_wait();
+  grid_release();
   const int row = blockIdx.x;
   const int* sl = slots + static_cast<size_t>(row) * top_k;
   if (SPARSE && __ldg(sl) < 0) return;
@@ -472,6 +483,8 @@ __global__ void __launch_bounds__(256) moe_combine_kernel(
     const float* __restrict__ probs, int top_k, const __half* __restrict__ shared_out,
     const float* __restrict__ shared_gate, __half* __restrict__ out, int hidden,
     const PeerOut peers) {
+  grid_wait();
+  grid_release();
   const int row = blockIdx.x;
   for (int i = threadIdx.x * 8; i < hidden; i += blockDim.x * 8) {
     float acc[8] = {0, 0, 0, 0, 0, 0, 0, 0};
@@ -530,11 +543,11 @@ static int launch_dispatch(const int* ids, int rows, int top_k, int base_expert,
         kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem));
     if (e != cudaSuccess) return static_cast<int>(e);
   }
-  kernel<<<experts, rows * top_k >= 4096 ? 1024 : 256, smem, stream>>>(
-      ids, rows * top_k, base_expert, counts, offsets, tiles, meta, max_tiles, slots);
+  launch_early(kernel, experts, rows * top_k >= 4096 ? 1024 : 256, smem, stream, ids,
+               rows * top_k, base_expert, counts, offsets, tiles, meta, max_tiles, slots);
   if (q8 != nullptr)                                // nullptr: only the slot numbering is wanted
-    (top_k == 1 ? moe_scatter_kernel<true> : moe_scatter_kernel<false>)<<<rows, 128, 0, stream>>>(
-        slots, top_k, q8, scale, K, q8_sorted, scale_sorted);
+    launch_early(top_k == 1 ? moe_scatter_kernel<true> : moe_scatter_kernel<false>, rows, 128, 0,
+                 stream, slots, top_k, q8, scale, K, q8_sorted, scale_sorted);
   return static_cast<int>(cudaGetLastError());
 }
 
@@ -562,7 +575,8 @@ int orinfer_router_topk(const __half* x, const __half* w, int rows, int hidden, 
                     ((rows >= 256 && rows <= 640) || (rows > 1100 && rows < 1900)));
   const int cl = hidden <= 2048 ? 4 : 8;
   if (!few && rows >= ROUTER_MANY && hidden % (cl * 128) == 0 && hidden / cl >= 384 &&
-      hidden / cl <= 512 && total <= ROUTER_TILES * 8 && router_rows_smem(hidden, total, cl) <= 220 * 1024 &&
+      hidden / cl <= 512 && total <= ROUTER_TILES * 8 &&
+      router_rows_smem(hidden, total, cl) <= 220 * 1024 &&
       runtime_ensure_init() == cudaSuccess)
     return (cl == 4 ? launch_router_rows<4> : launch_router_rows<8>)(
         x, w, rows, hidden, experts, has_shared, top_k, renorm, ids, probs, shared_gate, stream);
@@ -579,8 +593,8 @@ int orinfer_router_topk(const __half* x, const __half* w, int rows, int hidden, 
     ORINFER_ROUTER(3, 8);
 #undef ORINFER_ROUTER
   }
-  router_topk_kernel<<<rows, 256, (experts + 1) * sizeof(float), stream>>>(
-      x, w, hidden, experts, has_shared, top_k, renorm, ids, probs, shared_gate);
+  launch_early(router_topk_kernel, rows, 256, (experts + 1) * sizeof(float), stream, x, w, hidden,
+               experts, has_shared, top_k, renorm, ids, probs, shared_gate);
   return static_cast<int>(cudaGetLastError());
 }
 
@@ -641,8 +655,8 @@ int orinfer_moe_combine(const __half* expert_out, const int* slots, const float*
                         __half* out, int hidden, cudaStream_t stream) {
   if (rows <= 0) return 0;
   if (hidden % 8) return -1;
-  moe_combine_kernel<<<rows, 256, 0, stream>>>(expert_out, slots, probs, top_k, shared_out,
-                                               shared_gate, out, hidden, PeerOut{});
+  launch_early(moe_combine_kernel, rows, 256, 0, stream, expert_out, slots, probs, top_k,
+               shared_out, shared_gate, out, hidden, PeerOut{});
   return static_cast<int>(cudaGetLastError());
 }
 

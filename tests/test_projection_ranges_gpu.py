@@ -175,3 +175,52 @@ def test_fused_projection_forms_equal_separate_kernels(dev, fmt, m, n, k):
         out = torch.empty_like(want)
         assert F.qgemv_fused(pre, x, None, None, signs, codes, ws, fmt, n, k, m, out=out)
         assert torch.equal(out, want)
+
+
+@pytest.mark.parametrize("fmt", ["w8", "q4", "q2"])
+@pytest.mark.parametrize("m", [1, 8, 40, 300])
+def test_kernels_that_start_early_keep_the_stream_order(dev, fmt, m):
+    """Row preparations and projections one behind the other, each reading what the one before wrote
+    and overwriting what an earlier one read, weights copied right before their use: eagerly without
+    a wait and in a graph, against the same calls with a wait after each."""
+    from orinfer_b200.ops import functional as F
+    g = torch.Generator().manual_seed(m)
+    k, n = 1024, 2048
+    up, ups, _ = _int_weight(fmt, n, k, g)
+    down, downs, _ = _int_weight(fmt, k, n // 2, g)
+    banks = [t.to(dev) for t in (up, ups, down, downs)]
+    live = [torch.empty_like(t) for t in banks]
+    x0 = torch.randn(m, k, generator=g).half().to(dev)
+    x, gu = torch.empty_like(x0), torch.empty(m, n, dtype=torch.float16, device=dev)
+    norm = torch.ones(k, dtype=torch.float16, device=dev)
+    q8, s8 = torch.empty(m, k, dtype=torch.int8, device=dev), torch.empty(m, device=dev)
+    qm = torch.empty(m, n // 2, dtype=torch.int8, device=dev)
+
+    def chain(wait):
+        step = torch.cuda.synchronize if wait else (lambda: None)
+        x.copy_(x0)
+        for i in range(4):
+            for to, bank in zip(live, banks):
+                to.copy_(bank.roll(i, 0) if bank.dim() > 1 else bank)
+            step()
+            F.act_prep(x, None, norm, None, q_out=q8, scale_out=s8)
+            step()
+            F.qgemm(q8, s8, live[0], live[1], fmt, n, out=gu)
+            step()
+            F.act_prep(gu, None, None, None, swiglu=True, q_out=qm, scale_out=s8)
+            step()
+            F.qgemm(qm, s8, live[2], live[3], fmt, k, out=x)
+            step()
+
+    chain(True)
+    want = x.clone()
+    assert bool(want.isfinite().all())
+    for _ in range(10):
+        chain(False)
+        assert torch.equal(x, want)
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph):
+        chain(False)
+    for _ in range(10):
+        graph.replay()
+        assert torch.equal(x, want)
