@@ -1223,7 +1223,7 @@ int orinfer_gdn_scan(const __half* qkv, const float* ab, const float* a_log, con
     static const int slot = runtime_new_slot();
     if (const int e = runtime_allow_smem(slot, gdn_chunk_kernel, sizeof(ChunkSmem))) return e;
     // Not early: its few long CTAs would gather, two to an SM, where the kernel before ends first
-    // (convolution, scan and norm of two runs of 1050 rows 260 us, 245 so; two of 1500 357 and 335).
+    // (the mixer of two runs of 1050 rows 260 us, 245 so; of two of 1500 rows 357 and 335).
     gdn_chunk_kernel<<<dim3(hv * 2, n_segs), CHUNK_THREADS, sizeof(ChunkSmem), stream>>>(
         qkv, conv_dim, ab, a_log, dt_bias, sg, row_slot, row_pos, hk, hv, state, out);
   }
