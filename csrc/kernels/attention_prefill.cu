@@ -14,7 +14,10 @@
 //   * eight warps per tile own two threads per query row, each with half of the step's keys: they
 //     read S from TMEM, apply scale and the causal mask, and write P as FP16 over their half of S,
 //     where the second MMA reads it as its A operand.  The two meet once per step, for the row's
-//     maximum.  P is relative to the row's running maximum, so its largest weight is exactly 1 and
+//     maximum, and hand over the sum of the weights, which are added in the order of the keys
+//     (sums of their own per half would save 7 % of 4096 rows and 4 to 10 % of short chunks, and
+//     move FP16 outputs by a step, which the INT8 rows of the next projection make a code step).
+//     P is relative to the row's running maximum, so its largest weight is exactly 1 and
 //     O is rescaled whenever a row of the warp finds a larger score;
 //   * warp 0 loads the Q tiles once with a 3-D TMA (d, head, position).
 // With one tile S is double buffered instead.  Head size 256 has room for no more (Q 64 KB, two K
@@ -24,15 +27,15 @@
 //
 // A step of two tiles is a chain per tile (softmax, P V, Q K^T of the next step) and two of them
 // hide each other only in part: 5500 cycles for 128 keys with one softmax thread per row and the
-// MMAs issued inside a branch on the lane, 5000 with two threads, about 4400 since the whole warp
-// runs the issuing loop.  The tensor core needs 2050 of them, the exponentials as many.
+// MMAs issued inside a branch on the lane, about 4700 with two threads and a whole warp in the
+// issuing loop.  The tensor core needs 2050 of them, the exponentials as many.
 // One 4096-token chunk, 32 / 8 heads of 128: 377 us with one tile per CTA and P in shared memory,
-// 244 with two tiles and P in TMEM, 213 with two threads per row, 194 now (709 TFLOP/s causal);
-// 512 tokens 18.3 -> 15.3 -> 13.8 us, 17 tokens 10.8 -> 8.5 -> 7.7.  A reference that follows the
+// 243 with two tiles and P in TMEM, 206 with two threads per row and a whole issuing warp (667
+// TFLOP/s causal); 512 tokens 19 -> 14 us, 64 behind 1000 29 -> 22.  A reference that follows the
 // maximum only when it lags by 2^8 saves another tenth (fewer rescales of O) but rounds the largest
 // weights in FP16: the error against 64 bits grows by 1.8 % there and by 3.7 % for 500 rows behind
-// 1000.  Chunks of 777 and 646 rows behind 3000 positions, 16 / 2 gated heads of 256: 354 -> 284 ->
-// 244 with K and V freed apart, 227 now (180 CTAs: 1.2 waves).
+// 1000.  Chunks of 777 and 646 rows behind 3000 positions, 16 / 2 gated heads of 256: 354 -> 276 ->
+// 244 with K and V freed apart, 223 now (180 CTAs: 1.2 waves).
 // Output is O / sum, optionally times sigmoid(gate), in FP16.  Replaces the prefill
 // configurations of causal_attention_int8 and dequantize_attention_kv
 // (kernels/cuda/model/attention_rows.py:61-276, kernels/cuda/model/kv_int8.py:210-247).
@@ -60,7 +63,10 @@ struct Smem {
   static constexpr int V_OFF = K_OFF + 2 * NSUB * KSUB;  // two V buffers
   static constexpr int BAR_OFF = V_OFF + 2 * NSUB * KSUB;
   static constexpr int MAX_OFF = BAR_OFF + 256;          // [NQ][2 steps][2 halves][128] row maxima
-  static constexpr int TOTAL = MAX_OFF + NQ * 4 * TILE * 4 + 1024;
+  static constexpr int SUM_OFF = MAX_OFF + NQ * 4 * TILE * 4;   // [NQ][128] sums of first halves
+  static constexpr int PAIR_OFF = SUM_OFF + NQ * TILE * 4;      // [NQ][QUADS][128], see `pair`
+  static constexpr int QUADS = KT == 64 ? 0 : D == 128 && NQ == 2 ? 7 : 8;
+  static constexpr int TOTAL = PAIR_OFF + NQ * QUADS * TILE * 16 + 1024;
   static_assert(TOTAL <= 227 * 1024, "exceeds the shared memory of one CTA");
 };
 
@@ -156,7 +162,8 @@ __global__ void __launch_bounds__(Smem<D, NQ>::THREADS, 1) attn_prefill_kernel(
   uint64_t* o_done = bars + 9;        // [2] O += PV finished (per tile)
   uint64_t* k_free = bars + 11;       // [2] the last MMA that read K buffer b finished
   uint64_t* v_free = bars + 13;       // [2] the same for V
-  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 15);
+  uint64_t* sum_ready = bars + 15;    // [NQ][4] sums of the first halves of 32 rows
+  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 15 + 4 * NQ);
 
   const int warp = warp_same(threadIdx.x >> 5), lane = threadIdx.x & 31;
   grid_wait();
@@ -190,6 +197,7 @@ __global__ void __launch_bounds__(Smem<D, NQ>::THREADS, 1) attn_prefill_kernel(
       mbar_init(&k_free[b], 1);
       mbar_init(&v_free[b], 1);
     }
+    for (int b = 0; b < 4 * NQ; ++b) mbar_init(&sum_ready[b], 1);
     mbar_fence_init();
     prefetch_tmap(&tmap_q);
   }
@@ -380,6 +388,13 @@ __global__ void __launch_bounds__(Smem<D, NQ>::THREADS, 1) attn_prefill_kernel(
     auto meet = [&]() {                                     // the two warps of these rows
       asm volatile("bar.sync %0, 64;" ::"r"(1 + q * 4 + quad) : "memory");
     };
+    // A row's weights are added up in the order of its keys: the thread of the second half goes on
+    // where that of the first one ended.  It does so when P is on its way; until then it keeps the
+    // sums of two weights, four to a quad, in registers or (two tiles) most of them in shared
+    // memory.
+    float* first_sum = reinterpret_cast<float*>(smem + L::SUM_OFF) + q * TILE + row;
+    float4* quads = reinterpret_cast<float4*>(smem + L::PAIR_OFF) + q * L::QUADS * TILE + row;
+    uint64_t* handed = &sum_ready[q * 4 + quad];
     float m_run = -INFINITY, l_run = 0.f;
     bool ok = true;
     for (int j = 0; j < steps; ++j) {
@@ -424,16 +439,21 @@ __global__ void __launch_bounds__(Smem<D, NQ>::THREADS, 1) attn_prefill_kernel(
       const float m_tile = fmaxf(slot[0], slot[TILE]) * scale;      // -inf stays -inf
       const float m_new = fmaxf(m_run, m_tile);
       const float corr = m_new == -INFINITY ? 1.f : ex2(m_run - m_new);
-      // pass 2: probabilities -> FP16 over the scores already read, row sum
+      // pass 2: probabilities -> FP16 over the scores already read; their sum, or its terms
       float l_tile = 0.f;
+      float4 kept[KH / 8 > L::QUADS ? KH / 8 - L::QUADS : 1];
+      auto quad_of = [&](int i) -> float4& {
+        return i < L::QUADS ? quads[i * TILE] : kept[i < L::QUADS ? 0 : i - L::QUADS];
+      };
       auto weigh = [&](int c0) {
         uint32_t packed[16];
+        float pair[16];
         if (full_warp) {
 #pragma unroll
           for (int i = 0; i < 32; i += 2) {
             const float p0 = ex2(fmaf(__uint_as_float(r[i]), scale, -m_new));
             const float p1 = ex2(fmaf(__uint_as_float(r[i + 1]), scale, -m_new));
-            l_tile += p0 + p1;
+            pair[i / 2] = p0 + p1;
             const __half2 hp = __floats2half2_rn(p0, p1);
             packed[i / 2] = *reinterpret_cast<const uint32_t*>(&hp);
           }
@@ -444,18 +464,31 @@ __global__ void __launch_bounds__(Smem<D, NQ>::THREADS, 1) attn_prefill_kernel(
             float p1 = ex2(fmaf(__uint_as_float(r[i + 1]), scale, -m_new));
             if (key0 + c0 + i > q_pos) p0 = 0.f;
             if (key0 + c0 + i + 1 > q_pos) p1 = 0.f;
-            l_tile += p0 + p1;
+            pair[i / 2] = p0 + p1;
             const __half2 hp = __floats2half2_rn(p0, p1);
             packed[i / 2] = *reinterpret_cast<const uint32_t*>(&hp);
           }
         }
         tmem_st_32x16(tmem_sj + c0 / 2, packed);
+        if (half == 0) {
+#pragma unroll
+          for (int i = 0; i < 16; ++i) l_tile += pair[i];
+        } else {
+#pragma unroll
+          for (int i = 0; i < 16; i += 4)
+            quad_of((c0 + 2 * i) / 8) = make_float4(pair[i], pair[i + 1], pair[i + 2], pair[i + 3]);
+        }
       };
       weigh(0);
       if (KH == 64) {
         tmem_ld_32x32(tmem_sj + 32, r);
         tc_wait_ld();
         weigh(32);
+      }
+      if (half == 0) {
+        *first_sum = l_tile;
+        __syncwarp();
+        if (lane == 0) mbar_arrive(handed);
       }
       // O holds steps 0..j-1 once PV of step j-1 is done.  Waited for at every step, so that no
       // wait is ever two phases away from its barrier; NQ = 2: it is done, QK ran after it.
@@ -476,23 +509,31 @@ __global__ void __launch_bounds__(Smem<D, NQ>::THREADS, 1) attn_prefill_kernel(
         }
       }
       tc_wait_st();
-      l_run = l_run * corr + l_tile;
       m_run = m_new;
       tc_fence_before();
       __syncwarp();
       if (lane == 0) mbar_arrive(&p_ready[sb]);
+      if (half == 1) {
+        ok = mbar_wait(handed, j & 1, status, STATUS_EPILOGUE_WAIT, 0x200 | j);
+        ok = __all_sync(0xffffffffu, ok);
+        l_tile = *first_sum;
+#pragma unroll
+        for (int i = 0; i < KH / 8; ++i) {
+          const float4 v = quad_of(i);
+          l_tile = (((l_tile + v.x) + v.y) + v.z) + v.w;
+        }
+        l_run = l_run * corr + l_tile;
+      }
     }
     if (ok && steps > 0) {
       ok = mbar_wait(&o_done[q], (steps - 1) & 1, status, STATUS_EPILOGUE_WAIT, 0x300);
       ok = __all_sync(0xffffffffu, ok);
     }
-    // both halves of the row sum
-    float* sums = row_max + (steps & 1) * 2 * TILE;
-    sums[half * TILE] = l_run;
+    if (half == 1) *first_sum = l_run;
     meet();
     if (ok && steps > 0) {
       tc_fence_after();
-      const float l_all = sums[0] + sums[TILE];
+      const float l_all = *first_sum;
       const float inv = l_all > 0.f ? 1.f / l_all : 0.f;
       const size_t orow = static_cast<size_t>(ch.row_start + first + p_rel) * qh + head;
 #pragma unroll 1

@@ -224,3 +224,30 @@ def test_attention_prefill_largest_weight_is_exact(dev, d, kvh, qh, rows):
         # one FP16 rounding of the output (2^-11); scores of up to 2^4 in FP32, a sum of up to 600
         # FP32 weights and their exponentials: below 2^-17
         assert bool(((out[r].double() - ref).abs() <= ref.abs() * (2.0 ** -11 + 2.0 ** -17)).all()), r
+
+
+@pytest.mark.parametrize("d,kvh,qh", [(64, 2, 4), (128, 1, 5), (256, 1, 8)])
+@pytest.mark.parametrize("rows", [128, 5200])
+def test_attention_prefill_adds_weights_in_the_order_of_keys(dev, d, kvh, qh, rows):
+    """Two keys of weight 1 at the start of a step and about 2^-26 for the others, which vanish one
+    pair after the other in a sum of 2 (ulp 2^-22) and in FP16 weights: the sum is exactly 2 and the
+    output the FP16 tie (1 + 1 + 3 * 2^-10) / 2, to even upwards.  Sums of their own over the later
+    keys would reach 2^-21 and more, and tip the tie downwards."""
+    from orinfer_b200.ops import functional as F
+    step = 64 if d == 256 else 128                             # keys per step
+    pages = (rows + 127) // 128
+    table = torch.arange(1, pages + 1, dtype=torch.int32, device=dev)[None]
+    kc = torch.zeros(pages + 1, 128, kvh, d, dtype=torch.int8, device=dev)
+    vc = torch.ones_like(kc)
+    ks = torch.full((pages + 1, 128, kvh, d // 64), 2.0, dtype=torch.float16, device=dev)
+    vs = torch.ones_like(ks)
+    # scores are q . k / sqrt(d), weights their exponentials: q . k of -26 * ln 2 * sqrt(d)
+    kc[:, :, :, 0] = -round(26 * math.log(2) * math.sqrt(d) / (4 if d == 256 else 2))
+    kc[1, :2, :, 0] = 0
+    vs[1, 0], vs[1, 1] = 1 + 2.0 ** -10, 1 + 2.0 ** -9
+    q = torch.zeros(rows, qh, d, dtype=torch.float16, device=dev)
+    q[:, :, 0] = 2 if d == 256 else 1
+    out = torch.empty(rows, qh * d, dtype=torch.float16, device=dev)
+    chunk = torch.tensor([[0, rows, 0, 0]], dtype=torch.int32, device=dev)
+    assert F.attention_prefill(q, None, chunk, rows, table, kc, vc, ks, vs, out=out)
+    assert bool((out[1:step] == 1 + 2.0 ** -9).all())
