@@ -113,6 +113,10 @@ __device__ __forceinline__ bool mbar_wait_abortable(uint64_t* bar, uint32_t pari
   }
 }
 
+// The answer of a bounded wait for a warp that goes on as a whole: each lane gets its own, and lanes
+// that gave up must not part from the others ahead of a __syncwarp or of a signal for all of them.
+__device__ __forceinline__ bool warp_all(bool ok) { return __all_sync(0xffffffffu, ok) != 0; }
+
 // ---------------------------------------------------------------- overlapping launches
 // A kernel started by launch_early may be resident before the kernels ahead of it on its stream
 // have ended.  Every CTA of it calls grid_wait before it touches memory that they write or read and

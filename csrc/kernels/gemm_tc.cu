@@ -308,7 +308,7 @@ __global__ void __launch_bounds__(THREADS, 1) qgemm_tc_kernel(
         const int s = kb % SB;
         // the codes of this phase are only requested after the tensor core released the
         // stage, so their arrival also means the INT8 tile of this stage may be overwritten
-        ok = mbar_wait(&c_full[s], (kb / SB) & 1, status, STATUS_DECODE_WAIT, kb);
+        ok = warp_all(mbar_wait(&c_full[s], (kb / SB) & 1, status, STATUS_DECODE_WAIT, kb));
         if (!ok) break;
         const unsigned char* cs = code_s + s * L::CODE_BYTES;
         unsigned char* bs = b_s + s * L::B_BYTES;
@@ -974,8 +974,10 @@ __global__ void __launch_bounds__(THREADS, 1) qgemm_ps_kernel(
       if (FMT != 0) {
         for (int kb = 0; ok && kb < kbs; ++kb, ++cc, ++cb) {
           const uint32_t sc = cc % SC, sb = cb % SBD;
-          ok = PS_WAIT(&c_full[sc], (cc / SC) & 1, STATUS_DECODE_WAIT, kb);
-          if (ok) ok = PS_WAIT(&b_empty[sb], ((cb / SBD) & 1) ^ 1, STATUS_DECODE_WAIT, 0x800 | kb);
+          ok = warp_all(PS_WAIT(&c_full[sc], (cc / SC) & 1, STATUS_DECODE_WAIT, kb));
+          if (ok)
+            ok = warp_all(
+                PS_WAIT(&b_empty[sb], ((cb / SBD) & 1) ^ 1, STATUS_DECODE_WAIT, 0x800 | kb));
           if (!ok) break;
           const unsigned char* cs = code_s + sc * L::CODE_BYTES;
           unsigned char* bs = b_s + sb * L::B_BYTES;
@@ -1380,8 +1382,10 @@ __global__ void __launch_bounds__(THREADS, 1) qgemm_pair_kernel(
       if (FMT != 0) {
         for (int kb = 0; ok && kb < kbs; ++kb, ++cc, ++cb) {
           const uint32_t sc = cc % SC, sb = cb % SBD;
-          ok = PR_WAIT(&c_full[sc], (cc / SC) & 1, STATUS_DECODE_WAIT, kb);
-          if (ok) ok = PR_WAIT(&b_empty[sb], ((cb / SBD) & 1) ^ 1, STATUS_DECODE_WAIT, 0x800 | kb);
+          ok = warp_all(PR_WAIT(&c_full[sc], (cc / SC) & 1, STATUS_DECODE_WAIT, kb));
+          if (ok)
+            ok = warp_all(
+                PR_WAIT(&b_empty[sb], ((cb / SBD) & 1) ^ 1, STATUS_DECODE_WAIT, 0x800 | kb));
           if (!ok) break;
           const unsigned char* cs = code_s + sc * L::CODE_BYTES;
           unsigned char* bs = b_s + sb * L::B_BYTES;

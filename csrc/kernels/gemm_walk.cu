@@ -415,7 +415,7 @@ __global__ void __launch_bounds__(Layout<FMT, MT>::THREADS, 1) qgemm_walk_kernel
     uint2 word[2];
     auto read = [&]() {
       const uint32_t sc = cr % SC;
-      ok = WALK_WAIT(&c_full[sc], (cr / SC) & 1, STATUS_DECODE_WAIT, cr & 0x7ff);
+      ok = warp_all(WALK_WAIT(&c_full[sc], (cr / SC) & 1, STATUS_DECODE_WAIT, cr & 0x7ff));
       const unsigned char* cs = code_s + sc * L::CODES;
 #pragma unroll
       for (int i = 0; i < 2; ++i) {
@@ -432,7 +432,8 @@ __global__ void __launch_bounds__(Layout<FMT, MT>::THREADS, 1) qgemm_walk_kernel
       if (cr < all) read();
       const uint32_t sb = cb % S;
       if (ok)
-        ok = WALK_WAIT(&empty[sb], ((cb / S) & 1) ^ 1, STATUS_DECODE_WAIT, 0x800 | (cb & 0x7ff));
+        ok = warp_all(WALK_WAIT(&empty[sb], ((cb / S) & 1) ^ 1, STATUS_DECODE_WAIT,
+                                0x800 | (cb & 0x7ff)));
       if (!ok) break;
       unsigned char* bs = smem + sb * L::STAGE + MT * TILE;
 #pragma unroll

@@ -1,0 +1,61 @@
+"""Rules that the kernels' source has to keep and that no run on a GPU would show broken."""
+import re
+from pathlib import Path
+
+import pytest
+
+KERNELS = Path(__file__).resolve().parents[1] / "csrc" / "kernels"
+SOURCES = sorted(p for p in KERNELS.iterdir() if p.suffix in (".cu", ".cuh"))
+WAIT = re.compile(r"\b(?:mbar_wait|mbar_wait_abortable|PS_WAIT|PR_WAIT|WALK_WAIT)\(")
+
+
+def _code(path):
+    """The source without comments, directives and macro bodies, its lines kept."""
+    text = re.sub(r"/\*.*?\*/", lambda m: "\n" * m[0].count("\n"), path.read_text(), flags=re.S)
+    lines, macro = [], False
+    for line in (re.sub(r"//.*", "", line) for line in text.split("\n")):
+        skip = macro or line.lstrip().startswith("#")
+        macro = skip and line.rstrip().endswith("\\")
+        lines.append("" if skip else line)
+    return "\n".join(lines)
+
+
+def _statements(code):
+    """(line, text, headers of the blocks around it) of every statement."""
+    blocks, start, depth = [], 0, 0
+    for i, ch in enumerate(code):
+        if ch in "()":
+            depth += 1 if ch == "(" else -1
+        elif ch == "{" and (depth == 0 or code[:i].rstrip().endswith(")")):
+            blocks.append((code[start:i].strip(), depth))
+            start, depth = i + 1, 0
+        elif ch == "}" and depth == 0:
+            if blocks:
+                depth = blocks.pop()[1]
+            start = i + 1
+        elif ch == ";" and depth == 0:
+            text = code[start:i]
+            lead = len(text) - len(text.lstrip())
+            yield code.count("\n", 0, start + lead) + 1, text.strip(), [b for b, _ in blocks]
+            start = i + 1
+
+
+@pytest.mark.parametrize("path", SOURCES, ids=lambda p: p.name)
+def test_warps_agree_on_waits_that_may_give_up(path):
+    """A bounded wait is answered lane by lane.  Where a warp goes on as a whole (it meets at a
+    __syncwarp, votes, or signals for all its lanes), lanes that gave up and lanes that did not must
+    not part: the answers are voted on, in the statement of the wait or in the next one."""
+    one = re.compile(r"lane == 0|threadIdx\.x == 0|tid == 0|\bt == 0|leader")
+    code, wrong = _code(path), []
+    statements = list(_statements(code))
+    for n, (line, text, blocks) in enumerate(statements):
+        if not WAIT.search(text) or "inline__" in text:
+            continue
+        if any(one.search(b) for b in blocks) or one.search(text.split("wait")[0]):
+            continue
+        follows = statements[n + 1][1] if n + 1 < len(statements) else ""
+        # the drain at a role's end asks for no answer
+        answered = re.search(r"=|return|if", WAIT.split(text)[0].rsplit(")", 1)[-1])
+        if answered and "_all_sync(" not in text + follows and "warp_all(" not in text + follows:
+            wrong.append(f"{path.name}:{line}: {' '.join(text.split())[:90]}")
+    assert not wrong, "\n".join(wrong)
