@@ -113,9 +113,21 @@ __device__ __forceinline__ bool mbar_wait_abortable(uint64_t* bar, uint32_t pari
   }
 }
 
-// The answer of a bounded wait for a warp that goes on as a whole: each lane gets its own, and lanes
-// that gave up must not part from the others ahead of a __syncwarp or of a signal for all of them.
+// The answer of a bounded wait for a warp that goes on as a whole: each lane gets its own, and
+// lanes that gave up must not part from the others ahead of a __syncwarp or of a signal for all.
 __device__ __forceinline__ bool warp_all(bool ok) { return __all_sync(0xffffffffu, ok) != 0; }
+
+// A warp hands a slab of a ring back to the bulk copies that refill it.  A load that is still
+// queued when its warp arrives is no use of the slab that the arrival waits for, and the copy
+// writes through another proxy, which waits for nothing else: a warp that loads words now, uses
+// them a round later and arrives between can get the next slab's bytes (seen in the walking GEMM,
+// a few weight rows in ten thousand).  So the arrival depends on `seen`, a value that cannot be
+// there before every word that this lane has read is in a register: the warp votes on a bit of it,
+// and the vote decides which of two lanes arrives.
+__device__ __forceinline__ void hand_back(uint64_t* bar, uint32_t seen) {
+  const unsigned votes = __ballot_sync(0xffffffffu, seen & 1u);
+  if ((threadIdx.x & 31u) == (votes & 1u)) mbar_arrive(bar);
+}
 
 // ---------------------------------------------------------------- overlapping launches
 // A kernel started by launch_early may be resident before the kernels ahead of it on its stream

@@ -454,13 +454,9 @@ __global__ void __launch_bounds__(Layout<FMT, MT>::THREADS, 1) qgemm_walk_kernel
       __syncwarp();
       if (lane == 0) mbar_arrive(&full[sb]);
       ++cb;
-      // The slab of the words just read goes back.  Reads may still be queued when their warp
-      // signals (handed back without more, slabs were refilled too early, and a few weight rows in
-      // ten thousand came out wrong), so the signal depends on every word: either lane will do.
-      const uint32_t mix = (word[0].x ^ word[0].y) + (word[1].x ^ word[1].y);
-      const int from = __any_sync(0xffffffffu, mix == 0x9e3779b9u) ? 1 : 0;
-      for (; cf < cr; ++cf)
-        if (lane == from) mbar_arrive(&c_empty[cf % SC]);
+      // the slab of the words just read, which the next round uses, goes back (see hand_back)
+      const uint32_t seen = word[0].x ^ word[0].y ^ word[1].x ^ word[1].y;
+      for (; cf < cr; ++cf) hand_back(&c_empty[cf % SC], seen);
     }
   }
 #undef WALK_WAIT

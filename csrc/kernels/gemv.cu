@@ -891,8 +891,8 @@ __global__ void __launch_bounds__((1 + STREAM_MAX) * 32) w8_stream_kernel(
       mma_i8_16832(acc[0], x.x, y.x, x.y, y.y, b.x, b.y);
       mma_i8_16832(acc[1], x.z, y.z, x.w, y.w, b.z, b.w);
     }
-    __syncwarp();
-    if (lane == 0) mbar_arrive(&empty[s]);
+    // every word of the tile went into one of these two chains of sums
+    hand_back(&empty[s], static_cast<uint32_t>(acc[0][0] ^ acc[1][0]));
 #pragma unroll
     for (int e = 0; e < 4; ++e) {
       const int m = 2 * t + (e & 1), at = n + (e >> 1) * 8;

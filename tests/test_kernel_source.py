@@ -59,3 +59,12 @@ def test_warps_agree_on_waits_that_may_give_up(path):
         if answered and "_all_sync(" not in text + follows and "warp_all(" not in text + follows:
             wrong.append(f"{path.name}:{line}: {' '.join(text.split())[:90]}")
     assert not wrong, "\n".join(wrong)
+
+
+@pytest.mark.parametrize("name", ["gemm_walk.cu", "gemv.cu"])
+def test_rings_that_bulk_copies_refill_are_handed_back_behind_their_reads(name):
+    """A warp that reads a slab into registers gives it back through hand_back, whose arrival
+    depends on what was read."""
+    code = _code(KERNELS / name)
+    assert re.search(r"hand_back\(&(c_)?empty\[", code)
+    assert not re.search(r"mbar_arrive\(&(c_)?empty\[", code)

@@ -62,7 +62,7 @@ def test_streamed_int8_projections_are_exact(dev, m, n, k):
     a = torch.randint(-127, 128, (m, k), generator=g, device=dev, dtype=torch.int8)
     sa = torch.rand(m, generator=g, device=dev) * 0.05 + 1e-3
     want = _scaled(a, sa, w, ws)
-    for f32 in (False, True):
+    for f32 in (False, True) * 5:            # repeated: stages are refilled while others run
         out = F.qgemm(a, sa, w, ws, "w8", n, out_f32=f32, path=1)
         assert torch.equal(out, want if f32 else want.half())
 
