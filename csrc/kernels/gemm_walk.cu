@@ -38,8 +38,10 @@ constexpr int TILE = 128 * 128;                    // bytes of an INT8 tile
 constexpr int FIRST_EPI = 4, EPI_WARPS = 8, FIRST_DEC = FIRST_EPI + EPI_WARPS, DEC_WARPS = 16;
 constexpr int PITCH = 80;                          // staged row piece: 32 columns FP16 + pad
 
-// A stage of the ring is a k-block of MT activation tiles and one weight tile, with one barrier for
-// "filled" (copies and decode warps) and one for "multiplied".
+// A stage of the ring is a k-block of MT activation tiles and one weight tile, with a barrier each
+// for "activations landed", "weights there" (copied, or decoded) and "multiplied".  Only its own
+// copies complete a barrier that a copying warp waits for before it leaves: had the activations one
+// with the decode warps, and had those given up, that wait would run to its limit for every stage.
 template <int FMT, int MT>
 struct Layout {
   static constexpr int THREADS = (FMT == 0 ? FIRST_DEC : FIRST_DEC + DEC_WARPS) * 32;
@@ -121,7 +123,8 @@ __global__ void __launch_bounds__(Layout<FMT, MT>::THREADS, 1) qgemm_walk_kernel
   float* scale_s = reinterpret_cast<float*>(smem + L::SCALE_OFF);
   int2* list = reinterpret_cast<int2*>(smem + L::LIST_OFF);    // first row, expert and rows
   uint64_t* bars = reinterpret_cast<uint64_t*>(smem + L::BAR_OFF);
-  uint64_t* full = bars;                       // [S]    stage filled
+  uint64_t* a_full = bars;                     // [S]    activations of a stage landed
+  uint64_t* full = a_full + S;                 // [S]    its weights landed or decoded
   uint64_t* empty = full + S;                  // [S]    its MMAs retired
   uint64_t* c_full = empty + S;                // [SC]   packed codes landed
   uint64_t* c_empty = c_full + SC;             // [SC]   every decode warp has read them
@@ -130,7 +133,7 @@ __global__ void __launch_bounds__(Layout<FMT, MT>::THREADS, 1) qgemm_walk_kernel
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(acc_empty + BUFS);
   volatile int* abort_w = reinterpret_cast<volatile int*>(tmem_slot + 1);
   int* hits = reinterpret_cast<int*>(tmem_slot + 2);           // [32]
-  static_assert((2 * S + 2 * SC + 2 * BUFS) * 8 + 8 + 128 <= 512, "barriers");
+  static_assert((3 * S + 2 * SC + 2 * BUFS) * 8 + 8 + 128 <= 512, "barriers");
 
   const int tid = threadIdx.x, warp = warp_same(tid >> 5), lane = tid & 31;
   if (p.tiles != nullptr) grid_wait();          // the table
@@ -187,7 +190,8 @@ __global__ void __launch_bounds__(Layout<FMT, MT>::THREADS, 1) qgemm_walk_kernel
 
   if (tid == 0) {
     for (int s = 0; s < S; ++s) {
-      mbar_init(&full[s], FMT == 0 ? 2 : 1 + DEC_WARPS);
+      mbar_init(&a_full[s], 1);
+      mbar_init(&full[s], FMT == 0 ? 1 : DEC_WARPS);
       mbar_init(&empty[s], 1);
     }
     for (int s = 0; s < SC; ++s) {
@@ -230,11 +234,11 @@ __global__ void __launch_bounds__(Layout<FMT, MT>::THREADS, 1) qgemm_walk_kernel
         for (int kb = 0; kb < kblocks; ++kb) {
           ok = WALK_WAIT(&empty[s], phase ^ 1, STATUS_TMA_WAIT, kb);
           if (!ok) break;
-          mbar_expect_tx(&full[s], T.mt_act * TILE);
+          mbar_expect_tx(&a_full[s], T.mt_act * TILE);
 #pragma unroll
           for (int i = 0; i < MT; ++i)
             if (i < T.mt_act)
-              tma_load_2d(smem + s * L::STAGE + i * TILE, &tmap_a, &full[s], kb * BK,
+              tma_load_2d(smem + s * L::STAGE + i * TILE, &tmap_a, &a_full[s], kb * BK,
                           T.m0 + i * BM);
           ++issued;
           if (++s == S) {
@@ -245,7 +249,7 @@ __global__ void __launch_bounds__(Layout<FMT, MT>::THREADS, 1) qgemm_walk_kernel
       }
       // no copy of ours is in flight when the CTA ends
       for (uint32_t c = issued > S ? issued - S : 0; c < issued; ++c)
-        mbar_wait(&full[c % S], (c / S) & 1, status, STATUS_TMA_WAIT, 0x4000);
+        mbar_wait(&a_full[c % S], (c / S) & 1, status, STATUS_TMA_WAIT, 0x4000);
     }
   } else if (warp == 2) {
     if (lane == 0) {
@@ -294,10 +298,11 @@ __global__ void __launch_bounds__(Layout<FMT, MT>::THREADS, 1) qgemm_walk_kernel
       const uint32_t buf = it % BUFS, acc = tmem_base + buf * MT * BN;
       // the epilogue has read out what these accumulators held before
       if (it >= BUFS)
-        ok = __all_sync(0xffffffffu, WALK_WAIT(&acc_empty[buf], (it / BUFS - 1) & 1,
-                                               STATUS_MMA_WAIT, 0x3000));
+        ok = warp_all(
+            WALK_WAIT(&acc_empty[buf], (it / BUFS - 1) & 1, STATUS_MMA_WAIT, 0x3000));
       for (int kb = 0; ok && kb < kblocks; ++kb) {
-        ok = __all_sync(0xffffffffu, WALK_WAIT(&full[s], phase, STATUS_MMA_WAIT, kb));
+        ok = warp_all(WALK_WAIT(&full[s], phase, STATUS_MMA_WAIT, 0x2000 | kb) &&
+                      WALK_WAIT(&a_full[s], phase, STATUS_MMA_WAIT, kb));
         if (!ok) break;
         tc_fence_after();
         const uint64_t ad = ring + static_cast<uint64_t>(s * L::STAGE / 16);

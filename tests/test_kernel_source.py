@@ -68,3 +68,18 @@ def test_rings_that_bulk_copies_refill_are_handed_back_behind_their_reads(name):
     code = _code(KERNELS / name)
     assert re.search(r"hand_back\(&(c_)?empty\[", code)
     assert not re.search(r"mbar_arrive\(&(c_)?empty\[", code)
+
+
+@pytest.mark.parametrize("path", SOURCES, ids=lambda p: p.name)
+def test_copies_in_flight_are_waited_for_on_barriers_of_their_own(path):
+    """Before a copying warp leaves, it waits for what it has in flight, without a look at the abort
+    word: on barriers with one arrival, its own, so that the bytes alone complete them."""
+    code = _code(path)
+    for kernel in re.split(r"__global__", code)[1:]:
+        counts = dict(re.findall(r"mbar_init\(&?(\w+)(?:\[\w+\])?, (.+?)\);", kernel))
+        names = re.findall(r"(?:for \([^;]*;[^;]*;[^;{]*\)|if \(.*\))\s+mbar_wait\(&(\w+)\[", kernel)
+        for name in names:
+            alias = re.search(r"uint64_t\* " + name + r" = (.+?);", kernel)
+            owners = [name] if name in counts else re.findall(r"\w+", alias[1])
+            for count in (counts[o] for o in owners if o in counts):
+                assert count == "1" or re.fullmatch(r"FMT == 0 \? 1 : .+", count), (name, count)
