@@ -37,12 +37,12 @@ struct RowScales {
       const unsigned short* u = reinterpret_cast<const unsigned short*>(p);
 #pragma unroll
       for (int i = 0; i < (G + 1) / 2; ++i)
-        w[i] = static_cast<uint32_t>(__ldg(u + 2 * i)) |
-               (G == 1 ? 0u : static_cast<uint32_t>(__ldg(u + 2 * i + 1)) << 16);
+        w[i] = static_cast<uint32_t>(u[2 * i]) |
+               (G == 1 ? 0u : static_cast<uint32_t>(u[2 * i + 1]) << 16);
     } else if (G == 2) {
-      w[0] = __ldg(reinterpret_cast<const uint32_t*>(p));
+      w[0] = *reinterpret_cast<const uint32_t*>(p);
     } else {
-      const uint2 v = __ldg(reinterpret_cast<const uint2*>(p));
+      const uint2 v = *reinterpret_cast<const uint2*>(p);
       w[0] = v.x;
       w[(G + 1) / 2 - 1] = v.y;
     }
@@ -122,10 +122,9 @@ __device__ __forceinline__ void cp_async16(uint32_t smem, const void* gmem) {
 template <int D, bool WIDE, bool APART>
 __global__ void __launch_bounds__(
     ATTN_WARPS * 32, D == 64 && !APART ? 3 : AttnTile<D>::MIN_CTAS) attn_rows_kernel(
-    const __half* __restrict__ q, const __half* __restrict__ gate, const int* __restrict__ row_req,
-    const int* __restrict__ row_pos, const int* __restrict__ page_table, int max_pages,
-    const int8_t* __restrict__ kc, const int8_t* __restrict__ vc, const __half* __restrict__ ks,
-    const __half* __restrict__ vs, __half* __restrict__ out, int qh, int kvh, int splits,
+    const __half* q, const __half* gate, const int* row_req, const int* row_pos,
+    const int* page_table, int max_pages, const int8_t* kc, const int8_t* vc, const __half* ks,
+    const __half* vs, __half* __restrict__ out, int qh, int kvh, int splits,
     float* __restrict__ scratch, int rep, int apart_keys) {
   constexpr int G = AttnTile<D>::G, KB = AttnTile<D>::KB;
   constexpr int NT = KB / 8, UT = KB / 16;         // 8-key score tiles, 16-key value tiles
@@ -162,8 +161,8 @@ __global__ void __launch_bounds__(
       for (int i = 0; i < 8; ++i) w[i] = 0u;
       if (g < rep) {
         if (WIDE) {
-          *reinterpret_cast<uint4*>(w) = __ldg(reinterpret_cast<const uint4*>(p));
-          *reinterpret_cast<uint4*>(w + 4) = __ldg(reinterpret_cast<const uint4*>(p) + 1);
+          *reinterpret_cast<uint4*>(w) = *reinterpret_cast<const uint4*>(p);
+          *reinterpret_cast<uint4*>(w + 4) = reinterpret_cast<const uint4*>(p)[1];
         } else {
 #pragma unroll
           for (int i = 0; i < 8; ++i) w[i] = pack_half2(p[2 * i], p[2 * i + 1]);
@@ -425,9 +424,8 @@ __global__ void __launch_bounds__(
 }
 
 template <int D>
-__global__ void attn_merge_kernel(const float* __restrict__ scratch,
-                                  const __half* __restrict__ gate, __half* __restrict__ out,
-                                  int qh, int splits) {
+__global__ void attn_merge_kernel(
+    const float* scratch, const __half* gate, __half* __restrict__ out, int qh, int splits) {
   grid_wait();
   grid_release();
   const int row = blockIdx.x, head = blockIdx.y;

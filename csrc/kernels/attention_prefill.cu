@@ -141,11 +141,10 @@ struct Chunk {            // one prefill chunk of one request
 
 template <int D, int NQ>
 __global__ void __launch_bounds__(Smem<D, NQ>::THREADS, 1) attn_prefill_kernel(
-    const __grid_constant__ CUtensorMap tmap_q, const Chunk* __restrict__ chunks,
-    const int* __restrict__ page_table, int max_pages, const int8_t* __restrict__ kc,
-    const int8_t* __restrict__ vc, const __half* __restrict__ ks, const __half* __restrict__ vs,
-    const __half* __restrict__ gate, __half* __restrict__ out, int qh, int kvh, int rep,
-    int num_pages, int* status) {
+    const __grid_constant__ CUtensorMap tmap_q, const Chunk* chunks, const int* page_table,
+    int max_pages, const int8_t* kc, const int8_t* vc, const __half* ks, const __half* vs,
+    const __half* gate, __half* __restrict__ out, int qh, int kvh, int rep, int num_pages,
+    int* status) {
   using L = Smem<D, NQ>;
   constexpr int NSUB = L::NSUB, KT = L::KT;
   constexpr int GROUPS = D / 64;
@@ -311,11 +310,11 @@ __global__ void __launch_bounds__(Smem<D, NQ>::THREADS, 1) attn_prefill_kernel(
       for (int it = 0; it < ITERS; ++it) {
         const size_t at = static_cast<size_t>(it) * rows;
         if (k) {
-          kraw[it] = __ldg(reinterpret_cast<const uint4*>(kp + at * D));
+          kraw[it] = *reinterpret_cast<const uint4*>(kp + at * D);
           ksc[it] = ksp[at * GROUPS];
         }
         if (v) {
-          vraw[it] = __ldg(reinterpret_cast<const uint4*>(vp + at * D));
+          vraw[it] = *reinterpret_cast<const uint4*>(vp + at * D);
           vsc[it] = it * (DQ / CPK) < live ? vsp[at * GROUPS] : __half(0.f);
         }
       }

@@ -133,9 +133,14 @@ __device__ __forceinline__ void hand_back(uint64_t* bar, uint32_t seen) {
 // A kernel started by launch_early may be resident before the kernels ahead of it on its stream
 // have ended.  Every CTA of it calls grid_wait before it touches memory that they write or read and
 // before it may exit (a grid that ended early would release its successors too soon); only what is
-// constant from start-up on, such as the decode tables, is read ahead of it.  grid_release lets the
-// next kernel become resident in turn; kernels that allocate tensor memory call it after that, so
-// that a successor cannot take what they need.
+// constant from start-up on, such as the decode tables, is read ahead of it.  What a kernel in
+// front may have written is loaded by plain loads through pointers without __restrict__: the
+// read-only path (__ldg, and what the compiler makes of const __restrict__) is promised only for
+// data that nobody writes while the kernel lives, and such a load may move ahead of the wait.  That
+// goes for weights too, which a program may copy between two launches.  (It cost nothing: every
+// call measured took the same time within 1 %.)  grid_release lets the next kernel become resident
+// in turn; kernels that allocate tensor memory call it after that, so that a successor cannot take
+// what they need.
 __device__ __forceinline__ void grid_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 __device__ __forceinline__ void grid_release() {
   asm volatile("griddepcontrol.launch_dependents;" ::: "memory");

@@ -18,9 +18,9 @@ namespace cg = cooperative_groups;
 namespace orinfer {
 
 // ------------------------------------------------------------------ embedding
-__global__ void embed_w8_kernel(const int* __restrict__ ids, const int8_t* __restrict__ table,
-                                const __half* __restrict__ scales, __half* __restrict__ out,
-                                int hidden, int vocab, int* status) {
+__global__ void embed_w8_kernel(
+    const int* ids, const int8_t* table, const __half* scales, __half* __restrict__ out, int hidden,
+    int vocab, int* status) {
   grid_wait();
   grid_release();
   const int row = blockIdx.x;
@@ -71,10 +71,10 @@ __device__ __forceinline__ int a8_code_of(float v, float scale) {
 
 template <bool SWIGLU, int CL>
 __global__ void __launch_bounds__(512) act_prep_kernel(
-    const __half* __restrict__ x, float* __restrict__ resid, const __half* __restrict__ norm_w,
-    const int8_t* __restrict__ signs, int8_t* __restrict__ q_out, float* __restrict__ scale_out,
-    __half* __restrict__ y_out, int K, float eps, int zero_centered, InboxIn in, int* status,
-    AgOut ag, int rows, const int* __restrict__ row_limit, int row_base) {
+    const __half* x, float* resid, const __half* norm_w, const int8_t* signs,
+    int8_t* __restrict__ q_out, float* __restrict__ scale_out, __half* __restrict__ y_out, int K,
+    float eps, int zero_centered, InboxIn in, int* status, AgOut ag, int rows, const int* row_limit,
+    int row_base) {
   extern __shared__ float rowbuf_raw[];
   __shared__ float red[32];
   __shared__ float cl_slot[2];
@@ -286,10 +286,9 @@ struct RegRows {
 };
 template <bool SWIGLU, int NB>
 __global__ void __launch_bounds__(RegRows<NB>::THREADS, RegRows<NB>::CTAS) act_prep_regs_kernel(
-    const __half* __restrict__ x, float* __restrict__ resid, const __half* __restrict__ norm_w,
-    const int8_t* __restrict__ signs, int8_t* __restrict__ q_out, float* __restrict__ scale_out,
-    __half* __restrict__ y_out, int nblk, float eps, int zero_centered,
-    const int* __restrict__ row_limit) {
+    const __half* x, float* resid, const __half* norm_w, const int8_t* signs,
+    int8_t* __restrict__ q_out, float* __restrict__ scale_out, __half* __restrict__ y_out, int nblk,
+    float eps, int zero_centered, const int* row_limit) {
   const int row = blockIdx.x, warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   grid_wait();
   grid_release();
@@ -419,8 +418,9 @@ __global__ void ag_wait_kernel(AgIn in, int rows, int* status) {
 }
 
 // ------------------------------------------------------------------ RoPE tables
-__global__ void rope_table_kernel(const int* __restrict__ positions, float* __restrict__ cosb,
-                                  float* __restrict__ sinb, int rows, int half_dim, double theta) {
+__global__ void rope_table_kernel(
+    const int* positions, float* __restrict__ cosb, float* __restrict__ sinb, int rows,
+    int half_dim, double theta) {
   grid_wait();
   grid_release();
   const int idx = blockIdx.x * blockDim.x + threadIdx.x;
@@ -439,11 +439,9 @@ __global__ void rope_table_kernel(const int* __restrict__ positions, float* __re
 // Input row layout: q heads (D each, or 2D = query|gate when GATED), then K, then V.
 template <int D, bool GATED>
 __global__ void __launch_bounds__(256) qk_rope_kv_kernel(
-    const __half* __restrict__ qkv, const __half* __restrict__ wq, const __half* __restrict__ wk,
-    const float* __restrict__ cosb, const float* __restrict__ sinb,
-    const int* __restrict__ row_req, const int* __restrict__ row_pos,
-    const int* __restrict__ page_table, int max_pages, int qh, int kvh, float eps,
-    int zero_centered, __half* __restrict__ q_out, __half* __restrict__ gate_out,
+    const __half* qkv, const __half* wq, const __half* wk, const float* cosb, const float* sinb,
+    const int* row_req, const int* row_pos, const int* page_table, int max_pages, int qh, int kvh,
+    float eps, int zero_centered, __half* __restrict__ q_out, __half* __restrict__ gate_out,
     int8_t* __restrict__ kcache, int8_t* __restrict__ vcache, __half* __restrict__ kscale,
     __half* __restrict__ vscale, int num_pages, int* status) {
   constexpr int HALF = D / 2;

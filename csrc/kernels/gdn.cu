@@ -23,10 +23,8 @@ struct Segment {
 };
 
 // ---------------------------------------------------------------- small projection
-__global__ void __launch_bounds__(256) small_proj_kernel(const __half* __restrict__ x,
-                                                         const __half* __restrict__ w,
-                                                         float* __restrict__ out, int hidden,
-                                                         int n) {
+__global__ void __launch_bounds__(256) small_proj_kernel(
+    const __half* x, const __half* w, float* __restrict__ out, int hidden, int n) {
   grid_wait();
   grid_release();
   const int row = blockIdx.x, warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -100,10 +98,9 @@ __global__ void __launch_bounds__(D) gdn_conv_kernel(
 // 2100 rows x 8192 channels: 89 -> 25 us; 64 rows: 7.9 -> 5.0 us.
 template <int D, int R>
 __global__ void __launch_bounds__(256) gdn_conv_vec_kernel(
-    const __half* __restrict__ x, int x_stride, const __half* __restrict__ weight,
-    const __half* __restrict__ hist, const int* __restrict__ row_first,
-    const int* __restrict__ row_slot, const int* __restrict__ row_pos, int rows, int conv_dim,
-    int qk_channels, __half* __restrict__ y) {
+    const __half* x, int x_stride, const __half* weight, const __half* hist, const int* row_first,
+    const int* row_slot, const int* row_pos, int rows, int conv_dim, int qk_channels,
+    __half* __restrict__ y) {
   constexpr int LANES = D / 8;
   grid_wait();
   grid_release();
@@ -114,14 +111,14 @@ __global__ void __launch_bounds__(256) gdn_conv_vec_kernel(
   uint4 wr[4];
 #pragma unroll
   for (int i = 0; i < 4; ++i)
-    wr[i] = __ldg(reinterpret_cast<const uint4*>(weight + static_cast<size_t>(c) * 4) + i);
+    wr[i] = reinterpret_cast<const uint4*>(weight + static_cast<size_t>(c) * 4)[i];
   const __half* wh = reinterpret_cast<const __half*>(wr);
   uint4 win[4];                                    // rows row-3 .. row (as loaded)
 #pragma unroll
   for (int j = 0; j < 3; ++j) {
     const int src = row0 - 3 + j;
-    win[j + 1] = src >= 0 ? __ldg(reinterpret_cast<const uint4*>(
-                                x + static_cast<size_t>(src) * x_stride + c))
+    win[j + 1] = src >= 0 ? *reinterpret_cast<const uint4*>(
+                                x + static_cast<size_t>(src) * x_stride + c)
                           : make_uint4(0, 0, 0, 0);
   }
 #pragma unroll
@@ -130,7 +127,7 @@ __global__ void __launch_bounds__(256) gdn_conv_vec_kernel(
     if (row >= rows) break;
 #pragma unroll
     for (int j = 0; j < 3; ++j) win[j] = win[j + 1];
-    win[3] = __ldg(reinterpret_cast<const uint4*>(x + static_cast<size_t>(row) * x_stride + c));
+    win[3] = *reinterpret_cast<const uint4*>(x + static_cast<size_t>(row) * x_stride + c);
     const int first = row_first[row];
     uint4 tap[3] = {win[0], win[1], win[2]};
     if (row - first < 3) {                         // rows before the run come from its history
@@ -175,14 +172,9 @@ __global__ void __launch_bounds__(256) gdn_conv_vec_kernel(
 // blocks); VEC channels per thread.  (One CTA per segment with 2-byte accesses took 21 us for
 // 64 segments, this form 2.9 us.)
 template <int VEC>
-__global__ void __launch_bounds__(256) gdn_history_kernel(const __half* __restrict__ x,
-                                                          int x_stride,
-                                                          const Segment* __restrict__ segs,
-                                                          const int* __restrict__ row_slot,
-                                                          const int* __restrict__ row_pos,
-                                                          int conv_dim,
-                                                          __half* __restrict__ hist,
-                                                          const int* __restrict__ accepted) {
+__global__ void __launch_bounds__(256) gdn_history_kernel(
+    const __half* x, int x_stride, const Segment* segs, const int* row_slot, const int* row_pos,
+    int conv_dim, __half* hist, const int* accepted) {
   grid_wait();
   grid_release();
   Segment s = segs[blockIdx.x];
@@ -226,10 +218,8 @@ __global__ void __launch_bounds__(256) gdn_history_kernel(const __half* __restri
 // gdn_scan_split_kernel below.)
 template <int D, int DC>
 __global__ void __launch_bounds__(256) gdn_scan_kernel(
-    const __half* __restrict__ qkv, int conv_dim, const float* __restrict__ ab,
-    const float* __restrict__ a_log, const float* __restrict__ dt_bias,
-    const Segment* __restrict__ segs, const int* __restrict__ row_slot,
-    const int* __restrict__ row_pos, int hk, int hv, float* __restrict__ state,
+    const __half* qkv, int conv_dim, const float* ab, const float* a_log, const float* dt_bias,
+    const Segment* segs, const int* row_slot, const int* row_pos, int hk, int hv, float* state,
     float* __restrict__ out, float* __restrict__ factors, int long_rows) {
   // factors != nullptr: a verification pass.  The state is NOT written back; instead every
   // step records (decay, k[D], delta[D]) so that gdn_commit can replay exactly the accepted
@@ -346,10 +336,8 @@ __device__ __forceinline__ void cp_async16(void* smem, const void* gmem) {
 
 template <int D>
 __global__ void __launch_bounds__(256) gdn_scan_split_kernel(
-    const __half* __restrict__ qkv, int conv_dim, const float* __restrict__ ab,
-    const float* __restrict__ a_log, const float* __restrict__ dt_bias,
-    const Segment* __restrict__ segs, const int* __restrict__ row_slot,
-    const int* __restrict__ row_pos, int hk, int hv, float* __restrict__ state,
+    const __half* qkv, int conv_dim, const float* ab, const float* a_log, const float* dt_bias,
+    const Segment* segs, const int* row_slot, const int* row_pos, int hk, int hv, float* state,
     float* __restrict__ out, float* __restrict__ factors, int long_rows) {
   constexpr int DC = 32, SPLIT = D / DC, PARTS = 8, ROWS = D / PARTS, T = SCAN_STEPS;
   constexpr int CH = D / 4 + DC / 8;                 // 16-byte units of one staged row
@@ -1038,9 +1026,8 @@ __global__ void __launch_bounds__(256) gdn_commit_kernel(
 // sum of squares is built as in the warp form below, so a row gives the same bits through both.
 template <int D>
 __global__ void __launch_bounds__(D) gdn_gated_norm_kernel(
-    const float* __restrict__ o, const __half* __restrict__ z, int z_stride,
-    const __half* __restrict__ w, float eps, int sigmoid_gate, int hv,
-    __half* __restrict__ y) {
+    const float* o, const __half* z, int z_stride, const __half* w, float eps, int sigmoid_gate,
+    int hv, __half* __restrict__ y) {
   grid_wait();
   grid_release();
   const int row = blockIdx.x, h = blockIdx.y, d = threadIdx.x;
@@ -1069,9 +1056,8 @@ __global__ void __launch_bounds__(D) gdn_gated_norm_kernel(
 // rows 1.9 against 2.0, 64 rows 2.1 against 2.0.
 template <int D>
 __global__ void __launch_bounds__(256) gdn_gated_norm_warp_kernel(
-    const float* __restrict__ o, const __half* __restrict__ z, int z_stride,
-    const __half* __restrict__ w, float eps, int sigmoid_gate, int hv, long long items,
-    __half* __restrict__ y) {
+    const float* o, const __half* z, int z_stride, const __half* w, float eps, int sigmoid_gate,
+    int hv, long long items, __half* __restrict__ y) {
   constexpr int V = D / 32;
   struct __align__(V * 2) Half {
     __half h[V];

@@ -103,10 +103,9 @@ struct GroupDesc {
 template <int FMT, bool OUT_F32, int MT, int NB, bool GROUPED>
 __global__ void __launch_bounds__(THREADS, 1) qgemm_tc_kernel(
     const __grid_constant__ CUtensorMap tmap_a, const __grid_constant__ CUtensorMap tmap_b,
-    const unsigned char* __restrict__ w, const float* __restrict__ a_scale,
-    const __half* __restrict__ w_scale, void* __restrict__ out, int M, int N, int K,
-    const E8pTables* __restrict__ tables, int* status, PeerOut po, GroupDesc grp, AgIn ag,
-    int* __restrict__ partial, int* __restrict__ tickets, int n_begin, int n_end, int probe) {
+    const unsigned char* w, const float* a_scale, const __half* w_scale, void* __restrict__ out,
+    int M, int N, int K, const E8pTables* __restrict__ tables, int* status, PeerOut po,
+    GroupDesc grp, AgIn ag, int* partial, int* tickets, int n_begin, int n_end, int probe) {
   // probe (timing experiments only; results are then meaningless): bit 0 = issue no MMAs,
   // bit 1 = copy no operands (the loaders only signal), bit 2 = decode nothing, bit 3 = the
   // epilogue stores nothing to global memory, bit 4 = no epilogue at all, bit 5 = no k-blocks,
@@ -1475,9 +1474,8 @@ int launch_pair(const int8_t* a, const float* a_scale, const void* w, const __ha
 // One thread per 8 columns; the arithmetic is the GEMM epilogue's, so a split GEMM returns
 // bit for bit what the unsplit one does.
 __global__ void __launch_bounds__(256) splitk_finalize_kernel(
-    const int* __restrict__ partial, int splits, const float* __restrict__ a_scale,
-    const __half* __restrict__ w_scale, __half* __restrict__ out, int M, int N, PeerOut po,
-    int ag_scales, int n_begin, int width) {
+    const int* partial, int splits, const float* a_scale, const __half* w_scale,
+    __half* __restrict__ out, int M, int N, PeerOut po, int ag_scales, int n_begin, int width) {
   grid_wait();
   grid_release();
   const int groups = width / 8;

@@ -340,12 +340,12 @@ __global__ void __launch_bounds__(Layout<FMT, MT>::THREADS, 1) qgemm_walk_kernel
 #pragma unroll
       for (int s = 0; s < MT; ++s) {
         const int m = T.m0 + s * BM + row;
-        sa[s] = m < T.m_limit ? __ldg(p.a_scale + m) : 0.f;
+        sa[s] = m < T.m_limit ? p.a_scale[m] : 0.f;
       }
       float2 w2 = make_float2(0.f, 0.f);
       if (nw + lane * 2 < p.n_end)
-        w2 = __half22float2(__ldg(reinterpret_cast<const __half2*>(
-            p.w_scale + static_cast<size_t>(T.expert) * p.N + nw + lane * 2)));
+        w2 = __half22float2(*reinterpret_cast<const __half2*>(
+            p.w_scale + static_cast<size_t>(T.expert) * p.N + nw + lane * 2));
       __syncwarp();
       reinterpret_cast<float2*>(ws)[lane] = w2;
       ok = WALK_WAIT(&acc_full[buf], (it / BUFS) & 1, STATUS_EPILOGUE_WAIT, 0);

@@ -15,8 +15,7 @@ namespace orinfer {
 constexpr int W8_WARPS = 8;
 
 template <int MT>
-__device__ __forceinline__ void stage_activations(int8_t* dst, const int8_t* __restrict__ a, int M,
-                                                  int K) {
+__device__ __forceinline__ void stage_activations(int8_t* dst, const int8_t* a, int M, int K) {
   const int chunks = MT * K / 16;
   for (int c = threadIdx.x; c < chunks; c += blockDim.x) {
     const int m = (c * 16) / K;
@@ -136,29 +135,27 @@ struct GemvEarly {
   float scale;
   __half w_scale;
   __device__ __forceinline__ void load(const E8pTables* __restrict__ tables,
-                                       const int8_t* __restrict__ a,
-                                       const float* __restrict__ a_scale,
-                                       const __half* __restrict__ ws, int n_count, int M, int K,
-                                       bool plain, int tid) {
+                                       const int8_t* a, const float* a_scale, const __half* ws,
+                                       int n_count, int M, int K, bool plain, int tid) {
     if (FMT != 0) fill.load(tables, tid);
     grid_wait();
     grid_release();
-    w_scale = tid < n_count ? __ldg(ws + tid) : __half(0.f);
+    w_scale = tid < n_count ? ws[tid] : __half(0.f);
     scale = 0.f;
     if (plain) {
 #pragma unroll
       for (int i = 0; i < ROWS; ++i) {
         const int c = tid + i * THREADS;
-        rows[i] = c * 16 < M * K ? __ldg(reinterpret_cast<const int4*>(a) + c)
+        rows[i] = c * 16 < M * K ? reinterpret_cast<const int4*>(a)[c]
                                  : make_int4(0, 0, 0, 0);
       }
-      if (tid < M) scale = __ldg(a_scale + tid);
+      if (tid < M) scale = a_scale[tid];
     }
   }
   // the tables, the outputs' scales (sw) and zeroed sums
   __device__ __forceinline__ void store(unsigned char* smem, float* sw,
-                                        const __half* __restrict__ ws, int n_count, int* sums,
-                                        int n_sums, int tid) const {
+                                        const __half* ws, int n_count, int* sums, int n_sums,
+                                        int tid) const {
     if (FMT != 0) fill.store(smem, tid);
     if (tid < n_count) sw[tid] = __half2float(w_scale);
     for (int i = tid + THREADS; i < n_count; i += THREADS) sw[i] = __half2float(ws[i]);
@@ -170,8 +167,8 @@ struct GemvEarly {
 // rows, or by the row preparation of fz.pre, one row at a time in fbuf [K].
 template <int FMT, int MT, int THREADS, bool DP4A>
 __device__ __forceinline__ void gemv_rows(int8_t* act, int* asum, float* scale_s, float* fbuf,
-                                          float* red, float* blk_sum, const int8_t* __restrict__ a,
-                                          const float* __restrict__ a_scale, int M, int K,
+                                          float* red, float* blk_sum, const int8_t* a,
+                                          const float* a_scale, int M, int K,
                                           const GemvFuse& fz,
                                           const GemvEarly<FMT, THREADS>& early) {
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
@@ -328,7 +325,7 @@ __device__ __forceinline__ void gemv_finish(int* acc_s, const int* asum, const f
                                             int* last_flag, const float* sw_s,
                                             void* __restrict__ out, int M, int N, int out_f32,
                                             const PeerOut& po, int ll_seq, int np, int k_parts,
-                                            int n_base, int n_count, int* __restrict__ ws,
+                                            int n_base, int n_count, int* ws,
                                             const GemvFuse& fz) {
   const int tid = threadIdx.x;
   const PeerOut* peer = po.tp > 0 ? &po : nullptr;
@@ -420,10 +417,9 @@ __device__ __forceinline__ void gemv_finish(int* acc_s, const int* asum, const f
 
 template <int FMT, int MT>
 __global__ void __launch_bounds__(GEMV_THREADS, 1) qgemv_kernel(
-    const int8_t* __restrict__ a, const float* __restrict__ a_scale, const void* __restrict__ w,
-    const __half* __restrict__ w_scale, void* __restrict__ out, int M, int N, int K, int out_f32,
-    const E8pTables* __restrict__ tables, PeerOut po, int n_parts, int k_parts, int max_groups,
-    int* __restrict__ ws, GemvFuse fz) {
+    const int8_t* a, const float* a_scale, const void* w, const __half* w_scale,
+    void* __restrict__ out, int M, int N, int K, int out_f32, const E8pTables* __restrict__ tables,
+    PeerOut po, int n_parts, int k_parts, int max_groups, int* ws, GemvFuse fz) {
   constexpr int THREADS = GEMV_THREADS;
   constexpr int ROWS = 16, DEPTH = FMT == 2 ? 4 : 2;     // rows of a group, units in flight
   using Unit = GemvUnit<FMT>;
@@ -476,18 +472,18 @@ __global__ void __launch_bounds__(GEMV_THREADS, 1) qgemv_kernel(
       if (FMT == 0) {
         const uint4* p = reinterpret_cast<const uint4*>(w) + static_cast<size_t>(n) * (K / 16) +
                          lkb * 8 + t;
-        const uint4 x = __ldg(p), y = __ldg(p + 4);
+        const uint4 x = *p, y = p[4];
         v.w[h][0] = x.x; v.w[h][1] = x.y; v.w[h][2] = x.z; v.w[h][3] = x.w;
         v.w[h][4 % Unit::WORDS] = y.x; v.w[h][5 % Unit::WORDS] = y.y;
         v.w[h][6 % Unit::WORDS] = y.z; v.w[h][7 % Unit::WORDS] = y.w;
       } else if (FMT == 1) {
         const uint4 x =
-            __ldg(reinterpret_cast<const uint4*>(w) + (static_cast<size_t>(lkb) * N + n) * 4 + t);
+            reinterpret_cast<const uint4*>(w)[(static_cast<size_t>(lkb) * N + n) * 4 + t];
         v.w[h][0] = x.x; v.w[h][1] = x.y;
         v.w[h][2 % Unit::WORDS] = x.z; v.w[h][3 % Unit::WORDS] = x.w;
       } else {
         const uint2 x =
-            __ldg(reinterpret_cast<const uint2*>(w) + (static_cast<size_t>(lkb) * N + n) * 4 + t);
+            reinterpret_cast<const uint2*>(w)[(static_cast<size_t>(lkb) * N + n) * 4 + t];
         v.w[h][0] = x.x; v.w[h][1] = x.y;
       }
     }
@@ -595,10 +591,9 @@ struct Dp4a {
 
 template <int FMT, int MT>
 __global__ void __launch_bounds__(Dp4a<FMT, MT>::THREADS, 1) e8p_dp4a_kernel(
-    const int8_t* __restrict__ a, const float* __restrict__ a_scale, const uint4* __restrict__ w,
-    const __half* __restrict__ w_scale, void* __restrict__ out, int M, int N, int K, int out_f32,
-    const E8pTables* __restrict__ tables, PeerOut po, int n_parts, int k_parts, int max_groups,
-    int* __restrict__ ws, GemvFuse fz) {
+    const int8_t* a, const float* a_scale, const uint4* w, const __half* w_scale,
+    void* __restrict__ out, int M, int N, int K, int out_f32, const E8pTables* __restrict__ tables,
+    PeerOut po, int n_parts, int k_parts, int max_groups, int* ws, GemvFuse fz) {
   constexpr int THREADS = Dp4a<FMT, MT>::THREADS, DEPTH = 4;
   constexpr int ROWS = FMT == 1 ? 8 : 16;        // output rows of a group
   constexpr int LPR = 32 / ROWS;                 // lanes per row, 16 bytes of codes each
@@ -640,7 +635,7 @@ __global__ void __launch_bounds__(Dp4a<FMT, MT>::THREADS, 1) e8p_dp4a_kernel(
     uint4 v = make_uint4(0, 0, 0, 0);
     if (uu < u_hi) {
       const int n = min(lg * ROWS + row, N - 1);
-      v = __ldg(w + (static_cast<size_t>(lkb) * N + n) * LPR + part);
+      v = w[(static_cast<size_t>(lkb) * N + n) * LPR + part];
       if (++lkb == kb_hi) {
         lkb = kb_lo;
         ++lg;
@@ -757,9 +752,8 @@ inline bool w8_by_rows(int M, int N, int K) {
 
 template <int MT>
 __global__ void __launch_bounds__(W8_WARPS * 32) w8_gemv_kernel(
-    const int8_t* __restrict__ a, const float* __restrict__ a_scale, const int8_t* __restrict__ w,
-    const __half* __restrict__ w_scale, void* __restrict__ out, int M, int N, int K, int out_f32,
-    PeerOut po) {
+    const int8_t* a, const float* a_scale, const int8_t* w, const __half* w_scale,
+    void* __restrict__ out, int M, int N, int K, int out_f32, PeerOut po) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
   grid_wait();
   grid_release();
@@ -776,7 +770,7 @@ __global__ void __launch_bounds__(W8_WARPS * 32) w8_gemv_kernel(
   for (int m = 0; m < MT; ++m) acc[m] = 0;
 #pragma unroll 4
   for (int k = lane * 16; k < K; k += 512) {
-    const int4 wv = __ldg(reinterpret_cast<const int4*>(wr + k));
+    const int4 wv = *reinterpret_cast<const int4*>(wr + k);
 #pragma unroll
     for (int m = 0; m < MT; ++m) {
       const int4 av = *reinterpret_cast<const int4*>(act + m * K + k);
@@ -824,9 +818,8 @@ inline bool w8_streams(int M, int N, int K) {
 }
 
 __global__ void __launch_bounds__((1 + STREAM_MAX) * 32) w8_stream_kernel(
-    const int8_t* __restrict__ a, const float* __restrict__ a_scale, const int8_t* __restrict__ w,
-    const __half* __restrict__ w_scale, void* __restrict__ out, int M, int N, int K, int out_f32,
-    int stages, int* status) {
+    const int8_t* a, const float* a_scale, const int8_t* w, const __half* w_scale,
+    void* __restrict__ out, int M, int N, int K, int out_f32, int stages, int* status) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
   __shared__ __align__(8) uint64_t full[STREAM_MAX], empty[STREAM_MAX];
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, g = lane >> 2, t = lane & 3;
@@ -930,11 +923,10 @@ struct ExpertUnit {
 // MIXED takes the tiles of at most most_rows rows and leaves the others to another kernel.
 template <int FMT, bool MIXED>
 __global__ void __launch_bounds__(GEMV_THREADS, 1) qgemv_grouped_kernel(
-    const int8_t* __restrict__ a, const float* __restrict__ a_scale,
-    const unsigned char* __restrict__ w, const __half* __restrict__ w_scale,
+    const int8_t* a, const float* a_scale, const unsigned char* w, const __half* w_scale,
     __half* __restrict__ out, int N, int K, long long bank_bytes,
-    const E8pTables* __restrict__ tables, const int* __restrict__ tiles,
-    const int* __restrict__ meta, int most_rows, int listed) {
+    const E8pTables* __restrict__ tables, const int* tiles, const int* meta, int most_rows,
+    int listed) {
   using W = GemvUnit<FMT>;
   constexpr int NB = 2;                            // eight-row blocks per pass over the weights
   extern __shared__ __align__(16) unsigned char smem_raw[];
@@ -959,7 +951,7 @@ __global__ void __launch_bounds__(GEMV_THREADS, 1) qgemv_grouped_kernel(
     int count = 0;
     for (int base = 0; base < n_tiles; base += GEMV_THREADS) {
       const int at = base + tid;
-      const bool hit = at < n_tiles && __ldg(tiles + at * 4 + 2) <= most_rows;
+      const bool hit = at < n_tiles && tiles[at * 4 + 2] <= most_rows;
       const unsigned ballot = __ballot_sync(0xffffffffu, hit);
       if (lane == 0) hits[warp] = __popc(ballot);
       __syncthreads();
@@ -998,8 +990,8 @@ __global__ void __launch_bounds__(GEMV_THREADS, 1) qgemv_grouped_kernel(
   for (int item = blockIdx.x * (WARPS / ks) + warp / ks; item < items; item += stride) {
     const int at = item / groups, n0 = (item - at * groups) * 16;
     const int tile = MIXED && list != nullptr ? list[at] : at;
-    const int expert = __ldg(tiles + tile * 4), first = __ldg(tiles + tile * 4 + 1);
-    const int rows = __ldg(tiles + tile * 4 + 2);
+    const int expert = tiles[tile * 4], first = tiles[tile * 4 + 1];
+    const int rows = tiles[tile * 4 + 2];
     const unsigned char* bank = w + static_cast<size_t>(expert) * bank_bytes;
     for (int r0 = 0; r0 < rows; r0 += 8 * NB) {
       const int nb = min(NB, (rows - r0 + 7) / 8);
@@ -1016,24 +1008,24 @@ __global__ void __launch_bounds__(GEMV_THREADS, 1) qgemv_grouped_kernel(
           if (FMT == 0) {
             const uint4* p = reinterpret_cast<const uint4*>(bank) +
                              static_cast<size_t>(n) * (K / 16) + kb * 8 + t;
-            const uint4 x = __ldg(p), y = __ldg(p + 4);
+            const uint4 x = *p, y = p[4];
             v.u.w[h][0] = x.x; v.u.w[h][1] = x.y; v.u.w[h][2 % W::WORDS] = x.z;
             v.u.w[h][3 % W::WORDS] = x.w; v.u.w[h][4 % W::WORDS] = y.x;
             v.u.w[h][5 % W::WORDS] = y.y; v.u.w[h][6 % W::WORDS] = y.z;
             v.u.w[h][7 % W::WORDS] = y.w;
           } else if (FMT == 1) {
-            const uint4 x = __ldg(reinterpret_cast<const uint4*>(bank) +
-                                  (static_cast<size_t>(kb) * N + n) * 4 + t);
+            const uint4 x = reinterpret_cast<const uint4*>(
+                bank)[(static_cast<size_t>(kb) * N + n) * 4 + t];
             v.u.w[h][0] = x.x; v.u.w[h][1] = x.y;
             v.u.w[h][2 % W::WORDS] = x.z; v.u.w[h][3 % W::WORDS] = x.w;
           } else {
-            const uint2 x = __ldg(reinterpret_cast<const uint2*>(bank) +
-                                  (static_cast<size_t>(kb) * N + n) * 4 + t);
+            const uint2 x = reinterpret_cast<const uint2*>(
+                bank)[(static_cast<size_t>(kb) * N + n) * 4 + t];
             v.u.w[h][0] = x.x; v.u.w[h][1] = x.y;
           }
         }
-        v.act[0] = __ldg(reinterpret_cast<const uint4*>(arow[0] + kb * 128 + piece0));
-        v.act[1] = __ldg(reinterpret_cast<const uint4*>(arow[0] + kb * 128 + piece1));
+        v.act[0] = *reinterpret_cast<const uint4*>(arow[0] + kb * 128 + piece0);
+        v.act[1] = *reinterpret_cast<const uint4*>(arow[0] + kb * 128 + piece1);
       };
       int acc[NB][4], asum[NB];
 #pragma unroll
@@ -1077,8 +1069,8 @@ __global__ void __launch_bounds__(GEMV_THREADS, 1) qgemv_grouped_kernel(
                 x1 = j & 1 ? p.w : p.y;
               } else {
                 if (b >= nb) break;
-                const uint2 p = __ldg(reinterpret_cast<const uint2*>(
-                    arow[b] + kb * 128 + (j >> 1 ? piece1 : piece0) + (j & 1) * 8));
+                const uint2 p = *reinterpret_cast<const uint2*>(
+                    arow[b] + kb * 128 + (j >> 1 ? piece1 : piece0) + (j & 1) * 8);
                 x0 = p.x;
                 x1 = p.y;
               }

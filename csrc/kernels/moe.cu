@@ -87,9 +87,8 @@ __device__ __forceinline__ void topk_row(float* logits, int row, int experts, in
 
 // General form: one CTA per token row, one warp per expert at a time.
 __global__ void __launch_bounds__(256) router_topk_kernel(
-    const __half* __restrict__ x, const __half* __restrict__ w, int hidden, int experts,
-    int has_shared, int top_k, int renorm, int* __restrict__ ids, float* __restrict__ probs,
-    float* __restrict__ shared_gate) {
+    const __half* x, const __half* w, int hidden, int experts, int has_shared, int top_k,
+    int renorm, int* __restrict__ ids, float* __restrict__ probs, float* __restrict__ shared_gate) {
   extern __shared__ float logits[];                 // [experts + 1]
   grid_wait();
   grid_release();
@@ -137,9 +136,8 @@ constexpr int ROUTER_CL = 8;
 
 template <int MAXT, int WARPS>
 __global__ void __cluster_dims__(ROUTER_CL, 1, 1) __launch_bounds__(WARPS * 32) router_mma_kernel(
-    const __half* __restrict__ x, const __half* __restrict__ w, int rows, int hidden, int experts,
-    int has_shared, int top_k, int renorm, int* __restrict__ ids, float* __restrict__ probs,
-    float* __restrict__ shared_gate) {
+    const __half* x, const __half* w, int rows, int hidden, int experts, int has_shared, int top_k,
+    int renorm, int* __restrict__ ids, float* __restrict__ probs, float* __restrict__ shared_gate) {
   constexpr int CL = ROUTER_CL, ROWS = 16, COLS = MAXT * 8 + 1, OWN = ROWS / CL;
   extern __shared__ float router_smem[];
   float(*part)[ROWS][COLS] = reinterpret_cast<float(*)[ROWS][COLS]>(router_smem);
@@ -163,15 +161,15 @@ __global__ void __cluster_dims__(ROUTER_CL, 1, 1) __launch_bounds__(WARPS * 32) 
   const int k_lo = hidden / WARPS * warp, k_hi = k_lo + hidden / WARPS;
 #pragma unroll 1
   for (int k = k_lo; k < k_hi; k += 32) {
-    const uint4 a = __ldg(reinterpret_cast<const uint4*>(xa + k));
-    const uint4 b = __ldg(reinterpret_cast<const uint4*>(xb + k));
+    const uint4 a = *reinterpret_cast<const uint4*>(xa + k);
+    const uint4 b = *reinterpret_cast<const uint4*>(xb + k);
     uint4 wv[MAXT];
 #pragma unroll
     for (int i = 0; i < MAXT; ++i)
       if (i < nt) {
         const int e = min((t_lo + i) * 8 + g, total - 1);
         const __half* we = w + static_cast<size_t>(e) * hidden + t * 8 + k;
-        wv[i] = __ldg(reinterpret_cast<const uint4*>(we));
+        wv[i] = *reinterpret_cast<const uint4*>(we);
       }
 #pragma unroll
     for (int i = 0; i < MAXT; ++i)
@@ -247,9 +245,8 @@ __device__ __forceinline__ void ldmatrix4(uint32_t (&r)[4], const void* p) {
 
 template <int CL>
 __global__ void __cluster_dims__(CL, 1, 1) __launch_bounds__(256, 1) router_rows_kernel(
-    const __half* __restrict__ x, const __half* __restrict__ w, int rows, int hidden, int experts,
-    int has_shared, int top_k, int renorm, int* __restrict__ ids, float* __restrict__ probs,
-    float* __restrict__ shared_gate) {
+    const __half* x, const __half* w, int rows, int hidden, int experts, int has_shared, int top_k,
+    int renorm, int* __restrict__ ids, float* __restrict__ probs, float* __restrict__ shared_gate) {
   constexpr int ROWS = ROUTER_ROWS, OWN = ROWS / CL, PER = (ROUTER_TILES + 3) / 4;
   extern __shared__ __align__(16) unsigned char router_raw[];
   const int total = experts + (has_shared ? 1 : 0), tiles = (total + 7) / 8;
@@ -377,9 +374,8 @@ static int launch_router_rows(const __half* x, const __half* w, int rows, int hi
 // More threads where there are many assignments to walk (16384 of them: 26 us with 256).
 template <int THREADS>
 __global__ void __launch_bounds__(THREADS) moe_plan_kernel(
-    const int* __restrict__ ids, int assigns, int base_expert, int* __restrict__ counts,
-    int* __restrict__ offsets, int* __restrict__ tiles, int* __restrict__ meta, int max_tiles,
-    int* __restrict__ slots) {
+    const int* ids, int assigns, int base_expert, int* counts, int* offsets, int* tiles, int* meta,
+    int max_tiles, int* slots) {
   extern __shared__ int hist[];                     // [experts]
   constexpr int WARPS = THREADS / 32;
   __shared__ int red[2][WARPS], warp_count[WARPS];
@@ -457,21 +453,20 @@ __global__ void __launch_bounds__(THREADS) moe_plan_kernel(
 // rank go nowhere, and looking first costs 0.2 to 0.5 us of 4 to 7.
 template <bool SPARSE>
 __global__ void __launch_bounds__(128) moe_scatter_kernel(
-    const int* __restrict__ slots, int top_k, const int8_t* __restrict__ q8,
-    const float* __restrict__ scale, int K, int8_t* __restrict__ q8_sorted,
-    float* __restrict__ scale_sorted) {
+    const int* slots, int top_k, const int8_t* q8, const float* scale, int K,
+    int8_t* __restrict__ q8_sorted, float* __restrict__ scale_sorted) {
   grid_wait();
   grid_release();
   const int row = blockIdx.x;
   const int* sl = slots + static_cast<size_t>(row) * top_k;
-  if (SPARSE && __ldg(sl) < 0) return;
+  if (SPARSE && *sl < 0) return;
   const float s = scale[row];
   for (int j = threadIdx.x; j < top_k; j += blockDim.x)
     if (sl[j] >= 0) scale_sorted[sl[j]] = s;
   for (int c = threadIdx.x; c < K / 16; c += blockDim.x) {
     const int4 v = reinterpret_cast<const int4*>(q8 + static_cast<size_t>(row) * K)[c];
     for (int j = 0; j < top_k; ++j) {
-      const int slot = __ldg(sl + j);
+      const int slot = sl[j];
       if (slot >= 0) reinterpret_cast<int4*>(q8_sorted + static_cast<size_t>(slot) * K)[c] = v;
     }
   }
@@ -479,9 +474,8 @@ __global__ void __launch_bounds__(128) moe_scatter_kernel(
 
 // out[row] = fp16( sum_k prob[row,k] * expert_out[slot(row,k)] + gate[row] * shared[row] )
 __global__ void __launch_bounds__(256) moe_combine_kernel(
-    const __half* __restrict__ expert_out, const int* __restrict__ slots,
-    const float* __restrict__ probs, int top_k, const __half* __restrict__ shared_out,
-    const float* __restrict__ shared_gate, __half* __restrict__ out, int hidden,
+    const __half* expert_out, const int* slots, const float* probs, int top_k,
+    const __half* shared_out, const float* shared_gate, __half* __restrict__ out, int hidden,
     const PeerOut peers) {
   grid_wait();
   grid_release();

@@ -77,9 +77,61 @@ def test_copies_in_flight_are_waited_for_on_barriers_of_their_own(path):
     code = _code(path)
     for kernel in re.split(r"__global__", code)[1:]:
         counts = dict(re.findall(r"mbar_init\(&?(\w+)(?:\[\w+\])?, (.+?)\);", kernel))
-        names = re.findall(r"(?:for \([^;]*;[^;]*;[^;{]*\)|if \(.*\))\s+mbar_wait\(&(\w+)\[", kernel)
+        names = re.findall(
+            r"(?:for \([^;]*;[^;]*;[^;{]*\)|if \(.*\))\s+mbar_wait\(&(\w+)\[", kernel)
         for name in names:
             alias = re.search(r"uint64_t\* " + name + r" = (.+?);", kernel)
             owners = [name] if name in counts else re.findall(r"\w+", alias[1])
             for count in (counts[o] for o in owners if o in counts):
                 assert count == "1" or re.fullmatch(r"FMT == 0 \? 1 : .+", count), (name, count)
+
+
+def _closing(code, at):
+    """Index behind the bracket that closes the one at `at`."""
+    pairs, depth = {"(": 1, ")": -1, "{": 1, "}": -1}, 0
+    for i in range(at, len(code)):
+        depth += pairs.get(code[i], 0)
+        if depth == 0:
+            return i + 1
+    raise ValueError(code[at:at + 80])
+
+
+def _functions(code):
+    """(kind, name, parameters, body) of every function of the source."""
+    for word in ("__launch_bounds__", "__cluster_dims__"):
+        while word + "(" in code:
+            at = code.index(word + "(")
+            code = code[:at] + code[_closing(code, at + len(word)):]
+    for m in re.finditer(r"__(global|device)__\s[^;({=]*?(\w+)\(", code):
+        end = _closing(code, m.end() - 1)
+        tail = re.match(r"\s*(const\s*)?\{", code[end:])
+        if tail:                                                   # not a declaration
+            body = end + tail.end() - 1
+            yield m[1], m[2], code[m.end():end - 1], code[body:_closing(code, body)]
+
+
+def test_kernels_that_start_early_load_through_the_coherent_path():
+    """A kernel that is resident while the ones in front of it still write must not read what they
+    write through the read-only path, nor let the compiler move a load ahead of its grid_wait: no
+    __ldg, and no __restrict__ on what it reads.  The decode tables are constant from start-up on."""
+    both = {"resid", "state", "hist", "partial", "tickets", "ws"}   # read and written
+    plainly = {"gdn_chunk_kernel"}                                  # waits, but is not launched early
+    early, wrong = 0, []
+    for path in SOURCES:
+        functions = list(_functions(_code(path)))
+        waits = lambda body: "grid_wait()" in body or "early.load(" in body
+        if path.suffix == ".cuh" or not any(waits(body) for *_, body in functions):
+            continue
+        for kind, name, parameters, body in functions:
+            if name in plainly or kind == "global" and not waits(body):
+                continue
+            early += kind == "global"
+            for p in re.split(r",\s*", parameters):
+                read = re.search(r"const (\w+)(?:<\w+>)?\* __restrict__", p)
+                if (read and not read[1].startswith("E8p")) or (
+                        "__restrict__" in p and p.split()[-1] in both):
+                    wrong.append(f"{path.name}: {name}: {' '.join(p.split())}")
+            if "__ldg(" in body:
+                wrong.append(f"{path.name}: {name}: __ldg")
+    assert early > 25
+    assert not wrong, "\n".join(wrong)
