@@ -444,6 +444,17 @@ __global__ void attn_merge_kernel(
   }
 }
 
+// Whether a launch of the row kernel may start early.  Of 64 and 128 channels three and more CTAs
+// fit an SM, and a grid of more than one and little more than two per SM then gathers where the
+// kernel in front ends first, while other SMs get one CTA or none: 32 / 8 heads of 128, contexts of
+// 1500 to 3000, 32 rows (256 CTAs) 62 us early and 48 plainly (a decode step of two layers 413 and
+// 385), 28 and 37 rows (224, 296) 61 and 62 against 50, 38 rows (304) 63 against 60, 40 rows (320)
+// 63 against 64, 17 rows of 3 splits (408) 29 against 32; 128 rows of two KV heads of 256 (256)
+// 38.5 against 39.5.
+inline bool attn_starts_early(int head_dim, long long ctas) {
+  return head_dim > 128 || ctas <= 148 || ctas >= 312;
+}
+
 template <int D>
 static int launch_attn(const __half* q, const __half* gate, const int* row_req, const int* row_pos,
                        const int* page_table, int max_pages, const int8_t* kc, const int8_t* vc,
@@ -464,8 +475,13 @@ static int launch_attn(const __half* q, const __half* gate, const int* row_req, 
   static const int slot[4] = {runtime_new_slot(), runtime_new_slot(), runtime_new_slot(),
                               runtime_new_slot()};
   if (const int e = runtime_allow_smem(slot[2 * apart + wide], kernel, SMEM)) return e;
-  launch_early(kernel, grid, ATTN_WARPS * 32, SMEM, stream, q, gate, row_req, row_pos, page_table,
-               max_pages, kc, vc, ks, vs, out, qh, kvh, splits, scratch, rep, apart_keys);
+  if (attn_starts_early(D, static_cast<long long>(rows) * kvh * splits))
+    launch_early(kernel, grid, ATTN_WARPS * 32, SMEM, stream, q, gate, row_req, row_pos, page_table,
+                 max_pages, kc, vc, ks, vs, out, qh, kvh, splits, scratch, rep, apart_keys);
+  else
+    kernel<<<grid, ATTN_WARPS * 32, SMEM, stream>>>(q, gate, row_req, row_pos, page_table,
+                                                    max_pages, kc, vc, ks, vs, out, qh, kvh,
+                                                    splits, scratch, rep, apart_keys);
   if (splits > 1)
     launch_early(attn_merge_kernel<D>, dim3(rows, qh), D < 128 ? 64 : 128, 0, stream, scratch, gate,
                  out, qh, splits);
@@ -479,6 +495,11 @@ using namespace orinfer;
 extern "C" size_t orinfer_attention_scratch_bytes(int rows, int qh, int head_dim, int splits) {
   if (splits <= 1) return 0;
   return static_cast<size_t>(rows) * qh * splits * (head_dim + 2) * sizeof(float);
+}
+
+// Whether the row kernel of such a call may start ahead of the end of the kernel in front.
+extern "C" int orinfer_attention_starts_early(int rows, int kvh, int head_dim, int splits) {
+  return attn_starts_early(head_dim, static_cast<long long>(rows) * kvh * splits) ? 1 : 0;
 }
 
 extern "C" int orinfer_attention(const __half* q, const __half* gate, const int* row_req,

@@ -98,3 +98,16 @@ def test_the_draft_head_is_part_of_the_plan(tmp_path):
         del broken["tensors"]["mtp.fc.scale"]
         with pytest.raises(PlanError, match="mtp.fc"):
             validate_plan(cfg, L, S, max_context=256, descriptor=broken)
+
+
+def test_attention_rows_of_one_to_two_blocks_per_sm_wait_for_their_turn():
+    """Where more than two blocks fit an SM, a launch of between one and little more than two per SM
+    gathers on few SMs when it starts early; it keeps its place behind the kernel in front."""
+    from orinfer_b200.ops import native
+    early = lambda rows, kvh, d, splits=1: bool(native.lib().orinfer_attention_starts_early(
+        rows, kvh, d, splits))
+    assert early(1, 8, 128) and early(18, 8, 128) and early(37, 4, 64)
+    assert not any(early(rows, 8, 128) for rows in range(19, 39))
+    assert not early(64, 4, 64) and not early(19, 8, 128, splits=2)
+    assert early(39, 8, 128) and early(17, 8, 128, splits=3) and early(128, 8, 128)
+    assert all(early(rows, 2, 256) for rows in (1, 74, 80, 128, 150))
