@@ -134,6 +134,7 @@ int orinfer_qgemm(int fmt, const int8_t* a, const float* a_scale, const void* w,
                   int force_path, cudaStream_t stream);
 
 // ---- mixture of experts
+int orinfer_router_form(int rows, int hidden, int experts, int has_shared);
 int orinfer_router_topk(const __half* x, const __half* w, int rows, int hidden, int experts,
                         int has_shared, int top_k, int renorm, int* ids, float* probs,
                         float* shared_gate, cudaStream_t stream);
@@ -159,11 +160,14 @@ int orinfer_qgemm_set_variant(int fmt, int m_lo, int m_hi, int n, int k, int mt,
                               int splits);
 void orinfer_qgemm_clear_variants();
 void orinfer_qgemm_plan(int fmt, int M, int N, int K, int out_f32, int* out);
+int orinfer_qgemm_walks(int fmt, int M, int N, int K, int out_f32);
 int orinfer_qgemm_grouped(int fmt, const int8_t* a, const float* a_scale, const void* w,
                           const __half* w_scale, void* out, int S, int N, int K, int experts,
                           const int* tiles, const int* meta, int max_tiles, cudaStream_t stream,
                           int expected, int tallest);
-// Number of kernel launches it makes.
+// The kernels it takes, and the number of launches it makes.
+int orinfer_qgemm_grouped_form(int fmt, int S, int experts, int max_tiles, int expected,
+                               int tallest);
 int orinfer_qgemm_grouped_launches(int fmt, int S, int experts, int max_tiles, int expected,
                                    int tallest);
 

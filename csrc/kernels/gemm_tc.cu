@@ -1762,6 +1762,15 @@ inline bool walks(int fmt, int mt, int M, int n) {
   return g_impl == 1 && g_probe == 0 && tiles > NUM_SMS && (fmt == 0 || mt <= 2);
 }
 
+// Columns that a plan leaves to the one-tile launch, or to the walking one, before its tail.
+inline int main_columns(const Plan& p, int N) {
+  return p.tail_splits > 0 ? ((N + 127) / 128 - p.tail_tiles) * 128 : N;
+}
+// Whether the walking kernel takes them (one GPU).
+inline bool plan_walks(int fmt, const Plan& p, int M, int N, int out_f32) {
+  return !out_f32 && p.nb == 128 && p.splits == 1 && walks(fmt, p.mt, M, main_columns(p, N));
+}
+
 template <int FMT>
 int launch_fmt(const int8_t* a, const float* a_scale, const void* w, const __half* w_scale,
                void* out, int M, int N, int K, int out_f32, cudaStream_t stream,
@@ -1773,24 +1782,20 @@ int launch_fmt(const int8_t* a, const float* a_scale, const void* w, const __hal
     return launch_pair<FMT, false>(a, a_scale, w, w_scale, out, M, N, K, stream, po, ag);
   }
   const Plan plan = make_plan(FMT, M, N, K, out_f32, po.tp != 0);
-  const int mt = plan.mt, nb = plan.nb, splits = plan.splits;
-  auto walk_call = [&](int n_end) {
-    return WalkCall{a, a_scale, w, w_scale, static_cast<__half*>(out), M, N, K, n_end, nullptr,
-                    nullptr, 0, 1, 0};
-  };
+  const int mt = plan.mt, nb = plan.nb, splits = plan.splits, cut = main_columns(plan, N);
+  const bool walk = po.tp == 0 && ag.tp == 0 && plan_walks(FMT, plan, M, N, out_f32);
+  const WalkCall walk_call{a, a_scale, w, w_scale, static_cast<__half*>(out), M, N, K, cut,
+                           nullptr, nullptr, 0, 1, 0};
   if (plan.tail_splits > 0) {
-    const long ntiles = (N + 127) / 128;
-    const int cut = static_cast<int>(ntiles - plan.tail_tiles) * 128;
     // the tail runs as 128-row tiles: more CTAs of less work each, and small accumulator
     // tiles whose splits are added inside the kernel
     const int ts = plan.tail_splits;
 #define ORINFER_TWO(MTV)                                                                        \
   {                                                                                             \
     const int r =                                                                               \
-        walks(FMT, MTV, M, cut) && ag.tp == 0                                                   \
-            ? qgemm_walk_dispatch(FMT, MTV > 1 ? 2 : 1, walk_call(cut), stream)                 \
-            : launch<FMT, false, MTV, 128>(a, a_scale, w, w_scale, out, M, N, K, stream, po,    \
-                                           none, 1, 0, ag, 1, 0, cut);                          \
+        walk ? qgemm_walk_dispatch(FMT, MTV > 1 ? 2 : 1, walk_call, stream)                     \
+             : launch<FMT, false, MTV, 128>(a, a_scale, w, w_scale, out, M, N, K, stream, po,   \
+                                            none, 1, 0, ag, 1, 0, cut);                         \
     if (r) return r;                                                                            \
     return launch<FMT, false, 1, 128>(a, a_scale, w, w_scale, out, M, N, K, stream, po, none,  \
                                       1, 0, ag, ts, cut, N);                                   \
@@ -1800,8 +1805,7 @@ int launch_fmt(const int8_t* a, const float* a_scale, const void* w, const __hal
     ORINFER_TWO(1)
 #undef ORINFER_TWO
   }
-  if (!out_f32 && nb == 128 && splits == 1 && po.tp == 0 && ag.tp == 0 && walks(FMT, mt, M, N))
-    return qgemm_walk_dispatch(FMT, mt > 1 ? 2 : 1, walk_call(N), stream);
+  if (walk) return qgemm_walk_dispatch(FMT, mt > 1 ? 2 : 1, walk_call, stream);
 #define ORINFER_GO(F32, MTV, NBV)                                                              \
   return launch<FMT, F32, MTV, NBV>(a, a_scale, w, w_scale, out, M, N, K, stream, po, none, 1, \
                                     0, ag, splits)
@@ -1924,6 +1928,12 @@ extern "C" void orinfer_qgemm_plan(int fmt, int M, int N, int K, int out_f32, in
   out[3] = p.tail_splits;
 }
 
+// Whether the walking kernel takes the shape on one GPU, a peeled tail apart.
+extern "C" int orinfer_qgemm_walks(int fmt, int M, int N, int K, int out_f32) {
+  const tc::Plan p = tc::make_plan(fmt, M, N, K, out_f32, false);
+  return tc::plan_walks(fmt, p, M, N, out_f32) ? 1 : 0;
+}
+
 extern "C" int orinfer_qgemm(int fmt, const int8_t* a, const float* a_scale, const void* w,
                              const __half* w_scale, void* out, int M, int N, int K, int out_f32,
                              int force_path, cudaStream_t stream) {
@@ -2007,6 +2017,24 @@ static GroupedPlan grouped_plan(int fmt, int S, int experts, int max_tiles, int 
   return tall > room || max_tiles > 16384 ? GroupedPlan{false, 0} : GroupedPlan{true, tall};
 }
 
+// Row tiles of one expert per CTA: two where experts have about half a tile of rows or more (INT8
+// nearly a whole one: nothing to decode, so a second tile only saves the copy of the weights),
+// four where they have several.
+static int grouped_row_tiles(int fmt, int expected, int experts) {
+  const long long two = (fmt == 0 ? 112LL : 64LL) * experts, four = 256LL * experts;
+  return tc::g_impl != 1 ? 1 : (expected >= four ? 4 : (expected >= two ? 2 : 1));
+}
+
+// Whether the walking kernel takes the tiles of a grouped call, however many there are.  Whole
+// layers of experts of 768: 128 Q4 experts, 2048 rows 447 -> 340 us, 300 rows 300 -> 213; INT8 390
+// -> 281; and with fewer tiles than SMs, 4 and 8 experts, 64 rows 62 -> 48 and 64 -> 50 (INT8 58 ->
+// 37 and 58 -> 42), 512 rows 79 -> 65 and 75 -> 65 (a part of these is the early start of their
+// kernels).  Codes that serve four row tiles stay with the one-tile kernel, as in `walks`.
+static bool grouped_walks(int fmt, int max_tiles, int mt) {
+  return tc::g_impl == 1 && tc::g_probe == 0 && max_tiles <= walk_list_room(fmt) &&
+         (fmt == 0 || mt <= 2);
+}
+
 template <int FMT>
 static int qgemm_grouped_fmt(const int8_t* a, const float* a_scale, const void* w,
                              const __half* w_scale, void* out, int S, int N, int K, int experts,
@@ -2029,17 +2057,8 @@ static int qgemm_grouped_fmt(const int8_t* a, const float* a_scale, const void* 
                                                                               : max_tiles,
                                              ag, 1, 0, N);
   }
-  // Row tiles of one expert per CTA: two where experts have about half a tile of rows or more (INT8
-  // nearly a whole one: nothing to decode, so a second tile only saves the copy of the weights),
-  // four where they have several.
-  const long long two = (FMT == 0 ? 112LL : 64LL) * experts;
-  const long long four = 256LL * experts;
-  const int mt = tc::g_impl != 1 ? 1 : (expected >= four ? 4 : (expected >= two ? 2 : 1));
-  // More tiles than SMs: the walking kernel (128 Q4 experts of 768, both projections and all: 2048
-  // rows 447 -> 340 us, 300 rows 300 -> 213; INT8 390 -> 281).  Codes that serve four row tiles
-  // stay with the one-tile kernel, as in `walks`.
-  if (tc::g_impl == 1 && tc::g_probe == 0 && max_tiles <= walk_list_room(FMT) &&
-      (FMT == 0 || mt <= 2))
+  const int mt = grouped_row_tiles(FMT, expected, experts);
+  if (grouped_walks(FMT, max_tiles, mt))
     return qgemm_walk_dispatch(FMT, mt > 1 ? 2 : 1,
                                WalkCall{a, a_scale, w, w_scale, static_cast<__half*>(out), S, N, K,
                                         N, tiles, meta, bank, experts, max_tiles},
@@ -2069,6 +2088,16 @@ extern "C" int orinfer_qgemm_grouped(int fmt, const int8_t* a, const float* a_sc
   if (fmt == 1) ORINFER_GROUPED(1);
   ORINFER_GROUPED(2);
 #undef ORINFER_GROUPED
+}
+
+// The kernels of a grouped call: 0 small-M, 1 small-M and persistent, 2 one tile per CTA,
+// 3 walking.
+extern "C" int orinfer_qgemm_grouped_form(int fmt, int S, int experts, int max_tiles, int expected,
+                                          int tallest) {
+  if (expected <= 0 || expected > S) expected = S;
+  const GroupedPlan p = grouped_plan(fmt, S, experts, max_tiles, expected, tallest);
+  if (p.rows_kernel) return p.listed > 0 ? 1 : 0;
+  return grouped_walks(fmt, max_tiles, grouped_row_tiles(fmt, expected, experts)) ? 3 : 2;
 }
 
 extern "C" int orinfer_qgemm_grouped_launches(int fmt, int S, int experts, int max_tiles,

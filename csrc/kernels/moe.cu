@@ -549,14 +549,8 @@ static int launch_dispatch(const int* ids, int rows, int top_k, int base_expert,
 
 using namespace orinfer;
 
-extern "C" {
-
-int orinfer_router_topk(const __half* x, const __half* w, int rows, int hidden, int experts,
-                        int has_shared, int top_k, int renorm, int* ids, float* probs,
-                        float* shared_gate, cudaStream_t stream) {
-  if (rows <= 0) return 0;
-  if (hidden % 8 || top_k < 1 || top_k > experts || experts > 4096) return -1;
-  const int total = experts + (has_shared ? 1 : 0);
+// The router's form: rows per CTA or cluster.
+static int router_form(int rows, int hidden, int total) {
   // Few experts leave most of a cluster's CTAs without a tile, and its two exchanges cost more than
   // reading a small matrix per row: 8 experts x 2048 channels, 16 rows, 4.6 us in the general
   // form against 6.3, 2048 rows 13.6 against 17.7; 16 experts 5.9 against 6.6; but 16 x 4096 11.0
@@ -570,11 +564,28 @@ int orinfer_router_topk(const __half* x, const __half* w, int rows, int hidden, 
   const int cl = hidden <= 2048 ? 4 : 8;
   if (!few && rows >= ROUTER_MANY && hidden % (cl * 128) == 0 && hidden / cl >= 384 &&
       hidden / cl <= 512 && total <= ROUTER_TILES * 8 &&
-      router_rows_smem(hidden, total, cl) <= 220 * 1024 &&
-      runtime_ensure_init() == cudaSuccess)
-    return (cl == 4 ? launch_router_rows<4> : launch_router_rows<8>)(
+      router_rows_smem(hidden, total, cl) <= 220 * 1024)
+    return ROUTER_ROWS;
+  return !few && hidden % 256 == 0 && total <= 8 * 8 * 9 ? 16 : 1;
+}
+
+extern "C" {
+
+int orinfer_router_form(int rows, int hidden, int experts, int has_shared) {
+  return router_form(rows, hidden, experts + (has_shared ? 1 : 0));
+}
+
+int orinfer_router_topk(const __half* x, const __half* w, int rows, int hidden, int experts,
+                        int has_shared, int top_k, int renorm, int* ids, float* probs,
+                        float* shared_gate, cudaStream_t stream) {
+  if (rows <= 0) return 0;
+  if (hidden % 8 || top_k < 1 || top_k > experts || experts > 4096) return -1;
+  const int total = experts + (has_shared ? 1 : 0);
+  const int form = runtime_ensure_init() == cudaSuccess ? router_form(rows, hidden, total) : 1;
+  if (form == ROUTER_ROWS)
+    return (hidden <= 2048 ? launch_router_rows<4> : launch_router_rows<8>)(
         x, w, rows, hidden, experts, has_shared, top_k, renorm, ids, probs, shared_gate, stream);
-  if (!few && hidden % 256 == 0 && total <= 8 * 8 * 9 && runtime_ensure_init() == cudaSuccess) {
+  if (form == 16) {
     // Wide routers read their matrix from few SMs in a decode step: more warps, more loads in
     // flight (16 rows, 512 experts: 26 -> 16 us).
 #define ORINFER_ROUTER(MAXT, WARPS)                                                  \

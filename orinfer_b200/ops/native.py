@@ -68,6 +68,9 @@ def _load() -> ctypes.CDLL:
         "orinfer_qgemm_launches_fmt": ([I, I, I, I, I, I], I),
         "orinfer_qgemm_set_variant": ([I, I, I, I, I, I, I, I], I),
         "orinfer_qgemm_clear_variants": ([], None),
+        "orinfer_qgemm_walks": ([I, I, I, I, I], I),
+        "orinfer_qgemm_grouped_form": ([I, I, I, I, I, I], I),
+        "orinfer_router_form": ([I, I, I, I], I),
         "orinfer_qgemm_plan": ([I, I, I, I, I, P], None),
         "orinfer_act_prep_limited": ([P, P, P, P, I, I, I, P, P], I),
         "orinfer_small_proj": ([P, P, P, I, I, I, P], I),

@@ -83,14 +83,16 @@ def test_router_sums_keep_fp32_accuracy(dev, hidden, experts, shared):
     assert float((probs.double() - p).norm() / p.norm()) < limit
 
 
-@pytest.mark.parametrize("rows,hidden,experts,top_k,shared", [
-    (512, 2048, 128, 8, False), (513, 2048, 135, 8, True), (575, 1536, 40, 40, False),
-    (1100, 3072, 97, 6, True), (640, 4096, 129, 1, False), (700, 2048, 33, 33, False),
-    (40, 2048, 64, 35, True)])
-def test_router_rows_form_and_long_choices(dev, rows, hidden, experts, top_k, shared):
-    """The form for many rows at the edges of its row and expert tiles and both spans, and choices
-    past the 32nd."""
+@pytest.mark.parametrize("rows,hidden,experts,top_k,shared,form", [
+    (512, 2048, 128, 8, False, 64), (513, 2048, 135, 8, True, 64), (575, 1536, 43, 40, False, 64),
+    (1100, 3072, 97, 6, True, 64), (640, 4096, 129, 1, False, 64), (700, 2048, 33, 33, False, 64),
+    (575, 1536, 40, 40, False, 1), (40, 2048, 64, 35, True, 16)])
+def test_router_rows_form_and_long_choices(dev, rows, hidden, experts, top_k, shared, form):
+    """The form for many rows at the edges of its row and expert tiles and both spans of four and
+    eight CTAs, and choices past the 32nd in all forms."""
     from orinfer_b200.ops import functional as F
+    from orinfer_b200.ops import native
+    assert native.lib().orinfer_router_form(rows, hidden, experts, int(shared)) == form
     g = torch.Generator(device=dev).manual_seed(experts + rows)
     y = torch.randn(rows, hidden, generator=g, device=dev).half()
     w = (torch.randn(experts + int(shared), hidden, generator=g, device=dev) * 0.02).half()
@@ -242,6 +244,37 @@ def test_grouped_projection_splits_by_tile_height(dev, fmt, experts, rows, top_k
     acc = torch.einsum("rk,rnk->rn", src, ints.view(experts, n, k)[flat[order]].double()).float()
     want = acc * ws.view(experts, n).to(dev)[flat[order]].float() * sa[order // top_k, None]
     assert torch.equal(out, want.half())
+
+
+@pytest.mark.parametrize("short,tall", [(383, 200), (384, 256), (383, 129)])
+def test_walked_tile_lists_of_several_passes(dev, short, tall):
+    """More INT8 experts than the 384 threads of the walking kernel, so that its CTAs list the tiles
+    in two passes, and an expert of two tiles across the seam (codes have more threads than room
+    for tiles)."""
+    from orinfer_b200.ops import functional as F
+    from orinfer_b200.ops import native
+    n, k, fmt = 128, 128, "w8"
+    counts = [120] * (short - 1) + [97, tall, 1, 0, 128]
+    experts, s = len(counts), sum(counts)
+    g = torch.Generator().manual_seed(short + tall)
+    codes, ws, _ = _int_weight(fmt, experts * n, k, g)
+    codes, ws = codes.view(experts, n, k).to(dev), ws.view(experts, n).to(dev)
+    a = torch.randint(-127, 128, (s, k), generator=g, dtype=torch.int8).to(dev)
+    sa = (torch.rand(s, generator=g) * 0.05 + 1e-3).to(dev)
+    ids = torch.repeat_interleave(torch.arange(experts), torch.tensor(counts)).to(torch.int32)
+    sc = F.MoeScratch(s, 1, experts, k, 64, dev)
+    F.moe_dispatch(ids[:, None].to(dev), a, sa, experts, sc, s)
+    tiles = int(sc.meta[0])
+    assert tiles > 384
+    assert native.lib().orinfer_qgemm_grouped_form(F.FMT[fmt], s, experts, sc.tiles.shape[0], s,
+                                                   s) == 3
+    out = torch.full((s, n), float("nan"), dtype=torch.float16, device=dev)
+    F.qgemm_grouped(sc.q8, sc.scale, codes, ws, fmt, n, out, sc, s)
+    at = 0
+    for e, c in enumerate(counts):                       # the rows are in expert order already
+        want = _scaled(a[at:at + c], sa[at:at + c], codes[e], ws[e])
+        assert torch.equal(out[at:at + c], want.half()), e
+        at += c
 
 
 def _grouped_us(dev, ids, experts, n, k, fmt, banks):

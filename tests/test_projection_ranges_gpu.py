@@ -97,14 +97,23 @@ def test_walked_tiles_are_exact(dev, fmt, m, n, k):
     eight-row piece of a tile, single k-blocks, fewer k-blocks than ring stages; repeated, since its
     warps run ahead of each other."""
     from orinfer_b200.ops import functional as F
+    from orinfer_b200.ops import native
+    lib = native.lib()
     g = torch.Generator().manual_seed(m + n + k)
     codes, ws, w = _int_weight(fmt, n, k, g)
     a = torch.randint(-127, 128, (m, k), generator=g, dtype=torch.int8)
     sa = torch.rand(m, generator=g) * 0.05 + 1e-3
     want = _scaled(a.to(dev), sa.to(dev), w.to(dev), ws.to(dev)).half()
     a, sa, codes, ws = a.to(dev), sa.to(dev), codes.to(dev), ws.to(dev)
-    for _ in range(5):
-        assert torch.equal(F.qgemm(a, sa, codes, ws, fmt, n), want)
+    if m > 256 and fmt != "w8":                            # codes: two row tiles, not four
+        assert not lib.orinfer_qgemm_walks(F.FMT[fmt], m, n, k, 0)
+        assert lib.orinfer_qgemm_set_variant(F.FMT[fmt], m, m, n, k, 2, 128, 1) == 0
+    try:
+        assert lib.orinfer_qgemm_walks(F.FMT[fmt], m, n, k, 0)
+        for _ in range(5):
+            assert torch.equal(F.qgemm(a, sa, codes, ws, fmt, n), want)
+    finally:
+        lib.orinfer_qgemm_clear_variants()
 
 
 @pytest.mark.parametrize("rows", [1, 7, 149, 300, 2049])
