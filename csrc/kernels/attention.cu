@@ -81,8 +81,11 @@ struct RowScales {
 // cores, with the weights going through shared memory: it was bound by those instructions.  32
 // query / 8 KV heads of 128: 128 rows of 320..640 keys 209 -> 53 us with the products on the
 // tensor cores and loads through registers, 41 us with the loads in cp.async rings (132 MB: 3.2
-// TB/s); 6 rows of 12000..24000 keys 432 -> 78 -> 62 us (235 MB: 3.8 TB/s).  The loads in flight
-// bound it: three CTAs of 128 threads hold 96 KB of them per SM.
+// TB/s); 6 rows of 12000..24000 keys 432 -> 78 -> 62 us (235 MB: 3.8 TB/s).  A block's own work
+// bounds it: 57 and 62 % of the issue slots and half of the ALU pipe (copies and their addresses,
+// scale shuffles, a permute and a subtraction per pair of INT8 values, the head and remainder, two
+// maxima per block) with under three warps per scheduler, which wait for fixed latencies and for
+// each other; for loads they wait a third of that (0.3 to 0.6 warps per issue).
 template <int D>
 struct AttnTile {
   static constexpr int G = D / 64;                 // scale groups per row

@@ -574,9 +574,11 @@ int runtime_new_slot();
 // Launch of a kernel that calls grid_wait (see there): what lies between two kernels of a stream,
 // also inside a graph, falls together with the end of the first (one decode step of eight requests,
 // 27 kernels, 241 -> 232 us; 1 x 19456 x 2560 12.9 -> 11.8; 16 rows on 512 Q2 experts 113 -> 105).
-// Not for grids of many CTAs, each of which pays for the wait: with all of them started this way
-// 2048 rows on 128 experts took 348 us (310 now, 311 without) and a recurrent mixer of two prompts
-// 274 (245 now).
+// A kernel that finds its stream idle gains nothing by it.  Not for grids of many CTAs, each of
+// which pays for the wait: with all of them started this way 2048 rows on 128 experts took 348 us
+// against 310 with this bound and 311 with none of them, and a recurrent mixer of two prompts 274
+// against 260; nor where few long CTAs would gather (see attn_starts_early and the chunked
+// recurrence).
 constexpr long long EARLY_CTAS = 4 * 148;
 template <class... P, class... A>
 void launch_early(void (*kernel)(P...), dim3 grid, dim3 block, size_t smem, cudaStream_t stream,

@@ -95,7 +95,8 @@ __global__ void __launch_bounds__(D) gdn_conv_kernel(
 // rows: the three earlier rows stay in registers, so a packet's rows are read once instead of
 // four times two bytes at a time.  A head is D / 8 neighbouring lanes.  Grid (row strips,
 // conv_dim / 2048); R = 1 for decode-sized packets, where the strips would be too few CTAs.
-// 2100 rows x 8192 channels: 89 -> 25 us; 64 rows: 7.9 -> 5.0 us.
+// 2100 rows x 8192 channels: 89 -> 36 us (issue slots 61 %, DRAM 12 %: instructions, not bytes); 64
+// rows: 7.9 -> 5.0 us.
 template <int D, int R>
 __global__ void __launch_bounds__(256) gdn_conv_vec_kernel(
     const __half* x, int x_stride, const __half* weight, const __half* hist, const int* row_first,
@@ -501,8 +502,9 @@ __global__ void __launch_bounds__(256) gdn_scan_split_kernel(
 // below 1/2 a row 1.6e-7 and 1.1e-7 (1.5e-7 and 1.1e-7).
 //
 // 32 heads of 128 channels, one run of 1050 rows: 406 us as a scan (0.39 us per dependent step),
-// 195 us here (166 with chained sums), 164 since the helpers alone copy the chunks; 16 runs of 64
-// rows: 192 -> 84 -> 78 us.
+// 195 us here (166 with chained sums), 164 since the helpers alone copy the chunks (two such runs,
+// 128 CTAs, 190); 16 runs of 64 rows: 192 -> 84 -> 78 us.  Two CTAs per SM leave 168 registers and
+// 168 bytes of spills a thread; issue slots 30 %, tensor pipe 24 %: dependent steps in few warps.
 // Runs below GDN_LONG_ROWS keep the scan: one run of 36 rows takes 17.2 us there and 19.4 here, of
 // 40 rows 19.4 both ways, of 63 rows 28.0 and 19.4 (two runs of 50: 33 and 20).  The scan's bits
 // are those of a verification pass, whose segments are shorter.
@@ -1209,7 +1211,8 @@ int orinfer_gdn_scan(const __half* qkv, const float* ab, const float* a_log, con
     static const int slot = runtime_new_slot();
     if (const int e = runtime_allow_smem(slot, gdn_chunk_kernel, sizeof(ChunkSmem))) return e;
     // Not early: its few long CTAs would gather, two to an SM, where the kernel before ends first
-    // (the mixer of two runs of 1050 rows 260 us, 245 so; of two of 1500 rows 357 and 335).
+    // (the mixer of two runs of 1050 rows 260 us, 245 so, each in turn on one card; of two of 1500
+    // rows 357 and 335).
     gdn_chunk_kernel<<<dim3(hv * 2, n_segs), CHUNK_THREADS, sizeof(ChunkSmem), stream>>>(
         qkv, conv_dim, ab, a_log, dt_bias, sg, row_slot, row_pos, hk, hv, state, out);
   }

@@ -1756,7 +1756,7 @@ inline Plan make_plan(int fmt, int M, int N, int K, int out_f32, bool fused) {
 // tiles per CTA: from a second wave of tiles on.  Its tiles have two row tiles at most, so lattice
 // codes that serve four stay here: 2048 x 19456 x 2560 Q4 118 us against 139, 1024 rows 67 against
 // 79, 600 rows 64 against 62; 200 x 40000 x 1024 31 against 27; INT8 2048 x 19456 x 2560 117
-// against 86.
+// against 86 (126 with the issuing loop of one lane that the one-tile kernel had before).
 inline bool walks(int fmt, int mt, int M, int n) {
   const long tiles = static_cast<long>((M + BM * mt - 1) / (BM * mt)) * ((n + 127) / 128);
   return g_impl == 1 && g_probe == 0 && tiles > NUM_SMS && (fmt == 0 || mt <= 2);

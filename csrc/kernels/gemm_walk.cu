@@ -18,11 +18,12 @@
 // accumulators (MT = 1 or 2).
 //
 // What bounds it: INT8 weights take 67 cycles per 128 x 128 x 32 MMA when their copies are there
-// (2048 x 19456 x 2560 122 -> 86 us, 2.4 PFLOP/s).  Lattice codes: the decode warps, 1100 to 1500
+// (2048 x 19456 x 2560 126 -> 86 us, 2.4 PFLOP/s).  Lattice codes: the decode warps, 1100 to 1500
 // cycles per k-block (72 % of the shared-memory pipe, 66 % of the issue slots, 21 % of the tensor
 // core); signs from arithmetic instead of lookups, and with them a conflict-free
 // table, made that a sixth longer.  128 Q4 experts of 768 with 128 rows each, a whole layer:
-// 447 -> 340 us.
+// 447 -> 340 us (463 -> 326 with the router's and the launches' share; votes on every wait and the
+// activations' own barrier cost 1.5 % of it).
 #include <cuda.h>
 
 #include "api.h"

@@ -582,8 +582,10 @@ __global__ void __launch_bounds__(GEMV_THREADS, 1) qgemv_kernel(
 // activations per row and code word.  Lane l holds row l / LPR of a group and an LPR-th of the
 // k-block, DEPTH units in flight.  1 x 19456 x 2560 14.8 -> 12.9 us, 1 x 2560 x 9728 12.1 -> 10.9,
 // 1 x 6144 x 2560 Q2 6.8 -> 6.6 with the fields multiplied as they are looked up and the small
-// loads ahead of the weights.  About 2 us are launch, 2.5 the first loads, 6 the products (two
-// thirds of the shared-memory reads and of the instructions that an SM can issue), 1 the outputs.
+// loads ahead of the weights; with the early start too, eight weights in turn in a graph, one row
+// 15.1 -> 11.8, 11.3 -> 9.2 and 6.7 -> 5.7, two rows 16.4 -> 13.9, 12.9 -> 11.0 and 7.5 -> 6.4 (12
+// bytes of spills a thread).  About 2 us are launch, 2.5 the first loads, 6 the products (63 % of
+// the issue slots, half of the ALU pipe), 1 the outputs.
 template <int FMT, int MT>
 struct Dp4a {
   static constexpr int THREADS = MT <= 2 ? 1024 : 512;             // registers
@@ -738,7 +740,8 @@ __global__ void __launch_bounds__(Dp4a<FMT, MT>::THREADS, 1) e8p_dp4a_kernel(
 // need, the activations read from shared memory once per weight row.  Small projections are up to
 // twice as fast this way as with the persistent CTAs of the MMA form; from three rows on its reads
 // lose to the MMAs once there is work for every SM.
-//   one row: 6144 x 2560 3.7 us against 6.9, the 151936-row head 74 against 75
+//   one row: 6144 x 2560 3.7 us against 6.9, a 151936-row head 74 against 75 (with peers: on one
+//     GPU such a head is a stream, see w8_streams)
 //   four: 1024 x 1024 2.7 against 5.2, 4096 x 4096 6.0 against 6.9, 5120 x 9728 15.7 against 16.2,
 //     6144 x 2560 7.4 against 6.7, 9728 x 1024 5.8 against 6.0, 12288 x 1024 7.0 against 6.1
 //   eight: 1024 x 1024 4.0 against 5.9, 2048 x 4096 6.5 against 6.9, 4096 x 2560 7.7 against 7.2,
@@ -799,8 +802,9 @@ __global__ void __launch_bounds__(W8_WARPS * 32) w8_gemv_kernel(
 // into a ring with bulk copies, and each stage of the ring has a warp of its own that multiplies
 // the tile it holds (MMAs as above: 16 weight rows x 8 activation rows) and stores its outputs.
 // Rows lie 64 bytes past a multiple of 128 apart in shared memory, so 16-byte reads of two rows
-// meet on no bank. 151936 x 2560 (389 MB): one row 73.7 -> 57.8 us (6.7 TB/s), four 74.5 -> 60.2,
-// eight 76.7 -> 63.4. Below about 24 M weights the set-up of the rings costs more than it gives:
+// meet on no bank. 151936 x 2560 (389 MB): one row 75 -> 57.6 us (6.75 TB/s, with four matrices in
+// turn as with one: reads alone, above the 6.54 TB/s of a copy), two 79 -> 58.4, four 76 -> 60.2,
+// eight 78 -> 63.7.  Below about 24 M weights the set-up of the rings costs more than it gives:
 // one row of 12288 x 2560 9.3 -> 9.1 us, eight rows 12.5 both ways, but 6144 x 2560 5.7 -> 6.7 and
 // 9.1 -> 9.9.  It takes three stages: with the two that eight rows of 4096 channels leave, 32000
 // rows gain nothing.

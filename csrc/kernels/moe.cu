@@ -230,10 +230,11 @@ static int launch_router(const __half* x, const __half* w, int rows, int hidden,
 // expert tiles each, and the CTAs add up each other's parts for 64 / CL rows of the top-k.  Sums as
 // above: 16 products in the tensor core, pairs of those added in FP32 in two alternating sums per
 // CTA (probabilities of 128 experts: 1.18e-7 from exact at 2048 channels, 1.50e-7 at 4096; above
-// 1.18e-7 and 1.62e-7). 128 experts x 2048 channels, 2048 rows: 46.4 -> 19.8 us, 1024 rows 27.2 ->
-// 19.5, 512 rows 22.8 -> 19.5; fewer rows are one wave of the form above (384: 10.1 us).  Half of
-// it is the top-k, two rows per warp: with choices kept in memory and renormalised there it took 15
-// us more.
+// 1.18e-7 and 1.62e-7).  At most 136 expert rows and 512 channels a CTA fit its shared memory; at
+// least 384 channels, because the parts of 136 experts take the place of the 64 rows.  128 experts
+// x 2048 channels, 2048 rows: 46.4 -> 19.8 us, 1024 rows 27.2 -> 19.5, 512 rows 22.8 -> 19.5; fewer
+// rows are one wave of the form above (384: 10.1 us).  Half of it is the top-k, two rows per warp:
+// with choices kept in memory and renormalised there it took 15 us more.
 constexpr int ROUTER_ROWS = 64, ROUTER_TILES = 17, ROUTER_MANY = 512;
 
 __device__ __forceinline__ void ldmatrix4(uint32_t (&r)[4], const void* p) {
