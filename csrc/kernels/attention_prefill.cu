@@ -15,7 +15,7 @@
 //     read S from TMEM, apply scale and the causal mask, and write P as FP16 over their half of S,
 //     where the second MMA reads it as its A operand.  The two meet once per step, for the row's
 //     maximum, and hand over the sum of the weights, which are added in the order of the keys
-//     (sums of their own per half would save 7 % of 4096 rows and 4 to 10 % of short chunks, and
+//     (sums of their own per half would save 5 % of 4096 rows and 4 to 9 % of short chunks, and
 //     move FP16 outputs by a step, which the INT8 rows of the next projection make a code step).
 //     P is relative to the row's running maximum, so its largest weight is exactly 1 and
 //     O is rescaled whenever a row of the warp finds a larger score;
@@ -30,7 +30,7 @@
 // MMAs issued inside a branch on the lane, about 4700 with two threads and a whole warp in the
 // issuing loop.  The tensor core needs 2050 of them, the exponentials as many.
 // One 4096-token chunk, 32 / 8 heads of 128: 377 us with one tile per CTA and P in shared memory,
-// 243 with two tiles and P in TMEM, 206 with two threads per row and a whole issuing warp (667
+// 243 with two tiles and P in TMEM, 203 with two threads per row and a whole issuing warp (677
 // TFLOP/s causal); 512 tokens 19 -> 14 us, 64 behind 1000 29 -> 22.  A reference that follows the
 // maximum only when it lags by 2^8 saves another tenth (fewer rescales of O) but rounds the largest
 // weights in FP16: the error against 64 bits grows by 1.8 % there and by 3.7 % for 500 rows behind
