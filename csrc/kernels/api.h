@@ -174,6 +174,7 @@ int orinfer_qgemm_grouped_launches(int fmt, int S, int experts, int max_tiles, i
 // ---- attention over the paged INT8 KV cache
 size_t orinfer_attention_scratch_bytes(int rows, int qh, int head_dim, int splits);
 int orinfer_attention_starts_early(int rows, int kvh, int head_dim, int splits);
+int orinfer_attention_in_digits(int qh, int kvh, int head_dim, int max_pages, int splits);
 int orinfer_attention(const __half* q, const __half* gate, const int* row_req, const int* row_pos,
                       const int* page_table, int max_pages, const int8_t* kcache,
                       const int8_t* vcache, const __half* kscale, const __half* vscale,

@@ -8,6 +8,7 @@
 // (kernels/cuda/model/attention_rows.py:61-276,280-400).
 #include "api.h"
 #include "common.cuh"
+#include "tma.h"
 
 namespace orinfer {
 
@@ -434,11 +435,467 @@ __global__ void __launch_bounds__(
   attn_finish<D, 8>(s_o, s_m, s_l, apart, idle, rep, row, h, qh, split, splits, gate, out, scratch);
 }
 
+// ---------------------------------------------------------------- digit form
+// The same attention for at most four query heads per KV head, with both products on the INT8
+// tensor cores and no conversion of what the cache holds.
+//   S = Q K^T: the query, FP16, becomes a fixed-point number of 31 bits under a power of two per
+//   head, and that four signed digits to the base 256; rows 4 i + r of A are digit i (the largest
+//   first) of head r.  INT32 sums over 64 channels are exact, and the digits' sums meet in FP32.
+//   O = P V: the FP32 weight x value scale becomes a fixed-point number of 31 bits, four digits,
+//   in the same rows, and the sums stay in INT32 accumulators from block to block.
+// The weights are relative to a reference that follows the row's maximum only when that is more
+// than 2^DIGIT_LAG above it, and the value scales to the power of two above all seen: only when one
+// of them moves are the accumulators rescaled, in place.  With the lag all used up a weight keeps
+// 27 bits below the largest, and 30 at best; a query value is exact down to 2^-19 of its head's
+// largest and rounded at 2^-31 of that below it.  Error against 64 bits ahead of the output's FP16
+// rounding (2.07e-4): 8 rows of 900 keys 1.7e-7 (the form above 1.6e-7), 3 rows of 20000 2.0e-7
+// (9.2e-7), with six times the scores 6.5e-7 (7.8e-7); a lag of 2^6 gave 2.2e-7, 2.5e-7 and 7.1e-7.
+//
+// K and V come by TMA as they lie in the cache, a box of 32 keys each, swizzled for ldmatrix; V's
+// fragments are transposed by the load (m16n16 b8).  A lane owns eight keys of a block in both
+// products; which ones is chosen so that neither side's loads meet on a bank.
+//
+// A block of 32 keys is 400 instructions of a warp where the form above takes about 900.  32 / 8
+// heads of 128: 6 rows of 12000..24000 keys 62.7 -> 50.3 us (235 MB; the blocks alone run at the
+// memory's rate), 38 rows of 1500..3000 57.5 -> 38.5, 128 rows of 320..640 38.7 -> 34.2.  The last
+// is 2.3 waves of CTAs, each of which waits 4000 cycles for its row, pages and first block and
+// takes 3000 to finish besides the 12000 of its blocks.  Tried: blocks of 64 keys with one buffer
+// (the same), the heads of a row side by side in the grid (the same, long rows 4 % slower), a warp
+// per row of up to 512 keys (the same with 128 rows, 64 rows 28.4 against 21.8), scales by loads
+// into registers (the loop's move waits for them: the same, long rows 2 % quicker).
+template <int D>
+struct DigitTile {
+  static constexpr int G = D / 64, KB = 32, KSTEPS = D / 32;
+  static constexpr int ROWS = KB * D;                    // K or V of one block
+  static constexpr int STAGES = 2;
+  static constexpr int RING = ATTN_WARPS * STAGES * 2 * ROWS;
+  static constexpr int SMEM = RING + 1024;
+  static constexpr int MIN_CTAS = D == 128 ? 3 : 4;
+  // 16-byte unit `u` of row `key`: the hardware's 128- or 64-byte swizzle
+  __device__ static uint32_t unit(int key, int u) {
+    return key * D + ((D == 128 ? u ^ (key & 7) : u ^ ((key >> 1) & 3)) << 4);
+  }
+  // The key of a 16-key half block that lane t of a quad owns as its number x (0..3): 2t, 2t + 1
+  // and two of the upper eight, rotated so that the eight rows that a load reads together (all t
+  // with one x pair for K, two t with all x for V) differ modulo 8.
+  __device__ static int key_of(int t, int x) {
+    return x < 2 ? 2 * t + x : 8 + ((2 * t + 4 + (x & 1)) & 7);
+  }
+};
+constexpr float DIGIT_LAG = 3.f;                         // in powers of two
+constexpr int DIGIT_BITS = 27;                           // 30 less the lag
+// Keys of a warp after which the accumulators are scaled down: a digit's sum grows by at most
+// 128 x 127 a key.
+constexpr int DIGIT_BLOCKS = (1 << 16) / 32;
+
+__device__ __forceinline__ void mma_s8(int (&c)[4], const uint32_t (&a)[4], uint32_t b0,
+                                       uint32_t b1) {
+  asm volatile(
+      "mma.sync.aligned.m16n8k32.row.col.s32.s8.s8.s32 {%0, %1, %2, %3}, {%4, %5, %6, %7}, "
+      "{%8, %9}, {%0, %1, %2, %3};"
+      : "+r"(c[0]), "+r"(c[1]), "+r"(c[2]), "+r"(c[3])
+      : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1));
+}
+__device__ __forceinline__ float ex2_ftz(float x) {
+  float y;
+  asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
+  return y;
+}
+__device__ __forceinline__ float two_to(int e) {         // e in -126..127
+  return __uint_as_float(static_cast<uint32_t>(127 + e) << 23);
+}
+
+// the scales of two neighbouring keys
+template <int G>
+__device__ __forceinline__ void load_pair(float (&v)[2 * G], const float* p) {
+  if (G == 2) {
+    const float4 x = *reinterpret_cast<const float4*>(p);
+    v[0] = x.x; v[1] = x.y; v[2 * G - 2] = x.z; v[2 * G - 1] = x.w;
+  } else {
+    const float2 x = *reinterpret_cast<const float2*>(p);
+    v[0] = x.x; v[1] = x.y;
+  }
+}
+
+template <int D, bool APART>
+__global__ void __launch_bounds__(ATTN_WARPS * 32, DigitTile<D>::MIN_CTAS) attn_digits_kernel(
+    const __grid_constant__ CUtensorMap tmap_k, const __grid_constant__ CUtensorMap tmap_v,
+    const __half* q, const __half* gate, const int* row_req, const int* row_pos,
+    const int* page_table, int max_pages, const __half* ks, const __half* vs,
+    __half* __restrict__ out, int qh, int kvh, int splits, float* __restrict__ scratch, int rep,
+    int apart_keys, int* status) {
+  using T = DigitTile<D>;
+  constexpr int G = T::G, KB = T::KB, KSTEPS = T::KSTEPS;
+  grid_wait();
+  grid_release();
+  const int row = blockIdx.x, split = blockIdx.z;
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  const int g = lane >> 2, t = lane & 3, upper = lane >> 4, head = g & 3;
+  const int kv_len = row_pos[row] + 1;
+  const bool apart = APART && kv_len <= apart_keys;
+  if (apart && (blockIdx.y & (ATTN_WARPS - 1)) != 0) return;
+  const int h = apart ? min(static_cast<int>(blockIdx.y) + warp, kvh - 1) : blockIdx.y;
+  const bool idle = apart && static_cast<int>(blockIdx.y) + warp >= kvh;
+  const int per = (kv_len + splits - 1) / splits;
+  const int k_lo = split * per, k_hi = min(kv_len, k_lo + per);
+  const int* pages = page_table + static_cast<size_t>(row_req[row]) * max_pages;
+
+  extern __shared__ unsigned char digits_smem[];
+  unsigned char* smem = digits_smem + ((1024u - (smem_u32(digits_smem) & 1023u)) & 1023u);
+  float(*s_o)[4][D] = reinterpret_cast<float(*)[4][D]>(smem);   // the warps' results, at the end
+  __shared__ float s_m[ATTN_WARPS][4], s_l[ATTN_WARPS][4];
+  __shared__ __align__(16) uint4 s_q[KSTEPS][32];
+  // scales of two blocks, K's and V's: [pair of keys][group][key of the pair]
+  __shared__ __align__(16) float s_scale[ATTN_WARPS][2][2][KB / 2][G][2];
+  __shared__ uint32_t s_raw[ATTN_WARPS][2][2][32];
+  __shared__ uint64_t bars[ATTN_WARPS][T::STAGES];
+  uint64_t* full = bars[warp];                     // K and V of a stage have landed
+
+  // the query: lane (g, t) holds channels 32 s + 4 t .. and 32 s + 16 + 4 t .. of its head
+  const __half* q_at = q + (static_cast<size_t>(row) * qh + h * rep + head) * D + 4 * t;
+  uint2 raw[KSTEPS][2];
+#pragma unroll
+  for (int s = 0; s < KSTEPS; ++s)
+#pragma unroll
+    for (int i = 0; i < 2; ++i)
+      raw[s][i] = head < rep ? *reinterpret_cast<const uint2*>(q_at + 32 * s + 16 * i)
+                             : make_uint2(0u, 0u);
+
+  // ---- this warp's ring; the first blocks are on their way before the query is looked at
+  const int step = apart ? 1 : ATTN_WARPS;
+  const int b_hi = k_hi > k_lo && !idle ? (k_hi + KB - 1) / KB : 0;
+  const int b0 = k_hi > k_lo ? k_lo / KB + (apart ? 0 : warp) : 0;
+  const int mine = b0 < b_hi ? (b_hi - b0 + step - 1) / step : 0;
+  // Page ids of this warp's blocks, a lane each, 32 blocks at a time and as many ahead: one that is
+  // fetched when it is needed holds up the copies and the scales behind it.
+  auto pages_from = [&](int n) {
+    return n + lane < mine ? pages[((b0 + (n + lane) * step) * KB) >> 7] : 0;
+  };
+  int page_ids = pages_from(0), page_ids_next = pages_from(32);
+  unsigned char* ring = smem + warp * T::STAGES * 2 * T::ROWS;
+  auto issue = [&](int n, int page) {              // one lane
+    unsigned char* to = ring + (n & 1) * 2 * T::ROWS;
+    const int slot = page * 128 + (((b0 + n * step) * KB) & 127);
+    mbar_expect_tx(&full[n & 1], 2 * T::ROWS);
+    tma_load_3d(to, &tmap_k, &full[n & 1], 0, h, slot);
+    tma_load_3d(to + T::ROWS, &tmap_v, &full[n & 1], 0, h, slot);
+  };
+  // The scales of key `lane` of a block as they lie in the cache, two blocks ahead of their use: by
+  // cp.async, since a load into a register that the loop moves on is waited for there.  One group's
+  // two bytes come with a neighbour's (the slots are an even number).
+  const uint32_t raw_u = smem_u32(&s_raw[warp][0][0][lane]);
+  auto fetch_scales = [&](int n, int page) {
+    const size_t slot =
+        static_cast<size_t>(page) * 128 + (((b0 + n * step) * KB) & 127) + lane;
+    const size_t at = (slot * kvh + h) * G & ~static_cast<size_t>(1);
+    const uint32_t to = raw_u + (n & 1) * 256;
+    asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"(to), "l"(ks + at) : "memory");
+    asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"(to + 128), "l"(vs + at)
+                 : "memory");
+  };
+  {
+    const int page0 = __shfl_sync(0xffffffffu, page_ids, 0);
+    const int page1 = __shfl_sync(0xffffffffu, page_ids, 1);
+    if (lane == 0) {
+      for (int i = 0; i < T::STAGES; ++i) mbar_init(&full[i], 1);
+      mbar_fence_init();
+      if (mine > 0) issue(0, page0);
+      if (mine > 1) issue(1, page1);
+    }
+    if (mine > 0) fetch_scales(0, page0);
+    asm volatile("cp.async.commit_group;" ::: "memory");
+    if (mine > 1) fetch_scales(1, page1);
+    asm volatile("cp.async.commit_group;" ::: "memory");
+  }
+
+  // ---- its digits: rows g and g + 8 of A are digits `upper` and 2 + `upper`
+  const uint32_t sel = upper ? 0x4062u : 0x5173u;  // their bytes in two numbers
+  float f_head;                                    // the unit of the second one's sums
+  uint32_t qa[KSTEPS][4];
+  {
+    __half2 big2 = __half2half2(__ushort_as_half(0));
+#pragma unroll
+    for (int s = 0; s < KSTEPS; ++s)
+#pragma unroll
+      for (int i = 0; i < 4; ++i)
+        big2 = __hmax2_nan(big2, __habs2(reinterpret_cast<const __half2*>(raw[s])[i]));
+    __half big_h = __hmax_nan(__low2half(big2), __high2half(big2));
+#pragma unroll
+    for (int o = 1; o < 4; o <<= 1)
+      big_h = __hmax_nan(big_h, __shfl_xor_sync(0xffffffffu, big_h, o));
+    const float big = __half2float(big_h);
+    const bool finite = big < INFINITY;
+    // |q| < 2^e and the fixed-point values below 2^30
+    const int e = max(-30, min(16, static_cast<int>(__float_as_uint(big) >> 23) - 126));
+    f_head = finite ? two_to(e - 30) * (upper ? 1.f : 256.f) : __int_as_float(0x7fc00000);
+    const float up = two_to(30 - e);
+#pragma unroll
+    for (int s = 0; s < KSTEPS; ++s) {
+      if (!apart && (s & (ATTN_WARPS - 1)) != warp) continue;
+      uint32_t(&a)[4] = qa[s];
+#pragma unroll
+      for (int i = 0; i < 2; ++i) {
+        uint32_t u[4];
+#pragma unroll
+        for (int j = 0; j < 4; ++j)
+          u[j] = static_cast<uint32_t>(__float2int_rn(
+                     __half2float(reinterpret_cast<const __half*>(&raw[s][i])[j]) * up)) +
+                 0x80808080u;
+        const uint32_t p01 = __byte_perm(u[0], u[1], sel), p23 = __byte_perm(u[2], u[3], sel);
+        a[2 * i] = __byte_perm(p01, p23, 0x5410) ^ 0x80808080u;
+        a[2 * i + 1] = __byte_perm(p01, p23, 0x7632) ^ 0x80808080u;
+      }
+      if (!apart) s_q[s][lane] = make_uint4(a[0], a[1], a[2], a[3]);
+    }
+  }
+  __syncthreads();
+  if (!apart) {
+#pragma unroll
+    for (int s = 0; s < KSTEPS; ++s) {
+      const uint4 v = s_q[s][lane];
+      qa[s][0] = v.x; qa[s][1] = v.y; qa[s][2] = v.z; qa[s][3] = v.w;
+    }
+  }
+  // A sum starts at 1.5 x 2^23, so that its bits are those of the float that much larger, and the
+  // bias leaves with the factors: (c + bias) w - bias (w + f) + (d + bias) f, exact up to the
+  // rounding of a float.
+  constexpr int BIAS = 0x4b400000;
+  const float w_top = f_head * 65536.f;
+  const float w_bias = -12582912.f * (w_top + f_head);
+
+  int acc[D / 8][4];
+#pragma unroll
+  for (int i = 0; i < D / 8; ++i)
+#pragma unroll
+    for (int j = 0; j < 4; ++j) acc[i][j] = 0;
+  float m_ref = -INFINITY, l_run = 0.f;
+  int e_run = -100;                                // the value scales seen are below 2^e_run
+  bool poison = false;                             // a value scale was no number
+  bool ok = true;
+
+  // row addresses of this lane: K's rows of tile i are keys 16 (i / 2) + key_of(row / 2, 2 (i % 2)
+  // + row % 2), four matrices of 16 bytes; V's are the keys of lane 16 m + 4 t + x
+  const uint32_t ring_u = smem_u32(ring);
+  const int kn = lane & 7, kt = (lane & 15) >> 2;
+  const int k_row[2] = {kn, 8 + ((kn + 4) & 7)};
+  const int v_row = 16 * (lane >> 4) + T::key_of(kt, lane & 3);
+  const float qscale = rsqrtf(static_cast<float>(D)) * 1.4426950408889634f;
+
+  // The scales of block n, by the lanes that fetched them, a block ahead of their use.  e_new and
+  // e_grows are that block's.
+  int e_new = -100;
+  bool e_grows = false;
+  auto place_scales = [&](int n) {
+    const int key = (b0 + n * step) * KB + lane;
+    const bool live = key >= k_lo && key < k_hi;
+    asm volatile("cp.async.wait_group 1;" ::: "memory");
+    uint32_t raw[2];
+#pragma unroll
+    for (int w = 0; w < 2; ++w) {
+      raw[w] = *reinterpret_cast<const volatile uint32_t*>(&s_raw[warp][n & 1][w][lane]);
+      if (G == 1 && ((lane & kvh) ^ h) & 1) raw[w] >>= 16;        // (a block's first slot is even)
+    }
+    const __half2 k2 = *reinterpret_cast<const __half2*>(&raw[0]);
+    const __half2 v2 = *reinterpret_cast<const __half2*>(&raw[1]);
+    float kf[G], vf[G];
+    uint32_t vbits = 0u;
+#pragma unroll
+    for (int c = 0; c < G; ++c) {
+      // keys outside the split: their (possibly never written) scales unused
+      kf[c] = live ? (c == 0 ? __low2float(k2) : __high2float(k2)) * qscale : 0.f;
+      vf[c] = live ? (c == 0 ? __low2float(v2) : __high2float(v2)) : 0.f;
+      vbits = max(vbits, __float_as_uint(fabsf(vf[c])));
+    }
+    vbits = __reduce_max_sync(0xffffffffu, vbits);
+    poison = poison || vbits >= 0x7f800000u;
+    const int e_block = min(static_cast<int>(vbits >> 23), 127 + 16) - 126;
+    const bool full_up = (n + 1) % DIGIT_BLOCKS == 0;
+    e_grows = e_block > e_new || full_up;
+    e_new = max(e_new, e_block) + (full_up ? 2 : 0);
+    const float unit = two_to(DIGIT_BITS - e_new);
+#pragma unroll
+    for (int c = 0; c < G; ++c) {
+      s_scale[warp][n & 1][0][lane >> 1][c][lane & 1] = kf[c];
+      s_scale[warp][n & 1][1][lane >> 1][c][lane & 1] = vf[c] * unit;
+    }
+  };
+  if (mine > 0) place_scales(0);
+  int page2 = __shfl_sync(0xffffffffu, page_ids, 2);
+  if (mine > 2) fetch_scales(2, page2);
+  asm volatile("cp.async.commit_group;" ::: "memory");
+
+  int n = 0;
+  for (; n < mine; ++n) {
+    const int key0 = (b0 + n * step) * KB, st = n & 1;
+    const bool edge = key0 < k_lo || key0 + KB > k_hi, grows = e_grows;
+    const int e_now = e_new;
+    ok = warp_all(mbar_wait(&full[st], (n >> 1) & 1, status, STATUS_TMA_WAIT, 0x20));
+    if (!ok) break;
+    __syncwarp();
+    // ---- scores: half m, this lane's key x of it
+    const uint32_t k_s = ring_u + st * 2 * T::ROWS, v_s = k_s + T::ROWS;
+    float s[2][4];
+    uint32_t kb[2][G][4];
+    auto load_k = [&](int i) {
+#pragma unroll
+      for (int c = 0; c < G; ++c)
+        asm volatile("ldmatrix.sync.aligned.m8n8.x4.shared.b16 {%0, %1, %2, %3}, [%4];"
+                     : "=r"(kb[i & 1][c][0]), "=r"(kb[i & 1][c][1]), "=r"(kb[i & 1][c][2]),
+                       "=r"(kb[i & 1][c][3])
+                     : "r"(k_s + T::unit(16 * (i >> 1) + k_row[i & 1], 4 * c + (lane >> 3)))
+                     : "memory");
+    };
+    load_k(0);
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+      int d[G][4];
+      if (i < 3) load_k(i + 1);
+#pragma unroll
+      for (int c = 0; c < G; ++c) {
+#pragma unroll
+        for (int e = 0; e < 4; ++e) d[c][e] = BIAS;
+        mma_s8(d[c], qa[2 * c], kb[i & 1][c][0], kb[i & 1][c][1]);
+      }
+#pragma unroll
+      for (int c = 0; c < G; ++c) mma_s8(d[c], qa[2 * c + 1], kb[i & 1][c][2], kb[i & 1][c][3]);
+      float kv[2 * G];
+      load_pair<G>(kv, s_scale[warp][st][0][8 * (i >> 1) + T::key_of(t, 2 * (i & 1)) / 2][0]);
+#pragma unroll
+      for (int e = 0; e < 2; ++e) {
+        float sum = 0.f;
+#pragma unroll
+        for (int c = 0; c < G; ++c) {
+          const float part = fmaf(__int_as_float(d[c][2 + e]), f_head,
+                                  fmaf(__int_as_float(d[c][e]), w_top, w_bias));
+          sum = c == 0 ? part * kv[e] : fmaf(part, kv[2 * c + e], sum);
+        }
+        s[i >> 1][2 * (i & 1) + e] = sum;
+      }
+    }
+    if (n + 1 < mine) place_scales(n + 1);
+    if ((n & 31) == 29) {                          // block n + 3 is the first of the next batch
+      page_ids = page_ids_next;
+      page_ids_next = pages_from((n | 31) + 33);
+    }
+    const int page3 = __shfl_sync(0xffffffffu, page_ids, (n + 3) & 31);
+    if (n + 3 < mine) fetch_scales(n + 3, page3);
+    asm volatile("cp.async.commit_group;" ::: "memory");
+#pragma unroll
+    for (int m = 0; m < 2; ++m)
+#pragma unroll
+      for (int x = 0; x < 4; ++x) s[m][x] += __shfl_xor_sync(0xffffffffu, s[m][x], 16);
+    if (edge) {
+#pragma unroll
+      for (int m = 0; m < 2; ++m)
+#pragma unroll
+        for (int x = 0; x < 4; ++x) {
+          const int key = key0 + 16 * m + T::key_of(t, x);
+          if (key < k_lo || key >= k_hi) s[m][x] = -INFINITY;
+        }
+    }
+    // ---- softmax state
+    float mb = s[0][0];
+#pragma unroll
+    for (int i = 1; i < 8; ++i) mb = fmaxf(mb, s[i >> 2][i & 3]);
+    mb = fmaxf(mb, __shfl_xor_sync(0xffffffffu, mb, 1));
+    mb = fmaxf(mb, __shfl_xor_sync(0xffffffffu, mb, 2));
+    if (__any_sync(0xffffffffu, mb > m_ref + DIGIT_LAG) || grows) {
+      const float m_new = mb > m_ref + DIGIT_LAG ? mb : m_ref;
+      const float corr = m_ref == -INFINITY ? 0.f : exp2f(m_ref - m_new);
+      const float f = corr * two_to(max(e_run - e_now, -126));
+      l_run *= corr;
+      if (n > 0) {
+        // two digits of a sum, 2^16 apart, as one number and back
+#pragma unroll
+        for (int i = 0; i < D / 8; ++i)
+#pragma unroll
+          for (int e = 0; e < 2; ++e) {
+            const float v = fmaf(static_cast<float>(acc[i][e]), 65536.f,
+                                 static_cast<float>(acc[i][2 + e])) * f;
+            const float top = rintf(v * (1.f / 65536.f));
+            acc[i][e] = __float2int_rn(top);
+            acc[i][2 + e] = __float2int_rn(fmaf(top, -65536.f, v));
+          }
+      }
+      m_ref = m_new;
+      e_run = e_now;
+    }
+    uint32_t a[G][4];
+#pragma unroll
+    for (int m = 0; m < 2; ++m) {
+#pragma unroll
+      for (int x = 0; x < 4; ++x) {
+        s[m][x] = ex2_ftz(s[m][x] - m_ref);
+        l_run += s[m][x];
+      }
+      float w[2][2 * G];                           // two pairs of keys
+#pragma unroll
+      for (int i = 0; i < 2; ++i)
+        load_pair<G>(w[i], s_scale[warp][st][1][8 * m + T::key_of(t, 2 * i) / 2][0]);
+#pragma unroll
+      for (int c = 0; c < G; ++c) {
+        uint32_t u[4];
+#pragma unroll
+        for (int x = 0; x < 4; ++x)
+          u[x] = static_cast<uint32_t>(__float2int_rn(s[m][x] * w[x >> 1][2 * c + (x & 1)])) +
+                 0x80808080u;
+        const uint32_t p01 = __byte_perm(u[0], u[1], sel), p23 = __byte_perm(u[2], u[3], sel);
+        a[c][2 * m] = __byte_perm(p01, p23, 0x5410) ^ 0x80808080u;
+        a[c][2 * m + 1] = __byte_perm(p01, p23, 0x7632) ^ 0x80808080u;
+      }
+    }
+    // ---- values
+    uint32_t vb[2][4];
+    auto load_v = [&](int j) {
+      asm volatile("ldmatrix.sync.aligned.m16n16.x2.trans.shared.b8 {%0, %1, %2, %3}, [%4];"
+                   : "=r"(vb[j & 1][0]), "=r"(vb[j & 1][1]), "=r"(vb[j & 1][2]), "=r"(vb[j & 1][3])
+                   : "r"(v_s + T::unit(v_row, j))
+                   : "memory");
+    };
+    load_v(0);
+#pragma unroll
+    for (int j = 0; j < D / 16; ++j) {
+      if (j + 1 < D / 16) load_v(j + 1);
+      mma_s8(acc[2 * j], a[j / 4], vb[j & 1][0], vb[j & 1][2]);
+      mma_s8(acc[2 * j + 1], a[j / 4], vb[j & 1][1], vb[j & 1][3]);
+    }
+    __syncwarp();
+    if (lane == 0 && n + T::STAGES < mine) issue(n + T::STAGES, page2);
+    page2 = page3;
+  }
+  // a warp that gave up waits for what it has in flight
+  if (!ok)
+    for (int i = n; i < mine && i < n + T::STAGES; ++i)
+      mbar_wait(&full[i & 1], (i >> 1) & 1, status, STATUS_TMA_WAIT, 0x22);
+  __syncthreads();                               // the rings become the result buffers
+  // ---- this warp's result, back to the unscaled weights
+  l_run += __shfl_xor_sync(0xffffffffu, l_run, 1);
+  l_run += __shfl_xor_sync(0xffffffffu, l_run, 2);
+  const float back = poison ? __int_as_float(0x7fc00000)
+                            : two_to(max(e_run - DIGIT_BITS, -126)) * (upper ? 1.f : 256.f);
+#pragma unroll
+  for (int j = 0; j < D / 8; ++j) {
+    float v[2];
+#pragma unroll
+    for (int e = 0; e < 2; ++e) {
+      v[e] = fmaf(static_cast<float>(acc[j][e]), 65536.f, static_cast<float>(acc[j][2 + e])) * back;
+      v[e] += __shfl_xor_sync(0xffffffffu, v[e], 16);
+    }
+    if (upper == (j & 1))
+      *reinterpret_cast<float2*>(&s_o[warp][head][8 * j + 2 * t]) = make_float2(v[0], v[1]);
+  }
+  if (lane < 16 && t == 0) {
+    s_m[warp][head] = m_ref;
+    s_l[warp][head] = l_run;
+  }
+  attn_finish<D, 4>(s_o, s_m, s_l, apart, idle, rep, row, h, qh, split, splits, gate, out, scratch);
+}
+
 // One CTA per row and head.  The records' maxima and sums are read by a lane each and handed round,
-// the outputs eight records at a time, since a call of few rows waits for each load in turn: with a
-// record per step of the loop, and attn_finish computing every factor anew for each channel, one row
-// of 2000 keys and 32 / 8 heads of 128 took 10.7 us (now 8.3), 16 / 2 heads of 256 (32 records) 15.1
-// (10.0), 64 rows of 640 keys unsplit 26.8 (22.9).
+// the outputs eight records at a time, since a call of few rows waits for each load in turn: with
+// a record per step of the loop, and attn_finish computing every factor anew for each channel, one
+// row of 2000 keys and 32 / 8 heads of 128 took 10.7 us (now 8.3), 16 / 2 heads of 256 (32 records)
+// 15.1 (10.0), 64 rows of 640 keys unsplit 26.8 (22.9).
 template <int D>
 __global__ void attn_merge_kernel(
     const float* scratch, const __half* gate, __half* __restrict__ out, int qh, int splits) {
@@ -487,6 +944,36 @@ inline bool attn_starts_early(int head_dim, long long ctas) {
   return head_dim > 128 || ctas <= 148 || ctas >= 312;
 }
 
+// Up to four query heads per KV head fill the sixteen rows of digits; five and more would take a
+// second tile and twice the accumulators, and channels above 128 have no room for theirs.  A CTA
+// should have ten blocks or more, as far as the page table's width tells: the digits of a query and
+// the sums' way back cost what a few blocks save (8 rows of 300 keys 7.0 us both ways, 1 row of 100
+// 3.6 and 3.8, of 2000 in 32 splits 8.3 and 8.2; 64 rows of 300 17.6 and 15.5).
+constexpr int DIGIT_MIN_KEYS = 320;
+inline bool attn_digits(int head_dim, int rep, int max_pages, int splits, bool wide, const void* kc,
+                        const void* vc) {
+  const long long keys = static_cast<long long>(max_pages) * 128 / splits;
+  return head_dim <= 128 && rep <= 4 && wide && keys >= DIGIT_MIN_KEYS &&
+         ((reinterpret_cast<uintptr_t>(kc) | reinterpret_cast<uintptr_t>(vc)) & 15) == 0;
+}
+
+// The cache as [slots][heads][D] bytes, in boxes of 32 keys of a head.  Which pages are there only
+// the page table knows, so the number of slots is left open.
+template <int D>
+static bool kv_map(CUtensorMap* map, const int8_t* cache, int kvh) {
+  PFN_encodeTiled enc = runtime_tma_encoder();
+  if (!enc) return false;
+  cuuint64_t dims[3] = {static_cast<cuuint64_t>(D), static_cast<cuuint64_t>(kvh), 1ull << 31};
+  cuuint64_t strides[2] = {static_cast<cuuint64_t>(D), static_cast<cuuint64_t>(kvh) * D};
+  cuuint32_t box[3] = {static_cast<cuuint32_t>(D), 1, 32};
+  cuuint32_t estr[3] = {1, 1, 1};
+  return enc(map, CU_TENSOR_MAP_DATA_TYPE_UINT8, 3, const_cast<int8_t*>(cache), dims, strides, box,
+             estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
+             D == 128 ? CU_TENSOR_MAP_SWIZZLE_128B : CU_TENSOR_MAP_SWIZZLE_64B,
+             CU_TENSOR_MAP_L2_PROMOTION_L2_128B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) ==
+         CUDA_SUCCESS;
+}
+
 template <int D>
 static int launch_attn(const __half* q, const __half* gate, const int* row_req, const int* row_pos,
                        const int* page_table, int max_pages, const int8_t* kc, const int8_t* vc,
@@ -495,25 +982,39 @@ static int launch_attn(const __half* q, const __half* gate, const int* row_req, 
   dim3 grid(rows, kvh, splits);
   const bool wide = ((reinterpret_cast<uintptr_t>(q) & 15) | (reinterpret_cast<uintptr_t>(ks) & 7) |
                      (reinterpret_cast<uintptr_t>(vs) & 7)) == 0;
-  constexpr int SMEM = AttnTile<D>::SMEM;
   const long long ctas = splits > 1 || kvh < ATTN_WARPS ? 0 : static_cast<long long>(rows) * kvh;
   const long long waves = ctas / (148 * AttnTile<D>::MIN_CTAS);
   const int apart_keys = AttnTile<D>::KB * static_cast<int>(waves < 4 ? waves : 4);
   const bool apart = apart_keys > 0;
-  auto kernel =
-      wide ? (apart ? attn_rows_kernel<D, true, true> : attn_rows_kernel<D, true, false>)
-           : (apart ? attn_rows_kernel<D, false, true> : attn_rows_kernel<D, false, false>);
   if (runtime_ensure_init() != cudaSuccess) return -2;
-  static const int slot[4] = {runtime_new_slot(), runtime_new_slot(), runtime_new_slot(),
-                              runtime_new_slot()};
-  if (const int e = runtime_allow_smem(slot[2 * apart + wide], kernel, SMEM)) return e;
-  if (attn_starts_early(D, static_cast<long long>(rows) * kvh * splits))
-    launch_early(kernel, grid, ATTN_WARPS * 32, SMEM, stream, q, gate, row_req, row_pos, page_table,
-                 max_pages, kc, vc, ks, vs, out, qh, kvh, splits, scratch, rep, apart_keys);
-  else
-    kernel<<<grid, ATTN_WARPS * 32, SMEM, stream>>>(q, gate, row_req, row_pos, page_table,
-                                                    max_pages, kc, vc, ks, vs, out, qh, kvh,
-                                                    splits, scratch, rep, apart_keys);
+  const bool early = attn_starts_early(D, static_cast<long long>(rows) * kvh * splits);
+  auto start = [&](auto kernel, size_t smem, auto... args) {
+    if (early)
+      launch_early(kernel, grid, ATTN_WARPS * 32, smem, stream, args...);
+    else
+      kernel<<<grid, ATTN_WARPS * 32, smem, stream>>>(args...);
+  };
+  CUtensorMap tk, tv;
+  if (attn_digits(D, rep, max_pages, splits, wide, kc, vc) && kv_map<D>(&tk, kc, kvh) &&
+      kv_map<D>(&tv, vc, kvh)) {
+    constexpr int D_ = D == 256 ? 128 : D;         // (256 channels: never)
+    auto kernel = apart ? attn_digits_kernel<D_, true> : attn_digits_kernel<D_, false>;
+    static const int slot[2] = {runtime_new_slot(), runtime_new_slot()};
+    constexpr int SMEM = DigitTile<D_>::SMEM;
+    if (const int e = runtime_allow_smem(slot[apart], kernel, SMEM)) return e;
+    start(kernel, SMEM, tk, tv, q, gate, row_req, row_pos, page_table, max_pages, ks, vs, out, qh,
+          kvh, splits, scratch, rep, apart_keys, runtime_status_ptr());
+  } else {
+    auto kernel =
+        wide ? (apart ? attn_rows_kernel<D, true, true> : attn_rows_kernel<D, true, false>)
+             : (apart ? attn_rows_kernel<D, false, true> : attn_rows_kernel<D, false, false>);
+    static const int slot[4] = {runtime_new_slot(), runtime_new_slot(), runtime_new_slot(),
+                                runtime_new_slot()};
+    constexpr int SMEM = AttnTile<D>::SMEM;
+    if (const int e = runtime_allow_smem(slot[2 * apart + wide], kernel, SMEM)) return e;
+    start(kernel, SMEM, q, gate, row_req, row_pos, page_table, max_pages, kc, vc, ks, vs, out, qh,
+          kvh, splits, scratch, rep, apart_keys);
+  }
   if (splits > 1)
     launch_early(attn_merge_kernel<D>, dim3(rows, qh), D < 128 ? 64 : 128, 0, stream, scratch, gate,
                  out, qh, splits);
@@ -532,6 +1033,13 @@ extern "C" size_t orinfer_attention_scratch_bytes(int rows, int qh, int head_dim
 // Whether the row kernel of such a call may start ahead of the end of the kernel in front.
 extern "C" int orinfer_attention_starts_early(int rows, int kvh, int head_dim, int splits) {
   return attn_starts_early(head_dim, static_cast<long long>(rows) * kvh * splits) ? 1 : 0;
+}
+
+// Whether such a call takes the digit form (given aligned tensors).
+extern "C" int orinfer_attention_in_digits(int qh, int kvh, int head_dim, int max_pages,
+                                           int splits) {
+  if (kvh <= 0 || qh % kvh || splits < 1) return 0;
+  return attn_digits(head_dim, qh / kvh, max_pages, splits, true, nullptr, nullptr) ? 1 : 0;
 }
 
 extern "C" int orinfer_attention(const __half* q, const __half* gate, const int* row_req,

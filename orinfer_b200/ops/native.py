@@ -58,6 +58,7 @@ def _load() -> ctypes.CDLL:
         "orinfer_e8p_encode": ([P, P, c_longlong, P], I),
         "orinfer_router_topk": ([P, P, I, I, I, I, I, I, P, P, P, P], I),
         "orinfer_attention_starts_early": ([I, I, I, I], I),
+        "orinfer_attention_in_digits": ([I, I, I, I, I], I),
         "orinfer_moe_dispatch": ([P, I, I, I, P, P, I, P, P, P, P, I, P, P, P, P], I),
         "orinfer_moe_combine": ([P, P, P, I, I, P, P, P, I, P], I),
         "orinfer_qgemm_grouped": ([I, P, P, P, P, P, I, I, I, I, P, P, I, P, I, I], I),

@@ -251,3 +251,116 @@ def test_attention_prefill_adds_weights_in_the_order_of_keys(dev, d, kvh, qh, ro
     chunk = torch.tensor([[0, rows, 0, 0]], dtype=torch.int32, device=dev)
     assert F.attention_prefill(q, None, chunk, rows, table, kc, vc, ks, vs, out=out)
     assert bool((out[1:step] == 1 + 2.0 ** -9).all())
+
+
+def _walk(dev, n, qh, kvh, d, seed, grow=0.0):
+    """One request of n keys whose scores and value scales grow along the context."""
+    g = torch.Generator().manual_seed(seed)
+    pages = (n + 127) // 128
+    table = (torch.randperm(pages, generator=g) + 1).to(torch.int32)[None].to(dev)
+    shape = (pages + 1, 128, kvh)
+    kc = torch.randint(-127, 128, (*shape, d), generator=g, dtype=torch.int8).to(dev)
+    vc = torch.randint(-127, 128, (*shape, d), generator=g, dtype=torch.int8).to(dev)
+    up = torch.zeros(shape[:2])
+    up[table[0].long().cpu()] = (torch.arange(pages * 128).view(pages, 128) / n * grow)
+    ks = ((torch.rand(*shape, d // 64, generator=g) * 0.02 + 1e-3) * (1 + up)[..., None, None])
+    vs = torch.rand(*shape, d // 64, generator=g) * 0.02 * torch.exp2(up)[..., None, None]
+    q = torch.randn(1, qh, d, generator=g).half().to(dev)
+    one = torch.zeros(1, dtype=torch.int32, device=dev)
+    return q, one, one + n - 1, table, kc, vc, ks.half().to(dev), vs.half().to(dev)
+
+
+def _in_digits(qh, kvh, d, table, splits):
+    from orinfer_b200.ops import native
+    return bool(native.lib().orinfer_attention_in_digits(qh, kvh, d, table.shape[1], splits))
+
+
+# contexts of a warp around 32 blocks, where it fetches the next page ids, references that move with
+# the context, an odd and an even number of heads
+@pytest.mark.parametrize("qh,kvh,d", [(4, 1, 128), (6, 3, 64), (4, 2, 64), (3, 3, 128), (8, 1, 128)])
+@pytest.mark.parametrize("n", [3713, 3968, 4096, 4129, 8257, 12400])
+@pytest.mark.parametrize("grow,splits", [(0.0, 1), (6.0, 1), (6.0, 5)])
+def test_attention_rows_walk_many_pages(dev, qh, kvh, d, n, grow, splits):
+    from orinfer_b200.ops import functional as F
+    q, req, pos, table, kc, vc, ks, vs = _walk(dev, n, qh, kvh, d, n + qh, grow)
+    assert _in_digits(qh, kvh, d, table, splits) == (qh // kvh <= 4)
+    out = F.attention(q, None, req, pos, table, kc, vc, ks, vs, splits=splits).view(-1)
+    pick = lambda c: c[table[0].long()].reshape(-1, *c.shape[2:])[:n]
+    ref = _attention64(q[0], pick(kc), pick(vc), pick(ks), pick(vs)).reshape(-1)
+    lim = ref.abs() * 2.0 ** -11 + 2.0 ** -18 * ref.abs().max() + 2.0 ** -25
+    assert bool(((out.double() - ref).abs() <= lim).all())
+
+
+def test_attention_rows_sums_of_a_long_context_do_not_overflow(dev):
+    """Weights, values and scales alike: integer sums grow as fast as they can, past the 65536 keys of
+    a warp after which they are scaled down."""
+    from orinfer_b200.ops import functional as F
+    n, kvh, d = 600_000, 1, 64
+    pages = (n + 127) // 128
+    table = torch.arange(pages, dtype=torch.int32, device=dev)[None]
+    assert _in_digits(4, kvh, d, table, 1)
+    for value, scale in ((127, 0.0117), (-127, 0.00781)):
+        kc = torch.zeros(pages, 128, kvh, d, dtype=torch.int8, device=dev)
+        vc = torch.full_like(kc, value)
+        s = torch.full((pages, 128, kvh, 1), scale, device=dev).half()
+        q = torch.ones(1, 4, d, device=dev).half()
+        one = torch.zeros(1, dtype=torch.int32, device=dev)
+        out = F.attention(q, None, one, one + n - 1, table, kc, vc, s, s, splits=1)
+        want = value * float(s[0, 0, 0, 0])
+        # one FP16 rounding, and FP32 sums of 150 000 equal weights per warp (2^-24 each at worst
+        # of the sum so far: 2^-9 in all, which both sums, of weights and of values, share)
+        assert bool(((out.double() - want).abs() <= abs(want) * 2.0 ** -8).all()), out
+
+
+@pytest.mark.parametrize("bad", [float("inf"), float("nan")])
+def test_attention_rows_keep_the_other_heads_of_a_bad_query(dev, bad):
+    from orinfer_b200.ops import functional as F
+    q, req, pos, table, kc, vc, ks, vs = _walk(dev, 300, 8, 2, 128, 5)
+    assert _in_digits(8, 2, 128, table, 1)
+    good = F.attention(q, None, req, pos, table, kc, vc, ks, vs, splits=1).view(8, 128)
+    q[0, 2, 77] = bad
+    out = F.attention(q, None, req, pos, table, kc, vc, ks, vs, splits=1).view(8, 128)
+    keep = torch.arange(8, device=dev) != 2
+    assert torch.equal(out[keep], good[keep])
+    assert not torch.equal(out[2], good[2])
+
+
+# a query whose values span all of FP16, down to the smallest: rounded at 2^-31 of the largest
+def test_attention_rows_of_a_query_of_many_binades(dev):
+    from orinfer_b200.ops import functional as F
+    for top in (0.0, 12.0):
+        q, req, pos, table, kc, vc, ks, vs = _walk(dev, 800, 4, 1, 128, 9)
+        assert _in_digits(4, 1, 128, table, 2)
+        g = torch.Generator().manual_seed(1)
+        q = (q.float() * torch.exp2(top - torch.rand(q.shape, generator=g).to(dev) * 30)).half()
+        ks = (ks.float() * 2.0 ** -top).half()
+        out = F.attention(q, None, req, pos, table, kc, vc, ks, vs, splits=2).view(-1)
+        pick = lambda c: c[table[0].long()].reshape(-1, *c.shape[2:])[:800]
+        ref = _attention64(q[0], pick(kc), pick(vc), pick(ks), pick(vs)).reshape(-1)
+        lim = ref.abs() * 2.0 ** -11 + 2.0 ** -18 * ref.abs().max() + 2.0 ** -25
+        assert bool(((out.double() - ref).abs() <= lim).all())
+
+
+# the forms of short contexts again, with a page table wide enough for the digit form
+@pytest.mark.parametrize("qh,kvh,d", [(8, 8, 64), (14, 7, 64), (5, 5, 128), (32, 8, 128)])
+@pytest.mark.parametrize("waves", [0.9, 1.1, 2.1, 4.2])
+def test_attention_rows_of_short_contexts_in_digits(dev, qh, kvh, d, waves):
+    from orinfer_b200.ops import functional as F
+    lens = [1, 2, 15, 16, 17, 31, 32, 33, 48, 49, 63, 64, 65, 96, 97, 127, 128, 129, 160, 256]
+    rows = int(waves * 148 * {64: 4, 128: 3}[d] / kvh)
+    q, req, pos, table, kc, vc, ks, vs = _short_rows(dev, rows, qh, kvh, d, lens)
+    for i, n in enumerate(lens):                    # slots never written hold anything
+        if n % 128:
+            page = table[i, (n - 1) // 128].long()
+            ks[page, (n - 1) % 128 + 1:] = float("nan")
+            vs[page, (n - 1) % 128 + 1:] = float("inf")
+    wide = torch.cat([table, torch.zeros_like(table)], 1)
+    assert _in_digits(qh, kvh, d, wide, 1)
+    out = F.attention(q[req.long()].contiguous(), None, req, pos, wide, kc, vc, ks, vs,
+                      splits=1).view(rows, qh * d)
+    for i, n in enumerate(lens[:rows]):
+        pick = lambda c: c[table[i].long()].reshape(-1, *c.shape[2:])[:n]
+        ref = _attention64(q[i], pick(kc), pick(vc), pick(ks), pick(vs)).reshape(-1)
+        lim = ref.abs() * 2.0 ** -11 + 2.0 ** -18 * ref.abs().max() + 2.0 ** -25
+        got = out[i::len(lens)].double()
+        assert bool(((got - ref).abs() <= lim).all()), n
