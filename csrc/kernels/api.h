@@ -228,6 +228,7 @@ int orinfer_gdn_conv(const __half* x, int x_stride, const __half* weight, __half
                      const int* row_first, const int* row_slot, const int* row_pos,
                      const int* segs, int n_segs, int rows, int hk, int hv, int head_dim, __half* y,
                      cudaStream_t stream, int update_history);
+int orinfer_gdn_pipelined(int hv, int n_segs, int max_seg_rows);
 int orinfer_gdn_scan(const __half* qkv, const float* ab, const float* a_log, const float* dt_bias,
                      const int* segs, int n_segs, const int* row_slot, const int* row_pos, int hk,
                      int hv, int head_dim, float* state, float* out, cudaStream_t stream,

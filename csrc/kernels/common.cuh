@@ -598,6 +598,36 @@ void launch_early(void (*kernel)(P...), dim3 grid, dim3 block, size_t smem, cuda
 }
 
 // ---------------------------------------------------------------- math
+// Two FP32 operations by one instruction, each rounded as by itself: no quicker in the pipe, but
+// one issue slot instead of two.
+__device__ __forceinline__ unsigned long long pair_bits(float2 a) {
+  unsigned long long r;
+  asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(a.x), "f"(a.y));
+  return r;
+}
+__device__ __forceinline__ float2 pair_of(unsigned long long r) {
+  float2 a;
+  asm("mov.b64 {%0, %1}, %2;" : "=f"(a.x), "=f"(a.y) : "l"(r));
+  return a;
+}
+__device__ __forceinline__ float2 fma2(float2 a, float2 b, float2 c) {
+  unsigned long long d;
+  asm("fma.rn.f32x2 %0, %1, %2, %3;"
+      : "=l"(d)
+      : "l"(pair_bits(a)), "l"(pair_bits(b)), "l"(pair_bits(c)));
+  return pair_of(d);
+}
+__device__ __forceinline__ float2 mul2(float2 a, float2 b) {
+  unsigned long long d;
+  asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(d) : "l"(pair_bits(a)), "l"(pair_bits(b)));
+  return pair_of(d);
+}
+__device__ __forceinline__ float2 add2(float2 a, float2 b) {
+  unsigned long long d;
+  asm("add.rn.f32x2 %0, %1, %2;" : "=l"(d) : "l"(pair_bits(a)), "l"(pair_bits(b)));
+  return pair_of(d);
+}
+
 __device__ __forceinline__ float warp_sum(float v) {
 #pragma unroll
   for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);

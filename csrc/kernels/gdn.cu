@@ -12,15 +12,9 @@
 // (kernels/cuda/model/gdn_sequence.py:19-250) and gated_norm (op17_gdn_gated_norm.py:15-71).
 #include "api.h"
 #include "common.cuh"
+#include "gdn_chunk.cuh"
 
 namespace orinfer {
-
-// The state slot of a segment is row_slot[row_start]; a segment whose first row sits at
-// position 0 of its request starts from a zero state and a zero history, so a reused slot
-// needs no reset.
-struct Segment {
-  int row_start, rows, pad0, pad1;
-};
 
 // ---------------------------------------------------------------- small projection
 __global__ void __launch_bounds__(256) small_proj_kernel(
@@ -508,8 +502,7 @@ __global__ void __launch_bounds__(256) gdn_scan_split_kernel(
 // Runs below GDN_LONG_ROWS keep the scan: one run of 36 rows takes 17.2 us there and 19.4 here, of
 // 40 rows 19.4 both ways, of 63 rows 28.0 and 19.4 (two runs of 50: 33 and 20).  The scan's bits
 // are those of a verification pass, whose segments are shorter.
-constexpr int GDN_LONG_ROWS = 40;
-constexpr int CHUNK = 32, CHUNK_THREADS = 192;
+constexpr int CHUNK_THREADS = 192;
 struct ChunkSmem {
   __half k[3][CHUNK][136], q[3][CHUNK][136];   // rows padded to 17 16-byte units (ldmatrix)
   __half v[3][CHUNK][72];
@@ -519,37 +512,6 @@ struct ChunkSmem {
   float eg[2][CHUNK], beta[2][CHUNK], tail[2][CHUNK], total[2];
 };
 
-__device__ __forceinline__ void ldsm_x4(uint32_t (&r)[4], const void* p) {
-  asm volatile("ldmatrix.sync.aligned.m8n8.x4.shared.b16 {%0, %1, %2, %3}, [%4];"
-               : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3])
-               : "r"(smem_u32(p))
-               : "memory");
-}
-__device__ __forceinline__ void ldsm_x4_t(uint32_t (&r)[4], const void* p) {
-  asm volatile("ldmatrix.sync.aligned.m8n8.x4.trans.shared.b16 {%0, %1, %2, %3}, [%4];"
-               : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3])
-               : "r"(smem_u32(p))
-               : "memory");
-}
-// D += A B on 16 x 8 x 8 TF32 tiles: lane (g, t) holds A rows g, g + 8 at k = t (a0, a1) and
-// k = t + 4 (a2, a3), B column g at k = t and t + 4.
-__device__ __forceinline__ void mma_tf32(float (&c)[4], const uint32_t (&a)[4], uint32_t b0,
-                                         uint32_t b1) {
-  asm volatile(
-      "mma.sync.aligned.m16n8k8.row.col.f32.tf32.tf32.f32 {%0, %1, %2, %3}, {%4, %5, %6, %7}, "
-      "{%8, %9}, {%0, %1, %2, %3};"
-      : "+f"(c[0]), "+f"(c[1]), "+f"(c[2]), "+f"(c[3])
-      : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1));
-}
-__device__ __forceinline__ uint32_t to_tf32(float x) {
-  uint32_t r;
-  asm("cvt.rna.tf32.f32 %0, %1;" : "=r"(r) : "f"(x));
-  return r;
-}
-__device__ __forceinline__ void split_tf32(float x, uint32_t& hi, uint32_t& lo) {
-  hi = to_tf32(x);
-  lo = to_tf32(x - __uint_as_float(hi));
-}
 // FP16 head and remainder of two values (already scaled into the FP16 range)
 __device__ __forceinline__ void split_half2(float x, float y, uint32_t& hi, uint32_t& lo) {
   const __half2 h = __floats2half2_rn(x, y);
@@ -565,26 +527,6 @@ __device__ __forceinline__ void split_half3(float x, float y, uint32_t& hi, uint
   hi = *reinterpret_cast<const uint32_t*>(&h);
   split_half2(x - f.x, y - f.y, mid, lo);
 }
-// largest value of the four lanes that share a row
-__device__ __forceinline__ float quad_max(float x) {
-  x = fmaxf(x, __shfl_xor_sync(0xffffffffu, x, 1));
-  return fmaxf(x, __shfl_xor_sync(0xffffffffu, x, 2));
-}
-// e with |x| < 2^e (at least -100, at most 129) and powers of two
-__device__ __forceinline__ int bound_exp(float x) {
-  return max(-100, static_cast<int>((__float_as_uint(x) >> 23) & 255u) - 126);
-}
-__device__ __forceinline__ float pow2i(int e) {
-  return __uint_as_float(static_cast<uint32_t>(127 + e) << 23);
-}
-
-// e^x, x FP64: the FP32 exponential of the rounded argument, corrected by what the rounding lost
-__device__ __forceinline__ float exp_pair(double x) {
-  const float hi = static_cast<float>(x);
-  const float e = expf(hi);
-  return fmaf(e, static_cast<float>(x - static_cast<double>(hi)), e);
-}
-
 // D[i][0..7] (u-th group of eight columns) += X^T(16 x 32) M^T for a 32 x 32 matrix M in shared
 // memory with zeros on and above the diagonal: X and M split into TF32 pairs.  A zero does not
 // hide an infinity or a NaN of a later row in a tensor-core product, so a block on the diagonal
@@ -1128,11 +1070,22 @@ static void launch_history(const __half* x, int x_stride, const Segment* segs, i
                  x_stride, segs, row_slot, row_pos, conv_dim, hist, accepted);
 }
 
+// Whether long runs take the kernel of gdn_pipe.cu: where its CTAs have an SM each, or the runs are
+// long enough to make up for their waves (figures there).  A caller that does not know the longest run
+// gives the rows in all.
+static bool gdn_pipelined(int hv, int n_segs, int max_seg_rows) {
+  return 2LL * hv * n_segs <= 148 || max_seg_rows >= 384LL * n_segs;
+}
+
 }  // namespace orinfer
 
 using namespace orinfer;
 
 extern "C" {
+
+int orinfer_gdn_pipelined(int hv, int n_segs, int max_seg_rows) {
+  return gdn_pipelined(hv, n_segs, max_seg_rows) ? 1 : 0;
+}
 
 int orinfer_small_proj(const __half* x, const __half* w, float* out, int rows, int hidden, int n,
                        cudaStream_t stream) {
@@ -1208,13 +1161,18 @@ int orinfer_gdn_scan(const __half* qkv, const float* ab, const float* a_log, con
   if (head_dim == 128 && factors == nullptr && aligned(qkv, 16) &&
       max_seg_rows >= (n_segs == 1 ? GDN_LONG_ROWS : 64)) {
     long_rows = GDN_LONG_ROWS;
-    static const int slot = runtime_new_slot();
-    if (const int e = runtime_allow_smem(slot, gdn_chunk_kernel, sizeof(ChunkSmem))) return e;
-    // Not early: its few long CTAs would gather, two to an SM, where the kernel before ends first
-    // (the mixer of two runs of 1050 rows 260 us, 245 so, each in turn on one card; of two of 1500
-    // rows 357 and 335).
-    gdn_chunk_kernel<<<dim3(hv * 2, n_segs), CHUNK_THREADS, sizeof(ChunkSmem), stream>>>(
-        qkv, conv_dim, ab, a_log, dt_bias, sg, row_slot, row_pos, hk, hv, state, out);
+    if (gdn_pipelined(hv, n_segs, max_seg_rows)) {
+      if (const int e = gdn_pipe_launch(qkv, conv_dim, ab, a_log, dt_bias, sg, n_segs, row_slot,
+                                        row_pos, hk, hv, state, out, stream))
+        return e;
+    } else {
+      static const int slot = runtime_new_slot();
+      if (const int e = runtime_allow_smem(slot, gdn_chunk_kernel, sizeof(ChunkSmem))) return e;
+      // Not early: its few long CTAs would gather, two to an SM, where the kernel before ends
+      // first (the mixer of two runs of 1050 rows 260 us, 245 so, of two of 1500 357 and 335).
+      gdn_chunk_kernel<<<dim3(hv * 2, n_segs), CHUNK_THREADS, sizeof(ChunkSmem), stream>>>(
+          qkv, conv_dim, ab, a_log, dt_bias, sg, row_slot, row_pos, hk, hv, state, out);
+    }
   }
 #define ORINFER_SCAN(KERNEL, GRID_X)                                                       \
   launch_early(KERNEL, dim3(GRID_X, n_segs), 256, 0, stream, qkv, conv_dim, ab, a_log,     \

@@ -229,3 +229,82 @@ def test_gdn_chunks_contain_non_finite_rows(dev, what, row):
         assert torch.equal(torch.isfinite(got), fine)
         diff = (got.double() - want)[fine]
         assert float(diff.norm() / want[fine].norm()) < 1e-6
+
+
+def _runs(dev, lens, hv, strength, seed):
+    """A packet of runs, every other one continued: the arguments of a scan and its 64-bit answer."""
+    g = torch.Generator().manual_seed(seed)
+    rand = lambda *n: torch.randn(*n, generator=g).to(dev)
+    hk, d, rows = max(1, hv // 2), 128, sum(lens)
+    a_log, dt = rand(hv) * 0.5 + strength, rand(hv) * 0.5 - 2
+    ab = rand(rows, 2 * hv)
+    qk = torch.nn.functional.normalize(rand(rows, 2 * hk, d), dim=-1)
+    qkv = torch.cat([qk.reshape(rows, -1), rand(rows, hv * d)], 1).half()
+    state = rand(len(lens), hv, d, d) * 0.2
+    segs, slot, pos, at = [], [], [], 0
+    for i, n in enumerate(lens):
+        segs.append([at, n, 0, 0])
+        slot += [i] * n
+        pos += list(range(50 * (i % 2), 50 * (i % 2) + n))
+        at += n
+    t = lambda x: torch.tensor(x, dtype=torch.int32, device=dev)
+    part = lambda i: qkv[:, i * hk * d:(i + 1) * hk * d].double().reshape(rows, hk, d)
+    log_decay = -torch.exp(a_log.double()) * torch.nn.functional.softplus(
+        ab[:, :hv].double() + dt.double(), threshold=60)
+
+    def exact(i):
+        sl = slice(segs[i][0], segs[i][0] + lens[i])
+        return _recurrence64(part(0)[sl].repeat_interleave(hv // hk, 1) / math.sqrt(d),
+                             part(1)[sl].repeat_interleave(hv // hk, 1),
+                             qkv[sl, 2 * hk * d:].double().reshape(lens[i], hv, d), log_decay[sl],
+                             torch.sigmoid(ab[sl, hv:].double()),
+                             start[i].double() * (i % 2)) + (sl,)
+
+    start = state.clone()
+    args = (qkv, ab, a_log, dt, t(segs), len(lens), t(slot), t(pos), hk, hv, d, state)
+    return args, state, exact
+
+
+# both chunked kernels over the same lengths: alone on their SMs, and with more CTAs than SMs
+@pytest.mark.parametrize("n", [40, 63, 64, 65, 95, 97, 129, 257, 383, 384])
+@pytest.mark.parametrize("many", [False, True])
+def test_gdn_chunked_kernels_over_their_lengths(dev, n, many):
+    from orinfer_b200.ops import functional as F
+    from orinfer_b200.ops import native
+    hv = 8
+    lens = [n, 41] if not many else [n, 41, 64] * 4
+    assert native.lib().orinfer_gdn_pipelined(hv, len(lens), sum(lens)) == int(not many)
+    args, state, exact = _runs(dev, lens, hv, -1.0, n)
+    out = F.gdn_scan(*args)
+    for i in range(len(lens)):
+        ref, s, sl = exact(i)
+        # as in test_gdn_chunks_keep_fp32_accuracy, over a whole run
+        assert float((out[sl].double() - ref).norm() / ref.norm()) < 2.0 ** -21
+        assert float((state[i].double() - s).norm() / s.norm()) < 2.0 ** -21
+
+
+@pytest.mark.parametrize("row", [3, 45, 95])
+def test_gdn_many_runs_contain_non_finite_rows(dev, row):
+    from orinfer_b200.ops import functional as F
+    lens = [96] * 12
+    args, state, _ = _runs(dev, lens, 8, -1.0, row)
+    fine = F.gdn_scan(*[a.clone() if torch.is_tensor(a) else a for a in args])
+    args[0][96 * 5 + row, 2 * 4 * 128 + 2 * 128 + 9] = math.inf           # a value of run 5, head 2
+    out = F.gdn_scan(*args)
+    bad = torch.zeros_like(out, dtype=torch.bool)
+    bad[96 * 5 + row:96 * 6, 2, 9] = True
+    assert torch.equal(torch.isfinite(out), ~bad)
+    # the sums of its warp are made in another order
+    assert float((out - fine)[~bad].norm() / fine[~bad].norm()) < 1e-6
+
+
+def test_gdn_keys_of_any_size(dev):
+    """The state is scaled by a bound that takes the keys' size into account."""
+    from orinfer_b200.ops import functional as F
+    for size in (2.0 ** -6, 0.5, 1.4):               # above sqrt(2) the recurrence itself diverges
+        args, state, exact = _runs(dev, [150], 4, -1.0, 3)
+        args[0][:, 2 * 128:4 * 128] *= size
+        out = F.gdn_scan(*args)
+        ref, s, sl = exact(0)
+        assert float((out.double() - ref).norm() / ref.norm()) < 2.0 ** -20
+        assert float((state[0].double() - s).norm() / s.norm()) < 2.0 ** -20
