@@ -71,7 +71,7 @@ __global__ void __launch_bounds__(D) gdn_conv_kernel(
     }
     acc = fmaf(v, __half2float(wc[j]), acc);
   }
-  float val = round_f16(acc * sigmoid_f32(acc));
+  float val = round_f16(acc * sigmoid_pair(make_float2(acc, acc)).x);
   if (head < qk_heads) {
     __shared__ float red[D / 32];
     float ss = warp_sum(val * val);
@@ -85,81 +85,124 @@ __global__ void __launch_bounds__(D) gdn_conv_kernel(
   y[static_cast<size_t>(row) * conv_dim + c] = __float2half_rn(val);
 }
 
-// The same convolution, eight channels per thread (16-byte loads and stores) over R consecutive
-// rows: the three earlier rows stay in registers, so a packet's rows are read once instead of
-// four times two bytes at a time.  A head is D / 8 neighbouring lanes.  Grid (row strips,
-// conv_dim / 2048); R = 1 for decode-sized packets, where the strips would be too few CTAs.
-// 2100 rows x 8192 channels: 89 -> 36 us (issue slots 61 %, DRAM 12 %: instructions, not bytes); 64
-// rows: 7.9 -> 5.0 us.
+// The same convolution, eight channels per thread (16-byte loads and stores) over a strip of
+// consecutive rows: the three earlier rows stay in registers as floats, so a packet's rows are read
+// and converted once, and the arithmetic goes two channels to an instruction (sigmoid_pair).  A
+// head is D / 8 neighbouring lanes.  Grid (strips, conv_dim / 2048), as many strips as fit the
+// machine at once: what a strip costs ahead of its first row is paid by one wave of CTAs.  R = 1:
+// strips of one row, for packets that have no more rows than that.
+// 2100 rows x 8192 channels: 89 us a row at a time, 36 in strips of eight rows and 45 instructions
+// a value, 27 now with 21 (68 MB; issue slots 50 %, the exponential and reciprocal unit 38 %,
+// sixteen warps per SM); 64 rows 7.6 -> 6.8 us.
 template <int D, int R>
-__global__ void __launch_bounds__(256) gdn_conv_vec_kernel(
+__global__ void __launch_bounds__(256, 2) gdn_conv_vec_kernel(
     const __half* x, int x_stride, const __half* weight, const __half* hist, const int* row_first,
-    const int* row_slot, const int* row_pos, int rows, int conv_dim, int qk_channels,
+    const int* row_slot, const int* row_pos, int rows, int conv_dim, int qk_channels, int strip,
     __half* __restrict__ y) {
   constexpr int LANES = D / 8;
   grid_wait();
   grid_release();
-  const int c = (blockIdx.y * 256 + threadIdx.x) * 8, row0 = blockIdx.x * R;
+  const int c = (blockIdx.y * 256 + threadIdx.x) * 8, row0 = blockIdx.x * strip;
+  const int end = min(rows, row0 + strip);
+  if (row0 >= rows) return;
   if (c >= conv_dim) return;                       // whole heads, so whole lane groups
   const unsigned group = LANES == 32 ? 0xffffffffu
                                      : ((1u << LANES) - 1u) << (threadIdx.x & 31 & ~(LANES - 1));
-  uint4 wr[4];
+  auto load = [&](int row) {
+    return *reinterpret_cast<const uint4*>(x + static_cast<size_t>(row) * x_stride + c);
+  };
+  auto floats = [](float2 (&to)[4], const uint4& raw) {
+    const __half2* h = reinterpret_cast<const __half2*>(&raw);
 #pragma unroll
-  for (int i = 0; i < 4; ++i)
-    wr[i] = reinterpret_cast<const uint4*>(weight + static_cast<size_t>(c) * 4)[i];
-  const __half* wh = reinterpret_cast<const __half*>(wr);
-  uint4 win[4];                                    // rows row-3 .. row (as loaded)
+    for (int i = 0; i < 4; ++i) to[i] = __half22float2(h[i]);
+  };
+  float2 w[4][4];                                  // [tap][pair of channels]
+#pragma unroll
+  for (int i = 0; i < 4; ++i) {
+    const uint4 raw = reinterpret_cast<const uint4*>(weight + static_cast<size_t>(c) * 4)[i];
+    const __half* h = reinterpret_cast<const __half*>(&raw);
+#pragma unroll
+    for (int j = 0; j < 4; ++j) w[j][i] = make_float2(__half2float(h[j]), __half2float(h[4 + j]));
+  }
+  // Row r is in win[r % 4] and comes R rows ahead of its use.  A strip that lies inside a run,
+  // three rows from its first, needs nothing else.
+  float2 win[4][4];
+  uint4 next[R];
+#pragma unroll
+  for (int u = 0; u < R; ++u)
+    if (row0 + u < end) next[u] = load(row0 + u);
 #pragma unroll
   for (int j = 0; j < 3; ++j) {
     const int src = row0 - 3 + j;
-    win[j + 1] = src >= 0 ? *reinterpret_cast<const uint4*>(
-                                x + static_cast<size_t>(src) * x_stride + c)
-                          : make_uint4(0, 0, 0, 0);
+    floats(win[j + 1], src >= 0 ? load(src) : make_uint4(0, 0, 0, 0));
   }
+  const int first0 = row_first[row0];
+  const bool inside = row0 - first0 >= 3 && row_first[end - 1] == first0;
+  int row = row0;
+  auto one_row = [&](int u) {                      // u = row % R
+    floats(win[u], next[u]);
+    if (row + R < end) next[u] = load(row + R);
+    const int first = inside ? first0 : row_first[row];
+    float2 acc[4];
 #pragma unroll
-  for (int r = 0; r < R; ++r) {
-    const int row = row0 + r;
-    if (row >= rows) break;
-#pragma unroll
-    for (int j = 0; j < 3; ++j) win[j] = win[j + 1];
-    win[3] = *reinterpret_cast<const uint4*>(x + static_cast<size_t>(row) * x_stride + c);
-    const int first = row_first[row];
-    uint4 tap[3] = {win[0], win[1], win[2]};
+    for (int i = 0; i < 4; ++i) acc[i] = make_float2(0.f, 0.f);
     if (row - first < 3) {                         // rows before the run come from its history
       const bool fresh = row_pos[first] == 0;
       const int slot = row_slot[row];
 #pragma unroll
       for (int j = 0; j < 3; ++j) {
         const int back = first - (row - 3 + j);    // 1..3 rows before the run
-        if (back > 0)
-          tap[j] = fresh ? make_uint4(0, 0, 0, 0)
-                         : *reinterpret_cast<const uint4*>(
-                               hist + (static_cast<size_t>(slot) * 3 + (3 - back)) * conv_dim + c);
+        float2 tap[4];
+        if (back > 0) {
+          const __half* kept = hist + (static_cast<size_t>(slot) * 3 + (3 - back)) * conv_dim + c;
+          floats(tap, fresh ? make_uint4(0, 0, 0, 0) : *reinterpret_cast<const uint4*>(kept));
+        } else {
+#pragma unroll
+          for (int i = 0; i < 4; ++i) tap[i] = win[(u + 1 + j) & 3][i];
+        }
+#pragma unroll
+        for (int i = 0; i < 4; ++i) acc[i] = fma2(tap[i], w[j][i], acc[i]);
       }
+    } else {
+#pragma unroll
+      for (int j = 0; j < 3; ++j)
+#pragma unroll
+        for (int i = 0; i < 4; ++i) acc[i] = fma2(win[(u + 1 + j) & 3][i], w[j][i], acc[i]);
     }
-    float val[8], ss = 0.f;
+    float ss = 0.f;
+    uint4 packed;
+    __half2* h = reinterpret_cast<__half2*>(&packed);
 #pragma unroll
-    for (int e = 0; e < 8; ++e) {
-      float acc = 0.f;
-#pragma unroll
-      for (int j = 0; j < 4; ++j)
-        acc = fmaf(__half2float(reinterpret_cast<const __half*>(j < 3 ? &tap[j] : &win[3])[e]),
-                   __half2float(wh[e * 4 + j]), acc);
-      val[e] = round_f16(acc * sigmoid_f32(acc));
-      ss = fmaf(val[e], val[e], ss);
+    for (int i = 0; i < 4; ++i) {
+      acc[i] = fma2(win[u][i], w[3][i], acc[i]);
+      acc[i] = mul2(acc[i], sigmoid_pair(acc[i]));
+      h[i] = __floats2half2_rn(acc[i].x, acc[i].y);
     }
     if (c < qk_channels) {
+#pragma unroll
+      for (int i = 0; i < 4; ++i) {
+        acc[i] = __half22float2(h[i]);
+        ss = fmaf(acc[i].x, acc[i].x, ss);
+        ss = fmaf(acc[i].y, acc[i].y, ss);
+      }
 #pragma unroll
       for (int o = 1; o < LANES; o <<= 1) ss += __shfl_xor_sync(group, ss, o);
       const float inv = rsqrtf(ss + 1e-6f);
 #pragma unroll
-      for (int e = 0; e < 8; ++e) val[e] *= inv;
+      for (int i = 0; i < 4; ++i) {
+        const float2 n = mul2(acc[i], make_float2(inv, inv));
+        h[i] = __floats2half2_rn(n.x, n.y);
+      }
     }
-    __align__(16) __half h[8];
+    *reinterpret_cast<uint4*>(y + static_cast<size_t>(row) * conv_dim + c) = packed;
+  };
+  while (row < end) {
 #pragma unroll
-    for (int e = 0; e < 8; ++e) h[e] = __float2half_rn(val[e]);
-    *reinterpret_cast<uint4*>(y + static_cast<size_t>(row) * conv_dim + c) =
-        *reinterpret_cast<const uint4*>(h);
+    for (int u = 0; u < R; ++u) {
+      if (row >= end) break;
+      one_row(u);
+      ++row;
+    }
   }
 }
 
@@ -989,13 +1032,14 @@ __global__ void __launch_bounds__(D) gdn_gated_norm_kernel(
   const float tot = warp_sum(red[d & 31]);
   const float n = v * rsqrtf(tot / D + eps) * __half2float(w[d]);
   const float zf = __half2float(z[static_cast<size_t>(row) * z_stride + h * D + d]);
-  const float sg = sigmoid_f32(zf);
+  const float sg = sigmoid_pair(make_float2(zf, zf)).x;       // the bits of the form below
   const float gate = sigmoid_gate ? sg : zf * sg;
   y[(static_cast<size_t>(row) * hv + h) * D + d] = __float2half_rn(n * gate);
 }
 
 // The same, one warp per (row, head): D / 32 neighbouring channels per lane, no block barrier.
-// 2600 rows x 32 heads of 128: 45 -> 19 us (85 MB).  A few heads are quicker with a thread per
+// 2600 rows x 32 heads of 128: 45 -> 19 us (85 MB); 2100 rows 17 -> 15 with two values to an
+// instruction (68 MB).  A few heads are quicker with a thread per
 // channel, which computes one sigmoid instead of four: 4 rows x 32 heads 1.2 us against 1.6, 48
 // rows 1.9 against 2.0, 64 rows 2.1 against 2.0.
 template <int D>
@@ -1025,11 +1069,14 @@ __global__ void __launch_bounds__(256) gdn_gated_norm_warp_kernel(
   const float r = rsqrtf(warp_sum(ss) / D + eps);
   Half out;
 #pragma unroll
-  for (int i = 0; i < V; ++i) {
-    const float n = v.f[i] * r * __half2float(wh.h[i]);
-    const float zf = __half2float(zh.h[i]);
-    const float sg = sigmoid_f32(zf);
-    out.h[i] = __float2half_rn(n * (sigmoid_gate ? sg : zf * sg));
+  for (int i = 0; i < V; i += 2) {
+    const float2 zf = make_float2(__half2float(zh.h[i]), __half2float(zh.h[i + 1]));
+    const float2 wf = make_float2(__half2float(wh.h[i]), __half2float(wh.h[i + 1]));
+    const float2 n = mul2(mul2(make_float2(v.f[i], v.f[i + 1]), make_float2(r, r)), wf);
+    const float2 sg = sigmoid_pair(zf);
+    const float2 res = mul2(n, sigmoid_gate ? sg : mul2(zf, sg));
+    out.h[i] = __float2half_rn(res.x);
+    out.h[i + 1] = __float2half_rn(res.y);
   }
   *reinterpret_cast<Half*>(y + item * D + lane * V) = out;
 }
@@ -1050,13 +1097,12 @@ static void launch_conv(const __half* x, int x_stride, const __half* weight, con
     return;
   }
   const int cols = (conv_dim + 2047) / 2048;
-  if (rows * cols >= 8 * 4 * 148)                // strips of eight rows still fill the machine
-    launch_early(gdn_conv_vec_kernel<D, 8>, dim3((rows + 7) / 8, cols), 256, 0, stream, x,
-                 x_stride, weight, hist, row_first, row_slot, row_pos, rows, conv_dim, 2 * hk * D,
-                 y);
-  else
-    launch_early(gdn_conv_vec_kernel<D, 1>, dim3(rows, cols), 256, 0, stream, x, x_stride, weight,
-                 hist, row_first, row_slot, row_pos, rows, conv_dim, 2 * hk * D, y);
+  const int most = 2 * 148 / cols > 1 ? 2 * 148 / cols : 1;      // strips at once
+  const int strip = (rows + most - 1) / most;
+  const dim3 grid((rows + strip - 1) / strip, cols);
+  auto kernel = strip > 1 ? gdn_conv_vec_kernel<D, 4> : gdn_conv_vec_kernel<D, 1>;
+  launch_early(kernel, grid, 256, 0, stream, x, x_stride, weight, hist, row_first, row_slot,
+               row_pos, rows, conv_dim, 2 * hk * D, strip, y);
 }
 
 static void launch_history(const __half* x, int x_stride, const Segment* segs, int n_segs,
@@ -1071,8 +1117,8 @@ static void launch_history(const __half* x, int x_stride, const Segment* segs, i
 }
 
 // Whether long runs take the kernel of gdn_pipe.cu: where its CTAs have an SM each, or the runs are
-// long enough to make up for their waves (figures there).  A caller that does not know the longest run
-// gives the rows in all.
+// long enough to make up for their waves (figures there).  A caller that does not know the longest
+// run gives the rows in all.
 static bool gdn_pipelined(int hv, int n_segs, int max_seg_rows) {
   return 2LL * hv * n_segs <= 148 || max_seg_rows >= 384LL * n_segs;
 }

@@ -308,3 +308,55 @@ def test_gdn_keys_of_any_size(dev):
         ref, s, sl = exact(0)
         assert float((out.double() - ref).norm() / ref.norm()) < 2.0 ** -20
         assert float((state[0].double() - s).norm() / s.norm()) < 2.0 ** -20
+
+
+# strips of one row, of a few, and as many as fit the machine, with runs that begin anywhere in one
+@pytest.mark.parametrize("rows", [1, 73, 75, 149, 297, 1187])
+@pytest.mark.parametrize("hk,hv", [(1, 2), (8, 24)])
+def test_gdn_conv_strips(dev, rows, hk, hv):
+    from orinfer_b200.ops import functional as F
+    g = torch.Generator().manual_seed(rows + hk)
+    d, conv = 128, (2 * hk + hv) * 128
+    x = (torch.randn(rows, conv + 64, generator=g) * 2).half().to(dev)
+    w = (torch.randn(conv, 4, generator=g) * 0.4).half().to(dev)
+    lens = [n for n in (rows // 3, 1, 2, rows - rows // 3 - 3) if n > 0] if rows > 6 else [rows]
+    hist = torch.randn(len(lens), 3, conv, generator=g).half().to(dev)
+    segs, first, slot, pos, at = [], [], [], [], 0
+    for i, n in enumerate(lens):
+        segs.append([at, n, 0, 0])
+        first += [at] * n
+        slot += [i] * n
+        pos += list(range(7 * (i % 2), 7 * (i % 2) + n))
+        at += n
+    t = lambda v: torch.tensor(v, dtype=torch.int32, device=dev)
+    args = (t(first), t(slot), t(pos), t(segs), len(lens), rows, hk, hv, d)
+    y = F.gdn_conv(x, w, hist.clone(), *args)
+    y_gen = F.gdn_conv(_unaligned(x), w, hist.clone(), *args)
+    for (at, n, _, _), h, i in zip(segs, hist, range(len(lens))):
+        full = torch.cat([h.double() * (i % 2), x[at:at + n, :conv].double()])
+        ref = sum(full[j:j + n] * w[:, j].double() for j in range(4))
+        ref = (ref * torch.sigmoid(ref)).half().double()
+        qk = ref[:, :2 * hk * d].reshape(n, -1, d)
+        ref[:, :2 * hk * d] = (qk * torch.rsqrt((qk * qk).sum(-1, keepdim=True) + 1e-6)).reshape(n, -1)
+        for got in (y, y_gen):                        # as in test_gdn_conv_forms_agree
+            assert bool(((got[at:at + n].double() - ref).abs() <= ref.abs() * 2.0 ** -9 + 1e-6).all())
+
+
+def test_gdn_gates_and_values_at_the_ends_of_their_range(dev):
+    """Infinities, NaNs and arguments whose exponential leaves FP32, in the two-value sigmoid."""
+    from orinfer_b200.ops import functional as F
+    z = torch.tensor([math.inf, -math.inf, math.nan, 0.0, 60000.0, -60000.0, -87.0, -89.0, 89.0,
+                      -20.0, 20.0, -104.0], device=dev).half()
+    rows, hv, d = 400, 4, 128
+    proj = z.repeat(rows, 43)[:, :hv * d].contiguous()
+    o = torch.ones(rows, hv, d, device=dev)
+    w = torch.full((d,), 4.0, device=dev).half()
+    for sig in (True, False):
+        y = F.gdn_gated_norm(o, proj, w, 0.0, rows, hv, d, sigmoid_gate=sig)
+        zz = proj.double()
+        ref = (torch.sigmoid(zz) * (1.0 if sig else zz) * 4).half()
+        got, want = y.double(), ref.double()
+        if not sig:                                   # minus infinity times a sigmoid of zero
+            want = torch.where(proj == -math.inf, math.nan, want)
+        same = (got == want) | (got.isnan() & want.isnan()) | ((got - want).abs() <= want.abs() * 2.0 ** -10)
+        assert bool(same.all()), (proj[~same][:4], got[~same][:4], want[~same][:4])
