@@ -1,4 +1,6 @@
 """Projections and row preparation at the edges of their tiles."""
+import math
+
 import pytest
 import torch
 
@@ -233,3 +235,34 @@ def test_kernels_that_start_early_keep_the_stream_order(dev, fmt, m):
     for _ in range(10):
         graph.replay()
         assert torch.equal(x, want)
+
+
+# rows of a warp each, which larger packets take, against the same rows in small packets
+@pytest.mark.parametrize("k", [128, 256, 384, 512, 640, 768, 896, 1024, 1152])
+@pytest.mark.parametrize("signed", [True, False])
+def test_swiglu_rows_of_large_packets_have_the_bits_of_small_ones(dev, k, signed):
+    from orinfer_b200.ops import functional as F
+    g = torch.Generator().manual_seed(k)
+    rows = 1024 + 5 * k // 128
+    x = torch.randn(rows, 2 * k, generator=g) * torch.exp2(torch.randint(-13, 5, (rows, 1), generator=g))
+    x[3] = 0                                           # an empty row
+    x[5, :k] = -300                                    # sigmoids below the normal numbers
+    x[7, 2], x[9, k + 1], x[11, 0] = math.nan, math.inf, -math.inf
+    x[13, :k], x[13, k:] = 2.0 ** -9, 2.0 ** -14       # scales among FP16's subnormal numbers
+    x = x.half().to(dev)
+    signs = (torch.randint(0, 2, (k,), generator=g) * 2 - 1).to(torch.int8).to(dev) if signed else None
+    y = torch.empty(rows, k, dtype=torch.float16, device=dev)
+    q, s = F.act_prep(x, None, None, signs, swiglu=True, y_out=y)
+    for at in range(0, rows, 512):
+        part = x[at:at + 512].contiguous()
+        y1 = torch.empty(part.shape[0], k, dtype=torch.float16, device=dev)
+        q1, s1 = F.act_prep(part, None, None, signs, swiglu=True, y_out=y1)
+        same = lambda a, b: torch.equal(torch.nan_to_num(a.float(), 1e9), torch.nan_to_num(b.float(), 1e9))
+        assert same(y[at:at + 512], y1) and same(s[at:at + 512], s1)
+        assert torch.equal(q[at:at + 512], q1)
+    # a count on the device limits the rows
+    q2, s2 = torch.full_like(q, 77), torch.full_like(s, 77)
+    F.act_prep_limited(x, signs, torch.tensor([1025], dtype=torch.int32, device=dev), swiglu=True,
+                       rows=rows, q_out=q2, scale_out=s2)
+    assert torch.equal(q2[:1025], q[:1025]) and bool((q2[1025:] == 77).all())
+    assert bool((s2[1025:] == 77).all())
