@@ -35,7 +35,8 @@
 // maximum only when it lags by 2^8 saves another tenth (fewer rescales of O) but rounds the largest
 // weights in FP16: the error against 64 bits grows by 1.8 % there and by 3.7 % for 500 rows behind
 // 1000.  Chunks of 777 and 646 rows behind 3000 positions, 16 / 2 gated heads of 256: 354 -> 276 ->
-// 244 with K and V freed apart, 223 now (180 CTAs: 1.2 waves).
+// 244 with K and V freed apart, 223 with plain loads, 161 with the gates asked for ahead (one at a
+// time, two bytes of a row per lane, a tile's epilogue took 30 us; 17 rows 41 -> 10 us).
 // Output is O / sum, optionally times sigmoid(gate), in FP16.  Replaces the prefill
 // configurations of causal_attention_int8 and dequantize_attention_kv
 // (kernels/cuda/model/attention_rows.py:61-276, kernels/cuda/model/kv_int8.py:210-247).
@@ -132,6 +133,39 @@ __device__ __forceinline__ uint4 dequant8(uint32_t w0, uint32_t w1, __half2 scal
   return out;
 }
 
+// The gates of 32 channels of an output row (a row of its own per lane, so each load waits for a line
+// of its own: they are asked for well ahead of their use).
+struct Gates {
+  uint4 w[4];
+  __device__ __forceinline__ void load(const __half* gate, size_t at) {
+    if ((reinterpret_cast<uintptr_t>(gate) & 15) == 0) {
+#pragma unroll
+      for (int i = 0; i < 4; ++i) w[i] = reinterpret_cast<const uint4*>(gate + at)[i];
+    } else {
+      __half* h = reinterpret_cast<__half*>(w);
+#pragma unroll
+      for (int i = 0; i < 32; ++i) h[i] = gate[at + i];
+    }
+  }
+};
+// Eight channels of an output row, times the sigmoids of their gates.
+__device__ __forceinline__ void store_gated(float (&v)[8], bool gated, const uint4& gates,
+                                            __half* out) {
+  __align__(16) __half h[8];
+  if (gated) {
+    const __half2* g = reinterpret_cast<const __half2*>(&gates);
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+      const float2 sg = sigmoid_pair(__half22float2(g[i]));
+      v[2 * i] *= sg.x;
+      v[2 * i + 1] *= sg.y;
+    }
+  }
+#pragma unroll
+  for (int i = 0; i < 8; ++i) h[i] = __float2half_rn(v[i]);
+  *reinterpret_cast<uint4*>(out) = *reinterpret_cast<const uint4*>(h);
+}
+
 struct Chunk {            // one prefill chunk of one request
   int row_start;          // first packed row
   int q_len;              // rows in the chunk
@@ -139,7 +173,7 @@ struct Chunk {            // one prefill chunk of one request
   int slot;               // row of the page table
 };
 
-template <int D, int NQ>
+template <int D, int NQ, bool GATED>
 __global__ void __launch_bounds__(Smem<D, NQ>::THREADS, 1) attn_prefill_kernel(
     const __grid_constant__ CUtensorMap tmap_q, const Chunk* chunks, const int* page_table,
     int max_pages, const int8_t* kc, const int8_t* vc, const __half* ks, const __half* vs,
@@ -524,6 +558,10 @@ __global__ void __launch_bounds__(Smem<D, NQ>::THREADS, 1) attn_prefill_kernel(
         l_run = l_run * corr + l_tile;
       }
     }
+    const bool gated = GATED && valid;
+    const size_t orow = static_cast<size_t>(ch.row_start + first + p_rel) * qh + head;
+    Gates ahead;
+    if (gated) ahead.load(gate, orow * D + half * DH);
     if (ok && steps > 0) {
       ok = mbar_wait(&o_done[q], (steps - 1) & 1, status, STATUS_EPILOGUE_WAIT, 0x300);
       ok = __all_sync(0xffffffffu, ok);
@@ -534,27 +572,22 @@ __global__ void __launch_bounds__(Smem<D, NQ>::THREADS, 1) attn_prefill_kernel(
       tc_fence_after();
       const float l_all = *first_sum;
       const float inv = l_all > 0.f ? 1.f / l_all : 0.f;
-      const size_t orow = static_cast<size_t>(ch.row_start + first + p_rel) * qh + head;
 #pragma unroll 1
       for (int c0 = 0; c0 < DH; c0 += 32) {
         uint32_t r[32];
         tmem_ld_32x32(tmem_oq + c0, r);
+        const size_t at = orow * D + half * DH + c0;
+        const Gates now = ahead;
+        if (gated && c0 + 32 < DH) ahead.load(gate, at + 32);
         tc_wait_ld();
         if (valid) {
-          const size_t at = orow * D + half * DH + c0;
-          __align__(16) __half hv[32];
 #pragma unroll
-          for (int i = 0; i < 32; ++i) {
-            float v = __uint_as_float(r[i]) * inv;
-            if (gate) {
-              const float gv = __half2float(gate[at + i]);
-              v *= __fdiv_rn(1.f, 1.f + expf(-gv));
-            }
-            hv[i] = __float2half_rn(v);
+          for (int i = 0; i < 32; i += 8) {
+            float v[8];
+#pragma unroll
+            for (int k = 0; k < 8; ++k) v[k] = __uint_as_float(r[i + k]) * inv;
+            store_gated(v, gated, now.w[i / 8], out + at + i);
           }
-          uint4* o = reinterpret_cast<uint4*>(out + at);
-#pragma unroll
-          for (int i = 0; i < 4; ++i) o[i] = reinterpret_cast<const uint4*>(hv)[i];
         }
       }
     }
@@ -584,10 +617,11 @@ int launch(const __half* q, const __half* gate, const Chunk* chunks, int n_chunk
           estr, CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B,
           CU_TENSOR_MAP_L2_PROMOTION_L2_128B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) != CUDA_SUCCESS)
     return -3;
-  static const int slot = runtime_new_slot();
-  if (const int e = runtime_allow_smem(slot, attn_prefill_kernel<D, NQ>, L::TOTAL)) return e;
+  static const int slot[2] = {runtime_new_slot(), runtime_new_slot()};
+  auto kernel = gate ? attn_prefill_kernel<D, NQ, true> : attn_prefill_kernel<D, NQ, false>;
+  if (const int e = runtime_allow_smem(slot[gate != nullptr], kernel, L::TOTAL)) return e;
   dim3 grid((max_q_len + NQ * P - 1) / (NQ * P), kvh, n_chunks);
-  launch_early(attn_prefill_kernel<D, NQ>, grid, L::THREADS, L::TOTAL, stream, tq, chunks,
+  launch_early(kernel, grid, L::THREADS, L::TOTAL, stream, tq, chunks,
                page_table, max_pages, kc, vc, ks, vs, gate, out, qh, kvh, rep, num_pages,
                runtime_status_ptr());
   return static_cast<int>(cudaGetLastError());

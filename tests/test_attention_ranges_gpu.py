@@ -364,3 +364,29 @@ def test_attention_rows_of_short_contexts_in_digits(dev, qh, kvh, d, waves):
         lim = ref.abs() * 2.0 ** -11 + 2.0 ** -18 * ref.abs().max() + 2.0 ** -25
         got = out[i::len(lens)].double()
         assert bool(((got - ref).abs() <= lim).all()), n
+
+
+# gates at any address, and as large as they come
+@pytest.mark.parametrize("qh,kvh,d,rows", [(8, 1, 256, 37), (4, 2, 128, 70), (16, 2, 256, 300),
+                                           (2, 2, 64, 33)])
+@pytest.mark.parametrize("aligned", [True, False])
+def test_attention_prefill_gates(dev, qh, kvh, d, rows, aligned):
+    from orinfer_b200.ops import functional as F
+    _, req, pos, table, kc, vc, ks, vs = _walk(dev, rows + 90, qh, kvh, d, rows)
+    g = torch.Generator().manual_seed(d)
+    q = torch.randn(rows, qh, d, generator=g).half().to(dev)
+    size = torch.exp2(torch.rand(rows, qh, d, generator=g) * 14)
+    gate = torch.randn(rows, qh, d, generator=g) * size
+    gate[0, 0, :4] = torch.tensor([math.inf, -math.inf, 90.0, -90.0])
+    gate = gate.half().to(dev)
+    if not aligned:
+        gate = _unaligned(gate)
+    out = torch.empty(rows, qh * d, dtype=torch.float16, device=dev)
+    chunks = torch.tensor([[0, rows, 90, 0]], dtype=torch.int32, device=dev)
+    assert F.attention_prefill(q, gate, chunks, rows, table, kc, vc, ks, vs, out=out)
+    plain = torch.empty_like(out)
+    assert F.attention_prefill(q, None, chunks, rows, table, kc, vc, ks, vs, out=plain)
+    want = plain.double() * torch.sigmoid(gate.double()).view(rows, -1)
+    # the ungated output has one FP16 rounding (2^-11), the gated one another
+    lim = want.abs() * 2.0 ** -10 + 2.0 ** -24
+    assert bool(((out.double() - want).abs() <= lim).all())
