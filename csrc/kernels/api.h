@@ -183,6 +183,8 @@ int orinfer_attention(const __half* q, const __half* gate, const int* row_req, c
 
 // Prefill chunks on tensor cores.  chunks: device int32 [n_chunks, 4] =
 // (first packed row, rows, absolute position of the first row, page-table row).
+// Parts that the keys of a tile are cut into (heads of 256 channels).
+int orinfer_attention_prefill_parts(int ctas, int max_pages);
 // Returns -4 for a head size it does not implement (use orinfer_attention instead).
 int orinfer_attention_prefill(const __half* q, const __half* gate, const int* chunks, int n_chunks,
                               int max_q_len, int total_rows, const int* page_table, int max_pages,

@@ -1,10 +1,9 @@
-// Causal GQA flash attention for prefill chunks over the paged INT8 KV cache, on
-// tcgen05 tensor cores with TMEM accumulators.
-//
-// A query tile is 128 rows: P = 128 / rep consecutive query positions of one request times the
-// `rep` query heads that share one KV head (the heads are packed into the MMA M axis so each
-// INT8 K/V page is dequantised once for all of them).  One CTA owns NQ tiles: in large packets of
-// head sizes 64 and 128 two neighbouring ones, so that a dequantised page serves 256 rows and the
+// Causal GQA flash attention for prefill chunks over the paged INT8 KV cache, on tcgen05 tensor
+// cores with TMEM accumulators.
+//  A query tile is 128 rows: P = 128 / rep consecutive query positions of one request times the
+// `rep` query heads that share one KV head (the heads are packed into the MMA M axis so each INT8
+// K/V page is dequantised once for all of them).  One CTA owns NQ tiles: in large packets of head
+// sizes 64 and 128 two neighbouring ones, so that a dequantised page serves 256 rows and the
 // tensor core works on one tile while the softmax warps of the other are busy.  Per step of KT
 // keys:
 //   * eight warps read the INT8 page and its group-64 FP16 scales straight from global memory (a
@@ -16,30 +15,30 @@
 //     where the second MMA reads it as its A operand.  The two meet once per step, for the row's
 //     maximum, and hand over the sum of the weights, which are added in the order of the keys
 //     (sums of their own per half would save 5 % of 4096 rows and 4 to 9 % of short chunks, and
-//     move FP16 outputs by a step, which the INT8 rows of the next projection make a code step).
-//     P is relative to the row's running maximum, so its largest weight is exactly 1 and
-//     O is rescaled whenever a row of the warp finds a larger score;
+//     move FP16 outputs by a step, which the INT8 rows of the next projection make a code step). P
+//     is relative to the row's running maximum, so its largest weight is exactly 1 and O is
+//     rescaled whenever a row of the warp finds a larger score;
 //   * warp 0 loads the Q tiles once with a 3-D TMA (d, head, position).
 // With one tile S is double buffered instead.  Head size 256 has room for no more (Q 64 KB, two K
 // and two V buffers of 32 KB; TMEM: two S of 64 columns and O of 256) and walks the cache in half
-// pages.
-// CTAs are ordered from the last query positions (the longest walks) to the first.
-//
-// A step of two tiles is a chain per tile (softmax, P V, Q K^T of the next step) and two of them
+// pages. CTAs are ordered from the last query positions (the longest walks) to the first.
+//  A step of two tiles is a chain per tile (softmax, P V, Q K^T of the next step) and two of them
 // hide each other only in part: 5500 cycles for 128 keys with one softmax thread per row and the
 // MMAs issued inside a branch on the lane, about 4700 with two threads and a whole warp in the
-// issuing loop.  The tensor core needs 2050 of them, the exponentials as many.
-// One 4096-token chunk, 32 / 8 heads of 128: 377 us with one tile per CTA and P in shared memory,
-// 243 with two tiles and P in TMEM, 203 with two threads per row and a whole issuing warp (677
-// TFLOP/s causal); 512 tokens 19 -> 14 us, 64 behind 1000 29 -> 22.  A reference that follows the
-// maximum only when it lags by 2^8 saves another tenth (fewer rescales of O) but rounds the largest
-// weights in FP16: the error against 64 bits grows by 1.8 % there and by 3.7 % for 500 rows behind
-// 1000.  Chunks of 777 and 646 rows behind 3000 positions, 16 / 2 gated heads of 256: 354 -> 276 ->
-// 244 with K and V freed apart, 223 with plain loads, 161 with the gates asked for ahead (one at a
-// time, two bytes of a row per lane, a tile's epilogue took 30 us; 17 rows 41 -> 10 us).
-// Output is O / sum, optionally times sigmoid(gate), in FP16.  Replaces the prefill
-// configurations of causal_attention_int8 and dequantize_attention_kv
-// (kernels/cuda/model/attention_rows.py:61-276, kernels/cuda/model/kv_int8.py:210-247).
+// issuing loop.  The tensor core needs 2050 of them, the exponentials as many. One 4096-token
+// chunk, 32 / 8 heads of 128: 377 us with one tile per CTA and P in shared memory, 243 with two
+// tiles and P in TMEM, 203 with two threads per row and a whole issuing warp (677 TFLOP/s causal);
+// 512 tokens 19 -> 14 us, 64 behind 1000 29 -> 22.  A reference that follows the maximum only when
+// it lags by 2^8 saves another tenth (fewer rescales of O) but rounds the largest weights in FP16:
+// the error against 64 bits grows by 1.8 % there and by 3.7 % for 500 rows behind 1000.  Chunks of
+// 777 and 646 rows behind 3000 positions, 16 / 2 gated heads of 256: 354 -> 276 -> 244 with K and
+// V freed apart, 223 with plain loads, 161 with the gates asked for ahead (one at a time, two
+// bytes of a row per lane, a tile's epilogue took 30 us; 17 rows 41 -> 10 us).  Where the tiles
+// are fewer than half the SMs, a cluster cuts the keys of each (SPLIT): 64 rows behind 1000 32 ->
+// @S1@, 500 behind 1000 44 -> @S2@, 64 behind 20000 @S3@. Output is O / sum, optionally times
+// sigmoid(gate), in FP16.  Replaces the prefill configurations of causal_attention_int8 and
+// dequantize_attention_kv (kernels/cuda/model/attention_rows.py:61-276,
+// kernels/cuda/model/kv_int8.py:210-247).
 #include <cuda.h>
 
 #include "api.h"
@@ -133,8 +132,8 @@ __device__ __forceinline__ uint4 dequant8(uint32_t w0, uint32_t w1, __half2 scal
   return out;
 }
 
-// The gates of 32 channels of an output row (a row of its own per lane, so each load waits for a line
-// of its own: they are asked for well ahead of their use).
+// The gates of 32 channels of an output row (a row of its own per lane, so each load waits for a
+// line of its own: they are asked for well ahead of their use).
 struct Gates {
   uint4 w[4];
   __device__ __forceinline__ void load(const __half* gate, size_t at) {
@@ -173,12 +172,30 @@ struct Chunk {            // one prefill chunk of one request
   int slot;               // row of the page table
 };
 
-template <int D, int NQ, bool GATED>
+// SPLIT (one tile per CTA): the CTAs of a cluster take the tile's keys in equal parts, and each
+// then puts one slice of the channels together from everybody's shared memory.
+__device__ __forceinline__ float4 cluster_float4(uint32_t addr) {
+  float4 v;
+  asm volatile("ld.shared::cluster.v4.f32 {%0, %1, %2, %3}, [%4];"
+               : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w)
+               : "r"(addr)
+               : "memory");
+  return v;
+}
+__device__ __forceinline__ float cluster_float(uint32_t addr) {
+  float v;
+  asm volatile("ld.shared::cluster.f32 %0, [%1];" : "=f"(v) : "r"(addr) : "memory");
+  return v;
+}
+constexpr int SPLIT_STEPS = 3;               // a part has at least as many steps
+
+template <int D, int NQ, bool GATED, bool SPLIT>
 __global__ void __launch_bounds__(Smem<D, NQ>::THREADS, 1) attn_prefill_kernel(
     const __grid_constant__ CUtensorMap tmap_q, const Chunk* chunks, const int* page_table,
     int max_pages, const int8_t* kc, const int8_t* vc, const __half* ks, const __half* vs,
     const __half* gate, __half* __restrict__ out, int qh, int kvh, int rep, int num_pages,
-    int* status) {
+    int ranks, int* status) {
+  static_assert(!SPLIT || NQ == 1, "a split tile has its CTA to itself");
   using L = Smem<D, NQ>;
   constexpr int NSUB = L::NSUB, KT = L::KT;
   constexpr int GROUPS = D / 64;
@@ -204,7 +221,10 @@ __global__ void __launch_bounds__(Smem<D, NQ>::THREADS, 1) attn_prefill_kernel(
   const int h = blockIdx.y;                       // kv head
   const int P = TILE / rep;                       // query positions per tile
   // first chunk-relative position of this CTA's tiles; long walks start first
-  const int p_first = static_cast<int>(gridDim.x - 1 - blockIdx.x) * NQ * P;
+  const int rank = SPLIT ? static_cast<int>(cluster_ctarank()) : 0;
+  const int tile = SPLIT ? blockIdx.x / ranks : blockIdx.x;
+  const int tiles = SPLIT ? gridDim.x / ranks : gridDim.x;
+  const int p_first = (tiles - 1 - tile) * NQ * P;
   if (p_first >= ch.q_len) return;
   // steps that any row of tile q can see (0: the chunk ends before the tile)
   auto steps_of = [&](int q) {
@@ -217,6 +237,13 @@ __global__ void __launch_bounds__(Smem<D, NQ>::THREADS, 1) attn_prefill_kernel(
   for (int q = 0; q < NQ; ++q) {
     n_steps[q] = steps_of(q);
     n_max = max(n_max, n_steps[q]);
+  }
+  int j0 = 0;                                     // this CTA's first step; others count from it
+  if (SPLIT) {
+    const int parts = max(1, min(ranks, n_max / SPLIT_STEPS));
+    j0 = rank < parts ? n_max * rank / parts : 0;
+    n_max = rank < parts ? n_max * (rank + 1) / parts - j0 : 0;
+    n_steps[0] = n_max;
   }
 
   if (threadIdx.x == 0) {
@@ -302,8 +329,10 @@ __global__ void __launch_bounds__(Smem<D, NQ>::THREADS, 1) attn_prefill_kernel(
       if (ok && j < steps[q]) issue_qk(q, j);
       if (ok && q == NQ - 1) tc_commit_by(leader, &k_free[j & 1]);
     };
+    if (!SPLIT || last > 0) {
 #pragma unroll
-    for (int q = 0; q < NQ; ++q) next_qk(q, 0);
+      for (int q = 0; q < NQ; ++q) next_qk(q, 0);
+    }
     for (int j = 0; j < last && ok; ++j) {
       const bool more = j + 1 < last;
       if (NQ == 1 && more) next_qk(0, j + 1);
@@ -332,14 +361,15 @@ __global__ void __launch_bounds__(Smem<D, NQ>::THREADS, 1) attn_prefill_kernel(
     const int rows = (DQ / CPK) * kvh;               // the rows of a thread are that far apart
     auto load = [&](int j, int page, bool k, bool v) {
       // one base address per step
-      const size_t slot = (static_cast<size_t>(page) * 128 + j * KT % TILE + u / CPK) * kvh + h;
+      const size_t slot =
+          (static_cast<size_t>(page) * 128 + (j0 + j) * KT % TILE + u / CPK) * kvh + h;
       const int8_t* kp = kc + slot * D + (u % CPK) * 16;
       const int8_t* vp = vc + slot * D + (u % CPK) * 16;
       const __half* ksp = ks + slot * GROUPS + (u % CPK) / 4;
       const __half* vsp = vs + slot * GROUPS + (u % CPK) / 4;
       // Keys past the last position that a row of this CTA sees may be slots never written.  Their
       // weight is zero, but zero times an infinite or NaN value is not: they get no value scale.
-      const int live = kv_end - j * KT - u / CPK;
+      const int live = kv_end - (j0 + j) * KT - u / CPK;
 #pragma unroll
       for (int it = 0; it < ITERS; ++it) {
         const size_t at = static_cast<size_t>(it) * rows;
@@ -372,14 +402,17 @@ __global__ void __launch_bounds__(Smem<D, NQ>::THREADS, 1) attn_prefill_kernel(
       if (lane == 0 && v) mbar_arrive(&v_ready[buf]);
     };
     auto page_of = [&](int j) {
-      const int page = pages[j * KT / TILE];
+      const int page = pages[(j0 + j) * KT / TILE];
       if (page >= 0 && page < num_pages) return page;
       report_status(status, STATUS_BAD_INDEX, 3);
       return 0;
     };
     bool ok = true;
-    int page = page_of(0);
-    load(0, page, true, true);
+    int page = 0;
+    if (!SPLIT || n_max > 0) {
+      page = page_of(0);
+      load(0, page, true, true);
+    }
     if (n_max > 1) page = page_of(1);
     // a buffer was last read by the MMAs of step j - 2
     auto released = [&](uint64_t* free, int j) {
@@ -441,7 +474,7 @@ __global__ void __launch_bounds__(Smem<D, NQ>::THREADS, 1) attn_prefill_kernel(
         continue;
       }
       tc_fence_after();
-      const int key0 = j * KT + half * KH;
+      const int key0 = (j0 + j) * KT + half * KH;
       // Only the last page of a row can hold keys beyond its position; every earlier page
       // takes the mask-free path.
       const bool full_warp = __all_sync(0xffffffffu, key0 + KH - 1 <= q_pos);
@@ -558,7 +591,7 @@ __global__ void __launch_bounds__(Smem<D, NQ>::THREADS, 1) attn_prefill_kernel(
         l_run = l_run * corr + l_tile;
       }
     }
-    const bool gated = GATED && valid;
+    const bool gated = GATED && !SPLIT && valid;
     const size_t orow = static_cast<size_t>(ch.row_start + first + p_rel) * qh + head;
     Gates ahead;
     if (gated) ahead.load(gate, orow * D + half * DH);
@@ -568,7 +601,29 @@ __global__ void __launch_bounds__(Smem<D, NQ>::THREADS, 1) attn_prefill_kernel(
     }
     if (half == 1) *first_sum = l_run;
     meet();
-    if (ok && steps > 0) {
+    if (SPLIT) {
+      // this part's O, four channels of all rows at a time, where K and V were; its maximum and sum
+      tc_fence_after();
+      float* stat = reinterpret_cast<float*>(smem + L::MAX_OFF);
+      if (half == 0) {
+        stat[row] = ok && steps > 0 ? m_run : -INFINITY;
+        stat[TILE + row] = *first_sum;
+      }
+      float4* part = reinterpret_cast<float4*>(smem + L::K_OFF);
+      if (ok && steps > 0) {
+#pragma unroll 1
+        for (int c0 = 0; c0 < DH; c0 += 32) {
+          uint32_t r[32];
+          tmem_ld_32x32(tmem_oq + c0, r);
+          tc_wait_ld();
+#pragma unroll
+          for (int i = 0; i < 32; i += 4)
+            part[(half * DH + c0 + i) / 4 * TILE + row] =
+                make_float4(__uint_as_float(r[i]), __uint_as_float(r[i + 1]),
+                            __uint_as_float(r[i + 2]), __uint_as_float(r[i + 3]));
+        }
+      }
+    } else if (ok && steps > 0) {
       tc_fence_after();
       const float l_all = *first_sum;
       const float inv = l_all > 0.f ? 1.f / l_all : 0.f;
@@ -595,13 +650,71 @@ __global__ void __launch_bounds__(Smem<D, NQ>::THREADS, 1) attn_prefill_kernel(
   tc_fence_before();
   __syncthreads();
   if (warp == 1) tmem_dealloc(tmem_base, TMEM_COLS);
+  if (SPLIT) {
+    static_assert(!SPLIT || 4 * NSUB * L::KSUB >= D * TILE * 4, "O takes the place of K and V");
+    cluster_sync_all();
+    if (warp >= 2 && warp < 10) {
+      const int half = ((warp - 2) >> 2) & 1, row = (warp & 3) * 32 + lane;
+      const int p_rel = row / rep, head = h * rep + row % rep;
+      const int slice = D / ranks / 2, c_lo = rank * 2 * slice + half * slice;   // channels
+      if (row < P * rep && p_first + p_rel < ch.q_len) {
+        const uint32_t stat = smem_u32(smem + L::MAX_OFF) + row * 4;
+        const uint32_t part = smem_u32(smem + L::K_OFF) + (c_lo / 4 * TILE + row) * 16;
+        float m = -INFINITY, l = 0.f;
+        for (int s = 0; s < ranks; ++s) m = fmaxf(m, cluster_float(mapa_u32(stat, s)));
+        float f[8];
+#pragma unroll
+        for (int s = 0; s < 8; ++s) {
+          if (s >= ranks) break;
+          const float ms = cluster_float(mapa_u32(stat, s));
+          f[s] = ms == -INFINITY ? 0.f : ex2(ms - m);
+          if (f[s] != 0.f) l = fmaf(cluster_float(mapa_u32(stat + TILE * 4, s)), f[s], l);
+        }
+        const float inv = l > 0.f ? 1.f / l : 0.f;
+        const size_t at =
+            (static_cast<size_t>(ch.row_start + p_first + p_rel) * qh + head) * D + c_lo;
+#pragma unroll 1
+        for (int c = 0; c < slice; c += 8) {
+          float v[8];
+          uint4 gates = make_uint4(0, 0, 0, 0);
+          if (GATED) {
+            if ((reinterpret_cast<uintptr_t>(gate) & 15) == 0) {
+              gates = *reinterpret_cast<const uint4*>(gate + at + c);
+            } else {
+#pragma unroll
+              for (int i = 0; i < 8; ++i) reinterpret_cast<__half*>(&gates)[i] = gate[at + c + i];
+            }
+          }
+#pragma unroll
+          for (int i = 0; i < 8; ++i) v[i] = 0.f;
+#pragma unroll
+          for (int s = 0; s < 8; ++s) {
+            if (s >= ranks) break;
+            if (f[s] == 0.f) continue;               // (nothing was put there)
+#pragma unroll
+            for (int k = 0; k < 2; ++k) {
+              const float4 o = cluster_float4(mapa_u32(part + (c / 4 + k) * TILE * 16, s));
+              v[4 * k] = fmaf(o.x, f[s], v[4 * k]);
+              v[4 * k + 1] = fmaf(o.y, f[s], v[4 * k + 1]);
+              v[4 * k + 2] = fmaf(o.z, f[s], v[4 * k + 2]);
+              v[4 * k + 3] = fmaf(o.w, f[s], v[4 * k + 3]);
+            }
+          }
+#pragma unroll
+          for (int i = 0; i < 8; ++i) v[i] *= inv;
+          store_gated(v, GATED, gates, out + at + c);
+        }
+      }
+    }
+    cluster_sync_all();                              // nobody leaves while its memory is read
+  }
 }
 
-template <int D, int NQ>
+template <int D, int NQ, bool SPLIT = false>
 int launch(const __half* q, const __half* gate, const Chunk* chunks, int n_chunks, int max_q_len,
            int total_rows, const int* page_table, int max_pages, const int8_t* kc,
            const int8_t* vc, const __half* ks, const __half* vs, __half* out, int qh, int kvh,
-           int num_pages, cudaStream_t stream) {
+           int num_pages, cudaStream_t stream, int ranks = 1) {
   using L = Smem<D, NQ>;
   const int rep = qh / kvh;
   const int P = TILE / rep;
@@ -618,12 +731,30 @@ int launch(const __half* q, const __half* gate, const Chunk* chunks, int n_chunk
           CU_TENSOR_MAP_L2_PROMOTION_L2_128B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) != CUDA_SUCCESS)
     return -3;
   static const int slot[2] = {runtime_new_slot(), runtime_new_slot()};
-  auto kernel = gate ? attn_prefill_kernel<D, NQ, true> : attn_prefill_kernel<D, NQ, false>;
+  auto kernel = gate ? attn_prefill_kernel<D, NQ, true, SPLIT>
+                     : attn_prefill_kernel<D, NQ, false, SPLIT>;
   if (const int e = runtime_allow_smem(slot[gate != nullptr], kernel, L::TOTAL)) return e;
-  dim3 grid((max_q_len + NQ * P - 1) / (NQ * P), kvh, n_chunks);
-  launch_early(kernel, grid, L::THREADS, L::TOTAL, stream, tq, chunks,
-               page_table, max_pages, kc, vc, ks, vs, gate, out, qh, kvh, rep, num_pages,
-               runtime_status_ptr());
+  dim3 grid((max_q_len + NQ * P - 1) / (NQ * P) * ranks, kvh, n_chunks);
+  if (SPLIT) {
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = grid;
+    cfg.blockDim = L::THREADS;
+    cfg.dynamicSmemBytes = L::TOTAL;
+    cfg.stream = stream;
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeClusterDimension;
+    attr[0].val.clusterDim.x = ranks;
+    attr[0].val.clusterDim.y = 1;
+    attr[0].val.clusterDim.z = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = 1;
+    const cudaError_t e = cudaLaunchKernelEx(&cfg, kernel, tq, chunks, page_table, max_pages, kc,
+                                             vc, ks, vs, gate, out, qh, kvh, rep, num_pages, ranks,
+                                             runtime_status_ptr());
+    return static_cast<int>(e != cudaSuccess ? e : cudaGetLastError());
+  }
+  launch_early(kernel, grid, L::THREADS, L::TOTAL, stream, tq, chunks, page_table, max_pages, kc,
+               vc, ks, vs, gate, out, qh, kvh, rep, num_pages, ranks, runtime_status_ptr());
   return static_cast<int>(cudaGetLastError());
 }
 
@@ -631,6 +762,29 @@ int launch(const __half* q, const __half* gate, const Chunk* chunks, int n_chunk
 }  // namespace orinfer
 
 using namespace orinfer;
+
+// Into how many parts the keys of a tile go, the steps counted from the page table's width (heads of
+// 256 channels, one tile per CTA).  A step takes 1.35 us, a CTA about six of them besides, and a
+// part five more to be put together with the others; a larger number has to save 15 %.  (More parts
+// than SMs did not pay: 180 CTAs of 60 steps 161 us whole, 152 in two parts, 195 in four, but 188 of
+// 12 steps 45 and 72.)
+static int prefill_ranks(long long ctas, long long steps) {
+  int best = 1;
+  double least = 0;
+  for (int s = 1; s <= 8; s *= 2) {
+    if (s > 1 && ctas * s > 148) break;
+    const double waves = static_cast<double>((ctas * s + 147) / 148);
+    const double cost = waves * (static_cast<double>(steps) / s + (s > 1 ? 11.0 : 6.0));
+    if (s == 1 || cost < least * 0.85) {
+      least = cost;
+      best = s;
+    }
+  }
+  return best;
+}
+extern "C" int orinfer_attention_prefill_parts(int ctas, int max_pages) {
+  return prefill_ranks(ctas, static_cast<long long>(max_pages) * 2);
+}
 
 // chunks: int32 [n_chunks, 4] = (row_start, q_len, pos0, page-table row) on the device.
 extern "C" int orinfer_attention_prefill(const __half* q, const __half* gate, const int* chunks,
@@ -660,7 +814,14 @@ extern "C" int orinfer_attention_prefill(const __half* q, const __half* gate, co
   if (head_dim == 128) ORINFER_PREFILL(128, 2);
   if (head_dim == 64 && one) ORINFER_PREFILL(64, 1);
   if (head_dim == 64) ORINFER_PREFILL(64, 2);
-  if (head_dim == 256) ORINFER_PREFILL(256, 1);
 #undef ORINFER_PREFILL
+  if (head_dim == 256) {
+    const long long ctas = (longest < packed ? longest : packed) * kvh;
+    const int ranks = prefill_ranks(ctas, static_cast<long long>(max_pages) * 2);
+    return (ranks > 1 ? fa::launch<256, 1, true> : fa::launch<256, 1, false>)(
+        q, gate, ch, n_chunks, max_q_len, total_rows, page_table, max_pages, kc, vc, ks, vs, out,
+        qh, kvh, num_pages, stream, ranks);
+  }
+
   return -4;          // unsupported head size: caller falls back to the row kernel
 }

@@ -390,3 +390,53 @@ def test_attention_prefill_gates(dev, qh, kvh, d, rows, aligned):
     # the ungated output has one FP16 rounding (2^-11), the gated one another
     lim = want.abs() * 2.0 ** -10 + 2.0 ** -24
     assert bool(((out.double() - want).abs() <= lim).all())
+
+
+# tiles whose keys are cut over a cluster: as few as the rows have, ragged chunks (clusters without a
+# tile), parts without a step, slots never written
+@pytest.mark.parametrize("rows,past,qh,kvh,parts", [(16, 4000, 8, 1, 8), (33, 900, 16, 2, 4),
+                                                    (64, 1000, 16, 2, 4), (150, 2000, 16, 2, 4),
+                                                    (230, 1700, 8, 1, 4), (400, 1500, 16, 2, 2),
+                                                    (5, 3000, 2, 2, 8)])
+@pytest.mark.parametrize("gated", [True, False])
+def test_attention_prefill_cut_over_a_cluster(dev, rows, past, qh, kvh, parts, gated):
+    from orinfer_b200.ops import functional as F
+    from orinfer_b200.ops import native
+    d, g = 256, torch.Generator().manual_seed(rows)
+    sizes, pasts = [rows, max(1, rows // 3)], [past, 5]
+    pages = [(n + p + 127) // 128 for n, p in zip(sizes, pasts)]
+    table = torch.zeros(2, max(pages), dtype=torch.int32)
+    order = torch.randperm(sum(pages), generator=g) + 1
+    table[0, :pages[0]], table[1, :pages[1]] = order[:pages[0]], order[pages[0]:]
+    shape = (sum(pages) + 1, 128, kvh)
+    kc = torch.randint(-127, 128, (*shape, d), generator=g, dtype=torch.int8)
+    vc = torch.randint(-127, 128, (*shape, d), generator=g, dtype=torch.int8)
+    ks = (torch.rand(*shape, 4, generator=g) * 0.02 + 1e-3).half()
+    vs = (torch.rand(*shape, 4, generator=g) * 0.02 + 1e-3).half()
+    for i in range(2):
+        n = sizes[i] + pasts[i]
+        ks[table[i, pages[i] - 1], (n - 1) % 128 + 1:] = math.nan
+        vs[table[i, pages[i] - 1], (n - 1) % 128 + 1:] = math.inf
+    total = sum(sizes)
+    q = torch.randn(total, qh, d, generator=g).half()
+    gate = torch.randn(total, qh, d, generator=g).half() if gated else None
+    tile_rows = 128 // (qh // kvh)
+    tiles = min((rows + tile_rows - 1) // tile_rows * 2, total // tile_rows + 2)
+    assert native.lib().orinfer_attention_prefill_parts(tiles * kvh, table.shape[1]) == parts
+    out = torch.empty(total, qh * d, dtype=torch.float16, device=dev)
+    chunks = torch.tensor([[0, sizes[0], past, 0], [sizes[0], sizes[1], 5, 1]], dtype=torch.int32)
+    on = lambda t: None if t is None else t.to(dev)
+    assert F.attention_prefill(on(q), on(gate), on(chunks), rows, on(table), on(kc), on(vc), on(ks),
+                               on(vs), out=out)
+    assert native.read_status() == 0
+    at = 0
+    for i in range(2):
+        pick = lambda c: c[table[i, :pages[i]].long()].reshape(-1, *c.shape[2:])[:sizes[i] + pasts[i]]
+        for r in range(0, sizes[i], max(1, sizes[i] // 7)):
+            n = pasts[i] + r + 1
+            ref = _attention64(q[at + r], pick(kc)[:n], pick(vc)[:n], pick(ks)[:n], pick(vs)[:n],
+                               None if gate is None else gate[at + r]).reshape(-1)
+            # keys, values and weights in FP16 (2^-11 each) under a softmax of many terms, FP16 output
+            err = (out[at + r].cpu().double() - ref).norm() / ref.norm()
+            assert float(err) < 2e-3, (i, r, float(err))
+        at += sizes[i]
