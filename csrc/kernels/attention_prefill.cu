@@ -1,6 +1,7 @@
 // Causal GQA flash attention for prefill chunks over the paged INT8 KV cache, on tcgen05 tensor
 // cores with TMEM accumulators.
-//  A query tile is 128 rows: P = 128 / rep consecutive query positions of one request times the
+//
+// A query tile is 128 rows: P = 128 / rep consecutive query positions of one request times the
 // `rep` query heads that share one KV head (the heads are packed into the MMA M axis so each INT8
 // K/V page is dequantised once for all of them).  One CTA owns NQ tiles: in large packets of head
 // sizes 64 and 128 two neighbouring ones, so that a dequantised page serves 256 rows and the
@@ -22,7 +23,8 @@
 // With one tile S is double buffered instead.  Head size 256 has room for no more (Q 64 KB, two K
 // and two V buffers of 32 KB; TMEM: two S of 64 columns and O of 256) and walks the cache in half
 // pages. CTAs are ordered from the last query positions (the longest walks) to the first.
-//  A step of two tiles is a chain per tile (softmax, P V, Q K^T of the next step) and two of them
+//
+// A step of two tiles is a chain per tile (softmax, P V, Q K^T of the next step) and two of them
 // hide each other only in part: 5500 cycles for 128 keys with one softmax thread per row and the
 // MMAs issued inside a branch on the lane, about 4700 with two threads and a whole warp in the
 // issuing loop.  The tensor core needs 2050 of them, the exponentials as many. One 4096-token
@@ -33,12 +35,13 @@
 // the error against 64 bits grows by 1.8 % there and by 3.7 % for 500 rows behind 1000.  Chunks of
 // 777 and 646 rows behind 3000 positions, 16 / 2 gated heads of 256: 354 -> 276 -> 244 with K and
 // V freed apart, 223 with plain loads, 161 with the gates asked for ahead (one at a time, two
-// bytes of a row per lane, a tile's epilogue took 30 us; 17 rows 41 -> 10 us).  Where the tiles
-// are fewer than half the SMs, a cluster cuts the keys of each (SPLIT): 64 rows behind 1000 32 ->
-// @S1@, 500 behind 1000 44 -> @S2@, 64 behind 20000 @S3@. Output is O / sum, optionally times
-// sigmoid(gate), in FP16.  Replaces the prefill configurations of causal_attention_int8 and
-// dequantize_attention_kv (kernels/cuda/model/attention_rows.py:61-276,
-// kernels/cuda/model/kv_int8.py:210-247).
+// bytes of a row per lane, a tile's epilogue took 30 us; 17 rows 41 -> 10 us).
+// Where the tiles are fewer than half the SMs, the CTAs of a cluster cut the keys of each (SPLIT,
+// heads of 256 channels): 64 rows behind 1000 positions 32 -> 18.5 us, 500 behind 1000 44 -> 32.5,
+// 64 behind 20000 450 -> 72.
+// Output is O / sum, optionally times sigmoid(gate), in FP16.  Replaces the prefill
+// configurations of causal_attention_int8 and dequantize_attention_kv
+// (kernels/cuda/model/attention_rows.py:61-276, kernels/cuda/model/kv_int8.py:210-247).
 #include <cuda.h>
 
 #include "api.h"
@@ -763,11 +766,11 @@ int launch(const __half* q, const __half* gate, const Chunk* chunks, int n_chunk
 
 using namespace orinfer;
 
-// Into how many parts the keys of a tile go, the steps counted from the page table's width (heads of
-// 256 channels, one tile per CTA).  A step takes 1.35 us, a CTA about six of them besides, and a
+// Into how many parts the keys of a tile go, the steps counted from the page table's width (heads
+// of 256 channels, one tile per CTA).  A step takes 1.35 us, a CTA about six of them besides, and a
 // part five more to be put together with the others; a larger number has to save 15 %.  (More parts
-// than SMs did not pay: 180 CTAs of 60 steps 161 us whole, 152 in two parts, 195 in four, but 188 of
-// 12 steps 45 and 72.)
+// than SMs did not pay: 180 CTAs of 60 steps 161 us whole, 152 in two parts, 195 in four, but 188
+// of 12 steps 45 and 72.)
 static int prefill_ranks(long long ctas, long long steps) {
   int best = 1;
   double least = 0;

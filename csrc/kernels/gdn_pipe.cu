@@ -15,11 +15,11 @@
 // unrolled: 8500 cycles a round, rolled 6300); all loads ahead, four sums in turn instead of two,
 // state and output warps on schedulers of their own, or outputs held back until S^T k is through:
 // no change.
-//  32 heads of 128 channels, convolution and norm included: one run of 1050 rows 205 -> 154 us,
-// two 245 -> 180, one of 4000 731 -> 544, two of 64 29.0 -> 24.4, one of 40 24.9 -> 21.2.  With
-// more CTAs than SMs, two waves of these stand against one of two per SM: three runs of 40 rows 31
-// against 37, of 250 88 against 94, eight of 160 136 against 138, and from some 400 rows on these
-// win again (three of 500 177 -> 169, eight of 500 364 -> 348).
+// 32 heads of 128 channels, with the convolution and the norm of then: one run of 1050 rows 205 ->
+// 155 us, two 245 -> 181, one of 4000 725 -> 547, two of 250 71 -> 54, two of 64 29.1 -> 24.5, one
+// of 40 24.4 -> 21.  With more CTAs than SMs, two waves of these stand against one of two per SM:
+// three runs of 40 rows 31 against 37, of 250 88 against 94, sixteen of 64 115 against 127, and from
+// some 400 rows on these win again (three of 1000 337 -> 315, eight of 500 364 -> 349).
 #include "api.h"
 #include "common.cuh"
 #include "gdn_chunk.cuh"
