@@ -154,6 +154,7 @@ int orinfer_moe_combine_peer(const __half* expert_out, const int* slots, const f
                              int rows, int top_k, const __half* shared_out,
                              const float* shared_gate, const OrinferPeerOut* peers, int hidden,
                              cudaStream_t stream);
+int orinfer_qgemm_small_rows(int fmt, int M, int N, int K);
 int orinfer_qgemm_launches(int M, int N, int K, int out_f32, int force_path);
 int orinfer_qgemm_launches_fmt(int fmt, int M, int N, int K, int out_f32, int force_path);
 int orinfer_qgemm_set_variant(int fmt, int m_lo, int m_hi, int n, int k, int mt, int nb,

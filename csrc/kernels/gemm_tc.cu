@@ -28,6 +28,9 @@ namespace orinfer {
 int qgemv_dispatch(int fmt, const int8_t* a, const float* as, const void* w, const __half* ws,
                    void* out, int M, int N, int K, int out_f32, cudaStream_t stream,
                    const PeerOut* peer);
+bool qgemv_wide(int fmt, int M, int N, int K);
+int qgemv_wide_dispatch(int fmt, const int8_t* a, const float* as, const void* w, const __half* ws,
+                        void* out, int M, int N, int K, int out_f32, cudaStream_t stream);
 int qgemv_grouped_dispatch(int fmt, const int8_t* a, const float* as, const void* w,
                            const __half* ws, void* out, int N, int K, long long bank,
                            const int* tiles, const int* meta, int most_rows, int max_tiles,
@@ -1856,6 +1859,8 @@ static int qgemm_any(int fmt, const int8_t* a, const float* a_scale, const void*
     }
     return 0;
   }
+  if (force_path == 0 && peer == nullptr && qgemv_wide(fmt, M, N, K))
+    return qgemv_wide_dispatch(fmt, a, a_scale, w, w_scale, out, M, N, K, out_f32, stream);
   PeerOut po{};
   if (peer != nullptr) po = *peer;
   if (fmt == 0)
@@ -1869,6 +1874,7 @@ static int qgemm_any(int fmt, const int8_t* a, const float* a_scale, const void*
 extern "C" int orinfer_qgemm_launches_fmt(int fmt, int M, int N, int K, int out_f32,
                                           int force_path) {
   if (force_path == 1 || (force_path == 0 && M <= 8)) return (M + 7) / 8;
+  if (force_path == 0 && qgemv_wide(fmt, M, N, K)) return 1;
   const tc::Plan p = tc::make_plan(fmt, M, N, K, out_f32, false);
   // K splits are added up inside the one-tile kernel when the tiles are small; otherwise,
   // and in the persistent forms, a second pass adds them
@@ -1880,6 +1886,11 @@ extern "C" int orinfer_qgemm_launches_fmt(int fmt, int M, int N, int K, int out_
   const bool second =
       p.splits > 1 && !(tc::g_impl == 1 && tc::splitk_in_kernel(p.mt, 128, p.splits));
   return second ? 2 : 1;
+}
+
+// Whether nine to sixteen rows take the small-M kernels (on one GPU, without a forced path).
+extern "C" int orinfer_qgemm_small_rows(int fmt, int M, int N, int K) {
+  return M <= 8 || qgemv_wide(fmt, M, N, K) ? 1 : 0;
 }
 
 extern "C" int orinfer_qgemm_launches(int M, int N, int K, int out_f32, int force_path) {

@@ -1,4 +1,4 @@
-// Small-M quantised GEMM (decode path, M <= 8): weight-bandwidth bound.  Each CTA
+// Small-M quantised GEMM (decode path, M <= 8, and up to 16): weight-bandwidth bound.  Each CTA
 // owns a few output rows and streams their weights once; lanes decode E8P codes through a
 // shared-memory value table and the products with the INT8 activations staged in shared
 // memory run on the tensor cores (mma.sync, 16 weight rows x 8 activation rows), or by dp4a for
@@ -94,6 +94,8 @@ struct GemvUnit {
 template <int FMT, int MT, bool DP4A>
 __device__ __forceinline__ int act_pos(int m, int k, int K) {
   if (DP4A) return m * K + k;
+  if (MT == 16)                                  // two planes of eight rows, as the MMAs take them
+    return (m >> 3) * 8 * K + act_pos<FMT, MT == 16 ? 8 : MT, false>(m & 7, k, K);
   if (FMT == 0) return ((k >> 6) * MT + m) * 64 + (k & 63);
   const int o = (k >> 3) & 15;
   return (((k >> 7) * 16 + (o & 3) * 4 + (o >> 2)) * MT + m) * 8 + (k & 7);
@@ -332,13 +334,14 @@ __device__ __forceinline__ void gemv_finish(int* acc_s, const int* asum, const f
   const bool ll = peer != nullptr && po.rows_per == LL_MODE;
   // sum_k a_k w_k from the staged integers: Q4 2*acc - 75*S, Q2 2*acc - 15*S
   constexpr int UNIT = FMT == 0 ? 1 : 2, BIAS = FMT == 0 ? 0 : (FMT == 1 ? 75 : 15);
+  constexpr size_t WS_COLS = MT > 8 ? GEMV_WS_COLS / 2 : GEMV_WS_COLS;
   bool finalize = true;
   if (k_parts > 1) {
     // add this CTA's integers to the workspace; the last CTA of the n-part finishes
     for (int i = tid; i < n_count * MT; i += THREADS) {
       const int m = i / n_count, r = i % n_count;
       const int v = acc_s[r * MT + m];
-      if (m < M && v != 0) atomicAdd(ws + static_cast<size_t>(m) * GEMV_WS_COLS + n_base + r, v);
+      if (m < M && v != 0) atomicAdd(ws + m * WS_COLS + n_base + r, v);
     }
     __threadfence();
     __syncthreads();
@@ -356,7 +359,7 @@ __device__ __forceinline__ void gemv_finish(int* acc_s, const int* asum, const f
         const int m = i / n_count, r = i % n_count;
         int v = 0;
         if (m < M) {
-          int* p = ws + static_cast<size_t>(m) * GEMV_WS_COLS + n_base + r;
+          int* p = ws + m * WS_COLS + n_base + r;
           v = __ldcg(p);
           *p = 0;
         }
@@ -510,7 +513,9 @@ __global__ void __launch_bounds__(GEMV_THREADS, 1) qgemv_kernel(
 #pragma unroll
     for (int i = 0; i < DEPTH; ++i) fetch(buf[i], u_lo + i);
   }
-  int acc[4] = {0, 0, 0, 0};
+  constexpr int COLS = MT == 16 ? 2 : 1;           // eight activation rows each
+  constexpr int MC = MT == 16 ? 8 : MT;
+  int acc[COLS][4] = {};
   const uint32_t lane4 = lane * 4;
   for (int base = u_lo; base < u_hi; base += DEPTH) {
 #pragma unroll
@@ -520,22 +525,34 @@ __global__ void __launch_bounds__(GEMV_THREADS, 1) qgemv_kernel(
         if (FMT == 0) {
 #pragma unroll
           for (int j = 0; j < 2; ++j) {
-            int4 b = make_int4(0, 0, 0, 0);
-            if (g < MT)
-              b = *reinterpret_cast<const int4*>(
-                  act + act_pos<FMT, MT, false>(g, ckb * 128 + j * 64 + t * 16, K));
+            int4 b[COLS];
+#pragma unroll
+            for (int c = 0; c < COLS; ++c) {
+              b[c] = make_int4(0, 0, 0, 0);
+              if (g < MC)
+                b[c] = *reinterpret_cast<const int4*>(
+                    act + act_pos<FMT, MT, false>(g + 8 * c, ckb * 128 + j * 64 + t * 16, K));
+            }
             const uint32_t* r0 = buf[i].w[0] + (j * 4) % Unit::WORDS;
             const uint32_t* r1 = buf[i].w[1] + (j * 4) % Unit::WORDS;
-            mma_i8_16832(acc, r0[0], r1[0], r0[1], r1[1], b.x, b.y);
-            mma_i8_16832(acc, r0[2 % Unit::WORDS], r1[2 % Unit::WORDS], r0[3 % Unit::WORDS],
-                         r1[3 % Unit::WORDS], b.z, b.w);
+#pragma unroll
+            for (int c = 0; c < COLS; ++c) {
+              mma_i8_16832(acc[c], r0[0], r1[0], r0[1], r1[1], b[c].x, b[c].y);
+              mma_i8_16832(acc[c], r0[2 % Unit::WORDS], r1[2 % Unit::WORDS], r0[3 % Unit::WORDS],
+                           r1[3 % Unit::WORDS], b[c].z, b[c].w);
+            }
           }
         } else {
 #pragma unroll
           for (int j = 0; j < 4; ++j) {
-            int2 b = make_int2(0, 0);
-            if (g < MT)
-              b = *reinterpret_cast<const int2*>(act + ((ckb * 16 + j * 4 + t) * MT + g) * 8);
+            int2 b[COLS];
+#pragma unroll
+            for (int c = 0; c < COLS; ++c) {
+              b[c] = make_int2(0, 0);
+              if (g < MC)
+                b[c] = *reinterpret_cast<const int2*>(
+                    act + c * 8 * K + ((ckb * 16 + j * 4 + t) * MC + g) * 8);
+            }
             uint32_t lo[2] = {0u, 0u}, hi[2] = {0u, 0u};
 #pragma unroll
             for (int h = 0; h < 2; ++h) {
@@ -547,19 +564,23 @@ __global__ void __launch_bounds__(GEMV_THREADS, 1) qgemv_kernel(
               lo[h] = v.x;
               hi[h] = v.y;
             }
-            mma_i8_16832(acc, lo[0], lo[1], hi[0], hi[1], b.x, b.y);
+#pragma unroll
+            for (int c = 0; c < COLS; ++c)
+              mma_i8_16832(acc[c], lo[0], lo[1], hi[0], hi[1], b[c].x, b[c].y);
           }
         }
         fetch(buf[i], base + i + DEPTH);
         const bool last_of_group = ckb + 1 == kb_hi, last_unit = base + i + 1 == u_hi;
         if (last_of_group || last_unit) {
 #pragma unroll
-          for (int e = 0; e < 4; ++e) {
-            const int m = 2 * t + (e & 1);
-            if (m < MT && !(half && e >= 2))
-              atomicAdd(&acc_s[(cg * ROWS + g + (e >> 1) * 8) * MT + m], acc[e]);
-            acc[e] = 0;
-          }
+          for (int c = 0; c < COLS; ++c)
+#pragma unroll
+            for (int e = 0; e < 4; ++e) {
+              const int m = 2 * t + (e & 1) + 8 * c;
+              if (m < MT && !(half && e >= 2))
+                atomicAdd(&acc_s[(cg * ROWS + g + (e >> 1) * 8) * MT + m], acc[c][e]);
+              acc[c][e] = 0;
+            }
         }
         if (last_of_group) {
           ckb = kb_lo;
@@ -807,7 +828,9 @@ __global__ void __launch_bounds__(W8_WARPS * 32) w8_gemv_kernel(
 // eight 78 -> 63.7.  Below about 24 M weights the set-up of the rings costs more than it gives:
 // one row of 12288 x 2560 9.3 -> 9.1 us, eight rows 12.5 both ways, but 6144 x 2560 5.7 -> 6.7 and
 // 9.1 -> 9.9.  It takes three stages: with the two that eight rows of 4096 channels leave, 32000
-// rows gain nothing.
+// rows gain nothing.  Nine to sixteen rows (a second set of products, fewer stages) from 100 M
+// weights on: 151936 x 2560 72 to 74 us against 81 to 83 in the form above, 40000 x 2560 28 both,
+// 19456 x 2560 20 against 18.
 constexpr int STREAM_ROWS = 16, STREAM_MAX = 8;
 
 inline int w8_stream_stages(int M, int K) {
@@ -818,9 +841,11 @@ inline int w8_stream_stages(int M, int K) {
 }
 
 inline bool w8_streams(int M, int N, int K) {
-  return w8_stream_stages(M, K) >= 3 && static_cast<long long>(N) * K >= 24000000;
+  return w8_stream_stages(M, K) >= 3 &&
+         static_cast<long long>(N) * K >= (M > 8 ? 100000000 : 24000000);
 }
 
+template <int PLANES>                                      // of eight activation rows
 __global__ void __launch_bounds__((1 + STREAM_MAX) * 32) w8_stream_kernel(
     const int8_t* a, const float* a_scale, const int8_t* w, const __half* w_scale,
     void* __restrict__ out, int M, int N, int K, int out_f32, int stages, int* status) {
@@ -866,37 +891,49 @@ __global__ void __launch_bounds__((1 + STREAM_MAX) * 32) w8_stream_kernel(
     return;
   }
   const int s = warp - 1;
-  const float sa0 = 2 * t < M ? a_scale[2 * t] : 0.f;
-  const float sa1 = 2 * t + 1 < M ? a_scale[2 * t + 1] : 0.f;
-  const unsigned char* brow = act + min(g, M - 1) * stride + t * 16;
+  float sa[PLANES][2];
+  const unsigned char* brow[PLANES];
+  bool live[PLANES];                                       // columns past the last row are zero
+#pragma unroll
+  for (int p = 0; p < PLANES; ++p) {
+#pragma unroll
+    for (int e = 0; e < 2; ++e)
+      sa[p][e] = 8 * p + 2 * t + e < M ? a_scale[8 * p + 2 * t + e] : 0.f;
+    live[p] = 8 * p + g < M;
+    brow[p] = act + min(8 * p + g, M - 1) * stride + t * 16;
+  }
   const unsigned char* r0 = ring + static_cast<size_t>(s * STREAM_ROWS + g) * stride + t * 16;
   const unsigned char* r1 = r0 + 8 * stride;
-  const bool live = g < M;                                 // columns past the last row are zero
   for (int i = s; i < count; i += stages) {
     const int n = (blockIdx.x + i * gridDim.x) * STREAM_ROWS + g;
     const float w0 = n < N ? __half2float(w_scale[n]) : 0.f;
     const float w1 = n + 8 < N ? __half2float(w_scale[n + 8]) : 0.f;
     const bool ok = mbar_wait(&full[s], (i / stages) & 1, status, STATUS_DECODE_WAIT, i);
     if (!__all_sync(0xffffffffu, ok)) break;
-    int acc[2][4] = {};
+    int acc[PLANES][2][4] = {};
 #pragma unroll 4
     for (int k = 0; k < K; k += 64) {
       const uint4 x = *reinterpret_cast<const uint4*>(r0 + k);
       const uint4 y = *reinterpret_cast<const uint4*>(r1 + k);
-      uint4 b = make_uint4(0, 0, 0, 0);
-      if (live) b = *reinterpret_cast<const uint4*>(brow + k);
-      mma_i8_16832(acc[0], x.x, y.x, x.y, y.y, b.x, b.y);
-      mma_i8_16832(acc[1], x.z, y.z, x.w, y.w, b.z, b.w);
+#pragma unroll
+      for (int p = 0; p < PLANES; ++p) {
+        uint4 b = make_uint4(0, 0, 0, 0);
+        if (live[p]) b = *reinterpret_cast<const uint4*>(brow[p] + k);
+        mma_i8_16832(acc[p][0], x.x, y.x, x.y, y.y, b.x, b.y);
+        mma_i8_16832(acc[p][1], x.z, y.z, x.w, y.w, b.z, b.w);
+      }
     }
     // every word of the tile went into one of these two chains of sums
-    hand_back(&empty[s], static_cast<uint32_t>(acc[0][0] ^ acc[1][0]));
+    hand_back(&empty[s], static_cast<uint32_t>(acc[0][0][0] ^ acc[0][1][0]));
 #pragma unroll
-    for (int e = 0; e < 4; ++e) {
-      const int m = 2 * t + (e & 1), at = n + (e >> 1) * 8;
-      if (m < M && at < N)
-        store_row<1>(out, out_f32, m, at, N, acc[0][e] + acc[1][e], e >> 1 ? w1 : w0,
-                     e & 1 ? sa1 : sa0);
-    }
+    for (int p = 0; p < PLANES; ++p)
+#pragma unroll
+      for (int e = 0; e < 4; ++e) {
+        const int m = 8 * p + 2 * t + (e & 1), at = n + (e >> 1) * 8;
+        if (m < M && at < N)
+          store_row<1>(out, out_f32, m, at, N, acc[p][0][e] + acc[p][1][e], e >> 1 ? w1 : w0,
+                       sa[p][e & 1]);
+      }
   }
 }
 
@@ -1250,7 +1287,7 @@ static int launch_gemv(const int8_t* a, const float* as, const void* w, const __
                                               g.max_groups, runtime_gemv_workspace(), fz);
     return static_cast<int>(cudaGetLastError());
   };
-  if constexpr (FMT != 0)
+  if constexpr (FMT != 0 && MT <= 8)
     if (gemv_dp4a(FMT, MT, N, K, fz.pre != 0))
       return start(e8p_dp4a_kernel<FMT, MT>, Dp4a<FMT, MT>::THREADS, static_cast<const uint4*>(w),
                    slot[0]);
@@ -1280,10 +1317,11 @@ static int launch_w8_stream(const int8_t* a, const float* as, const void* w, con
                             void* out, int M, int N, int K, int out_f32, cudaStream_t stream) {
   const int stages = w8_stream_stages(M, K);
   const size_t smem = static_cast<size_t>(K + 64) * (M + stages * STREAM_ROWS);
-  static const int slot = runtime_new_slot();
-  if (const int e = runtime_allow_smem(slot, w8_stream_kernel, GEMV_SMEM_LIMIT)) return e;
+  static const int slot[2] = {runtime_new_slot(), runtime_new_slot()};
+  auto kernel = M > 8 ? w8_stream_kernel<2> : w8_stream_kernel<1>;
+  if (const int e = runtime_allow_smem(slot[M > 8], kernel, GEMV_SMEM_LIMIT)) return e;
   const int tiles = (N + STREAM_ROWS - 1) / STREAM_ROWS;
-  launch_early(w8_stream_kernel, tiles < 148 ? tiles : 148, (1 + stages) * 32, smem, stream, a,
+  launch_early(kernel, tiles < 148 ? tiles : 148, (1 + stages) * 32, smem, stream, a,
                as, reinterpret_cast<const int8_t*>(w), ws, out, M, N, K, out_f32, stages,
                runtime_status_ptr());
   return static_cast<int>(cudaGetLastError());
@@ -1329,6 +1367,31 @@ int qgemv_dispatch(int fmt, const int8_t* a, const float* as, const void* w, con
   if (fmt == 2) return BY_M(launch_gemv, 2, );
 #undef BY_M
   return -1;
+}
+
+// Nine to sixteen rows take a second set of products over the same decoded weights: exact sums, so
+// the bits of the tensor-core GEMM, which decodes a tile for 128 rows however few there are.  Q4,
+// sixteen rows: 19456 x 2560 28.2 -> 18.0 us (eight rows 14.6), 12288 x 2048 22.5 -> 12.9, 6144 x
+// 2560 12.4 -> 11.2, 1024 x 2048 11.8 -> 8.0; INT8 19456 x 2560 26.2 -> 17.8, 151936 x 2560 as a
+// stream 96 -> 74.  Short rows (4096 x 768 5.6 against 7.1) and long ones, whose activations
+// fill the shared memory of the one CTA (2560 x 8192 16.3 against 17.2, 2560 x 9728 16.8 against
+// 19.7), stay on the tensor cores, as do launches to peers.
+bool qgemv_wide(int fmt, int M, int N, int K) {
+  if (M <= 8 || M > 16) return false;
+  if (fmt == 0 && w8_streams(M, N, K)) return true;
+  if (K < 1024 || K > 6144) return false;
+  const GemvGrid g = gemv_grid(fmt, N, K);
+  if (g.k_parts > 1 && N > GEMV_WS_COLS / 2) return false;
+  return fmt == 0 || gemv_smem(fmt, 16, g, K, false) <= GEMV_SMEM_LIMIT;
+}
+int qgemv_wide_dispatch(int fmt, const int8_t* a, const float* as, const void* w, const __half* ws,
+                        void* out, int M, int N, int K, int out_f32, cudaStream_t stream) {
+  const PeerOut po{};
+  if (fmt == 0 && w8_streams(M, N, K))
+    return launch_w8_stream(a, as, w, ws, out, M, N, K, out_f32, stream);
+  if (fmt == 0) return launch_gemv<0, 16>(a, as, w, ws, out, M, N, K, out_f32, stream, po);
+  if (fmt == 1) return launch_gemv<1, 16>(a, as, w, ws, out, M, N, K, out_f32, stream, po);
+  return launch_gemv<2, 16>(a, as, w, ws, out, M, N, K, out_f32, stream, po);
 }
 
 // Projection of at most 8 rows with the row preparation fused in (see GemvFuse); E8P weights.

@@ -65,6 +65,7 @@ def _load() -> ctypes.CDLL:
         "orinfer_qgemm_grouped_launches": ([I, I, I, I, I, I], I),
         "orinfer_moe_dispatch_ep": ([P, I, I, I, I, P, P, I, P, P, P, P, I, P, P, P, P], I),
         "orinfer_sample_topk": ([P, I, I, c_longlong, P, P, P, P, P, P, P], I),
+        "orinfer_qgemm_small_rows": ([I, I, I, I], I),
         "orinfer_qgemm_launches": ([I, I, I, I, I], I),
         "orinfer_qgemm_launches_fmt": ([I, I, I, I, I, I], I),
         "orinfer_qgemm_set_variant": ([I, I, I, I, I, I, I, I], I),

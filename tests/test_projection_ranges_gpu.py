@@ -266,3 +266,40 @@ def test_swiglu_rows_of_large_packets_have_the_bits_of_small_ones(dev, k, signed
                        rows=rows, q_out=q2, scale_out=s2)
     assert torch.equal(q2[:1025], q[:1025]) and bool((q2[1025:] == 77).all())
     assert bool((s2[1025:] == 77).all())
+
+
+# nine to sixteen rows on the small-M kernels: row groups cut by N, K splits (their workspace halved
+# in width), the shortest and longest rows they take, and one past each
+@pytest.mark.parametrize("fmt", ["w8", "q4", "q2"])
+@pytest.mark.parametrize("m", [9, 12, 16])
+@pytest.mark.parametrize("n,k,small", [(8, 1024, True), (24, 1152, True), (2376, 1024, True),
+                                       (264, 6144, True), (2560, 4096, True), (6152, 2176, True),
+                                       (40000, 1024, True), (512, 896, False), (264, 6272, False)])
+def test_sixteen_row_projections_are_exact(dev, fmt, m, n, k, small):
+    from orinfer_b200.ops import functional as F
+    from orinfer_b200.ops import native
+    assert native.lib().orinfer_qgemm_small_rows(F.FMT[fmt], m, n, k) == int(small)
+    assert not native.lib().orinfer_qgemm_small_rows(F.FMT[fmt], 17, n, k)
+    g = torch.Generator().manual_seed(m * n + k)
+    codes, ws, w = _int_weight(fmt, n, k, g)
+    a = torch.randint(-127, 128, (m, k), generator=g, dtype=torch.int8)
+    sa = torch.rand(m, generator=g) * 0.05 + 1e-3
+    want = _scaled(a, sa, w, ws)
+    for f32 in (False, True, False):                   # repeated: the workspace is left empty
+        out = F.qgemm(a.to(dev), sa.to(dev), codes.to(dev), ws.to(dev), fmt, n, out_f32=f32)
+        assert torch.equal(out.cpu(), want if f32 else want.half())
+
+
+@pytest.mark.parametrize("m", [9, 13, 16])
+@pytest.mark.parametrize("n,k", [(97664, 1024), (100008, 1152), (32008, 3200)])
+def test_streamed_int8_projections_of_sixteen_rows_are_exact(dev, m, n, k):
+    from orinfer_b200.ops import functional as F
+    g = torch.Generator(device=dev).manual_seed(m * n + k)
+    w = torch.randint(-127, 128, (n, k), generator=g, device=dev, dtype=torch.int8)
+    ws = (torch.rand(n, generator=g, device=dev) * 0.01 + 1e-3).half()
+    a = torch.randint(-127, 128, (m, k), generator=g, device=dev, dtype=torch.int8)
+    sa = torch.rand(m, generator=g, device=dev) * 0.05 + 1e-3
+    want = _scaled(a, sa, w, ws)
+    for f32 in (False, True) * 5:            # repeated: stages are refilled while others run
+        out = F.qgemm(a, sa, w, ws, "w8", n, out_f32=f32)
+        assert torch.equal(out, want if f32 else want.half())
