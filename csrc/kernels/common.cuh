@@ -426,38 +426,61 @@ struct E8pTables {
   uint32_t sg[256];
 };
 
-// Shared-memory working copy: COPIES replicas interleaved word by word, lane l reads replica
-// l % COPIES.  The lookups of a warp are random in the entry index; with one copy they
-// collide on the 32 banks about 3.5-fold, with 8 copies about 2-fold, with 32 copies never.
+// Shared-memory working copy of the tensor-core kernels: COPIES replicas, an entry's words of both
+// tables in one row, lane l reads replica l % COPIES.  The lookups of a warp are random in the
+// entry. Of the two that a code takes, the lower lanes do the one in e2 first and the upper lanes
+// the one in sg: with 16 replicas the two halves of a warp then read different halves of the banks
+// and never collide, where 32 lanes in one table of 16 replicas do, two and two; with 8 or 4 they
+// collide less (2048 x 19456 x 2560 Q4 116.2 -> 111.5 us, 1024 rows 64.5 -> 62.4, 512 rows 39.0 ->
+// 38.3; 64 x 2560 x 9728 16.9 -> 16.4).
 template <int COPIES>
 struct E8pLut {
-  uint32_t e2[256 * COPIES];
-  uint32_t sg[256 * COPIES];
+  uint32_t w[256][2][COPIES];                           // [entry][e2, sg][replica]
 };
 
 template <int COPIES>
 __device__ __forceinline__ void e8p_lut_init(E8pLut<COPIES>* sm, const E8pTables* __restrict__ g,
                                              int tid, int nthreads) {
   static_assert(COPIES % 4 == 0, "filled with 16-byte stores");
-  constexpr int PER = COPIES / 4;                       // 16-byte stores per entry
-  for (int j = tid; j < 256 * PER; j += nthreads) {
-    const int i = j / PER;
-    const uint32_t a = g->e2[i], b = g->sg[i];
-    reinterpret_cast<uint4*>(sm->e2)[j] = make_uint4(a, a, a, a);
-    reinterpret_cast<uint4*>(sm->sg)[j] = make_uint4(b, b, b, b);
+  constexpr int PER = COPIES / 4;                       // 16-byte stores per word
+  for (int j = tid; j < 512 * PER; j += nthreads) {
+    const int i = j / (2 * PER);
+    const uint32_t v = (j / PER) & 1 ? g->sg[i] : g->e2[i];
+    reinterpret_cast<uint4*>(sm->w)[j] = make_uint4(v, v, v, v);
   }
 }
 
-// The 4-bit fields v of the code in the low (HALF = 0) or high (HALF = 1) half of `word`.
-template <int COPIES, int HALF>
-__device__ __forceinline__ uint32_t e8p_fields(uint32_t word, const E8pLut<COPIES>* __restrict__ sm,
-                                               int copy) {
-  const uint32_t idx = __byte_perm(word, 0, HALF ? 0x4443 : 0x4441);
-  const uint32_t sgn = __byte_perm(word, 0, HALF ? 0x4442 : 0x4440);
-  return sm->e2[idx * COPIES + copy] ^ sm->sg[sgn * COPIES + copy];
-}
+// What a lane needs for its lookups: where its replica's words stand in the first row, the half's
+// first lookup (a) and second (b), and the byte selectors of their entries.
+template <int COPIES>
+struct E8pLane {
+  const unsigned char *a, *b;
+  uint32_t sel_a, sel_b;
+  __device__ __forceinline__ E8pLane(const E8pLut<COPIES>* lut, int lane) {
+    const int upper = (lane >> 4) & 1;
+    a = reinterpret_cast<const unsigned char*>(&lut->w[0][upper][lane & (COPIES - 1)]);
+    b = reinterpret_cast<const unsigned char*>(&lut->w[0][upper ^ 1][lane & (COPIES - 1)]);
+    sel_a = 0x4441 - upper;
+    sel_b = 0x4440 + upper;
+  }
+};
 
 constexpr uint32_t E8P_NIB = 0x0f0f0f0fu;
+
+// The fields v of the code in the low (HALF = 0) or high (HALF = 1) half of `word`: even ones in
+// the low halves of the bytes (lo), odd ones still in the high halves (hi).
+template <int HALF, int COPIES>
+__device__ __forceinline__ void e8p_fields(uint32_t word, const E8pLane<COPIES>& t, uint32_t& lo,
+                                           uint32_t& hi) {
+  constexpr uint32_t ROW = 8 * COPIES;
+  const uint32_t ia = __byte_perm(word, 0, t.sel_a + 2 * HALF);
+  const uint32_t ib = __byte_perm(word, 0, t.sel_b + 2 * HALF);
+  const uint32_t x = *reinterpret_cast<const uint32_t*>(t.a + ia * ROW);
+  const uint32_t y = *reinterpret_cast<const uint32_t*>(t.b + ib * ROW);
+  // one instruction each: (x ^ y) & NIB, (x ^ y) & ~NIB
+  asm("lop3.b32 %0, %1, %2, %3, 0x28;" : "=r"(lo) : "r"(x), "r"(y), "r"(E8P_NIB));
+  asm("lop3.b32 %0, %1, %2, %3, 0x14;" : "=r"(hi) : "r"(x), "r"(y), "r"(E8P_NIB));
+}
 
 // The form of the small-M kernels: 32 replicas, and an entry's two words in one 256-byte row, so
 // that an address is a byte permute of the code word and the lane's offset (4 * lane) and nothing
@@ -523,25 +546,22 @@ __device__ __forceinline__ int dp4a_us(uint32_t w, int a, int c) {
 
 // One Q4 word (coarse U16 low, residual U16 high) -> eight INT8 weights 4*c0 + c1.
 template <int COPIES>
-__device__ __forceinline__ uint2 e8p_decode_q4(uint32_t word, const E8pLut<COPIES>* __restrict__ sm,
-                                               int copy) {
-  const uint32_t v0 = e8p_fields<COPIES, 0>(word, sm, copy);
-  const uint32_t v1 = e8p_fields<COPIES, 1>(word, sm, copy);
+__device__ __forceinline__ uint2 e8p_decode_q4(uint32_t word, const E8pLane<COPIES>& t) {
+  uint32_t l0, h0, l1, h1;
+  e8p_fields<0>(word, t, l0, h0);
+  e8p_fields<1>(word, t, l1, h1);
   // biased byte 8*v0 + 2*v1 + (128 - 75) is in 73..183: no carries; XOR 0x80 -> two's complement
-  uint32_t lo = (v0 & E8P_NIB) * 8u + 0x35353535u;
-  lo = ((v1 & E8P_NIB) * 2u + lo) ^ 0x80808080u;
-  uint32_t hi = ((v0 >> 4) & E8P_NIB) * 8u + 0x35353535u;
-  hi = (((v1 >> 4) & E8P_NIB) * 2u + hi) ^ 0x80808080u;
-  return make_uint2(lo, hi);
+  const uint32_t lo = l1 * 2u + (l0 * 8u + 0x35353535u);
+  const uint32_t hi = (h0 >> 1) + (h1 >> 3) + 0x35353535u;
+  return make_uint2(lo ^ 0x80808080u, hi ^ 0x80808080u);
 }
 
 // One Q2 code (HALF of `word`) -> eight INT8 weights 2*v - 15.
-template <int COPIES, int HALF>
-__device__ __forceinline__ uint2 e8p_decode8(uint32_t word, const E8pLut<COPIES>* __restrict__ sm,
-                                             int copy) {
-  const uint32_t v = e8p_fields<COPIES, HALF>(word, sm, copy);
-  return make_uint2(((v & E8P_NIB) * 2u + 0x71717171u) ^ 0x80808080u,
-                    (((v >> 4) & E8P_NIB) * 2u + 0x71717171u) ^ 0x80808080u);
+template <int HALF, int COPIES>
+__device__ __forceinline__ uint2 e8p_decode_q2(uint32_t word, const E8pLane<COPIES>& t) {
+  uint32_t lo, hi;
+  e8p_fields<HALF>(word, t, lo, hi);
+  return make_uint2((lo * 2u + 0x71717171u) ^ 0x80808080u, ((hi >> 3) + 0x71717171u) ^ 0x80808080u);
 }
 
 // Host-side runtime state, one set per device (runtime.cu): the status word that bounded

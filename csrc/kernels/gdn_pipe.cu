@@ -14,12 +14,12 @@
 // chain.  On the way: code that does not stay in the instruction cache cost most (T, P and A
 // unrolled: 8500 cycles a round, rolled 6300); all loads ahead, four sums in turn instead of two,
 // state and output warps on schedulers of their own, or outputs held back until S^T k is through:
-// no change.
-// 32 heads of 128 channels, with the convolution and the norm of then: one run of 1050 rows 205 ->
-// 155 us, two 245 -> 181, one of 4000 725 -> 547, two of 250 71 -> 54, two of 64 29.1 -> 24.5, one
-// of 40 24.4 -> 21.  With more CTAs than SMs, two waves of these stand against one of two per SM:
-// three runs of 40 rows 31 against 37, of 250 88 against 94, sixteen of 64 115 against 127, and from
-// some 400 rows on these win again (three of 1000 337 -> 315, eight of 500 364 -> 349).
+// no change.  32 heads of 128 channels, with the convolution and the norm of then: one run of 1050
+// rows 205 -> 155 us, two 245 -> 181, one of 4000 725 -> 547, two of 250 71 -> 54, two of 64 29.1
+// -> 24.5, one of 40 24.4 -> 21.  With more CTAs than SMs, two waves of these stand against one of
+// two per SM: three runs of 40 rows 31 against 37, of 250 88 against 94, sixteen of 64 115 against
+// 127, and from some 400 rows on these win again (three of 1000 337 -> 315, eight of 500 364 ->
+// 349).
 #include "api.h"
 #include "common.cuh"
 #include "gdn_chunk.cuh"

@@ -70,11 +70,11 @@ struct Layout {
   static constexpr int SA_FIT = (BUDGET - SB * BC_BYTES) / A_BYTES;
   static constexpr int SA = SA_FIT >= 4 ? 4 : SA_FIT;
   static_assert(SA >= 2 && SB >= 2, "at least double buffering");
-  // Copies of the decode tables: the lookups of a warp are random and collide about 3-fold with 4
-  // copies, 1.5-fold with 16.  Q4 looks up twice per code and gains where a CTA decodes wide tiles
-  // (19456 x 2560: 128 rows 33.6 -> 30.6 us, 2048 rows 128 -> 125 for the projection); Q2 and
-  // narrow tiles lose the time it takes to fill more copies (5120 x 2048, 512 rows, Q2: 25.0
-  // against 25.9 us), as do they all once the rings leave no room.
+  // Copies of the decode tables: the lookups of a warp are random and collide the less the more
+  // copies there are, with 16 not at all.  Q4 takes two codes per eight weights and gains where a
+  // CTA decodes wide tiles (19456 x 2560: 128 rows 33.6 -> 30.6 us, 2048 rows 128 -> 125 for the
+  // projection); Q2 and narrow tiles lose the time it takes to fill more copies (5120 x 2048, 512
+  // rows, Q2: 25.0 against 25.9 us), as do they all once the rings leave no room.
   static constexpr int RINGS = SA * A_BYTES + SB * BC_BYTES;
   static constexpr int LUT_COPIES =
       FMT != 1 || NB != 128 ? 4
@@ -305,7 +305,7 @@ __global__ void __launch_bounds__(THREADS, 1) qgemm_tc_kernel(
     bool ok = true;
     if (FMT != 0) {
       const int chunk = t & 7, rbase = t >> 3;          // 64 weight rows per pass
-      const int copy = t & (L::LUT_COPIES - 1);
+      const E8pLane<L::LUT_COPIES> look(lut, lane);
       for (int kb = 0; kb < kblocks; ++kb) {
         const int s = kb % SB;
         // the codes of this phase are only requested after the tensor core released the
@@ -322,13 +322,13 @@ __global__ void __launch_bounds__(THREADS, 1) qgemm_tc_kernel(
           if (row < rows_valid) {
             if (FMT == 1) {
               const uint2 wd = *reinterpret_cast<const uint2*>(cs + row * 64 + chunk * 8);
-              const uint2 q0 = e8p_decode_q4(wd.x, lut, copy);
-              const uint2 q1 = e8p_decode_q4(wd.y, lut, copy);
+              const uint2 q0 = e8p_decode_q4(wd.x, look);
+              const uint2 q1 = e8p_decode_q4(wd.y, look);
               v = make_uint4(q0.x, q0.y, q1.x, q1.y);
             } else {
               const uint32_t wd = *reinterpret_cast<const uint32_t*>(cs + row * 32 + chunk * 4);
-              const uint2 q0 = e8p_decode8<L::LUT_COPIES, 0>(wd, lut, copy);
-              const uint2 q1 = e8p_decode8<L::LUT_COPIES, 1>(wd, lut, copy);
+              const uint2 q0 = e8p_decode_q2<0>(wd, look);
+              const uint2 q1 = e8p_decode_q2<1>(wd, look);
               v = make_uint4(q0.x, q0.y, q1.x, q1.y);
             }
           }
@@ -853,7 +853,7 @@ __global__ void __launch_bounds__(THREADS, 1) qgemm_ps_kernel(
     // ---------------- producers (lattice decode) and epilogue
     const int t512 = threadIdx.x - ROLE_THREADS;                  // 0..511
     const int chunk = t512 & 7, rbase = t512 >> 3;      // 64 weight rows per pass
-    const int copy = t512 & (L::LUT_COPIES - 1);
+    const E8pLane<L::LUT_COPIES> look(lut, lane);
     const int quad = warp & 3;                          // TMEM lane quadrant of this warp
     const int part = (warp - 3) >> 2;                   // 0..3: which 32-column chunks
     const int row = quad * 32 + lane;
@@ -991,13 +991,13 @@ __global__ void __launch_bounds__(THREADS, 1) qgemm_ps_kernel(
             if (wrow < T.rows_valid) {
               if (FMT == 1) {
                 const uint2 wd = *reinterpret_cast<const uint2*>(cs + wrow * 64 + chunk * 8);
-                const uint2 q0 = e8p_decode_q4(wd.x, lut, copy);
-                const uint2 q1 = e8p_decode_q4(wd.y, lut, copy);
+                const uint2 q0 = e8p_decode_q4(wd.x, look);
+                const uint2 q1 = e8p_decode_q4(wd.y, look);
                 v = make_uint4(q0.x, q0.y, q1.x, q1.y);
               } else {
                 const uint32_t wd = *reinterpret_cast<const uint32_t*>(cs + wrow * 32 + chunk * 4);
-                const uint2 q0 = e8p_decode8<L::LUT_COPIES, 0>(wd, lut, copy);
-                const uint2 q1 = e8p_decode8<L::LUT_COPIES, 1>(wd, lut, copy);
+                const uint2 q0 = e8p_decode_q2<0>(wd, look);
+                const uint2 q1 = e8p_decode_q2<1>(wd, look);
                 v = make_uint4(q0.x, q0.y, q1.x, q1.y);
               }
             }
@@ -1283,7 +1283,7 @@ __global__ void __launch_bounds__(THREADS, 1) qgemm_pair_kernel(
     // ---------------- producers (lattice decode of this CTA's weight rows) and epilogue
     const int t512 = threadIdx.x - ROLE_THREADS;
     const int chunk = t512 & 7, rbase = t512 >> 3;
-    const int copy = t512 & (L::LUT_COPIES - 1);
+    const E8pLane<L::LUT_COPIES> look(lut, lane);
     const int quad = warp & 3;
     const int part = (warp - 3) >> 2;
     const int row = quad * 32 + lane;
@@ -1398,13 +1398,13 @@ __global__ void __launch_bounds__(THREADS, 1) qgemm_pair_kernel(
             if (wrow < T.rows_valid) {
               if (FMT == 1) {
                 const uint2 wd = *reinterpret_cast<const uint2*>(cs + wrow * 64 + chunk * 8);
-                const uint2 q0 = e8p_decode_q4(wd.x, lut, copy);
-                const uint2 q1 = e8p_decode_q4(wd.y, lut, copy);
+                const uint2 q0 = e8p_decode_q4(wd.x, look);
+                const uint2 q1 = e8p_decode_q4(wd.y, look);
                 v = make_uint4(q0.x, q0.y, q1.x, q1.y);
               } else {
                 const uint32_t wd = *reinterpret_cast<const uint32_t*>(cs + wrow * 32 + chunk * 4);
-                const uint2 q0 = e8p_decode8<L::LUT_COPIES, 0>(wd, lut, copy);
-                const uint2 q1 = e8p_decode8<L::LUT_COPIES, 1>(wd, lut, copy);
+                const uint2 q0 = e8p_decode_q2<0>(wd, look);
+                const uint2 q1 = e8p_decode_q2<1>(wd, look);
                 v = make_uint4(q0.x, q0.y, q1.x, q1.y);
               }
             }

@@ -20,10 +20,10 @@
 // What bounds it: INT8 weights take 67 cycles per 128 x 128 x 32 MMA when their copies are there
 // (2048 x 19456 x 2560 126 -> 86 us, 2.4 PFLOP/s).  Lattice codes: the decode warps, 1100 to 1500
 // cycles per k-block (72 % of the shared-memory pipe, 66 % of the issue slots, 21 % of the tensor
-// core); signs from arithmetic instead of lookups, and with them a conflict-free
-// table, made that a sixth longer.  128 Q4 experts of 768 with 128 rows each, a whole layer:
-// 447 -> 340 us (463 -> 326 with the router's and the launches' share; votes on every wait and the
-// activations' own barrier cost 1.5 % of it).
+// core, while lookups still collided: 15 us of a layer's 305 went with that); signs from
+// arithmetic instead of lookups made that a sixth longer.  128 Q4 experts of 768 with 128 rows
+// each, a whole layer: 447 -> 340 us (463 -> 326 with the router's and the launches' share; votes
+// on every wait and the activations' own barrier cost 1.5 % of it).
 #include <cuda.h>
 
 #include "api.h"
@@ -79,36 +79,6 @@ struct Args {
 struct Tile {
   int n0, m0, m_limit, expert, mt_act;
 };
-
-// As e8p_decode_q4 and e8p_decode8, with the fields taken apart by one logic instruction each: even
-// ones in the low halves of the bytes (lo), odd ones still in the high halves (hi).
-template <int COPIES, int HALF>
-__device__ __forceinline__ void fields(uint32_t word, const E8pLut<COPIES>* __restrict__ lut,
-                                       int copy, uint32_t& lo, uint32_t& hi) {
-  const uint32_t idx = __byte_perm(word, 0, HALF ? 0x4443 : 0x4441);
-  const uint32_t sgn = __byte_perm(word, 0, HALF ? 0x4442 : 0x4440);
-  const uint32_t e = lut->e2[idx * COPIES + copy], s = lut->sg[sgn * COPIES + copy];
-  asm("lop3.b32 %0, %1, %2, %3, 0x28;" : "=r"(lo) : "r"(e), "r"(s), "r"(E8P_NIB));
-  asm("lop3.b32 %0, %1, %2, %3, 0x14;" : "=r"(hi) : "r"(e), "r"(s), "r"(E8P_NIB));
-}
-template <int COPIES>
-__device__ __forceinline__ uint2 decode_q4(uint32_t word, const E8pLut<COPIES>* __restrict__ lut,
-                                           int copy) {
-  uint32_t l0, h0, l1, h1;
-  fields<COPIES, 0>(word, lut, copy, l0, h0);
-  fields<COPIES, 1>(word, lut, copy, l1, h1);
-  const uint32_t lo = l1 * 2u + (l0 * 8u + 0x35353535u);
-  const uint32_t hi = (h0 >> 1) + (h1 >> 3) + 0x35353535u;
-  return make_uint2(lo ^ 0x80808080u, hi ^ 0x80808080u);
-}
-template <int COPIES, int HALF>
-__device__ __forceinline__ uint2 decode_q2(uint32_t word, const E8pLut<COPIES>* __restrict__ lut,
-                                           int copy) {
-  uint32_t lo, hi;
-  fields<COPIES, HALF>(word, lut, copy, lo, hi);
-  return make_uint2((lo * 2u + 0x71717171u) ^ 0x80808080u,
-                    ((hi >> 3) + 0x71717171u) ^ 0x80808080u);
-}
 
 template <int FMT, int MT>
 __global__ void __launch_bounds__(Layout<FMT, MT>::THREADS, 1) qgemm_walk_kernel(
@@ -411,7 +381,7 @@ __global__ void __launch_bounds__(Layout<FMT, MT>::THREADS, 1) qgemm_walk_kernel
   } else if (FMT != 0 && warp >= FIRST_DEC) {
     // ---------------- lattice decode: 64 rows of 16 bytes x 8 threads per pass
     const int t = tid - FIRST_DEC * 32, chunk = t & 7, first = t >> 3;
-    const int copy = lane & (L::COPIES - 1);
+    const E8pLane<L::COPIES> look(lut, lane);
     // The code words of a k-block are read while the one before it waits for its place.
     uint32_t cr = 0, cb = 0, cf = 0;               // k-blocks read, decoded and handed back
     const int me = blockIdx.x, ctas = gridDim.x;
@@ -447,11 +417,11 @@ __global__ void __launch_bounds__(Layout<FMT, MT>::THREADS, 1) qgemm_walk_kernel
         const int row = first + 64 * i;
         uint2 x, y;
         if constexpr (FMT == 1) {
-          x = decode_q4(cur[i].x, lut, copy);
-          y = decode_q4(cur[i].y, lut, copy);
+          x = e8p_decode_q4(cur[i].x, look);
+          y = e8p_decode_q4(cur[i].y, look);
         } else {
-          x = decode_q2<L::COPIES, 0>(cur[i].x, lut, copy);
-          y = decode_q2<L::COPIES, 1>(cur[i].x, lut, copy);
+          x = e8p_decode_q2<0>(cur[i].x, look);
+          y = e8p_decode_q2<1>(cur[i].x, look);
         }
         // (rows past the matrix: their codes are stale, their products are not stored)
         *reinterpret_cast<uint4*>(bs + swz128(row, chunk)) = make_uint4(x.x, x.y, y.x, y.y);
