@@ -18,12 +18,18 @@
 // accumulators (MT = 1 or 2).
 //
 // What bounds it: INT8 weights take 67 cycles per 128 x 128 x 32 MMA when their copies are there
-// (2048 x 19456 x 2560 126 -> 86 us, 2.4 PFLOP/s).  Lattice codes: the decode warps, 1100 to 1500
-// cycles per k-block (72 % of the shared-memory pipe, 66 % of the issue slots, 21 % of the tensor
-// core, while lookups still collided: 15 us of a layer's 305 went with that); signs from
-// arithmetic instead of lookups made that a sixth longer.  128 Q4 experts of 768 with 128 rows
-// each, a whole layer: 447 -> 340 us (463 -> 326 with the router's and the launches' share; votes
-// on every wait and the activations' own barrier cost 1.5 % of it).
+// (2048 x 19456 x 2560 126 -> 86 us, 2.4 PFLOP/s).  Lattice codes: the decode warps (66 % of the
+// issue slots).  With all sixteen on one k-block, each decoded for 540 to 650 of its 1280 to 1500
+// cycles; the rest were two waits (170 each), the fence and the hand-overs.  So groups of them take
+// k-blocks in turn, each warp with twice (Q2 with one row tile: four times) as many rows between
+// two waits: 128 Q4 experts of 768, a whole layer, 2048 rows 292 -> 270 us, 1024 rows 243 -> 210,
+// 300 rows 211 -> 179; 512 Q2 experts of 512, 2048 rows 619 -> 539, 1024 rows 519 -> 439 (Q4 in
+// four groups: 223 where two take 214).  Signs from arithmetic instead of lookups made a layer a
+// sixth longer; codes loaded into registers from global memory four k-blocks ahead, with a 64 KB
+// table whose addresses are single byte permutes (a quarter fewer instructions), 303 against 292
+// us: the loads are waited for.  The whole layer came from 447 us over 340 (this kernel) and 326
+// (the router's and the launches' share; votes on every wait and the activations' own barrier cost
+// 1.5 %), and 15 us of 305 went with lookups that collide.
 #include <cuda.h>
 
 #include "api.h"
@@ -53,6 +59,13 @@ struct Layout {
   static constexpr int SC = FMT == 0 ? 1 : (FMT == 1 ? 4 : 8); // packed codes
   static constexpr int BUFS = 2;                               // accumulator sets in TMEM
   static constexpr int COPIES = 16;
+  // Groups of decode warps, which take k-blocks in turn.  A group waits for a stage by the parity
+  // of its barrier, which tells one use from the next but not from the one after that.  With no
+  // more groups than stages no group is two uses ahead: its own k-block c - GROUPS went into a
+  // stage that c - GROUPS - S had left, and with that every k-block up to c - 2 S.  A slab of codes
+  // is always the same group's.
+  static constexpr int GROUPS = FMT == 2 && S >= 4 ? 4 : 2, GROUP_WARPS = DEC_WARPS / GROUPS;
+  static_assert(FMT == 0 || (GROUPS <= S && SC % GROUPS == 0), "parities of the rings");
   static constexpr int TABLES = FMT == 0 ? 0 : static_cast<int>(sizeof(E8pLut<COPIES>));
   static constexpr int CODE_OFF = S * STAGE;
   static constexpr int TABLE_OFF = CODE_OFF + SC * CODES;
@@ -162,12 +175,12 @@ __global__ void __launch_bounds__(Layout<FMT, MT>::THREADS, 1) qgemm_walk_kernel
   if (tid == 0) {
     for (int s = 0; s < S; ++s) {
       mbar_init(&a_full[s], 1);
-      mbar_init(&full[s], FMT == 0 ? 1 : DEC_WARPS);
+      mbar_init(&full[s], FMT == 0 ? 1 : L::GROUP_WARPS);
       mbar_init(&empty[s], 1);
     }
     for (int s = 0; s < SC; ++s) {
       mbar_init(&c_full[s], 1);
-      mbar_init(&c_empty[s], DEC_WARPS);
+      mbar_init(&c_empty[s], L::GROUP_WARPS);
     }
     for (int b = 0; b < BUFS; ++b) {
       mbar_init(&acc_full[b], 1);
@@ -379,49 +392,42 @@ __global__ void __launch_bounds__(Layout<FMT, MT>::THREADS, 1) qgemm_walk_kernel
       }
     }
   } else if (FMT != 0 && warp >= FIRST_DEC) {
-    // ---------------- lattice decode: 64 rows of 16 bytes x 8 threads per pass
-    const int t = tid - FIRST_DEC * 32, chunk = t & 7, first = t >> 3;
+    // ---------------- lattice decode: a group's rows of 16 bytes x 8 threads per pass
+    constexpr int STEP = L::GROUP_WARPS * 4, PASSES = BN / STEP;
+    const int t = tid - FIRST_DEC * 32, chunk = t & 7, first = (t >> 3) % STEP;
     const E8pLane<L::COPIES> look(lut, lane);
-    // The code words of a k-block are read while the one before it waits for its place.
-    uint32_t cr = 0, cb = 0, cf = 0;               // k-blocks read, decoded and handed back
     const int me = blockIdx.x, ctas = gridDim.x;
     const int own_tiles = total > me ? (total - 1 - me) / ctas + 1 : 0;
     const uint32_t all = static_cast<uint32_t>(own_tiles) * kblocks;
-    bool ok = true;
-    uint2 word[2];
-    auto read = [&]() {
-      const uint32_t sc = cr % SC;
-      ok = warp_all(WALK_WAIT(&c_full[sc], (cr / SC) & 1, STATUS_DECODE_WAIT, cr & 0x7ff));
+    for (uint32_t cb = (warp - FIRST_DEC) / L::GROUP_WARPS; cb < all; cb += L::GROUPS) {
+      const uint32_t sc = cb % SC, sb = cb % S;
+      bool ok = warp_all(WALK_WAIT(&c_full[sc], (cb / SC) & 1, STATUS_DECODE_WAIT, cb & 0x7ff));
+      if (!ok) break;
       const unsigned char* cs = code_s + sc * L::CODES;
+      uint2 word[PASSES];
+      uint32_t seen = 0;
 #pragma unroll
-      for (int i = 0; i < 2; ++i) {
-        const int row = first + 64 * i;
+      for (int i = 0; i < PASSES; ++i) {
+        const int row = first + STEP * i;
         word[i] = make_uint2(0u, 0u);
         if (FMT == 1) word[i] = *reinterpret_cast<const uint2*>(cs + row * 64 + chunk * 8);
         else word[i].x = *reinterpret_cast<const uint32_t*>(cs + row * 32 + chunk * 4);
+        seen ^= word[i].x ^ word[i].y;
       }
-      ++cr;
-    };
-    if (all > 0) read();
-    while (ok && cb < all) {
-      const uint2 cur[2] = {word[0], word[1]};
-      if (cr < all) read();
-      const uint32_t sb = cb % S;
-      if (ok)
-        ok = warp_all(WALK_WAIT(&empty[sb], ((cb / S) & 1) ^ 1, STATUS_DECODE_WAIT,
-                                0x800 | (cb & 0x7ff)));
+      ok = warp_all(WALK_WAIT(&empty[sb], ((cb / S) & 1) ^ 1, STATUS_DECODE_WAIT,
+                              0x800 | (cb & 0x7ff)));
       if (!ok) break;
       unsigned char* bs = smem + sb * L::STAGE + MT * TILE;
 #pragma unroll
-      for (int i = 0; i < 2; ++i) {
-        const int row = first + 64 * i;
+      for (int i = 0; i < PASSES; ++i) {
+        const int row = first + STEP * i;
         uint2 x, y;
         if constexpr (FMT == 1) {
-          x = e8p_decode_q4(cur[i].x, look);
-          y = e8p_decode_q4(cur[i].y, look);
+          x = e8p_decode_q4(word[i].x, look);
+          y = e8p_decode_q4(word[i].y, look);
         } else {
-          x = e8p_decode_q2<0>(cur[i].x, look);
-          y = e8p_decode_q2<1>(cur[i].x, look);
+          x = e8p_decode_q2<0>(word[i].x, look);
+          y = e8p_decode_q2<1>(word[i].x, look);
         }
         // (rows past the matrix: their codes are stale, their products are not stored)
         *reinterpret_cast<uint4*>(bs + swz128(row, chunk)) = make_uint4(x.x, x.y, y.x, y.y);
@@ -429,10 +435,7 @@ __global__ void __launch_bounds__(Layout<FMT, MT>::THREADS, 1) qgemm_walk_kernel
       fence_proxy_async();
       __syncwarp();
       if (lane == 0) mbar_arrive(&full[sb]);
-      ++cb;
-      // the slab of the words just read, which the next round uses, goes back (see hand_back)
-      const uint32_t seen = word[0].x ^ word[0].y ^ word[1].x ^ word[1].y;
-      for (; cf < cr; ++cf) hand_back(&c_empty[cf % SC], seen);
+      hand_back(&c_empty[sc], seen);
     }
   }
 #undef WALK_WAIT
