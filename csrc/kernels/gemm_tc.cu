@@ -1626,29 +1626,10 @@ int launch(const int8_t* a, const float* a_scale, const void* w, const __half* w
   return static_cast<int>(cudaGetLastError());
 }
 
-// Tile choice.  Rows: as many accumulators as the packet fills (each decoded weight tile is
-// then multiplied against up to 512 rows).  Weight rows per CTA: the widest tile that still
-// gives the grid about one CTA per SM, so narrow projections (N = hidden) do not leave most
-// of the machine idle.  FP32 output is only used by the (very wide) vocabulary head.
 // Cells of the split-K workspace one split of an M x N product needs: its tiles are stored
 // whole, so both extents round up to the largest tile.
 inline size_t padded_cells(int M, int N) {
   return static_cast<size_t>((M + 4 * BM - 1) / (4 * BM)) * (4 * BM) * ((N + 127) / 128) * 128;
-}
-
-inline int plan_splits(int M, int N, int K, int out_f32) {
-  const int mt = M > 2 * BM ? 4 : (M > BM ? 2 : 1);
-  const long c128 = static_cast<long>((M + BM * mt - 1) / (BM * mt)) * ((N + 127) / 128);
-  int splits = 1;
-  if (!out_f32 && c128 <= 74 && K / BK >= 8 && N % 8 == 0) {
-    splits = static_cast<int>(148 / c128);
-    splits = splits > K / BK / 8 ? K / BK / 8 : splits;          // at least 8 k-blocks each
-    splits = splits > 8 ? 8 : splits;
-    while (splits > 1 &&
-           static_cast<size_t>(splits) * padded_cells(M, N) * 4 > SPLITK_WORKSPACE_BYTES)
-      --splits;
-  }
-  return splits < 1 ? 1 : splits;
 }
 
 // ---------------------------------------------------------------- launch plan
@@ -1692,7 +1673,74 @@ inline int tail_splits_for(int M, int K, int tail_tiles) {
   return static_cast<int>(ts > 8 ? 8 : (ts < 1 ? 1 : ts));
 }
 
-inline Plan make_plan(int fmt, int M, int N, int K, int out_f32, bool fused) {
+// Whether an (MT * 128) x 128 tiling of M rows and n columns goes to the kernel that walks many
+// tiles per CTA: from a second wave of tiles on.  Its tiles have two row tiles at most, so plans
+// of lattice codes that serve four stay with the one-tile kernel (whether two and a walk are
+// cheaper is cheapest_plan's question: 2048 x 19456 x 2560 Q4 111 us on both, 4096 rows 212 and
+// 207); INT8 2048 x 19456 x 2560 117 against 86 (126 with the issuing loop of one lane that the
+// one-tile kernel had before).
+inline bool walks(int fmt, int mt, int M, int n) {
+  const long tiles = static_cast<long>((M + BM * mt - 1) / (BM * mt)) * ((n + 127) / 128);
+  return g_impl == 1 && g_probe == 0 && tiles > NUM_SMS && (fmt == 0 || mt <= 2);
+}
+
+// Microseconds that a plan takes on one GPU, about: waves of CTAs, each with a part that does not
+// depend on K (its start and its epilogue, which grows with the tile) and k-blocks that cost the
+// slowest of the decode (per 128 weight rows), the MMAs (per 128 x 128) and the activation tiles
+// (per 128 rows) on top of their waits.  The walking kernel starts once and overlaps the rest, but
+// its decode and its MMAs share the shared memory, so that they add up; K splits pay for their
+// partial sums (per MB).  Fitted to 8436 timings: three formats, ten projections of 2048..9728
+// channels, 130..3000 rows, every plan; 8 % from them on average.
+inline float plan_cost(int fmt, int M, int N, int K, const Plan& p) {
+  static constexpr float DECODE[3] = {0.f, 0.34f, 0.28f};
+  static constexpr float WALKED[3] = {0.03f, 0.305f, 0.165f}, PER_ROWS[3] = {0.2f, 0.145f, 0.17f};
+  const bool walk = p.nb == 128 && p.splits == 1 && walks(fmt, p.mt, M, N);
+  const float mt = static_cast<float>(walk && p.mt > 2 ? 2 : p.mt), nb = p.nb / 128.f;
+  const int rows = 128 * static_cast<int>(mt), kb = (K / BK + p.splits - 1) / p.splits;
+  const long tiles = static_cast<long>((M + rows - 1) / rows) * ((N + p.nb - 1) / p.nb) * p.splits;
+  // a peeled tail is half a wave
+  const float waves = p.tail_splits > 0 ? static_cast<float>(tiles / NUM_SMS) + 0.5f
+                                        : static_cast<float>((tiles + NUM_SMS - 1) / NUM_SMS);
+  if (walk) {
+    // its row tiles past the last row are not multiplied
+    const float used = static_cast<float>((M + BM - 1) / BM) / ((M + rows - 1) / rows);
+    return 4.7f + waves * kb * (WALKED[fmt] + PER_ROWS[fmt] * used);
+  }
+  const float block = 0.18f + fmaxf(fmaxf(DECODE[fmt] * nb, 0.095f * mt * nb), 0.077f * mt);
+  const float sums = p.splits > 1 ? 4.2f + 0.76e-6f * M * N * p.splits : 0.f;
+  return waves * (0.75f + 3.f * mt * nb + kb * block) + sums;
+}
+
+// The plan of least cost, for more than one row tile and the channels that the costs were fitted
+// for; `p` where nothing is 3 % below it.  Against the rules of make_plan with the packaged table,
+// 612 shapes (130..4096 rows, half of them not in the fit) take 20 % less time on average, the
+// worst 4 % more: 512 x 12288 x 2048 Q4 32.9 -> 22.4 us, 512 x 2560 x 9728 37.9 -> 27.3, 600 x
+// 19456 x 2560 63.5 -> 48.2.  Over the fitted shapes the best plan of each is 4 % below.  A tile
+// of one row tile and fewer than 128 weight rows never pays: every CTA reads all rows, for little.
+inline Plan cheapest_plan(int fmt, int M, int N, int K, const Plan& p) {
+  if (M <= BM || K / BK < 16) return p;
+  Plan best = p;
+  float least = 0.97f * plan_cost(fmt, M, N, K, p);
+  for (int mt = 1; mt <= 4 && (mt == 1 || M > BM * (mt / 2)); mt *= 2) {
+    const long tiles = static_cast<long>((M + BM * mt - 1) / (BM * mt)) * ((N + 127) / 128);
+    for (int nb = 128; nb >= (mt == 1 ? 128 : 32); nb /= 2) {
+      for (int splits = 1; splits <= 8; ++splits) {
+        if (splits > 1 && (nb != 128 || N % 8 != 0 || tiles > 74 || splits > K / BK / 2 ||
+                           splits * padded_cells(M, N) * 4 > SPLITK_WORKSPACE_BYTES))
+          break;
+        const Plan q{mt, nb, splits, 0, 0};
+        const float cost = plan_cost(fmt, M, N, K, q);
+        if (cost < least) {
+          best = q;
+          least = cost;
+        }
+      }
+    }
+  }
+  return best;
+}
+
+inline Plan make_plan(int fmt, int M, int N, int K, int out_f32, bool fused, bool one_gpu) {
   Plan p{};
   p.mt = M > 2 * BM ? 4 : (M > BM ? 2 : 1);
   if (!out_f32) {
@@ -1725,7 +1773,7 @@ inline Plan make_plan(int fmt, int M, int N, int K, int out_f32, bool fused) {
   if (narrow && M > BM && K / BK <= 48) {
     p.mt = M <= 6 * BM ? 2 : 4;
     p.nb = M <= 2 * BM ? 32 : 64;
-    return p;
+    return one_gpu ? cheapest_plan(fmt, M, N, K, p) : p;
   }
   if (narrow) {
     int splits = static_cast<int>(148 / c128);
@@ -1752,17 +1800,7 @@ inline Plan make_plan(int fmt, int M, int N, int K, int out_f32, bool fused) {
     p.tail_tiles = static_cast<int>(ntiles - keep);
     p.tail_splits = tail_splits_for(M, K, p.tail_tiles);
   }
-  return p;
-}
-
-// Whether an (MT * 128) x 128 tiling of M rows and n columns goes to the kernel that walks many
-// tiles per CTA: from a second wave of tiles on.  Its tiles have two row tiles at most, so lattice
-// codes that serve four stay here: 2048 x 19456 x 2560 Q4 118 us against 139, 1024 rows 67 against
-// 79, 600 rows 64 against 62; 200 x 40000 x 1024 31 against 27; INT8 2048 x 19456 x 2560 117
-// against 86 (126 with the issuing loop of one lane that the one-tile kernel had before).
-inline bool walks(int fmt, int mt, int M, int n) {
-  const long tiles = static_cast<long>((M + BM * mt - 1) / (BM * mt)) * ((n + 127) / 128);
-  return g_impl == 1 && g_probe == 0 && tiles > NUM_SMS && (fmt == 0 || mt <= 2);
+  return one_gpu && !out_f32 ? cheapest_plan(fmt, M, N, K, p) : p;
 }
 
 // Columns that a plan leaves to the one-tile launch, or to the walking one, before its tail.
@@ -1784,7 +1822,7 @@ int launch_fmt(const int8_t* a, const float* a_scale, const void* w, const __hal
       return launch_pair<FMT, true>(a, a_scale, w, w_scale, out, M, N, K, stream, po, ag);
     return launch_pair<FMT, false>(a, a_scale, w, w_scale, out, M, N, K, stream, po, ag);
   }
-  const Plan plan = make_plan(FMT, M, N, K, out_f32, po.tp != 0);
+  const Plan plan = make_plan(FMT, M, N, K, out_f32, po.tp != 0, po.tp == 0 && ag.tp == 0);
   const int mt = plan.mt, nb = plan.nb, splits = plan.splits, cut = main_columns(plan, N);
   const bool walk = po.tp == 0 && ag.tp == 0 && plan_walks(FMT, plan, M, N, out_f32);
   const WalkCall walk_call{a, a_scale, w, w_scale, static_cast<__half*>(out), M, N, K, cut,
@@ -1875,7 +1913,7 @@ extern "C" int orinfer_qgemm_launches_fmt(int fmt, int M, int N, int K, int out_
                                           int force_path) {
   if (force_path == 1 || (force_path == 0 && M <= 8)) return (M + 7) / 8;
   if (force_path == 0 && qgemv_wide(fmt, M, N, K)) return 1;
-  const tc::Plan p = tc::make_plan(fmt, M, N, K, out_f32, false);
+  const tc::Plan p = tc::make_plan(fmt, M, N, K, out_f32, false, true);
   // K splits are added up inside the one-tile kernel when the tiles are small; otherwise,
   // and in the persistent forms, a second pass adds them
   if (p.tail_splits > 0) {
@@ -1932,7 +1970,7 @@ extern "C" int orinfer_qgemm_set_impl(int impl) {
 
 // The plan for a shape: out[0..3] = mt, nb, splits, tail_splits.
 extern "C" void orinfer_qgemm_plan(int fmt, int M, int N, int K, int out_f32, int* out) {
-  const tc::Plan p = tc::make_plan(fmt, M, N, K, out_f32, false);
+  const tc::Plan p = tc::make_plan(fmt, M, N, K, out_f32, false, true);
   out[0] = p.mt;
   out[1] = p.nb;
   out[2] = p.splits;
@@ -1941,7 +1979,7 @@ extern "C" void orinfer_qgemm_plan(int fmt, int M, int N, int K, int out_f32, in
 
 // Whether the walking kernel takes the shape on one GPU, a peeled tail apart.
 extern "C" int orinfer_qgemm_walks(int fmt, int M, int N, int K, int out_f32) {
-  const tc::Plan p = tc::make_plan(fmt, M, N, K, out_f32, false);
+  const tc::Plan p = tc::make_plan(fmt, M, N, K, out_f32, false, true);
   return tc::plan_walks(fmt, p, M, N, out_f32) ? 1 : 0;
 }
 

@@ -118,6 +118,30 @@ def test_walked_tiles_are_exact(dev, fmt, m, n, k):
         lib.orinfer_qgemm_clear_variants()
 
 
+@pytest.mark.parametrize("fmt", ["w8", "q4", "q2"])
+@pytest.mark.parametrize("m", [129, 300, 513, 1100])
+@pytest.mark.parametrize("n,k", [(1000, 2048), (2568, 4096), (6144, 2048), (12296, 2176)])
+def test_plans_of_least_cost_are_exact(dev, fmt, m, n, k):
+    """Plans chosen by their cost: narrow and wide tiles, K splits and walked tiles, columns that no
+    tile width divides; without a tuned table."""
+    from orinfer_b200.ops import functional as F
+    from orinfer_b200.ops import native
+    from orinfer_b200.tuning import tables
+    lib = native.lib()
+    g = torch.Generator().manual_seed(m + n + k)
+    codes, ws, w = _int_weight(fmt, n, k, g)
+    a = torch.randint(-127, 128, (m, k), generator=g, dtype=torch.int8)
+    sa = torch.rand(m, generator=g) * 0.05 + 1e-3
+    want = _scaled(a.to(dev), sa.to(dev), w.to(dev), ws.to(dev)).half()
+    lib.orinfer_qgemm_clear_variants()
+    try:
+        for _ in range(2):
+            out = F.qgemm(a.to(dev), sa.to(dev), codes.to(dev), ws.to(dev), fmt, n)
+            assert torch.equal(out, want)
+    finally:
+        tables.load_default(lib)
+
+
 @pytest.mark.parametrize("rows", [1, 7, 149, 300, 2049])
 @pytest.mark.parametrize("k", [128, 384, 768, 2176, 6144, 6272, 9728, 16384])
 @pytest.mark.parametrize("mode", ["norm", "plain", "swiglu", "bare"])
