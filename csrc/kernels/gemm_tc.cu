@@ -2076,12 +2076,17 @@ static int grouped_row_tiles(int fmt, int expected, int experts) {
 
 // Whether the walking kernel takes the tiles of a grouped call, however many there are.  Whole
 // layers of experts of 768: 128 Q4 experts, 2048 rows 447 -> 340 us, 300 rows 300 -> 213; INT8 390
-// -> 281; and with fewer tiles than SMs, 4 and 8 experts, 64 rows 62 -> 48 and 64 -> 50 (INT8 58 ->
-// 37 and 58 -> 42), 512 rows 79 -> 65 and 75 -> 65 (a part of these is the early start of their
-// kernels).  Codes that serve four row tiles stay with the one-tile kernel, as in `walks`.
-static bool grouped_walks(int fmt, int max_tiles, int mt) {
+// -> 281; and with fewer tiles than SMs, 4 and 8 experts, 64 rows 62 -> 48 and 64 -> 50 (INT8 58
+// -> 37 and 58 -> 42), 512 rows 79 -> 65 and 75 -> 65 (a part of these is the early start of their
+// kernels).  Codes that serve four row tiles stay with the one-tile kernel where few experts leave
+// it less than about a wave of them (16 such tiles with 12 or 16 weight tiles each): 8 Q4 experts
+// of 768, 512 rows 78.5 against 82.1 us, 300 rows 69.8 against 80.2.  From there on the walk is
+// shorter: 16 experts, 600 rows 108 -> 106, 1100 rows 171 -> 144; 32 experts, 2500 rows 318 ->
+// 258; 128 experts, 4200 rows 580 -> 472, 9000 rows 1117 -> 988 (Q2 550 -> 432 and 1073 -> 911).
+static bool grouped_walks(int fmt, int max_tiles, int mt, int expected, int experts) {
+  const long long tall = (expected / experts + 511) / 512 * static_cast<long long>(experts);
   return tc::g_impl == 1 && tc::g_probe == 0 && max_tiles <= walk_list_room(fmt) &&
-         (fmt == 0 || mt <= 2);
+         (fmt == 0 || mt <= 2 || tall >= 16);
 }
 
 template <int FMT>
@@ -2107,7 +2112,7 @@ static int qgemm_grouped_fmt(const int8_t* a, const float* a_scale, const void* 
                                              ag, 1, 0, N);
   }
   const int mt = grouped_row_tiles(FMT, expected, experts);
-  if (grouped_walks(FMT, max_tiles, mt))
+  if (grouped_walks(FMT, max_tiles, mt, expected, experts))
     return qgemm_walk_dispatch(FMT, mt > 1 ? 2 : 1,
                                WalkCall{a, a_scale, w, w_scale, static_cast<__half*>(out), S, N, K,
                                         N, tiles, meta, bank, experts, max_tiles},
@@ -2146,7 +2151,8 @@ extern "C" int orinfer_qgemm_grouped_form(int fmt, int S, int experts, int max_t
   if (expected <= 0 || expected > S) expected = S;
   const GroupedPlan p = grouped_plan(fmt, S, experts, max_tiles, expected, tallest);
   if (p.rows_kernel) return p.listed > 0 ? 1 : 0;
-  return grouped_walks(fmt, max_tiles, grouped_row_tiles(fmt, expected, experts)) ? 3 : 2;
+  const int mt = grouped_row_tiles(fmt, expected, experts);
+  return grouped_walks(fmt, max_tiles, mt, expected, experts) ? 3 : 2;
 }
 
 extern "C" int orinfer_qgemm_grouped_launches(int fmt, int S, int experts, int max_tiles,

@@ -277,6 +277,39 @@ def test_walked_tile_lists_of_several_passes(dev, short, tall):
         at += c
 
 
+@pytest.mark.parametrize("fmt", ["q4", "q2"])
+def test_walked_experts_of_many_row_tiles(dev, fmt):
+    """Codes of experts with three row tiles and more, which the walking kernel takes two at a time:
+    odd numbers of them, a single row in the last, experts without rows."""
+    from orinfer_b200.ops import functional as F
+    from orinfer_b200.ops import native
+    n, k = 256, 256
+    counts = [257, 600, 0, 385, 128, 1025, 512, 300, 1, 640, 513, 256, 129, 900, 383, 300]
+    experts, s = len(counts), sum(counts)
+    assert s >= 256 * experts
+    g = torch.Generator().manual_seed(s)
+    codes, ws, _ = _int_weight(fmt, experts * n, k, g)
+    split = [codes[:, i * n:(i + 1) * n] for i in range(experts)]
+    ints = _int_weight_of(fmt, codes, ws, experts * n, k).to(dev).view(experts, n, k)
+    ws = ws.view(experts, n).to(dev)
+    a = torch.randint(-127, 128, (s, k), generator=g, dtype=torch.int8).to(dev)
+    sa = (torch.rand(s, generator=g) * 0.05 + 1e-3).to(dev)
+    ids = torch.repeat_interleave(torch.arange(experts), torch.tensor(counts)).to(torch.int32)
+    sc = F.MoeScratch(s, 1, experts, k, 64, dev)
+    F.moe_dispatch(ids[:, None].to(dev), a, sa, experts, sc, s)
+    form = native.lib().orinfer_qgemm_grouped_form
+    assert form(F.FMT[fmt], s, experts, sc.tiles.shape[0], s, s) == 3
+    assert form(F.FMT[fmt], 4096, 8, sc.tiles.shape[0], 4096, 512) == 2      # few: one wave
+    out = torch.full((s, n), float("nan"), dtype=torch.float16, device=dev)
+    banks = torch.stack(split).contiguous().to(dev)
+    F.qgemm_grouped(sc.q8, sc.scale, banks, ws, fmt, n, out, sc, s)
+    at = 0
+    for e, c in enumerate(counts):                       # the rows are in expert order already
+        want = _scaled(a[at:at + c], sa[at:at + c], ints[e], ws[e])
+        assert torch.equal(out[at:at + c], want.half()), e
+        at += c
+
+
 def _grouped_us(dev, ids, experts, n, k, fmt, banks):
     from orinfer_b200.ops import functional as F
     rows, top_k = ids.shape
