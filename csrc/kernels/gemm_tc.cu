@@ -1897,7 +1897,9 @@ static int qgemm_any(int fmt, const int8_t* a, const float* a_scale, const void*
     }
     return 0;
   }
-  if (force_path == 0 && peer == nullptr && qgemv_wide(fmt, M, N, K))
+  // (operands at other addresses go to the tensor-core kernels, which refuse what TMA cannot read)
+  const uintptr_t at = reinterpret_cast<uintptr_t>(a) | reinterpret_cast<uintptr_t>(w);
+  if (force_path == 0 && peer == nullptr && at % 16 == 0 && qgemv_wide(fmt, M, N, K))
     return qgemv_wide_dispatch(fmt, a, a_scale, w, w_scale, out, M, N, K, out_f32, stream);
   PeerOut po{};
   if (peer != nullptr) po = *peer;

@@ -327,3 +327,24 @@ def test_streamed_int8_projections_of_sixteen_rows_are_exact(dev, m, n, k):
     for f32 in (False, True) * 5:            # repeated: stages are refilled while others run
         out = F.qgemm(a, sa, w, ws, "w8", n, out_f32=f32)
         assert torch.equal(out, want if f32 else want.half())
+
+
+# operands that TMA cannot read are refused by the host, on either side of the rule for few rows
+@pytest.mark.parametrize("fmt", ["w8", "q4", "q2"])
+@pytest.mark.parametrize("m", [9, 16, 17])
+@pytest.mark.parametrize("what", ["a", "codes"])
+def test_unaligned_operands_of_nine_rows_and_more_are_refused(dev, fmt, m, what):
+    from orinfer_b200.ops import functional as F
+    from orinfer_b200.ops import native
+    n, k = 2376, 1024
+    codes, ws, _ = _int_weight(fmt, n, k, torch.Generator().manual_seed(m))
+    a = torch.ones(m, k, dtype=torch.int8)
+
+    def off(t):                                        # eight bytes past a 16-byte boundary
+        by = 8 // t.element_size()
+        return torch.cat([t.flatten()[:by], t.flatten()]).to(dev)[by:].view(t.shape)
+
+    assert off(a).data_ptr() % 16 == 8 and torch.equal(off(codes).cpu(), codes)
+    with pytest.raises(native.KernelError):
+        F.qgemm(off(a) if what == "a" else a.to(dev), torch.ones(m, device=dev),
+                off(codes) if what == "codes" else codes.to(dev), ws.to(dev), fmt, n)
