@@ -1207,7 +1207,8 @@ int orinfer_gdn_scan(const __half* qkv, const float* ab, const float* a_log, con
   if (head_dim == 128 && factors == nullptr && aligned(qkv, 16) &&
       max_seg_rows >= (n_segs == 1 ? GDN_LONG_ROWS : 64)) {
     long_rows = GDN_LONG_ROWS;
-    if (gdn_pipelined(hv, n_segs, max_seg_rows)) {
+    // (it moves state and outputs in pairs)
+    if (gdn_pipelined(hv, n_segs, max_seg_rows) && aligned(state, 8) && aligned(out, 8)) {
       if (const int e = gdn_pipe_launch(qkv, conv_dim, ab, a_log, dt_bias, sg, n_segs, row_slot,
                                         row_pos, hk, hv, state, out, stream))
         return e;

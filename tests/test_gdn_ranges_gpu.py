@@ -283,6 +283,30 @@ def test_gdn_chunked_kernels_over_their_lengths(dev, n, many):
         assert float((state[i].double() - s).norm() / s.norm()) < 2.0 ** -21
 
 
+# a state and outputs at any FP32 address, in both forms of long runs and the scan
+@pytest.mark.parametrize("lens", [[100], [257, 41], [96] * 12, [33]])
+@pytest.mark.parametrize("what", ["state", "out"])
+def test_gdn_scan_at_any_address(dev, lens, what):
+    from orinfer_b200.ops import functional as F
+
+    def off(t):
+        return torch.cat([t.flatten()[:1], t.flatten()])[1:].view(t.shape)
+
+    args, state, exact = _runs(dev, lens, 8, -1.0, len(lens))
+    out = torch.empty(sum(lens), 8, 128, device=dev)
+    if what == "state":
+        state = off(state)
+    else:
+        out = off(out)
+    assert (state if what == "state" else out).data_ptr() % 8 == 4
+    F.gdn_scan(*args[:-1], state, out=out)
+    for i in range(len(lens)):
+        ref, s, sl = exact(i)
+        # as in test_gdn_chunks_keep_fp32_accuracy, over a whole run
+        assert float((out[sl].double() - ref).norm() / ref.norm()) < 2.0 ** -21
+        assert float((state[i].double() - s).norm() / s.norm()) < 2.0 ** -21
+
+
 @pytest.mark.parametrize("row", [3, 45, 95])
 def test_gdn_many_runs_contain_non_finite_rows(dev, row):
     from orinfer_b200.ops import functional as F
