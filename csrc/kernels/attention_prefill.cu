@@ -709,6 +709,7 @@ __global__ void __launch_bounds__(Smem<D, NQ>::THREADS, 1) attn_prefill_kernel(
         }
       }
     }
+    __syncwarp();                                    // (the barrier wants whole warps)
     cluster_sync_all();                              // nobody leaves while its memory is read
   }
 }

@@ -86,6 +86,18 @@ def test_copies_in_flight_are_waited_for_on_barriers_of_their_own(path):
                 assert count == "1" or re.fullmatch(r"FMT == 0 \? 1 : .+", count), (name, count)
 
 
+@pytest.mark.parametrize("path", SOURCES, ids=lambda p: p.name)
+def test_whole_warps_arrive_at_cluster_barriers(path):
+    """The cluster barrier is of the aligned form, which every lane of a warp executes together: no
+    branch that lanes may take apart lies between it and the barrier or __syncwarp before it."""
+    for part in _code(path).split("cluster_sync_all();")[:-1]:
+        code = re.split(r"__sync(?:threads|warp)\(\);", part)[-1]
+        assert code != part, path.name
+        whole = re.compile(r"warp == \d|SPLIT")
+        apart = [c for c in re.findall(r"\bif \((.*?)\)", code) if not whole.fullmatch(c)]
+        assert not apart and not re.search(r"\b(for|while)\b", code), (path.name, code[-300:])
+
+
 def _closing(code, at):
     """Index behind the bracket that closes the one at `at`."""
     pairs, depth = {"(": 1, ")": -1, "{": 1, "}": -1}, 0
