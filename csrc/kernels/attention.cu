@@ -441,23 +441,30 @@ __global__ void __launch_bounds__(
 //   S = Q K^T: the query, FP16, becomes a fixed-point number of 31 bits under a power of two per
 //   head, and that four signed digits to the base 256; rows 4 i + r of A are digit i (the largest
 //   first) of head r.  INT32 sums over 64 channels are exact, and the digits' sums meet in FP32.
-//   O = P V: the FP32 weight x value scale becomes a fixed-point number of 31 bits, four digits,
+//   O = P V: the FP32 weight x value scale becomes a fixed-point number of 32 bits, four digits,
 //   in the same rows, and the sums stay in INT32 accumulators from block to block.
-// The weights are relative to a reference that follows the row's maximum only when that is more
-// than 2^DIGIT_LAG above it, and the value scales to the power of two above all seen: only when one
-// of them moves are the accumulators rescaled, in place.  With the lag all used up a weight keeps
-// 27 bits below the largest, and 30 at best; a query value is exact down to 2^-19 of its head's
-// largest and rounded at 2^-31 of that below it.  Error against 64 bits ahead of the output's FP16
-// rounding (2.07e-4): 8 rows of 900 keys 1.7e-7 (the form above 1.6e-7), 3 rows of 20000 2.0e-7
-// (9.2e-7), with six times the scores 6.5e-7 (7.8e-7); a lag of 2^6 gave 2.2e-7, 2.5e-7 and 7.1e-7.
+// The weights are relative to a power of two per head, which follows the row's maximum when that is
+// more than 2^DIGIT_LAG above it.  The products with the value scales have a unit per head and
+// group of 64 channels, in which the largest of them so far takes 27 to 31 bits: one that has
+// outgrown its unit shows in its first digit, and only then is the unit chosen anew, for the
+// largest product of the block, and the group's accumulators are rescaled, in place.  (Under one
+// unit for all heads, groups and keys, above the largest value scale, a group of scales 2^-k of the
+// others lost k bits, and so did all keys beside one with a large scale and no weight.)  A query
+// value is exact down to 2^-19 of its head's largest and rounded at 2^-31 of that below it.
+// Error against 64 bits ahead of the output's FP16 rounding (2.07e-4): 8 rows of 900 keys 1.7e-7
+// (the form above 1.8e-7), 3 rows of 20000 2.1e-7 (2.6e-6), with six times the scores 3.5e-7
+// (3.6e-7) and 5.6e-7 (1.2e-6); 4 rows of 900 with one group's value scales 2^-10 of the other's
+// 1.7e-7 in that group (1.8e-7, under one unit 2.4e-5), 2^-14 1.7e-7 (2.6e-7, 3.9e-4), with one key
+// of 2^10 times the scale and no weight 1.5e-7 (1.7e-7, 6.3e-6).
 //
 // K and V come by TMA as they lie in the cache, a box of 32 keys each, swizzled for ldmatrix; V's
 // fragments are transposed by the load (m16n16 b8).  A lane owns eight keys of a block in both
 // products; which ones is chosen so that neither side's loads meet on a bank.
 //
 // A block of 32 keys is 400 instructions of a warp where the form above takes about 900.  32 / 8
-// heads of 128: 6 rows of 12000..24000 keys 62.7 -> 50.3 us (235 MB; the blocks alone run at the
-// memory's rate), 38 rows of 1500..3000 57.5 -> 38.5, 128 rows of 320..640 38.7 -> 34.2.  The last
+// heads of 128: 6 rows of 12000..24000 keys 62.7 -> 49.8 us (235 MB; the blocks alone run at the
+// memory's rate), 38 rows of 1500..3000 57.5 -> 39.3, 128 rows of 320..640 38.7 -> 33.9.  (A unit
+// that gives the largest product one bit more is outgrown so often that the last takes 34.4.)  It
 // is 2.3 waves of CTAs, each of which waits 4000 cycles for its row, pages and first block and
 // takes 3000 to finish besides the 12000 of its blocks.  Tried: blocks of 64 keys with one buffer
 // (the same), the heads of a row side by side in the grid (the same, long rows 4 % slower), a warp
@@ -482,8 +489,9 @@ struct DigitTile {
     return x < 2 ? 2 * t + x : 8 + ((2 * t + 4 + (x & 1)) & 7);
   }
 };
-constexpr float DIGIT_LAG = 3.f;                         // in powers of two
-constexpr int DIGIT_BITS = 27;                           // 30 less the lag
+constexpr float DIGIT_LAG = 8.f;                         // of the weights' reference, binades
+constexpr int DIGIT_BITS = 27;                           // of the product that a unit is chosen for
+constexpr int DIGIT_UNIT_MAX = 100;                      // units are at most 2^this and begin so
 // Keys of a warp after which the accumulators are scaled down: a digit's sum grows by at most
 // 128 x 127 a key.
 constexpr int DIGIT_BLOCKS = (1 << 16) / 32;
@@ -668,9 +676,13 @@ __global__ void __launch_bounds__(ATTN_WARPS * 32, DigitTile<D>::MIN_CTAS) attn_
   for (int i = 0; i < D / 8; ++i)
 #pragma unroll
     for (int j = 0; j < 4; ++j) acc[i][j] = 0;
+  // per head: the weights are relative to 2^m_ref, a whole power, and the products with the scales
+  // of a group to its unit
   float m_ref = -INFINITY, l_run = 0.f;
-  int e_run = -100;                                // the value scales seen are below 2^e_run
-  bool poison = false;                             // a value scale was no number
+  float unit[G];
+#pragma unroll
+  for (int c = 0; c < G; ++c) unit[c] = two_to(DIGIT_UNIT_MAX);
+  uint32_t poison = 0u;                            // groups with a value scale that is no number
   bool ok = true;
 
   // row addresses of this lane: K's rows of tile i are keys 16 (i / 2) + key_of(row / 2, 2 (i % 2)
@@ -681,10 +693,7 @@ __global__ void __launch_bounds__(ATTN_WARPS * 32, DigitTile<D>::MIN_CTAS) attn_
   const int v_row = 16 * (lane >> 4) + T::key_of(kt, lane & 3);
   const float qscale = rsqrtf(static_cast<float>(D)) * 1.4426950408889634f;
 
-  // The scales of block n, by the lanes that fetched them, a block ahead of their use.  e_new and
-  // e_grows are that block's.
-  int e_new = -100;
-  bool e_grows = false;
+  // The scales of block n, by the lanes that fetched them, a block ahead of their use.
   auto place_scales = [&](int n) {
     const int key = (b0 + n * step) * KB + lane;
     const bool live = key >= k_lo && key < k_hi;
@@ -697,26 +706,17 @@ __global__ void __launch_bounds__(ATTN_WARPS * 32, DigitTile<D>::MIN_CTAS) attn_
     }
     const __half2 k2 = *reinterpret_cast<const __half2*>(&raw[0]);
     const __half2 v2 = *reinterpret_cast<const __half2*>(&raw[1]);
-    float kf[G], vf[G];
-    uint32_t vbits = 0u;
 #pragma unroll
     for (int c = 0; c < G; ++c) {
       // keys outside the split: their (possibly never written) scales unused
-      kf[c] = live ? (c == 0 ? __low2float(k2) : __high2float(k2)) * qscale : 0.f;
-      vf[c] = live ? (c == 0 ? __low2float(v2) : __high2float(v2)) : 0.f;
-      vbits = max(vbits, __float_as_uint(fabsf(vf[c])));
-    }
-    vbits = __reduce_max_sync(0xffffffffu, vbits);
-    poison = poison || vbits >= 0x7f800000u;
-    const int e_block = min(static_cast<int>(vbits >> 23), 127 + 16) - 126;
-    const bool full_up = (n + 1) % DIGIT_BLOCKS == 0;
-    e_grows = e_block > e_new || full_up;
-    e_new = max(e_new, e_block) + (full_up ? 2 : 0);
-    const float unit = two_to(DIGIT_BITS - e_new);
-#pragma unroll
-    for (int c = 0; c < G; ++c) {
-      s_scale[warp][n & 1][0][lane >> 1][c][lane & 1] = kf[c];
-      s_scale[warp][n & 1][1][lane >> 1][c][lane & 1] = vf[c] * unit;
+      const float kf = live ? (c == 0 ? __low2float(k2) : __high2float(k2)) * qscale : 0.f;
+      float vf = live ? (c == 0 ? __low2float(v2) : __high2float(v2)) : 0.f;
+      if (!(fabsf(vf) < INFINITY)) {
+        poison |= 1u << c;
+        vf = 0.f;
+      }
+      s_scale[warp][n & 1][0][lane >> 1][c][lane & 1] = kf;
+      s_scale[warp][n & 1][1][lane >> 1][c][lane & 1] = vf;
     }
   };
   if (mine > 0) place_scales(0);
@@ -727,8 +727,7 @@ __global__ void __launch_bounds__(ATTN_WARPS * 32, DigitTile<D>::MIN_CTAS) attn_
   int n = 0;
   for (; n < mine; ++n) {
     const int key0 = (b0 + n * step) * KB, st = n & 1;
-    const bool edge = key0 < k_lo || key0 + KB > k_hi, grows = e_grows;
-    const int e_now = e_new;
+    const bool edge = key0 < k_lo || key0 + KB > k_hi;
     ok = warp_all(mbar_wait(&full[st], (n >> 1) & 1, status, STATUS_TMA_WAIT, 0x20));
     if (!ok) break;
     __syncwarp();
@@ -799,50 +798,113 @@ __global__ void __launch_bounds__(ATTN_WARPS * 32, DigitTile<D>::MIN_CTAS) attn_
     for (int i = 1; i < 8; ++i) mb = fmaxf(mb, s[i >> 2][i & 3]);
     mb = fmaxf(mb, __shfl_xor_sync(0xffffffffu, mb, 1));
     mb = fmaxf(mb, __shfl_xor_sync(0xffffffffu, mb, 2));
-    if (__any_sync(0xffffffffu, mb > m_ref + DIGIT_LAG) || grows) {
-      const float m_new = mb > m_ref + DIGIT_LAG ? mb : m_ref;
-      const float corr = m_ref == -INFINITY ? 0.f : exp2f(m_ref - m_new);
-      const float f = corr * two_to(max(e_run - e_now, -126));
-      l_run *= corr;
-      if (n > 0) {
-        // two digits of a sum, 2^16 apart, as one number and back
+    // `f`: factors of the sums so far.  A reference that moves by whole powers leaves them alone,
+    // since the units make up for it.
+    float f[G];
 #pragma unroll
-        for (int i = 0; i < D / 8; ++i)
+    for (int c = 0; c < G; ++c) f[c] = 1.f;
+    bool rescale = false;
+    if (__any_sync(0xffffffffu, mb > m_ref + DIGIT_LAG)) {
+      if (mb > m_ref + DIGIT_LAG) {
+        const float m_new = ceilf(mb);
+        const bool first = m_ref == -INFINITY;
+        const int up = static_cast<int>(fminf(m_new - m_ref, 250.f));
+        l_run *= ex2_ftz(m_ref - m_new);
 #pragma unroll
-          for (int e = 0; e < 2; ++e) {
-            const float v = fmaf(static_cast<float>(acc[i][e]), 65536.f,
-                                 static_cast<float>(acc[i][2 + e])) * f;
-            const float top = rintf(v * (1.f / 65536.f));
-            acc[i][e] = __float2int_rn(top);
-            acc[i][2 + e] = __float2int_rn(fmaf(top, -65536.f, v));
-          }
+        for (int c = 0; c < G; ++c) {
+          const int was = __float_as_int(unit[c]) >> 23;
+          const int now = first ? was : min(was + up, 127 + DIGIT_UNIT_MAX);
+          // (where the unit cannot follow as far)
+          if (!first && now < was + up) f[c] = __int_as_float(max(127 + now - was - up, 0) << 23);
+          rescale = rescale || f[c] != 1.f;
+          unit[c] = __int_as_float(now << 23);
+        }
+        m_ref = m_new;
       }
-      m_ref = m_new;
-      e_run = e_now;
     }
-    uint32_t a[G][4];
+    if (n > 0 && n % DIGIT_BLOCKS == 0) {
+      rescale = true;
 #pragma unroll
-    for (int m = 0; m < 2; ++m) {
+      for (int c = 0; c < G; ++c) {
+        f[c] *= 0.25f;
+        unit[c] *= 0.25f;
+      }
+    }
+#pragma unroll
+    for (int m = 0; m < 2; ++m)
 #pragma unroll
       for (int x = 0; x < 4; ++x) {
         s[m][x] = ex2_ftz(s[m][x] - m_ref);
         l_run += s[m][x];
       }
-      float w[2][2 * G];                           // two pairs of keys
-#pragma unroll
-      for (int i = 0; i < 2; ++i)
-        load_pair<G>(w[i], s_scale[warp][st][1][8 * m + T::key_of(t, 2 * i) / 2][0]);
+    // The largest product of the block gets DIGIT_BITS bits where it has outgrown its unit.
+    auto fit = [&] {
 #pragma unroll
       for (int c = 0; c < G; ++c) {
-        uint32_t u[4];
+        float big = 0.f;
 #pragma unroll
-        for (int x = 0; x < 4; ++x)
-          u[x] = static_cast<uint32_t>(__float2int_rn(s[m][x] * w[x >> 1][2 * c + (x & 1)])) +
-                 0x80808080u;
-        const uint32_t p01 = __byte_perm(u[0], u[1], sel), p23 = __byte_perm(u[2], u[3], sel);
-        a[c][2 * m] = __byte_perm(p01, p23, 0x5410) ^ 0x80808080u;
-        a[c][2 * m + 1] = __byte_perm(p01, p23, 0x7632) ^ 0x80808080u;
+        for (int m = 0; m < 2; ++m)
+#pragma unroll
+          for (int i = 0; i < 2; ++i) {
+            float w[2 * G];
+            load_pair<G>(w, s_scale[warp][st][1][8 * m + T::key_of(t, 2 * i) / 2][0]);
+            big = fmaxf(big, fmaxf(fabsf(s[m][2 * i] * w[2 * c]),
+                                   fabsf(s[m][2 * i + 1] * w[2 * c + 1])));
+          }
+        big = fmaxf(big, __shfl_xor_sync(0xffffffffu, big, 1));
+        big = fmaxf(big, __shfl_xor_sync(0xffffffffu, big, 2));
+        if (big * unit[c] >= 1073741824.f) {       // 2^30
+          const float now = two_to(DIGIT_BITS + 126 - (__float_as_int(big) >> 23));
+          f[c] *= __int_as_float(__float_as_int(now) - __float_as_int(unit[c]) + (127 << 23));
+          unit[c] = now;
+        }
       }
+    };
+    uint32_t a[G][4];
+    auto digits = [&] {                            // true: a product has outgrown its unit
+      uint32_t over = 0u;                          // a top digit of -128: 2^31 or close to it
+#pragma unroll
+      for (int m = 0; m < 2; ++m) {
+        float w[2][2 * G];                         // two pairs of keys
+#pragma unroll
+        for (int i = 0; i < 2; ++i)
+          load_pair<G>(w[i], s_scale[warp][st][1][8 * m + T::key_of(t, 2 * i) / 2][0]);
+#pragma unroll
+        for (int c = 0; c < G; ++c) {
+          uint32_t u[4];
+#pragma unroll
+          for (int x = 0; x < 4; ++x)
+            u[x] = static_cast<uint32_t>(
+                       __float2int_rn(s[m][x] * w[x >> 1][2 * c + (x & 1)] * unit[c])) +
+                   0x80808080u;
+          const uint32_t p01 = __byte_perm(u[0], u[1], sel), p23 = __byte_perm(u[2], u[3], sel);
+          const uint32_t top = __byte_perm(p01, p23, 0x5410);
+          a[c][2 * m] = top ^ 0x80808080u;
+          a[c][2 * m + 1] = __byte_perm(p01, p23, 0x7632) ^ 0x80808080u;
+          over |= (top - 0x01010101u) & ~top;
+        }
+      }
+      return !upper && (over & 0x80808080u) != 0u; // (the lower lanes hold the top digits)
+    };
+    if (n == 0) fit();
+    if (__any_sync(0xffffffffu, digits() || rescale) && n > 0) {
+      fit();
+      // two digits of a sum, 2^16 apart, as one number and back
+#pragma unroll
+      for (int c = 0; c < G; ++c) {
+        if (f[c] == 1.f) continue;
+#pragma unroll
+        for (int i = 8 * c; i < 8 * c + 8; ++i)
+#pragma unroll
+          for (int e = 0; e < 2; ++e) {
+            const float v = fmaf(static_cast<float>(acc[i][e]), 65536.f,
+                                 static_cast<float>(acc[i][2 + e])) * f[c];
+            const float top = rintf(v * (1.f / 65536.f));
+            acc[i][e] = __float2int_rn(top);
+            acc[i][2 + e] = __float2int_rn(fmaf(top, -65536.f, v));
+          }
+      }
+      digits();
     }
     // ---- values
     uint32_t vb[2][4];
@@ -871,14 +933,20 @@ __global__ void __launch_bounds__(ATTN_WARPS * 32, DigitTile<D>::MIN_CTAS) attn_
   // ---- this warp's result, back to the unscaled weights
   l_run += __shfl_xor_sync(0xffffffffu, l_run, 1);
   l_run += __shfl_xor_sync(0xffffffffu, l_run, 2);
-  const float back = poison ? __int_as_float(0x7fc00000)
-                            : two_to(max(e_run - DIGIT_BITS, -126)) * (upper ? 1.f : 256.f);
+  poison = __reduce_or_sync(0xffffffffu, poison);
+  float back[G];
+#pragma unroll
+  for (int c = 0; c < G; ++c)
+    back[c] = poison >> c & 1 ? __int_as_float(0x7fc00000)
+                              : __int_as_float((254 << 23) - __float_as_int(unit[c])) *
+                                    (upper ? 1.f : 256.f);
 #pragma unroll
   for (int j = 0; j < D / 8; ++j) {
     float v[2];
 #pragma unroll
     for (int e = 0; e < 2; ++e) {
-      v[e] = fmaf(static_cast<float>(acc[j][e]), 65536.f, static_cast<float>(acc[j][2 + e])) * back;
+      v[e] = fmaf(static_cast<float>(acc[j][e]), 65536.f, static_cast<float>(acc[j][2 + e])) *
+             back[j / 8];
       v[e] += __shfl_xor_sync(0xffffffffu, v[e], 16);
     }
     if (upper == (j & 1))

@@ -291,25 +291,57 @@ def test_attention_rows_walk_many_pages(dev, qh, kvh, d, n, grow, splits):
     assert bool(((out.double() - ref).abs() <= lim).all())
 
 
+# value scales of one group far below those of the other, a key of huge value scale whose weight is
+# nil or not, and both against the group's own values: each keeps the bits of FP32 products
+@pytest.mark.parametrize("qh,kvh,n,splits", [(4, 1, 900, 1), (8, 2, 4129, 1), (4, 2, 3000, 3)])
+@pytest.mark.parametrize("what", ["group", "nil", "heavy"])
+@pytest.mark.parametrize("k", [6, 10, 14])
+def test_attention_rows_keep_the_bits_of_small_value_scales(dev, qh, kvh, n, splits, what, k):
+    from orinfer_b200.ops import functional as F
+    d, rep = 128, qh // kvh
+    q, req, pos, table, kc, vc, ks, vs = _walk(dev, n, qh, kvh, d, n + k)
+    assert _in_digits(qh, kvh, d, table, splits)
+    vs = (vs.float() * 2.0 ** 10).half()                  # (2^-14 of it is a normal FP16 number)
+    if what == "group":
+        vs[..., 1] = (vs[..., 1].float() * 2.0 ** -k).half()
+    else:
+        vs = (vs.float() * 2.0 ** -k).half()
+        page, slot = int(table[0, 2]), 77                 # key 333
+        vs[page, slot] = 16.0
+        if what == "nil":                                 # far below every head's maximum
+            q = q.view(kvh, rep, d)[:, :1].expand(kvh, rep, d).reshape(1, qh, d).contiguous()
+            kc[page, slot] = -(q[0, ::rep].sign() * 127).to(torch.int8)
+            ks[page, slot] = 0.5
+    out = F.attention(q, None, req, pos, table, kc, vc, ks, vs, splits=splits).view(qh, -1, 64)
+    pick = lambda c: c[table[0].long()].reshape(-1, *c.shape[2:])[:n]
+    ref = _attention64(q[0], pick(kc), pick(vc), pick(ks), pick(vs)).reshape(qh, -1, 64)
+    # one FP16 rounding, and FP32 sums of terms that may cancel: a few 2^-22 of the group's largest;
+    # outputs below the smallest normal FP16 number are rounded at 2^-25
+    lim = ref.abs() * 2.0 ** -11 + 2.0 ** -20 * ref.abs().amax(-1, keepdim=True) + 2.0 ** -25
+    assert bool(((out.double() - ref).abs() <= lim).all())
+
+
 def test_attention_rows_sums_of_a_long_context_do_not_overflow(dev):
-    """Weights, values and scales alike: integer sums grow as fast as they can, past the 65536 keys of
-    a warp after which they are scaled down."""
+    """Where a weight of 1 times the scale has 27 bits, 1.125 * 2^26 has the digits 5, -128, 0 and 0, and
+    128 x 127 a key passes 2^31 after 132 105 of a warp's 150 000 keys, were the sums not scaled down
+    on the way (with a bit less or more 1.25 and 1.0625 have them).  Weights and their sum are exact,
+    so only the output is rounded."""
     from orinfer_b200.ops import functional as F
     n, kvh, d = 600_000, 1, 64
     pages = (n + 127) // 128
     table = torch.arange(pages, dtype=torch.int32, device=dev)[None]
     assert _in_digits(4, kvh, d, table, 1)
-    for value, scale in ((127, 0.0117), (-127, 0.00781)):
+    for value, size in ((127, 1.125), (-127, 1.125), (127, 1.25), (-127, 1.0625)):
         kc = torch.zeros(pages, 128, kvh, d, dtype=torch.int8, device=dev)
         vc = torch.full_like(kc, value)
-        s = torch.full((pages, 128, kvh, 1), scale, device=dev).half()
+        s = torch.full((pages, 128, kvh, 1), size * 2.0 ** -7, device=dev).half()
         q = torch.ones(1, 4, d, device=dev).half()
         one = torch.zeros(1, dtype=torch.int32, device=dev)
         out = F.attention(q, None, one, one + n - 1, table, kc, vc, s, s, splits=1)
-        want = value * float(s[0, 0, 0, 0])
-        # one FP16 rounding, and FP32 sums of 150 000 equal weights per warp (2^-24 each at worst
-        # of the sum so far: 2^-9 in all, which both sums, of weights and of values, share)
-        assert bool(((out.double() - want).abs() <= abs(want) * 2.0 ** -8).all()), out
+        want = value * size * 2.0 ** -7
+        # one FP16 rounding, a few FP32 ones
+        lim = abs(want) * (2.0 ** -11 + 2.0 ** -20)
+        assert bool(((out.double() - want).abs() <= lim).all()), out
 
 
 @pytest.mark.parametrize("bad", [float("inf"), float("nan")])
