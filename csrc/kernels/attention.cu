@@ -439,8 +439,9 @@ __global__ void __launch_bounds__(
 // The same attention for at most four query heads per KV head, with both products on the INT8
 // tensor cores and no conversion of what the cache holds.
 //   S = Q K^T: the query, FP16, becomes a fixed-point number of 31 bits under a power of two per
-//   head, and that four signed digits to the base 256; rows 4 i + r of A are digit i (the largest
-//   first) of head r.  INT32 sums over 64 channels are exact, and the digits' sums meet in FP32.
+//   head and group of 64 channels, and that four signed digits to the base 256; rows 4 i + r of A
+//   are digit i (the largest first) of head r.  INT32 sums over a group are exact, and the digits'
+//   sums meet in FP32.
 //   O = P V: the FP32 weight x value scale becomes a fixed-point number of 32 bits, four digits,
 //   in the same rows, and the sums stay in INT32 accumulators from block to block.
 // The weights are relative to a power of two per head, which follows the row's maximum when that is
@@ -450,7 +451,7 @@ __global__ void __launch_bounds__(
 // largest product of the block, and the group's accumulators are rescaled, in place.  (Under one
 // unit for all heads, groups and keys, above the largest value scale, a group of scales 2^-k of the
 // others lost k bits, and so did all keys beside one with a large scale and no weight.)  A query
-// value is exact down to 2^-19 of its head's largest and rounded at 2^-31 of that below it.
+// value is exact down to 2^-19 of its group's largest and rounded at 2^-31 of that below it.
 // Error against 64 bits ahead of the output's FP16 rounding (2.07e-4): 8 rows of 900 keys 1.7e-7
 // (the form above 1.8e-7), 3 rows of 20000 2.1e-7 (2.6e-6), with six times the scores 3.5e-7
 // (3.6e-7) and 5.6e-7 (1.2e-6); 4 rows of 900 with one group's value scales 2^-10 of the other's
@@ -618,12 +619,13 @@ __global__ void __launch_bounds__(ATTN_WARPS * 32, DigitTile<D>::MIN_CTAS) attn_
 
   // ---- its digits: rows g and g + 8 of A are digits `upper` and 2 + `upper`
   const uint32_t sel = upper ? 0x4062u : 0x5173u;  // their bytes in two numbers
-  float f_head;                                    // the unit of the second one's sums
+  float f_head[G];                                 // the unit of the second one's sums
   uint32_t qa[KSTEPS][4];
-  {
+#pragma unroll
+  for (int c = 0; c < G; ++c) {
     __half2 big2 = __half2half2(__ushort_as_half(0));
 #pragma unroll
-    for (int s = 0; s < KSTEPS; ++s)
+    for (int s = 2 * c; s < 2 * c + 2; ++s)
 #pragma unroll
       for (int i = 0; i < 4; ++i)
         big2 = __hmax2_nan(big2, __habs2(reinterpret_cast<const __half2*>(raw[s])[i]));
@@ -635,10 +637,10 @@ __global__ void __launch_bounds__(ATTN_WARPS * 32, DigitTile<D>::MIN_CTAS) attn_
     const bool finite = big < INFINITY;
     // |q| < 2^e and the fixed-point values below 2^30
     const int e = max(-30, min(16, static_cast<int>(__float_as_uint(big) >> 23) - 126));
-    f_head = finite ? two_to(e - 30) * (upper ? 1.f : 256.f) : __int_as_float(0x7fc00000);
+    f_head[c] = finite ? two_to(e - 30) * (upper ? 1.f : 256.f) : __int_as_float(0x7fc00000);
     const float up = two_to(30 - e);
 #pragma unroll
-    for (int s = 0; s < KSTEPS; ++s) {
+    for (int s = 2 * c; s < 2 * c + 2; ++s) {
       if (!apart && (s & (ATTN_WARPS - 1)) != warp) continue;
       uint32_t(&a)[4] = qa[s];
 #pragma unroll
@@ -668,8 +670,12 @@ __global__ void __launch_bounds__(ATTN_WARPS * 32, DigitTile<D>::MIN_CTAS) attn_
   // bias leaves with the factors: (c + bias) w - bias (w + f) + (d + bias) f, exact up to the
   // rounding of a float.
   constexpr int BIAS = 0x4b400000;
-  const float w_top = f_head * 65536.f;
-  const float w_bias = -12582912.f * (w_top + f_head);
+  float w_top[G], w_bias[G];
+#pragma unroll
+  for (int c = 0; c < G; ++c) {
+    w_top[c] = f_head[c] * 65536.f;
+    w_bias[c] = -12582912.f * (w_top[c] + f_head[c]);
+  }
 
   int acc[D / 8][4];
 #pragma unroll
@@ -764,8 +770,8 @@ __global__ void __launch_bounds__(ATTN_WARPS * 32, DigitTile<D>::MIN_CTAS) attn_
         float sum = 0.f;
 #pragma unroll
         for (int c = 0; c < G; ++c) {
-          const float part = fmaf(__int_as_float(d[c][2 + e]), f_head,
-                                  fmaf(__int_as_float(d[c][e]), w_top, w_bias));
+          const float part = fmaf(__int_as_float(d[c][2 + e]), f_head[c],
+                                  fmaf(__int_as_float(d[c][e]), w_top[c], w_bias[c]));
           sum = c == 0 ? part * kv[e] : fmaf(part, kv[2 * c + e], sum);
         }
         s[i >> 1][2 * (i & 1) + e] = sum;

@@ -321,6 +321,33 @@ def test_attention_rows_keep_the_bits_of_small_value_scales(dev, qh, kvh, n, spl
     assert bool(((out.double() - ref).abs() <= lim).all())
 
 
+# a group of query values far below the other, whose keys make up for it: seen in the records of the
+# splits, which no FP16 rounding hides
+@pytest.mark.parametrize("k", [8, 16, 22])
+@pytest.mark.parametrize("group", [0, 1])
+def test_attention_rows_keep_the_bits_of_small_query_groups(dev, k, group):
+    from orinfer_b200.ops import functional as F
+    n, qh, d, splits = 700, 4, 128, 2
+    g = torch.Generator().manual_seed(k)
+    q, req, pos, table, kc, vc, ks, vs = _walk(dev, n, qh, 1, d, n + k)
+    assert _in_digits(qh, 1, d, table, splits)
+    q = torch.randn(1, qh, 2, 64, generator=g)
+    q[:, :, group] *= 2.0 ** (k // 2 - k)
+    q[:, :, 1 - group] *= 2.0 ** (k // 2)
+    q = q.view(1, qh, d).half().to(dev)
+    ks[..., group] = (ks[..., group].float() * 2.0 ** (k - k // 2)).half()
+    ks[..., 1 - group] = (ks[..., 1 - group].float() * 2.0 ** -(k // 2)).half()
+    scratch = torch.empty(qh * splits * (d + 2), device=dev)
+    F.attention(q, None, req, pos, table, kc, vc, ks, vs, splits=splits, scratch=scratch)
+    rec = scratch.view(qh, splits, d + 2).double()
+    part = torch.exp2(rec[..., 0] - rec[..., 0].amax(1, keepdim=True))[..., None]
+    out = (rec[..., 2:] * part).sum(1) / (rec[..., 1:2] * part).sum(1)
+    pick = lambda c: c[table[0].long()].reshape(-1, *c.shape[2:])[:n]
+    ref = _attention64(q[0], pick(kc), pick(vc), pick(ks), pick(vs))
+    # scores of up to 2^4 in FP32, whose error is the weights': 2^-19
+    assert float((out - ref).norm() / ref.norm()) < 2.0 ** -19
+
+
 def test_attention_rows_sums_of_a_long_context_do_not_overflow(dev):
     """Where a weight of 1 times the scale has 27 bits, 1.125 * 2^26 has the digits 5, -128, 0 and 0, and
     128 x 127 a key passes 2^31 after 132 105 of a warp's 150 000 keys, were the sums not scaled down
@@ -342,6 +369,19 @@ def test_attention_rows_sums_of_a_long_context_do_not_overflow(dev):
         # one FP16 rounding, a few FP32 ones
         lim = abs(want) * (2.0 ** -11 + 2.0 ** -20)
         assert bool(((out.double() - want).abs() <= lim).all()), out
+
+
+@pytest.mark.parametrize("bad", [float("inf"), float("nan")])
+@pytest.mark.parametrize("splits", [1, 2])
+def test_attention_rows_keep_the_other_group_of_a_bad_value_scale(dev, bad, splits):
+    from orinfer_b200.ops import functional as F
+    q, req, pos, table, kc, vc, ks, vs = _walk(dev, 700, 8, 2, 128, 5)
+    assert _in_digits(8, 2, 128, table, splits)
+    good = F.attention(q, None, req, pos, table, kc, vc, ks, vs, splits=splits).view(2, 4, 2, 64)
+    vs[int(table[0, 1]), 50, 1, 0] = bad                  # KV head 1, its lower group
+    out = F.attention(q, None, req, pos, table, kc, vc, ks, vs, splits=splits).view(2, 4, 2, 64)
+    assert bool(out[1, :, 0].isnan().all())
+    assert torch.equal(out[0], good[0]) and torch.equal(out[1, :, 1], good[1, :, 1])
 
 
 @pytest.mark.parametrize("bad", [float("inf"), float("nan")])
