@@ -454,7 +454,7 @@ __global__ void __launch_bounds__(
 // value is exact down to 2^-19 of its group's largest and rounded at 2^-31 of that below it.
 // Error against 64 bits ahead of the output's FP16 rounding (2.07e-4): 8 rows of 900 keys 1.7e-7
 // (the form above 1.8e-7), 3 rows of 20000 2.1e-7 (2.6e-6), with six times the scores 3.5e-7
-// (3.6e-7) and 5.6e-7 (1.2e-6); 4 rows of 900 with one group's value scales 2^-10 of the other's
+// (3.6e-7) and 5.2e-7 (1.2e-6); 4 rows of 900 with one group's value scales 2^-10 of the other's
 // 1.7e-7 in that group (1.8e-7, under one unit 2.4e-5), 2^-14 1.7e-7 (2.6e-7, 3.9e-4), with one key
 // of 2^10 times the scale and no weight 1.5e-7 (1.7e-7, 6.3e-6).
 //
@@ -836,13 +836,14 @@ __global__ void __launch_bounds__(ATTN_WARPS * 32, DigitTile<D>::MIN_CTAS) attn_
         unit[c] *= 0.25f;
       }
     }
+    float sums[2];                                 // a block's weights first: shorter chains of sums
 #pragma unroll
-    for (int m = 0; m < 2; ++m)
+    for (int m = 0; m < 2; ++m) {
 #pragma unroll
-      for (int x = 0; x < 4; ++x) {
-        s[m][x] = ex2_ftz(s[m][x] - m_ref);
-        l_run += s[m][x];
-      }
+      for (int x = 0; x < 4; ++x) s[m][x] = ex2_ftz(s[m][x] - m_ref);
+      sums[m] = (s[m][0] + s[m][1]) + (s[m][2] + s[m][3]);
+    }
+    l_run += sums[0] + sums[1];
     // The largest product of the block gets DIGIT_BITS bits where it has outgrown its unit.
     auto fit = [&] {
 #pragma unroll

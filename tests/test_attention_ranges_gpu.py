@@ -348,6 +348,34 @@ def test_attention_rows_keep_the_bits_of_small_query_groups(dev, k, group):
     assert float((out - ref).norm() / ref.norm()) < 2.0 ** -19
 
 
+# equal weights, which round the same way at every step of a sum
+def test_attention_rows_add_a_block_of_weights_at_a_time(dev):
+    from orinfer_b200.ops import functional as F
+    n, d, splits = 240_000, 128, 2
+    pages = (n + 127) // 128
+    table = torch.arange(pages, dtype=torch.int32, device=dev)[None]
+    kc = torch.zeros(pages, 128, 1, d, dtype=torch.int8, device=dev)
+    kc[..., 0] = 1
+    for k in range(0, n, n // splits):                    # every warp begins with weights of 1
+        kc.view(-1, d)[k:k + 128] = 0
+    vc = torch.full_like(kc, 100)
+    s = torch.ones(pages, 128, 1, 2, device=dev).half()
+    one = torch.zeros(1, dtype=torch.int32, device=dev)
+    scratch = torch.empty(4 * splits * (d + 2), device=dev)
+    assert _in_digits(4, 1, d, table, splits)
+    err = []
+    for i in range(24):                                   # weights from 0.51 to 0.99, a head each
+        q = torch.zeros(1, 4, d, device=dev)
+        q[0, :, 0] = -torch.linspace(0.01 + i / 25, 0.045 + i / 25, 4) * math.log(2) * math.sqrt(d)
+        F.attention(q.half(), None, one, one + n - 1, table, kc, vc, s, s, splits=splits, scratch=scratch)
+        rec = scratch.view(4, splits, d + 2).double()
+        err.append(float((rec[..., 2:] / rec[..., 1:2] / 100 - 1).abs().max()))
+    # a sum of as many terms as a warp has blocks of 32 keys, each step within 2^-24 of the sum so
+    # far, half of the last one on average; 2^-21 for the rest
+    blocks = n // splits // 32 // 4
+    assert max(err) <= blocks / 2 * 2.0 ** -24 + 2.0 ** -21, max(err)
+
+
 def test_attention_rows_sums_of_a_long_context_do_not_overflow(dev):
     """Where a weight of 1 times the scale has 27 bits, 1.125 * 2^26 has the digits 5, -128, 0 and 0, and
     128 x 127 a key passes 2^31 after 132 105 of a warp's 150 000 keys, were the sums not scaled down
