@@ -182,16 +182,17 @@ int orinfer_attention(const __half* q, const __half* gate, const int* row_req, c
                       __half* out, int rows, int qh, int kvh, int head_dim, int splits,
                       float* scratch, cudaStream_t stream);
 
+// Parts that the keys of a prefill tile are cut into (heads of 256 channels).
+int orinfer_attention_prefill_parts(int ctas, int max_pages);
 // Prefill chunks on tensor cores.  chunks: device int32 [n_chunks, 4] =
 // (first packed row, rows, absolute position of the first row, page-table row).
-// Parts that the keys of a tile are cut into (heads of 256 channels).
-int orinfer_attention_prefill_parts(int ctas, int max_pages);
+// context: positions that the chunks reach at most, 0 for as many as the page table has.
 // Returns -4 for a head size it does not implement (use orinfer_attention instead).
 int orinfer_attention_prefill(const __half* q, const __half* gate, const int* chunks, int n_chunks,
                               int max_q_len, int total_rows, const int* page_table, int max_pages,
                               const int8_t* kcache, const int8_t* vcache, const __half* kscale,
                               const __half* vscale, __half* out, int qh, int kvh, int head_dim,
-                              int num_pages, cudaStream_t stream);
+                              int num_pages, int context, cudaStream_t stream);
 
 // ---- expert-parallel all-to-alls over peer memory (moe_a2a.cu); cap = owned rows x top_k
 typedef struct OrinferA2aDispatch {

@@ -767,11 +767,13 @@ int launch(const __half* q, const __half* gate, const Chunk* chunks, int n_chunk
 
 using namespace orinfer;
 
-// Into how many parts the keys of a tile go, the steps counted from the page table's width (heads
-// of 256 channels, one tile per CTA).  A step takes 1.35 us, a CTA about six of them besides, and a
-// part five more to be put together with the others; a larger number has to save 15 %.  (More parts
-// than SMs did not pay: 180 CTAs of 60 steps 161 us whole, 152 in two parts, 195 in four, but 188
-// of 12 steps 45 and 72.)
+// Into how many parts the keys of a tile go (heads of 256 channels, one tile per CTA), the steps
+// counted from the longest context, or where the caller does not know it from the page table's
+// width: a serving engine's tables have the width of the longest context there may be, and 17 rows
+// without a prefix are one step.  A step takes 1.35 us, a CTA about six of them besides, and a part
+// five more to be put together with the others; a larger number has to save 15 %.  (More parts than
+// SMs did not pay: 180 CTAs of 60 steps 161 us whole, 152 in two parts, 195 in four, but 188 of 12
+// steps 45 and 72.)
 static int prefill_ranks(long long ctas, long long steps) {
   int best = 1;
   double least = 0;
@@ -791,12 +793,13 @@ extern "C" int orinfer_attention_prefill_parts(int ctas, int max_pages) {
 }
 
 // chunks: int32 [n_chunks, 4] = (row_start, q_len, pos0, page-table row) on the device.
+// context: positions that the chunks reach at most (pos0 + q_len), 0 where the caller cannot tell.
 extern "C" int orinfer_attention_prefill(const __half* q, const __half* gate, const int* chunks,
                                          int n_chunks, int max_q_len, int total_rows,
                                          const int* page_table, int max_pages, const int8_t* kc,
                                          const int8_t* vc, const __half* ks, const __half* vs,
                                          __half* out, int qh, int kvh, int head_dim, int num_pages,
-                                         cudaStream_t stream) {
+                                         int context, cudaStream_t stream) {
   if (n_chunks <= 0 || max_q_len <= 0) return 0;
   if (kvh <= 0 || qh % kvh || qh / kvh > 16) return -1;
   if (runtime_ensure_init() != cudaSuccess) return -2;
@@ -821,7 +824,8 @@ extern "C" int orinfer_attention_prefill(const __half* q, const __half* gate, co
 #undef ORINFER_PREFILL
   if (head_dim == 256) {
     const long long ctas = (longest < packed ? longest : packed) * kvh;
-    const int ranks = prefill_ranks(ctas, static_cast<long long>(max_pages) * 2);
+    const long long steps = static_cast<long long>(max_pages) * 2, known = (context + 63LL) / 64;
+    const int ranks = prefill_ranks(ctas, context > 0 && known < steps ? known : steps);
     return (ranks > 1 ? fa::launch<256, 1, true> : fa::launch<256, 1, false>)(
         q, gate, ch, n_chunks, max_q_len, total_rows, page_table, max_pages, kc, vc, ks, vs, out,
         qh, kvh, num_pages, stream, ranks);

@@ -1120,6 +1120,7 @@ class Engine:
         if chunked:
             packet.chunks = dev["chunks"].view(-1, 4)
             packet.max_q_len = max(spec["chunks"][1::4])
+            packet.max_chunk_kv = max(map(sum, zip(spec["chunks"][1::4], spec["chunks"][2::4])))
             packet.decode_rows = spec["n_decode"]
         return packet
 
@@ -1336,7 +1337,8 @@ class Engine:
         st = Packet(packet.ids.clone(), packet.row_req.clone(), packet.row_pos.clone(),
                     packet.page_table, packet.rows, packet.max_kv_len,
                     packet.logit_rows.clone(), chunks=packet.chunks.clone(),
-                    max_q_len=packet.max_q_len, decode_rows=0)
+                    max_q_len=packet.max_q_len, decode_rows=0,
+                    max_chunk_kv=self.max_context)       # replayed behind prefixes of any length
         out = self.runner.greedy(st, need_logits=need)       # this step's run, outside capture
         torch.cuda.synchronize()
         graph = torch.cuda.CUDAGraph()

@@ -138,6 +138,9 @@ class Packet:
     # Encoder passes: row r may attend to keys 0..attend_pos[r] instead of 0..row_pos[r]
     # (all rows of a bidirectional input carry the last position).  int32 [rows].
     attend_pos: Optional[torch.Tensor] = None
+    # Host-side bound on the keys that the prefill chunks reach (0: ``max_kv_len``, which also
+    # counts the decode rows); their attention launch is chosen by it.
+    max_chunk_kv: int = 0
 
     def ensure_segments(self) -> None:
         if self.segments is not None:
@@ -219,7 +222,7 @@ class ModelRunner:
             done = F.attention_prefill(ws.q, gate, p.chunks, p.max_q_len, p.page_table,
                                        self.kv.k[kv_slot], self.kv.v[kv_slot],
                                        self.kv.ks[kv_slot], self.kv.vs[kv_slot], out=ws.attn,
-                                       total_rows=rows)
+                                       total_rows=rows, max_kv_len=p.max_chunk_kv or p.max_kv_len)
             if done:
                 row_rows = p.decode_rows
         if row_rows > 0:

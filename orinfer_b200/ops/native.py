@@ -82,7 +82,7 @@ def _load() -> ctypes.CDLL:
         "orinfer_gdn_commit": ([P, I, P, P, I, P, P, P, I, I, I, P, P, P], I),
         "orinfer_gdn_gated_norm": ([P, P, I, P, c_float, I, I, I, I, P, P], I),
         "orinfer_attention_prefill_parts": ([I, I], I),
-        "orinfer_attention_prefill": ([P, P, P, I, I, I, P, I, P, P, P, P, P, I, I, I, I, P], I),
+        "orinfer_attention_prefill": ([P, P, P, I, I, I, P, I, P, P, P, P, P, I, I, I, I, I, P], I),
     }
     for name, (args, res) in sig.items():
         if hasattr(lib, name):

@@ -540,3 +540,35 @@ def test_attention_prefill_cut_over_a_cluster(dev, rows, past, qh, kvh, parts, g
             err = (out[at + r].cpu().double() - ref).norm() / ref.norm()
             assert float(err) < 2e-3, (i, r, float(err))
         at += sizes[i]
+
+
+# the page table of a serving engine is as wide as the longest context there may be: which launch a
+# packet gets, and with it the bits, depends on the context alone
+@pytest.mark.parametrize("rows,past", [(17, 0), (64, 0), (64, 330), (130, 400), (64, 1000)])
+def test_attention_prefill_of_a_packet_does_not_depend_on_the_width_of_its_table(dev, rows, past):
+    import dataclasses
+    from orinfer_b200.config import PRESETS
+    from orinfer_b200.models.runner import KVPool, ModelRunner, Packet
+    from orinfer_b200.models.weights import random_model
+    cfg = dataclasses.replace(PRESETS["tiny"], layers=1, q_heads=8, kv_heads=1, head_dim=256,
+                              gated_attention=True)
+    w = random_model(cfg, seed=0).to(dev)
+    g = torch.Generator().manual_seed(rows + past)
+    pages = (rows + past + 127) // 128
+    t = lambda v: torch.tensor(v, dtype=torch.int32, device=dev)
+    runner = ModelRunner(w, KVPool.allocate(cfg, pages + 1, dev), max_rows=rows)
+    kv = runner.kv
+    for c in (kv.k[0], kv.v[0]):
+        c.copy_(torch.randint(-127, 128, c.shape, generator=g, dtype=torch.int8))
+    for c in (kv.ks[0], kv.vs[0]):
+        c.copy_((torch.rand(c.shape, generator=g) * 0.02 + 1e-3).half())
+    ids = torch.randint(0, cfg.vocab, (rows,), generator=g).int().to(dev)
+    out = []
+    for width in (pages, 256):
+        table = torch.zeros(1, width, dtype=torch.int32, device=dev)
+        table[0, :pages] = torch.arange(1, pages + 1)
+        p = Packet(ids, t([0] * rows), t(list(range(past, past + rows))), table, rows, past + rows,
+                   chunks=t([[0, rows, past, 0]]), max_q_len=rows)
+        out.append(runner.greedy(p, need_logits=True)[1].clone())
+        out.append(runner.ws.attn[:rows].clone())
+    assert torch.equal(out[1], out[3]) and torch.equal(out[0], out[2])
