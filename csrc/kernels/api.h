@@ -176,11 +176,12 @@ int orinfer_qgemm_grouped_launches(int fmt, int S, int experts, int max_tiles, i
 size_t orinfer_attention_scratch_bytes(int rows, int qh, int head_dim, int splits);
 int orinfer_attention_starts_early(int rows, int kvh, int head_dim, int splits);
 int orinfer_attention_in_digits(int qh, int kvh, int head_dim, int max_pages, int splits);
+// context: keys that any row sees at most, 0 for as many as the page table has.
 int orinfer_attention(const __half* q, const __half* gate, const int* row_req, const int* row_pos,
                       const int* page_table, int max_pages, const int8_t* kcache,
                       const int8_t* vcache, const __half* kscale, const __half* vscale,
                       __half* out, int rows, int qh, int kvh, int head_dim, int splits,
-                      float* scratch, cudaStream_t stream);
+                      float* scratch, int context, cudaStream_t stream);
 
 // Parts that the keys of a prefill tile are cut into (heads of 256 channels).
 int orinfer_attention_prefill_parts(int ctas, int max_pages);

@@ -1021,13 +1021,21 @@ inline bool attn_starts_early(int head_dim, long long ctas) {
 
 // Up to four query heads per KV head fill the sixteen rows of digits; five and more would take a
 // second tile and twice the accumulators, and channels above 128 have no room for theirs.  A CTA
-// should have ten blocks or more, as far as the page table's width tells: the digits of a query and
-// the sums' way back cost what a few blocks save (8 rows of 300 keys 7.0 us both ways, 1 row of 100
-// 3.6 and 3.8, of 2000 in 32 splits 8.3 and 8.2; 64 rows of 300 17.6 and 15.5).
+// should have ten blocks or more, counted from the longest context, or where the caller does not
+// know it from the page table's width (a serving engine's tables have the width of the longest
+// context there may be): the digits of a query, the units of a first block and the sums' way back
+// cost what a few blocks save.  The form above and this one, 32 / 8 heads of 128: 1 row of 60 keys
+// 3.5 and 3.7 us, of 900 (68 a CTA) 5.9 and 6.3, 8 rows of 300 (76) 6.8 and 7.0, of 900 (170) 12.0
+// and 11.2, of 3000 (512) 19.5 and 17.5, 32 rows of 300 10.9 and 10.0, of 3000 48.7 and 37.1.  16 /
+// 8 heads of 64: 16 rows of 60 2.9 and 3.2, of 900 (341) 10.0 and 10.2, of 3000 (1024) 17.5 and
+// 15.4, 128 rows of 450 21.5 and 19.1.  So the line is a compromise: from 150 to 320 keys this form
+// saves 5 % at 128 channels and costs 2 at 64.  Above it one kind of call is slower, a little more
+// than a wave of CTAs with contexts of one length: 32 rows of 900, 32 / 16 heads of 128, 33.5 and
+// 36.2 (ragged ones 30.5 and 27.0).
 constexpr int DIGIT_MIN_KEYS = 320;
-inline bool attn_digits(int head_dim, int rep, int max_pages, int splits, bool wide, const void* kc,
+inline bool attn_digits(int head_dim, int rep, int pages, int splits, bool wide, const void* kc,
                         const void* vc) {
-  const long long keys = static_cast<long long>(max_pages) * 128 / splits;
+  const long long keys = static_cast<long long>(pages) * 128 / splits;
   return head_dim <= 128 && rep <= 4 && wide && keys >= DIGIT_MIN_KEYS &&
          ((reinterpret_cast<uintptr_t>(kc) | reinterpret_cast<uintptr_t>(vc)) & 15) == 0;
 }
@@ -1053,7 +1061,7 @@ template <int D>
 static int launch_attn(const __half* q, const __half* gate, const int* row_req, const int* row_pos,
                        const int* page_table, int max_pages, const int8_t* kc, const int8_t* vc,
                        const __half* ks, const __half* vs, __half* out, int rows, int qh, int kvh,
-                       int rep, int splits, float* scratch, cudaStream_t stream) {
+                       int rep, int splits, float* scratch, int context, cudaStream_t stream) {
   dim3 grid(rows, kvh, splits);
   const bool wide = ((reinterpret_cast<uintptr_t>(q) & 15) | (reinterpret_cast<uintptr_t>(ks) & 7) |
                      (reinterpret_cast<uintptr_t>(vs) & 7)) == 0;
@@ -1070,7 +1078,9 @@ static int launch_attn(const __half* q, const __half* gate, const int* row_req, 
       kernel<<<grid, ATTN_WARPS * 32, smem, stream>>>(args...);
   };
   CUtensorMap tk, tv;
-  if (attn_digits(D, rep, max_pages, splits, wide, kc, vc) && kv_map<D>(&tk, kc, kvh) &&
+  const int known = (context + 127) / 128;
+  const int pages = context > 0 && known < max_pages ? known : max_pages;
+  if (attn_digits(D, rep, pages, splits, wide, kc, vc) && kv_map<D>(&tk, kc, kvh) &&
       kv_map<D>(&tv, vc, kvh)) {
     constexpr int D_ = D == 256 ? 128 : D;         // (256 channels: never)
     auto kernel = apart ? attn_digits_kernel<D_, true> : attn_digits_kernel<D_, false>;
@@ -1121,14 +1131,15 @@ extern "C" int orinfer_attention(const __half* q, const __half* gate, const int*
                                  const int* row_pos, const int* page_table, int max_pages,
                                  const int8_t* kc, const int8_t* vc, const __half* ks,
                                  const __half* vs, __half* out, int rows, int qh, int kvh,
-                                 int head_dim, int splits, float* scratch, cudaStream_t stream) {
+                                 int head_dim, int splits, float* scratch, int context,
+                                 cudaStream_t stream) {
   if (rows <= 0) return 0;
   if (splits < 1 || (splits > 1 && scratch == nullptr) || kvh <= 0 || qh % kvh) return -1;
   const int rep = qh / kvh;
 #define CASE(DD)                                                                            \
   if (head_dim == DD)                                                                       \
     return launch_attn<DD>(q, gate, row_req, row_pos, page_table, max_pages, kc, vc, ks, vs, \
-                           out, rows, qh, kvh, rep, splits, scratch, stream);
+                           out, rows, qh, kvh, rep, splits, scratch, context, stream);
   // query heads per KV head: the eight rows of a score tile (five only at D = 128)
   if (rep != 1 && rep != 2 && rep != 4 && rep != 8 && !(rep == 5 && head_dim == 128)) return -1;
   CASE(64) CASE(128) CASE(256)

@@ -232,7 +232,8 @@ class ModelRunner:
             see = p.row_pos if p.attend_pos is None else p.attend_pos
             F.attention(ws.q, gate, p.row_req, see, p.page_table, self.kv.k[kv_slot],
                         self.kv.v[kv_slot], self.kv.ks[kv_slot], self.kv.vs[kv_slot],
-                        splits=splits, scratch=scratch, out=ws.attn, rows=row_rows)
+                        splits=splits, scratch=scratch, out=ws.attn, rows=row_rows,
+                        max_kv_len=p.max_kv_len)
 
     def _fused_layer(self, lw: LayerWeights, kv_slot: int, p: Packet, rows: int) -> bool:
         """One dense decoder layer of a decode-sized packet with the row kernels fused into

@@ -183,7 +183,10 @@ def attention(q: torch.Tensor, gate: Optional[torch.Tensor], row_req: torch.Tens
               row_pos: torch.Tensor, page_table: torch.Tensor, kcache: torch.Tensor,
               vcache: torch.Tensor, kscale: torch.Tensor, vscale: torch.Tensor, *, splits: int = 1,
               scratch: Optional[torch.Tensor] = None, out: Optional[torch.Tensor] = None,
-              rows: Optional[int] = None) -> torch.Tensor:
+              rows: Optional[int] = None, max_kv_len: Optional[int] = None) -> torch.Tensor:
+    """Attention of single rows over the paged cache, row r against keys 0..row_pos[r].
+    ``max_kv_len``: keys that any row sees at most, where the host knows it (one of two kernels is
+    chosen by it; without it, by the width of the page table)."""
     _cuda(q, row_req, page_table, kcache)
     n, qh, d = q.shape
     kvh = kcache.shape[2]
@@ -195,7 +198,7 @@ def attention(q: torch.Tensor, gate: Optional[torch.Tensor], row_req: torch.Tens
     check(native.lib().orinfer_attention(
         ptr(q), ptr(gate), ptr(row_req), ptr(row_pos), ptr(page_table), page_table.shape[1],
         ptr(kcache), ptr(vcache), ptr(kscale), ptr(vscale), ptr(out), n if rows is None else rows,
-        qh, kvh, d, splits, ptr(scratch), stream()), "attention")
+        qh, kvh, d, splits, ptr(scratch), max_kv_len or 0, stream()), "attention")
     count_launches(2 if splits > 1 else 1)
     return out
 

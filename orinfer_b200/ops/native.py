@@ -54,7 +54,7 @@ def _load() -> ctypes.CDLL:
         "orinfer_argmax": ([P, I, I, P, P, P, P], I),
         "orinfer_qgemm": ([I, P, P, P, P, P, I, I, I, I, I, P], I),
         "orinfer_attention_scratch_bytes": ([I, I, I, I], c_size_t),
-        "orinfer_attention": ([P, P, P, P, P, I, P, P, P, P, P, I, I, I, I, I, P, P], I),
+        "orinfer_attention": ([P, P, P, P, P, I, P, P, P, P, P, I, I, I, I, I, P, I, P], I),
         "orinfer_e8p_encode": ([P, P, c_longlong, P], I),
         "orinfer_router_topk": ([P, P, I, I, I, I, I, I, P, P, P, P], I),
         "orinfer_attention_starts_early": ([I, I, I, I], I),

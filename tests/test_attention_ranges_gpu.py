@@ -546,12 +546,26 @@ def test_attention_prefill_cut_over_a_cluster(dev, rows, past, qh, kvh, parts, g
 # packet gets, and with it the bits, depends on the context alone
 @pytest.mark.parametrize("rows,past", [(17, 0), (64, 0), (64, 330), (130, 400), (64, 1000)])
 def test_attention_prefill_of_a_packet_does_not_depend_on_the_width_of_its_table(dev, rows, past):
+    cfg = dict(q_heads=8, kv_heads=1, head_dim=256, gated_attention=True)
+    out = _packet_of_one_layer(dev, cfg, rows, past, prefill=True)
+    assert torch.equal(out[1], out[3]) and torch.equal(out[0], out[2])
+
+
+@pytest.mark.parametrize("rows,past", [(1, 100), (1, 900), (6, 1500), (3, 4000)])
+def test_attention_of_a_decode_packet_does_not_depend_on_the_width_of_its_table(dev, rows, past):
+    cfg = dict(q_heads=8, kv_heads=2, head_dim=128)
+    out = _packet_of_one_layer(dev, cfg, rows, past, prefill=False)
+    assert torch.equal(out[1], out[3]) and torch.equal(out[0], out[2])
+
+
+def _packet_of_one_layer(dev, geometry, rows, past, prefill):
+    """Logits and attention outputs of a packet of one request, a prefill chunk or verification rows,
+    with a page table that fits and one of 256 pages."""
     import dataclasses
     from orinfer_b200.config import PRESETS
     from orinfer_b200.models.runner import KVPool, ModelRunner, Packet
     from orinfer_b200.models.weights import random_model
-    cfg = dataclasses.replace(PRESETS["tiny"], layers=1, q_heads=8, kv_heads=1, head_dim=256,
-                              gated_attention=True)
+    cfg = dataclasses.replace(PRESETS["tiny"], layers=1, **geometry)
     w = random_model(cfg, seed=0).to(dev)
     g = torch.Generator().manual_seed(rows + past)
     pages = (rows + past + 127) // 128
@@ -568,7 +582,7 @@ def test_attention_prefill_of_a_packet_does_not_depend_on_the_width_of_its_table
         table = torch.zeros(1, width, dtype=torch.int32, device=dev)
         table[0, :pages] = torch.arange(1, pages + 1)
         p = Packet(ids, t([0] * rows), t(list(range(past, past + rows))), table, rows, past + rows,
-                   chunks=t([[0, rows, past, 0]]), max_q_len=rows)
+                   chunks=t([[0, rows, past, 0]]) if prefill else None, max_q_len=rows)
         out.append(runner.greedy(p, need_logits=True)[1].clone())
         out.append(runner.ws.attn[:rows].clone())
-    assert torch.equal(out[1], out[3]) and torch.equal(out[0], out[2])
+    return out
