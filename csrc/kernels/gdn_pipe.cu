@@ -82,6 +82,13 @@ __device__ __forceinline__ void split_half2(float2 x, uint32_t& hi, uint32_t& lo
 __device__ __forceinline__ void split_half3(float2 x, uint32_t& hi, uint32_t& mid, uint32_t& lo) {
   split_half2(split_head(x, hi), mid, lo);
 }
+// The same with the remainder 2^11 times as large, so that its smallest step is 2^-35, not 2^-24
+constexpr float REST_UP = 2048.f;
+__device__ __forceinline__ void split_state(float2 x, uint32_t& hi, uint32_t& lo) {
+  const float2 rest = mul2(split_head(x, hi), make_float2(REST_UP, REST_UP));
+  const __half2 l = __floats2half2_rn(rest.x, rest.y);
+  lo = *reinterpret_cast<const uint32_t*>(&l);
+}
 // d += a, two by two
 __device__ __forceinline__ void add4(float (&d)[4], const float (&a)[4]) {
   const float2 x = add2(make_float2(d[0], d[1]), make_float2(a[0], a[1]));
@@ -151,7 +158,9 @@ __device__ __forceinline__ void mul_lower(float (&d)[N][2][4], const float (*m)[
   }
 }
 
-// D (32 x 8) = X S for N such D and slices of S: X a chunk's rows of k or q, S as `s` holds it
+// D (32 x 8) = X S for N such D and slices of S: X a chunk's rows of k or q, S as `s` holds it. The
+// remainders' sums are scaled back before those of the heads (under 1 % of a run; sums of their own
+// took 4 %, heads and remainders made behind the true maximum 2 %).
 template <int N, int UNROLL>
 __device__ __forceinline__ void mul_state(float (&d)[N][2][4], const __half (*x)[136],
                                           const __half (*s)[2][128][8], int lane) {
@@ -177,7 +186,7 @@ __device__ __forceinline__ void mul_state(float (&d)[N][2][4], const __half (*x)
     for (int n = 0; n < N; ++n) ldsm_x4_t(f[n][1], &s[n][0][32 * u + lane][0]);
     float part[N][2][4] = {};
 #pragma unroll
-    for (int w = 0; w < 2; ++w)
+    for (int w = 0; w < 2; ++w) {
 #pragma unroll
       for (int k = 0; k < 2; ++k)
 #pragma unroll
@@ -185,7 +194,14 @@ __device__ __forceinline__ void mul_state(float (&d)[N][2][4], const __half (*x)
 #pragma unroll
           for (int m = 0; m < 2; ++m)              // the sums take turns
             mma_f16(part[n][m], a[m][k][0], a[m][k][1], a[m][k][2], a[m][k][3], f[n][w][2 * k],
-                     f[n][w][2 * k + 1]);
+                    f[n][w][2 * k + 1]);
+      if (w == 0) {
+#pragma unroll
+        for (int n = 0; n < N; ++n)
+#pragma unroll
+          for (int e = 0; e < 8; ++e) part[n][e >> 2][e & 3] *= 1.f / REST_UP;
+      }
+    }
 #pragma unroll
     for (int n = 0; n < N; ++n)
 #pragma unroll
@@ -298,7 +314,7 @@ __global__ void __launch_bounds__(THREADS, 1) gdn_pipe_kernel(
 #pragma unroll
       for (int h = 0; h < 2; ++h) {
         uint32_t hi, lo;
-        split_half2(mul2(make_float2(s_acc[i][2 * h], s_acc[i][2 * h + 1]), up), hi, lo);
+        split_state(mul2(make_float2(s_acc[i][2 * h], s_acc[i][2 * h + 1]), up), hi, lo);
         *reinterpret_cast<uint32_t*>(&sm.s[next][warp][0][16 * i + 8 * h + g][2 * t]) = hi;
         *reinterpret_cast<uint32_t*>(&sm.s[next][warp][1][16 * i + 8 * h + g][2 * t]) = lo;
       }
@@ -379,8 +395,9 @@ __global__ void __launch_bounds__(THREADS, 1) gdn_pipe_kernel(
                       lo[r][h]);
       const float2 total2 = make_float2(sm.total[ring], sm.total[ring]);
       // The next S is split as it is made, under a bound of it: e^G S and the sum of the |Delta|
-      // times the largest |k|.  Half a dozen bits more than it needs cost nothing: heads and
-      // remainders have 2^38 steps below the bound and use 2^22 of them.
+      // times the largest |k|, which can be half a dozen bits above its largest element.  Heads and
+      // remainders have 2^49 steps below the bound, so an element keeps 22 bits down to 2^-27 of it
+      // (gdn_chunk_kernel, whose remainders are not scaled up, down to 2^-16 of the largest).
       d_sum += __shfl_xor_sync(0xffffffffu, d_sum, 1);
       d_sum += __shfl_xor_sync(0xffffffffu, d_sum, 2);
       all_rows();

@@ -322,6 +322,41 @@ def test_gdn_many_runs_contain_non_finite_rows(dev, row):
     assert float((out - fine)[~bad].norm() / fine[~bad].norm()) < 1e-6
 
 
+# small elements of a state beside large ones that a chunk's rows overwrite with changing signs, so
+# that a bound of the state stands far above it: rows of queries that read the small ones alone
+@pytest.mark.parametrize("n", [64, 200])
+@pytest.mark.parametrize("small", [2.0 ** -8, 2.0 ** -16])
+def test_gdn_small_elements_of_a_state_keep_their_bits(dev, n, small):
+    from orinfer_b200.ops import functional as F
+    from orinfer_b200.ops import native
+    hv, d = 2, 128
+    assert native.lib().orinfer_gdn_pipelined(hv, 1, n)
+    g = torch.Generator().manual_seed(n)
+    q, k, v = torch.zeros(n, 1, d), torch.zeros(n, 1, d), torch.ones(n, hv, d)
+    q[..., 2:] = torch.nn.functional.normalize(torch.randn(n, 1, d - 2, generator=g), dim=-1)
+    k[..., 1] = 1
+    v[1::2] = -1
+    qkv = torch.cat([q.reshape(n, -1), k.reshape(n, -1), v.reshape(n, -1)], 1).half().to(dev)
+    state = torch.randn(1, hv, d, d, generator=g) * small
+    state[:, :, :2] = 1
+    state = state.to(dev)
+    s0 = state[0].double()
+    ab = torch.randn(n, 2 * hv, generator=g).to(dev)
+    ab[:, hv:] = 3.0
+    a_log, dt = torch.full((hv,), -5.0, device=dev), torch.zeros(hv, device=dev)
+    t = lambda x: torch.tensor(x, dtype=torch.int32, device=dev)
+    out = F.gdn_scan(qkv, ab, a_log, dt, t([[0, n, 0, 0]]), 1, t([0] * n),
+                     t(list(range(9, 9 + n))), 1, hv, d, state)
+    part = lambda i: qkv[:, i * d:(i + 1) * d].double().reshape(n, 1, d).repeat_interleave(hv, 1)
+    decay = -torch.exp(a_log.double()) * torch.nn.functional.softplus(ab[:, :hv].double())
+    ref, s = _recurrence64(part(0) / math.sqrt(d), part(1),
+                           qkv[:, 2 * d:].double().reshape(n, hv, d), decay,
+                           torch.sigmoid(ab[:, hv:].double()), s0)
+    # as in test_gdn_chunks_keep_fp32_accuracy, over a whole run
+    assert float((out.double() - ref).norm() / ref.norm()) < 2.0 ** -20
+    assert float((state[0].double() - s).norm() / s.norm()) < 2.0 ** -20
+
+
 def test_gdn_keys_of_any_size(dev):
     """The state is scaled by a bound that takes the keys' size into account."""
     from orinfer_b200.ops import functional as F
