@@ -89,6 +89,9 @@ int orinfer_qgemm_ag(int fmt, const int8_t* a, const float* a_scale, const void*
 // may then read the activation buffer with ordinary loads.
 int orinfer_ag_wait(const OrinferAgIn* ag, int rows, cudaStream_t stream);
 
+// Both forms of the kernels' sigmoid (n even), for checks of their accuracy.
+int orinfer_sigmoids(const float* x, float* single, float* pair, long long n, cudaStream_t stream);
+
 int orinfer_act_prep_limited(const __half* x, const int8_t* signs, int8_t* q_out,
                              float* scale_out, int rows, int K, int swiglu, const int* row_limit,
                              cudaStream_t stream);

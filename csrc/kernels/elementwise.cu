@@ -591,6 +591,15 @@ static bool launch_swiglu_rows(const __half* x, const int8_t* signs, int8_t* q_o
   return true;
 }
 
+__global__ void sigmoids_kernel(const float* x, float* single, float* pair, long long pairs) {
+  const long long i = static_cast<long long>(blockIdx.x) * 256 + threadIdx.x;
+  if (i >= pairs) return;
+  const float2 v = reinterpret_cast<const float2*>(x)[i];
+  reinterpret_cast<float2*>(pair)[i] = sigmoid_pair(v);
+  single[2 * i] = sigmoid_f32(v.x);
+  single[2 * i + 1] = sigmoid_f32(v.y);
+}
+
 __global__ void ag_wait_kernel(AgIn in, int rows, int* status) {
   if (threadIdx.x == 0 && blockIdx.x == 0) ag_wait(in, 0, rows - 1, status);
 }
@@ -986,6 +995,16 @@ int orinfer_qk_rope_kv(const __half* qkv, const __half* wq, const __half* wk, co
   else if (head_dim == 256 && gated) LAUNCH(256, true);
   else return -1;
 #undef LAUNCH
+  return static_cast<int>(cudaGetLastError());
+}
+
+// The kernels' two sigmoids of n values (n even), as they are: their accuracy is checked on these.
+int orinfer_sigmoids(const float* x, float* single, float* pair, long long n,
+                     cudaStream_t stream) {
+  if (n <= 0) return 0;
+  if (n % 2 || (reinterpret_cast<uintptr_t>(x) | reinterpret_cast<uintptr_t>(pair)) % 8) return -1;
+  sigmoids_kernel<<<static_cast<unsigned>((n / 2 + 255) / 256), 256, 0, stream>>>(x, single, pair,
+                                                                                 n / 2);
   return static_cast<int>(cudaGetLastError());
 }
 

@@ -75,6 +75,7 @@ def _load() -> ctypes.CDLL:
         "orinfer_router_form": ([I, I, I, I], I),
         "orinfer_qgemm_plan": ([I, I, I, I, I, P], None),
         "orinfer_act_prep_limited": ([P, P, P, P, I, I, I, P, P], I),
+        "orinfer_sigmoids": ([P, P, P, c_longlong, P], I),
         "orinfer_small_proj": ([P, P, P, I, I, I, P], I),
         "orinfer_gdn_conv": ([P, I, P, P, P, P, P, P, I, I, I, I, I, P, P, I], I),
         "orinfer_gdn_pipelined": ([I, I, I], I),

@@ -419,3 +419,43 @@ def test_gdn_gates_and_values_at_the_ends_of_their_range(dev):
             want = torch.where(proj == -math.inf, math.nan, want)
         same = (got == want) | (got.isnan() & want.isnan()) | ((got - want).abs() <= want.abs() * 2.0 ** -10)
         assert bool(same.all()), (proj[~same][:4], got[~same][:4], want[~same][:4])
+
+
+def test_both_sigmoids_keep_their_accuracy(dev):
+    """Every 61st float between 2^-30 and 87 of both signs, against 64 bits."""
+    from orinfer_b200.ops import native
+    bits = torch.arange(0x30800000, 0x42AE0000, 61, dtype=torch.int32, device=dev)
+    x = bits.view(torch.float32)
+    x = torch.cat([x, -x, torch.tensor([0.0, -0.0], device=dev)])
+    one, pair = torch.empty_like(x), torch.empty_like(x)
+    run = lambda n: native.check(native.lib().orinfer_sigmoids(
+        x.data_ptr(), one.data_ptr(), pair.data_ptr(), n, torch.cuda.current_stream().cuda_stream), "")
+    run(x.numel())
+    want = torch.sigmoid(x.double())
+    rel = lambda got: float(((got.double() - want) / want).abs().max())
+    # half a step of the result, one and a half of the exponential and its argument's rounding
+    assert rel(pair) < 2.0 ** -22.3 and rel(one) < 2.0 ** -22.1, (rel(pair), rel(one))
+    x[:8] = torch.tensor([-87.5, -88.5, -90.0, -110.0, -1e30, -math.inf, math.inf, math.nan], device=dev)
+    run(8)
+    for got in (one, pair):
+        assert bool((got[:6].abs() <= 2.0 ** -125).all()) and float(got[6]) == 1 and got[7].isnan()
+
+
+# how often an FP16 value of the convolution is not the correctly rounded one
+def test_gdn_conv_values_are_rounded_as_the_sigmoid_allows(dev):
+    from orinfer_b200.ops import functional as F
+    g = torch.Generator(device=dev).manual_seed(7)
+    rows, hk, hv, d = 2000, 1, 30, 128
+    conv = (2 * hk + hv) * d
+    x = torch.randn(rows, conv, generator=g, device=dev).half()
+    w = (torch.randn(conv, 4, generator=g, device=dev) * 0.3).half()
+    t = lambda v: torch.tensor(v, dtype=torch.int32, device=dev)
+    y = F.gdn_conv(x, w, torch.zeros(1, 3, conv, device=dev).half(), t([0] * rows), t([0] * rows),
+                   t(list(range(rows))), t([[0, rows, 0, 0]]), 1, rows, hk, hv, d)
+    full = torch.cat([torch.zeros(3, conv, device=dev), x]).double()
+    acc = sum(full[j:j + rows] * w[:, j].double() for j in range(4))
+    want = (acc * torch.sigmoid(acc)).half()
+    off = (y != want)[:, 2 * hk * d:].double().mean()
+    # a value is off if it lies nearer to a tie than its error: steps of 2^-10 to 2^-11 of the value
+    # and errors of 2^-23 to 2^-22 (four products, the sigmoid, a product)
+    assert 0 < float(off) < 2.0 ** -12
