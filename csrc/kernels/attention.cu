@@ -836,7 +836,7 @@ __global__ void __launch_bounds__(ATTN_WARPS * 32, DigitTile<D>::MIN_CTAS) attn_
         unit[c] *= 0.25f;
       }
     }
-    float sums[2];                                 // a block's weights first: shorter chains of sums
+    float sums[2];                                 // a block's weights first: short chains of sums
 #pragma unroll
     for (int m = 0; m < 2; ++m) {
 #pragma unroll
@@ -1021,17 +1021,17 @@ inline bool attn_starts_early(int head_dim, long long ctas) {
 
 // Up to four query heads per KV head fill the sixteen rows of digits; five and more would take a
 // second tile and twice the accumulators, and channels above 128 have no room for theirs.  A CTA
-// should have ten blocks or more, counted from the longest context, or where the caller does not
-// know it from the page table's width (a serving engine's tables have the width of the longest
-// context there may be): the digits of a query, the units of a first block and the sums' way back
-// cost what a few blocks save.  The form above and this one, 32 / 8 heads of 128: 1 row of 60 keys
-// 3.5 and 3.7 us, of 900 (68 a CTA) 5.9 and 6.3, 8 rows of 300 (76) 6.8 and 7.0, of 900 (170) 12.0
-// and 11.2, of 3000 (512) 19.5 and 17.5, 32 rows of 300 10.9 and 10.0, of 3000 48.7 and 37.1.  16 /
-// 8 heads of 64: 16 rows of 60 2.9 and 3.2, of 900 (341) 10.0 and 10.2, of 3000 (1024) 17.5 and
-// 15.4, 128 rows of 450 21.5 and 19.1.  So the line is a compromise: from 150 to 320 keys this form
-// saves 5 % at 128 channels and costs 2 at 64.  Above it one kind of call is slower, a little more
-// than a wave of CTAs with contexts of one length: 32 rows of 900, 32 / 16 heads of 128, 33.5 and
-// 36.2 (ragged ones 30.5 and 27.0).
+// should have ten blocks or more, counted from the pages of the longest context and one more for
+// the keys to come, or where the caller does not know it from the page table's width (a serving
+// engine's tables have the width of the longest context there may be): the digits of a query, the
+// units of a first block and the sums' way back cost what a few blocks save.  The form above and
+// this one, 32 / 8 heads of 128: 1 row of 60 keys 3.5 and 3.7 us, of 900 (68 a CTA) 5.9 and 6.3, 8
+// rows of 300 (76) 6.8 and 7.0, of 900 (170) 12.0 and 11.2, of 3000 (512) 19.5 and 17.5, 32 rows of
+// 300 10.9 and 10.0, of 3000 48.7 and 37.1.  16 / 8 heads of 64: 16 rows of 60 2.9 and 3.2, of 900
+// (341) 10.0 and 10.2, of 3000 (1024) 17.5 and 15.4, 128 rows of 450 21.5 and 19.1.  So the line is
+// a compromise: from 150 to 320 keys this form saves 5 % at 128 channels and costs 2 at 64.  Above
+// it one kind of call is slower, a little more than a wave of CTAs with contexts of one length: 32
+// rows of 900, 32 / 16 heads of 128, 33.5 and 36.2 (ragged ones 30.5 and 27.0).
 constexpr int DIGIT_MIN_KEYS = 320;
 inline bool attn_digits(int head_dim, int rep, int pages, int splits, bool wide, const void* kc,
                         const void* vc) {
@@ -1078,8 +1078,7 @@ static int launch_attn(const __half* q, const __half* gate, const int* row_req, 
       kernel<<<grid, ATTN_WARPS * 32, smem, stream>>>(args...);
   };
   CUtensorMap tk, tv;
-  const int known = (context + 127) / 128;
-  const int pages = context > 0 && known < max_pages ? known : max_pages;
+  const int pages = context > 0 ? (context + 127) / 128 + 1 : max_pages;
   if (attn_digits(D, rep, pages, splits, wide, kc, vc) && kv_map<D>(&tk, kc, kvh) &&
       kv_map<D>(&tv, vc, kvh)) {
     constexpr int D_ = D == 256 ? 128 : D;         // (256 channels: never)
