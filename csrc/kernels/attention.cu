@@ -462,15 +462,18 @@ __global__ void __launch_bounds__(
 // fragments are transposed by the load (m16n16 b8).  A lane owns eight keys of a block in both
 // products; which ones is chosen so that neither side's loads meet on a bank.
 //
-// A block of 32 keys is 400 instructions of a warp where the form above takes about 900.  32 / 8
-// heads of 128: 6 rows of 12000..24000 keys 62.7 -> 49.8 us (235 MB; the blocks alone run at the
-// memory's rate), 38 rows of 1500..3000 57.5 -> 39.3, 128 rows of 320..640 38.7 -> 33.9.  (A unit
-// that gives the largest product one bit more is outgrown so often that the last takes 34.4.)  It
-// is 2.3 waves of CTAs, each of which waits 4000 cycles for its row, pages and first block and
-// takes 3000 to finish besides the 12000 of its blocks.  Tried: blocks of 64 keys with one buffer
-// (the same), the heads of a row side by side in the grid (the same, long rows 4 % slower), a warp
-// per row of up to 512 keys (the same with 128 rows, 64 rows 28.4 against 21.8), scales by loads
-// into registers (the loop's move waits for them: the same, long rows 2 % quicker).
+// A block of 32 keys is 520 instructions of a warp where the form above takes 1060 (counted between
+// 4096 and 8192 keys), and a warp of a CTA has 930 besides.  32 / 8 heads of 128: 6 rows of
+// 12000..24000 keys 62.7 -> 49.8 us (235 MB; the blocks alone run at the memory's rate), 38 rows of
+// 1500..3000 57.5 -> 39.4, 128 rows of 320..640 38.7 -> 33.9.  (A unit that gives the largest
+// product one bit more is outgrown so often that the last takes 34.4.)  It is 2.3 waves of CTAs,
+// each of which waits 4000 cycles for its row, pages and first block and takes 3000 to finish
+// besides the 12000 of its blocks: 39 % of the issue slots, a warp waits 1.7 cycles an instruction
+// for the one before it, 1.4 for shared memory, exchanges and conversions, 1.1 for loads.  Tried:
+// blocks of 64 keys with one buffer (the same), the heads of a row side by side in the grid (the
+// same, long rows 4 % slower), a warp per row of up to 512 keys (the same with 128 rows, 64 rows
+// 28.4 against 21.8), scales by loads into registers (the loop's move waits for them: the same,
+// long rows 2 % quicker), two products to an instruction (128 rows 5 % slower).
 template <int D>
 struct DigitTile {
   static constexpr int G = D / 64, KB = 32, KSTEPS = D / 32;

@@ -36,9 +36,11 @@
 // 777 and 646 rows behind 3000 positions, 16 / 2 gated heads of 256: 354 -> 276 -> 244 with K and
 // V freed apart, 223 with plain loads, 161 with the gates asked for ahead (one at a time, two
 // bytes of a row per lane, a tile's epilogue took 30 us; 17 rows 41 -> 10 us).
-// Where the tiles are fewer than half the SMs, the CTAs of a cluster cut the keys of each (SPLIT,
-// heads of 256 channels): 64 rows behind 1000 positions 32 -> 18.5 us, 500 behind 1000 44 -> 32.5,
-// 64 behind 20000 450 -> 72.
+// Where the tiles are fewer than half the SMs, the CTAs of a cluster cut the keys of each (SPLIT):
+// 64 rows behind 1000 positions 32 -> 18.5 us, 500 behind 1000 44 -> 32.5, 64 behind 20000 450 ->
+// 72.  Heads of 64 and 128 channels are left whole: a step serves twice as many keys, so that a
+// walk is half as long, and their FP16 outputs would move by a step here and there, which the INT8
+// rows of the next projection make a code step (what the split would save there was not measured).
 // Output is O / sum, optionally times sigmoid(gate), in FP16.  Replaces the prefill
 // configurations of causal_attention_int8 and dequantize_attention_kv
 // (kernels/cuda/model/attention_rows.py:61-276, kernels/cuda/model/kv_int8.py:210-247).

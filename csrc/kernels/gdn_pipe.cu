@@ -9,17 +9,18 @@
 //     of that.
 // gdn_chunk_kernel, whose four warps carry the state and form the outputs, waits for its chain of
 // some 2000 instructions a chunk and fills 30 % of the issue slots; two of its CTAs fit an SM and
-// hide each other.  Here the chain is a third as long.  What bounds a round (about 5800 cycles) is
-// shared memory (4300 cycles of operands, the k rows once per eight channels) and the state warps'
-// chain.  On the way: code that does not stay in the instruction cache cost most (T, P and A
-// unrolled: 8500 cycles a round, rolled 6300); all loads ahead, four sums in turn instead of two,
-// state and output warps on schedulers of their own, or outputs held back until S^T k is through:
-// no change.  32 heads of 128 channels, with the convolution and the norm of then: one run of 1050
-// rows 205 -> 155 us, two 245 -> 181, one of 4000 725 -> 547, two of 250 71 -> 54, two of 64 29.1
-// -> 24.5, one of 40 24.4 -> 21.  With more CTAs than SMs, two waves of these stand against one of
-// two per SM: three runs of 40 rows 31 against 37, of 250 88 against 94, sixteen of 64 115 against
-// 127, and from some 400 rows on these win again (three of 1000 337 -> 315, eight of 500 364 ->
-// 349).
+// hide each other.  Here the chain is a third as long.  What bounds a round (about 6300 cycles) is
+// shared memory (its pipe is busy for 4300 of them: operands, the k rows once per eight channels)
+// and the state warps' chain; issue slots are 45 % in use, the tensor core 37 %.  On the way: code
+// that does not stay in the instruction cache cost most (T, P and A unrolled: 8500 cycles a round,
+// rolled 6300); all loads ahead, four sums in turn instead of two, state and output warps on
+// schedulers of their own, or outputs held back until S^T k is through: no change.  32 heads of 128
+// channels, with the convolution and the norm of then: one run of 1050 rows 205 -> 155 us, two 245
+// -> 181, one of 4000 725 -> 547, two of 250 71 -> 54, two of 64 29.1 -> 24.5, one of 40 24.4 ->
+// 21.
+// With more CTAs than SMs, two waves of these stand against one of two per SM: three runs of 40
+// rows 31 against 37, of 250 88 against 94, sixteen of 64 115 against 127, and from some 400 rows
+// on these win again (three of 1000 337 -> 315, eight of 500 364 -> 349).
 #include "api.h"
 #include "common.cuh"
 #include "gdn_chunk.cuh"

@@ -18,18 +18,19 @@
 // accumulators (MT = 1 or 2).
 //
 // What bounds it: INT8 weights take 67 cycles per 128 x 128 x 32 MMA when their copies are there
-// (2048 x 19456 x 2560 126 -> 86 us, 2.4 PFLOP/s).  Lattice codes: the decode warps (66 % of the
-// issue slots).  With all sixteen on one k-block, each decoded for 540 to 650 of its 1280 to 1500
-// cycles; the rest were two waits (170 each), the fence and the hand-overs.  So groups of them take
-// k-blocks in turn, each warp with twice (Q2 with one row tile: four times) as many rows between
-// two waits: 128 Q4 experts of 768, a whole layer, 2048 rows 292 -> 270 us, 1024 rows 243 -> 210,
-// 300 rows 211 -> 179; 512 Q2 experts of 512, 2048 rows 619 -> 539, 1024 rows 519 -> 439 (Q4 in
-// four groups: 223 where two take 214).  Signs from arithmetic instead of lookups made a layer a
-// sixth longer; codes loaded into registers from global memory four k-blocks ahead, with a 64 KB
-// table whose addresses are single byte permutes (a quarter fewer instructions), 303 against 292
-// us: the loads are waited for.  The whole layer came from 447 us over 340 (this kernel) and 326
-// (the router's and the launches' share; votes on every wait and the activations' own barrier cost
-// 1.5 %), and 15 us of 305 went with lookups that collide.
+// (2048 x 19456 x 2560 126 -> 86 us, 2.4 PFLOP/s).  Lattice codes: the decode warps (67 % of the
+// issue slots, the shared-memory pipe as busy, the tensor core 27 %).  With all sixteen on one
+// k-block, each decoded for 540 to 650 of its 1280 to 1500 cycles; the rest were two waits (170
+// each), the fence and the hand-overs.  So groups of them take k-blocks in turn, each warp with
+// twice (Q2 with one row tile: four times) as many rows between two waits: 128 Q4 experts of 768, a
+// whole layer, 2048 rows 292 -> 270 us, 1024 rows 243 -> 210, 300 rows 211 -> 179; 512 Q2 experts
+// of 512, 2048 rows 619 -> 539, 1024 rows 519 -> 439 (Q4 in four groups: 223 where two take 214).
+// Signs from arithmetic instead of lookups made a layer a sixth longer; codes loaded into registers
+// from global memory four k-blocks ahead, with a 64 KB table whose addresses are single byte
+// permutes (a quarter fewer instructions), 303 against 292 us: the loads are waited for.  The whole
+// layer came from 447 us over 340 (this kernel) and 326 (the router's and the launches' share;
+// votes on every wait and the activations' own barrier cost 1.5 %), and 15 us of 305 went with
+// lookups that collide.
 #include <cuda.h>
 
 #include "api.h"
