@@ -1,6 +1,8 @@
 // C ABI of liborinfer_kernels.so.  Every entry point takes raw device pointers and
 // the CUDA stream to launch on, returns 0 on success, a negative value for a
 // rejected argument, or the cudaError_t of the launch.  None of them synchronises.
+// Projections that split their channels over CTAs share one workspace per device, so that
+// projections on one device belong on one stream, or on streams that wait for one another.
 #pragma once
 
 #include <cuda_fp16.h>

@@ -321,6 +321,33 @@ def test_attention_rows_keep_the_bits_of_small_value_scales(dev, qh, kvh, n, spl
     assert bool(((out.double() - ref).abs() <= lim).all())
 
 
+# scores that leap by many binades from block to block, up or down, over tiny value scales: references
+# move, units follow as far as they go
+@pytest.mark.parametrize("leap", [5, 20, 70, 130])
+@pytest.mark.parametrize("up", [True, False])
+@pytest.mark.parametrize("d", [64, 128])
+def test_attention_rows_of_scores_that_leap(dev, leap, up, d):
+    from orinfer_b200.ops import functional as F
+    n, qh = 128 * 6, 4
+    q, req, pos, table, kc, vc, ks, vs = _walk(dev, n, qh, 1, d, leap)
+    assert _in_digits(qh, 1, d, table, 1)
+    step = torch.arange(n, device=dev) // 128               # a block of each warp per step
+    kc[table[0].long()] = torch.randint(-9, 10, (6, 128, 1, d), device=dev, dtype=torch.int8)
+    flat = (table[0].long()[:, None] * 128 + torch.arange(128, device=dev)).flatten()
+    kc.view(-1, 1, d)[flat, :, 0] = (20 * (step if up else 5 - step))[:, None].to(torch.int8)
+    ks[:] = 1 / 64
+    q[..., 0] = leap * math.log(2) * math.sqrt(d) * 64 / 20
+    vs.view(-1, 1, d // 64)[flat] = (vs.view(-1, 1, d // 64)[flat].float() + 0.01).half()
+    small = step % 2 == (0 if up else 1)                     # every other step's scales are tiny
+    vs.view(-1, 1, d // 64)[flat[small]] *= 2.0 ** -9
+    out = F.attention(q, None, req, pos, table, kc, vc, ks, vs, splits=1).view(-1)
+    pick = lambda c: c[table[0].long()].reshape(-1, *c.shape[2:])[:n]
+    ref = _attention64(q[0], pick(kc), pick(vc), pick(ks), pick(vs)).reshape(-1)
+    # one FP16 rounding; scores of up to 650 binades in FP32, 2^-15 of a weight
+    lim = ref.abs() * (2.0 ** -11 + 2.0 ** -14) + 2.0 ** -14 * ref.abs().max() + 2.0 ** -25
+    assert bool(((out.double() - ref).abs() <= lim).all())
+
+
 # a group of query values far below the other, whose keys make up for it: seen in the records of the
 # splits, which no FP16 rounding hides
 @pytest.mark.parametrize("k", [8, 16, 22])
